@@ -46,6 +46,7 @@ struct BwdParams {
     __half* dq; __half* dk; __half* dv;
     long long sdq_b, sdq_h, sdq_t, sdk_b, sdk_h, sdk_t, sdv_b, sdv_h, sdv_t;
     int B, H, T, Tpad;
+    int d;                      // head_dim: D or less (columns [d, D) read as zero and are not stored)
     int causal;
     float scale;
     unsigned int* err;
@@ -489,7 +490,7 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 #pragma unroll
             for (int c = 0; c < NP; ++c) {
                 const int row = row0 + c;
-                if (row < p.T) {
+                if (row < p.T && col < p.d) {
                     *reinterpret_cast<uint4*>(dkb + (long long)row * p.sdk_t) = kc[c];
                     *reinterpret_cast<uint4*>(dvb + (long long)row * p.sdv_t) = vc[c];
                 }
@@ -728,10 +729,11 @@ attn_bwd_dq_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             transpose_pieces<NP>(qc, (uint32_t)lane);
             const int row0 = pend_row - lane + (lane & ~(NP - 1));
             __half* qb = pend_ptr + (lane & (NP - 1)) * 8;     // row 0 of the slice, this lane's piece
+            const bool col_ok = g * DH + (lane & (NP - 1)) * 8 < p.d;
 #pragma unroll
             for (int c = 0; c < NP; ++c) {
                 const int row = row0 + c;
-                if (row < p.T) *reinterpret_cast<uint4*>(qb + (long long)row * p.sdq_t) = qc[c];
+                if (row < p.T && col_ok) *reinterpret_cast<uint4*>(qb + (long long)row * p.sdq_t) = qc[c];
             }
             return true;
         };
@@ -953,7 +955,7 @@ attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     const int row = row0 + c;
-                    if (row < p.T) *reinterpret_cast<uint4*>(qb + (long long)row * p.sdq_t + part * 64) = pc[c];
+                    if (row < p.T && part * 64 + (lane & 7) * 8 < p.d) *reinterpret_cast<uint4*>(qb + (long long)row * p.sdq_t + part * 64) = pc[c];
                 }
             }
         }
@@ -971,7 +973,7 @@ attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const
 template <int D>
 __global__ void __launch_bounds__(256)
 attn_bwd_prep_f16_kernel(const __half* __restrict__ o, const __half* __restrict__ d_o, const float* __restrict__ lse,
-                         float* __restrict__ delta, float* __restrict__ lse2, int B, int H, int T, int Tpad,
+                         float* __restrict__ delta, float* __restrict__ lse2, int B, int H, int T, int d, int Tpad,
                          long long so_b, long long so_h, long long so_t, long long sdo_b, long long sdo_h,
                          long long sdo_t) {
     constexpr int LPR = D / 8;                               // lanes per row
@@ -994,7 +996,7 @@ attn_bwd_prep_f16_kernel(const __half* __restrict__ o, const __half* __restrict_
             valid[u] = row[u] < rows && t < (unsigned)T;
             a[u] = make_uint4(0u, 0u, 0u, 0u);
             g[u] = a[u];
-            if (valid[u]) {
+            if (valid[u] && sub * 8 < d) {
                 const unsigned b = bh / (unsigned)H, h = bh % (unsigned)H;
                 a[u] = *reinterpret_cast<const uint4*>(o + b * so_b + h * so_h + (long long)t * so_t + sub * 8);
                 g[u] = *reinterpret_cast<const uint4*>(d_o + b * sdo_b + h * sdo_h + (long long)t * sdo_t + sub * 8);
@@ -1032,10 +1034,10 @@ int bwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
                const float* lse, const void* d_o, void* dq, void* dk, void* dv, void* workspace, bool keep_ds) {
     CUtensorMap tq, tk, tv, tdo;
     int rc;
-    if ((rc = make_tmap_bhtd_f16(ctx, &tq, q, d->B, d->H, d->T, D, d->q_strides, BT))) return rc;
-    if ((rc = make_tmap_bhtd_f16(ctx, &tk, k, d->B, d->H, d->T, D, d->k_strides, BT))) return rc;
-    if ((rc = make_tmap_bhtd_f16(ctx, &tv, v, d->B, d->H, d->T, D, d->v_strides, BT))) return rc;
-    if ((rc = make_tmap_bhtd_f16(ctx, &tdo, d_o, d->B, d->H, d->T, D, d->do_strides, BT))) return rc;
+    if ((rc = make_tmap_bhtd_f16(ctx, &tq, q, d->B, d->H, d->T, d->D, d->q_strides, BT))) return rc;
+    if ((rc = make_tmap_bhtd_f16(ctx, &tk, k, d->B, d->H, d->T, d->D, d->k_strides, BT))) return rc;
+    if ((rc = make_tmap_bhtd_f16(ctx, &tv, v, d->B, d->H, d->T, d->D, d->v_strides, BT))) return rc;
+    if ((rc = make_tmap_bhtd_f16(ctx, &tdo, d_o, d->B, d->H, d->T, d->D, d->do_strides, BT))) return rc;
     const int nq = (d->T + BT - 1) / BT;
     const int Tpad = nq * BT;
     const long long BH = (long long)d->B * d->H;
@@ -1051,7 +1053,7 @@ int bwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
         const long long want = (prep_rows + per_block - 1) / per_block;
         const unsigned prep_grid = (unsigned)(want < 8LL * ctx->sm_count ? want : 8LL * ctx->sm_count);
         attn_bwd_prep_f16_kernel<D><<<prep_grid, 256, 0, ctx->stream>>>(
-            (const __half*)o, (const __half*)d_o, lse, delta, lse2, d->B, d->H, d->T, Tpad, d->o_strides[0],
+            (const __half*)o, (const __half*)d_o, lse, delta, lse2, d->B, d->H, d->T, d->D, Tpad, d->o_strides[0],
             d->o_strides[1], d->o_strides[2], d->do_strides[0], d->do_strides[1], d->do_strides[2]);
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -1062,7 +1064,7 @@ int bwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
     p.sdq_b = d->dq_strides[0]; p.sdq_h = d->dq_strides[1]; p.sdq_t = d->dq_strides[2];
     p.sdk_b = d->dk_strides[0]; p.sdk_h = d->dk_strides[1]; p.sdk_t = d->dk_strides[2];
     p.sdv_b = d->dv_strides[0]; p.sdv_h = d->dv_strides[1]; p.sdv_t = d->dv_strides[2];
-    p.B = d->B; p.H = d->H; p.T = d->T; p.Tpad = Tpad; p.causal = d->causal; p.scale = d->scale;
+    p.B = d->B; p.H = d->H; p.T = d->T; p.Tpad = Tpad; p.d = d->D; p.causal = d->causal; p.scale = d->scale;
     p.err = ctx->dev_err;
     p.ds_pairs = d->causal ? (long long)nq * (nq + 1) / 2 : (long long)nq * nq;
     p.ds = keep_ds ? (__half*)((char*)workspace + 2 * stat_bytes) : nullptr;
@@ -1072,8 +1074,8 @@ int bwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
     const unsigned persistent = (unsigned)(grid < ctx->sm_count ? grid : ctx->sm_count);
     p.sched = deers_get_schedule(ctx, d->B, d->H, nq, d->causal, (int)persistent, &p.sched_rows);
     const size_t smem_a = DkvSmem<D>::TOTAL, smem_b = DqSmem<D>::TOTAL;
-    DEERS_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_bwd_dkdv_f16_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
-    DEERS_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_bwd_dq_f16_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
+    DEERS_SMEM_ONCE(ctx, (attn_bwd_dkdv_f16_kernel<D>), smem_a);
+    DEERS_SMEM_ONCE(ctx, (attn_bwd_dq_f16_kernel<D>), smem_b);
     {
         KernelTimerScope ts(ctx, DEERS_K_BWD_MAIN);
         attn_bwd_dkdv_f16_kernel<D><<<persistent, DKV_THREADS, smem_a, ctx->stream>>>(tq, tk, tv, tdo, p);
@@ -1081,7 +1083,7 @@ int bwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     if (keep_ds) {
         const size_t smem_c = DqsSmem<D>::TOTAL;
-        DEERS_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_bwd_dq_from_ds_f16_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c));
+        DEERS_SMEM_ONCE(ctx, (attn_bwd_dq_from_ds_f16_kernel<D>), smem_c);
         KernelTimerScope ts(ctx, DEERS_K_BWD_DQ);
         attn_bwd_dq_from_ds_f16_kernel<D><<<persistent, 192, smem_c, ctx->stream>>>(tk, p);
     } else {
@@ -1109,9 +1111,9 @@ size_t attn_bwd_f16_workspace_bytes(const deers_attn_desc* d, bool keep_ds) {
 int launch_attn_bwd_f16(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const void* k, const void* v,
                         const void* o, const float* lse, const void* d_o, void* dq, void* dk, void* dv,
                         void* workspace, bool keep_ds) {
-    if (d->D == 64) return bwd_launch<64>(ctx, d, q, k, v, o, lse, d_o, dq, dk, dv, workspace, keep_ds);
-    if (d->D == 128) return bwd_launch<128>(ctx, d, q, k, v, o, lse, d_o, dq, dk, dv, workspace, keep_ds);
-    return DEERS_ERR_UNSUPPORTED;
+    // Any multiple of 8: columns between head_dim and the tile width are zero-filled by TMA and never stored.
+    if (d->D <= 64) return bwd_launch<64>(ctx, d, q, k, v, o, lse, d_o, dq, dk, dv, workspace, keep_ds);
+    return bwd_launch<128>(ctx, d, q, k, v, o, lse, d_o, dq, dk, dv, workspace, keep_ds);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1139,7 +1141,7 @@ int deers_b200_attn_bwd_f16_static(deers_ctx* ctx, const deers_attn_desc* d, con
     const int rc = deers_check_bwd_args(d, q, k, v, o, lse, d_o, dq, dk, dv);
     if (rc) return rc;
     if (d->dtype != DEERS_F16) return DEERS_ERR_DTYPE;
-    if (d->D != 64 && d->D != 128) return DEERS_ERR_UNSUPPORTED;      // the zero-padded path needs room for copies
+    if (d->D != 64 && d->D != 128) return DEERS_ERR_UNSUPPORTED;      // this entry point serves the full tile widths
     if (ctx->device < 0 || ctx->device >= 64) return DEERS_ERR_DEVICE;
     const size_t need = attn_bwd_f16_workspace_bytes(d, false);
     if (need > sizeof(float) * kStaticScratchFloats) {

@@ -47,6 +47,7 @@ struct FwdParams {
     float* lse;
     long long so_b, so_h, so_t;
     int B, H, T;
+    int d;                      // head_dim: D or less (columns [d, D) read as zero and are not stored)
     int causal;
     float scale;
     unsigned int* err;
@@ -323,11 +324,12 @@ attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             }
             transpose_pieces<NP>(oc, (uint32_t)lane);
             const int grow0 = pend_grow - lane + (lane & ~(NP - 1));
-            __half* ob = p.o + b * p.so_b + h * p.so_h + g * DH + (lane & (NP - 1)) * 8;
+            const int col = g * DH + (lane & (NP - 1)) * 8;
+            __half* ob = p.o + b * p.so_b + h * p.so_h + col;
 #pragma unroll
             for (int c = 0; c < NP; ++c) {
                 const int grow = grow0 + c;
-                if (grow < p.T) *reinterpret_cast<uint4*>(ob + (long long)grow * p.so_t) = oc[c];
+                if (grow < p.T && col < p.d) *reinterpret_cast<uint4*>(ob + (long long)grow * p.so_t) = oc[c];
             }
             if (g == 0 && pend_grow < p.T) p.lse[(long long)pend_bh * p.T + pend_grow] = (pend_m + log2f(l)) * LN2;
             return true;
@@ -454,15 +456,15 @@ int fwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
                float* lse) {
     CUtensorMap tq, tk, tv;
     int rc;
-    if ((rc = make_tmap_bhtd_f16(ctx, &tq, q, d->B, d->H, d->T, D, d->q_strides, BM))) return rc;
-    if ((rc = make_tmap_bhtd_f16(ctx, &tk, k, d->B, d->H, d->T, D, d->k_strides, BN))) return rc;
-    if ((rc = make_tmap_bhtd_f16(ctx, &tv, v, d->B, d->H, d->T, D, d->v_strides, BN))) return rc;
+    if ((rc = make_tmap_bhtd_f16(ctx, &tq, q, d->B, d->H, d->T, d->D, d->q_strides, BM))) return rc;
+    if ((rc = make_tmap_bhtd_f16(ctx, &tk, k, d->B, d->H, d->T, d->D, d->k_strides, BN))) return rc;
+    if ((rc = make_tmap_bhtd_f16(ctx, &tv, v, d->B, d->H, d->T, d->D, d->v_strides, BN))) return rc;
     FwdParams p;
     p.o = (__half*)o; p.lse = lse;
     p.so_b = d->o_strides[0]; p.so_h = d->o_strides[1]; p.so_t = d->o_strides[2];
-    p.B = d->B; p.H = d->H; p.T = d->T; p.causal = d->causal; p.scale = d->scale; p.err = ctx->dev_err;
+    p.B = d->B; p.H = d->H; p.T = d->T; p.d = d->D; p.causal = d->causal; p.scale = d->scale; p.err = ctx->dev_err;
     const size_t smem = FwdSmem<D>::TOTAL;
-    DEERS_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_fwd_f16_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DEERS_SMEM_ONCE(ctx, (attn_fwd_f16_kernel<D>), smem);
     const long long nq = (d->T + BM - 1) / BM;
     const long long items = nq * d->B * d->H;
     if (items > 0x7fffffffLL) return DEERS_ERR_SHAPE;
@@ -481,7 +483,8 @@ int fwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
 
 int launch_attn_fwd_f16(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const void* k, const void* v,
                         void* o, float* lse) {
-    if (d->D == 64) return fwd_launch<64>(ctx, d, q, k, v, o, lse);
-    if (d->D == 128) return fwd_launch<128>(ctx, d, q, k, v, o, lse);
-    return DEERS_ERR_UNSUPPORTED;
+    // Any multiple of 8: TMA fills the columns between head_dim and the tile width with zeros (they change neither
+    // Q K^T nor P V), and the epilogue does not store them.
+    if (d->D <= 64) return fwd_launch<64>(ctx, d, q, k, v, o, lse);
+    return fwd_launch<128>(ctx, d, q, k, v, o, lse);
 }

@@ -7,6 +7,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
+
 #include "../../include/deers_b200.h"
 
 constexpr int DEERS_KT_RING = 512;
@@ -85,6 +87,18 @@ struct KernelTimerScope {
                      cudaGetErrorString(_e));                                                 \
             return DEERS_ERR_CUDA;                                                            \
         }                                                                                     \
+    } while (0)
+
+// Opts a kernel into `bytes` of dynamic shared memory, once per call site (kernel instantiation) and device: the
+// attribute stays with the function, and setting it on every launch costs the host about as much as a tensor map.
+#define DEERS_SMEM_ONCE(ctx, kernel, bytes)                                                                         \
+    do {                                                                                                            \
+        static std::atomic<unsigned long long> _done{0};                                                            \
+        const unsigned long long _bit = 1ull << ((ctx)->device & 63);                                               \
+        if (!(_done.load(std::memory_order_acquire) & _bit)) {                                                      \
+            DEERS_CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes))); \
+            _done.fetch_or(_bit, std::memory_order_release);                                                        \
+        }                                                                                                           \
     } while (0)
 
 // Device-side error codes (upper byte: which kernel, lower bits: which wait).

@@ -1,0 +1,37 @@
+"""Kernel and dispatch edges: the sizes where a tile, a remainder or a choice of variant can go wrong, against the
+CPU oracle (or float64 where the oracle has no such op)."""
+import numpy as np
+import pytest
+import torch
+
+from tests.helpers import TOL_F16, assert_close
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D,T", [(8, 1), (56, 129), (72, 127), (80, 300), (120, 257)])
+def test_f16_head_dims_in_place_with_strided_rows(D, T):
+    """Head dims between the tile widths: the columns a tile has beyond head_dim must neither be read (they belong to
+    the neighbouring head of a [B,T,3C] buffer here) nor written (the output is a slice of a larger buffer)."""
+    from deers_b200 import ops
+    from oracle import ref
+    B, H = 2, 3
+    C = H * D
+    rng = np.random.default_rng(D + T)
+    qkv = torch.from_numpy(rng.standard_normal((B, T, 3 * C)).astype(np.float16)).cuda()
+    q, k, v = (qkv[..., i * C:(i + 1) * C].view(B, T, H, D).permute(0, 2, 1, 3) for i in range(3))
+    do = torch.from_numpy(rng.standard_normal((B, H, T, D)).astype(np.float16)).cuda()
+    big = torch.full((B, T, H, D + 8), 7.0, dtype=torch.float16, device="cuda")
+    out = big[..., :D].permute(0, 2, 1, 3)
+    scale = ops.default_scale(D)
+    o, lse = ops.attention_fwd(q, k, v, scale, out=out)
+    dvb = torch.full((B, T, H, D + 8), 7.0, dtype=torch.float16, device="cuda")
+    for ws_pass in (1, 2):
+        ws = torch.empty(ops.workspace_bytes(q, scale, True, ws_pass), dtype=torch.uint8, device="cuda")
+        dq, dk, dv = ops.attention_bwd(q, k, v, o, lse, do, scale, workspace=ws, dv_out=dvb[..., :D].permute(0, 2, 1, 3))
+        ops.Context.current(q.device).sync()
+        host = [t.float().cpu().numpy() for t in (q, k, v, do)]
+        want = ref.attn_fwd_bwd(*[np.ascontiguousarray(a) for a in host])
+        for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), (o, lse, dq, dk, dv), want):
+            assert_close(g.float().cpu().numpy(), w, TOL_F16, f"D {D} T {T} {name}")
+    assert torch.all(big[..., D:] == 7.0) and torch.all(dvb[..., D:] == 7.0), "columns beyond head_dim are not ours"
