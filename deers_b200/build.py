@@ -12,6 +12,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libdeers_b200.so")
+HOST_SRC = os.path.join(CSRC, "host_ext.cpp")
+HOST_EXT = os.path.join(LIB_DIR, "_deers_host.so")      # native host layer of the Python mirror (ops.py)
 SOURCES = ["ctx.cu", "attn_f32.cu", "umma_selftest.cu", "attn_fwd_f16_sm100.cu", "attn_bwd_f16_sm100.cu",
            "rope_pack.cu", "optim.cu", "rmsnorm.cu", "attn_decode.cu", "gemm_f16_sm100.cu", "gemm_f16x3_sm100.cu", "gemm_f32.cu",
            "gpt_ops.cu", "gpt_model.cu", "comm.cu"]
@@ -62,5 +64,29 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def build_host(force: bool = False, verbose: bool = False) -> str:
+    """The CPython extension ops.py calls: host code only, linked against the library above and torch."""
+    header = os.path.join(HERE, "..", "include", "deers_b200.h")
+    if not force and not _stale(HOST_EXT, [HOST_SRC, header]):
+        return HOST_EXT
+    import sysconfig
+
+    import torch
+    t = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{t}/include",
+           f"-I{t}/include/torch/csrc/api/include", f"-I{cuda}/include", f"-I{sysconfig.get_paths()['include']}", HOST_SRC,
+           "-o", HOST_EXT, f"-L{LIB_DIR}", "-ldeers_b200", f"-L{t}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
+           "-ltorch", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    out = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if out.returncode != 0 or verbose:
+        sys.stderr.write(f"--- host_ext.cpp\n{out.stdout}\n")
+    if out.returncode != 0:
+        raise RuntimeError("g++ failed")
+    return HOST_EXT
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
+    print(build_host(force="--force" in sys.argv, verbose="--verbose" in sys.argv))

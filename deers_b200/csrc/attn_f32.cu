@@ -521,17 +521,10 @@ bool rows_vec_ok(const void* ptr, const int64_t* s) {
     return (((uintptr_t)ptr) & 15u) == 0 && (s[0] & 3) == 0 && (s[1] & 3) == 0 && (s[2] & 3) == 0;
 }
 
-template <typename K>
-int set_smem(deers_ctx* ctx, K kernel, size_t bytes) {
-    DEERS_CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    return DEERS_OK;
-}
-
 template <int DP>
 int fwd_impl(deers_ctx* ctx, const F32Params& p) {
     const size_t smem = (size_t)(3 * BM * (DP + 4) + BM * PLD) * sizeof(float);
-    int rc = set_smem(ctx, attn_fwd_f32_kernel<DP>, smem);
-    if (rc) return rc;
+    DEERS_SMEM_ONCE(ctx, (attn_fwd_f32_kernel<DP>), smem);
     dim3 grid((p.T + BM - 1) / BM, p.B * p.H);
     {
         KernelTimerScope ts(ctx, DEERS_K_FWD);
@@ -553,8 +546,7 @@ int bwd_impl(deers_ctx* ctx, const F32Params& p) {
     const size_t smem_kv = (size_t)(4 * BM * (DP + 4) + 2 * BM * PLD + 2 * BM) * sizeof(float);
     const size_t smem_q = (size_t)(4 * BM * (DP + 4) + BM * PLD + 2 * BM) * sizeof(float);
     const size_t smem = smem_kv > smem_q ? smem_kv : smem_q;
-    int rc = set_smem(ctx, attn_bwd_f32_kernel<DP>, smem);
-    if (rc) return rc;
+    DEERS_SMEM_ONCE(ctx, (attn_bwd_f32_kernel<DP>), smem);
     dim3 grid((p.T + BM - 1) / BM, p.B * p.H, 2);
     {
         KernelTimerScope ts(ctx, DEERS_K_BWD_MAIN);

@@ -190,7 +190,7 @@ int make_tmap_matrix(deers_ctx* ctx, CUtensorMap* out, const void* base, long lo
 
 template <int A_MN, int B_MN>
 int gemm_launch(deers_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p) {
-    DEERS_CUDA_TRY(ctx, cudaFuncSetAttribute(gemm_f16_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM));
+    DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<A_MN, B_MN>), G_SMEM);
     const long long tiles = (long long)((p.M + GM - 1) / GM) * ((p.N + GN - 1) / GN);
     const unsigned grid = (unsigned)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
     {

@@ -318,7 +318,7 @@ X3Plan x3_plan(int M, int N, int K, int sm_count) {
 
 template <int A_MN, int B_MN>
 int x3_launch(deers_ctx* ctx, const CUtensorMap* t, const X3Params& p, unsigned grid) {
-    DEERS_CUDA_TRY(ctx, cudaFuncSetAttribute(gemm_f16x3_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)X_SMEM));
+    DEERS_SMEM_ONCE(ctx, (gemm_f16x3_kernel<A_MN, B_MN>), X_SMEM);
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM_X3);
         gemm_f16x3_kernel<A_MN, B_MN><<<grid, X_THREADS, X_SMEM, ctx->stream>>>(t[0], t[1], t[2], t[3], p);

@@ -26,6 +26,24 @@ from .errors import DeviceMismatch, DTypeMismatch, LayoutMismatch
 _DTYPES = {torch.float16: _lib.F16, torch.float32: _lib.F32}
 
 
+def _load_host():
+    """The native host layer (csrc/host_ext.cpp): argument checks, allocation and the C-ABI call of an operator in one
+    CPython call.  Like the library it has no fallback."""
+    import importlib.machinery
+    import importlib.util
+    import os
+    path = os.path.join(os.path.dirname(_lib.LIB_PATH), "_deers_host.so")
+    if not os.path.exists(path):
+        raise ImportError(f"{path} is missing: run `python -m deers_b200.build`")
+    loader = importlib.machinery.ExtensionFileLoader("_deers_host", path)
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_deers_host", loader))
+    loader.exec_module(mod)
+    return mod
+
+
+_host = _load_host()
+
+
 class Context:
     """One library context per (device, stream): the analogue of deers' global CudaRuntime
     (src/storage/cuda.rs:455-521).  Work is enqueued on torch's current stream."""
@@ -54,6 +72,11 @@ class Context:
             ctx._stream_obj = stream_obj     # keeps the stream alive: its handle value cannot be reused by another
             cls._cache[key] = ctx
         return ctx
+
+    @classmethod
+    def _handle_for(cls, device: int) -> int:
+        """The handle of the current stream's context, for the native host layer."""
+        return cls.current(torch.device("cuda", device)).handle.value
 
     def sync(self) -> None:
         """Device::synchronize (src/device.rs:66-72); raises if a kernel reported an error."""
@@ -85,6 +108,9 @@ class Context:
         return [float(e) for e in errs]
 
 
+_host.setup(Context._handle_for, lambda status, handle: _lib.check(status, ctypes.c_void_p(handle)))
+
+
 def _strides(t: torch.Tensor):
     return (ctypes.c_int64 * 4)(*t.stride())
 
@@ -112,7 +138,8 @@ def _usable(t: torch.Tensor) -> bool:
     align = 16 if t.dtype == torch.float16 else 4
     if t.data_ptr() % align:
         return False
-    return all((t.stride(i) * esize) % align == 0 or t.shape[i] == 1 for i in range(3))
+    narrow = esize == 2 and t.shape[3] not in (64, 128)      # expanded axes are compacted there (host_ext.cpp)
+    return all(t.shape[i] == 1 or ((t.stride(i) * esize) % align == 0 and not (narrow and t.stride(i) == 0)) for i in range(3))
 
 
 def _compact(t: torch.Tensor) -> torch.Tensor:
@@ -131,6 +158,12 @@ def _desc(q, k, v, o, d_o=None, dq=None, dk=None, dv=None, scale=1.0, causal=Tru
     return d
 
 
+def _taken(name: str, result):
+    if result is None:
+        raise LayoutMismatch(f"{name}: the arguments are not tensors of one CUDA device")
+    return result
+
+
 def default_scale(head_dim: int) -> float:
     """1/sqrt(head_dim) computed in f64 as the module does (src/models/gpt.rs:139)."""
     return 1.0 / math.sqrt(float(head_dim))
@@ -147,27 +180,15 @@ def attention_fwd(q, k, v, scale: float, causal: bool = True, token_major_out: b
     and the returned tensor is the [B,H,T,D] view of it, so the module's
     ``permute([0,2,1,3]).reshape([B,T,C])`` (src/models/gpt.rs:144) is a free view instead of the
     compaction copy of src/ops.rs:913: the kernels write through the view's strides."""
+    got = _host.attn_fwd(q, k, v, scale, causal, token_major_out, out)
+    if got is not None:
+        return got
     _check_inputs("attention_fwd", (q, k, v))
     q, k, v = _compact(q), _compact(k), _compact(v)
-    ctx = Context.current(q.device)
-    if out is not None:
-        if out.shape != q.shape or out.dtype != q.dtype or out.device != q.device or not _usable(out):
-            raise LayoutMismatch(f"attention_fwd: out must match q ({tuple(q.shape)}, {q.dtype}) with unit inner stride")
-        o = out
-    elif token_major_out:
-        B, H, T, D = q.shape
-        o = torch.empty((B, T, H, D), dtype=q.dtype, device=q.device).permute(0, 2, 1, 3)
-    else:
-        o = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-    lse = torch.empty(q.shape[:3], dtype=torch.float32, device=q.device)
-    d = _desc(q, k, v, o, scale=scale, causal=causal)
-    # The forward needs scratch only for f16 head dims other than 64 / 128 (zero-padded copies of Q, K, V, O).
-    need = int(_lib.lib().deers_b200_attn_workspace_bytes(ctypes.byref(d), 0))
-    ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
-    _lib.check(_lib.lib().deers_b200_attn_fwd(ctx.handle, ctypes.byref(d), q.data_ptr(), k.data_ptr(),
-                                              v.data_ptr(), o.data_ptr(), lse.data_ptr(),
-                                              ws.data_ptr() if need else None, need), ctx.handle)
-    return o, lse
+    Context.current(q.device)                # raises for a CPU tensor
+    if out is not None and (out.shape != q.shape or out.dtype != q.dtype or out.device != q.device or not _usable(out)):
+        raise LayoutMismatch(f"attention_fwd: out must match q ({tuple(q.shape)}, {q.dtype}) with unit inner stride")
+    return _taken("attention_fwd", _host.attn_fwd(q, k, v, scale, causal, token_major_out, out))
 
 
 def workspace_bytes(q, scale: float = 1.0, causal: bool = True, pass_: int = 1) -> int:
@@ -182,30 +203,15 @@ def attention_bwd(q, k, v, o, lse, d_o, scale: float, causal: bool = True, works
     `pass_=1` bytes the recomputing one; without it the function allocates.  `dv_out` (a [B,H,T,D] view
     with inner stride 1, e.g. the v slice of a fused dqkv buffer seen head-major) receives dV in place
     instead: the kernels write through its strides."""
+    got = _host.attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace, dv_out)
+    if got is not None:
+        return got
     _check_inputs("attention_bwd", (q, k, v, o, d_o))
     q, k, v, o, d_o = _compact(q), _compact(k), _compact(v), _compact(o), _compact(d_o)
-    ctx = Context.current(q.device)
-    dq, dk = (torch.empty(q.shape, dtype=q.dtype, device=q.device) for _ in range(2))
-    if dv_out is not None:
-        if tuple(dv_out.shape) != tuple(q.shape) or dv_out.dtype != q.dtype or not _usable(dv_out):
-            raise LayoutMismatch("attention_bwd: dv_out must be a [B,H,T,D] view with inner stride 1 and aligned rows")
-        dv = dv_out
-    else:
-        dv = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-    d = _desc(q, k, v, o, d_o, dq, dk, dv, scale=scale, causal=causal)
-    need = int(_lib.lib().deers_b200_attn_workspace_bytes(ctypes.byref(d), 1))
-    if workspace is None or workspace.numel() * workspace.element_size() < need:
-        # The larger size lets the f16 backward keep its dS tiles (two tile products fewer); taken when it is
-        # a small part of what the device has free, else the backward recomputes.
-        fast = int(_lib.lib().deers_b200_attn_workspace_bytes(ctypes.byref(d), 2))
-        if fast > need and fast <= torch.cuda.mem_get_info(q.device)[0] // 4:
-            need = fast
-        workspace = torch.empty(max(need, 256), dtype=torch.uint8, device=q.device)
-    _lib.check(_lib.lib().deers_b200_attn_bwd(ctx.handle, ctypes.byref(d), q.data_ptr(), k.data_ptr(),
-                                              v.data_ptr(), o.data_ptr(), lse.data_ptr(), d_o.data_ptr(),
-                                              dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), workspace.data_ptr(),
-                                              workspace.numel() * workspace.element_size()), ctx.handle)
-    return dq, dk, dv
+    Context.current(q.device)
+    if dv_out is not None and (tuple(dv_out.shape) != tuple(q.shape) or dv_out.dtype != q.dtype or not _usable(dv_out)):
+        raise LayoutMismatch("attention_bwd: dv_out must be a [B,H,T,D] view with inner stride 1 and aligned rows")
+    return _taken("attention_bwd", _host.attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace, dv_out))
 
 
 def precompute_rotary_embeddings(seq_len: int, head_dim: int, base: float = 10000.0,
@@ -222,17 +228,6 @@ def precompute_rotary_embeddings(seq_len: int, head_dim: int, base: float = 1000
     freqs = torch.arange(seq_len, dtype=torch.float32)[:, None] * inv_freq[None, :]
     shape = (1, seq_len, 1, half)
     return (freqs.cos().to(dtype).reshape(shape).to(device), freqs.sin().to(dtype).reshape(shape).to(device))
-
-
-def _rope_call(src, cos, sin, dst, src_strides, dst_strides, B, T, H, D, inverse: bool) -> None:
-    ctx = Context.current(src.device)
-    d = _lib.RopeDesc()
-    d.B, d.T, d.H, d.D = B, T, H, D
-    d.dtype, d.inverse = _DTYPES[src.dtype], int(inverse)
-    d.src_strides = (ctypes.c_int64 * 4)(*src_strides)
-    d.dst_strides = (ctypes.c_int64 * 4)(*dst_strides)
-    _lib.check(_lib.lib().deers_b200_rope_pack(ctx.handle, ctypes.byref(d), src.data_ptr(), cos.data_ptr(),
-                                               sin.data_ptr(), dst.data_ptr()), ctx.handle)
 
 
 def _check_rope(name: str, x, cos, sin, T: int, D: int):
@@ -278,8 +273,7 @@ class RotaryPack:
     def forward(self) -> torch.Tensor:
         B, T, H, D = self.x.shape
         y = torch.empty((B, H, T, D), dtype=self.x.dtype, device=self.x.device)
-        ys = y.stride()
-        _rope_call(self.x, self.cos, self.sin, y, self.x.stride(), (ys[0], ys[2], ys[1], ys[3]), B, T, H, D, False)
+        _taken("RotaryPack", _host.rope_pack(self.x, self.cos, self.sin, y, False, False))
         return y
 
     def backward(self, grads: "GradientStore", out_grad: torch.Tensor, dx_out: Optional[torch.Tensor] = None) -> None:
@@ -297,8 +291,7 @@ class RotaryPack:
             dx = dx_out
         else:
             dx = torch.empty((B, T, H, D), dtype=self.x.dtype, device=self.x.device)
-        gs = g.stride()
-        _rope_call(g, self.cos, self.sin, dx, (gs[0], gs[2], gs[1], gs[3]), dx.stride(), B, T, H, D, True)
+        _taken("RotaryPack.backward", _host.rope_pack(g, self.cos, self.sin, dx, True, True))
         grads.accumulate(self.x, dx)
 
     def dependencies(self) -> List[torch.Tensor]:
@@ -354,6 +347,8 @@ class CausalAttention:
     @classmethod
     def new(cls, q, k, v, scale: Optional[float] = None, causal: bool = True,
             token_major_out: bool = False) -> "CausalAttention":
+        if _host.compatible(q, k, v):
+            return cls(q, k, v, default_scale(q.shape[3]) if scale is None else scale, causal, token_major_out)
         _check_inputs("CausalAttention", (q, k, v))
         if q.device.type != "cuda":
             raise DeviceMismatch("CausalAttention: the fused op runs on the CUDA device only")
@@ -598,6 +593,11 @@ def attention_decode(q, k_cache, v_cache, scale: Optional[float] = None, causal:
     """``softmax(scale * q @ k^T + causal_mask(B, Tq, Tk - Tq)) @ v`` for Tq new rows against Tk cached rows
     (the mask of src/nn/functional.rs:12-55 with seqlen_offset = Tk - Tq).  q: [B,H,Tq,D]; caches:
     [B,H,Tk,D] (views of a larger cache are read in place).  Returns o [B,H,Tq,D] (and lse [B,H,Tq])."""
+    if scale is None and q.dim() == 4:
+        scale = default_scale(q.shape[3])
+    got = _host.attn_decode(q, k_cache, v_cache, scale, causal, want_lse) if scale is not None else None
+    if got is not None:
+        return got
     if q.dim() != 4 or k_cache.dim() != 4 or v_cache.dim() != 4:
         raise LayoutMismatch("attention_decode: expected [B, H, T, D] tensors")
     B, H, Tq, D = q.shape
@@ -614,31 +614,14 @@ def attention_decode(q, k_cache, v_cache, scale: Optional[float] = None, causal:
     if q.device.type != "cuda":
         raise DeviceMismatch("attention_decode: the op runs on the CUDA device only")
     q, k_cache, v_cache = (t if t.stride(3) == 1 else t.contiguous() for t in (q, k_cache, v_cache))
-    ctx = Context.current(q.device)
-    o = torch.empty_like(q, memory_format=torch.contiguous_format)
-    lse = torch.empty((B, H, Tq), dtype=torch.float32, device=q.device) if want_lse else None
-    d = _lib.DecodeDesc()
-    d.B, d.H, d.Tq, d.Tk, d.D = B, H, Tq, Tk, D
-    d.dtype, d.causal, d.scale = _DTYPES[q.dtype], int(causal), default_scale(D) if scale is None else float(scale)
-    d.q_strides, d.k_strides, d.v_strides, d.o_strides = _strides(q), _strides(k_cache), _strides(v_cache), _strides(o)
-    need = int(_lib.lib().deers_b200_attn_decode_workspace_bytes(ctypes.byref(d)))
-    ws = torch.empty(max(need, 256), dtype=torch.uint8, device=q.device)
-    _lib.check(_lib.lib().deers_b200_attn_decode(ctx.handle, ctypes.byref(d), q.data_ptr(), k_cache.data_ptr(),
-                                                 v_cache.data_ptr(), o.data_ptr(),
-                                                 lse.data_ptr() if lse is not None else None, ws.data_ptr(), need),
-               ctx.handle)
-    return (o, lse) if want_lse else o
+    return _taken("attention_decode", _host.attn_decode(q, k_cache, v_cache, scale, causal, want_lse))
 
 
 # ---------------------------------------------------------------------------------------------
 # Linear projections (f16): forward and the two backward products on the tcgen05 GEMM
 # ---------------------------------------------------------------------------------------------
-def _gemm(M, N, K, a, a_mn, b, b_mn, dev, dtype):
-    ctx = Context.current(dev)
-    c = torch.empty((M, N), dtype=dtype, device=dev)
-    _lib.check(_lib.lib().deers_b200_gemm_f16(ctx.handle, M, N, K, a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(),
-                                              b.stride(0), int(b_mn), c.data_ptr(), c.stride(0)), ctx.handle)
-    return c
+def _gemm(M, N, K, a, a_mn, b, b_mn):
+    return _taken("Linear", _host.gemm_f16(M, N, K, a, a_mn, b, b_mn))
 
 
 class Linear:
@@ -664,7 +647,7 @@ class Linear:
     def forward(self) -> torch.Tensor:
         K, N = self.weight.shape
         x2 = self.x.reshape(-1, K)
-        y = _gemm(x2.shape[0], N, K, x2, False, self.weight, True, self.x.device, self.x.dtype)
+        y = _gemm(x2.shape[0], N, K, x2, False, self.weight, True)
         return y.reshape(*self.x.shape[:-1], N)
 
     def backward(self, grads: GradientStore, out_grad: torch.Tensor) -> None:
@@ -673,8 +656,8 @@ class Linear:
         g2 = out_grad.reshape(-1, N)
         g2 = g2 if g2.is_contiguous() else g2.contiguous()
         rows = x2.shape[0]
-        dx = _gemm(rows, K, N, g2, False, self.weight, False, self.x.device, self.x.dtype)
-        dw = _gemm(K, N, rows, x2, True, g2, True, self.x.device, self.x.dtype)
+        dx = _gemm(rows, K, N, g2, False, self.weight, False)
+        dw = _gemm(K, N, rows, x2, True, g2, True)
         grads.accumulate(self.x, dx.reshape(self.x.shape))
         grads.accumulate(self.weight, dw)
 
