@@ -59,6 +59,7 @@ struct deers_ctx {
     cudaStream_t h2d_stream, d2h_stream;
     cudaEvent_t pipe_ev[3][3];      // [buffer set][h2d done, compute done, d2h done]
     bool pipe_ready;
+    int cluster_capacity[9];        // [n]: clusters of n blocks the device holds at once (gemm_f32.cu; 0: not asked yet)
 };
 
 // Brackets one kernel launch with events when timing is on.  A full ring drops the sample.
@@ -141,10 +142,8 @@ int run_selftest_umma(deers_ctx* ctx, float* max_abs_err);
 int run_selftest_wait(deers_ctx* ctx, unsigned int limit_ms, int* result_host);
 
 // f32 GEMM (gemm_f32.cu)
-size_t gemm_f32_workspace_bytes(const deers_ctx* ctx, int M, int N, int K);
 int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long long lda, int a_mn, const float* b,
-                    long long ldb, int b_mn, float* c, long long ldc, int epi, const float* r, long long ldr, float* aux,
-                    void* workspace, size_t ws_bytes, bool counters_zero);
+                    long long ldb, int b_mn, float* c, long long ldc, int epi, const float* r, long long ldr, float* aux);
 // RMSNorm (rmsnorm.cu)
 int launch_rmsnorm_fwd(deers_ctx* ctx, long long rows, int C, double eps, const float* x, float* y, float* inv_norm);
 int launch_rmsnorm_bwd(deers_ctx* ctx, long long rows, int C, const float* x, const float* inv_norm, const float* dy,

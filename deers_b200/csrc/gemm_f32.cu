@@ -3,25 +3,32 @@
 // (src/ops.rs:1089-1101).  The reference sends these to cublasGemmStridedBatchedEx with
 // CUBLAS_COMPUTE_32F (src/storage/cuda.rs:1098-1128), i.e. full f32 arithmetic; so does this kernel.
 //
-// One kernel template covers C[M,N] = A * B for either storage order of A and of B, arbitrary leading
-// dimensions and alignments (16-byte loads when base and leading dimension allow, guarded scalar loads
-// otherwise, zero fill beyond the edges), with an epilogue applied while the tile is still in registers:
+// C[M,N] = A * B for either storage order of A and of B, arbitrary leading dimensions and alignments, with an epilogue
+// applied to the finished tile:
 //   NONE      C = acc
 //   ADD       C = R + acc                 the residual connections of the block (gpt.rs:237-239)
 //   RELU_SQ   r = max(acc, 0); C = r*r; AUX = r     relu and y*y of the MLP (gpt.rs:194-196)
 //   MUL_AUX2  t = acc * AUX; C = t + t    the backward of y*y and relu in one (ops.rs:210-214, 560-568)
-// 256 * KS threads own a BM x BN tile (register patches of TM x TN, operands double-buffered in shared
-// memory, 16 * KS deep; with KS = 2 the two halves of the block each multiply 16 of a stage's 32 k and the
-// patches are added through shared memory at the end: twice the warps per tile for the small shapes whose
-// grids do not fill the SMs and that otherwise wait on shared-memory latency with two warps per scheduler).  Shapes with few output tiles and a long reduction (weight gradients, the head's
-// input gradient) are split along K across gridDim.z: every part writes its partial tile to the
-// workspace, the part that arrives last (one atomic counter per tile, no waiting) adds the parts in
-// index order and runs the epilogue, so results do not depend on arrival order.
+//
+// What bounds it: the model's products are small (1024 x 576 x 192 and the like): 150 tiles of 64 x 64, one per SM, so
+// a product takes as long as ONE block takes for its walk over K.  The block is built around that walk:
+//   * 128 threads own the tile (patches of PM x PN) and KS such groups split every stage's k, so that each scheduler
+//     has four warps to hide shared-memory and FFMA latency with, at 3 LDS.128 per 32 FFMA;
+//   * operands travel by cp.async straight into shared memory in their storage order (no transposition, no
+//     registers), up to STAGES * 32 k ahead: for K = 192 the whole operand is in flight at once;
+//   * k groups, and the blocks of a cluster that split a long K among them (weight gradients), meet in shared
+//     memory: group 0..KS-1 of block 0..P-1 are added in that order by the threads that write the tile (distributed
+//     shared memory, one cluster barrier), so nothing goes through global memory, no counter, no workspace, and the
+//     result does not depend on timing.
 #include "common.cuh"
 
-namespace {
+#include <cooperative_groups.h>
 
-constexpr int GK = 16;                                  // depth of one shared-memory stage
+namespace {
+namespace cg = cooperative_groups;
+
+constexpr int BK = 64;                                  // depth of one stage
+constexpr int MAX_PARTS = 8;                            // blocks of a cluster along K (portable cluster size)
 
 struct GemmArgs {
     const float* a; const float* b; float* c;
@@ -29,12 +36,9 @@ struct GemmArgs {
     float* aux;              // RELU_SQ: written; MUL_AUX2: read; [M][ldc]
     long long lda, ldb, ldc, ldr;
     int M, N, K;
-    int a_mn, b_mn;          // 0: K contiguous, 1: M / N contiguous
     int a_vec, b_vec, c_vec; // 16-byte accesses allowed
     int epi;
-    int k_chunk;             // K elements per gridDim.z part (multiple of GK)
-    float* partial;          // split-K: [tile][part][BM*BN]
-    unsigned int* counters;  // split-K: one per tile, zero on entry, left zero
+    int k_chunk;             // K elements per part (multiple of BK)
 };
 
 __device__ __forceinline__ float4 ld4(const float* p, int valid, bool vec) {
@@ -47,303 +51,368 @@ __device__ __forceinline__ float4 ld4(const float* p, int valid, bool vec) {
     return v;
 }
 
-// Loads one BROWS x GKS operand tile into registers.  contiguous-K storage: rows = tile rows (m or n),
-// GKS / 4 threads cover the k of a row; contiguous-MN storage: rows = k, float4 along m / n.
-template <int BR, int KS>
-struct TileLoader {
-    static constexpr int GKS = GK * KS;
-    static constexpr int NT = 256 * KS;
-    static constexpr int NV = BR * GKS / 4 / NT;         // float4 per thread
-    float4 v[NV];
-    __device__ __forceinline__ void load(const float* base, long long ld, int mn_major, bool vec, int r0, int rmax,
-                                         int k0, int kmax) {
+// Asynchronous copies of 16 / 4 bytes; bytes beyond `n` are written as zeros without being read.
+__device__ __forceinline__ void cp16(float* dst, const float* src, int n) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp4(float* dst, const float* src, int n) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// One operand's stage in shared memory, in its storage order: R rows (m or n) of BK k when k is contiguous, BK rows of
+// R when m / n is.  Row strides are 4 mod 32 words (16-byte pieces of 8 consecutive rows fall into different banks).
+template <int R, bool MN, int GT>
+struct Operand {
+    static constexpr int LD = MN ? R + 4 : BK + 4;
+    static constexpr int FLOATS = MN ? BK * LD : R * LD;
+    static constexpr int LEN = MN ? R : BK, ROWS = MN ? BK : R;     // contiguous floats per row, rows
+    static constexpr int NP = ROWS * LEN / 4 / GT;                  // 16-byte pieces per thread and stage
+    static_assert(NP * GT * 4 == ROWS * LEN, "whole pieces per thread");
+    const float* base;
+    const float* src[NP];    // this thread's pieces of the next stage
+    int dst[NP];             // their places in the stage (floats)
+    int along_r[NP];         // floats of a piece inside the matrix along m / n (K order: 4 or 0)
+    int along_k[NP];         // k of a piece inside the stage
+    long long step;          // from one stage to the next
+    __device__ __forceinline__ void init(const float* b, long long ld, int r0, int rmax, int k0) {
+        base = b;
+        step = MN ? BK * ld : BK;
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int idx = threadIdx.x + i * NT;
-            if (!mn_major) {
-                const int row = idx / (GKS / 4), kq = (idx % (GKS / 4)) * 4;
-                const int gr = r0 + row, gk = k0 + kq;
-                const int valid = gr < rmax ? kmax - gk : 0;
-                v[i] = ld4(base + (long long)gr * ld + gk, valid, vec);
-            } else {
-                const int k = idx / (BR / 4), rq = (idx % (BR / 4)) * 4;
-                const int gk = k0 + k, gr = r0 + rq;
-                const int valid = gk < kmax ? rmax - gr : 0;
-                v[i] = ld4(base + (long long)gk * ld + gr, valid, vec);
-            }
+        for (int i = 0; i < NP; ++i) {
+            const int idx = threadIdx.x + i * GT;
+            const int row = idx / (LEN / 4), col = (idx % (LEN / 4)) * 4;
+            const int r = r0 + (MN ? col : row), k = MN ? row : col;
+            along_k[i] = k;
+            along_r[i] = MN ? min(4, max(0, rmax - r)) : (r < rmax ? 4 : 0);
+            dst[i] = row * LD + col;
+            src[i] = b + (MN ? (long long)(k0 + k) * ld + r : (long long)r * ld + k0 + k);
         }
     }
-    __device__ __forceinline__ void store(float (*s)[BR + 4], int mn_major) const {
+    // Enqueues the next stage's pieces; kv is the number of its k that exist.
+    __device__ __forceinline__ void fetch(float* s, int kv, bool vec) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int idx = threadIdx.x + i * NT;
-            if (!mn_major) {
-                const int row = idx / (GKS / 4), kq = (idx % (GKS / 4)) * 4;
-                s[kq + 0][row] = v[i].x; s[kq + 1][row] = v[i].y; s[kq + 2][row] = v[i].z; s[kq + 3][row] = v[i].w;
+        for (int i = 0; i < NP; ++i) {
+            int valid = along_r[i];
+            if (kv < BK) valid = MN ? (along_k[i] < kv ? valid : 0) : min(valid, max(0, kv - along_k[i]));
+            const float* p = valid > 0 ? src[i] : base;
+            if (vec) {
+                cp16(s + dst[i], p, 4 * valid);
             } else {
-                const int k = idx / (BR / 4), rq = (idx % (BR / 4)) * 4;
-                *reinterpret_cast<float4*>(&s[k][rq]) = v[i];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) cp4(s + dst[i] + e, valid > e ? p + e : base, valid > e ? 4 : 0);
             }
+            src[i] += step;
+        }
+    }
+    // Index inside the tile of element i of thread group coordinate t: contiguous groups of four for MN order (one
+    // LDS.128 per four), interleaved for K order (one LDS.128 per row and four k).
+    template <int P>
+    static __device__ __forceinline__ int index(int t, int i) {
+        constexpr int G = R / P;                                   // thread groups along this side
+        if (!MN) return t + G * i;
+        if (P >= 4) return (i / 4) * (4 * G) + t * 4 + (i % 4);
+        return t * P + i;
+    }
+    // The P elements of this thread: K order reads four k at a time (v[i][kk]), MN order one k at a time (v[i][0]).
+    static constexpr int KV = MN ? 1 : 4;
+    template <int P>
+    static __device__ __forceinline__ void read(const float* s, int t, int k, float (&v)[P][KV]) {
+        if constexpr (!MN) {
+#pragma unroll
+            for (int i = 0; i < P; ++i) {
+                const float4 x = *reinterpret_cast<const float4*>(s + index<P>(t, i) * LD + k);
+                v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+            }
+        } else if constexpr (P >= 4) {
+#pragma unroll
+            for (int i = 0; i < P; i += 4) {
+                const float4 x = *reinterpret_cast<const float4*>(s + k * LD + index<P>(t, i));
+                v[i][0] = x.x; v[i + 1][0] = x.y; v[i + 2][0] = x.z; v[i + 3][0] = x.w;
+            }
+        } else {
+            const float2 x = *reinterpret_cast<const float2*>(s + k * LD + index<P>(t, 0));
+            v[0][0] = x.x; v[1][0] = x.y;
         }
     }
 };
 
-template <int BM, int BN, int TM, int TN, int KS>
-__global__ void __launch_bounds__(256 * KS) gemm_f32_kernel(const GemmArgs g) {
-    static_assert((BM / TM) * (BN / TN) == 256, "256 threads per tile and k half");
-    constexpr int GKS = GK * KS;
-    __shared__ __align__(16) float As[2][GKS][BM + 4];
-    __shared__ __align__(16) float Bs[2][GKS][BN + 4];
-    __shared__ int s_last;
-    const int tid = threadIdx.x % 256, kh = threadIdx.x / 256;      // position in the tile, k half
-    const int tx = tid % (BN / TN), ty = tid / (BN / TN);
+template <int PM, int PN, int KS, bool A_MN, bool B_MN>
+struct GemmShape {
+    static constexpr int BM = 8 * PM, BN = 16 * PN, GT = 128 * KS;
+    using OA = Operand<BM, A_MN, GT>;
+    using OB = Operand<BN, B_MN, GT>;
+    static constexpr int STAGE = OA::FLOATS + OB::FLOATS;
+    static constexpr int RLD = BN + 4;                              // row stride of the patch staging tile
+    static constexpr int RED = KS * BM * RLD;
+    static constexpr int STAGES = BM * BN > 64 * 64 ? 3 : 4;
+    static constexpr size_t SMEM = (size_t)(STAGES * STAGE > RED ? STAGES * STAGE : RED) * sizeof(float);
+};
+
+template <int PM, int PN, int KS, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(128 * KS) gemm_f32_kernel(const GemmArgs g) {
+    using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
+    constexpr int BM = S::BM, BN = S::BN, GT = S::GT, STAGES = S::STAGES, KG = BK / KS;
+    extern __shared__ __align__(16) float smem[];
+    const int tid = threadIdx.x % 128, kg = threadIdx.x / 128;      // position in the tile, k group
+    const int w = tid / 32, lane = tid % 32;
+    const int ty = (w & 1) * 4 + lane / 8, tx = (w >> 1) * 8 + lane % 8;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int kbeg = blockIdx.z * g.k_chunk;
     const int kend = min(g.K, kbeg + g.k_chunk);
+    const int nk = kend > kbeg ? (kend - kbeg + BK - 1) / BK : 0;
 
-    float acc[TM][TN];
+    typename S::OA la;
+    typename S::OB lb;
+    la.init(g.a, g.lda, m0, g.M, kbeg);
+    lb.init(g.b, g.ldb, n0, g.N, kbeg);
+    int kv = kend - kbeg;                                           // k left to fetch
+    float* st_in = smem;                                            // stage to fill next
+    auto fetch = [&]() {
+        if (kv > 0) {
+            la.fetch(st_in, kv, g.a_vec);
+            lb.fetch(st_in + S::OA::FLOATS, kv, g.b_vec);
+            kv -= BK;
+            st_in = st_in + S::STAGE == smem + STAGES * S::STAGE ? smem : st_in + S::STAGE;
+        }
+        cp_commit();
+    };
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int t = 0; t < STAGES - 1; ++t) fetch();
 
-    TileLoader<BM, KS> la;
-    TileLoader<BN, KS> lb;
-    const int nk = (kend - kbeg + GKS - 1) / GKS;
-    if (nk > 0) {
-        la.load(g.a, g.lda, g.a_mn, g.a_vec, m0, g.M, kbeg, kend);
-        lb.load(g.b, g.ldb, g.b_mn, g.b_vec, n0, g.N, kbeg, kend);
-        la.store(As[0], g.a_mn);
-        lb.store(Bs[0], g.b_mn);
+    float acc[PM][PN];
+#pragma unroll
+    for (int i = 0; i < PM; ++i)
+#pragma unroll
+        for (int j = 0; j < PN; ++j) acc[i][j] = 0.f;
+
+    const float* sa = smem;
+    for (int t = 0; t < nk; ++t) {
+        cp_wait<STAGES - 2>();
+        __syncthreads();                                            // stage t has landed, stage t-1 is free
+        fetch();
+        const float* sb = sa + S::OA::FLOATS;
+#pragma unroll
+        for (int k = 0; k < KG; k += 4) {
+            float a[PM][S::OA::KV], b[PN][S::OB::KV];
+            if constexpr (!A_MN) S::OA::template read<PM>(sa, ty, kg * KG + k, a);
+            if constexpr (!B_MN) S::OB::template read<PN>(sb, tx, kg * KG + k, b);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                if constexpr (A_MN) S::OA::template read<PM>(sa, ty, kg * KG + k + kk, a);
+                if constexpr (B_MN) S::OB::template read<PN>(sb, tx, kg * KG + k + kk, b);
+#pragma unroll
+                for (int i = 0; i < PM; ++i)
+#pragma unroll
+                    for (int j = 0; j < PN; ++j) acc[i][j] = fmaf(a[i][A_MN ? 0 : kk], b[j][B_MN ? 0 : kk], acc[i][j]);
+            }
+        }
+        sa = sa + S::STAGE == smem + STAGES * S::STAGE ? smem : sa + S::STAGE;
+    }
+    cp_wait<0>();
+    __syncthreads();                                                // operand stages are free: patches meet here
+
+    float* red = smem;
+#pragma unroll
+    for (int i = 0; i < PM; ++i) {
+        float* row = red + (kg * BM + S::OA::template index<PM>(ty, i)) * S::RLD;
+        if constexpr (B_MN && PN >= 4) {
+#pragma unroll
+            for (int j = 0; j < PN; j += 4)
+                *reinterpret_cast<float4*>(row + S::OB::template index<PN>(tx, j)) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < PN; ++j) row[S::OB::template index<PN>(tx, j)] = acc[i][j];
+        }
     }
     __syncthreads();
-    for (int kt = 0; kt < nk; ++kt) {
-        const int cur = kt & 1;
-        if (kt + 1 < nk) {
-            la.load(g.a, g.lda, g.a_mn, g.a_vec, m0, g.M, kbeg + (kt + 1) * GKS, kend);
-            lb.load(g.b, g.ldb, g.b_mn, g.b_vec, n0, g.N, kbeg + (kt + 1) * GKS, kend);
-        }
-#pragma unroll
-        for (int k = kh * GK; k < (kh + 1) * GK; ++k) {
-            float af[TM], bf[TN];
-            // a thread's rows / columns come in groups of four, the groups BM/2 (BN/2) apart, so that the
-            // lanes of a warp read consecutive 16-byte pieces
-#pragma unroll
-            for (int h = 0; h < TM / 4; ++h) {
-                const float4 t = *reinterpret_cast<const float4*>(&As[cur][k][h * (BM / (TM / 4)) + ty * 4]);
-                af[h * 4 + 0] = t.x; af[h * 4 + 1] = t.y; af[h * 4 + 2] = t.z; af[h * 4 + 3] = t.w;
-            }
-#pragma unroll
-            for (int h = 0; h < TN / 4; ++h) {
-                const float4 t = *reinterpret_cast<const float4*>(&Bs[cur][k][h * (BN / (TN / 4)) + tx * 4]);
-                bf[h * 4 + 0] = t.x; bf[h * 4 + 1] = t.y; bf[h * 4 + 2] = t.z; bf[h * 4 + 3] = t.w;
-            }
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(af[i], bf[j], acc[i][j]);
-        }
-        if (kt + 1 < nk) {
-            la.store(As[cur ^ 1], g.a_mn);
-            lb.store(Bs[cur ^ 1], g.b_mn);
-        }
-        __syncthreads();
-    }
 
-    // ---- the k halves of the block meet: the upper half hands its patch over through shared memory (the
-    // operand buffers are free after the loop's last barrier) and only stays for the barriers below
-    const bool owner = kh == 0;
-    if (KS > 1) {
-        static_assert(KS == 1 || sizeof(As) >= 256 * TM * TN * sizeof(float), "patch exchange fits in the A buffers");
-        float4* red = reinterpret_cast<float4*>(&As[0][0][0]);
-        if (!owner) {
+    // Rows of the tile this block finishes: all of them, or its share of the cluster's.
+    const int parts = gridDim.z, rank = blockIdx.z;
+    int r_begin = 0, r_end = BM;
+    if (parts > 1) {
+        for (int idx = threadIdx.x; idx < BM * BN / 4; idx += GT) {
+            float* q = red + (idx / (BN / 4)) * S::RLD + (idx % (BN / 4)) * 4;
+            float4 v = *reinterpret_cast<float4*>(q);
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN / 4; ++j)
-                    red[(i * (TN / 4) + j) * 256 + tid] =
-                        make_float4(acc[i][j * 4], acc[i][j * 4 + 1], acc[i][j * 4 + 2], acc[i][j * 4 + 3]);
-        }
-        __syncthreads();
-        if (owner) {
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN / 4; ++j) {
-                    const float4 t = red[(i * (TN / 4) + j) * 256 + tid];
-                    acc[i][j * 4] += t.x; acc[i][j * 4 + 1] += t.y; acc[i][j * 4 + 2] += t.z; acc[i][j * 4 + 3] += t.w;
-                }
-        }
-    }
-
-    // ---- split-K: park the partial tile; the last part to arrive adds all parts in index order
-    if (gridDim.z > 1) {
-        const int tile = blockIdx.y * gridDim.x + blockIdx.x;
-        float4* mine = reinterpret_cast<float4*>(g.partial) +
-                       ((size_t)tile * gridDim.z + blockIdx.z) * (BM * BN / 4);
-        if (owner) {
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN / 4; ++j)
-                    mine[(i * (TN / 4) + j) * 256 + tid] =
-                        make_float4(acc[i][j * 4], acc[i][j * 4 + 1], acc[i][j * 4 + 2], acc[i][j * 4 + 3]);
-        }
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const unsigned int prev = atomicAdd(&g.counters[tile], 1u);
-            s_last = prev == gridDim.z - 1;
-            if (s_last) g.counters[tile] = 0;                     // ready for the next launch
-        }
-        __syncthreads();
-        if (!s_last || !owner) return;
-        __threadfence();
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-        const float4* parts = reinterpret_cast<const float4*>(g.partial) + (size_t)tile * gridDim.z * (BM * BN / 4);
-        for (unsigned int z = 0; z < gridDim.z; ++z) {
-            const float4* p = parts + (size_t)z * (BM * BN / 4);
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN / 4; ++j) {
-                    const float4 t = __ldcg(&p[(i * (TN / 4) + j) * 256 + tid]);
-                    acc[i][j * 4] += t.x; acc[i][j * 4 + 1] += t.y; acc[i][j * 4 + 2] += t.z; acc[i][j * 4 + 3] += t.w;
-                }
-        }
-    }
-
-    // ---- epilogue
-    if (!owner) return;
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int m = m0 + (i / 4) * (BM / (TM / 4)) + ty * 4 + (i % 4);
-        if (m >= g.M) continue;
-#pragma unroll
-        for (int h = 0; h < TN / 4; ++h) {
-            const int n = n0 + h * (BN / (TN / 4)) + tx * 4;
-            if (n >= g.N) continue;
-            float o[4] = {acc[i][h * 4], acc[i][h * 4 + 1], acc[i][h * 4 + 2], acc[i][h * 4 + 3]};
-            float x[4] = {0.f, 0.f, 0.f, 0.f};
-            const int valid = g.N - n;
-            float* cp = g.c + (long long)m * g.ldc + n;
-            if (g.epi == DEERS_EPI_ADD) {
-                const float4 t = ld4(g.r + (long long)m * g.ldr + n, valid, g.c_vec);
-                o[0] = t.x + o[0]; o[1] = t.y + o[1]; o[2] = t.z + o[2]; o[3] = t.w + o[3];
-            } else if (g.epi == DEERS_EPI_RELU_SQ) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) { x[e] = fmaxf(o[e], 0.f); o[e] = x[e] * x[e]; }
-            } else if (g.epi == DEERS_EPI_MUL_AUX2) {
-                const float4 t = ld4(g.aux + (long long)m * g.ldc + n, valid, g.c_vec);
-                o[0] *= t.x; o[1] *= t.y; o[2] *= t.z; o[3] *= t.w;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) o[e] = o[e] + o[e];
+            for (int z = 1; z < KS; ++z) {
+                const float4 u = *reinterpret_cast<const float4*>(q + z * BM * S::RLD);
+                v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
             }
-            if (g.c_vec && valid >= 4) {
-                *reinterpret_cast<float4*>(cp) = make_float4(o[0], o[1], o[2], o[3]);
-                if (g.epi == DEERS_EPI_RELU_SQ)
-                    *reinterpret_cast<float4*>(g.aux + (long long)m * g.ldc + n) = make_float4(x[0], x[1], x[2], x[3]);
-            } else {
-                for (int e = 0; e < 4 && e < valid; ++e) {
-                    cp[e] = o[e];
-                    if (g.epi == DEERS_EPI_RELU_SQ) g.aux[(long long)m * g.ldc + n + e] = x[e];
-                }
+            *reinterpret_cast<float4*>(q) = v;
+        }
+        cg::this_cluster().sync();
+        const int share = (BM + parts - 1) / parts;
+        r_begin = rank * share;
+        r_end = min(BM, r_begin + share);
+    }
+    for (int idx = r_begin * (BN / 4) + threadIdx.x; idx < r_end * (BN / 4); idx += GT) {
+        const int row = idx / (BN / 4), col = (idx % (BN / 4)) * 4;
+        const int m = m0 + row, n = n0 + col;
+        const float* q = red + row * S::RLD + col;
+        float4 v;
+        if (parts > 1) {
+            v = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int z = 0; z < parts; ++z) {
+                const float4 u = *reinterpret_cast<const float4*>(cg::this_cluster().map_shared_rank(q, z));
+                v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+            }
+        } else {
+            v = *reinterpret_cast<const float4*>(q);
+#pragma unroll
+            for (int z = 1; z < KS; ++z) {
+                const float4 u = *reinterpret_cast<const float4*>(q + z * BM * S::RLD);
+                v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+            }
+        }
+        if (m >= g.M || n >= g.N) continue;
+        const int valid = g.N - n;
+        float o[4] = {v.x, v.y, v.z, v.w}, x[4] = {0.f, 0.f, 0.f, 0.f};
+        float* cp = g.c + (long long)m * g.ldc + n;
+        if (g.epi == DEERS_EPI_ADD) {
+            const float4 t = ld4(g.r + (long long)m * g.ldr + n, valid, g.c_vec);
+            o[0] = t.x + o[0]; o[1] = t.y + o[1]; o[2] = t.z + o[2]; o[3] = t.w + o[3];
+        } else if (g.epi == DEERS_EPI_RELU_SQ) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { x[e] = fmaxf(o[e], 0.f); o[e] = x[e] * x[e]; }
+        } else if (g.epi == DEERS_EPI_MUL_AUX2) {
+            const float4 t = ld4(g.aux + (long long)m * g.ldc + n, valid, g.c_vec);
+            o[0] *= t.x; o[1] *= t.y; o[2] *= t.z; o[3] *= t.w;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = o[e] + o[e];
+        }
+        if (g.c_vec && valid >= 4) {
+            *reinterpret_cast<float4*>(cp) = make_float4(o[0], o[1], o[2], o[3]);
+            if (g.epi == DEERS_EPI_RELU_SQ)
+                *reinterpret_cast<float4*>(g.aux + (long long)m * g.ldc + n) = make_float4(x[0], x[1], x[2], x[3]);
+        } else {
+            for (int e = 0; e < 4 && e < valid; ++e) {
+                cp[e] = o[e];
+                if (g.epi == DEERS_EPI_RELU_SQ) g.aux[(long long)m * g.ldc + n + e] = x[e];
             }
         }
     }
+    if (parts > 1) cg::this_cluster().sync();                       // nobody leaves while a peer still reads its patch
 }
 
 struct GemmPlan {
-    int cfg;        // 0: 128x128, 1: 64x128, 2: 64x64
-    int bm, bn;
+    int cfg;        // index into kVariants
     int tiles_m, tiles_n, parts, k_chunk;
 };
 
-GemmPlan plan_gemm(int M, int N, int K, int sm_count) {
-    static const int kBM[3] = {128, 64, 64}, kBN[3] = {128, 128, 64}, kKS[3] = {1, 1, 2};
-    GemmPlan p{};
-    int pick = 2;
-    for (int c = 0; c < 3; ++c) {
-        const long long tiles = (long long)((M + kBM[c] - 1) / kBM[c]) * ((N + kBN[c] - 1) / kBN[c]);
-        // the padding a tile shape adds to M (an [M=192] gradient wastes a quarter of a 128-row tile)
-        const double waste = (double)((M + kBM[c] - 1) / kBM[c] * kBM[c]) * ((N + kBN[c] - 1) / kBN[c] * kBN[c]) /
-                             ((double)M * N);
-        if (tiles >= 2LL * sm_count && waste <= 1.15) { pick = c; break; }
+// Tile variants with what was measured of them (cycles at 1.965 GHz, from products of several K in a graph): a
+// block's walk over 64 k, and what a launch costs around it.
+struct Variant { int bm, bn; double walk, around; };
+constexpr Variant kVariants[4] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {32, 64, 2360, 4000}, {32, 32, 1680, 3200}};
+
+// How many clusters of 1..MAX_PARTS blocks (one block per SM) the device holds at a time: a cluster lives inside one
+// GPC, so e.g. 48 clusters of three do not fit 148 SMs although their 144 blocks would.
+int cluster_capacity(deers_ctx* ctx) {
+    if (ctx->cluster_capacity[1] > 0) return DEERS_OK;
+    using S = GemmShape<8, 4, 4, false, true>;
+    const auto kernel = gemm_f32_kernel<8, 4, 4, false, true>;
+    DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<8, 4, 4, false, true>), S::SMEM);
+    for (int parts = 2; parts <= MAX_PARTS; ++parts) {
+        cudaLaunchConfig_t lc{};
+        lc.gridDim = dim3(1, 1, parts);
+        lc.blockDim = dim3(S::GT);
+        lc.dynamicSmemBytes = S::SMEM;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = (unsigned)parts;
+        lc.attrs = at; lc.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &lc) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        ctx->cluster_capacity[parts] = n;
     }
-    p.cfg = pick; p.bm = kBM[pick]; p.bn = kBN[pick];
-    p.tiles_m = (M + p.bm - 1) / p.bm;
-    p.tiles_n = (N + p.bn - 1) / p.bn;
-    const long long tiles = (long long)p.tiles_m * p.tiles_n;
-    int parts = 1;
-    if (tiles < 2LL * sm_count) {
-        parts = (int)((3LL * sm_count + tiles - 1) / tiles);
-        const int max_parts = K / (8 * GK) > 1 ? K / (8 * GK) : 1;      // at least 8 stages per part
-        if (parts > max_parts) parts = max_parts;
-        if (parts > 64) parts = 64;
-    }
-    const int gks = GK * kKS[pick];
-    int chunk = ((K + parts - 1) / parts + gks - 1) / gks * gks;
-    if (chunk < gks) chunk = gks;
-    p.k_chunk = chunk;
-    p.parts = (K + chunk - 1) / chunk;
-    if (p.parts < 1) p.parts = 1;
-    return p;
+    ctx->cluster_capacity[1] = ctx->sm_count;
+    return DEERS_OK;
 }
 
-size_t plan_workspace(const GemmPlan& p) {
-    if (p.parts <= 1) return 0;
-    const size_t tiles = (size_t)p.tiles_m * p.tiles_n;
-    return 256 + ((tiles * sizeof(unsigned int) + 255) / 256) * 256 + tiles * p.parts * p.bm * p.bn * sizeof(float);
+// Picks the variant and the K split with the least estimated time: the blocks an SM has to run one after another times
+// a block's walk over its K, plus what a block spends before and after it (and at the cluster's meeting).
+GemmPlan plan_gemm(int M, int N, int K, const int* capacity) {
+    GemmPlan best{};
+    double best_cost = -1.0;
+    const int steps = (K + BK - 1) / BK;
+    for (int c = 0; c < 4; ++c) {
+        const Variant& v = kVariants[c];
+        const long long tm = (M + v.bm - 1) / v.bm, tn = (N + v.bn - 1) / v.bn;
+        for (int parts = 1; parts <= MAX_PARTS; ++parts) {
+            const int chunk = (steps + parts - 1) / parts;
+            if (parts > 1 && (chunk < 2 || (long long)chunk * (parts - 1) >= steps)) continue;      // no empty part
+            if (capacity[parts] < 1) continue;
+            const double waves = (double)((tm * tn + capacity[parts] - 1) / capacity[parts]);
+            const double cost = waves * chunk * v.walk + v.around + 1200.0 * (waves - 1.0) + (parts > 1 ? 3300.0 : 0.0);
+            if (best_cost < 0.0 || cost < best_cost) {
+                best_cost = cost;
+                best.cfg = c; best.tiles_m = (int)tm; best.tiles_n = (int)tn; best.parts = parts; best.k_chunk = chunk * BK;
+            }
+        }
+    }
+    if (K == 0) { best.parts = 1; best.k_chunk = BK; }
+    return best;
+}
+
+template <int PM, int PN, int KS, bool A_MN, bool B_MN>
+int launch_variant(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g) {
+    using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
+    const auto kernel = gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>;
+    DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>), S::SMEM);
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(p.tiles_n, p.tiles_m, p.parts);
+    lc.blockDim = dim3(S::GT);
+    lc.dynamicSmemBytes = S::SMEM;
+    lc.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    if (p.parts > 1) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = (unsigned)p.parts;
+        lc.attrs = at; lc.numAttrs = 1;
+    }
+    DEERS_CUDA_TRY(ctx, cudaLaunchKernelEx(&lc, kernel, g));
+    return DEERS_OK;
+}
+
+template <int PM, int PN, int KS>
+int launch_orders(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g, int a_mn, int b_mn) {
+    if (a_mn) return b_mn ? launch_variant<PM, PN, KS, true, true>(ctx, p, g) : launch_variant<PM, PN, KS, true, false>(ctx, p, g);
+    return b_mn ? launch_variant<PM, PN, KS, false, true>(ctx, p, g) : launch_variant<PM, PN, KS, false, false>(ctx, p, g);
 }
 
 }  // namespace
 
-size_t gemm_f32_workspace_bytes(const deers_ctx* ctx, int M, int N, int K) {
-    return plan_workspace(plan_gemm(M, N, K, ctx ? ctx->sm_count : 148));
-}
-
-// counters_zero: the caller guarantees that the counter words at the start of the workspace are zero (they
-// are left zero by every launch); otherwise they are cleared on the stream first.
 int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long long lda, int a_mn, const float* b,
-                    long long ldb, int b_mn, float* c, long long ldc, int epi, const float* r, long long ldr, float* aux,
-                    void* workspace, size_t ws_bytes, bool counters_zero) {
+                    long long ldb, int b_mn, float* c, long long ldc, int epi, const float* r, long long ldr, float* aux) {
     if (M == 0 || N == 0) return DEERS_OK;
-    const GemmPlan p = plan_gemm(M, N, K, ctx->sm_count);
+    int rc = cluster_capacity(ctx);
+    if (rc) return rc;
+    GemmPlan p = plan_gemm(M, N, K, ctx->cluster_capacity);
     GemmArgs g{};
     g.a = a; g.b = b; g.c = c; g.r = r; g.aux = aux;
     g.lda = lda; g.ldb = ldb; g.ldc = ldc; g.ldr = ldr;
-    g.M = M; g.N = N; g.K = K; g.a_mn = a_mn; g.b_mn = b_mn; g.epi = epi;
+    g.M = M; g.N = N; g.K = K; g.epi = epi;
     g.a_vec = ((uintptr_t)a & 15u) == 0 && lda % 4 == 0;
     g.b_vec = ((uintptr_t)b & 15u) == 0 && ldb % 4 == 0;
     g.c_vec = ((uintptr_t)c & 15u) == 0 && ldc % 4 == 0 && (!r || (((uintptr_t)r & 15u) == 0 && ldr % 4 == 0)) &&
               (!aux || ((uintptr_t)aux & 15u) == 0);
     g.k_chunk = p.k_chunk;
-    if (p.parts > 1) {
-        if (!workspace || ws_bytes < plan_workspace(p) || ((uintptr_t)workspace & 255u) != 0) return DEERS_ERR_WORKSPACE;
-        const size_t tiles = (size_t)p.tiles_m * p.tiles_n;
-        const size_t cbytes = ((tiles * sizeof(unsigned int) + 255) / 256) * 256;
-        g.counters = (unsigned int*)workspace;
-        g.partial = (float*)((char*)workspace + cbytes);
-        if (!counters_zero) DEERS_CUDA_TRY(ctx, cudaMemsetAsync(workspace, 0, cbytes, ctx->stream));
-    }
-    const dim3 grid(p.tiles_n, p.tiles_m, p.parts);
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM);
-        if (p.cfg == 0) gemm_f32_kernel<128, 128, 8, 8, 1><<<grid, 256, 0, ctx->stream>>>(g);
-        else if (p.cfg == 1) gemm_f32_kernel<64, 128, 4, 8, 1><<<grid, 256, 0, ctx->stream>>>(g);
-        else gemm_f32_kernel<64, 64, 4, 4, 2><<<grid, 512, 0, ctx->stream>>>(g);
+        if (p.cfg == 0) rc = launch_orders<8, 8, 2>(ctx, p, g, a_mn, b_mn);
+        else if (p.cfg == 1) rc = launch_orders<8, 4, 4>(ctx, p, g, a_mn, b_mn);
+        else if (p.cfg == 2) rc = launch_orders<4, 4, 4>(ctx, p, g, a_mn, b_mn);
+        else rc = launch_orders<4, 2, 4>(ctx, p, g, a_mn, b_mn);
     }
     ctx->launches += 1;
-    DEERS_CUDA_TRY(ctx, cudaGetLastError());
-    return DEERS_OK;
+    return rc;
 }
 
 extern "C" size_t deers_b200_gemm_f32_workspace_bytes(deers_ctx* ctx, int32_t M, int32_t N, int32_t K) {
     if (!ctx || M < 0 || N < 0 || K < 0) return 0;
-    return gemm_f32_workspace_bytes(ctx, M, N, K);
+    return 0;                                                       // K splits meet in shared memory
 }
 
 extern "C" int deers_b200_gemm_f32(deers_ctx* ctx, int32_t M, int32_t N, int32_t K, const float* a, int64_t lda,
@@ -371,7 +440,7 @@ extern "C" int deers_b200_gemm_f32(deers_ctx* ctx, int32_t M, int32_t N, int32_t
             aux = epilogue->aux;
         }
     }
+    (void)workspace; (void)workspace_bytes;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    return launch_gemm_f32(ctx, M, N, K, a, lda, a_mn_major, b, ldb, b_mn_major, c, ldc, epi, r, ldr, aux, workspace,
-                           workspace_bytes, false);
+    return launch_gemm_f32(ctx, M, N, K, a, lda, a_mn_major, b, ldb, b_mn_major, c, ldc, epi, r, ldr, aux);
 }

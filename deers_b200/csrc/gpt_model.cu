@@ -53,9 +53,6 @@ struct deers_gpt {
     std::vector<LayerAct> la;
     float *dx_a, *dx_b, *dtmp, *dh, *dqkv, *dqk, *attn_ws;
     size_t attn_ws_bytes;
-    void* gemm_ws;
-    void* gemm_ws_side;          // split-K workspace of the weight-gradient stream
-    size_t gemm_ws_bytes;
     // second stream for the weight gradients; events are markers only (no timing)
     cudaStream_t side;
     cudaEvent_t ev_fork, ev_join, ev_done[4];
@@ -91,8 +88,7 @@ namespace {
 int gemm(deers_gpt* m, int M, int N, int K, const float* a, long long lda, int a_mn, const float* b, long long ldb, int b_mn,
          float* c, long long ldc, int epi = DEERS_EPI_NONE, const float* r = nullptr, long long ldr = 0,
          float* aux = nullptr) {
-    return launch_gemm_f32(m->ctx, M, N, K, a, lda, a_mn, b, ldb, b_mn, c, ldc, epi, r, ldr, aux,
-                           m->on_side ? m->gemm_ws_side : m->gemm_ws, m->gemm_ws_bytes, true);
+    return launch_gemm_f32(m->ctx, M, N, K, a, lda, a_mn, b, ldb, b_mn, c, ldc, epi, r, ldr, aux);
 }
 
 // Launches made while a SideScope lives go to the weight-gradient stream, ordered after everything the main
@@ -475,26 +471,6 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
     m->norm_dev = nullptr;
     size_t total = 0;
     for (auto& s : slots) total += align64(s.n);
-    // split-K workspace: the largest any GEMM of the step asks for (tokens vary: take the maximum over B*T <= N by
-    // probing the shapes at full size, which is where the partial tiles are largest)
-    size_t gws = 0;
-    {
-        const int n = (int)N, c = (int)C, h = (int)Hm, v = (int)V;
-        const int shapes[][3] = {{n, 3 * c, c}, {n, c, c}, {n, h, c}, {n, c, h}, {n, v, c}, {c, v, n}, {n, c, v},
-                                 {h, c, n}, {c, h, n}, {c, c, n}, {c, 3 * c, n}, {n, c, 3 * c}};
-        for (auto& s : shapes) {
-            for (int frac = 1; frac <= 64; frac *= 2) {               // smaller batches change the split, not the bound by much
-                const int tok = n / frac > 0 ? n / frac : 1;
-                const int M2 = s[0] == n ? tok : s[0], N2 = s[1] == n ? tok : s[1], K2 = s[2] == n ? tok : s[2];
-                const size_t b = gemm_f32_workspace_bytes(ctx, M2, N2, K2);
-                gws = b > gws ? b : gws;
-            }
-        }
-    }
-    // any token count in between stays below (tiles + 3 * SMs) partial tiles of at most 128 x 128 floats
-    const size_t gws_floor = (size_t)5 * ctx->sm_count * 128 * 128 * sizeof(float) + 65536;
-    if (gws < gws_floor) gws = gws_floor;
-    m->gemm_ws_bytes = gws;
     const size_t opt_bytes = deers_b200_optim_scratch_bytes();
     const size_t id_bytes = ((size_t)N * sizeof(long long) + 255) / 256 * 256;
     auto up256 = [](size_t b) { return (b + 255) / 256 * 256; };
@@ -503,18 +479,16 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
     const size_t x3 = m->tc_head ? up256(((size_t)148 * 16384 + N * C) * sizeof(float) * 2) : 0;
     m->x3_ws_bytes = x3;
     const size_t tc_bytes = m->tc_head ? 2 * (xf_h + w_h + dl_h) + 2 * x3 : 0;
-    const size_t bytes = total * sizeof(float) + 2 * (gws + 256) + opt_bytes + 256 + 2 * id_bytes + tc_bytes;
+    const size_t bytes = total * sizeof(float) + opt_bytes + 256 + 2 * id_bytes + tc_bytes;
     char* base = nullptr;
     if (!rc && cudaMalloc((void**)&base, bytes) != cudaSuccess) rc = DEERS_ERR_CUDA;
-    if (!rc && cudaMemsetAsync(base, 0, bytes, ctx->stream) != cudaSuccess) rc = DEERS_ERR_CUDA;   // split-K counters start at zero
+    if (!rc && cudaMemsetAsync(base, 0, bytes, ctx->stream) != cudaSuccess) rc = DEERS_ERR_CUDA;
     if (!rc) {
         m->act_base = (float*)base;
         float* p = (float*)base;
         for (auto& s : slots) { *s.p = p; p += align64(s.n); }
         m->norm_dev = m->loss_dev + 1;
         char* q = (char*)p;
-        m->gemm_ws = gws ? q : nullptr; q += (gws + 255) / 256 * 256;
-        m->gemm_ws_side = gws ? q : nullptr; q += (gws + 255) / 256 * 256;
         m->optim_scratch = q; q += (opt_bytes + 255) / 256 * 256;
         m->ids_dev = (long long*)q; q += id_bytes;
         m->tgt_dev = (long long*)q; q += id_bytes;

@@ -35,3 +35,30 @@ def test_f16_head_dims_in_place_with_strided_rows(D, T):
         for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), (o, lse, dq, dk, dv), want):
             assert_close(g.float().cpu().numpy(), w, TOL_F16, f"D {D} T {T} {name}")
     assert torch.all(big[..., D:] == 7.0) and torch.all(dvb[..., D:] == 7.0), "columns beyond head_dim are not ours"
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 3, 5), (31, 33, 63), (32, 32, 64), (33, 65, 65), (63, 129, 191), (64, 64, 1025),
+                                   (100, 40, 4099), (192, 190, 1023), (1024, 576, 70), (2050, 1030, 40)])
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 1), (0, 0), (1, 1), (1, 0)])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_f32_gemm_tiles_clusters_and_remainders(M, N, K, a_mn, b_mn, aligned):
+    """Every tile variant, K split over a cluster or not, with tiles, stages and parts that do not come out even."""
+    from deers_b200 import gpt
+    rng = np.random.default_rng(M + 7 * N + 13 * K)
+    a = rng.standard_normal((M, K)).astype(np.float32)
+    b = rng.standard_normal((K, N)).astype(np.float32)
+    want = a.astype(np.float64) @ b.astype(np.float64)
+
+    def place(x):
+        pad = 0 if aligned else 3                          # an odd leading dimension rules out 16-byte copies
+        big = torch.full((x.shape[0], x.shape[1] + pad), float("nan"), device="cuda")
+        big[:, :x.shape[1]] = torch.from_numpy(np.ascontiguousarray(x)).cuda()
+        return big[:, :x.shape[1]]
+    ta, tb = place(a.T if a_mn else a), place(b if b_mn else b.T)
+    big = torch.full((M + 1, N + 3), float("nan"), device="cuda")
+    got = gpt.gemm_f32(ta, tb, bool(a_mn), bool(b_mn), out=big[:M, :N])
+    torch.cuda.synchronize()
+    # K rounded sums of unit-variance products: sqrt(K) growth, 2^-24 each, against sqrt(K) * (largest of the draws)
+    tol = 2e-6 * max(1.0, np.sqrt(K) / 4) * max(1.0, np.abs(want).max())
+    assert np.abs(got.cpu().numpy() - want).max() <= tol
+    assert torch.isnan(big[M]).all() and torch.isnan(big[:M, N:]).all(), "nothing outside C is written"
