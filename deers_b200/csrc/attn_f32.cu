@@ -1,18 +1,25 @@
 // f32 causal attention for sm_100a: FFMA register tiling, no tensor cores and no
 // TF32, so that the result holds 1e-4 against the CPU path of the reference
-// (src/storage/cpu.rs:688-791 of deers).  Forward is one pass with an online
-// softmax (row max / row sum reduced by warp shuffles); backward recomputes P
-// from the saved lse and is split in two atomic-free kernels: a KV-tile-stationary
-// one that owns dK/dV and a Q-tile-stationary one that owns dQ.  All three take
-// [B,H,T,D] strides, so no compaction copy is needed around them.
+// (src/storage/cpu.rs:688-791 of deers).  Forward is one pass with an online softmax; backward recomputes P
+// from the saved lse and has two kinds of blocks in one launch, neither with atomics: key-tile-stationary ones own
+// dK/dV, query-tile-stationary ones own dQ.  All take [B,H,T,D] strides, so no compaction copy is needed around them.
+//
+// What bounds it: at the model's sizes (24 slices of 256 x 32) the arithmetic is 2 us of the chip's FFMA time; the
+// rest is the length of one block's walk.  So a block owns few rows (32) and splits its walk: NG groups of two
+// warps take every NG-th tile of the other side, each with its own softmax state (or gradient sums) and its own
+// tiles in shared memory, and meet once at the end in group order.  A group never waits for another: its two
+// warps meet at a named barrier, and the P / dS tile a product reads was written by the same warp.
+// Within a group thread (ty, tx) of 8 x 8 owns rows 4 ty .. 4 ty + 3 and columns tx, tx + 8, ... of a 32 x BN score tile
+// (4 x 8 or 4 x 4 patches: 12 LDS.128 per 128 FFMA) and rows 4 ty .. with float4 columns 4 tx + 32 j of the
+// accumulators.  Tiles arrive by cp.async: the next K (or Q) is fetched while the current one's scores are turned
+// into the second product, the next V (or dO) while the next scores are computed.
 #include "common.cuh"
 
 namespace {
 
-constexpr int BM = 64;        // query rows per tile
-constexpr int BN = 64;        // key/value rows per tile
-constexpr int NT = 256;       // threads per CTA: 16 x 16, each owns a 4 x 4 patch of a 64 x 64 tile
-constexpr int PLD = BN + 4;   // leading dimension of the P / dS staging tiles
+constexpr int BM = 32;        // stationary rows per block
+constexpr int NG = 4;         // groups of 64 threads per block
+constexpr int NT = 64 * NG;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LN2 = 0.6931471805599453f;
 
@@ -20,499 +27,543 @@ struct Strides3 { long long b, h, t; };
 
 struct F32Params {
     const float* q; const float* k; const float* v; const float* o; const float* d_o;
-    float* out_o; float* lse_out; const float* lse; float* delta;
+    float* out_o; float* lse_out; const float* lse;
     float* dq; float* dk; float* dv;
     Strides3 sq, sk, sv, so, sdo, sdq, sdk, sdv;
     int B, H, T, D;
     int causal;
-    int vec;            // 1: every row start is 16-byte aligned and D % 4 == 0
+    int vec;            // 1: every row start of the inputs is 16-byte aligned and D % 4 == 0
+    int vec_out;        // the same for the outputs
     float scale;
 };
 
-// Copies rows [row0, row0+64) x [0, DP) of a [T, D] matrix (row stride `st`) into
-// shared memory with leading dimension DP+4, zero-filling rows >= T and columns >= D.
-template <int DP>
-__device__ __forceinline__ void load_tile(float* __restrict__ dst, const float* __restrict__ src,
-                                          int row0, int T, int D, long long st, int vec) {
-    constexpr int LD = DP + 4;
+__device__ __forceinline__ void cp16(float* dst, const float* src, int n) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp4(float* dst, const float* src, int n) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// The two warps of a group meet (barrier 0 is __syncthreads).
+__device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory"); }
+
+// Enqueues rows [row0, row0 + ROWS) x [0, DP) of a [T, D] matrix for shared memory (row stride DP + 4), zeros
+// beyond T and D; COUNT threads of index t share the pieces.
+template <int DP, int ROWS, int COUNT>
+__device__ __forceinline__ void fetch_tile(float* __restrict__ dst, const float* __restrict__ src, int row0, int T, int D,
+                                           long long st, int vec, int t) {
     constexpr int C4 = DP / 4;
-    for (int idx = threadIdx.x; idx < BM * C4; idx += NT) {
+    constexpr int PIECES = ROWS * C4;
+#pragma unroll
+    for (int i = 0; i < (PIECES + COUNT - 1) / COUNT; ++i) {
+        const int idx = t + i * COUNT;
+        if (PIECES % COUNT != 0 && idx >= PIECES) break;
         const int r = idx / C4, c = (idx % C4) * 4;
-        const int row = row0 + r;
-        float4 val = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row < T) {
-            const float* p = src + (long long)row * st + c;
-            if (vec) {
-                if (c < D) val = *reinterpret_cast<const float4*>(p);
-            } else {
-                if (c + 0 < D) val.x = p[0];
-                if (c + 1 < D) val.y = p[1];
-                if (c + 2 < D) val.z = p[2];
-                if (c + 3 < D) val.w = p[3];
+        const bool row_ok = row0 + r < T;
+        const float* p = src + (long long)(row0 + r) * st + c;
+        float* d = dst + r * (DP + 4) + c;
+        if (vec) {
+            const bool ok = row_ok && c < D;
+            cp16(d, ok ? p : src, ok ? 16 : 0);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const bool ok = row_ok && c + e < D;
+                cp4(d + e, ok ? p + e : src, ok ? 4 : 0);
             }
         }
-        *reinterpret_cast<float4*>(dst + r * LD + c) = val;
     }
 }
 
-// The same tile in two halves, global -> registers (fetch) and registers -> shared memory (put), so that the
-// next tile of a walk is in flight while the current one is multiplied.  Used for head dims up to 64 (two or
-// four float4 per thread and tile); at 128 the kernels have no registers to spare and load in place.
-template <int DP>
-struct TileRegs {
-    static constexpr int C4 = DP / 4;
-    static constexpr int NV = BM * C4 / NT;
-    float4 v[NV];
-    __device__ __forceinline__ void fetch(const float* __restrict__ src, int row0, int T, int D, long long st, int vec) {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int idx = threadIdx.x + i * NT;
-            const int r = idx / C4, c = (idx % C4) * 4;
-            const int row = row0 + r;
-            float4 val = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (row < T) {
-                const float* p = src + (long long)row * st + c;
-                if (vec) {
-                    if (c < D) val = *reinterpret_cast<const float4*>(p);
-                } else {
-                    if (c + 0 < D) val.x = p[0];
-                    if (c + 1 < D) val.y = p[1];
-                    if (c + 2 < D) val.z = p[2];
-                    if (c + 3 < D) val.w = p[3];
-                }
-            }
-            v[i] = val;
-        }
-    }
-    __device__ __forceinline__ void put(float* __restrict__ dst) const {
-        constexpr int LD = DP + 4;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int idx = threadIdx.x + i * NT;
-            *reinterpret_cast<float4*>(dst + (idx / C4) * LD + (idx % C4) * 4) = v[i];
-        }
-    }
-};
-__host__ __device__ constexpr bool prefetch_tiles(int DP) { return DP <= 64; }
-
-// s[r][c] = sum_d A[ty*4+r][d] * Bm[tx+16c][d] for two [64][DP+4] shared tiles.
-template <int DP>
-__device__ __forceinline__ void tile_nt(const float* __restrict__ A, const float* __restrict__ Bm,
-                                        int ty, int tx, float (&s)[4][4]) {
+// s[r][c] = sum_d A[4 ty + r][d] * B[tx + 8 c][d]
+template <int DP, int NC>
+__device__ __forceinline__ void tile_nt(const float* __restrict__ A, const float* __restrict__ Bm, int ty, int tx, float (&s)[4][NC]) {
     constexpr int LD = DP + 4;
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) s[r][c] = 0.f;
-#pragma unroll 4
+        for (int c = 0; c < NC; ++c) s[r][c] = 0.f;
+#pragma unroll 2
     for (int d = 0; d < DP; d += 4) {
-        float4 a[4], b[4];
+        float4 a[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(A + (ty * 4 + r) * LD + d);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const float4*>(Bm + (tx + 16 * c) * LD + d);
+        for (int c = 0; c < NC; ++c) {
+            const float4 b = *reinterpret_cast<const float4*>(Bm + (tx + 8 * c) * LD + d);
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                s[r][c] = fmaf(a[r].x, b[c].x, s[r][c]);
-                s[r][c] = fmaf(a[r].y, b[c].y, s[r][c]);
-                s[r][c] = fmaf(a[r].z, b[c].z, s[r][c]);
-                s[r][c] = fmaf(a[r].w, b[c].w, s[r][c]);
+            for (int r = 0; r < 4; ++r) {
+                s[r][c] = fmaf(a[r].x, b.x, s[r][c]);
+                s[r][c] = fmaf(a[r].y, b.y, s[r][c]);
+                s[r][c] = fmaf(a[r].z, b.z, s[r][c]);
+                s[r][c] = fmaf(a[r].w, b.w, s[r][c]);
             }
+        }
     }
 }
 
-// acc[r][c] += sum_k Ps[ty*4+r][k] * Vs[k][tx+16c]   (P row-major [64][PLD], V [64][DP+4])
-template <int DP>
-__device__ __forceinline__ void tile_pv(const float* __restrict__ Ps, const float* __restrict__ Vs,
-                                        int ty, int tx, float (&acc)[4][DP / 16]) {
+// acc[r][4 j + e] += sum_k P[4 ty + r][k] * X[k][4 tx + 32 j + e], k < KN (P row stride PLD)
+template <int DP, int KN, int PLD>
+__device__ __forceinline__ void tile_pv(const float* __restrict__ Ps, const float* __restrict__ X, int ty, int tx, float (&acc)[4][DP / 8]) {
     constexpr int LD = DP + 4;
 #pragma unroll 2
-    for (int k = 0; k < BN; k += 4) {
+    for (int k = 0; k < KN; k += 4) {
         float4 p[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) p[r] = *reinterpret_cast<const float4*>(Ps + (ty * 4 + r) * PLD + k);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
-            float vv[DP / 16];
 #pragma unroll
-            for (int c = 0; c < DP / 16; ++c) vv[c] = Vs[(k + kk) * LD + tx + 16 * c];
+            for (int j = 0; j < DP / 32; ++j) {
+                const float4 x = *reinterpret_cast<const float4*>(X + (k + kk) * LD + tx * 4 + 32 * j);
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float pr = kk == 0 ? p[r].x : kk == 1 ? p[r].y : kk == 2 ? p[r].z : p[r].w;
-#pragma unroll
-                for (int c = 0; c < DP / 16; ++c) acc[r][c] = fmaf(pr, vv[c], acc[r][c]);
+                for (int r = 0; r < 4; ++r) {
+                    const float pr = kk == 0 ? p[r].x : kk == 1 ? p[r].y : kk == 2 ? p[r].z : p[r].w;
+                    acc[r][4 * j + 0] = fmaf(pr, x.x, acc[r][4 * j + 0]);
+                    acc[r][4 * j + 1] = fmaf(pr, x.y, acc[r][4 * j + 1]);
+                    acc[r][4 * j + 2] = fmaf(pr, x.z, acc[r][4 * j + 2]);
+                    acc[r][4 * j + 3] = fmaf(pr, x.w, acc[r][4 * j + 3]);
+                }
             }
         }
     }
 }
 
-// acc[r][c] += sum_q Ps[q][ty*4+r] * Xs[q][tx+16c]   (transposed use of a [64][PLD] tile)
-template <int DP>
-__device__ __forceinline__ void tile_tn(const float* __restrict__ Ps, const float* __restrict__ Xs,
-                                        int ty, int tx, float (&acc)[4][DP / 16]) {
-    constexpr int LD = DP + 4;
-#pragma unroll 4
-    for (int qi = 0; qi < BM; ++qi) {
-        const float4 p = *reinterpret_cast<const float4*>(Ps + qi * PLD + ty * 4);
-        float xv[DP / 16];
+// Row reductions over the eight threads that share a row.
+__device__ __forceinline__ float row_max(float x) {
 #pragma unroll
-        for (int c = 0; c < DP / 16; ++c) xv[c] = Xs[qi * LD + tx + 16 * c];
+    for (int o = 4; o >= 1; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+    return x;
+}
+__device__ __forceinline__ float row_sum(float x) {
 #pragma unroll
-        for (int c = 0; c < DP / 16; ++c) {
-            acc[0][c] = fmaf(p.x, xv[c], acc[0][c]);
-            acc[1][c] = fmaf(p.y, xv[c], acc[1][c]);
-            acc[2][c] = fmaf(p.z, xv[c], acc[2][c]);
-            acc[3][c] = fmaf(p.w, xv[c], acc[3][c]);
-        }
-    }
+    for (int o = 4; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
 }
 
-__device__ __forceinline__ float half_warp_max(float x) {
+template <int DP>
+__device__ __forceinline__ void put_acc(float* dst, int ty, int tx, const float (&acc)[4][DP / 8]) {
 #pragma unroll
-    for (int o = 8; o >= 1; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
-    return x;
-}
-__device__ __forceinline__ float half_warp_sum(float x) {
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int o = 8; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    return x;
+        for (int j = 0; j < DP / 32; ++j)
+            *reinterpret_cast<float4*>(dst + (ty * 4 + r) * (DP + 4) + tx * 4 + 32 * j) =
+                make_float4(acc[r][4 * j], acc[r][4 * j + 1], acc[r][4 * j + 2], acc[r][4 * j + 3]);
 }
+
+// One 16-byte piece of an output row, element by element where alignment or D ask for it.
+__device__ __forceinline__ void store4(float* p, float4 v, int valid, int vec) {
+    if (vec) { if (valid > 0) *reinterpret_cast<float4*>(p) = v; return; }
+    if (valid > 0) p[0] = v.x;
+    if (valid > 1) p[1] = v.y;
+    if (valid > 2) p[2] = v.z;
+    if (valid > 3) p[3] = v.w;
+}
+
+template <int DP>
+struct Tile {
+    static constexpr int BN = DP <= 64 ? 64 : 32;               // rows of a streamed tile
+    static constexpr int NC = BN / 8;                           // score columns per thread
+    static constexpr int LD = DP + 4;
+    static constexpr int ROWS = BM * LD;                        // a stationary tile
+    static constexpr int STREAM = BN * LD;                      // a streamed tile
+    // forward: Q | per group: K, V, P.  The merge at the end reuses the groups' K (partial O) and P (max, sum).
+    static constexpr int FWD_PLD = BN + 4;
+    static constexpr int FWD_GROUP = 2 * STREAM + BM * FWD_PLD;
+    static constexpr size_t FWD_SMEM = (size_t)(ROWS + NG * FWD_GROUP) * sizeof(float);
+    // backward: two stationary tiles | per group: two streamed tiles, half a P / dS tile (32 columns), row statistics
+    static constexpr int BWD_PLD = 36;
+    static constexpr int BWD_BN = 32;
+    static constexpr int BWD_STREAM = BWD_BN * LD;
+    static constexpr int BWD_GROUP = 2 * BWD_STREAM + BM * BWD_PLD + 2 * BWD_BN;
+    static constexpr size_t BWD_SMEM = (size_t)(2 * ROWS + 2 * BM + NG * BWD_GROUP) * sizeof(float);
+};
 
 // ---------------------------------------------------------------------------
-// Forward: one CTA per (batch*head, 64-row query tile).  Heavy (late) query
-// tiles are scheduled first so that the causal triangle balances.
+// Forward: one block per (batch*head, 32-row query tile); the heaviest (latest) query tiles of all slices first.
 // ---------------------------------------------------------------------------
 template <int DP>
 __global__ void __launch_bounds__(NT) attn_fwd_f32_kernel(const F32Params p) {
+    using L = Tile<DP>;
+    constexpr int BN = L::BN, NC = L::NC, LD = L::LD, PLD = L::FWD_PLD;
     extern __shared__ __align__(16) float smem[];
-    constexpr int LD = DP + 4;
+    const int g = threadIdx.x / 64, t = threadIdx.x % 64;
+    const int ty = (t / 32) * 4 + (t % 32) / 8, tx = t % 8;
     float* Qs = smem;
-    float* Ks = Qs + BM * LD;
-    float* Vs = Ks + BN * LD;
-    float* Ps = Vs + BN * LD;
+    float* Ks = Qs + L::ROWS + g * L::FWD_GROUP;
+    float* Vs = Ks + L::STREAM;
+    float* Ps = Vs + L::STREAM;
 
     const int nq = (p.T + BM - 1) / BM;
-    const int qt = nq - 1 - (int)blockIdx.x;
-    const int bh = blockIdx.y;
+    const int q0 = (nq - 1 - (int)blockIdx.y) * BM;
+    const int bh = blockIdx.x;
     const int b = bh / p.H, h = bh % p.H;
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-    const int q0 = qt * BM;
-
-    const float* qb = p.q + b * p.sq.b + h * p.sq.h;
     const float* kb = p.k + b * p.sk.b + h * p.sk.h;
     const float* vb = p.v + b * p.sv.b + h * p.sv.h;
+    const int keys = p.causal ? min(p.T, q0 + BM) : p.T;
+    const int ntiles = (keys + BN - 1) / BN;
 
-    load_tile<DP>(Qs, qb, q0, p.T, p.D, p.sq.t, p.vec);
+    fetch_tile<DP, BM, NT>(Qs, p.q + b * p.sq.b + h * p.sq.h, q0, p.T, p.D, p.sq.t, p.vec, threadIdx.x);
+    if (g < ntiles) fetch_tile<DP, BN, 64>(Ks, kb, g * BN, p.T, p.D, p.sk.t, p.vec, t);
+    cp_commit();
+    if (g < ntiles) fetch_tile<DP, BN, 64>(Vs, vb, g * BN, p.T, p.D, p.sv.t, p.vec, t);
+    cp_commit();
+    cp_wait<1>();
+    __syncthreads();                                            // Q is shared by the groups
 
-    float m[4], l[4], acc[4][DP / 16];
+    float m[4], l[4], acc[4][DP / 8];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         m[r] = -INFINITY; l[r] = 0.f;
 #pragma unroll
-        for (int c = 0; c < DP / 16; ++c) acc[r][c] = 0.f;
+        for (int c = 0; c < DP / 8; ++c) acc[r][c] = 0.f;
     }
     const float sl2 = p.scale * LOG2E;
-    const int last = p.causal ? qt : (p.T + BN - 1) / BN - 1;
 
-    TileRegs<prefetch_tiles(DP) ? DP : 16> kr, vr;     // unused (and tiny) when the tiles are loaded in place
-    if constexpr (prefetch_tiles(DP)) {
-        kr.fetch(kb, 0, p.T, p.D, p.sk.t, p.vec);
-        vr.fetch(vb, 0, p.T, p.D, p.sv.t, p.vec);
-    }
-    for (int j = 0; j <= last; ++j) {
+    for (int j = g; j < ntiles; j += NG) {
         const int k0 = j * BN;
-        __syncthreads();                       // previous tile fully consumed (and Q visible)
-        if constexpr (prefetch_tiles(DP)) {
-            kr.put(Ks); vr.put(Vs);
-            if (j < last) {                    // the next tile travels while this one is multiplied
-                kr.fetch(kb, k0 + BN, p.T, p.D, p.sk.t, p.vec);
-                vr.fetch(vb, k0 + BN, p.T, p.D, p.sv.t, p.vec);
-            }
-        } else {
-            load_tile<DP>(Ks, kb, k0, p.T, p.D, p.sk.t, p.vec);
-            load_tile<DP>(Vs, vb, k0, p.T, p.D, p.sv.t, p.vec);
-        }
-        __syncthreads();
-
-        float s[4][4];
-        tile_nt<DP>(Qs, Ks, ty, tx, s);
+        if (j != g) { cp_wait<1>(); group_sync(g); }            // this K tile has landed for both warps
+        float s[4][NC];
+        tile_nt<DP, NC>(Qs, Ks, ty, tx, s);
+        group_sync(g);                                          // K is consumed: the next one may land
+        if (j + NG < ntiles) fetch_tile<DP, BN, 64>(Ks, kb, k0 + NG * BN, p.T, p.D, p.sk.t, p.vec, t);
+        cp_commit();
+        const bool edge = k0 + BN > p.T || (p.causal && k0 + BN - 1 > q0);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int row = q0 + ty * 4 + r;
             float mx = -INFINITY;
+            if (edge) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int col = k0 + tx + 16 * c;
-                const bool masked = (col >= p.T) || (p.causal && col > row);
-                s[r][c] = masked ? -INFINITY : s[r][c] * sl2;
-                mx = fmaxf(mx, s[r][c]);
+                for (int c = 0; c < NC; ++c) {
+                    const int col = k0 + tx + 8 * c;
+                    s[r][c] = (col >= p.T || (p.causal && col > row)) ? -INFINITY : s[r][c] * sl2;
+                    mx = fmaxf(mx, s[r][c]);
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < NC; ++c) { s[r][c] *= sl2; mx = fmaxf(mx, s[r][c]); }
             }
-            mx = half_warp_max(mx);
-            const float m_new = fmaxf(m[r], mx);
+            const float m_new = fmaxf(m[r], row_max(mx));
             const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
             const float alpha = exp2f(m[r] - m_use);
             float rs = 0.f;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < NC; ++c) {
                 const float e = exp2f(s[r][c] - m_use);
                 rs += e;
-                Ps[(ty * 4 + r) * PLD + tx + 16 * c] = e;
+                Ps[(ty * 4 + r) * PLD + tx + 8 * c] = e;
             }
-            rs = half_warp_sum(rs);
-            l[r] = l[r] * alpha + rs;
+            l[r] = l[r] * alpha + row_sum(rs);
             m[r] = m_new;
 #pragma unroll
-            for (int c = 0; c < DP / 16; ++c) acc[r][c] *= alpha;
+            for (int c = 0; c < DP / 8; ++c) acc[r][c] *= alpha;
         }
-        __syncthreads();
-        tile_pv<DP>(Ps, Vs, ty, tx, acc);
+        cp_wait<1>();
+        group_sync(g);                                          // V has landed (and this warp's P rows are visible)
+        tile_pv<DP, BN, PLD>(Ps, Vs, ty, tx, acc);
+        group_sync(g);                                          // V is consumed
+        if (j + NG < ntiles) fetch_tile<DP, BN, 64>(Vs, vb, k0 + NG * BN, p.T, p.D, p.sv.t, p.vec, t);
+        cp_commit();
     }
+    cp_wait<0>();
 
+    // The groups meet: O = sum_g 2^(m_g - M) O_g / sum_g 2^(m_g - M) l_g, in group order.
+    put_acc<DP>(Ks, ty, tx, acc);
+    if (tx == 0) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) { Ps[ty * 4 + r] = m[r]; Ps[BM + ty * 4 + r] = l[r]; }
+    }
+    __syncthreads();
     float* ob = p.out_o + b * p.so.b + h * p.so.h;
+    constexpr int C4 = DP / 4;
+    for (int idx = threadIdx.x; idx < BM * C4; idx += NT) {
+        const int r = idx / C4, c = (idx % C4) * 4, row = q0 + r;
+        if (row >= p.T || c >= p.D) continue;
+        const float* grp = smem + L::ROWS;
+        float mg[NG], M = -INFINITY, sum = 0.f;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int row = q0 + ty * 4 + r;
-        if (row >= p.T) continue;
-        const float inv = 1.f / l[r];
+        for (int z = 0; z < NG; ++z) { mg[z] = grp[z * L::FWD_GROUP + 2 * L::STREAM + r]; M = fmaxf(M, mg[z]); }
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int c = 0; c < DP / 16; ++c) {
-            const int col = tx + 16 * c;
-            if (col < p.D) ob[(long long)row * p.so.t + col] = acc[r][c] * inv;
+        for (int z = 0; z < NG; ++z) {
+            const float w = exp2f(mg[z] - M);                   // a group without keys has m = -inf: weight 0
+            const float4 x = *reinterpret_cast<const float4*>(grp + z * L::FWD_GROUP + r * LD + c);
+            sum += w * grp[z * L::FWD_GROUP + 2 * L::STREAM + BM + r];
+            v.x = fmaf(w, x.x, v.x); v.y = fmaf(w, x.y, v.y); v.z = fmaf(w, x.z, v.z); v.w = fmaf(w, x.w, v.w);
         }
-        if (tx == 0) p.lse_out[((long long)bh) * p.T + row] = (m[r] + log2f(l[r])) * LN2;
+        const float inv = 1.f / sum;
+        store4(ob + (long long)row * p.so.t + c, make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv), p.D - c, p.vec_out);
+        if (c == 0) p.lse_out[(long long)bh * p.T + row] = (M + log2f(sum)) * LN2;
     }
 }
 
 // ---------------------------------------------------------------------------
-// delta[bh][t] = sum_d dO[t][d] * O[t][d]  (= rowsum(dP * P)); one warp per row.
+// Backward
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) attn_delta_f32_kernel(const F32Params p) {
-    const long long row = (long long)blockIdx.x * 8 + threadIdx.x / 32;
-    const int lane = threadIdx.x % 32;
-    const long long rows = (long long)p.B * p.H * p.T;
-    if (row >= rows) return;
-    const int t = (int)(row % p.T);
-    const int bh = (int)(row / p.T);
-    const int b = bh / p.H, h = bh % p.H;
-    const float* o = p.o + b * p.so.b + h * p.so.h + (long long)t * p.so.t;
-    const float* g = p.d_o + b * p.sdo.b + h * p.sdo.h + (long long)t * p.sdo.t;
-    float acc = 0.f;
-    for (int d = lane; d < p.D; d += 32) acc = fmaf(o[d], g[d], acc);
+// delta = rowsum(dO * O) (= rowsum(dP * P)), LPR lanes per row: dO from its shared tile, O from global memory.  load() may
+// run long before dot(), so that the walk does not wait for global memory (head dims up to 32: 16 registers).
+template <int DP, int LPR>
+struct RowDelta {
+    static constexpr int N = DP / 4 / LPR;
+    static constexpr bool EARLY = N <= 4;
+    float4 o[EARLY ? N : 1];
+    __device__ __forceinline__ static float4 piece(const F32Params& p, const float* orow, int c) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.vec) {
+            if (c < p.D) v = *reinterpret_cast<const float4*>(orow + c);
+        } else {
+            if (c + 0 < p.D) v.x = orow[c + 0];
+            if (c + 1 < p.D) v.y = orow[c + 1];
+            if (c + 2 < p.D) v.z = orow[c + 2];
+            if (c + 3 < p.D) v.w = orow[c + 3];
+        }
+        return v;
+    }
+    __device__ __forceinline__ void load(const F32Params& p, const float* ob, int row, int part) {
+        if constexpr (EARLY) {
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (lane == 0) p.delta[row] = acc;
+            for (int i = 0; i < N; ++i) o[i] = row < p.T ? piece(p, ob + (long long)row * p.so.t, (part + LPR * i) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    __device__ __forceinline__ float dot(const F32Params& p, const float* ob, const float* g_row, int row, int part) {
+        float d = 0.f;
+        if (row < p.T) {
+#pragma unroll 4
+            for (int i = 0; i < N; ++i) {
+                const int c = (part + LPR * i) * 4;
+                float4 x;
+                if constexpr (EARLY) x = o[i]; else x = piece(p, ob + (long long)row * p.so.t, c);
+                const float4 y = *reinterpret_cast<const float4*>(g_row + c);
+                d = fmaf(x.x, y.x, d); d = fmaf(x.y, y.y, d); d = fmaf(x.z, y.z, d); d = fmaf(x.w, y.w, d);
+            }
+        }
+#pragma unroll
+        for (int off = LPR / 2; off >= 1; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
+        return d;
+    }
+};
+
+// Adds the groups' partial gradients (each parked in its first streamed tile) and stores the block's rows.
+template <int DP>
+__device__ __forceinline__ void merge_store(const F32Params& p, const float* parts, int stride, float* dst, long long st, int row0) {
+    constexpr int C4 = DP / 4;
+    for (int idx = threadIdx.x; idx < BM * C4; idx += NT) {
+        const int r = idx / C4, c = (idx % C4) * 4, row = row0 + r;
+        if (row >= p.T || c >= p.D) continue;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int z = 0; z < NG; ++z) {
+            const float4 x = *reinterpret_cast<const float4*>(parts + z * stride + r * (DP + 4) + c);
+            v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+        }
+        store4(dst + (long long)row * st + c, v, p.D - c, p.vec_out);
+    }
 }
 
-// Recomputes, for the 64 x 64 tile (q0, k0): P (0 where masked or out of range)
-// and dS = scale * P * (dP - delta).  Patch layout as tile_nt.
-template <int DP>
-__device__ __forceinline__ void recompute_p_ds(const F32Params& p, const float* Qs, const float* Ks,
-                                               const float* dOs, const float* Vs, const float* lse_s,
-                                               const float* delta_s, int q0, int k0, int ty, int tx,
-                                               float (&pp)[4][4], float (&ds)[4][4]) {
-    float dp[4][4];
-    tile_nt<DP>(Qs, Ks, ty, tx, pp);
-    tile_nt<DP>(dOs, Vs, ty, tx, dp);
+// Scores to P in place: rows are query rows (ROWS_ARE_Q) or key rows of the 32 x BN tile; l2 / dl hold lse * log2e and delta
+// of the tile's query rows.
+template <int NC, bool ROWS_ARE_Q>
+__device__ __forceinline__ void probabilities(const F32Params& p, float (&s)[4][NC], const float* l2, int row0, int col0, int ty, int tx) {
     const float sl2 = p.scale * LOG2E;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-        const int row = q0 + ty * 4 + r;
-        const float l2 = lse_s[ty * 4 + r] * LOG2E;
-        const float dl = delta_s[ty * 4 + r];
+        const int row = row0 + ty * 4 + r;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int col = k0 + tx + 16 * c;
-            const bool masked = (row >= p.T) || (col >= p.T) || (p.causal && col > row);
-            const float e = masked ? 0.f : exp2f(pp[r][c] * sl2 - l2);
-            pp[r][c] = e;
-            ds[r][c] = e * (dp[r][c] - dl) * p.scale;
+        for (int c = 0; c < NC; ++c) {
+            const int col = col0 + tx + 8 * c;
+            const bool masked = row >= p.T || col >= p.T || (p.causal && (ROWS_ARE_Q ? col > row : row > col));
+            const float lq = ROWS_ARE_Q ? l2[ty * 4 + r] : l2[tx + 8 * c];
+            s[r][c] = masked ? 0.f : exp2f(fmaf(s[r][c], sl2, -lq));
         }
     }
 }
 
-// ---------------------------------------------------------------------------
-// Backward, dK/dV: one CTA per (batch*head, KV tile); it visits every query tile
-// at or below its diagonal and keeps dK/dV in registers, so no atomics are needed.
-// ---------------------------------------------------------------------------
+// acc += tile * X with the 32 x BN tile handed through shared memory 32 columns at a time (rows stay inside a warp).
+template <int DP, int NC>
+__device__ __forceinline__ void staged_product(float* stage, const float (&v)[4][NC], const float* X, int ty, int tx, float (&acc)[4][DP / 8]) {
+    constexpr int PLD = Tile<DP>::BWD_PLD;
+#pragma unroll
+    for (int half = 0; half < NC / 4; ++half) {
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) stage[(ty * 4 + r) * PLD + tx + 8 * c] = v[r][half * 4 + c];
+        __syncwarp();
+        tile_pv<DP, 32, PLD>(stage, X + half * 32 * (DP + 4), ty, tx, acc);
+    }
+}
+
+// dK / dV of 32 key rows: the groups walk the query tiles at or below the diagonal.
 template <int DP>
-__device__ __forceinline__ void attn_bwd_dkdv_f32_body(const F32Params& p, float* smem) {
-    constexpr int LD = DP + 4;
+__device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt, int bh) {
+    using L = Tile<DP>;
+    constexpr int BN = L::BWD_BN, NC = BN / 8, LD = L::LD;
+    const int g = threadIdx.x / 64, t = threadIdx.x % 64;
+    const int ty = (t / 32) * 4 + (t % 32) / 8, tx = t % 8;
     float* Ks = smem;
-    float* Vs = Ks + BN * LD;
-    float* Qs = Vs + BN * LD;
-    float* dOs = Qs + BM * LD;
-    float* Ps = dOs + BM * LD;
-    float* dSs = Ps + BM * PLD;
-    float* lse_s = dSs + BM * PLD;
-    float* delta_s = lse_s + BM;
+    float* Vs = Ks + L::ROWS;
+    float* grp0 = smem + 2 * L::ROWS + 2 * BM;
+    float* Qs = grp0 + g * L::BWD_GROUP;
+    float* Gs = Qs + L::BWD_STREAM;
+    float* stage = Gs + L::BWD_STREAM;
+    float* l2 = stage + BM * L::BWD_PLD;
+    float* dl = l2 + BN;
 
-    const int kt = blockIdx.x;                 // low KV tiles carry the most work: scheduled first
-    const int bh = blockIdx.y;
     const int b = bh / p.H, h = bh % p.H;
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-    const int k0 = kt * BN;
-    const int nq = (p.T + BM - 1) / BM;
-
-    load_tile<DP>(Ks, p.k + b * p.sk.b + h * p.sk.h, k0, p.T, p.D, p.sk.t, p.vec);
-    load_tile<DP>(Vs, p.v + b * p.sv.b + h * p.sv.h, k0, p.T, p.D, p.sv.t, p.vec);
-
-    float dk[4][DP / 16], dv[4][DP / 16];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < DP / 16; ++c) { dk[r][c] = 0.f; dv[r][c] = 0.f; }
-
+    const int k0 = kt * BM;
     const float* qb = p.q + b * p.sq.b + h * p.sq.h;
     const float* gb = p.d_o + b * p.sdo.b + h * p.sdo.h;
-    const int i_first = p.causal ? kt : 0;
-    TileRegs<prefetch_tiles(DP) ? DP : 16> qr, gr;
-    if constexpr (prefetch_tiles(DP)) {
-        if (i_first < nq) {
-            qr.fetch(qb, i_first * BM, p.T, p.D, p.sq.t, p.vec);
-            gr.fetch(gb, i_first * BM, p.T, p.D, p.sdo.t, p.vec);
-        }
-    }
-    for (int i = i_first; i < nq; ++i) {
-        const int q0 = i * BM;
-        __syncthreads();
-        if constexpr (prefetch_tiles(DP)) {
-            qr.put(Qs); gr.put(dOs);
-            if (i + 1 < nq) {
-                qr.fetch(qb, q0 + BM, p.T, p.D, p.sq.t, p.vec);
-                gr.fetch(gb, q0 + BM, p.T, p.D, p.sdo.t, p.vec);
-            }
-        } else {
-            load_tile<DP>(Qs, qb, q0, p.T, p.D, p.sq.t, p.vec);
-            load_tile<DP>(dOs, gb, q0, p.T, p.D, p.sdo.t, p.vec);
-        }
-        if (threadIdx.x < BM) {
-            const int row = q0 + threadIdx.x;
-            lse_s[threadIdx.x] = row < p.T ? p.lse[(long long)bh * p.T + row] : 0.f;
-            delta_s[threadIdx.x] = row < p.T ? p.delta[(long long)bh * p.T + row] : 0.f;
-        }
-        __syncthreads();
-        float pp[4][4], ds[4][4];
-        recompute_p_ds<DP>(p, Qs, Ks, dOs, Vs, lse_s, delta_s, q0, k0, ty, tx, pp, ds);
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                Ps[(ty * 4 + r) * PLD + tx + 16 * c] = pp[r][c];
-                dSs[(ty * 4 + r) * PLD + tx + 16 * c] = ds[r][c];
-            }
-        __syncthreads();
-        tile_tn<DP>(Ps, dOs, ty, tx, dv);      // dV += P^T dO
-        tile_tn<DP>(dSs, Qs, ty, tx, dk);      // dK += dS^T Q
-    }
+    const float* ob = p.o + b * p.so.b + h * p.so.h;
+    const int first = p.causal ? k0 / BN : 0, ntiles = (p.T + BN - 1) / BN;
+    const int i0 = first + g;
 
-    float* dkb = p.dk + b * p.sdk.b + h * p.sdk.h;
-    float* dvb = p.dv + b * p.sdv.b + h * p.sdv.h;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int row = k0 + ty * 4 + r;
-        if (row >= p.T) continue;
-#pragma unroll
-        for (int c = 0; c < DP / 16; ++c) {
-            const int col = tx + 16 * c;
-            if (col < p.D) {
-                dkb[(long long)row * p.sdk.t + col] = dk[r][c];
-                dvb[(long long)row * p.sdv.t + col] = dv[r][c];
-            }
-        }
-    }
-}
+    fetch_tile<DP, BM, NT>(Ks, p.k + b * p.sk.b + h * p.sk.h, k0, p.T, p.D, p.sk.t, p.vec, threadIdx.x);
+    if (i0 < ntiles) fetch_tile<DP, BN, 64>(Qs, qb, i0 * BN, p.T, p.D, p.sq.t, p.vec, t);
+    cp_commit();
+    fetch_tile<DP, BM, NT>(Vs, p.v + b * p.sv.b + h * p.sv.h, k0, p.T, p.D, p.sv.t, p.vec, threadIdx.x);
+    if (i0 < ntiles) fetch_tile<DP, BN, 64>(Gs, gb, i0 * BN, p.T, p.D, p.sdo.t, p.vec, t);
+    cp_commit();
+    cp_wait<0>();
+    __syncthreads();                                            // K and V are shared by the groups
 
-// ---------------------------------------------------------------------------
-// Backward, dQ: one CTA per (batch*head, query tile), looping over the KV tiles
-// at or left of its diagonal.
-// ---------------------------------------------------------------------------
-template <int DP>
-__device__ __forceinline__ void attn_bwd_dq_f32_body(const F32Params& p, float* smem) {
-    constexpr int LD = DP + 4;
-    float* Ks = smem;
-    float* Vs = Ks + BN * LD;
-    float* Qs = Vs + BN * LD;
-    float* dOs = Qs + BM * LD;
-    float* dSs = dOs + BM * LD;
-    float* lse_s = dSs + BM * PLD;
-    float* delta_s = lse_s + BM;
-
-    const int nq = (p.T + BM - 1) / BM;
-    const int qt = nq - 1 - (int)blockIdx.x;
-    const int bh = blockIdx.y;
-    const int b = bh / p.H, h = bh % p.H;
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-    const int q0 = qt * BM;
-
-    load_tile<DP>(Qs, p.q + b * p.sq.b + h * p.sq.h, q0, p.T, p.D, p.sq.t, p.vec);
-    load_tile<DP>(dOs, p.d_o + b * p.sdo.b + h * p.sdo.h, q0, p.T, p.D, p.sdo.t, p.vec);
-    if (threadIdx.x < BM) {
-        const int row = q0 + threadIdx.x;
-        lse_s[threadIdx.x] = row < p.T ? p.lse[(long long)bh * p.T + row] : 0.f;
-        delta_s[threadIdx.x] = row < p.T ? p.delta[(long long)bh * p.T + row] : 0.f;
-    }
-
-    float dq[4][DP / 16];
+    float dk[4][DP / 8], dv[4][DP / 8];
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < DP / 16; ++c) dq[r][c] = 0.f;
+        for (int c = 0; c < DP / 8; ++c) { dk[r][c] = 0.f; dv[r][c] = 0.f; }
 
-    const float* kb = p.k + b * p.sk.b + h * p.sk.h;
-    const float* vb = p.v + b * p.sv.b + h * p.sv.h;
-    const int last = p.causal ? qt : (p.T + BN - 1) / BN - 1;
-    TileRegs<prefetch_tiles(DP) ? DP : 16> kr, vr;
-    if constexpr (prefetch_tiles(DP)) {
-        kr.fetch(kb, 0, p.T, p.D, p.sk.t, p.vec);
-        vr.fetch(vb, 0, p.T, p.D, p.sv.t, p.vec);
-    }
-    for (int j = 0; j <= last; ++j) {
-        const int k0 = j * BN;
-        __syncthreads();
-        if constexpr (prefetch_tiles(DP)) {
-            kr.put(Ks); vr.put(Vs);
-            if (j < last) {
-                kr.fetch(kb, k0 + BN, p.T, p.D, p.sk.t, p.vec);
-                vr.fetch(vb, k0 + BN, p.T, p.D, p.sv.t, p.vec);
-            }
-        } else {
-            load_tile<DP>(Ks, kb, k0, p.T, p.D, p.sk.t, p.vec);
-            load_tile<DP>(Vs, vb, k0, p.T, p.D, p.sv.t, p.vec);
+    RowDelta<DP, 2> rd;                                         // two threads per row of the 32-row tile
+    float lse_next = 0.f;
+    auto stats_ahead = [&](int q0) {
+        const int row = q0 + t / 2;
+        rd.load(p, ob, row, t % 2);
+        lse_next = row < p.T ? p.lse[(long long)bh * p.T + row] * LOG2E : 0.f;
+    };
+    static_assert(BN == 32, "two threads per row");
+    if (i0 < ntiles) stats_ahead(i0 * BN);
+    for (int i = i0; i < ntiles; i += NG) {
+        const int q0 = i * BN;
+        if (i != i0) { cp_wait<1>(); group_sync(g); }           // this Q tile has landed for both warps
+        float pp[4][NC], ds[4][NC];
+        tile_nt<DP, NC>(Ks, Qs, ty, tx, pp);                    // S^T
+        if (i != i0) { cp_wait<0>(); group_sync(g); }           // and so has dO
+        {
+            const float d = rd.dot(p, ob, Gs + (t / 2) * LD, q0 + t / 2, t % 2);
+            if (t % 2 == 0) { l2[t / 2] = lse_next; dl[t / 2] = d; }
         }
-        __syncthreads();
-        float pp[4][4], ds[4][4];
-        recompute_p_ds<DP>(p, Qs, Ks, dOs, Vs, lse_s, delta_s, q0, k0, ty, tx, pp, ds);
+        tile_nt<DP, NC>(Vs, Gs, ty, tx, ds);                    // dP^T
+        group_sync(g);                                          // statistics are visible
+        probabilities<NC, false>(p, pp, l2, k0, q0, ty, tx);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) dSs[(ty * 4 + r) * PLD + tx + 16 * c] = ds[r][c];
-        __syncthreads();
-        tile_pv<DP>(dSs, Ks, ty, tx, dq);      // dQ += dS K
+            for (int c = 0; c < NC; ++c) ds[r][c] = pp[r][c] * (ds[r][c] - dl[tx + 8 * c]) * p.scale;
+        staged_product<DP, NC>(stage, ds, Qs, ty, tx, dk);      // dK += dS^T Q
+        group_sync(g);                                          // Q is consumed
+        if (i + NG < ntiles) fetch_tile<DP, BN, 64>(Qs, qb, q0 + NG * BN, p.T, p.D, p.sq.t, p.vec, t);
+        cp_commit();
+        if (i + NG < ntiles) stats_ahead(q0 + NG * BN);
+        staged_product<DP, NC>(stage, pp, Gs, ty, tx, dv);      // dV += P^T dO
+        group_sync(g);
+        if (i + NG < ntiles) fetch_tile<DP, BN, 64>(Gs, gb, q0 + NG * BN, p.T, p.D, p.sdo.t, p.vec, t);
+        cp_commit();
     }
-
-    float* dqb = p.dq + b * p.sdq.b + h * p.sdq.h;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int row = q0 + ty * 4 + r;
-        if (row >= p.T) continue;
-#pragma unroll
-        for (int c = 0; c < DP / 16; ++c) {
-            const int col = tx + 16 * c;
-            if (col < p.D) dqb[(long long)row * p.sdq.t + col] = dq[r][c];
-        }
-    }
+    cp_wait<0>();
+    put_acc<DP>(Qs, ty, tx, dk);
+    put_acc<DP>(Gs, ty, tx, dv);
+    __syncthreads();
+    merge_store<DP>(p, grp0, L::BWD_GROUP, p.dk + b * p.sdk.b + h * p.sdk.h, p.sdk.t, k0);
+    merge_store<DP>(p, grp0 + L::BWD_STREAM, L::BWD_GROUP, p.dv + b * p.sdv.b + h * p.sdv.h, p.sdv.t, k0);
 }
 
-// dK/dV and dQ in one launch: the two walks share nothing but their inputs, so blockIdx.z picks the role
-// (z = 0: one KV tile per block, z = 1: one query tile per block) and both sets of blocks run side by side;
-// at the model's shapes each alone fills well under one block per SM.
+// dQ of 32 query rows: the groups walk the key tiles at or left of the diagonal.
 template <int DP>
-__global__ void __launch_bounds__(NT) attn_bwd_f32_kernel(const F32Params p) {
+__device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, int bh) {
+    using L = Tile<DP>;
+    constexpr int BN = L::BWD_BN, NC = BN / 8, LD = L::LD;
+    const int g = threadIdx.x / 64, t = threadIdx.x % 64;
+    const int ty = (t / 32) * 4 + (t % 32) / 8, tx = t % 8;
+    float* Qs = smem;
+    float* Gs = Qs + L::ROWS;
+    float* l2 = smem + 2 * L::ROWS;
+    float* dl = l2 + BM;
+    float* grp0 = dl + BM;
+    float* Ks = grp0 + g * L::BWD_GROUP;
+    float* Vs = Ks + L::BWD_STREAM;
+    float* stage = Vs + L::BWD_STREAM;
+
+    const int b = bh / p.H, h = bh % p.H;
+    const int q0 = qt * BM;
+    const float* kb = p.k + b * p.sk.b + h * p.sk.h;
+    const float* vb = p.v + b * p.sv.b + h * p.sv.h;
+    const int keys = p.causal ? min(p.T, q0 + BM) : p.T;
+    const int ntiles = (keys + BN - 1) / BN;
+
+    fetch_tile<DP, BM, NT>(Qs, p.q + b * p.sq.b + h * p.sq.h, q0, p.T, p.D, p.sq.t, p.vec, threadIdx.x);
+    if (g < ntiles) fetch_tile<DP, BN, 64>(Ks, kb, g * BN, p.T, p.D, p.sk.t, p.vec, t);
+    fetch_tile<DP, BM, NT>(Gs, p.d_o + b * p.sdo.b + h * p.sdo.h, q0, p.T, p.D, p.sdo.t, p.vec, threadIdx.x);
+    if (g < ntiles) fetch_tile<DP, BN, 64>(Vs, vb, g * BN, p.T, p.D, p.sv.t, p.vec, t);
+    cp_commit();
+    cp_wait<0>();
+    __syncthreads();                                            // Q and dO are shared by the groups
+    RowDelta<DP, 8> rd;
+    {
+        const int r = threadIdx.x / 8, row = q0 + r;            // eight threads per row
+        const float* ob = p.o + b * p.so.b + h * p.so.h;
+        rd.load(p, ob, row, threadIdx.x % 8);
+        const float d = rd.dot(p, ob, Gs + r * LD, row, threadIdx.x % 8);
+        if (threadIdx.x % 8 == 0) { l2[r] = row < p.T ? p.lse[(long long)bh * p.T + row] * LOG2E : 0.f; dl[r] = d; }
+    }
+
+    float dq[4][DP / 8];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < DP / 8; ++c) dq[r][c] = 0.f;
+    float pp[4][NC], ds[4][NC];
+    if (g < ntiles) tile_nt<DP, NC>(Qs, Ks, ty, tx, pp);        // the first S while the statistics are made
+    __syncthreads();
+
+    for (int j = g; j < ntiles; j += NG) {
+        const int k0 = j * BN;
+        if (j != g) {
+            cp_wait<0>();
+            group_sync(g);
+            tile_nt<DP, NC>(Qs, Ks, ty, tx, pp);
+        }
+        tile_nt<DP, NC>(Gs, Vs, ty, tx, ds);                    // dP
+        group_sync(g);                                          // V is consumed
+        if (j + NG < ntiles) fetch_tile<DP, BN, 64>(Vs, vb, k0 + NG * BN, p.T, p.D, p.sv.t, p.vec, t);
+        cp_commit();
+        probabilities<NC, true>(p, pp, l2, q0, k0, ty, tx);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) ds[r][c] = pp[r][c] * (ds[r][c] - dl[ty * 4 + r]) * p.scale;
+        staged_product<DP, NC>(stage, ds, Ks, ty, tx, dq);      // dQ += dS K
+        group_sync(g);
+        if (j + NG < ntiles) {
+            fetch_tile<DP, BN, 64>(Ks, kb, k0 + NG * BN, p.T, p.D, p.sk.t, p.vec, t);
+        }
+        cp_commit();
+    }
+    cp_wait<0>();
+    put_acc<DP>(Ks, ty, tx, dq);
+    __syncthreads();
+    merge_store<DP>(p, grp0, L::BWD_GROUP, p.dq + b * p.sdq.b + h * p.sdq.h, p.sdq.t, q0);
+}
+
+// Both roles in one launch: blockIdx.y = 2 n is the n-th heaviest key tile, 2 n + 1 the n-th heaviest query tile.
+template <int DP>
+__global__ void __launch_bounds__(NT, DP <= 64 ? 2 : 1) attn_bwd_f32_kernel(const F32Params p) {
     extern __shared__ __align__(16) float smem[];
-    if (blockIdx.z == 0) attn_bwd_dkdv_f32_body<DP>(p, smem);
-    else attn_bwd_dq_f32_body<DP>(p, smem);
+    const int n = blockIdx.y >> 1, tiles = (p.T + BM - 1) / BM;
+    if ((blockIdx.y & 1) == 0) bwd_dkdv<DP>(p, smem, n, blockIdx.x);
+    else bwd_dq<DP>(p, smem, tiles - 1 - n, blockIdx.x);
 }
 
 Strides3 s3(const int64_t* s) { return Strides3{(long long)s[0], (long long)s[1], (long long)s[2]}; }
@@ -523,12 +574,11 @@ bool rows_vec_ok(const void* ptr, const int64_t* s) {
 
 template <int DP>
 int fwd_impl(deers_ctx* ctx, const F32Params& p) {
-    const size_t smem = (size_t)(3 * BM * (DP + 4) + BM * PLD) * sizeof(float);
-    DEERS_SMEM_ONCE(ctx, (attn_fwd_f32_kernel<DP>), smem);
-    dim3 grid((p.T + BM - 1) / BM, p.B * p.H);
+    DEERS_SMEM_ONCE(ctx, (attn_fwd_f32_kernel<DP>), Tile<DP>::FWD_SMEM);
+    const dim3 grid(p.B * p.H, (p.T + BM - 1) / BM);
     {
         KernelTimerScope ts(ctx, DEERS_K_FWD);
-        attn_fwd_f32_kernel<DP><<<grid, NT, smem, ctx->stream>>>(p);
+        attn_fwd_f32_kernel<DP><<<grid, NT, Tile<DP>::FWD_SMEM, ctx->stream>>>(p);
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -537,23 +587,15 @@ int fwd_impl(deers_ctx* ctx, const F32Params& p) {
 
 template <int DP>
 int bwd_impl(deers_ctx* ctx, const F32Params& p) {
-    const long long rows = (long long)p.B * p.H * p.T;
-    {
-        KernelTimerScope ts(ctx, DEERS_K_BWD_PREP);
-        attn_delta_f32_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, ctx->stream>>>(p);
-    }
-    DEERS_CUDA_TRY(ctx, cudaGetLastError());
-    const size_t smem_kv = (size_t)(4 * BM * (DP + 4) + 2 * BM * PLD + 2 * BM) * sizeof(float);
-    const size_t smem_q = (size_t)(4 * BM * (DP + 4) + BM * PLD + 2 * BM) * sizeof(float);
-    const size_t smem = smem_kv > smem_q ? smem_kv : smem_q;
-    DEERS_SMEM_ONCE(ctx, (attn_bwd_f32_kernel<DP>), smem);
-    dim3 grid((p.T + BM - 1) / BM, p.B * p.H, 2);
+    DEERS_SMEM_ONCE(ctx, (attn_bwd_f32_kernel<DP>), Tile<DP>::BWD_SMEM);
+    const dim3 grid(p.B * p.H, 2 * ((p.T + BM - 1) / BM));
+    if (grid.y > 65535) return DEERS_ERR_SHAPE;
     {
         KernelTimerScope ts(ctx, DEERS_K_BWD_MAIN);
-        attn_bwd_f32_kernel<DP><<<grid, NT, smem, ctx->stream>>>(p);
+        attn_bwd_f32_kernel<DP><<<grid, NT, Tile<DP>::BWD_SMEM, ctx->stream>>>(p);
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
-    ctx->launches += 2;
+    ctx->launches += 1;
     return DEERS_OK;
 }
 
@@ -576,20 +618,24 @@ int launch_attn_fwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q
     p.q = q; p.k = k; p.v = v; p.out_o = o; p.lse_out = lse;
     p.vec = (d->D % 4 == 0) && rows_vec_ok(q, d->q_strides) && rows_vec_ok(k, d->k_strides) &&
             rows_vec_ok(v, d->v_strides);
+    p.vec_out = (d->D % 4 == 0) && rows_vec_ok(o, d->o_strides);
     if (d->D <= 32) return fwd_impl<32>(ctx, p);
     if (d->D <= 64) return fwd_impl<64>(ctx, p);
+    if (d->D <= 96) return fwd_impl<96>(ctx, p);
     return fwd_impl<128>(ctx, p);
 }
 
 int launch_attn_bwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q, const float* k,
                         const float* v, const float* o, const float* lse, const float* d_o, float* dq,
-                        float* dk, float* dv, float* delta) {
+                        float* dk, float* dv) {
     F32Params p = base_params(d);
     p.q = q; p.k = k; p.v = v; p.o = o; p.lse = lse; p.d_o = d_o;
-    p.dq = dq; p.dk = dk; p.dv = dv; p.delta = delta;
+    p.dq = dq; p.dk = dk; p.dv = dv;
     p.vec = (d->D % 4 == 0) && rows_vec_ok(q, d->q_strides) && rows_vec_ok(k, d->k_strides) &&
-            rows_vec_ok(v, d->v_strides) && rows_vec_ok(d_o, d->do_strides);
+            rows_vec_ok(v, d->v_strides) && rows_vec_ok(d_o, d->do_strides) && rows_vec_ok(o, d->o_strides);
+    p.vec_out = (d->D % 4 == 0) && rows_vec_ok(dq, d->dq_strides) && rows_vec_ok(dk, d->dk_strides) && rows_vec_ok(dv, d->dv_strides);
     if (d->D <= 32) return bwd_impl<32>(ctx, p);
     if (d->D <= 64) return bwd_impl<64>(ctx, p);
+    if (d->D <= 96) return bwd_impl<96>(ctx, p);
     return bwd_impl<128>(ctx, p);
 }

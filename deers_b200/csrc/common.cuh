@@ -129,7 +129,7 @@ int launch_attn_fwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q
                         const float* v, float* o, float* lse);
 int launch_attn_bwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q, const float* k,
                         const float* v, const float* o, const float* lse, const float* d_o, float* dq,
-                        float* dk, float* dv, float* delta);
+                        float* dk, float* dv);
 
 // f16 tcgen05 path (attn_f16_sm100.cu)
 int launch_attn_fwd_f16(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const void* k,

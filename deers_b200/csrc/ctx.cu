@@ -381,7 +381,7 @@ extern "C" int deers_b200_attn_bwd(deers_ctx* ctx, const deers_attn_desc* d, con
     if (d->dtype == DEERS_F32)
         return launch_attn_bwd_f32(ctx, d, (const float*)q, (const float*)k, (const float*)v,
                                    (const float*)o, lse, (const float*)d_o, (float*)dq, (float*)dk,
-                                   (float*)dv, (float*)workspace);
+                                   (float*)dv);
     const bool keep_ds = workspace_bytes >= attn_bwd_f16_workspace_bytes(d, true);
     return launch_attn_bwd_f16(ctx, d, q, k, v, o, lse, d_o, dq, dk, dv, workspace, keep_ds);
 }

@@ -62,3 +62,32 @@ def test_f32_gemm_tiles_clusters_and_remainders(M, N, K, a_mn, b_mn, aligned):
     tol = 2e-6 * max(1.0, np.sqrt(K) / 4) * max(1.0, np.abs(want).max())
     assert np.abs(got.cpu().numpy() - want).max() <= tol
     assert torch.isnan(big[M]).all() and torch.isnan(big[:M, N:]).all(), "nothing outside C is written"
+
+
+@pytest.mark.parametrize("T", [1, 31, 33, 64, 129, 257])
+@pytest.mark.parametrize("D", [3, 32, 36, 64, 92, 96, 100, 128])
+@pytest.mark.parametrize("causal", [True, False])
+def test_f32_attention_tiles_and_groups(T, D, causal):
+    """Rows per block, tiles per group and head-dim paddings that do not come out even; D = 3 takes the element path."""
+    from deers_b200 import ops
+    from oracle import ref
+    from tests.helpers import TOL_F32
+    rng = np.random.default_rng(T * 131 + D)
+    host = [rng.standard_normal((2, 2, T, D)).astype(np.float32) for _ in range(4)]
+    q, k, v, do = (torch.from_numpy(a).cuda() for a in host)
+    op = ops.CausalAttention.new(q, k, v, None, causal)
+    o = op.forward()
+    grads = ops.GradientStore()
+    op.backward(grads, do)
+    ops.Context.current(q.device).sync()
+    want = ref.attn_fwd_bwd(*host, causal=causal)
+    for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), [o, op.lse] + [grads.get(t) for t in (q, k, v)], want):
+        g = g.cpu().numpy()
+        if T == 1 and name in ("dq", "dk"):
+            # P = 1, so dS = dP - delta cancels to zero; what is left is the rounding of two D-term sums of dO * V,
+            # each within D * 2^-24 * sum |dO V|, times scale and the other operand (the oracle's own is as large)
+            sums = np.abs(host[3] * host[2]).sum(-1).max()
+            other = np.abs(host[1] if name == "dq" else host[0]).max()
+            assert np.abs(g - w).max() <= 4 * D * 2.0 ** -24 * sums * D ** -0.5 * other, name
+        else:
+            assert_close(g, w, TOL_F32, f"T {T} D {D} {name}")
