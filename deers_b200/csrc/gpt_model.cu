@@ -31,6 +31,17 @@ struct LayerAct {
     float *n1, *inv1, *qkv, *qk, *o, *lse, *x1, *inv2, *n2, *r, *h, *x2;
 };
 
+// The forward of a (batch, length) as a graph.  Sampling sends a prefix one token longer on every call, so lengths are
+// padded to a multiple of FWD_PAD: with a causal mask the rows behind a sequence's end change nothing in front of it.
+constexpr int FWD_PAD = 32;
+constexpr int FWD_GRAPHS = 8;
+struct FwdGraph {
+    int B, T;                    // B = 0: empty
+    bool ran;                    // has run eagerly once: the next call of this shape captures
+    cudaGraphExec_t exec;
+    unsigned long long last_use;
+};
+
 size_t align64(size_t n) { return (n + 63) / 64 * 64; }     // floats: 256-byte boundaries
 
 }  // namespace
@@ -75,6 +86,10 @@ struct deers_gpt {
     cudaGraphExec_t graph_exec;
     int graph_B, graph_T;
     int eager_steps_BT;          // eager steps run at (graph_B, graph_T) before capturing
+    // CUDA graphs of the forward alone, one per (B, padded T); the least recently used goes first
+    FwdGraph fwd_graph[FWD_GRAPHS];
+    unsigned long long fwd_clock;
+    bool head_pair_current;      // w_hi / w_lo hold the present head weight
 };
 
 namespace {
@@ -163,14 +178,16 @@ void rope_desc(const deers_gpt* m, int B, int T, int inverse, deers_rope_desc* d
     }
 }
 
-int forward(deers_gpt* m, const long long* ids, int B, int T) {
+// with_head_pair: the head weight's f16 pair is made here (a training step changes the weight every time); otherwise the
+// caller has it current.
+int forward(deers_gpt* m, const long long* ids, int B, int T, bool with_head_pair) {
     deers_ctx* ctx = m->ctx;
     const deers_gpt_config& c = m->cfg;
     const int C = c.n_embd, Hm = c.mlp_hidden_dim, V = c.vocab_size, H = c.n_head, D = m->D;
     const long long N = (long long)B * T;
     float* W = m->arena[0];
     for (bool& v : m->done_valid) v = false;
-    if (m->tc_head) {
+    if (m->tc_head && with_head_pair) {
         // the head weight's f16 pair (it changes every step) is made beside the blocks, not in front of the head
         SideScope side(m);
         GPT_TRY(side.rc);
@@ -336,7 +353,7 @@ int run_fwd_bwd(deers_gpt* m, int B, int T, bool with_norm) {
         // the shape has run eagerly once (every kernel's attributes are set): capture it
         cudaGraph_t graph = nullptr;
         if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            int rc = forward(m, m->ids_dev, B, T);
+            int rc = forward(m, m->ids_dev, B, T, true);
             if (!rc) rc = loss_and_backward(m, m->ids_dev, m->tgt_dev, B, T);
             if (!rc) rc = grad_norm(m);
             const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
@@ -357,10 +374,82 @@ int run_fwd_bwd(deers_gpt* m, int B, int T, bool with_norm) {
             m->graph_enabled = false;
         }
     }
-    GPT_TRY(forward(m, m->ids_dev, B, T));
+    GPT_TRY(forward(m, m->ids_dev, B, T, true));
     GPT_TRY(loss_and_backward(m, m->ids_dev, m->tgt_dev, B, T));
     if (with_norm) GPT_TRY(grad_norm(m));
     if (can_graph) m->eager_steps_BT += 1;
+    return DEERS_OK;
+}
+
+// ids [B, T] -> ids_dev [B, Tp], zeros behind each row's end
+__global__ void __launch_bounds__(256) pad_ids_kernel(const long long* __restrict__ src, long long* __restrict__ dst, int T, int Tp, int n) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n) dst[i] = i % Tp < T ? src[(long long)(i / Tp) * T + i % Tp] : 0;
+}
+
+// logits [B, Tp, ld] -> out [B, T, V]; blockIdx.y is a row of out.  Rows of an odd V start on any 4-byte boundary.
+__global__ void __launch_bounds__(256) copy_logits_kernel(const float* __restrict__ src, long long ld, float* __restrict__ dst, int T, int Tp, int V) {
+    const int row = blockIdx.y;
+    const float* s = src + ((long long)(row / T) * Tp + row % T) * ld;
+    float* d = dst + (long long)row * V;
+    for (int c = blockIdx.x * 1024 + threadIdx.x; c < V; c += gridDim.x * 1024) {
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = c + 256 * e < V ? __ldcs(s + c + 256 * e) : 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (c + 256 * e < V) __stcs(d + c + 256 * e, v[e]);
+    }
+}
+
+void drop_fwd_graphs(deers_gpt* m) {
+    for (FwdGraph& g : m->fwd_graph) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g = FwdGraph{};
+    }
+}
+
+// The forward on the ids staged as [B, T]: eagerly the first time a shape is seen, captured the second time, replayed
+// afterwards.
+int run_forward(deers_gpt* m, int B, int T) {
+    deers_ctx* ctx = m->ctx;
+    if (m->tc_head && !m->head_pair_current) {
+        GPT_TRY(launch_split_f16x3(ctx, m->cfg.n_embd, m->cfg.vocab_size, m->arena[0] + m->off_lm, m->Vld, 1.0f, m->w_hi, m->w_lo, m->Vld));
+        m->head_pair_current = true;
+    }
+    if (!m->graph_enabled || ctx->timing) return forward(m, m->ids_dev, B, T, false);
+    FwdGraph* slot = &m->fwd_graph[0];
+    for (FwdGraph& g : m->fwd_graph) {
+        if (g.B == B && g.T == T) { slot = &g; break; }
+        if (g.last_use < slot->last_use) slot = &g;
+    }
+    if (slot->B != B || slot->T != T) {
+        if (slot->exec) cudaGraphExecDestroy(slot->exec);
+        *slot = FwdGraph{};
+        slot->B = B; slot->T = T;
+    }
+    slot->last_use = ++m->fwd_clock;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool free_stream = ctx->stream != cudaStreamLegacy && cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess &&
+                             cap == cudaStreamCaptureStatusNone;
+    if (!slot->exec && slot->ran && free_stream) {
+        cudaGraph_t graph = nullptr;
+        if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+            const int rc = forward(m, m->ids_dev, B, T, false);
+            const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
+            if (rc || ce != cudaSuccess || !graph || cudaGraphInstantiate(&slot->exec, graph, 0) != cudaSuccess) slot->exec = nullptr;
+            if (graph) cudaGraphDestroy(graph);
+            if (rc) return rc;
+        }
+        if (!slot->exec) cudaGetLastError();                          // stays eager
+    }
+    if (slot->exec) {
+        DEERS_CUDA_TRY(ctx, cudaGraphLaunch(slot->exec, ctx->stream));
+        ctx->launches += 1;
+        return DEERS_OK;
+    }
+    GPT_TRY(forward(m, m->ids_dev, B, T, false));
+    slot->ran = free_stream;
     return DEERS_OK;
 }
 
@@ -409,6 +498,8 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
     m->tc_head = cfg->vocab_size >= 1024 && cfg->n_embd % 8 == 0 && cfg->n_embd >= 64;
     m->graph_enabled = true; m->graph_exec = nullptr; m->graph_B = m->graph_T = -1; m->eager_steps_BT = 0;
     m->on_side = false;
+    m->head_pair_current = false; m->fwd_clock = 0;
+    for (FwdGraph& g : m->fwd_graph) g = FwdGraph{};
     {
         // the weight-gradient stream and its markers; without them the step simply runs on one stream
         bool ok = cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking) == cudaSuccess;
@@ -532,6 +623,7 @@ extern "C" void deers_b200_gpt_destroy(deers_gpt* m) {
     cudaSetDevice(m->ctx->device);
     cudaStreamSynchronize(m->ctx->stream);
     drop_graph(m);
+    drop_fwd_graphs(m);
     if (m->side) { cudaStreamSynchronize(m->side); cudaStreamDestroy(m->side); }
     {
         cudaEvent_t evs[6] = {m->ev_fork, m->ev_join, m->ev_done[0], m->ev_done[1], m->ev_done[2], m->ev_done[3]};
@@ -570,6 +662,7 @@ extern "C" int deers_b200_gpt_param_set(deers_gpt* m, int index, int what, const
     float* p;
     long long r, c, ld;
     GPT_TRY(locate(m, index, what, &p, &r, &c, &ld));
+    m->head_pair_current = false;
     deers_ctx* ctx = m->ctx;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     DEERS_CUDA_TRY(ctx, cudaMemcpy2DAsync(p, (size_t)ld * sizeof(float), host, (size_t)c * sizeof(float),
@@ -594,7 +687,7 @@ extern "C" int deers_b200_gpt_param_get(deers_gpt* m, int index, int what, float
 extern "C" int deers_b200_gpt_set_graph(deers_gpt* m, int enable) {
     if (!m) return DEERS_ERR_NULL;
     m->graph_enabled = enable != 0;
-    if (!enable) { drop_graph(m); m->graph_B = m->graph_T = -1; }
+    if (!enable) { drop_fwd_graphs(m); drop_graph(m); m->graph_B = m->graph_T = -1; }
     return DEERS_OK;
 }
 
@@ -605,13 +698,19 @@ extern "C" int deers_b200_gpt_forward(deers_gpt* m, const int64_t* ids, int32_t 
     GPT_TRY(check_bt(m, B, T));
     deers_ctx* ctx = m->ctx;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    const long long N = (long long)B * T;
-    GPT_TRY(stage_ids(m, ids, nullptr, N, cudaMemcpyDeviceToDevice));
-    GPT_TRY(forward(m, m->ids_dev, B, T));
-    if (logits)
-        DEERS_CUDA_TRY(ctx, cudaMemcpy2DAsync(logits, (size_t)m->cfg.vocab_size * sizeof(float), m->logits,
-                                              (size_t)m->Vld * sizeof(float), (size_t)m->cfg.vocab_size * sizeof(float),
-                                              (size_t)N, cudaMemcpyDeviceToDevice, ctx->stream));
+    int Tp = (T + FWD_PAD - 1) / FWD_PAD * FWD_PAD;
+    if (Tp > m->cfg.sequence_len) Tp = m->cfg.sequence_len;           // the rotary cache and the buffers end there
+    const int n = B * Tp;
+    pad_ids_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>((const long long*)ids, m->ids_dev, T, Tp, n);
+    ctx->launches += 1;
+    GPT_TRY(run_forward(m, B, Tp));
+    if (logits) {
+        const int V = m->cfg.vocab_size;
+        const dim3 grid((unsigned)((V + 4095) / 4096), (unsigned)(B * T));
+        copy_logits_kernel<<<grid, 256, 0, ctx->stream>>>(m->logits, m->Vld, logits, T, Tp, V);
+        ctx->launches += 1;
+    }
+    DEERS_CUDA_TRY(ctx, cudaGetLastError());
     return DEERS_OK;
 }
 
@@ -623,6 +722,7 @@ extern "C" int deers_b200_gpt_forward_backward(deers_gpt* m, const int64_t* ids,
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     GPT_TRY(stage_ids(m, ids, targets, (long long)B * T, cudaMemcpyDeviceToDevice));
     GPT_TRY(run_fwd_bwd(m, B, T, false));
+    m->head_pair_current = m->tc_head;
     if (loss_dev)
         DEERS_CUDA_TRY(ctx, cudaMemcpyAsync(loss_dev, m->loss_dev, sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
     return DEERS_OK;
@@ -630,6 +730,7 @@ extern "C" int deers_b200_gpt_forward_backward(deers_gpt* m, const int64_t* ids,
 
 static int train_step_common(deers_gpt* m, int B, int T, const deers_adamw_hyper* hyper, double max_grad_norm) {
     GPT_TRY(run_fwd_bwd(m, B, T, true));
+    m->head_pair_current = false;                                     // the update below changes the head weight
     // clip_grad_norm + step_with_grads; "if grad_norm.is_finite() { step }" of tinystories_train.rs:213-216
     return launch_adamw(m->ctx, (int)m->opt.size(), m->opt.data(), hyper, m->norm_dev, max_grad_norm, true);
 }

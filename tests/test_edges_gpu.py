@@ -91,3 +91,35 @@ def test_f32_attention_tiles_and_groups(T, D, causal):
             assert np.abs(g - w).max() <= 4 * D * 2.0 ** -24 * sums * D ** -0.5 * other, name
         else:
             assert_close(g, w, TOL_F32, f"T {T} D {D} {name}")
+
+
+def test_gpt_forward_lengths_share_graphs_and_follow_the_weights():
+    """Lengths are padded to shared graphs (eager, captured, replayed): every length must give what the oracle gives,
+    before and after an optimizer step and after a weight upload (the head's f16 pair is kept between calls)."""
+    from deers_b200 import gpt
+    from oracle import ref
+    V, L, H, C, Hm, Tmax, B = 1030, 2, 2, 64, 128, 70, 2
+    cfg = (V, L, H, C, Hm)
+    params = ref.gpt_init_params(cfg, seed=3)
+    m = gpt.GPT(gpt.GPTConfig(V, Tmax, L, H, C, Hm), torch.device("cuda", torch.cuda.current_device()), B)
+    m.load_parameters(params)
+    rng = np.random.default_rng(4)
+    ids = rng.integers(0, V, (B, Tmax))
+
+    def check(T, b=B):
+        got = m.forward(torch.from_numpy(ids[:b, :T].copy()).cuda())
+        m.ctx.sync()
+        want = ref.gpt_step(cfg, params, ids[:b, :T], want_grads=False)["logits"]
+        # f32 sums of up to 1030 terms through two layers against the oracle's left-to-right sums
+        assert_close(got.cpu().numpy().reshape(np.asarray(want).shape), want, 1e-4, f"T {T}")
+    for T in (31, 32, 30, 33, 1, 33, 64, 40, 65, 70, 66, 69, 31, 5):
+        check(T)
+    check(50, 1), check(51, 1), check(52, 1)
+    tgt = torch.from_numpy(rng.integers(0, V, (B, 20))).cuda()
+    m.train_step(torch.from_numpy(ids[:, :20].copy()).cuda(), tgt, lr=1e-2)
+    m.ctx.sync()
+    params = [m.parameter(i) for i in range(m.num_parameters())]
+    check(40), check(41)
+    params = ref.gpt_init_params(cfg, seed=5)
+    m.load_parameters(params)
+    check(42), check(31)
