@@ -175,7 +175,7 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     volatile uint32_t* abort_s = tmem_base_s + 1;
     uint32_t* skip_s = tmem_base_s + 2;
 
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = uniform((int)threadIdx.x / 32), lane = threadIdx.x % 32;
     const int nq = (p.T + BT - 1) / BT;
     const int n_items = p.B * p.H * nq;
 
@@ -212,7 +212,7 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_base_s;
+    const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 
     if (warp == 0) {
@@ -252,29 +252,36 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        // The whole warp runs this; one elected lane issues (see elect_one).
+        {
             constexpr uint32_t IDESC_ST = idesc_f16(128, 128, 0, 0);   // S^T, dP^T: K-major A and B
             constexpr uint32_t IDESC_KV = idesc_f16(128, D, 0, 1);     // dV, dK: A from TMEM, MN-major B
             // Step-0 descriptors of every operand view, built once; each MMA adds a constant
             // (a single thread issues, so descriptor arithmetic must stay off the issue path).
             constexpr uint64_t STAGE_STEP = TILE_BYTES >> 4;           // next stage of Q / dO
-            const uint64_t k_km = desc_kmajor(smem_u32(sK), 0, BLOCK_BYTES);
-            const uint64_t v_km = desc_kmajor(smem_u32(sV), 0, BLOCK_BYTES);
-            const uint64_t q_km0 = desc_kmajor(smem_u32(sQ), 0, BLOCK_BYTES), q_mn0 = desc_mnmajor(smem_u32(sQ), 0, BLOCK_BYTES);
-            const uint64_t do_km0 = desc_kmajor(smem_u32(sDO), 0, BLOCK_BYTES), do_mn0 = desc_mnmajor(smem_u32(sDO), 0, BLOCK_BYTES);
+            const uint64_t k_km = desc_kmajor((uint32_t)uniform((int)smem_u32(sK)), 0, BLOCK_BYTES);
+            const uint64_t v_km = desc_kmajor((uint32_t)uniform((int)smem_u32(sV)), 0, BLOCK_BYTES);
+            const uint64_t q_km0 = desc_kmajor((uint32_t)uniform((int)smem_u32(sQ)), 0, BLOCK_BYTES), q_mn0 = desc_mnmajor((uint32_t)uniform((int)smem_u32(sQ)), 0, BLOCK_BYTES);
+            const uint64_t do_km0 = desc_kmajor((uint32_t)uniform((int)smem_u32(sDO)), 0, BLOCK_BYTES), do_mn0 = desc_mnmajor((uint32_t)uniform((int)smem_u32(sDO)), 0, BLOCK_BYTES);
             auto issue_st = [&](uint32_t qs) {
                 const uint64_t q_km = q_km0 + (uint64_t)qs * STAGE_STEP;
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks)
-                    umma_ss(tmem + TM_S, k_km + kmajor_step(ks, BLOCK_BYTES), q_km + kmajor_step(ks, BLOCK_BYTES), IDESC_ST, ks > 0);
-                umma_commit(&bars[A_S]);
+                    for (int ks = 0; ks < D / 16; ++ks)
+                        umma_ss(tmem + TM_S, k_km + kmajor_step(ks, BLOCK_BYTES), q_km + kmajor_step(ks, BLOCK_BYTES), IDESC_ST, ks > 0);
+                    umma_commit(&bars[A_S]);
+                }
+                __syncwarp();
             };
             auto issue_dpt = [&](uint32_t ds) {
                 const uint64_t do_km = do_km0 + (uint64_t)ds * STAGE_STEP;
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks)
-                    umma_ss(tmem + TM_DP, v_km + kmajor_step(ks, BLOCK_BYTES), do_km + kmajor_step(ks, BLOCK_BYTES), IDESC_ST, ks > 0);
-                umma_commit(&bars[A_DP]);
+                    for (int ks = 0; ks < D / 16; ++ks)
+                        umma_ss(tmem + TM_DP, v_km + kmajor_step(ks, BLOCK_BYTES), do_km + kmajor_step(ks, BLOCK_BYTES), IDESC_ST, ks > 0);
+                    umma_commit(&bars[A_DP]);
+                }
+                __syncwarp();
             };
             // A operand in TMEM: CW / 2 packed columns per compute warpgroup, the groups CW columns apart.
             auto a_tmem = [&](uint32_t base, int ks) {
@@ -282,53 +289,59 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             };
             uint32_t gi = 0;
             bool ok = true;
-            for (int4 cur = next_item(p, 0, n_items, nq), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); ok && cur.x >= 0;
-                     ++n4.x, cur = nxt, nxt = next_item(p, n4.x + 1, n_items, nq)) {
+            for (int4 cur = uniform(next_item(p, 0, n_items, nq)), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); ok && cur.x >= 0;
+                     ++n4.x, cur = uniform(nxt), nxt = next_item(p, n4.x + 1, n_items, nq)) {
                 const int n = n4.x, kt = cur.x, bh = cur.y;
                 const int niter = nq - (p.causal ? kt : 0);
-                if (!mbar_wait(ws, &bars[A_KV_FULL], (uint32_t)n & 1u, DEERS_KERR_BWD_F16 | 5)) break;
-                if (!mbar_wait(ws, &bars[A_Q_FULL + gi % 3u], (gi / 3u) & 1u, DEERS_KERR_BWD_F16 | 6)) break;
-                if (!mbar_wait(ws, &bars[A_DO_FULL + (gi & 1u)], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 7)) break;
+                if (!mbar_wait_warp(ws, &bars[A_KV_FULL], (uint32_t)n & 1u, DEERS_KERR_BWD_F16 | 5)) break;
+                if (!mbar_wait_warp(ws, &bars[A_Q_FULL + gi % 3u], (gi / 3u) & 1u, DEERS_KERR_BWD_F16 | 6)) break;
+                if (!mbar_wait_warp(ws, &bars[A_DO_FULL + (gi & 1u)], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 7)) break;
                 tc_fence_after_sync();
                 issue_st(gi % 3u);
                 issue_dpt(gi & 1u);
-                if (niter == 1) umma_commit(&bars[A_KV_EMPTY]);         // no further product reads K / V
+                if (niter == 1 && elect_one()) umma_commit(&bars[A_KV_EMPTY]);         // no further product reads K / V
                 for (int it = 0; it < niter; ++it, ++gi) {
                     const uint32_t qs = gi % 3u, ds = gi & 1u, par = gi & 1u;
                     const uint64_t q_mn = q_mn0 + (uint64_t)qs * STAGE_STEP, do_mn = do_mn0 + (uint64_t)ds * STAGE_STEP;
                     const bool more = it + 1 < niter;
                     // dV += P^T dO, then S^T of the next query tile: the pipe is in order, so the
                     // new S^T lands only after dV has consumed P^T from the same columns.
-                    if (!mbar_wait(ws, &bars[A_P], par, DEERS_KERR_BWD_F16 | 8)) { ok = false; break; }
+                    if (!mbar_wait_warp(ws, &bars[A_P], par, DEERS_KERR_BWD_F16 | 8)) { ok = false; break; }
                     // The previous item's dK / dV must have left TMEM before this item accumulates.
-                    if (it == 0 && !mbar_wait(ws, &bars[A_ACC_FREE], ((uint32_t)n & 1u) ^ 1u, DEERS_KERR_BWD_F16 | 9)) { ok = false; break; }
+                    if (it == 0 && !mbar_wait_warp(ws, &bars[A_ACC_FREE], ((uint32_t)n & 1u) ^ 1u, DEERS_KERR_BWD_F16 | 9)) { ok = false; break; }
                     tc_fence_after_sync();
+                    if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < BT / 16; ++ks)
-                        umma_ts(tmem + TM_DV, a_tmem(TM_S, ks), do_mn + mnmajor_step(ks), IDESC_KV, (it > 0 || ks > 0));
+                        for (int ks = 0; ks < BT / 16; ++ks)
+                            umma_ts(tmem + TM_DV, a_tmem(TM_S, ks), do_mn + mnmajor_step(ks), IDESC_KV, (it > 0 || ks > 0));
+                    }
+                    __syncwarp();
                     if (more) {
-                        if (!mbar_wait(ws, &bars[A_Q_FULL + (gi + 1u) % 3u], ((gi + 1u) / 3u) & 1u, DEERS_KERR_BWD_F16 | 10)) { ok = false; break; }
+                        if (!mbar_wait_warp(ws, &bars[A_Q_FULL + (gi + 1u) % 3u], ((gi + 1u) / 3u) & 1u, DEERS_KERR_BWD_F16 | 10)) { ok = false; break; }
                         tc_fence_after_sync();
                         issue_st((gi + 1u) % 3u);
                     }
                     // dK += dS^T Q, then dP^T of the next query tile over the consumed dS^T columns.
-                    if (!mbar_wait(ws, &bars[A_DS], par, DEERS_KERR_BWD_F16 | 11)) { ok = false; break; }
+                    if (!mbar_wait_warp(ws, &bars[A_DS], par, DEERS_KERR_BWD_F16 | 11)) { ok = false; break; }
                     tc_fence_after_sync();
+                    if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < BT / 16; ++ks)
-                        umma_ts(tmem + TM_DK, a_tmem(TM_DP, ks), q_mn + mnmajor_step(ks), IDESC_KV, (it > 0 || ks > 0));
-                    umma_commit(&bars[A_Q_EMPTY + qs]);                 // S^T and dK have both read this Q tile
+                        for (int ks = 0; ks < BT / 16; ++ks)
+                            umma_ts(tmem + TM_DK, a_tmem(TM_DP, ks), q_mn + mnmajor_step(ks), IDESC_KV, (it > 0 || ks > 0));
+                        umma_commit(&bars[A_Q_EMPTY + qs]);                 // S^T and dK have both read this Q tile
+                    }
+                    __syncwarp();
                     if (more) {
-                        if (!mbar_wait(ws, &bars[A_DO_FULL + (ds ^ 1u)], ((gi + 1u) >> 1) & 1u, DEERS_KERR_BWD_F16 | 12)) { ok = false; break; }
+                        if (!mbar_wait_warp(ws, &bars[A_DO_FULL + (ds ^ 1u)], ((gi + 1u) >> 1) & 1u, DEERS_KERR_BWD_F16 | 12)) { ok = false; break; }
                         tc_fence_after_sync();
                         issue_dpt(ds ^ 1u);
-                        if (it + 2 == niter) umma_commit(&bars[A_KV_EMPTY]);   // the last S^T and dP^T are issued
+                        if (it + 2 == niter && elect_one()) umma_commit(&bars[A_KV_EMPTY]);   // the last S^T and dP^T are issued
                     }
                     // dO of this iteration was last read by dV (and dP^T before it): its stage is free once
                     // everything issued so far has finished.
-                    umma_commit(&bars[A_DO_EMPTY + ds]);
+                    if (elect_one()) umma_commit(&bars[A_DO_EMPTY + ds]);
                 }
-                umma_commit(&bars[A_DONE]);
+                if (elect_one()) umma_commit(&bars[A_DONE]);
             }
         }
     } else {
@@ -545,7 +558,7 @@ attn_bwd_dq_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     volatile uint32_t* abort_s = tmem_base_s + 1;
     uint32_t* skip_s = tmem_base_s + 2;
 
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = uniform((int)threadIdx.x / 32), lane = threadIdx.x % 32;
     const int nq = (p.T + BT - 1) / BT;
     const int n_items = p.B * p.H * nq;
 
@@ -580,7 +593,7 @@ attn_bwd_dq_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_base_s;
+    const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 
     if (warp == 0) {
@@ -619,41 +632,48 @@ attn_bwd_dq_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        // The whole warp runs this; one elected lane issues (see elect_one).
+        {
             constexpr uint32_t IDESC_S = idesc_f16(128, 128, 0, 0);    // S, dP: K-major A and B
             constexpr uint32_t IDESC_DQ = idesc_f16(128, D, 0, 1);     // dQ: A from TMEM, MN-major B
             constexpr uint64_t STAGE_STEP = TILE_BYTES >> 4;
-            const uint64_t q_km = desc_kmajor(smem_u32(sQ), 0, BLOCK_BYTES), do_km = desc_kmajor(smem_u32(sDO), 0, BLOCK_BYTES);
-            const uint64_t k_km0 = desc_kmajor(smem_u32(sK), 0, BLOCK_BYTES), k_mn0 = desc_mnmajor(smem_u32(sK), 0, BLOCK_BYTES);
-            const uint64_t v_km0 = desc_kmajor(smem_u32(sV), 0, BLOCK_BYTES);
+            const uint64_t q_km = desc_kmajor((uint32_t)uniform((int)smem_u32(sQ)), 0, BLOCK_BYTES), do_km = desc_kmajor((uint32_t)uniform((int)smem_u32(sDO)), 0, BLOCK_BYTES);
+            const uint64_t k_km0 = desc_kmajor((uint32_t)uniform((int)smem_u32(sK)), 0, BLOCK_BYTES), k_mn0 = desc_mnmajor((uint32_t)uniform((int)smem_u32(sK)), 0, BLOCK_BYTES);
+            const uint64_t v_km0 = desc_kmajor((uint32_t)uniform((int)smem_u32(sV)), 0, BLOCK_BYTES);
             auto issue_s = [&](uint32_t st) {
                 const uint64_t k_km = k_km0 + (uint64_t)st * STAGE_STEP;
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks)
-                    umma_ss(tmem + TM_S, q_km + kmajor_step(ks, BLOCK_BYTES), k_km + kmajor_step(ks, BLOCK_BYTES), IDESC_S, ks > 0);
-                umma_commit(&bars[Q_S]);
+                    for (int ks = 0; ks < D / 16; ++ks)
+                        umma_ss(tmem + TM_S, q_km + kmajor_step(ks, BLOCK_BYTES), k_km + kmajor_step(ks, BLOCK_BYTES), IDESC_S, ks > 0);
+                    umma_commit(&bars[Q_S]);
+                }
+                __syncwarp();
             };
             // The V stage and the dP buffer both alternate with the parity of the KV step.
             auto issue_dp = [&](uint32_t st) {
                 const uint64_t v_km = v_km0 + (uint64_t)st * STAGE_STEP;
                 const uint32_t tm_dp = tmem + TM_DP + st * 128u;
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks)
-                    umma_ss(tm_dp, do_km + kmajor_step(ks, BLOCK_BYTES), v_km + kmajor_step(ks, BLOCK_BYTES), IDESC_S, ks > 0);
-                umma_commit(&bars[Q_DP + st]);
-                umma_commit(&bars[Q_V_EMPTY + st]);                    // dP is the only reader of a V tile
+                    for (int ks = 0; ks < D / 16; ++ks)
+                        umma_ss(tm_dp, do_km + kmajor_step(ks, BLOCK_BYTES), v_km + kmajor_step(ks, BLOCK_BYTES), IDESC_S, ks > 0);
+                    umma_commit(&bars[Q_DP + st]);
+                    umma_commit(&bars[Q_V_EMPTY + st]);                    // dP is the only reader of a V tile
+                }
+                __syncwarp();
             };
             uint32_t kvc = 0;                                   // K/V stage uses == KV iterations so far
             bool ok = true;
-            for (int4 cur = next_item(p, 0, n_items, nq), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); ok && cur.x >= 0;
-                     ++n4.x, cur = nxt, nxt = next_item(p, n4.x + 1, n_items, nq)) {
+            for (int4 cur = uniform(next_item(p, 0, n_items, nq)), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); ok && cur.x >= 0;
+                     ++n4.x, cur = uniform(nxt), nxt = next_item(p, n4.x + 1, n_items, nq)) {
                 const int n = n4.x, slot = cur.x, bh = cur.y;
                 const int qt = nq - 1 - slot;
                 const int ntiles = p.causal ? qt + 1 : nq;
                 const uint32_t tm_dq = tmem + TM_DQ;
-                if (!mbar_wait(ws, &bars[Q_QDO_FULL], (uint32_t)n & 1u, DEERS_KERR_BWD_F16 | 0x12)) break;
-                if (!mbar_wait(ws, &bars[Q_K_FULL + kvc % 3u], (kvc / 3u) & 1u, DEERS_KERR_BWD_F16 | 0x13)) break;
-                if (!mbar_wait(ws, &bars[Q_V_FULL + (kvc & 1u)], (kvc >> 1) & 1u, DEERS_KERR_BWD_F16 | 0x1c)) break;
+                if (!mbar_wait_warp(ws, &bars[Q_QDO_FULL], (uint32_t)n & 1u, DEERS_KERR_BWD_F16 | 0x12)) break;
+                if (!mbar_wait_warp(ws, &bars[Q_K_FULL + kvc % 3u], (kvc / 3u) & 1u, DEERS_KERR_BWD_F16 | 0x13)) break;
+                if (!mbar_wait_warp(ws, &bars[Q_V_FULL + (kvc & 1u)], (kvc >> 1) & 1u, DEERS_KERR_BWD_F16 | 0x1c)) break;
                 tc_fence_after_sync();
                 issue_s(kvc % 3u);
                 issue_dp(kvc & 1u);
@@ -664,31 +684,34 @@ attn_bwd_dq_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                     // S and dP of the next KV tile as soon as the compute threads have read this S:
                     // dP lands in the buffer whose dS the product issued one step ago has consumed
                     // (the pipe is in order), so the tensor core never waits for this step's dS.
-                    if (!mbar_wait(ws, &bars[Q_PDONE], par, DEERS_KERR_BWD_F16 | 0x14)) { ok = false; break; }
+                    if (!mbar_wait_warp(ws, &bars[Q_PDONE], par, DEERS_KERR_BWD_F16 | 0x14)) { ok = false; break; }
                     if (more) {
-                        if (!mbar_wait(ws, &bars[Q_K_FULL + ksn], ((kvc + 1u) / 3u) & 1u, DEERS_KERR_BWD_F16 | 0x15)) { ok = false; break; }
+                        if (!mbar_wait_warp(ws, &bars[Q_K_FULL + ksn], ((kvc + 1u) / 3u) & 1u, DEERS_KERR_BWD_F16 | 0x15)) { ok = false; break; }
                         tc_fence_after_sync();
                         issue_s(ksn);
-                        if (!mbar_wait(ws, &bars[Q_V_FULL + vsn], ((kvc + 1u) >> 1) & 1u, DEERS_KERR_BWD_F16 | 0x1d)) { ok = false; break; }
+                        if (!mbar_wait_warp(ws, &bars[Q_V_FULL + vsn], ((kvc + 1u) >> 1) & 1u, DEERS_KERR_BWD_F16 | 0x1d)) { ok = false; break; }
                         tc_fence_after_sync();
                         issue_dp(vsn);
                     } else {
-                        umma_commit(&bars[Q_QDO_EMPTY]);               // every product reading Q / dO has been issued
+                        if (elect_one()) umma_commit(&bars[Q_QDO_EMPTY]);               // every product reading Q / dO has been issued
                     }
                     // dQ += dS K
-                    if (!mbar_wait(ws, &bars[Q_DS + par], (kvc >> 1) & 1u, DEERS_KERR_BWD_F16 | 0x16)) { ok = false; break; }
+                    if (!mbar_wait_warp(ws, &bars[Q_DS + par], (kvc >> 1) & 1u, DEERS_KERR_BWD_F16 | 0x16)) { ok = false; break; }
                     // The previous item's dQ must have left TMEM before this item accumulates.
-                    if (j == 0 && n > 0 && !mbar_wait(ws, &bars[Q_DQ_FREE], ((uint32_t)n - 1u) & 1u, DEERS_KERR_BWD_F16 | 0x1a)) { ok = false; break; }
+                    if (j == 0 && n > 0 && !mbar_wait_warp(ws, &bars[Q_DQ_FREE], ((uint32_t)n - 1u) & 1u, DEERS_KERR_BWD_F16 | 0x1a)) { ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t k_mn = k_mn0 + (uint64_t)ks * STAGE_STEP;
                     const uint32_t tm_ds = tmem + TM_DP + par * 128u;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < BT / 16; ++ks)
-                        umma_ts(tm_dq, tm_ds + (uint32_t)(ks >> 2) * 64u + (uint32_t)(ks & 3) * 8u,
-                                k_mn + mnmajor_step(ks), IDESC_DQ, (j > 0 || ks > 0));
-                    umma_commit(&bars[Q_K_EMPTY + ks]);                // S and dQ have both read this K tile
+                        for (int ks = 0; ks < BT / 16; ++ks)
+                            umma_ts(tm_dq, tm_ds + (uint32_t)(ks >> 2) * 64u + (uint32_t)(ks & 3) * 8u,
+                                    k_mn + mnmajor_step(ks), IDESC_DQ, (j > 0 || ks > 0));
+                        umma_commit(&bars[Q_K_EMPTY + ks]);                // S and dQ have both read this K tile
+                    }
+                    __syncwarp();
                 }
-                umma_commit(&bars[Q_DONE]);
+                if (elect_one()) umma_commit(&bars[Q_DONE]);
             }
         }
     } else {
@@ -843,7 +866,7 @@ attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const
     volatile uint32_t* abort_s = tmem_base_s + 1;
     uint32_t* skip_s = tmem_base_s + 2;
 
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = uniform((int)threadIdx.x / 32), lane = threadIdx.x % 32;
     const int nq = (p.T + BT - 1) / BT;
     const int n_items = p.B * p.H * nq;
 
@@ -869,7 +892,7 @@ attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_base_s;
+    const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 
     if (warp == 0) {
@@ -900,30 +923,34 @@ attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        // The whole warp runs this; one elected lane issues (see elect_one).
+        {
             constexpr uint32_t IDESC = idesc_f16(128, D, 1, 1);        // both operands MN-major
             constexpr uint64_t STAGE_STEP = L::STAGE >> 4;
-            const uint64_t a0 = desc_mnmajor(smem_u32(smem), 0, BLOCK_BYTES);
-            const uint64_t b0 = desc_mnmajor(smem_u32(smem + L::DS), 0, BLOCK_BYTES);
+            const uint64_t a0 = desc_mnmajor((uint32_t)uniform((int)smem_u32(smem)), 0, BLOCK_BYTES);
+            const uint64_t b0 = desc_mnmajor((uint32_t)uniform((int)smem_u32(smem + L::DS)), 0, BLOCK_BYTES);
             uint32_t gi = 0;
             bool ok = true;
-            for (int4 cur = next_item(p, 0, n_items, nq), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); ok && cur.x >= 0;
-                     ++n4.x, cur = nxt, nxt = next_item(p, n4.x + 1, n_items, nq)) {
+            for (int4 cur = uniform(next_item(p, 0, n_items, nq)), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); ok && cur.x >= 0;
+                     ++n4.x, cur = uniform(nxt), nxt = next_item(p, n4.x + 1, n_items, nq)) {
                 const uint32_t n = (uint32_t)n4.x, buf = n & 1u;
                 const int qt = nq - 1 - cur.x;
                 const int ntiles = p.causal ? qt + 1 : nq;
-                if (!mbar_wait(ws, &bars[R_ACC_EMPTY + buf], ((n >> 1) & 1u) ^ 1u, DEERS_KERR_BWD_F16 | 0x31)) break;
+                if (!mbar_wait_warp(ws, &bars[R_ACC_EMPTY + buf], ((n >> 1) & 1u) ^ 1u, DEERS_KERR_BWD_F16 | 0x31)) break;
                 for (int j = 0; j < ntiles; ++j, ++gi) {
                     const uint32_t s = gi % (uint32_t)L::STAGES;
-                    if (!mbar_wait(ws, &bars[R_FULL + s], (gi / (uint32_t)L::STAGES) & 1u, DEERS_KERR_BWD_F16 | 0x32)) { ok = false; break; }
+                    if (!mbar_wait_warp(ws, &bars[R_FULL + s], (gi / (uint32_t)L::STAGES) & 1u, DEERS_KERR_BWD_F16 | 0x32)) { ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t a = a0 + (uint64_t)s * STAGE_STEP, bd = b0 + (uint64_t)s * STAGE_STEP;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < BT / 16; ++ks)
-                        umma_ss(tmem + buf * (uint32_t)D, a + mnmajor_step(ks), bd + mnmajor_step(ks), IDESC, (j > 0 || ks > 0));
-                    umma_commit(&bars[R_EMPTY + s]);
+                        for (int ks = 0; ks < BT / 16; ++ks)
+                            umma_ss(tmem + buf * (uint32_t)D, a + mnmajor_step(ks), bd + mnmajor_step(ks), IDESC, (j > 0 || ks > 0));
+                        umma_commit(&bars[R_EMPTY + s]);
+                    }
+                    __syncwarp();
                 }
-                if (ok) umma_commit(&bars[R_ACC_FULL + buf]);
+                if (ok && elect_one()) umma_commit(&bars[R_ACC_FULL + buf]);
             }
         }
     } else {

@@ -107,7 +107,7 @@ struct WorkCursor {
     // Item n becomes current; the table entry of item n+1 is requested now and not looked at before the
     // next call, so its L2 round trip is off the item boundary.
     __device__ __forceinline__ void fetch(const FwdParams& p, int nq, int n_items) {
-        const int4 e = e_next;
+        const int4 e = uniform(e_next);                     // every user runs as a whole warp
         e_next = table(p, n + 1, nq, n_items);
         w = e.x;
         if (e.x >= 0) {
@@ -153,7 +153,7 @@ attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     volatile uint32_t* abort_s = tmem_base_s + 1;
     uint32_t* skip_s = tmem_base_s + 2;
 
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = uniform((int)threadIdx.x / 32), lane = threadIdx.x % 32;
     const int nq = (p.T + BM - 1) / BM;
     const int n_items = p.B * p.H * nq;
 
@@ -187,89 +187,104 @@ attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_base_s;
+    const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
-        if (lane == 0) {
+        {
             WorkCursor c;
             c.init(p, nq, n_items);
             for (uint32_t g = 0; c.valid(n_items); ++g) {      // g: global step = K / V stage use
                 const int b = c.b, h = c.h;
                 if (c.j == 0) {
                     const int qb = c.n & 1;
-                    if (!mbar_wait(ws, &bars[F_Q_EMPTY + qb], (((uint32_t)c.n >> 1) & 1u) ^ 1u, DEERS_KERR_FWD_F16 | 1)) break;
-                    mbar_arrive_expect_tx(&bars[F_Q_FULL + qb], TILE_BYTES);
+                    if (!mbar_wait_warp(ws, &bars[F_Q_EMPTY + qb], (((uint32_t)c.n >> 1) & 1u) ^ 1u, DEERS_KERR_FWD_F16 | 1)) break;
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&bars[F_Q_FULL + qb], TILE_BYTES);
 #pragma unroll
-                    for (int blk = 0; blk < DBLK; ++blk)
-                        tma_load_4d(sQ + qb * TILE_BYTES + blk * BLOCK_BYTES, &tmap_q, &bars[F_Q_FULL + qb], blk * 64, c.qt * BM, h, b);
+                        for (int blk = 0; blk < DBLK; ++blk)
+                            tma_load_4d(sQ + qb * TILE_BYTES + blk * BLOCK_BYTES, &tmap_q, &bars[F_Q_FULL + qb], blk * 64, c.qt * BM, h, b);
+                    }
+                    __syncwarp();
                 }
                 const uint32_t st = g & 1u, ph = ((g >> 1) & 1u) ^ 1u;
-                if (!mbar_wait(ws, &bars[F_S_FULL + st], ph, DEERS_KERR_FWD_F16 | 2)) break;      // S of step g-2 done
-                mbar_arrive_expect_tx(&bars[F_K_FULL + st], TILE_BYTES);
+                if (!mbar_wait_warp(ws, &bars[F_S_FULL + st], ph, DEERS_KERR_FWD_F16 | 2)) break;      // S of step g-2 done
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&bars[F_K_FULL + st], TILE_BYTES);
 #pragma unroll
-                for (int blk = 0; blk < DBLK; ++blk)
-                    tma_load_4d(sK + st * TILE_BYTES + blk * BLOCK_BYTES, &tmap_k, &bars[F_K_FULL + st], blk * 64, c.j * BN, h, b);
-                if (!mbar_wait(ws, &bars[F_PV_DONE + st], ph, DEERS_KERR_FWD_F16 | 3)) break;     // P V of step g-2 done
-                mbar_arrive_expect_tx(&bars[F_V_FULL + st], TILE_BYTES);
+                    for (int blk = 0; blk < DBLK; ++blk)
+                        tma_load_4d(sK + st * TILE_BYTES + blk * BLOCK_BYTES, &tmap_k, &bars[F_K_FULL + st], blk * 64, c.j * BN, h, b);
+                }
+                __syncwarp();
+                if (!mbar_wait_warp(ws, &bars[F_PV_DONE + st], ph, DEERS_KERR_FWD_F16 | 3)) break;     // P V of step g-2 done
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&bars[F_V_FULL + st], TILE_BYTES);
 #pragma unroll
-                for (int blk = 0; blk < DBLK; ++blk)
-                    tma_load_4d(sV + st * TILE_BYTES + blk * BLOCK_BYTES, &tmap_v, &bars[F_V_FULL + st], blk * 64, c.j * BN, h, b);
+                    for (int blk = 0; blk < DBLK; ++blk)
+                        tma_load_4d(sV + st * TILE_BYTES + blk * BLOCK_BYTES, &tmap_v, &bars[F_V_FULL + st], blk * 64, c.j * BN, h, b);
+                }
+                __syncwarp();
                 c.advance(p, nq, n_items);
             }
         }
     } else if (warp == 1) {
         // ------------------------------ P V issuer ------------------------------
-        if (lane == 0) {
+        {
             constexpr uint32_t IDESC_O = idesc_f16(BM, D, 0, 1);       // O: A = P from TMEM, B = V MN-major
             constexpr uint64_t STAGE_STEP = TILE_BYTES >> 4;
-            const uint64_t v_mn0 = desc_mnmajor(smem_u32(sV), 0, BLOCK_BYTES);
+            const uint64_t v_mn0 = desc_mnmajor((uint32_t)uniform((int)smem_u32(sV)), 0, BLOCK_BYTES);
             WorkCursor pc;
             pc.init(p, nq, n_items);
             for (uint32_t gp = 0; pc.valid(n_items); ++gp) {
                 const uint32_t st = gp & 1u;
-                if (!mbar_wait(ws, &bars[F_P_FULL + st], (gp >> 1) & 1u, DEERS_KERR_FWD_F16 | 6)) break;
-                if (!mbar_wait(ws, &bars[F_V_FULL + st], (gp >> 1) & 1u, DEERS_KERR_FWD_F16 | 7)) break;
+                if (!mbar_wait_warp(ws, &bars[F_P_FULL + st], (gp >> 1) & 1u, DEERS_KERR_FWD_F16 | 6)) break;
+                if (!mbar_wait_warp(ws, &bars[F_V_FULL + st], (gp >> 1) & 1u, DEERS_KERR_FWD_F16 | 7)) break;
                 // The accumulator of item n was last used by item n-2: its epilogue must be over.
-                if (pc.j == 0 && !mbar_wait(ws, &bars[F_O_FREE + (pc.n & 1)], (((uint32_t)pc.n >> 1) & 1u) ^ 1u, DEERS_KERR_FWD_F16 | 8)) break;
+                if (pc.j == 0 && !mbar_wait_warp(ws, &bars[F_O_FREE + (pc.n & 1)], (((uint32_t)pc.n >> 1) & 1u) ^ 1u, DEERS_KERR_FWD_F16 | 8)) break;
                 tc_fence_after_sync();
                 const uint64_t v_mn = v_mn0 + (uint64_t)st * STAGE_STEP;
                 const uint32_t o_tmem = tmem + TM_O + (uint32_t)(pc.n & 1) * D;
                 const uint32_t p_tmem = tmem + TM_S + st * 128u;       // P sits where this step's S was
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < BN / 16; ++ks)
-                    umma_ts(o_tmem, p_tmem + (uint32_t)(ks / (CW / 16)) * CW + (uint32_t)(ks % (CW / 16)) * 8u, v_mn + mnmajor_step(ks),
-                            IDESC_O, (pc.j > 0 || ks > 0));
-                umma_commit(&bars[F_PV_DONE + st]);
-                if (pc.j == pc.ntiles - 1) umma_commit(&bars[F_O_DONE + (pc.n & 1)]);
+                    for (int ks = 0; ks < BN / 16; ++ks)
+                        umma_ts(o_tmem, p_tmem + (uint32_t)(ks / (CW / 16)) * CW + (uint32_t)(ks % (CW / 16)) * 8u, v_mn + mnmajor_step(ks),
+                                IDESC_O, (pc.j > 0 || ks > 0));
+                    umma_commit(&bars[F_PV_DONE + st]);
+                    if (pc.j == pc.ntiles - 1) umma_commit(&bars[F_O_DONE + (pc.n & 1)]);
+                }
+                __syncwarp();
                 pc.advance(p, nq, n_items);
             }
         }
     } else if (warp == S_WARP) {
         // ------------------------------ S issuer ------------------------------
-        if (lane == 0) {
+        {
             constexpr uint32_t IDESC_S = idesc_f16(BM, BN, 0, 0);      // S: K-major A (Q) and B (K)
             constexpr uint64_t STAGE_STEP = TILE_BYTES >> 4;
-            const uint64_t q_km0 = desc_kmajor(smem_u32(sQ), 0, BLOCK_BYTES);
-            const uint64_t k_km0 = desc_kmajor(smem_u32(sK), 0, BLOCK_BYTES);
+            const uint64_t q_km0 = desc_kmajor((uint32_t)uniform((int)smem_u32(sQ)), 0, BLOCK_BYTES);
+            const uint64_t k_km0 = desc_kmajor((uint32_t)uniform((int)smem_u32(sK)), 0, BLOCK_BYTES);
             WorkCursor sc;
             sc.init(p, nq, n_items);
             for (uint32_t gs = 0; sc.valid(n_items); ++gs) {
                 const uint32_t st = gs & 1u;
                 const int qb = sc.n & 1;
-                if (sc.j == 0 && !mbar_wait(ws, &bars[F_Q_FULL + qb], ((uint32_t)sc.n >> 1) & 1u, DEERS_KERR_FWD_F16 | 4)) break;
-                if (!mbar_wait(ws, &bars[F_K_FULL + st], (gs >> 1) & 1u, DEERS_KERR_FWD_F16 | 5)) break;
+                if (sc.j == 0 && !mbar_wait_warp(ws, &bars[F_Q_FULL + qb], ((uint32_t)sc.n >> 1) & 1u, DEERS_KERR_FWD_F16 | 4)) break;
+                if (!mbar_wait_warp(ws, &bars[F_K_FULL + st], (gs >> 1) & 1u, DEERS_KERR_FWD_F16 | 5)) break;
                 // This S tile still holds P of step gs-2 until the product reading it has finished.
-                if (!mbar_wait(ws, &bars[F_PV_DONE + st], ((gs >> 1) & 1u) ^ 1u, DEERS_KERR_FWD_F16 | 0x15)) break;
+                if (!mbar_wait_warp(ws, &bars[F_PV_DONE + st], ((gs >> 1) & 1u) ^ 1u, DEERS_KERR_FWD_F16 | 0x15)) break;
                 tc_fence_after_sync();
                 const uint64_t q_km = q_km0 + (uint64_t)qb * STAGE_STEP, k_km = k_km0 + (uint64_t)st * STAGE_STEP;
                 const uint32_t d_tmem = tmem + TM_S + st * 128u;
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks)
-                    umma_ss(d_tmem, q_km + kmajor_step(ks, BLOCK_BYTES), k_km + kmajor_step(ks, BLOCK_BYTES), IDESC_S, ks > 0);
-                umma_commit(&bars[F_S_FULL + st]);
-                if (sc.j == sc.ntiles - 1) umma_commit(&bars[F_Q_EMPTY + qb]);     // last product reading this Q
+                    for (int ks = 0; ks < D / 16; ++ks)
+                        umma_ss(d_tmem, q_km + kmajor_step(ks, BLOCK_BYTES), k_km + kmajor_step(ks, BLOCK_BYTES), IDESC_S, ks > 0);
+                    umma_commit(&bars[F_S_FULL + st]);
+                    if (sc.j == sc.ntiles - 1) umma_commit(&bars[F_Q_EMPTY + qb]); // last product reading this Q
+                }
+                __syncwarp();
                 sc.advance(p, nq, n_items);
             }
         }

@@ -53,7 +53,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     volatile uint32_t* abort_s = tmem_base_s + 1;
     uint32_t* skip_s = tmem_base_s + 2;
 
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = uniform((int)threadIdx.x / 32), lane = threadIdx.x % 32;
     const int tiles_m = (p.M + GM - 1) / GM, tiles_n = (p.N + GN - 1) / GN;
     const int n_tiles = tiles_m * tiles_n;
     const int kblocks = (p.K + GK - 1) / GK;
@@ -80,7 +80,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_base_s;
+    const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 
     if (warp == 0) {
@@ -116,29 +116,34 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        // The whole warp runs this; one elected lane issues (see elect_one).
+        {
             constexpr uint32_t IDESC = idesc_f16(GM, GN, A_MN, B_MN);
             constexpr uint64_t A_STEP = G_A_BYTES >> 4, B_STEP = G_B_BYTES >> 4;
-            const uint64_t a0 = A_MN ? desc_mnmajor(smem_u32(sA), 0, G_MN_BLOCK) : desc_kmajor(smem_u32(sA), 0, 0);
-            const uint64_t b0 = B_MN ? desc_mnmajor(smem_u32(sB), 0, G_MN_BLOCK) : desc_kmajor(smem_u32(sB), 0, 0);
+            const uint32_t sa0 = (uint32_t)uniform((int)smem_u32(sA)), sb0 = (uint32_t)uniform((int)smem_u32(sB));
+            const uint64_t a0 = A_MN ? desc_mnmajor(sa0, 0, G_MN_BLOCK) : desc_kmajor(sa0, 0, 0);
+            const uint64_t b0 = B_MN ? desc_mnmajor(sb0, 0, G_MN_BLOCK) : desc_kmajor(sb0, 0, 0);
             uint32_t g = 0;
             int n = 0;
             bool ok = true;
             for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x, ++n) {
                 const uint32_t buf = (uint32_t)n & 1u;
-                if (!mbar_wait(ws, &bars[G_ACC_EMPTY + buf], (((uint32_t)n >> 1) & 1u) ^ 1u, DEERS_KERR_GEMM | 2)) break;
+                if (!mbar_wait_warp(ws, &bars[G_ACC_EMPTY + buf], (((uint32_t)n >> 1) & 1u) ^ 1u, DEERS_KERR_GEMM | 2)) break;
                 for (int kb = 0; kb < kblocks; ++kb, ++g) {
                     const uint32_t s = g % G_STAGES;
-                    if (!mbar_wait(ws, &bars[G_FULL + s], (g / G_STAGES) & 1u, DEERS_KERR_GEMM | 3)) { ok = false; break; }
+                    if (!mbar_wait_warp(ws, &bars[G_FULL + s], (g / G_STAGES) & 1u, DEERS_KERR_GEMM | 3)) { ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t a = a0 + (uint64_t)s * A_STEP, b = b0 + (uint64_t)s * B_STEP;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < GK / 16; ++ks)                   // ks < 4: a K-major step stays inside its block
-                        umma_ss(tmem + buf * 256u, a + (A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0)),
-                                b + (B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0)), IDESC, (kb > 0 || ks > 0));
-                    umma_commit(&bars[G_EMPTY + s]);
+                        for (int ks = 0; ks < GK / 16; ++ks)               // ks < 4: a K-major step stays inside its block
+                            umma_ss(tmem + buf * 256u, a + (A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0)),
+                                    b + (B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0)), IDESC, (kb > 0 || ks > 0));
+                        umma_commit(&bars[G_EMPTY + s]);
+                        if (kb == kblocks - 1) umma_commit(&bars[G_ACC_FULL + buf]);
+                    }
+                    __syncwarp();
                 }
-                if (ok) umma_commit(&bars[G_ACC_FULL + buf]);
             }
         }
     } else {

@@ -57,7 +57,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_consta
     volatile uint32_t* abort_s = tmem_base_s + 1;
     uint32_t* skip_s = tmem_base_s + 2;
 
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = uniform((int)threadIdx.x / 32), lane = threadIdx.x % 32;
     const int tiles_m = (p.M + XM - 1) / XM, tiles_n = (p.N + XN - 1) / XN;
     const int n_units = tiles_m * tiles_n * p.parts;
 
@@ -83,7 +83,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_consta
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_base_s;
+    const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 
     // unit u -> (tile, part); consecutive units are the parts of one tile, so they run at the same time on
@@ -135,12 +135,14 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_consta
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        // The whole warp runs this; one elected lane issues (see elect_one).
+        {
             constexpr uint32_t IDESC = idesc_f16(XM, XN, A_MN, B_MN);
             constexpr uint64_t TILE_STEP = X_TILE >> 4, STAGE_STEP = X_STAGE >> 4;
-            const uint64_t a0 = A_MN ? desc_mnmajor(smem_u32(smem), 0, X_MN_BLOCK) : desc_kmajor(smem_u32(smem), 0, 0);
-            const uint64_t b0 = B_MN ? desc_mnmajor(smem_u32(smem + 2 * X_TILE), 0, X_MN_BLOCK)
-                                     : desc_kmajor(smem_u32(smem + 2 * X_TILE), 0, 0);
+            const uint32_t s0 = (uint32_t)uniform((int)smem_u32(smem));
+            const uint64_t a0 = A_MN ? desc_mnmajor(s0, 0, X_MN_BLOCK) : desc_kmajor(s0, 0, 0);
+            const uint64_t b0 = B_MN ? desc_mnmajor(s0 + 2 * X_TILE, 0, X_MN_BLOCK)
+                                     : desc_kmajor(s0 + 2 * X_TILE, 0, 0);
             uint32_t g = 0;
             int n = 0;
             bool ok = true;
@@ -149,25 +151,28 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_consta
                 unit(u, tm, tn, kb0, kb1);
                 const uint32_t buf = (uint32_t)n & 1u;
                 const uint32_t t_main = tmem + buf * 256u, t_corr = tmem + buf * 256u + 128u;
-                if (!mbar_wait(ws, &bars[X_ACC_EMPTY + buf], (((uint32_t)n >> 1) & 1u) ^ 1u, DEERS_KERR_GEMM | 0x12)) break;
+                if (!mbar_wait_warp(ws, &bars[X_ACC_EMPTY + buf], (((uint32_t)n >> 1) & 1u) ^ 1u, DEERS_KERR_GEMM | 0x12)) break;
                 for (int kb = kb0; kb < kb1; ++kb, ++g) {
                     const uint32_t s = g % X_STAGES;
-                    if (!mbar_wait(ws, &bars[X_FULL + s], (g / X_STAGES) & 1u, DEERS_KERR_GEMM | 0x13)) { ok = false; break; }
+                    if (!mbar_wait_warp(ws, &bars[X_FULL + s], (g / X_STAGES) & 1u, DEERS_KERR_GEMM | 0x13)) { ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t ah = a0 + (uint64_t)s * STAGE_STEP, al = ah + TILE_STEP;
                     const uint64_t bh = b0 + (uint64_t)s * STAGE_STEP, bl = bh + TILE_STEP;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < XK / 16; ++ks) {
-                        const uint64_t sa = A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0);
-                        const uint64_t sb = B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0);
-                        const uint32_t first = (kb > kb0 || ks > 0);
-                        umma_ss(t_main, ah + sa, bh + sb, IDESC, first);
-                        umma_ss(t_corr, ah + sa, bl + sb, IDESC, first);
-                        umma_ss(t_corr, al + sa, bh + sb, IDESC, 1u);
+                        for (int ks = 0; ks < XK / 16; ++ks) {
+                            const uint64_t sa = A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0);
+                            const uint64_t sb = B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0);
+                            const uint32_t first = (kb > kb0 || ks > 0);
+                            umma_ss(t_main, ah + sa, bh + sb, IDESC, first);
+                            umma_ss(t_corr, ah + sa, bl + sb, IDESC, first);
+                            umma_ss(t_corr, al + sa, bh + sb, IDESC, 1u);
+                        }
+                        umma_commit(&bars[X_EMPTY + s]);
+                        if (kb == kb1 - 1) umma_commit(&bars[X_ACC_FULL + buf]);
                     }
-                    umma_commit(&bars[X_EMPTY + s]);
+                    __syncwarp();
                 }
-                if (ok) umma_commit(&bars[X_ACC_FULL + buf]);
             }
         }
     } else {

@@ -79,6 +79,25 @@ __device__ __forceinline__ bool mbar_wait(const WaitState& ws, uint64_t* bar, ui
 }
 
 // ---------------------------------------------------------------------------
+// Warp-uniform issue
+// ---------------------------------------------------------------------------
+// tcgen05.mma takes its descriptors from uniform registers.  Under a single-lane branch (`if (lane == 0)`) every operand is
+// a per-thread value in the compiler's eyes, and each product pays for moving all of them over: about 110 cycles per
+// instruction beside busy compute warps, where the tensor core needs 64 (M = N = 128).  So the issuing warps run whole, on
+// values that are uniform by construction, and elect one lane for the instructions themselves: 64 to 67 cycles.
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ int4 uniform(const int4& v) { return make_int4(uniform(v.x), uniform(v.y), uniform(v.z), uniform(v.w)); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+// A wait by the whole warp; the answer is uniform.
+__device__ __forceinline__ bool mbar_wait_warp(const WaitState& ws, uint64_t* bar, uint32_t parity, uint32_t code) {
+    return __all_sync(0xffffffffu, mbar_wait(ws, bar, parity, code)) != 0;
+}
+
+// ---------------------------------------------------------------------------
 // Proxy fences
 // ---------------------------------------------------------------------------
 // Makes generic-proxy writes to shared memory visible to the async proxy (TMA, tcgen05.mma).
