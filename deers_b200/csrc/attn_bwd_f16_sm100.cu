@@ -25,8 +25,8 @@
 //   dK += dS^T Q   (A = dS^T from TMEM, B = Q MN-major)
 // dQ kernel: thread r (= query row r)
 //   S  = Q K^T, dP = dO V^T -> TMEM;  dS = P * (dP - delta) in place;  dQ += dS K (B = K MN-major)
-// Warp roles in both: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 two compute
-// warpgroups that split the 128 columns of S / dP (and the head_dim columns of the outputs).
+// Warp roles in both: warp 0 TMA producer, warp 1 MMA issuer, then two (dQ) or four (dK/dV) compute warpgroups
+// that split the 128 columns of S / dP (and the head_dim columns of the outputs).
 // Both kernels are persistent (one CTA per SM walking a strided list of tiles), so that the
 // loads and first products of the next tile overlap the tail and the epilogue of the current one.
 #include "sm100_ptx.cuh"
@@ -70,14 +70,8 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-// 1-D bulk copy global -> shared, completion counted on an mbarrier (16-byte aligned, size % 16 == 0).
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
-// The same with an L2 eviction-priority hint (a createpolicy value) for data that is read exactly once.
+// 1-D bulk copy global -> shared, completion counted on an mbarrier (16-byte aligned, size % 16 == 0), with an L2
+// eviction-priority hint (a createpolicy value) for data that is read exactly once.
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
     uint64_t pol;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
@@ -116,34 +110,47 @@ __device__ __forceinline__ int4 next_item(const BwdParams& p, int n, int n_items
 // ---------------------------------------------------------------------------------------------
 // dK / dV kernel (persistent: each CTA walks a strided list of KV tiles)
 // ---------------------------------------------------------------------------------------------
+// What bounds it at D = 128, per 128 x 128 step: 2048 cycles of tensor pipe and about as many of shared memory (S^T and dP^T
+// read both operands there at the full 128 bytes a cycle, and every byte of Q and dO arrives there), 1024 of the
+// special-function unit (one exponential per score), and the chain S^T -> P^T -> dV -> S^T(next) with the exponentials in
+// it.  Hence: dV starts on the first half of P^T's columns while the threads make the second; the statistics are read four
+// at a time and the multiply-adds run two to an instruction; arrivals are one per warp; a finished dS^T tile goes through
+// the stage of the dO tile it no longer needs and ONE bulk copy to global memory (stores from the compute threads cost
+// 1200 cycles a step); and an item's dK / dV leave TMEM after the next item's first P^T has been handed over.
+// B2 H16 T4096 D128, cycles per CTA: 433 k -> 378 k with dS kept, 357 k -> 328 k without.  A share of the exponentials
+// on the FMA pipe (polynomial) changed nothing: the phase is then bound by its instructions.
 // Dynamic shared memory only; the base must be 1024-byte aligned for the 128-byte swizzle (checked).
 template <int D>
 struct DkvSmem {
     static constexpr uint32_t TILE = 128u * D * 2u;
+    static constexpr int NSB = D == 64 ? 2 : 1;              // S^T tiles in TMEM: at D = 64 the accumulators leave room for two
     static constexpr uint32_t K = 0;
     static constexpr uint32_t V = K + TILE;
-    static constexpr uint32_t Q = V + TILE;                  // three stages: Q(i+1) feeds S^T while Q(i) still feeds dK
+    static constexpr uint32_t Q = V + TILE;
     static constexpr uint32_t DO = Q + 3 * TILE;             // two stages
-    static constexpr uint32_t LSE2 = DO + 2 * TILE;          // two stages of 128 floats
+    // dS^T tiles on their way to global memory, two blocks of 128 KV rows x 64 query columns each.  At D = 128 the tile of
+    // a step takes the place of the step's dO tile, which dV has read by then.
+    static constexpr uint32_t DS = D == 64 ? DO + 2 * TILE : DO;
+    static constexpr uint32_t DS_STEP = 2 * BLOCK_BYTES;
+    static constexpr uint32_t LSE2 = D == 64 ? DS + 2 * DS_STEP : DO + 2 * TILE;   // two stages of 128 floats, negated
     static constexpr uint32_t DELTA = LSE2 + 2 * BT * 4;
     static constexpr uint32_t BARS = DELTA + 2 * BT * 4;
-    static constexpr uint32_t TOTAL = BARS + 192;
+    static constexpr uint32_t TOTAL = BARS + 256;
 };
 
-enum DkvBar { A_KV_FULL = 0, A_KV_EMPTY = 1, A_Q_FULL = 2, A_Q_EMPTY = 5, A_DO_FULL = 8, A_DO_EMPTY = 10,
-              A_ST_FULL = 12, A_ST_EMPTY = 14, A_S = 16, A_DP = 17, A_P = 18, A_DS = 19, A_DONE = 20, A_ACC_FREE = 21,
-              A_COUNT = 22 };
+// A_S, A_P (first half of P^T's columns), A_P2 (second half) and A_DST (dS^T tile staged) are pairs indexed by the parity of
+// the step: their producers may be a step ahead of the waiter, and a pair keeps each barrier at most one phase ahead of it.
+enum DkvBar { A_KV_FULL = 0, A_KV_EMPTY = 1, A_Q_FULL = 2, A_Q_EMPTY = 5, A_DO_FULL = 8, A_DO_EMPTY = 10, A_ST_FULL = 12, A_S = 14,
+              A_P = 16, A_P2 = 18, A_DST = 20, A_DP = 22, A_DS = 23, A_DONE = 24, A_ACC_FREE = 25, A_COUNT = 26 };
 
-// Compute warpgroups of the dK / dV kernel: each owns 128 / DKV_NWG query columns of S^T / dP^T and
-// D / DKV_NWG columns of dK and dV.  Four (four warps per scheduler) measure 3 % faster than two on the same
-// GPU (6.36 against 6.56 ms at B64 H32 T2048 D128, both power-capped near 1.47 GHz).
+// Compute warpgroups of the dK / dV kernel: each owns 32 query columns of S^T / dP^T and D / 4 columns of dK and dV.
+// Four (four warps per scheduler) hide the TMEM and exponential latencies better than two.
 constexpr int DKV_NWG = 4;
 constexpr int DKV_THREADS = 64 + 128 * DKV_NWG;
 
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_x32(taddr, r); }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_x16(taddr, r); }
-__device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[32]) { tmem_st_x32(taddr, r); }
-__device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[16]) { tmem_st_x16(taddr, r); }
+
 
 template <int D>
 __global__ void __launch_bounds__(DKV_THREADS, 1)
@@ -153,15 +160,15 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     using L = DkvSmem<D>;
     constexpr uint32_t TILE_BYTES = L::TILE;
     constexpr int DBLK = D / 64;
-    constexpr int NWG = DKV_NWG;
-    constexpr int NCT = 128 * NWG;                          // compute threads
+    constexpr int NWG = DKV_NWG, NSB = L::NSB;
     constexpr int CW = BT / NWG;                            // query columns of S^T / dP^T per compute warpgroup
     constexpr int DH = D / NWG;                             // output columns per compute warpgroup
-    constexpr int EC = DH < 32 ? DH : 32;                   // columns per TMEM load in the epilogue
-    static_assert(CW % 32 == 0 && (DH == 16 || DH % 32 == 0), "unsupported warpgroup split");
+    constexpr int NCW = 4 * NWG;                            // compute warps (arrivals are one per warp)
+    static_assert(CW == 32 && (DH == 16 || DH == 32), "unsupported warpgroup split");
     constexpr uint32_t TMEM_COLS = 512;
-    // S^T (later P^T in place) | dP^T (later dS^T in place) | dV | dK
-    constexpr uint32_t TM_S = 0, TM_DP = 128, TM_DV = 256, TM_DK = 256 + D;
+    // S^T (later P^T in place), one or two | dP^T | dV | dK
+    constexpr uint32_t TM_S = 0, TM_DP = NSB * 128, TM_DV = TM_DP + 128, TM_DK = TM_DV + D;
+    static_assert(TM_DK + D <= TMEM_COLS, "TMEM");
 
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sK = smem + L::K;
@@ -192,14 +199,14 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         for (int s = 0; s < 3; ++s) { mbar_init(&bars[A_Q_FULL + s], 1); mbar_init(&bars[A_Q_EMPTY + s], 1); }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&bars[A_DO_FULL + s], 1); mbar_init(&bars[A_DO_EMPTY + s], 1);
-            mbar_init(&bars[A_ST_FULL + s], NCT);
+            mbar_init(&bars[A_ST_FULL + s], NCW);
+            mbar_init(&bars[A_S + s], 1); mbar_init(&bars[A_P + s], NCW); mbar_init(&bars[A_P2 + s], NCW);
+            mbar_init(&bars[A_DST + s], NCW);
         }
-        mbar_init(&bars[A_S], 1);
         mbar_init(&bars[A_DP], 1);
-        mbar_init(&bars[A_P], NCT);
-        mbar_init(&bars[A_DS], NCT);
+        mbar_init(&bars[A_DS], NCW);
         mbar_init(&bars[A_DONE], 1);
-        mbar_init(&bars[A_ACC_FREE], NCT);
+        mbar_init(&bars[A_ACC_FREE], NCW);
         fence_barrier_init();
         tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v); tma_prefetch_desc(&tmap_do);
     }
@@ -220,10 +227,21 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         if (lane == 0) {
             uint32_t gi = 0;                                    // query-tile iterations so far (all items)
             bool ok = true;
+            // With dS kept, this thread also takes the finished dS^T tiles to global memory: step gi - 2 used the stage that dO
+            // of step gi is about to fill (at D = 64 a tile of its own, with the same order).
+            uint8_t* ds_dst[2] = {nullptr, nullptr};
+            auto store_ds = [&](uint32_t x) -> bool {           // x: the step whose tile leaves
+                if (!mbar_wait(ws, &bars[A_DST + (x & 1u)], (x >> 1) & 1u, DEERS_KERR_BWD_F16 | 3)) return false;
+                bulk_store((x & 1u) ? ds_dst[1] : ds_dst[0], smem + L::DS + (x & 1u) * L::DS_STEP, L::DS_STEP);
+                bulk_commit_group();
+                bulk_wait_group_read<0>();
+                return true;
+            };
             for (int4 cur = next_item(p, 0, n_items, nq), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); ok && cur.x >= 0;
                      ++n4.x, cur = nxt, nxt = next_item(p, n4.x + 1, n_items, nq)) {
-                const int n = n4.x, kt = cur.x, bh = cur.y;
+                const int n = n4.x, kt = cur.x;
                 const int b = cur.z, h = cur.w;
+                uint8_t* ds_base = reinterpret_cast<uint8_t*>(p.ds) + (((long long)cur.y * p.ds_pairs) << 15);
                 const int i0 = p.causal ? kt : 0;
                 const int niter = nq - i0;
                 // K / V are single-buffered: wait until the previous item's S^T and dP^T products are done.
@@ -242,106 +260,113 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 #pragma unroll
                     for (int blk = 0; blk < DBLK; ++blk)
                         tma_load_4d(sQ + qs * TILE_BYTES + blk * BLOCK_BYTES, &tmap_q, &bars[A_Q_FULL + qs], blk * 64, q0, h, b);
-                    if (!mbar_wait(ws, &bars[A_DO_EMPTY + ds], ((gi >> 1) & 1u) ^ 1u, DEERS_KERR_BWD_F16 | 4)) { ok = false; break; }
+                    if (p.ds) {
+                        if (gi >= 2 && !store_ds(gi - 2u)) { ok = false; break; }
+                        uint8_t* dst = ds_base + (ds_pair(p, i0 + it, kt, nq) << 15);
+                        if (ds) ds_dst[1] = dst; else ds_dst[0] = dst;
+                    } else if (!mbar_wait(ws, &bars[A_DO_EMPTY + ds], ((gi >> 1) & 1u) ^ 1u, DEERS_KERR_BWD_F16 | 4)) { ok = false; break; }
                     mbar_arrive_expect_tx(&bars[A_DO_FULL + ds], TILE_BYTES);
 #pragma unroll
                     for (int blk = 0; blk < DBLK; ++blk)
                         tma_load_4d(sDO + ds * TILE_BYTES + blk * BLOCK_BYTES, &tmap_do, &bars[A_DO_FULL + ds], blk * 64, q0, h, b);
                 }
             }
+            if (p.ds) {
+                for (uint32_t x = gi < 2u ? 0u : gi - 2u; ok && x < gi; ++x) ok = store_ds(x);
+                bulk_wait_group<0>();
+            }
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp runs this; one elected lane issues (see elect_one).
-        {
-            constexpr uint32_t IDESC_ST = idesc_f16(128, 128, 0, 0);   // S^T, dP^T: K-major A and B
-            constexpr uint32_t IDESC_KV = idesc_f16(128, D, 0, 1);     // dV, dK: A from TMEM, MN-major B
-            // Step-0 descriptors of every operand view, built once; each MMA adds a constant
-            // (a single thread issues, so descriptor arithmetic must stay off the issue path).
-            constexpr uint64_t STAGE_STEP = TILE_BYTES >> 4;           // next stage of Q / dO
-            const uint64_t k_km = desc_kmajor((uint32_t)uniform((int)smem_u32(sK)), 0, BLOCK_BYTES);
-            const uint64_t v_km = desc_kmajor((uint32_t)uniform((int)smem_u32(sV)), 0, BLOCK_BYTES);
-            const uint64_t q_km0 = desc_kmajor((uint32_t)uniform((int)smem_u32(sQ)), 0, BLOCK_BYTES), q_mn0 = desc_mnmajor((uint32_t)uniform((int)smem_u32(sQ)), 0, BLOCK_BYTES);
-            const uint64_t do_km0 = desc_kmajor((uint32_t)uniform((int)smem_u32(sDO)), 0, BLOCK_BYTES), do_mn0 = desc_mnmajor((uint32_t)uniform((int)smem_u32(sDO)), 0, BLOCK_BYTES);
-            auto issue_st = [&](uint32_t qs) {
-                const uint64_t q_km = q_km0 + (uint64_t)qs * STAGE_STEP;
-                if (elect_one()) {
+        constexpr uint32_t IDESC_ST = idesc_f16(128, 128, 0, 0);       // S^T, dP^T: K-major A and B
+        constexpr uint32_t IDESC_KV = idesc_f16(128, D, 0, 1);         // dV, dK: K-major A, MN-major B
+        // Step-0 descriptors of every operand view, built once; each MMA adds a constant.
+        constexpr uint64_t STAGE_STEP = TILE_BYTES >> 4;               // next stage of Q / dO
+        const uint32_t s0 = (uint32_t)uniform((int)smem_u32(smem));
+        const uint64_t k_km = desc_kmajor(s0 + L::K, 0, BLOCK_BYTES), v_km = desc_kmajor(s0 + L::V, 0, BLOCK_BYTES);
+        const uint64_t q_km0 = desc_kmajor(s0 + L::Q, 0, BLOCK_BYTES), q_mn0 = desc_mnmajor(s0 + L::Q, 0, BLOCK_BYTES);
+        const uint64_t do_km0 = desc_kmajor(s0 + L::DO, 0, BLOCK_BYTES), do_mn0 = desc_mnmajor(s0 + L::DO, 0, BLOCK_BYTES);
+        // S^T of step x over the P^T of step x - NSB: the product that reads it has been issued, and the pipe is in order.
+        auto issue_st = [&](uint32_t x) -> bool {
+            const uint32_t qs = x % 3u;
+            if (!mbar_wait_warp(ws, &bars[A_Q_FULL + qs], (x / 3u) & 1u, DEERS_KERR_BWD_F16 | 6)) return false;
+            tc_fence_after_sync();
+            const uint64_t q_km = q_km0 + (uint64_t)qs * STAGE_STEP;
+            const uint32_t dst = tmem + TM_S + (NSB == 2 ? (x & 1u) * 128u : 0u);
+            if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < D / 16; ++ks)
-                        umma_ss(tmem + TM_S, k_km + kmajor_step(ks, BLOCK_BYTES), q_km + kmajor_step(ks, BLOCK_BYTES), IDESC_ST, ks > 0);
-                    umma_commit(&bars[A_S]);
-                }
-                __syncwarp();
-            };
-            auto issue_dpt = [&](uint32_t ds) {
-                const uint64_t do_km = do_km0 + (uint64_t)ds * STAGE_STEP;
-                if (elect_one()) {
+                for (int ks = 0; ks < D / 16; ++ks)
+                    umma_ss(dst, k_km + kmajor_step(ks, BLOCK_BYTES), q_km + kmajor_step(ks, BLOCK_BYTES), IDESC_ST, ks > 0);
+                umma_commit(&bars[A_S + (x & 1u)]);
+            }
+            __syncwarp();
+            return true;
+        };
+        // dP^T of step x over dS^T of step x - 1, whose product has been issued.
+        auto issue_dpt = [&](uint32_t x, bool last) -> bool {
+            if (!mbar_wait_warp(ws, &bars[A_DO_FULL + (x & 1u)], (x >> 1) & 1u, DEERS_KERR_BWD_F16 | 7)) return false;
+            tc_fence_after_sync();
+            const uint64_t do_km = do_km0 + (uint64_t)(x & 1u) * STAGE_STEP;
+            if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < D / 16; ++ks)
-                        umma_ss(tmem + TM_DP, v_km + kmajor_step(ks, BLOCK_BYTES), do_km + kmajor_step(ks, BLOCK_BYTES), IDESC_ST, ks > 0);
-                    umma_commit(&bars[A_DP]);
-                }
-                __syncwarp();
-            };
-            // A operand in TMEM: CW / 2 packed columns per compute warpgroup, the groups CW columns apart.
-            auto a_tmem = [&](uint32_t base, int ks) {
-                return tmem + base + (uint32_t)(ks / (CW / 16)) * (uint32_t)CW + (uint32_t)(ks % (CW / 16)) * 8u;
-            };
-            uint32_t gi = 0;
-            bool ok = true;
-            for (int4 cur = uniform(next_item(p, 0, n_items, nq)), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); ok && cur.x >= 0;
-                     ++n4.x, cur = uniform(nxt), nxt = next_item(p, n4.x + 1, n_items, nq)) {
-                const int n = n4.x, kt = cur.x, bh = cur.y;
-                const int niter = nq - (p.causal ? kt : 0);
-                if (!mbar_wait_warp(ws, &bars[A_KV_FULL], (uint32_t)n & 1u, DEERS_KERR_BWD_F16 | 5)) break;
-                if (!mbar_wait_warp(ws, &bars[A_Q_FULL + gi % 3u], (gi / 3u) & 1u, DEERS_KERR_BWD_F16 | 6)) break;
-                if (!mbar_wait_warp(ws, &bars[A_DO_FULL + (gi & 1u)], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 7)) break;
+                for (int ks = 0; ks < D / 16; ++ks)
+                    umma_ss(tmem + TM_DP, v_km + kmajor_step(ks, BLOCK_BYTES), do_km + kmajor_step(ks, BLOCK_BYTES), IDESC_ST, ks > 0);
+                umma_commit(&bars[A_DP]);
+                if (last) umma_commit(&bars[A_KV_EMPTY]);              // the item's last S^T and dP^T are issued
+            }
+            __syncwarp();
+            return true;
+        };
+        uint32_t gi = 0;
+        bool ok = true;
+        for (int4 cur = uniform(next_item(p, 0, n_items, nq)), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); ok && cur.x >= 0;
+                 ++n4.x, cur = uniform(nxt), nxt = next_item(p, n4.x + 1, n_items, nq)) {
+            const int n = n4.x;
+            const int niter = nq - (p.causal ? cur.x : 0);
+            if (!mbar_wait_warp(ws, &bars[A_KV_FULL], (uint32_t)n & 1u, DEERS_KERR_BWD_F16 | 5)) break;
+            if (!issue_st(gi) || !issue_dpt(gi, niter == 1)) break;
+            for (int it = 0; it < niter; ++it, ++gi) {
+                const uint32_t qs = gi % 3u, ds = gi & 1u;
+                const uint64_t q_mn = q_mn0 + (uint64_t)qs * STAGE_STEP, do_mn = do_mn0 + (uint64_t)ds * STAGE_STEP;
+                const bool more = it + 1 < niter;
+                if (NSB == 2 && more && !issue_st(gi + 1u)) { ok = false; break; }
+                // dV += P^T dO; the previous item's dK / dV must have left TMEM before this item accumulates.
+                if (!mbar_wait_warp(ws, &bars[A_P + ds], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 8)) { ok = false; break; }
+                if (it == 0 && !mbar_wait_warp(ws, &bars[A_ACC_FREE], ((uint32_t)n & 1u) ^ 1u, DEERS_KERR_BWD_F16 | 9)) { ok = false; break; }
                 tc_fence_after_sync();
-                issue_st(gi % 3u);
-                issue_dpt(gi & 1u);
-                if (niter == 1 && elect_one()) umma_commit(&bars[A_KV_EMPTY]);         // no further product reads K / V
-                for (int it = 0; it < niter; ++it, ++gi) {
-                    const uint32_t qs = gi % 3u, ds = gi & 1u, par = gi & 1u;
-                    const uint64_t q_mn = q_mn0 + (uint64_t)qs * STAGE_STEP, do_mn = do_mn0 + (uint64_t)ds * STAGE_STEP;
-                    const bool more = it + 1 < niter;
-                    // dV += P^T dO, then S^T of the next query tile: the pipe is in order, so the
-                    // new S^T lands only after dV has consumed P^T from the same columns.
-                    if (!mbar_wait_warp(ws, &bars[A_P], par, DEERS_KERR_BWD_F16 | 8)) { ok = false; break; }
-                    // The previous item's dK / dV must have left TMEM before this item accumulates.
-                    if (it == 0 && !mbar_wait_warp(ws, &bars[A_ACC_FREE], ((uint32_t)n & 1u) ^ 1u, DEERS_KERR_BWD_F16 | 9)) { ok = false; break; }
-                    tc_fence_after_sync();
-                    if (elect_one()) {
+                const uint32_t tm_p = tmem + TM_S + (NSB == 2 ? ds * 128u : 0u);
+                // 16 query columns of P^T are 8 packed TMEM columns; a warpgroup's 32 columns start 32 apart.  The even steps
+                // need only the first 16 columns of every warpgroup and run while the threads make the others.
+                if (elect_one()) {
 #pragma unroll
-                        for (int ks = 0; ks < BT / 16; ++ks)
-                            umma_ts(tmem + TM_DV, a_tmem(TM_S, ks), do_mn + mnmajor_step(ks), IDESC_KV, (it > 0 || ks > 0));
-                    }
-                    __syncwarp();
-                    if (more) {
-                        if (!mbar_wait_warp(ws, &bars[A_Q_FULL + (gi + 1u) % 3u], ((gi + 1u) / 3u) & 1u, DEERS_KERR_BWD_F16 | 10)) { ok = false; break; }
-                        tc_fence_after_sync();
-                        issue_st((gi + 1u) % 3u);
-                    }
-                    // dK += dS^T Q, then dP^T of the next query tile over the consumed dS^T columns.
-                    if (!mbar_wait_warp(ws, &bars[A_DS], par, DEERS_KERR_BWD_F16 | 11)) { ok = false; break; }
-                    tc_fence_after_sync();
-                    if (elect_one()) {
-#pragma unroll
-                        for (int ks = 0; ks < BT / 16; ++ks)
-                            umma_ts(tmem + TM_DK, a_tmem(TM_DP, ks), q_mn + mnmajor_step(ks), IDESC_KV, (it > 0 || ks > 0));
-                        umma_commit(&bars[A_Q_EMPTY + qs]);                 // S^T and dK have both read this Q tile
-                    }
-                    __syncwarp();
-                    if (more) {
-                        if (!mbar_wait_warp(ws, &bars[A_DO_FULL + (ds ^ 1u)], ((gi + 1u) >> 1) & 1u, DEERS_KERR_BWD_F16 | 12)) { ok = false; break; }
-                        tc_fence_after_sync();
-                        issue_dpt(ds ^ 1u);
-                        if (it + 2 == niter && elect_one()) umma_commit(&bars[A_KV_EMPTY]);   // the last S^T and dP^T are issued
-                    }
-                    // dO of this iteration was last read by dV (and dP^T before it): its stage is free once
-                    // everything issued so far has finished.
-                    if (elect_one()) umma_commit(&bars[A_DO_EMPTY + ds]);
+                    for (int ks = 0; ks < BT / 16; ks += 2)
+                        umma_ts(tmem + TM_DV, tm_p + (uint32_t)(ks >> 1) * 32u, do_mn + mnmajor_step(ks), IDESC_KV, (it > 0 || ks > 0));
                 }
-                if (elect_one()) umma_commit(&bars[A_DONE]);
+                __syncwarp();
+                if (!mbar_wait_warp(ws, &bars[A_P2 + ds], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 8)) { ok = false; break; }
+                tc_fence_after_sync();
+                if (elect_one()) {
+#pragma unroll
+                    for (int ks = 1; ks < BT / 16; ks += 2)
+                        umma_ts(tmem + TM_DV, tm_p + (uint32_t)(ks >> 1) * 32u + 8u, do_mn + mnmajor_step(ks), IDESC_KV, 1u);
+                    umma_commit(&bars[A_DO_EMPTY + ds]);               // dP^T and dV have both read this dO tile
+                }
+                __syncwarp();
+                if (NSB == 1 && more && !issue_st(gi + 1u)) { ok = false; break; }
+                // dK += dS^T Q
+                if (!mbar_wait_warp(ws, &bars[A_DS], gi & 1u, DEERS_KERR_BWD_F16 | 11)) { ok = false; break; }
+                tc_fence_after_sync();
+                if (elect_one()) {
+#pragma unroll
+                    for (int ks = 0; ks < BT / 16; ++ks)
+                        umma_ts(tmem + TM_DK, tmem + TM_DP + (uint32_t)(ks >> 1) * 32u + (uint32_t)(ks & 1) * 8u, q_mn + mnmajor_step(ks), IDESC_KV,
+                                (it > 0 || ks > 0));
+                    umma_commit(&bars[A_Q_EMPTY + qs]);                // S^T and dK have both read this Q tile
+                    if (!more) umma_commit(&bars[A_DONE]);
+                }
+                __syncwarp();
+                if (more && !issue_dpt(gi + 1u, it + 2 == niter)) { ok = false; break; }
             }
         }
     } else {
@@ -353,13 +378,14 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         const int r = lane_base + lane;
         const uint32_t t_lane = (uint32_t)lane_base << 16;
         const float sl2 = p.scale * LOG2E;
+        const uint64_t sl2_2 = pack_f32x2(sl2, sl2);
         uint32_t gi = 0;
         bool alive = true;
-        // The 128 lse * log2e and the 128 delta values of a query tile are staged in shared memory by the compute
+        // The 128 lse * log2e and the 128 delta values of a query tile are staged (negated) in shared memory by the compute
         // threads themselves: thread ct < 256 fetches element ct of the NEXT iteration's 256 values one iteration
         // ahead (a plain global load, in flight during this iteration's products) and stores it at the top of that
-        // iteration; every compute thread then arrives on the stage's barrier and waits for all before reading.  A stage is
-        // rewritten two iterations after it was read, and nobody gets there before all threads have passed the
+        // iteration; every compute warp then arrives on the stage's barrier and waits for all before reading.  A stage is
+        // rewritten two iterations after it was read, and nobody gets there before all warps have passed the
         // barrier of the iteration in between, i.e. have finished reading.  (An earlier version had the producer
         // warp bring these rows in with bulk copies; repeated full-size runs then showed, once in a few dozen, one
         // warp seeing a stale 32-byte piece of the delta row in the first iteration of an item.)
@@ -372,11 +398,51 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             const int4 first = next_item(p, 0, n_items, nq);
             if (stager && first.x >= 0) stat_next = __ldg(stat_src + (long long)first.y * p.Tpad + (p.causal ? first.x : 0) * BT);
         }
+        // this thread's row of the dS^T tile; its warpgroup's four 16-byte chunks start at chunk ch0 of the row
+        uint8_t* ds_row = smem + L::DS + (CW * g / 64) * BLOCK_BYTES + r * 128;   // (of the first stage)
+        const int ch0 = (CW * g % 64) / 8;
+
+        // The epilogue of an item (dK and dV of its KV tile leave TMEM) is deferred until the first P^T of the next item has
+        // been handed over, so that the tensor core's last products and that P^T overlap.
+        int pend_n = -1, pend_k0 = 0, pend_b = 0, pend_h = 0;
+        auto epilogue = [&]() -> bool {
+            if (pend_n < 0) return true;
+            const int n = pend_n;
+            pend_n = -1;
+            if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_DONE], (uint32_t)n & 1u, DEERS_KERR_BWD_F16 | 16))) return false;
+            tc_fence_after_sync();
+            // The thread's piece of a row, as 16-byte pieces, is transposed within lane groups so that every store
+            // instruction writes whole contiguous row segments.
+            constexpr int NP = DH / 8;
+            const int row0 = pend_k0 + lane_base + (lane & ~(NP - 1));
+            const int col = g * DH + (lane & (NP - 1)) * 8;
+#pragma unroll
+            for (int which = 0; which < 2; ++which) {
+                uint32_t xr[DH];
+                uint4 oc[NP];
+                tmem_ld(tmem + (which ? TM_DK : TM_DV) + t_lane + g * DH, xr);
+                tmem_wait_ld();
+                if (which) {                                // both accumulators are in registers: release TMEM
+                    tc_fence_before_sync();
+                    mbar_arrive_warp(&bars[A_ACC_FREE]);
+                }
+#pragma unroll
+                for (int q8 = 0; q8 < NP; ++q8) oc[q8] = pack8_f16(xr + q8 * 8, which ? p.scale : 1.0f);
+                transpose_pieces<NP>(oc, (uint32_t)lane);
+                __half* ob = which ? p.dk + pend_b * p.sdk_b + pend_h * p.sdk_h + col : p.dv + pend_b * p.sdv_b + pend_h * p.sdv_h + col;
+                const long long so_t = which ? p.sdk_t : p.sdv_t;
+#pragma unroll
+                for (int c = 0; c < NP; ++c) {
+                    const int row = row0 + c;
+                    if (row < p.T && col < p.d) *reinterpret_cast<uint4*>(ob + (long long)row * so_t) = oc[c];
+                }
+            }
+            return true;
+        };
 
         for (int4 cur = next_item(p, 0, n_items, nq), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); alive && cur.x >= 0;
                  ++n4.x, cur = nxt, nxt = next_item(p, n4.x + 1, n_items, nq)) {
-            const int n = n4.x, kt = cur.x, bh = cur.y;
-            const int b = cur.z, h = cur.w;
+            const int kt = cur.x, bh = cur.y;
             const int k0 = kt * BT;
             const int i0 = p.causal ? kt : 0;
             const int niter = nq - i0;
@@ -384,131 +450,91 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 
             for (int it = 0; it < niter; ++it, ++gi) {
                 const int i = i0 + it;
-                const uint32_t ss = gi & 1u, par = gi & 1u;
-                const float* lse2 = lse2_s + ss * BT + CW * g;
-                const float* dlt = delta_s + ss * BT + CW * g;
-                if (stager) stat_dst[ss * BT] = stat_next;  // this iteration's value, fetched one iteration ago
-                mbar_arrive(&bars[A_ST_FULL + ss]);
+                const uint32_t ss = gi & 1u;
+                const ulonglong2* nlse2 = reinterpret_cast<const ulonglong2*>(lse2_s + ss * BT + CW * g);     // four values each
+                const ulonglong2* ndelta = reinterpret_cast<const ulonglong2*>(delta_s + ss * BT + CW * g);
+                if (stager) stat_dst[ss * BT] = -stat_next; // this iteration's value, fetched one iteration ago
+                mbar_arrive_warp(&bars[A_ST_FULL + ss]);
                 // next iteration's value: the next query tile of this item, or the first one of the next item
                 if (stager) {
                     if (it + 1 < niter) stat_next = __ldg(stat_src + (long long)bh * p.Tpad + (i + 1) * BT);
                     else if (nxt.x >= 0) stat_next = __ldg(stat_src + (long long)nxt.y * p.Tpad + (p.causal ? nxt.x : 0) * BT);
                 }
                 if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_ST_FULL + ss], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 13))) { alive = false; break; }
-                if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_S], par, DEERS_KERR_BWD_F16 | 14))) { alive = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_S + ss], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 14))) { alive = false; break; }
                 tc_fence_after_sync();
                 const bool diag = p.causal && (i == kt);
+                const bool edge = diag || !kv_valid;        // only the diagonal / tail tile pays for masking
+                const uint32_t tm_s = tmem + TM_S + (NSB == 2 ? ss * 128u : 0u) + t_lane + CW * g;
                 uint32_t pk[CW / 2];                        // P^T row, CW query columns as f16 pairs
+                uint32_t sr[32];
+                tmem_ld_x32(tm_s, sr);
+                tmem_wait_ld();
+                // P^T replaces this warpgroup's part of S^T in TMEM, 16 columns (8 packed) at a time.
 #pragma unroll
-                for (int c = 0; c < CW / 32; ++c) {
-                    uint32_t sr[32];
-                    tmem_ld_x32(tmem + TM_S + t_lane + CW * g + c * 32, sr);
-                    tmem_wait_ld();
-                    if (diag || !kv_valid) {                // only the diagonal / tail tile pays for masking
+                for (int hf = 0; hf < 2; ++hf) {
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            const int cl = c * 32 + e * 2;  // column inside this warpgroup's half
-                            float p0 = ex2(fmaf(__uint_as_float(sr[e * 2]), sl2, -lse2[cl]));
-                            float p1 = ex2(fmaf(__uint_as_float(sr[e * 2 + 1]), sl2, -lse2[cl + 1]));
-                            if ((diag && (CW * g + cl) < r) || !kv_valid) p0 = 0.f;   // query index < key index: masked
-                            if ((diag && (CW * g + cl + 1) < r) || !kv_valid) p1 = 0.f;
-                            pk[c * 16 + e] = pack_half2(p0, p1);
+                    for (int e = hf * 4; e < hf * 4 + 4; ++e) {     // four columns
+                        const ulonglong2 nl = nlse2[e];
+                        float x0, x1, x2, x3;
+                        unpack_f32x2(fma2(pack_f32x2(sr[e * 4], sr[e * 4 + 1]), sl2_2, nl.x), x0, x1);
+                        unpack_f32x2(fma2(pack_f32x2(sr[e * 4 + 2], sr[e * 4 + 3]), sl2_2, nl.y), x2, x3);
+                        x0 = ex2(x0); x1 = ex2(x1); x2 = ex2(x2); x3 = ex2(x3);
+                        if (edge) {                         // query index < key index, or a key past the end: masked
+                            const int cl = CW * g + e * 4, lim = kv_valid ? r : 1 << 20;
+                            if (cl < lim) x0 = 0.f;
+                            if (cl + 1 < lim) x1 = 0.f;
+                            if (cl + 2 < lim) x2 = 0.f;
+                            if (cl + 3 < lim) x3 = 0.f;
                         }
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            const int cl = c * 32 + e * 2;
-                            pk[c * 16 + e] = pack_half2(ex2(fmaf(__uint_as_float(sr[e * 2]), sl2, -lse2[cl])),
-                                                        ex2(fmaf(__uint_as_float(sr[e * 2 + 1]), sl2, -lse2[cl + 1])));
-                        }
+                        pk[e * 2] = pack_half2(x0, x1);
+                        pk[e * 2 + 1] = pack_half2(x2, x3);
                     }
+                    tmem_st_x8(tm_s + hf * 8, &pk[hf * 8]);
+                    tmem_wait_st();
+                    tc_fence_before_sync();
+                    mbar_arrive_warp(&bars[(hf ? A_P2 : A_P) + ss]);
                 }
-                // P^T replaces this warpgroup's part of S^T in TMEM (CW / 2 packed columns).
-                tmem_st(tmem + TM_S + t_lane + CW * g, pk);
-                tmem_wait_st();
-                tc_fence_before_sync();
-                mbar_arrive(&bars[A_P]);
+                if (it == 0 && !epilogue()) { alive = false; break; }      // the previous item's dK and dV
 
-                if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_DP], par, DEERS_KERR_BWD_F16 | 15))) { alive = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_DP], gi & 1u, DEERS_KERR_BWD_F16 | 15))) { alive = false; break; }
                 tc_fence_after_sync();
+                uint32_t dr[32];
+                tmem_ld_x32(tmem + TM_DP + t_lane + CW * g, dr);
+                tmem_wait_ld();
                 uint32_t dd[CW / 2];                        // dS^T row, CW query columns as f16 pairs
 #pragma unroll
-                for (int c = 0; c < CW / 32; ++c) {
-                    uint32_t dr[32];
-                    tmem_ld_x32(tmem + TM_DP + t_lane + CW * g + c * 32, dr);
-                    tmem_wait_ld();
+                for (int e = 0; e < 8; ++e) {               // four columns
+                    const ulonglong2 nd = ndelta[e];
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) {
-                        const int cl = c * 32 + e * 2;
-                        const float2 pf = __half22float2(*reinterpret_cast<const __half2*>(&pk[c * 16 + e]));
-                        dd[c * 16 + e] = pack_half2(pf.x * (__uint_as_float(dr[e * 2]) - dlt[cl]),
-                                                    pf.y * (__uint_as_float(dr[e * 2 + 1]) - dlt[cl + 1]));
+                    for (int w = 0; w < 2; ++w) {
+                        const int at = e * 2 + w;
+                        const float2 pf = __half22float2(*reinterpret_cast<const __half2*>(&pk[at]));
+                        float d0, d1;
+                        unpack_f32x2(mul2(pack_f32x2(pf.x, pf.y), add2(pack_f32x2(dr[at * 2], dr[at * 2 + 1]), w ? nd.y : nd.x)), d0, d1);
+                        dd[at] = pack_half2(d0, d1);
                     }
                 }
-                tmem_st(tmem + TM_DP + t_lane + CW * g, dd);
+                tmem_st_x16(tmem + TM_DP + t_lane + CW * g, dd);
                 tmem_wait_st();
                 tc_fence_before_sync();
-                mbar_arrive(&bars[A_DS]);
+                mbar_arrive_warp(&bars[A_DS]);
                 if (p.ds) {
-                    // The same dS^T row also goes to global memory, already swizzled, for the dQ kernel (off the
-                    // critical path: the tensor core has what it needs).  The row's NCH 16-byte chunks are
-                    // transposed within NCH-lane groups first, so that one store instruction writes whole
-                    // NCH*16-byte row segments instead of 16 bytes in each of 32 rows.
-                    constexpr int NCH = CW / 8;                 // this warpgroup's chunks of a row
-                    uint8_t* tile = reinterpret_cast<uint8_t*>(p.ds) + (((long long)bh * p.ds_pairs + ds_pair(p, i, kt, nq)) << 15) +
-                                    (CW * g / 64) * (int)BLOCK_BYTES;
-                    const int ch0 = (CW * g % 64) / 8;          // first chunk inside the 64-column block
-                    uint4 pc[NCH];
+                    // The same tile goes to global memory for the dQ kernel: through shared memory, in the place of this step's
+                    // dO tile (dV has read it) and from there by one bulk copy.
+                    if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_DO_EMPTY + ss], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 17))) { alive = false; break; }
 #pragma unroll
-                    for (int ch = 0; ch < NCH; ++ch) pc[ch] = make_uint4(dd[4 * ch], dd[4 * ch + 1], dd[4 * ch + 2], dd[4 * ch + 3]);
-                    transpose_pieces<NCH>(pc, (uint32_t)lane);
-                    const int rbase = lane_base + (lane & ~(NCH - 1));  // pc[c] is now chunk (lane % NCH) of row rbase + c
-#pragma unroll
-                    for (int c = 0; c < NCH; ++c)     // streaming stores: the tiles are read once, by the next kernel
-                        __stcs(reinterpret_cast<uint4*>(tile + sw128_chunk_offset(rbase + c, ch0 + (lane & (NCH - 1)))), pc[c]);
+                    for (int c = 0; c < 4; ++c)
+                        *reinterpret_cast<uint4*>(ds_row + ss * L::DS_STEP + (((ch0 + c) ^ (r & 7)) << 4)) =
+                            make_uint4(dd[4 * c], dd[4 * c + 1], dd[4 * c + 2], dd[4 * c + 3]);
+                    fence_proxy_async_smem();
+                    mbar_arrive_warp(&bars[A_DST + ss]);
                 }
             }
             if (!alive) break;
-
-            // Epilogue: dK and dV of this KV tile leave TMEM; meanwhile the tensor core already
-            // computes S^T and dP^T of the next item.
-            if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_DONE], (uint32_t)n & 1u, DEERS_KERR_BWD_F16 | 16))) { alive = false; break; }
-            tc_fence_after_sync();
-            // The thread's half rows of dK and dV, as 16-byte pieces, are transposed within lane
-            // groups so that every store instruction writes whole contiguous row segments.
-            constexpr int NP = DH / 8;
-            uint4 kc[NP], vc[NP];
-#pragma unroll
-            for (int c = 0; c < DH / EC; ++c) {
-                uint32_t kr[EC], vr[EC];
-                tmem_ld(tmem + TM_DK + t_lane + g * DH + c * EC, kr);
-                tmem_ld(tmem + TM_DV + t_lane + g * DH + c * EC, vr);
-                tmem_wait_ld();
-                if (c == DH / EC - 1) {                     // accumulators are in registers: release TMEM early
-                    tc_fence_before_sync();
-                    mbar_arrive(&bars[A_ACC_FREE]);
-                }
-#pragma unroll
-                for (int q8 = 0; q8 < EC / 8; ++q8) {
-                    kc[c * (EC / 8) + q8] = pack8_f16(kr + q8 * 8, p.scale);
-                    vc[c * (EC / 8) + q8] = pack8_f16(vr + q8 * 8, 1.0f);
-                }
-            }
-            transpose_pieces<NP>(kc, (uint32_t)lane);
-            transpose_pieces<NP>(vc, (uint32_t)lane);
-            const int row0 = k0 + lane_base + (lane & ~(NP - 1));
-            const int col = g * DH + (lane & (NP - 1)) * 8;
-            __half* dkb = p.dk + b * p.sdk_b + h * p.sdk_h + col;
-            __half* dvb = p.dv + b * p.sdv_b + h * p.sdv_h + col;
-#pragma unroll
-            for (int c = 0; c < NP; ++c) {
-                const int row = row0 + c;
-                if (row < p.T && col < p.d) {
-                    *reinterpret_cast<uint4*>(dkb + (long long)row * p.sdk_t) = kc[c];
-                    *reinterpret_cast<uint4*>(dvb + (long long)row * p.sdv_t) = vc[c];
-                }
-            }
+            pend_n = n4.x; pend_k0 = k0; pend_b = cur.z; pend_h = cur.w;
         }
+        if (alive) epilogue();
     }
 
     __syncwarp();
@@ -667,7 +693,7 @@ attn_bwd_dq_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             bool ok = true;
             for (int4 cur = uniform(next_item(p, 0, n_items, nq)), nxt = next_item(p, 1, n_items, nq), n4 = make_int4(0, 0, 0, 0); ok && cur.x >= 0;
                      ++n4.x, cur = uniform(nxt), nxt = next_item(p, n4.x + 1, n_items, nq)) {
-                const int n = n4.x, slot = cur.x, bh = cur.y;
+                const int n = n4.x, slot = cur.x;
                 const int qt = nq - 1 - slot;
                 const int ntiles = p.causal ? qt + 1 : nq;
                 const uint32_t tm_dq = tmem + TM_DQ;
