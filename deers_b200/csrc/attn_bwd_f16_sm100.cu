@@ -32,6 +32,8 @@
 #include "sm100_ptx.cuh"
 #include "tma_host.cuh"
 
+#include <type_traits>
+
 
 namespace {
 using namespace sm100;
@@ -464,37 +466,43 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                 if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_S + ss], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 14))) { alive = false; break; }
                 tc_fence_after_sync();
                 const bool diag = p.causal && (i == kt);
-                const bool edge = diag || !kv_valid;        // only the diagonal / tail tile pays for masking
+                const bool edge = diag || k0 + BT > p.T;    // warp-uniform
                 const uint32_t tm_s = tmem + TM_S + (NSB == 2 ? ss * 128u : 0u) + t_lane + CW * g;
                 uint32_t pk[CW / 2];                        // P^T row, CW query columns as f16 pairs
                 uint32_t sr[32];
                 tmem_ld_x32(tm_s, sr);
                 tmem_wait_ld();
-                // P^T replaces this warpgroup's part of S^T in TMEM, 16 columns (8 packed) at a time.
+                // P^T replaces this warpgroup's part of S^T in TMEM, 16 columns (8 packed) at a time.  Two copies of the loop:
+                // only the diagonal / tail tile pays for masking (predicated off, the masks still cost their issue slots).
+                auto make_p = [&](auto edge_c) {
+                    constexpr bool EDGE = decltype(edge_c)::value;
 #pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
+                    for (int hf = 0; hf < 2; ++hf) {
 #pragma unroll
-                    for (int e = hf * 4; e < hf * 4 + 4; ++e) {     // four columns
-                        const ulonglong2 nl = nlse2[e];
-                        float x0, x1, x2, x3;
-                        unpack_f32x2(fma2(pack_f32x2(sr[e * 4], sr[e * 4 + 1]), sl2_2, nl.x), x0, x1);
-                        unpack_f32x2(fma2(pack_f32x2(sr[e * 4 + 2], sr[e * 4 + 3]), sl2_2, nl.y), x2, x3);
-                        x0 = ex2(x0); x1 = ex2(x1); x2 = ex2(x2); x3 = ex2(x3);
-                        if (edge) {                         // query index < key index, or a key past the end: masked
-                            const int cl = CW * g + e * 4, lim = kv_valid ? r : 1 << 20;
-                            if (cl < lim) x0 = 0.f;
-                            if (cl + 1 < lim) x1 = 0.f;
-                            if (cl + 2 < lim) x2 = 0.f;
-                            if (cl + 3 < lim) x3 = 0.f;
+                        for (int e = hf * 4; e < hf * 4 + 4; ++e) {     // four columns
+                            const ulonglong2 nl = nlse2[e];
+                            float x0, x1, x2, x3;
+                            unpack_f32x2(fma2(pack_f32x2(sr[e * 4], sr[e * 4 + 1]), sl2_2, nl.x), x0, x1);
+                            unpack_f32x2(fma2(pack_f32x2(sr[e * 4 + 2], sr[e * 4 + 3]), sl2_2, nl.y), x2, x3);
+                            x0 = ex2(x0); x1 = ex2(x1); x2 = ex2(x2); x3 = ex2(x3);
+                            if (EDGE) {                     // query index < key index, or a key past the end: masked
+                                const int cl = CW * g + e * 4, lim = kv_valid ? (diag ? r : 0) : 1 << 20;
+                                if (cl < lim) x0 = 0.f;
+                                if (cl + 1 < lim) x1 = 0.f;
+                                if (cl + 2 < lim) x2 = 0.f;
+                                if (cl + 3 < lim) x3 = 0.f;
+                            }
+                            pk[e * 2] = pack_half2(x0, x1);
+                            pk[e * 2 + 1] = pack_half2(x2, x3);
                         }
-                        pk[e * 2] = pack_half2(x0, x1);
-                        pk[e * 2 + 1] = pack_half2(x2, x3);
+                        tmem_st_x8(tm_s + hf * 8, &pk[hf * 8]);
+                        tmem_wait_st();
+                        tc_fence_before_sync();
+                        mbar_arrive_warp(&bars[(hf ? A_P2 : A_P) + ss]);
                     }
-                    tmem_st_x8(tm_s + hf * 8, &pk[hf * 8]);
-                    tmem_wait_st();
-                    tc_fence_before_sync();
-                    mbar_arrive_warp(&bars[(hf ? A_P2 : A_P) + ss]);
-                }
+                };
+                if (edge) make_p(std::true_type{});
+                else make_p(std::false_type{});
                 if (it == 0 && !epilogue()) { alive = false; break; }      // the previous item's dK and dV
 
                 if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_DP], gi & 1u, DEERS_KERR_BWD_F16 | 15))) { alive = false; break; }
