@@ -3,28 +3,32 @@
 // Persistent kernel: one CTA per SM walks a strided, heaviest-first list of work items, an item
 // being 128 query rows of one (batch, head) slice together with the key/value tiles (128 rows
 // each) at or left of its diagonal.  The whole list is treated as ONE stream of (item, KV tile)
-// steps, so loads and the S product run two steps ahead across item boundaries.
-//   warp 0      TMA producer: Q per item (2 buffers), K and V tiles through 2-stage rings
-//   last warp   issues the S = Q K^T products into a double-buffered TMEM tile, two steps ahead
-//   warp 1      issues the O += P V products, with P read from TMEM and the accumulator resident
-//               in TMEM (two O accumulators alternate between items).  One thread cannot issue
-//               both streams fast enough: its barrier waits and commits between the batches of
-//               eight instructions left the tensor core idle a third of the time.  The two
-//               streams are ordered by barriers only (S of step g+2 overwrites P of step g once
-//               the product that read it has completed).
-//   warps 2-17  four softmax warpgroups that split the 128 key columns of a step (32 each); thread r
-//               of a warpgroup owns query row r (= TMEM lane r).  Per step a thread reads its 32
-//               scores, exchanges its partial row max with the twin threads of the other
-//               warpgroups, keeps the running max / partial sum, stores P (f16 pairs) back into
-//               TMEM over the scores it has just read, and rescales its quarter of O only when the
-//               row max grew by more than 2^8.  At the end of an item the partial sums are
-//               combined, O is normalised and O and the row lse are stored.
+// steps, so loads and the S product run ahead across item boundaries.
+//   warp 0      TMA producer: Q per item (2 buffers), K tiles through a 2-stage ring
+//   warp 3      the same for V, which waits for other products than K does
+//   warp 2      issues the S = Q K^T products into three TMEM tiles in turn
+//   warp 1      issues the O += P V products, with P read from TMEM and the accumulator resident in TMEM; a product starts
+//               on the first half of P's columns.  The two streams are ordered by barriers only (S of step g+3 overwrites
+//               P of step g once the product that read it has completed).
+//   softmax     four warpgroups in two groups: group g takes the steps of parity g (score tile g), its two warpgroups
+//               split the 128 key columns (64 each); thread r of a warpgroup owns query row r (= TMEM lane r).  The groups
+//               run half a step apart, so that one's exponentials fill the special-function unit (1024 cycles a
+//               step, as many as the tensor core needs) while the other loads scores, finds maxima and synchronises.  Per
+//               step a thread reads its 64 scores, exchanges its partial row max with its twin, takes the row's reference
+//               maximum from the group of the step before and publishes the new one, stores P (f16 pairs) back into
+//               TMEM over the scores, and rescales its half of O only when the row max grew by more than 2^8.  At the
+//               end of an item the partial sums are combined, O is normalised and O and the row lse are stored.
+//   What bounds it at D = 128, per 128 x 128 step: 1024 cycles each of tensor pipe and special-function unit, 1280 of
+//   shared memory.  With all sixteen softmax warps in step (one step at a time, 32 columns each) a step took 2170 cycles; two
+//   groups with two S tiles 2250 (a group then waits for P V of its last step and for S), with three 1720.  The loops are
+//   rolled to 32 columns: unrolled further, warps in different phases evict one another's code.
+//   B2 H16 T4096 D128: 247 k -> 197 k cycles per CTA; B16 H12 T1024 D64: 118 k -> 99 k.
 // Scale, causal mask, softmax and both products happen in this one pass; the T x T scores
 // never reach global memory.
 #include "sm100_ptx.cuh"
 #include "tma_host.cuh"
 
-
+#include <type_traits>
 
 namespace {
 using namespace sm100;
@@ -35,12 +39,10 @@ constexpr uint32_t BLOCK_BYTES = 128 * 128;   // one 64-column block of a 128-ro
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LN2 = 0.6931471805599453f;
 constexpr float RESCALE_THRESHOLD = 8.0f;     // log2 units: P stays below 2^8, safe in f16
-// Softmax warpgroups per CTA.  Four (32 key columns each) rather than two: the softmax threads are bound by
-// instruction latency, not by any one pipe, and four resident warps per scheduler hide it better than two.
-constexpr int NWG = 4;
-constexpr int CW = 128 / NWG;                 // key columns of a step per warpgroup
-constexpr int FWD_THREADS = 32 * (2 + 4 * NWG + 1);
-constexpr int S_WARP = 2 + 4 * NWG;           // the warp that issues S
+constexpr int NWG = 4;                        // softmax warpgroups: two groups of two
+constexpr int CW = 64;                        // key columns of a step per warpgroup
+constexpr int SM_WARP0 = 4;                   // first softmax warp; warps 0-3 are the Q / K producer, P V issuer, S issuer, V producer
+constexpr int FWD_THREADS = 32 * (SM_WARP0 + 4 * NWG);
 
 struct FwdParams {
     __half* o;
@@ -61,6 +63,12 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float y;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
+
 // Dynamic shared memory only; the base must be 1024-byte aligned for the 128-byte swizzle (checked).
 template <int D>
 struct FwdSmem {
@@ -68,20 +76,20 @@ struct FwdSmem {
     static constexpr uint32_t Q = 0;                         // two buffers (alternate between items)
     static constexpr uint32_t K = Q + 2 * TILE;              // two stages
     static constexpr uint32_t V = K + 2 * TILE;              // two stages
-    static constexpr uint32_t XCH = V + 2 * TILE;            // [2 parities][NWG warpgroups][128] partial row max
-    static constexpr uint32_t LX = XCH + 2 * NWG * BM * 4;   // [2 parities][NWG warpgroups][128] partial row sum
-    static constexpr uint32_t BARS = LX + 2 * NWG * BM * 4;
+    static constexpr uint32_t XCH = V + 2 * TILE;            // [2 groups][2 parities][2 warpgroups][128] partial row max
+    static constexpr uint32_t MREF = XCH + 8 * BM * 4;       // [2 groups][128] reference maximum after the group's last step
+    static constexpr uint32_t LX = MREF + 2 * BM * 4;        // [4 items][NWG warpgroups][2][128] partial row sum, its reference maximum
+    static constexpr uint32_t BARS = LX + 8 * NWG * BM * 4;
     static constexpr uint32_t TOTAL = BARS + 256;
 };
 
-// P_FULL is split by step parity: S runs two steps ahead of P V, so the softmax threads can hand over
-// P of steps g and g+1 before the MMA thread has looked at step g; one barrier per parity keeps each
-// barrier at most one phase ahead of its waiter.
+// P_FULL (first half of P's columns) and P2_FULL (second half), S_FULL and PV_DONE are one barrier per S tile, so that each
+// stays at most one phase ahead of its waiter.
 // S_FULL (all S products of a step have finished) also tells the producer that the step's K stage is
 // free; PV_DONE (all P V products of a step have finished) also frees the V stage, tells the S
 // issuer that the step's P has been consumed and orders a rescale of O behind the product.
-enum FwdBar { F_Q_FULL = 0, F_Q_EMPTY = 2, F_K_FULL = 4, F_V_FULL = 6, F_PV_DONE = 8, F_S_FULL = 10,
-              F_P_FULL = 12, F_XCH = 14, F_LX = 15, F_O_DONE = 16, F_O_FREE = 18, F_COUNT = 20 };
+enum FwdBar { F_Q_FULL = 0, F_Q_EMPTY = 2, F_K_FULL = 4, F_V_FULL = 6, F_PV_DONE = 8, F_S_FULL = 11,
+              F_P_FULL = 14, F_XCH = 17, F_MREF = 19, F_LX = 21, F_O_DONE = 22, F_O_FREE = 24, F_P2_FULL = 26, F_COUNT = 29 };
 
 // Work order: groups of 16 slices; inside a group the heaviest (latest) query tiles of all its
 // slices come first (balance) and the group's K and V (a few MB) stay in L2.
@@ -139,14 +147,17 @@ attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     constexpr int DBLK = D / 64;
     constexpr int DH = D / NWG;                              // O columns per softmax warpgroup
     constexpr uint32_t TMEM_COLS = 512;
-    // S of even steps (P in place) | S of odd steps | O of even items | O of odd items
-    constexpr uint32_t TM_S = 0, TM_O = 256;
+    // three S tiles in turn (P in place) | O, two at D = 64 (even and odd items).  A third S tile is worth more than a second O:
+    // with two, a group waits for P V of its last step and then for S before it can start the next.
+    constexpr uint32_t TM_S = 0, TM_O = 384;
+    constexpr int NOB = D == 64 ? 2 : 1;
 
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sQ = smem + L::Q;
     uint8_t* sK = smem + L::K;
     uint8_t* sV = smem + L::V;
     float* xch = reinterpret_cast<float*>(smem + L::XCH);
+    float* mref = reinterpret_cast<float*>(smem + L::MREF);
     float* lx = reinterpret_cast<float*>(smem + L::LX);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BARS);
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + F_COUNT);
@@ -168,13 +179,15 @@ attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         for (int s = 0; s < 2; ++s) {
             mbar_init(&bars[F_Q_FULL + s], 1); mbar_init(&bars[F_Q_EMPTY + s], 1);
             mbar_init(&bars[F_K_FULL + s], 1);
-            mbar_init(&bars[F_V_FULL + s], 1); mbar_init(&bars[F_PV_DONE + s], 1);
-            mbar_init(&bars[F_S_FULL + s], 1);
-            mbar_init(&bars[F_P_FULL + s], 128 * NWG);
-            mbar_init(&bars[F_O_DONE + s], 1); mbar_init(&bars[F_O_FREE + s], 128 * NWG);
+            mbar_init(&bars[F_V_FULL + s], 1);
+            mbar_init(&bars[F_O_DONE + s], 1); mbar_init(&bars[F_O_FREE + s], 4 * NWG);
+            mbar_init(&bars[F_XCH + s], 8); mbar_init(&bars[F_MREF + s], 4);
         }
-        mbar_init(&bars[F_XCH], 128 * NWG);
-        mbar_init(&bars[F_LX], 128 * NWG);
+        for (int s = 0; s < 3; ++s) {
+            mbar_init(&bars[F_S_FULL + s], 1); mbar_init(&bars[F_PV_DONE + s], 1);
+            mbar_init(&bars[F_P_FULL + s], 8); mbar_init(&bars[F_P2_FULL + s], 8); // one arrival per warp of the step's group
+        }
+        mbar_init(&bars[F_LX], 4 * NWG);
         fence_barrier_init();
         tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v);
     }
@@ -208,21 +221,13 @@ attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     }
                     __syncwarp();
                 }
-                const uint32_t st = g & 1u, ph = ((g >> 1) & 1u) ^ 1u;
-                if (!mbar_wait_warp(ws, &bars[F_S_FULL + st], ph, DEERS_KERR_FWD_F16 | 2)) break;      // S of step g-2 done
+                const uint32_t st = g & 1u;
+                if (g >= 2 && !mbar_wait_warp(ws, &bars[F_S_FULL + (g - 2u) % 3u], ((g - 2u) / 3u) & 1u, DEERS_KERR_FWD_F16 | 2)) break;      // S of step g-2 done
                 if (elect_one()) {
                     mbar_arrive_expect_tx(&bars[F_K_FULL + st], TILE_BYTES);
 #pragma unroll
                     for (int blk = 0; blk < DBLK; ++blk)
                         tma_load_4d(sK + st * TILE_BYTES + blk * BLOCK_BYTES, &tmap_k, &bars[F_K_FULL + st], blk * 64, c.j * BN, h, b);
-                }
-                __syncwarp();
-                if (!mbar_wait_warp(ws, &bars[F_PV_DONE + st], ph, DEERS_KERR_FWD_F16 | 3)) break;     // P V of step g-2 done
-                if (elect_one()) {
-                    mbar_arrive_expect_tx(&bars[F_V_FULL + st], TILE_BYTES);
-#pragma unroll
-                    for (int blk = 0; blk < DBLK; ++blk)
-                        tma_load_4d(sV + st * TILE_BYTES + blk * BLOCK_BYTES, &tmap_v, &bars[F_V_FULL + st], blk * 64, c.j * BN, h, b);
                 }
                 __syncwarp();
                 c.advance(p, nq, n_items);
@@ -237,28 +242,40 @@ attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             WorkCursor pc;
             pc.init(p, nq, n_items);
             for (uint32_t gp = 0; pc.valid(n_items); ++gp) {
-                const uint32_t st = gp & 1u;
-                if (!mbar_wait_warp(ws, &bars[F_P_FULL + st], (gp >> 1) & 1u, DEERS_KERR_FWD_F16 | 6)) break;
+                const uint32_t st = gp & 1u, sb = gp % 3u;
+                if (!mbar_wait_warp(ws, &bars[F_P_FULL + sb], (gp / 3u) & 1u, DEERS_KERR_FWD_F16 | 6)) break;
                 if (!mbar_wait_warp(ws, &bars[F_V_FULL + st], (gp >> 1) & 1u, DEERS_KERR_FWD_F16 | 7)) break;
-                // The accumulator of item n was last used by item n-2: its epilogue must be over.
-                if (pc.j == 0 && !mbar_wait_warp(ws, &bars[F_O_FREE + (pc.n & 1)], (((uint32_t)pc.n >> 1) & 1u) ^ 1u, DEERS_KERR_FWD_F16 | 8)) break;
+                // The epilogue of the item that last used the accumulator must be over.
+                if (pc.j == 0 && !mbar_wait_warp(ws, &bars[F_O_FREE + pc.n % NOB], ((uint32_t)(pc.n / NOB) & 1u) ^ 1u, DEERS_KERR_FWD_F16 | 8)) break;
                 tc_fence_after_sync();
                 const uint64_t v_mn = v_mn0 + (uint64_t)st * STAGE_STEP;
-                const uint32_t o_tmem = tmem + TM_O + (uint32_t)(pc.n & 1) * D;
-                const uint32_t p_tmem = tmem + TM_S + st * 128u;       // P sits where this step's S was
+                const uint32_t o_tmem = tmem + TM_O + (uint32_t)(pc.n % NOB) * D;
+                const uint32_t p_tmem = tmem + TM_S + sb * 128u;       // P sits where this step's S was
+                // A warpgroup hands over the first 32 of its 64 columns, then the other 32: the product starts on the first.
                 if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < BN / 16; ++ks)
-                        umma_ts(o_tmem, p_tmem + (uint32_t)(ks / (CW / 16)) * CW + (uint32_t)(ks % (CW / 16)) * 8u, v_mn + mnmajor_step(ks),
-                                IDESC_O, (pc.j > 0 || ks > 0));
-                    umma_commit(&bars[F_PV_DONE + st]);
-                    if (pc.j == pc.ntiles - 1) umma_commit(&bars[F_O_DONE + (pc.n & 1)]);
+                    for (int i = 0; i < 4; ++i) {
+                        const int ks = (i >> 1) * 4 + (i & 1);
+                        umma_ts(o_tmem, p_tmem + (uint32_t)(ks >> 2) * CW + (uint32_t)(ks & 3) * 8u, v_mn + mnmajor_step(ks), IDESC_O, (pc.j > 0 || i > 0));
+                    }
+                }
+                __syncwarp();
+                if (!mbar_wait_warp(ws, &bars[F_P2_FULL + sb], (gp / 3u) & 1u, DEERS_KERR_FWD_F16 | 6)) break;
+                tc_fence_after_sync();
+                if (elect_one()) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int ks = (i >> 1) * 4 + 2 + (i & 1);
+                        umma_ts(o_tmem, p_tmem + (uint32_t)(ks >> 2) * CW + (uint32_t)(ks & 3) * 8u, v_mn + mnmajor_step(ks), IDESC_O, 1u);
+                    }
+                    umma_commit(&bars[F_PV_DONE + sb]);
+                    if (pc.j == pc.ntiles - 1) umma_commit(&bars[F_O_DONE + pc.n % NOB]);
                 }
                 __syncwarp();
                 pc.advance(p, nq, n_items);
             }
         }
-    } else if (warp == S_WARP) {
+    } else if (warp == 2) {
         // ------------------------------ S issuer ------------------------------
         {
             constexpr uint32_t IDESC_S = idesc_f16(BM, BN, 0, 0);      // S: K-major A (Q) and B (K)
@@ -268,196 +285,242 @@ attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             WorkCursor sc;
             sc.init(p, nq, n_items);
             for (uint32_t gs = 0; sc.valid(n_items); ++gs) {
-                const uint32_t st = gs & 1u;
+                const uint32_t st = gs & 1u, sb = gs % 3u;
                 const int qb = sc.n & 1;
                 if (sc.j == 0 && !mbar_wait_warp(ws, &bars[F_Q_FULL + qb], ((uint32_t)sc.n >> 1) & 1u, DEERS_KERR_FWD_F16 | 4)) break;
                 if (!mbar_wait_warp(ws, &bars[F_K_FULL + st], (gs >> 1) & 1u, DEERS_KERR_FWD_F16 | 5)) break;
-                // This S tile still holds P of step gs-2 until the product reading it has finished.
-                if (!mbar_wait_warp(ws, &bars[F_PV_DONE + st], ((gs >> 1) & 1u) ^ 1u, DEERS_KERR_FWD_F16 | 0x15)) break;
+                // This S tile still holds P of step gs-3 until the product reading it has finished.
+                if (!mbar_wait_warp(ws, &bars[F_PV_DONE + sb], ((gs / 3u) & 1u) ^ 1u, DEERS_KERR_FWD_F16 | 0x15)) break;
                 tc_fence_after_sync();
                 const uint64_t q_km = q_km0 + (uint64_t)qb * STAGE_STEP, k_km = k_km0 + (uint64_t)st * STAGE_STEP;
-                const uint32_t d_tmem = tmem + TM_S + st * 128u;
+                const uint32_t d_tmem = tmem + TM_S + sb * 128u;
                 if (elect_one()) {
 #pragma unroll
                     for (int ks = 0; ks < D / 16; ++ks)
                         umma_ss(d_tmem, q_km + kmajor_step(ks, BLOCK_BYTES), k_km + kmajor_step(ks, BLOCK_BYTES), IDESC_S, ks > 0);
-                    umma_commit(&bars[F_S_FULL + st]);
+                    umma_commit(&bars[F_S_FULL + sb]);
                     if (sc.j == sc.ntiles - 1) umma_commit(&bars[F_Q_EMPTY + qb]); // last product reading this Q
                 }
                 __syncwarp();
                 sc.advance(p, nq, n_items);
             }
         }
-    } else if (warp < S_WARP) {
+    } else if (warp == 3) {
+        // ------------------------------ V producer ------------------------------
+        // A warp of its own: V of a step waits for P V two steps back, and K of the next step must not wait behind it.
+        WorkCursor c;
+        c.init(p, nq, n_items);
+        for (uint32_t g = 0; c.valid(n_items); ++g) {
+            const uint32_t st = g & 1u;
+            if (g >= 2 && !mbar_wait_warp(ws, &bars[F_PV_DONE + (g - 2u) % 3u], ((g - 2u) / 3u) & 1u, DEERS_KERR_FWD_F16 | 3)) break;
+            if (elect_one()) {
+                mbar_arrive_expect_tx(&bars[F_V_FULL + st], TILE_BYTES);
+#pragma unroll
+                for (int blk = 0; blk < DBLK; ++blk)
+                    tma_load_4d(sV + st * TILE_BYTES + blk * BLOCK_BYTES, &tmap_v, &bars[F_V_FULL + st], blk * 64, c.j * BN, c.h, c.b);
+            }
+            __syncwarp();
+            c.advance(p, nq, n_items);
+        }
+    } else if (warp >= SM_WARP0) {
         // ------------------------------ softmax + epilogue ------------------------------
-        const int g = (warp - 2) >> 2;                          // warpgroup: key columns [CW*g, CW*g + CW)
+        const int wg = (warp - SM_WARP0) >> 2;                  // 0..3
+        const int grp = wg >> 1, half = wg & 1;                 // steps of parity grp, key columns [64 half, 64 half + 64)
         const int lane_base = (warp & 3) * 32;
         const int row = lane_base + lane;                       // row inside the query tile == TMEM lane
         const uint32_t t_lane = (uint32_t)lane_base << 16;
         const float sl2 = p.scale * LOG2E;
-        uint32_t gstep = 0;                                     // global step counter
+        uint32_t gstep0 = 0;                                    // global step of the item's first KV tile
         bool alive = true;
 
         // Deferred epilogue of the previous item (runs after this item's first P has been handed over).
         int pend_n = -1, pend_grow = 0, pend_bh = 0, pend_b = 0, pend_h = 0;
-        float pend_m = 0.f, pend_l = 0.f;
         auto epilogue = [&]() -> bool {
             if (pend_n < 0) return true;
             const int n = pend_n;
             pend_n = -1;
-            // Combine the partial row sums of the warpgroups (published when the item's last step ended,
-            // so this wait has long been satisfied).
-            float* lxp = lx + (n & 1) * NWG * BM;
+            // Combine the partial row sums of the warpgroups, each relative to the reference maximum its group saw last; the
+            // largest of these is the one O is scaled by.
+            const float* lxp = lx + (n & 3) * 2 * NWG * BM + row;
             if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[F_LX], (uint32_t)n & 1u, DEERS_KERR_FWD_F16 | 9))) return false;
-            float l = 0.f;
+            float m = -INFINITY, l = 0.f;
 #pragma unroll
-            for (int w = 0; w < NWG; ++w) l += lxp[w * BM + row];        // same order in every warpgroup
-            if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[F_O_DONE + (n & 1)], ((uint32_t)n >> 1) & 1u, DEERS_KERR_FWD_F16 | 10))) return false;
+            for (int w = 0; w < NWG; ++w) m = fmaxf(m, lxp[(2 * w + 1) * BM]);
+            const float m_safe = (m == -INFINITY) ? 0.f : m;
+#pragma unroll
+            for (int w = 0; w < NWG; ++w) l = fmaf(lxp[2 * w * BM], ex2(lxp[(2 * w + 1) * BM] - m_safe), l);   // same order everywhere
+            if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[F_O_DONE + n % NOB], (uint32_t)(n / NOB) & 1u, DEERS_KERR_FWD_F16 | 10))) return false;
             tc_fence_after_sync();
             const float inv = 1.f / l;
-            const int b = pend_b, h = pend_h;
-            // The thread's half row of O, as 16-byte pieces, is transposed within lane groups so
-            // that every store instruction writes whole contiguous row segments.
+            // The thread's quarter row of O, as 16-byte pieces, is transposed within lane groups so that
+            // every store instruction writes whole contiguous row segments.
             constexpr int NP = DH / 8;
             uint4 oc[NP];
             {
                 uint32_t r[DH];
-                const uint32_t to = tmem + TM_O + (uint32_t)(n & 1) * D + t_lane + g * DH;
-                if constexpr (DH == 64) {
-                    tmem_ld_x32(to, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-                    tmem_ld_x32(to + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[DH - 32]));
-                } else if constexpr (DH == 32) {
-                    tmem_ld_x32(to, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-                } else {
-                    tmem_ld_x16(to, *reinterpret_cast<uint32_t(*)[16]>(&r[0]));
-                }
+                const uint32_t to = tmem + TM_O + (uint32_t)(n % NOB) * D + t_lane + wg * DH;
+                if constexpr (DH == 32) tmem_ld_x32(to, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+                else tmem_ld_x16(to, *reinterpret_cast<uint32_t(*)[16]>(&r[0]));
                 tmem_wait_ld();
                 tc_fence_before_sync();
-                mbar_arrive(&bars[F_O_FREE + (n & 1)]);         // accumulator is in registers: release it
+                mbar_arrive_warp(&bars[F_O_FREE + n % NOB]);    // accumulator is in registers: release it
 #pragma unroll
                 for (int q8 = 0; q8 < NP; ++q8) oc[q8] = pack8_f16(r + q8 * 8, inv);
             }
             transpose_pieces<NP>(oc, (uint32_t)lane);
             const int grow0 = pend_grow - lane + (lane & ~(NP - 1));
-            const int col = g * DH + (lane & (NP - 1)) * 8;
-            __half* ob = p.o + b * p.so_b + h * p.so_h + col;
+            const int col = wg * DH + (lane & (NP - 1)) * 8;
+            __half* ob = p.o + pend_b * p.so_b + pend_h * p.so_h + col;
 #pragma unroll
             for (int c = 0; c < NP; ++c) {
                 const int grow = grow0 + c;
                 if (grow < p.T && col < p.d) *reinterpret_cast<uint4*>(ob + (long long)grow * p.so_t) = oc[c];
             }
-            if (g == 0 && pend_grow < p.T) p.lse[(long long)pend_bh * p.T + pend_grow] = (pend_m + log2f(l)) * LN2;
+            if (wg == 0 && pend_grow < p.T) p.lse[(long long)pend_bh * p.T + pend_grow] = (m + log2f(l)) * LN2;
             return true;
         };
 
         WorkCursor c;
         c.init(p, nq, n_items);
-        while (alive && c.valid(n_items)) {
-            const int n = c.n, qt = c.qt, ntiles = c.ntiles, bh = c.bh;
+        // One more round than items, without steps, for the last epilogue: it has a single call site (and one in
+        // the rare rescale: its code four times over no longer fits the instruction cache).
+        for (;;) {
+            const bool valid = c.valid(n_items);
+            const int n = c.n, qt = c.qt, ntiles = valid ? c.ntiles : 0;
             const int q0 = qt * BM;
-            float m_used = -INFINITY, l = 0.f;                  // l: partial sum over this warpgroup's columns
-            for (int j = 0; j < ntiles; ++j, ++gstep) {
-                const uint32_t sb = gstep & 1u;
-                if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[F_S_FULL + sb], (gstep >> 1) & 1u, DEERS_KERR_FWD_F16 | 11))) { alive = false; break; }
-                tc_fence_after_sync();
-                float s[CW];
-                const uint32_t ts = tmem + TM_S + sb * 128u + t_lane + CW * g;
-#pragma unroll
-                for (int cc = 0; cc < CW / 32; ++cc) tmem_ld_x32(ts + cc * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[cc * 32]));
-                tmem_wait_ld();
-                // Steps that touch the diagonal or the end of the sequence are scaled here and
-                // masked with -inf; all others keep raw scores and fold the scale into the
-                // exponent's FFMA.
-                const int k0 = j * BN;
-                const bool edge = (p.causal && j == qt) || (k0 + BN > p.T);
-                float c1 = sl2;
-                if (edge) {
-                    // Column CW*g + i of this tile is valid iff i <= lim: on the diagonal tile (where
-                    // k0 == q0) the key may not lie right of the query, and keys end at T.
-                    int lim = p.T - 1 - k0 - CW * g;
-                    if (p.causal && j == qt) lim = min(lim, row - CW * g);
-#pragma unroll
-                    for (int i = 0; i < CW; ++i) s[i] = (i > lim) ? -INFINITY : s[i] * sl2;
-                    c1 = 1.0f;
-                }
-                float mx = s[0];
-                if (c1 >= 0.f) {
-#pragma unroll
-                    for (int i = 1; i < CW; ++i) mx = fmaxf(mx, s[i]);
-                } else {
-#pragma unroll
-                    for (int i = 1; i < CW; ++i) mx = fminf(mx, s[i]);
-                }
-                mx *= c1;
-                // Exchange the partial row max with the twin threads of the other warpgroups.
-                float* xp = xch + sb * NWG * BM;
-                xp[g * BM + row] = mx;
-                mbar_arrive(&bars[F_XCH]);
-                if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[F_XCH], gstep & 1u, DEERS_KERR_FWD_F16 | 12))) { alive = false; break; }
-#pragma unroll
-                for (int w = 0; w < NWG; ++w) mx = fmaxf(mx, xp[w * BM + row]);
-
-                const float m_new = fmaxf(m_used, mx);
-                // Lazy rescale: keep the old reference max unless this row grew by more than 2^8.
-                const bool grow = (j > 0) && (m_new - m_used > RESCALE_THRESHOLD);
-                const float m_cur = (j == 0 || grow) ? m_new : m_used;
-                const float m_safe = (m_cur == -INFINITY) ? 0.f : m_cur;
-                const float alpha = (j == 0) ? 0.f : ex2(m_used - m_safe);
-                const bool warp_grow = __any_sync(0xffffffffu, grow);
-
-                uint32_t pk[CW / 2];
-                float rs = 0.f;
-#pragma unroll
-                for (int i = 0; i < CW / 2; ++i) {
-                    const float e0 = ex2(fmaf(s[2 * i], c1, -m_safe));
-                    const float e1 = ex2(fmaf(s[2 * i + 1], c1, -m_safe));
-                    rs += e0 + e1;
-                    pk[i] = pack_half2(e0, e1);
-                }
-                l = l * alpha + rs;
-                m_used = m_cur;
-
-                if (j > 0 && warp_grow) {
-                    // O += P V of the previous step must have landed before O is rescaled.
-                    if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[F_PV_DONE + ((gstep - 1u) & 1u)], ((gstep - 1u) >> 1) & 1u, DEERS_KERR_FWD_F16 | 13))) { alive = false; break; }
+            float m_seen = -INFINITY, l = 0.f;                  // l: partial sum over this warpgroup's columns, relative to 2^m_seen
+            for (int j = (int)((gstep0 ^ (uint32_t)grp) & 1u); alive; j += 2) {
+                if (j < ntiles) {
+                    const uint32_t gstep = gstep0 + (uint32_t)j;    // gstep & 1 == grp
+                    const uint32_t ph = (gstep >> 1) & 1u, sb = gstep % 3u;
+                    if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[F_S_FULL + sb], (gstep / 3u) & 1u, DEERS_KERR_FWD_F16 | 11))) { alive = false; break; }
                     tc_fence_after_sync();
-                    const uint32_t to = tmem + TM_O + (uint32_t)(n & 1) * D + t_lane + g * DH;
-                    if constexpr (DH % 32 == 0) {
+                    const uint32_t ts = tmem + TM_S + sb * 128u + t_lane + CW * half;
+                    // Column CW*half + i of this tile is valid iff i <= lim: on the diagonal tile (where k0 == q0) the key may not
+                    // lie right of the query, and keys end at T.
+                    const int k0 = j * BN;
+                    const bool edge = (p.causal && j == qt) || (k0 + BN > p.T);
+                    int lim = edge ? p.T - 1 - k0 - CW * half : CW;
+                    if (p.causal && j == qt) lim = min(lim, row - CW * half);
+                    // Two sweeps over the scores, 32 at a time: a row's 64 scores and their exponentials do not fit in 96 registers,
+                    // and reading TMEM again is cheaper than spilling.
+                    // Two copies of each loop: only the diagonal / tail tile pays for masking.
+                    float mx = -INFINITY;
+                    auto row_max = [&](auto edge_c) {
+                        constexpr bool EDGE = decltype(edge_c)::value;
+#pragma unroll 1
+                        for (int q = 0; q < CW / 32; ++q) {
+                            float s[32];
+                            tmem_ld_x32(ts + q * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
+                            tmem_wait_ld();
+                            if (EDGE) {
 #pragma unroll
-                        for (int cc = 0; cc < DH / 32; ++cc) {
+                                for (int i = 0; i < 32; ++i) s[i] = (i > lim - q * 32) ? -INFINITY : s[i] * sl2;
+                            }
+                            float m4[4] = {mx, s[0], s[1], s[2]};                // four chains: a single one is latency-bound
+#pragma unroll
+                            for (int i = 3; i < 31; i += 2) m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], s[i], s[i + 1]);
+                            mx = max3(max3(m4[0], m4[1], m4[2]), m4[3], s[31]);
+                        }
+                    };
+                    if (edge || sl2 < 0.f) row_max(std::true_type{});
+                    else { row_max(std::false_type{}); mx *= sl2; }
+                    // The reference maximum after the previous step, which the other group took.  Read before this warp's arrival
+                    // below: this group publishes its own after that exchange, and the other group may write again only then.
+                    float m_prev = -INFINITY;
+                    if (gstep > 0) {
+                        const uint32_t g1 = gstep - 1u;
+                        if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[F_MREF + (g1 & 1u)], (g1 >> 1) & 1u, DEERS_KERR_FWD_F16 | 14))) { alive = false; break; }
+                        if (j > 0) m_prev = mref[(g1 & 1u) * BM + row];
+                    }
+                    // Exchange the partial row max with the twin thread of the other warpgroup.
+                    float* xp = xch + (grp * 2 + ph) * 2 * BM + row;
+                    xp[half * BM] = mx;
+                    mbar_arrive_warp(&bars[F_XCH + grp]);
+                    if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[F_XCH + grp], ph, DEERS_KERR_FWD_F16 | 12))) { alive = false; break; }
+                    mx = fmaxf(mx, xp[(half ^ 1) * BM]);
+
+                    const float m_new = fmaxf(m_prev, mx);
+                    // Lazy rescale: keep the old reference max unless this row grew by more than 2^8.
+                    const bool grow = (j > 0) && (m_new - m_prev > RESCALE_THRESHOLD);
+                    const float m_cur = (j == 0 || grow) ? m_new : m_prev;
+                    if (half == 0) {
+                        mref[grp * BM + row] = m_cur;
+                        mbar_arrive_warp(&bars[F_MREF + grp]);
+                    }
+                    const float m_safe = (m_cur == -INFINITY) ? 0.f : m_cur;
+                    const bool warp_grow = __any_sync(0xffffffffu, grow);
+                    l *= ex2(m_seen - m_safe);                      // 0 * 0 the first time
+                    m_seen = m_cur;
+
+                    if (j > 0 && warp_grow) {
+                        // O += P V of the previous step must have landed before O is rescaled.  That product may be the item's
+                        // first and wait for the previous item's O tile to leave, which is then due here.
+                        if (!epilogue()) { alive = false; break; }
+                        const float alpha = ex2(m_prev - m_safe);
+                        const uint32_t g1 = gstep - 1u;
+                        if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[F_PV_DONE + g1 % 3u], (g1 / 3u) & 1u, DEERS_KERR_FWD_F16 | 13))) { alive = false; break; }
+                        tc_fence_after_sync();
+                        const uint32_t to = tmem + TM_O + (uint32_t)(n % NOB) * D + t_lane + half * (D / 2);
+#pragma unroll 1
+                        for (int cc = 0; cc < D / 2; cc += 32) {
                             uint32_t r[32];
-                            tmem_ld_x32(to + cc * 32, r);
+                            tmem_ld_x32(to + cc, r);
                             tmem_wait_ld();
 #pragma unroll
                             for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-                            tmem_st_x32(to + cc * 32, r);
+                            tmem_st_x32(to + cc, r);
                         }
-                    } else {
-                        uint32_t r[16];
-                        tmem_ld_x16(to, r);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-                        tmem_st_x16(to, r);
                     }
+
+                    const uint64_t c1_2 = pack_f32x2(sl2, sl2), nm_2 = pack_f32x2(-m_safe, -m_safe);
+                    uint64_t rs = 0;
+                    auto make_p = [&](auto edge_c) {
+                        constexpr bool EDGE = decltype(edge_c)::value;
+#pragma unroll 1
+                        for (int q = 0; q < CW / 32; ++q) {
+                            uint32_t sr[32], pk[16];
+                            tmem_ld_x32(ts + q * 32, sr);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) {
+                                float e0, e1;
+                                unpack_f32x2(fma2(pack_f32x2(sr[2 * i], sr[2 * i + 1]), c1_2, nm_2), e0, e1);
+                                e0 = ex2(e0); e1 = ex2(e1);
+                                if (EDGE) {
+                                    if (2 * i > lim - q * 32) e0 = 0.f;
+                                    if (2 * i + 1 > lim - q * 32) e1 = 0.f;
+                                }
+                                rs = add2(rs, pack_f32x2(e0, e1));
+                                pk[i] = pack_half2(e0, e1);
+                            }
+                            // P replaces scores that have been read (32 packed columns, 16 at a time).
+                            tmem_st_x16(ts + q * 16, pk);
+                            tmem_wait_st();
+                            tc_fence_before_sync();
+                            mbar_arrive_warp(&bars[F_P_FULL + sb + q * (F_P2_FULL - F_P_FULL)]);
+                        }
+                    };
+                    if (edge) make_p(std::true_type{});
+                    else make_p(std::false_type{});
+                    float r0, r1;
+                    unpack_f32x2(rs, r0, r1);
+                    l += r0 + r1;
                 }
-                // P replaces this warpgroup's part of S in TMEM (CW / 2 packed columns).
-                if constexpr (CW == 64) tmem_st_x32(ts, *reinterpret_cast<uint32_t(*)[32]>(&pk[0]));
-                else tmem_st_x16(ts, *reinterpret_cast<uint32_t(*)[16]>(&pk[0]));
-                tmem_wait_st();
-                tc_fence_before_sync();
-                mbar_arrive(&bars[F_P_FULL + sb]);
-                if (j == 0 && !epilogue()) { alive = false; break; }          // previous item's O tile
+                // the previous item's O tile, after this item's first P (or right away: an item without a step of this group)
+                if (!epilogue()) { alive = false; break; }
+                if (j + 2 >= ntiles) break;
             }
-            if (!alive) break;
-            pend_n = n; pend_grow = q0 + row; pend_bh = bh; pend_b = c.b; pend_h = c.h; pend_m = m_used; pend_l = l;
-            lx[(n & 1) * NWG * BM + g * BM + row] = l;                       // partial row sum for the epilogue
-            mbar_arrive(&bars[F_LX]);
+            if (!alive || !valid) break;
+            pend_n = n; pend_grow = q0 + row; pend_bh = c.bh; pend_b = c.b; pend_h = c.h;
+            float* lxp = lx + (n & 3) * 2 * NWG * BM + 2 * wg * BM + row;     // partial row sum for the epilogue
+            lxp[0] = l; lxp[BM] = m_seen;
+            mbar_arrive_warp(&bars[F_LX]);
+            gstep0 += (uint32_t)ntiles;
             // advance the cursor by a whole item
             c.j = ntiles - 1;
             c.advance(p, nq, n_items);
         }
-        if (alive) epilogue();
     }
 
     __syncwarp();

@@ -123,3 +123,27 @@ def test_gpt_forward_lengths_share_graphs_and_follow_the_weights():
     params = ref.gpt_init_params(cfg, seed=5)
     m.load_parameters(params)
     check(42), check(31)
+
+
+@pytest.mark.parametrize("B,H,T,D,causal", [(4, 100, 100, 64, True), (3, 133, 60, 128, True), (2, 149, 129, 64, True), (1, 200, 385, 128, True),
+                                            (5, 60, 250, 128, False), (1, 3, 1025, 64, False)])
+def test_f16_attention_short_items_in_a_row(B, H, T, D, causal):
+    """Every SM walks several items of one, two, three ... key tiles: items without a step of one softmax group, odd and even
+    step counts, the deferred epilogues.  Keys grow along the sequence, so the reference maximum moves by more than 2^8
+    and O is rescaled by either group."""
+    from deers_b200 import ops
+    from oracle import ref
+    rng = np.random.default_rng(T)
+    host = [rng.standard_normal((B, H, T, D)).astype(np.float32) for _ in range(4)]
+    host[1] *= (1.0 + 3.0 * (np.arange(T) // 128))[None, None, :, None]
+    host = [a.astype(np.float16).astype(np.float32) for a in host]
+    q, k, v, do = (torch.from_numpy(a).to("cuda", torch.float16) for a in host)
+    scale = ops.default_scale(D)
+    o, lse = ops.attention_fwd(q, k, v, scale, causal)
+    grads = [ops.attention_bwd(q, k, v, o, lse, do, scale, causal, workspace=torch.empty(ops.workspace_bytes(q, scale, causal, p),
+                                                                                         dtype=torch.uint8, device="cuda")) for p in (1, 2)]
+    ops.Context.current(q.device).sync()
+    want = ref.attn_fwd_bwd(*host, causal=causal)
+    for got in grads:
+        for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), (o, lse) + tuple(got), want):
+            assert_close(g.float().cpu().numpy(), w, TOL_F16, name)
