@@ -108,13 +108,13 @@ struct Operand {
         }
     }
     // Index inside the tile of element i of thread group coordinate t: contiguous groups of four for MN order (one
-    // LDS.128 per four), interleaved for K order (one LDS.128 per row and four k).
+    // LDS.128 per four; the last two of six are a group of two), interleaved for K order (one LDS.128 per row and four k).
     template <int P>
     static __device__ __forceinline__ int index(int t, int i) {
         constexpr int G = R / P;                                   // thread groups along this side
         if (!MN) return t + G * i;
-        if (P >= 4) return (i / 4) * (4 * G) + t * 4 + (i % 4);
-        return t * P + i;
+        const int q = i / 4 * 4, w = P - q >= 4 ? 4 : P - q;       // first element and width of i's group
+        return q * G + t * w + (i - q);
     }
     // The P elements of this thread: K order reads four k at a time (v[i][kk]), MN order one k at a time (v[i][0]).
     static constexpr int KV = MN ? 1 : 4;
@@ -126,15 +126,17 @@ struct Operand {
                 const float4 x = *reinterpret_cast<const float4*>(s + index<P>(t, i) * LD + k);
                 v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
             }
-        } else if constexpr (P >= 4) {
+        } else {
 #pragma unroll
             for (int i = 0; i < P; i += 4) {
-                const float4 x = *reinterpret_cast<const float4*>(s + k * LD + index<P>(t, i));
-                v[i][0] = x.x; v[i + 1][0] = x.y; v[i + 2][0] = x.z; v[i + 3][0] = x.w;
+                if (P - i >= 4) {
+                    const float4 x = *reinterpret_cast<const float4*>(s + k * LD + index<P>(t, i));
+                    v[i][0] = x.x; v[i + 1][0] = x.y; v[i + 2][0] = x.z; v[i + 3][0] = x.w;
+                } else {
+                    const float2 x = *reinterpret_cast<const float2*>(s + k * LD + index<P>(t, i));
+                    v[i][0] = x.x; v[i + 1][0] = x.y;
+                }
             }
-        } else {
-            const float2 x = *reinterpret_cast<const float2*>(s + k * LD + index<P>(t, 0));
-            v[0][0] = x.x; v[1][0] = x.y;
         }
     }
 };
@@ -218,10 +220,13 @@ __global__ void __launch_bounds__(128 * KS) gemm_f32_kernel(const GemmArgs g) {
 #pragma unroll
     for (int i = 0; i < PM; ++i) {
         float* row = red + (kg * BM + S::OA::template index<PM>(ty, i)) * S::RLD;
-        if constexpr (B_MN && PN >= 4) {
+        if constexpr (B_MN) {
 #pragma unroll
-            for (int j = 0; j < PN; j += 4)
-                *reinterpret_cast<float4*>(row + S::OB::template index<PN>(tx, j)) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+            for (int j = 0; j < PN; j += 4) {
+                float* q = row + S::OB::template index<PN>(tx, j);
+                if (PN - j >= 4) *reinterpret_cast<float4*>(q) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+                else *reinterpret_cast<float2*>(q) = make_float2(acc[i][j], acc[i][j + 1]);
+            }
         } else {
 #pragma unroll
             for (int j = 0; j < PN; ++j) row[S::OB::template index<PN>(tx, j)] = acc[i][j];
@@ -303,9 +308,11 @@ struct GemmPlan {
 };
 
 // Tile variants with what was measured of them (cycles at 1.965 GHz, from products of several K in a graph): a
-// block's walk over 64 k, and what a launch costs around it.
+// block's walk over 64 k, and what a launch costs around it.  The 96-wide tiles are there for products whose 64-wide tiles
+// just miss one wave (1024 x 768: 192 tiles on 148 SMs, 128 of 64 x 96; 13.3 -> 11.7 us at K = 192, and 16.3 -> 13.7 for
+// 1024 x 192 x 768 in clusters of four).
 struct Variant { int bm, bn; double walk, around; };
-constexpr Variant kVariants[4] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {32, 64, 2360, 4000}, {32, 32, 1680, 3200}};
+constexpr Variant kVariants[6] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {32, 64, 2360, 4000}, {32, 32, 1680, 3200}, {64, 96, 5400, 5300}, {32, 96, 3200, 4300}};
 
 // How many clusters of 1..MAX_PARTS blocks (one block per SM) the device holds at a time: a cluster lives inside one
 // GPC, so e.g. 48 clusters of three do not fit 148 SMs although their 144 blocks would.
@@ -337,7 +344,7 @@ GemmPlan plan_gemm(int M, int N, int K, const int* capacity) {
     GemmPlan best{};
     double best_cost = -1.0;
     const int steps = (K + BK - 1) / BK;
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < 6; ++c) {
         const Variant& v = kVariants[c];
         const long long tm = (M + v.bm - 1) / v.bm, tn = (N + v.bn - 1) / v.bn;
         for (int parts = 1; parts <= MAX_PARTS; ++parts) {
@@ -404,7 +411,9 @@ int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long lo
         if (p.cfg == 0) rc = launch_orders<8, 8, 2>(ctx, p, g, a_mn, b_mn);
         else if (p.cfg == 1) rc = launch_orders<8, 4, 4>(ctx, p, g, a_mn, b_mn);
         else if (p.cfg == 2) rc = launch_orders<4, 4, 4>(ctx, p, g, a_mn, b_mn);
-        else rc = launch_orders<4, 2, 4>(ctx, p, g, a_mn, b_mn);
+        else if (p.cfg == 3) rc = launch_orders<4, 2, 4>(ctx, p, g, a_mn, b_mn);
+        else if (p.cfg == 4) rc = launch_orders<8, 6, 4>(ctx, p, g, a_mn, b_mn);
+        else rc = launch_orders<4, 6, 4>(ctx, p, g, a_mn, b_mn);
     }
     ctx->launches += 1;
     return rc;
