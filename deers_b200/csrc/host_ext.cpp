@@ -251,10 +251,14 @@ PyObject* attn_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
     at::Tensor o = empty_like_of(q->sizes(), q->scalar_type(), *q), lse;
     if (want_lse) lse = empty_like_of(q->sizes().slice(0, 3), at::kFloat, *q);
     put_strides(d.q_strides, *q); put_strides(d.k_strides, *k); put_strides(d.v_strides, *v); put_strides(d.o_strides, o);
-    const size_t need = deers_b200_attn_decode_workspace_bytes(&d);
-    at::Tensor ws = scratch(need < 256 ? 256 : need, *q);
-    const int rc = deers_b200_attn_decode(ctx, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o.data_ptr(),
-                                          want_lse ? (float*)lse.data_ptr() : nullptr, ws.data_ptr(), need);
+    // most calls need no workspace (the chunks of a slice meet in shared memory): ask for one only when told so
+    float* lse_p = want_lse ? (float*)lse.data_ptr() : nullptr;
+    int rc = deers_b200_attn_decode(ctx, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o.data_ptr(), lse_p, nullptr, 0);
+    if (rc == DEERS_ERR_WORKSPACE) {
+        const size_t need = deers_b200_attn_decode_workspace_bytes(&d);
+        at::Tensor ws = scratch(need < 256 ? 256 : need, *q);
+        rc = deers_b200_attn_decode(ctx, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o.data_ptr(), lse_p, ws.data_ptr(), need);
+    }
     if (rc) return fail(rc, ctx);
     if (!want_lse) return THPVariable_Wrap(std::move(o));
     return wrap2(std::move(o), std::move(lse));

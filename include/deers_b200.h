@@ -311,7 +311,8 @@ int deers_b200_rmsnorm_bwd(deers_ctx* ctx, int64_t rows, int32_t C, const float*
  * elements, inner stride 1 (a cache allocated for more than Tk rows is passed with its own row / slice
  * strides).  f16 or f32 storage, f32 arithmetic; D <= 256, Tq <= 128, B*H <= 65535.  lse (optional, [B,H,Tq]
  * f32, natural log) like deers_b200_attn_fwd.  Workspace: deers_b200_attn_decode_workspace_bytes(desc)
- * of device memory.  Enqueued on the context's stream; no allocation, no synchronisation.
+ * of device memory; a call that does not need it (caches up to 8192 rows, or slices enough to fill the device, with rows of
+ * aligned 16-byte pieces) takes NULL, any other answers DEERS_ERR_WORKSPACE without one.  Enqueued on the context's stream; no allocation, no synchronisation.
  */
 typedef struct deers_decode_desc {
     int32_t B, H, Tq, Tk, D;

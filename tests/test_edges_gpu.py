@@ -147,3 +147,26 @@ def test_f16_attention_short_items_in_a_row(B, H, T, D, causal):
     for got in grads:
         for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), (o, lse) + tuple(got), want):
             assert_close(g.float().cpu().numpy(), w, TOL_F16, name)
+
+
+@pytest.mark.parametrize("B,H,Tq,Tk,D", [(1, 2, 1, 64, 64), (1, 2, 1, 65, 80), (1, 3, 2, 513, 96), (2, 1, 5, 4096, 32), (1, 1, 3, 4097, 80),
+                                         (1, 2, 1, 20001, 128), (1, 2, 7, 7, 48), (60, 12, 1, 130, 72), (1, 1, 9, 300, 256), (75, 8, 3, 50, 24)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_decode_chunks_clusters_and_row_lengths(B, H, Tq, Tk, D, dtype):
+    """One chunk, a cluster of chunks, chunks merged by a second launch; rows of any number of 16-byte pieces; chunks that a
+    causal query does not see."""
+    from deers_b200 import ops
+    from oracle import ref
+    from tests.helpers import TOL_F32
+    rng = np.random.default_rng(Tk + D)
+    q, k, v = (rng.standard_normal((B, H, t, D)).astype(np.float32) for t in (Tq, Tk, Tk))
+    if dtype == torch.float16:
+        q, k, v = (a.astype(np.float16).astype(np.float32) for a in (q, k, v))
+    tq, tk, tv = (torch.from_numpy(a).to("cuda", dtype) for a in (q, k, v))
+    for causal in (True, False):
+        want_o, want_lse = ref.attn_decode(q, k, v, None, causal)
+        o, lse = ops.attention_decode(tq, tk, tv, causal=causal, want_lse=True)
+        ops.Context.current(tq.device).sync()
+        tol = TOL_F16 if dtype == torch.float16 else TOL_F32
+        assert_close(o.float().cpu().numpy(), want_o, tol, "o")
+        assert_close(lse.cpu().numpy(), want_lse, tol, "lse")
