@@ -59,6 +59,7 @@ struct deers_ctx {
     cudaStream_t h2d_stream, d2h_stream;
     cudaEvent_t pipe_ev[3][3];      // [buffer set][h2d done, compute done, d2h done]
     bool pipe_ready;
+    int cluster_room_f16[9];        // the same for the f16 GEMM's CTAs (gemm_f16_sm100.cu)
     int cluster_capacity[9];        // [n]: clusters of n blocks the device holds at once (gemm_f32.cu; 0: not asked yet)
 };
 

@@ -170,3 +170,21 @@ def test_decode_chunks_clusters_and_row_lengths(B, H, Tq, Tk, D, dtype):
         tol = TOL_F16 if dtype == torch.float16 else TOL_F32
         assert_close(o.float().cpu().numpy(), want_o, tol, "o")
         assert_close(lse.cpu().numpy(), want_lse, tol, "lse")
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 8, 8), (128, 256, 512), (136, 200, 520), (768, 768, 8192), (120, 184, 8200), (1024, 776, 768),
+                                   (2000, 2312, 72), (264, 1040, 2056), (128, 8, 1288)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+def test_f16_gemm_split_k_and_tile_widths(M, N, K, a_mn, b_mn):
+    """One tile per cluster with its K shared out (parts of unequal length), 192- and 256-wide tiles, ragged edges.  Small
+    integers: every sum is exact in f32 and f16, so any K range dropped or counted twice shows."""
+    from deers_b200 import ops
+    rng = np.random.default_rng(M + N + K)
+    a = rng.integers(-1, 2, (K, M) if a_mn else (M, K)).astype(np.float16)
+    b = rng.integers(-1, 2, (K, N) if b_mn else (N, K)).astype(np.float16)
+    got = ops._gemm(M, N, K, torch.from_numpy(a).cuda(), int(a_mn), torch.from_numpy(b).cuda(), int(b_mn))
+    ops.Context.current(got.device).sync()
+    af, bf = a.astype(np.float64), b.astype(np.float64)
+    want = (af.T if a_mn else af) @ (bf if b_mn else bf.T)
+    assert np.abs(want).max() <= 2048
+    assert np.array_equal(got.float().cpu().numpy(), want.astype(np.float32))
