@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
 attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                          const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                          const BwdParams p) {
+    chain_wait();
     using L = DkvSmem<D>;
     constexpr uint32_t TILE_BYTES = L::TILE;
     constexpr int DBLK = D / 64;
@@ -278,6 +279,8 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                 bulk_wait_group<0>();
             }
         }
+        __syncwarp();
+        chain_next();                                           // all loads are under way: the end is near
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp runs this; one elected lane issues (see elect_one).
@@ -574,6 +577,7 @@ __global__ void __launch_bounds__(320, 1)
 attn_bwd_dq_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                        const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                        const BwdParams p) {
+    chain_wait();
     using L = DqSmem<D>;
     constexpr uint32_t TILE_BYTES = L::TILE;
     constexpr int DBLK = D / 64;
@@ -664,6 +668,8 @@ attn_bwd_dq_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 }
             }
         }
+        __syncwarp();
+        chain_next();                                           // all loads are under way: the end is near
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp runs this; one elected lane issues (see elect_one).
@@ -890,6 +896,7 @@ enum DqsBar { R_FULL = 0, R_EMPTY = 3, R_ACC_FULL = 6, R_ACC_EMPTY = 8, R_COUNT 
 template <int D>
 __global__ void __launch_bounds__(192, 1)
 attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const BwdParams p) {
+    chain_wait();
     using L = DqsSmem<D>;
     constexpr int DBLK = D / 64;
     constexpr uint32_t TMEM_COLS = 2 * D;                    // 128 or 256: a power of two
@@ -955,6 +962,8 @@ attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const
                 }
             }
         }
+        __syncwarp();
+        chain_next();                                           // all loads are under way: the end is near
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp runs this; one elected lane issues (see elect_one).
@@ -1037,6 +1046,7 @@ attn_bwd_prep_f16_kernel(const __half* __restrict__ o, const __half* __restrict_
                          float* __restrict__ delta, float* __restrict__ lse2, int B, int H, int T, int d, int Tpad,
                          long long so_b, long long so_h, long long so_t, long long sdo_b, long long sdo_h,
                          long long sdo_t) {
+    chain_begin();
     constexpr int LPR = D / 8;                               // lanes per row
     constexpr int RPW = 32 / LPR;                            // rows per warp load
     constexpr int U = 4;                                     // loads in flight per lane and tensor
@@ -1113,7 +1123,7 @@ int bwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
         const long long per_block = 8LL * 4 * (256 / D);           // 8 warps x 4 loads x rows per load
         const long long want = (prep_rows + per_block - 1) / per_block;
         const unsigned prep_grid = (unsigned)(want < 8LL * ctx->sm_count ? want : 8LL * ctx->sm_count);
-        attn_bwd_prep_f16_kernel<D><<<prep_grid, 256, 0, ctx->stream>>>(
+        launch_chained(ctx, attn_bwd_prep_f16_kernel<D>, prep_grid, 256, 0, 1,
             (const __half*)o, (const __half*)d_o, lse, delta, lse2, d->B, d->H, d->T, d->D, Tpad, d->o_strides[0],
             d->o_strides[1], d->o_strides[2], d->do_strides[0], d->do_strides[1], d->do_strides[2]);
     }
@@ -1137,19 +1147,20 @@ int bwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
     const size_t smem_a = DkvSmem<D>::TOTAL, smem_b = DqSmem<D>::TOTAL;
     DEERS_SMEM_ONCE(ctx, (attn_bwd_dkdv_f16_kernel<D>), smem_a);
     DEERS_SMEM_ONCE(ctx, (attn_bwd_dq_f16_kernel<D>), smem_b);
+    const ChainScope chain(ctx, BH * p.ds_pairs / persistent);
     {
         KernelTimerScope ts(ctx, DEERS_K_BWD_MAIN);
-        attn_bwd_dkdv_f16_kernel<D><<<persistent, DKV_THREADS, smem_a, ctx->stream>>>(tq, tk, tv, tdo, p);
+        launch_chained(ctx, attn_bwd_dkdv_f16_kernel<D>, persistent, DKV_THREADS, smem_a, 1, tq, tk, tv, tdo, p);
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     if (keep_ds) {
         const size_t smem_c = DqsSmem<D>::TOTAL;
         DEERS_SMEM_ONCE(ctx, (attn_bwd_dq_from_ds_f16_kernel<D>), smem_c);
         KernelTimerScope ts(ctx, DEERS_K_BWD_DQ);
-        attn_bwd_dq_from_ds_f16_kernel<D><<<persistent, 192, smem_c, ctx->stream>>>(tk, p);
+        launch_chained(ctx, attn_bwd_dq_from_ds_f16_kernel<D>, persistent, 192, smem_c, 1, tk, p);
     } else {
         KernelTimerScope ts(ctx, DEERS_K_BWD_DQ);
-        attn_bwd_dq_f16_kernel<D><<<persistent, 320, smem_b, ctx->stream>>>(tq, tk, tv, tdo, p);
+        launch_chained(ctx, attn_bwd_dq_f16_kernel<D>, persistent, 320, smem_b, 1, tq, tk, tv, tdo, p);
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     ctx->launches += 3;

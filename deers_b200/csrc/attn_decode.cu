@@ -47,6 +47,7 @@ __device__ __forceinline__ void st(__half* p, float v) { *p = __float2half_rn(v)
 
 template <typename T>
 __global__ void __launch_bounds__(128) decode_partial_kernel(const DecodeParams p) {
+    chain_begin();
     const int split = blockIdx.x, bh = blockIdx.y;
     const int b = bh / p.H, h = bh % p.H;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -152,6 +153,7 @@ enum DecodeEnd { DEC_TO_WORKSPACE = 0, DEC_ONE_CHUNK = 1, DEC_CLUSTER = 2 };   /
 // Tk2048 D128 takes 336 us instead of 323.
 template <typename T, int LPK, int END>
 __global__ void __launch_bounds__(128, END == DEC_CLUSTER ? 6 : 7) decode_vec_kernel(const DecodeParams p) {
+    chain_wait();
     constexpr int VEC = 16 / (int)sizeof(T);                     // channels per lane
     constexpr int KPW = 32 / LPK;                                // keys per warp instruction
     constexpr int U = 4;                                         // key groups in flight
@@ -257,6 +259,7 @@ __global__ void __launch_bounds__(128, END == DEC_CLUSTER ? 6 : 7) decode_vec_ke
         }
         __syncthreads();
         if (lane == 0) { sm_m[warp] = m; sm_l[warp] = l; }
+        if (i == p.Tq - 1) chain_next();
         if (sub == 0 && mine) {
 #pragma unroll
             for (int c = 0; c < VEC; ++c) sm_o[warp][cl * VEC + c] = acc[c];
@@ -328,6 +331,7 @@ __global__ void __launch_bounds__(128, END == DEC_CLUSTER ? 6 : 7) decode_vec_ke
 
 template <typename T>
 __global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams p) {
+    chain_begin();
     const long long row = blockIdx.x;                                        // (bh, i)
     const int bh = (int)(row / p.Tq), i = (int)(row % p.Tq);
     const int b = bh / p.H, h = bh % p.H;
@@ -433,19 +437,11 @@ extern "C" size_t deers_b200_attn_decode_workspace_bytes(const deers_decode_desc
 template <typename T, int LPK>
 static int decode_launch_vec(deers_ctx* ctx, const DecodeParams& p, const dim3& grid, bool cluster) {
     if (!cluster || p.splits == 1) {
-        if (cluster) decode_vec_kernel<T, LPK, DEC_ONE_CHUNK><<<grid, 128, 0, ctx->stream>>>(p);
-        else decode_vec_kernel<T, LPK, DEC_TO_WORKSPACE><<<grid, 128, 0, ctx->stream>>>(p);
+        if (cluster) launch_chained(ctx, decode_vec_kernel<T, LPK, DEC_ONE_CHUNK>, grid, 128, 0, 1, p);
+        else launch_chained(ctx, decode_vec_kernel<T, LPK, DEC_TO_WORKSPACE>, grid, 128, 0, 1, p);
         return DEERS_OK;
     }
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = grid;
-    lc.blockDim = dim3(128);
-    lc.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)p.splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    lc.attrs = at; lc.numAttrs = 1;
-    DEERS_CUDA_TRY(ctx, cudaLaunchKernelEx(&lc, decode_vec_kernel<T, LPK, DEC_CLUSTER>, p));
+    DEERS_CUDA_TRY(ctx, launch_chained(ctx, decode_vec_kernel<T, LPK, DEC_CLUSTER>, grid, 128, 0, p.splits, p));
     return DEERS_OK;
 }
 
@@ -453,13 +449,13 @@ template <typename T>
 static int decode_launch(deers_ctx* ctx, const DecodeParams& p, const dim3& grid, bool vec, bool cluster) {
     const int pieces = p.D * (int)sizeof(T) / 16;
     int rc = DEERS_OK;
-    if (!vec) decode_partial_kernel<T><<<grid, 128, 0, ctx->stream>>>(p);
+    if (!vec) launch_chained(ctx, decode_partial_kernel<T>, grid, 128, 0, 1, p);
     else if (pieces > 16) rc = decode_launch_vec<T, 32>(ctx, p, grid, cluster);
     else if (pieces > 8) rc = decode_launch_vec<T, 16>(ctx, p, grid, cluster);
     else if (pieces > 4) rc = decode_launch_vec<T, 8>(ctx, p, grid, cluster);
     else rc = decode_launch_vec<T, 4>(ctx, p, grid, cluster);
     if (rc || (vec && cluster)) return rc;
-    decode_combine_kernel<T><<<(unsigned)((long long)p.B * p.H * p.Tq), 128, 0, ctx->stream>>>(p);
+    launch_chained(ctx, decode_combine_kernel<T>, (unsigned)((long long)p.B * p.H * p.Tq), 128, 0, 1, p);
     ctx->launches += 1;
     return DEERS_OK;
 }

@@ -186,6 +186,7 @@ struct Tile {
 // ---------------------------------------------------------------------------
 template <int DP>
 __global__ void __launch_bounds__(NT) attn_fwd_f32_kernel(const F32Params p) {
+    chain_wait();
     using L = Tile<DP>;
     constexpr int BN = L::BN, NC = L::NC, LD = L::LD, PLD = L::FWD_PLD;
     extern __shared__ __align__(16) float smem[];
@@ -269,6 +270,7 @@ __global__ void __launch_bounds__(NT) attn_fwd_f32_kernel(const F32Params p) {
         cp_commit();
     }
     cp_wait<0>();
+    chain_next();
 
     // The groups meet: O = sum_g 2^(m_g - M) O_g / sum_g 2^(m_g - M) l_g, in group order.
     put_acc<DP>(Ks, ty, tx, acc);
@@ -473,6 +475,7 @@ __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt
         cp_commit();
     }
     cp_wait<0>();
+    chain_next();
     put_acc<DP>(Qs, ty, tx, dk);
     put_acc<DP>(Gs, ty, tx, dv);
     __syncthreads();
@@ -552,6 +555,7 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
         cp_commit();
     }
     cp_wait<0>();
+    chain_next();
     put_acc<DP>(Ks, ty, tx, dq);
     __syncthreads();
     merge_store<DP>(p, grp0, L::BWD_GROUP, p.dq + b * p.sdq.b + h * p.sdq.h, p.sdq.t, q0);
@@ -560,6 +564,7 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
 // Both roles in one launch: blockIdx.y = 2 n is the n-th heaviest key tile, 2 n + 1 the n-th heaviest query tile.
 template <int DP>
 __global__ void __launch_bounds__(NT, DP <= 64 ? 2 : 1) attn_bwd_f32_kernel(const F32Params p) {
+    chain_wait();
     extern __shared__ __align__(16) float smem[];
     const int n = blockIdx.y >> 1, tiles = (p.T + BM - 1) / BM;
     if ((blockIdx.y & 1) == 0) bwd_dkdv<DP>(p, smem, n, blockIdx.x);
@@ -578,7 +583,7 @@ int fwd_impl(deers_ctx* ctx, const F32Params& p) {
     const dim3 grid(p.B * p.H, (p.T + BM - 1) / BM);
     {
         KernelTimerScope ts(ctx, DEERS_K_FWD);
-        attn_fwd_f32_kernel<DP><<<grid, NT, Tile<DP>::FWD_SMEM, ctx->stream>>>(p);
+        launch_chained(ctx, attn_fwd_f32_kernel<DP>, grid, NT, Tile<DP>::FWD_SMEM, 1, p);
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -592,7 +597,7 @@ int bwd_impl(deers_ctx* ctx, const F32Params& p) {
     if (grid.y > 65535) return DEERS_ERR_SHAPE;
     {
         KernelTimerScope ts(ctx, DEERS_K_BWD_MAIN);
-        attn_bwd_f32_kernel<DP><<<grid, NT, Tile<DP>::BWD_SMEM, ctx->stream>>>(p);
+        launch_chained(ctx, attn_bwd_f32_kernel<DP>, grid, NT, Tile<DP>::BWD_SMEM, 1, p);
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     ctx->launches += 1;

@@ -142,6 +142,7 @@ template <int D>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const FwdParams p) {
+    chain_wait();
     using L = FwdSmem<D>;
     constexpr uint32_t TILE_BYTES = L::TILE;
     constexpr int DBLK = D / 64;
@@ -233,6 +234,8 @@ attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 c.advance(p, nq, n_items);
             }
         }
+        __syncwarp();
+        chain_next();                                           // all loads are under way: the end is near
     } else if (warp == 1) {
         // ------------------------------ P V issuer ------------------------------
         {
@@ -549,8 +552,9 @@ int fwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
     const unsigned grid = (unsigned)(items < ctx->sm_count ? items : ctx->sm_count);
     p.sched = deers_get_schedule(ctx, d->B, d->H, (int)nq, d->causal, (int)grid, &p.sched_rows);
     {
+        const ChainScope chain(ctx, items * (d->causal ? (nq + 1) / 2 : nq) / grid);
         KernelTimerScope ts(ctx, DEERS_K_FWD);
-        attn_fwd_f16_kernel<D><<<grid, FWD_THREADS, smem, ctx->stream>>>(tq, tk, tv, p);
+        launch_chained(ctx, attn_fwd_f16_kernel<D>, grid, FWD_THREADS, smem, 1, tq, tk, tv, p);
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());

@@ -8,6 +8,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <utility>
 
 #include "../../include/deers_b200.h"
 
@@ -59,6 +60,7 @@ struct deers_ctx {
     cudaStream_t h2d_stream, d2h_stream;
     cudaEvent_t pipe_ev[3][3];      // [buffer set][h2d done, compute done, d2h done]
     bool pipe_ready;
+    bool no_chain;                  // launches follow work of another stream: nothing to overlap with (launch_chained)
     int cluster_room_f16[9];        // the same for the f16 GEMM's CTAs (gemm_f16_sm100.cu)
     int cluster_capacity[9];        // [n]: clusters of n blocks the device holds at once (gemm_f32.cu; 0: not asked yet)
 };
@@ -102,6 +104,50 @@ struct KernelTimerScope {
             _done.fetch_or(_bit, std::memory_order_release);                                                        \
         }                                                                                                           \
     } while (0)
+
+// Back-to-back kernels.  A kernel launched by launch_chained() may be set up while the one before it still runs: it calls
+// chain_wait() before its first access to global memory (the predecessor has finished and its writes are visible; every
+// kernel of a chain waits, so this covers all before it) and chain_next() where its own successor may be set up.
+// Saves the launch gap of a microsecond or two: 54 kernels of a GPT forward on a short prompt 232 -> 206 us.  Where chain_next()
+// stands matters: a successor set up at the start of a kernel of few large blocks takes the idle SMs unevenly (252 us), so
+// those call it once their last loads are under way; kernels of small blocks call it first.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void chain_begin() { chain_next(); chain_wait(); }
+
+// False while capturing, unless a kernel of this stream is the one predecessor (ctx.cu).
+bool deers_can_chain(const deers_ctx* ctx);
+
+template <typename... P, typename... A>
+cudaError_t launch_chained(deers_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, dim3 cluster, A&&... args) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = grid;
+    lc.blockDim = block;
+    lc.dynamicSmemBytes = smem;
+    lc.stream = ctx->stream;
+    cudaLaunchAttribute at[2];
+    unsigned n = 0;
+    if (deers_can_chain(ctx)) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster.x * cluster.y * cluster.z > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster.x; at[n].val.clusterDim.y = cluster.y; at[n++].val.clusterDim.z = cluster.z;
+    }
+    lc.attrs = at; lc.numAttrs = n;
+    return cudaLaunchKernelEx(&lc, kernel, std::forward<A>(args)...);
+}
+
+// A long kernel of one block per SM gains nothing from an early start and loses: its blocks then land on the SMs in the order
+// in which the predecessor's leave, not neighbours next to one another (B8 H32 T4096 D128 forward and backward: 10470 us
+// unchained, 10870 chained).  steps: 128 x 128 score tiles (or the like, about half a microsecond) per block.
+struct ChainScope {
+    deers_ctx* ctx;
+    bool was;
+    ChainScope(deers_ctx* c, long long steps) : ctx(c), was(c->no_chain) { c->no_chain = was || steps > 128; }
+    ~ChainScope() { ctx->no_chain = was; }
+};
 
 // Device-side error codes (upper byte: which kernel, lower bits: which wait).
 enum {

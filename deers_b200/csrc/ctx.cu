@@ -199,6 +199,20 @@ extern "C" int deers_b200_sync(deers_ctx* ctx) {
     return DEERS_OK;
 }
 
+bool deers_can_chain(const deers_ctx* ctx) {
+    if (ctx->no_chain) return false;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) { cudaGetLastError(); return false; }
+    if (st == cudaStreamCaptureStatusNone) return true;
+    if (st != cudaStreamCaptureStatusActive) return false;
+    const cudaGraphNode_t* before = nullptr;
+    const cudaGraphEdgeData* edges = nullptr;
+    size_t n = 0;
+    cudaGraphNodeType type;
+    if (cudaStreamGetCaptureInfo_v3(ctx->stream, &st, nullptr, nullptr, &before, &edges, &n) != cudaSuccess) { cudaGetLastError(); return false; }
+    return n == 1 && cudaGraphNodeGetType(before[0], &type) == cudaSuccess && type == cudaGraphNodeTypeKernel;
+}
+
 // ---------------------------------------------------------------------------
 // Work schedule of the persistent kernels
 // ---------------------------------------------------------------------------

@@ -57,6 +57,7 @@ struct GemmParams {
 template <int A_MN, int B_MN, int GN, bool SPLIT>
 __global__ void __launch_bounds__(G_THREADS, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+    chain_wait();
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr uint32_t G_B_BYTES = GN * GK * 2;
     uint8_t* sA = smem;
@@ -136,6 +137,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
                 }
             }
         }
+        __syncwarp();
+        chain_next();                                           // all loads are under way: the end is near
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp runs this; one elected lane issues (see elect_one).
@@ -339,20 +342,12 @@ int gemm_launch(deers_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, co
         if (parts == 1) {
             DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<A_MN, B_MN, GN, false>), g_smem(GN));
             const unsigned grid = (unsigned)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
-            gemm_f16_kernel<A_MN, B_MN, GN, false><<<grid, G_THREADS, g_smem(GN), ctx->stream>>>(ta, tb, p);
+            const ChainScope chain(ctx, tiles * p.kb_chunk / grid);
+            launch_chained(ctx, gemm_f16_kernel<A_MN, B_MN, GN, false>, grid, G_THREADS, g_smem(GN), 1, ta, tb, p);
         } else {
             const auto kernel = gemm_f16_kernel<A_MN, B_MN, GN, true>;
             DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<A_MN, B_MN, GN, true>), g_smem(GN));
-            cudaLaunchConfig_t lc{};
-            lc.gridDim = dim3((unsigned)(tiles * parts));
-            lc.blockDim = dim3(G_THREADS);
-            lc.dynamicSmemBytes = g_smem(GN);
-            lc.stream = ctx->stream;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = (unsigned)parts; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-            lc.attrs = at; lc.numAttrs = 1;
-            DEERS_CUDA_TRY(ctx, cudaLaunchKernelEx(&lc, kernel, ta, tb, p));
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, (unsigned)(tiles * parts), G_THREADS, g_smem(GN), parts, ta, tb, p));
         }
     }
     ctx->launches += 1;

@@ -51,6 +51,7 @@ template <int A_MN, int B_MN>
 __global__ void __launch_bounds__(X_THREADS, 1)
 gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_constant__ CUtensorMap tm_al,
                   const __grid_constant__ CUtensorMap tm_bh, const __grid_constant__ CUtensorMap tm_bl, const X3Params p) {
+    chain_wait();
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + X_STAGES * X_STAGE);
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + X_COUNT);
@@ -133,6 +134,8 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_consta
                 }
             }
         }
+        __syncwarp();
+        chain_next();                                           // all loads are under way: the end is near
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp runs this; one elected lane issues (see elect_one).
@@ -237,6 +240,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_consta
 // c[m][n] = sum over parts (in index order) of partial[part][m][n]
 __global__ void __launch_bounds__(256) x3_reduce_kernel(const float* __restrict__ partial, int parts, long long MN,
                                                         int N, float* __restrict__ c, long long ldc) {
+    chain_begin();
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < MN; i += (long long)gridDim.x * 256) {
         float acc = partial[i];
         for (int pz = 1; pz < parts; ++pz) acc += partial[(long long)pz * MN + i];
@@ -248,6 +252,7 @@ __global__ void __launch_bounds__(256) x3_reduce_kernel(const float* __restrict_
 __global__ void __launch_bounds__(256) x3_split_kernel(const float* __restrict__ src, long long ld_src, long long rows, int cols,
                                                        float scale, __half* __restrict__ hi, __half* __restrict__ lo,
                                                        long long ld_dst, int vec) {
+    chain_begin();
     const int per_row = (cols + 7) / 8;
     const long long total = rows * per_row;
     for (long long t = (long long)blockIdx.x * 256 + threadIdx.x; t < total; t += (long long)gridDim.x * 256) {
@@ -326,7 +331,7 @@ int x3_launch(deers_ctx* ctx, const CUtensorMap* t, const X3Params& p, unsigned 
     DEERS_SMEM_ONCE(ctx, (gemm_f16x3_kernel<A_MN, B_MN>), X_SMEM);
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM_X3);
-        gemm_f16x3_kernel<A_MN, B_MN><<<grid, X_THREADS, X_SMEM, ctx->stream>>>(t[0], t[1], t[2], t[3], p);
+        launch_chained(ctx, gemm_f16x3_kernel<A_MN, B_MN>, grid, X_THREADS, X_SMEM, 1, t[0], t[1], t[2], t[3], p);
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -349,7 +354,7 @@ int launch_split_f16x3(deers_ctx* ctx, long long rows, int cols, const float* sr
     const long long cap = 16LL * ctx->sm_count;
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM_X3);
-        x3_split_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, ctx->stream>>>(src, ld_src, rows, cols, scale, (__half*)hi,
+        launch_chained(ctx, x3_split_kernel, (unsigned)(want < cap ? want : cap), 256, 0, 1, src, ld_src, rows, cols, scale, (__half*)hi,
                                                                                       (__half*)lo, ld_dst, vec);
     }
     ctx->launches += 1;
@@ -391,7 +396,7 @@ int launch_gemm_f16x3(deers_ctx* ctx, int M, int N, int K, const void* a_hi, con
         const long long cap = 8LL * ctx->sm_count;
         {
             KernelTimerScope ts(ctx, DEERS_K_GEMM_X3);
-            x3_reduce_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, ctx->stream>>>((const float*)workspace, pl.parts, MN, N, c, ldc);
+            launch_chained(ctx, x3_reduce_kernel, (unsigned)(want < cap ? want : cap), 256, 0, 1, (const float*)workspace, pl.parts, MN, N, c, ldc);
         }
         ctx->launches += 1;
         DEERS_CUDA_TRY(ctx, cudaGetLastError());

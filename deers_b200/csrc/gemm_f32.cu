@@ -155,6 +155,7 @@ struct GemmShape {
 
 template <int PM, int PN, int KS, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(128 * KS) gemm_f32_kernel(const GemmArgs g) {
+    chain_wait();
     using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
     constexpr int BM = S::BM, BN = S::BN, GT = S::GT, STAGES = S::STAGES, KG = BK / KS;
     extern __shared__ __align__(16) float smem[];
@@ -253,6 +254,7 @@ __global__ void __launch_bounds__(128 * KS) gemm_f32_kernel(const GemmArgs g) {
         r_begin = rank * share;
         r_end = min(BM, r_begin + share);
     }
+    chain_next();                                                   // (at the loop or earlier, successors crowd out the side stream)
     for (int idx = r_begin * (BN / 4) + threadIdx.x; idx < r_end * (BN / 4); idx += GT) {
         const int row = idx / (BN / 4), col = (idx % (BN / 4)) * 4;
         const int m = m0 + row, n = n0 + col;
@@ -368,18 +370,7 @@ int launch_variant(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g) {
     using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
     const auto kernel = gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>;
     DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>), S::SMEM);
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(p.tiles_n, p.tiles_m, p.parts);
-    lc.blockDim = dim3(S::GT);
-    lc.dynamicSmemBytes = S::SMEM;
-    lc.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    if (p.parts > 1) {
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = (unsigned)p.parts;
-        lc.attrs = at; lc.numAttrs = 1;
-    }
-    DEERS_CUDA_TRY(ctx, cudaLaunchKernelEx(&lc, kernel, g));
+    DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, dim3(p.tiles_n, p.tiles_m, p.parts), S::GT, S::SMEM, dim3(1, 1, p.parts), g));
     return DEERS_OK;
 }
 

@@ -123,6 +123,7 @@ struct SideScope {
             return;
         }
         m->ctx->stream = m->side;
+        m->ctx->no_chain = true;
         m->on_side = true;
     }
     int done(int i) {
@@ -132,7 +133,7 @@ struct SideScope {
         return DEERS_OK;
     }
     ~SideScope() {
-        if (active) { m->ctx->stream = main; m->on_side = false; }
+        if (active) { m->ctx->stream = main; m->ctx->no_chain = false; m->on_side = false; }
     }
 };
 
@@ -383,12 +384,14 @@ int run_fwd_bwd(deers_gpt* m, int B, int T, bool with_norm) {
 
 // ids [B, T] -> ids_dev [B, Tp], zeros behind each row's end
 __global__ void __launch_bounds__(256) pad_ids_kernel(const long long* __restrict__ src, long long* __restrict__ dst, int T, int Tp, int n) {
+    chain_begin();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i < n) dst[i] = i % Tp < T ? src[(long long)(i / Tp) * T + i % Tp] : 0;
 }
 
 // logits [B, Tp, ld] -> out [B, T, V]; blockIdx.y is a row of out.  Rows of an odd V start on any 4-byte boundary.
 __global__ void __launch_bounds__(256) copy_logits_kernel(const float* __restrict__ src, long long ld, float* __restrict__ dst, int T, int Tp, int V) {
+    chain_begin();
     const int row = blockIdx.y;
     const float* s = src + ((long long)(row / T) * Tp + row % T) * ld;
     float* d = dst + (long long)row * V;
@@ -701,13 +704,13 @@ extern "C" int deers_b200_gpt_forward(deers_gpt* m, const int64_t* ids, int32_t 
     int Tp = (T + FWD_PAD - 1) / FWD_PAD * FWD_PAD;
     if (Tp > m->cfg.sequence_len) Tp = m->cfg.sequence_len;           // the rotary cache and the buffers end there
     const int n = B * Tp;
-    pad_ids_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>((const long long*)ids, m->ids_dev, T, Tp, n);
+    launch_chained(ctx, pad_ids_kernel, (n + 255) / 256, 256, 0, 1, (const long long*)ids, m->ids_dev, T, Tp, n);
     ctx->launches += 1;
     GPT_TRY(run_forward(m, B, Tp));
     if (logits) {
         const int V = m->cfg.vocab_size;
         const dim3 grid((unsigned)((V + 4095) / 4096), (unsigned)(B * T));
-        copy_logits_kernel<<<grid, 256, 0, ctx->stream>>>(m->logits, m->Vld, logits, T, Tp, V);
+        launch_chained(ctx, copy_logits_kernel, grid, 256, 0, 1, m->logits, m->Vld, logits, T, Tp, V);
         ctx->launches += 1;
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());

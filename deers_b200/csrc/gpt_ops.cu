@@ -24,6 +24,7 @@ namespace {
 __global__ void __launch_bounds__(256) embedding_fwd_kernel(const float* __restrict__ w, const long long* __restrict__ ids,
                                                             long long n_ids, int C, long long V, float* __restrict__ out,
                                                             int vec, unsigned int* err) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long n = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (n >= n_ids) return;
@@ -46,6 +47,7 @@ __global__ void __launch_bounds__(256) embedding_fwd_kernel(const float* __restr
 __global__ void __launch_bounds__(256) embedding_bwd_kernel(const float* __restrict__ dout,
                                                             const long long* __restrict__ ids, long long n_ids, int C,
                                                             long long V, float* __restrict__ dw) {
+    chain_wait();
     __shared__ unsigned char s_flag[256];
     const long long n = blockIdx.x;
     const long long id = ids[n];
@@ -101,6 +103,7 @@ __global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const float* __r
                                                                 const long long* __restrict__ targets, long long V,
                                                                 float* __restrict__ lse, float* __restrict__ picked,
                                                                 unsigned int* err) {
+    chain_wait();
     __shared__ float red_m[8], red_s[8];
     const long long row = blockIdx.x;
     const float* x = logits + row * ld;
@@ -140,6 +143,7 @@ __global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const float* __r
 
 __global__ void __launch_bounds__(1024) cross_entropy_loss_kernel(const float* __restrict__ picked, long long rows,
                                                                   float neg_inv_rows, float* __restrict__ loss) {
+    chain_wait();
     __shared__ float red[32];
     float s = 0.f;
     for (long long j = threadIdx.x; j < rows; j += 1024) s += picked[j];
@@ -160,6 +164,7 @@ __global__ void __launch_bounds__(256) cross_entropy_bwd_kernel(const float* __r
                                                                 const float* __restrict__ lse, long long V, float g,
                                                                 float upstream, float* __restrict__ dlogits,
                                                                 long long ldd, int vec) {
+    chain_wait();
     const long long row = blockIdx.y;
     const float* x = logits + row * ld;
     float* d = dlogits + row * ldd;
@@ -204,6 +209,7 @@ __global__ void __launch_bounds__(256) cross_entropy_bwd_split_kernel(const floa
                                                                       const float* __restrict__ lse, long long V, float g,
                                                                       float upstream, float scale, __half* __restrict__ hi,
                                                                       __half* __restrict__ lo, long long ldd) {
+    chain_wait();
     const long long row = blockIdx.y;
     const float* x = logits + row * ld;
     __half* dh = hi + row * ldd;
@@ -252,7 +258,7 @@ int launch_cross_entropy_bwd_split(deers_ctx* ctx, const float* logits, long lon
     const dim3 grid((unsigned)per_row, (unsigned)rows);
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        cross_entropy_bwd_split_kernel<<<grid, 256, 0, ctx->stream>>>(logits, ld, targets, lse, V, (float)(-1.0 / (double)rows),
+        launch_chained(ctx, cross_entropy_bwd_split_kernel, grid, 256, 0, 1, logits, ld, targets, lse, V, (float)(-1.0 / (double)rows),
                                                                       upstream, scale, (__half*)hi, (__half*)lo, ldd);
     }
     ctx->launches += 1;
@@ -266,7 +272,7 @@ int launch_embedding_fwd(deers_ctx* ctx, const float* weight, const long long* i
     const int vec = C % 4 == 0 && (((uintptr_t)weight | (uintptr_t)out) & 15u) == 0;
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        embedding_fwd_kernel<<<(unsigned)((n_ids + 7) / 8), 256, 0, ctx->stream>>>(weight, ids, n_ids, C, V, out, vec,
+        launch_chained(ctx, embedding_fwd_kernel, (unsigned)((n_ids + 7) / 8), 256, 0, 1, weight, ids, n_ids, C, V, out, vec,
                                                                                   ctx->dev_err);
     }
     ctx->launches += 1;
@@ -280,7 +286,7 @@ int launch_embedding_bwd(deers_ctx* ctx, const float* dout, const long long* ids
     if (n_ids == 0) return DEERS_OK;
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        embedding_bwd_kernel<<<(unsigned)n_ids, 256, 0, ctx->stream>>>(dout, ids, n_ids, C, V, dweight);
+        launch_chained(ctx, embedding_bwd_kernel, (unsigned)n_ids, 256, 0, 1, dout, ids, n_ids, C, V, dweight);
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -291,8 +297,8 @@ int launch_cross_entropy_fwd(deers_ctx* ctx, const float* logits, long long ld, 
                              long long V, float* lse, float* picked, float* loss) {
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        cross_entropy_fwd_kernel<<<(unsigned)rows, 256, 0, ctx->stream>>>(logits, ld, targets, V, lse, picked, ctx->dev_err);
-        cross_entropy_loss_kernel<<<1, 1024, 0, ctx->stream>>>(picked, rows, (float)(-1.0 / (double)rows), loss);
+        launch_chained(ctx, cross_entropy_fwd_kernel, (unsigned)rows, 256, 0, 1, logits, ld, targets, V, lse, picked, ctx->dev_err);
+        launch_chained(ctx, cross_entropy_loss_kernel, 1, 1024, 0, 1, picked, rows, (float)(-1.0 / (double)rows), loss);
     }
     ctx->launches += 2;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -302,7 +308,7 @@ int launch_cross_entropy_fwd(deers_ctx* ctx, const float* logits, long long ld, 
 int launch_cross_entropy_loss(deers_ctx* ctx, const float* picked, long long rows, float* loss) {
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        cross_entropy_loss_kernel<<<1, 1024, 0, ctx->stream>>>(picked, rows, (float)(-1.0 / (double)rows), loss);
+        launch_chained(ctx, cross_entropy_loss_kernel, 1, 1024, 0, 1, picked, rows, (float)(-1.0 / (double)rows), loss);
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -318,7 +324,7 @@ int launch_cross_entropy_bwd(deers_ctx* ctx, const float* logits, long long ld, 
     const dim3 grid((unsigned)per_row, (unsigned)rows);
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        cross_entropy_bwd_kernel<<<grid, 256, 0, ctx->stream>>>(logits, ld, targets, lse, V, (float)(-1.0 / (double)rows),
+        launch_chained(ctx, cross_entropy_bwd_kernel, grid, 256, 0, 1, logits, ld, targets, lse, V, (float)(-1.0 / (double)rows),
                                                                 upstream, dlogits, ldd, vec);
     }
     ctx->launches += 1;

@@ -58,6 +58,7 @@ __device__ __forceinline__ int find_tensor(const OptTensors& t, int chunk) {
 // Partial sums of squares: block b takes chunks b, b + grid, ...; thread-local accumulation in
 // element order, then a fixed shuffle / shared-memory tree.
 __global__ void __launch_bounds__(256) grad_sq_sum_kernel(const __grid_constant__ OptTensors t, float* __restrict__ partial) {
+    chain_wait();
     const int total_chunks = t.chunk_start[t.count];
     float acc = 0.f;
     for (int chunk = blockIdx.x; chunk < total_chunks; chunk += gridDim.x) {
@@ -93,6 +94,7 @@ __global__ void __launch_bounds__(256) grad_sq_sum_kernel(const __grid_constant_
 
 // norm = sqrt(sum of the partials), summed by one block in a fixed order.
 __global__ void __launch_bounds__(1024) grad_norm_kernel(const float* __restrict__ partial, int n, float* __restrict__ norm) {
+    chain_wait();
     __shared__ float sh[1024];
     float acc = 0.f;
     for (int i = threadIdx.x; i < n; i += 1024) acc += partial[i];
@@ -137,6 +139,7 @@ __device__ __forceinline__ void adamw_element(const OptScalars& s, bool clip, fl
 template <int MODE>
 __global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ OptTensors t, const __grid_constant__ OptScalars s,
                                                     const float* __restrict__ norm) {
+    chain_wait();
     float scale;
     const bool clip = clip_scale(s, norm, scale);
     if (MODE == MODE_CLIP && !clip) return;
@@ -266,14 +269,14 @@ extern "C" int deers_b200_grad_norm(deers_ctx* ctx, int n_tensors, const deers_o
         if ((size_t)(n_partial + grid) * sizeof(float) > scratch_bytes) return DEERS_ERR_WORKSPACE;
         {
             KernelTimerScope ts(ctx, DEERS_K_OPTIM);
-            grad_sq_sum_kernel<<<grid, 256, 0, ctx->stream>>>(t, partial + n_partial);
+            launch_chained(ctx, grad_sq_sum_kernel, grid, 256, 0, 1, t, partial + n_partial);
         }
         ctx->launches += 1;
         n_partial += (int)grid;
     }
     {
         KernelTimerScope ts(ctx, DEERS_K_OPTIM);
-        grad_norm_kernel<<<1, 1024, 0, ctx->stream>>>(partial, n_partial, norm_dev);
+        launch_chained(ctx, grad_norm_kernel, 1, 1024, 0, 1, partial, n_partial, norm_dev);
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -291,8 +294,8 @@ static int optim_apply(deers_ctx* ctx, int n_tensors, const deers_optim_tensor* 
         const unsigned grid = optim_grid(ctx, t.chunk_start[t.count]);
         {
             KernelTimerScope ts(ctx, DEERS_K_OPTIM);
-            if (mode == MODE_STEP) adamw_kernel<MODE_STEP><<<grid, 256, 0, ctx->stream>>>(t, s, norm_dev);
-            else adamw_kernel<MODE_CLIP><<<grid, 256, 0, ctx->stream>>>(t, s, norm_dev);
+            if (mode == MODE_STEP) launch_chained(ctx, adamw_kernel<MODE_STEP>, grid, 256, 0, 1, t, s, norm_dev);
+            else launch_chained(ctx, adamw_kernel<MODE_CLIP>, grid, 256, 0, 1, t, s, norm_dev);
         }
         ctx->launches += 1;
     }

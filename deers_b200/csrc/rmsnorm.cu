@@ -31,6 +31,8 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
                                                       const float* __restrict__ add, float* __restrict__ out,
                                                       float* __restrict__ inv_io, long long rows, int C, float eps,
                                                       float inv_n) {
+    if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room)
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * 8;
@@ -147,6 +149,8 @@ __global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* __restr
                                                             const float* __restrict__ add, float* __restrict__ out,
                                                             float* __restrict__ inv_io, long long rows, int C, float eps,
                                                             float inv_n) {
+    if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room)
+    chain_wait();
     __shared__ float part[8];
     const int nv = C / 4;                                       // <= 256 * RN_MAXV
     for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -217,12 +221,12 @@ int rms_launch(deers_ctx* ctx, long long rows, int C, float eps, const float* x,
     const float inv_n = (float)(1.0 / (double)C);               // mean = sum * (1/n as f64 -> f32), src/tensor.rs:461-465
     {
         KernelTimerScope ts(ctx, DEERS_K_NORM);
-        if (vec) rmsnorm_kernel<BWD, true><<<grid, 256, 0, ctx->stream>>>(x, dy, add, out, inv, rows, C, eps, inv_n);
+        if (vec) launch_chained(ctx, rmsnorm_kernel<BWD, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n);
         else if (aligned && C <= 256 * RN_MAXV * 4) {
             const unsigned bgrid = (unsigned)(rows < cap ? rows : cap);
-            rmsnorm_block_kernel<BWD><<<bgrid, 256, 0, ctx->stream>>>(x, dy, add, out, inv, rows, C, eps, inv_n);
-        } else if (aligned) rmsnorm_kernel<BWD, false, true><<<grid, 256, 0, ctx->stream>>>(x, dy, add, out, inv, rows, C, eps, inv_n);
-        else rmsnorm_kernel<BWD, false><<<grid, 256, 0, ctx->stream>>>(x, dy, add, out, inv, rows, C, eps, inv_n);
+            launch_chained(ctx, rmsnorm_block_kernel<BWD>, bgrid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n);
+        } else if (aligned) launch_chained(ctx, rmsnorm_kernel<BWD, false, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n);
+        else launch_chained(ctx, rmsnorm_kernel<BWD, false>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n);
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());

@@ -57,6 +57,8 @@ __device__ __forceinline__ void rotate(const __half a, const __half b, const __h
 
 template <typename T, int V>
 __global__ void __launch_bounds__(256) rope_pack_kernel(const RopeParams p) {
+    if (!p.inverse) chain_next();                               // (backward: weight gradients run beside it, leave them the room)
+    chain_wait();
     const int half = p.D / 2;
     const int cpr = half / V;                                   // chunks (threads) per row
     const long long rows = (long long)p.B * p.T * p.H;
@@ -140,8 +142,8 @@ int rope_launch(deers_ctx* ctx, const deers_rope_desc* d, const RopeParams& p) {
     const unsigned grid = (unsigned)(want < cap ? want : cap);
     {
         KernelTimerScope ts(ctx, DEERS_K_ROPE);
-        if (vec) rope_pack_kernel<T, VMAX><<<grid, 256, 0, ctx->stream>>>(p);
-        else rope_pack_kernel<T, 1><<<grid, 256, 0, ctx->stream>>>(p);
+        if (vec) launch_chained(ctx, rope_pack_kernel<T, VMAX>, grid, 256, 0, 1, p);
+        else launch_chained(ctx, rope_pack_kernel<T, 1>, grid, 256, 0, 1, p);
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());

@@ -188,3 +188,50 @@ def test_f16_gemm_split_k_and_tile_widths(M, N, K, a_mn, b_mn):
     want = (af.T if a_mn else af) @ (bf if b_mn else bf.T)
     assert np.abs(want).max() <= 2048
     assert np.array_equal(got.float().cpu().numpy(), want.astype(np.float32))
+
+
+@pytest.mark.parametrize("B,H,T,D,dtype", [(1, 2, 64, 64, torch.float16), (2, 3, 127, 80, torch.float16), (1, 12, 128, 32, torch.float32)])
+def test_chained_kernels_see_their_predecessors(B, H, T, D, dtype):
+    """Each kernel of a sequence reads what the one before it (or a copy) has just written, over the same buffers again and
+    again: eagerly, and captured with a copy, a kernel and a join of two streams as the predecessor.  Bit for bit the same."""
+    from deers_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    src = [torch.randn((B, H, T, D), device="cuda", generator=gen).to(dtype) for _ in range(4)]
+    scale = ops.default_scale(D)
+    side = torch.cuda.Stream()
+
+    def chain(wait):
+        x, out = src[0].clone(), []
+        for _ in range(3):
+            o, lse = ops.attention_fwd(x, src[1], src[2], scale)
+            wait()
+            dq, dk, dv = ops.attention_bwd(x, src[1], src[2], o, lse, src[3], scale)
+            wait()
+            y = ops.attention_decode(dq, dk, o, scale)
+            x.copy_(y)                                                  # a copy as the predecessor
+            other = torch.cuda.current_stream()
+            side.wait_stream(other)
+            with torch.cuda.stream(side):
+                z = dv + x
+            x = ops.attention_decode(y, src[1], src[2], scale)
+            wait()
+            other.wait_stream(side)                                     # two predecessors
+            x = ops.attention_decode(x, z, dv, scale)
+            out += [o, lse, dq, dk, dv, y, z, x]
+        return out
+
+    st = torch.cuda.Stream()
+    st.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(st):
+        want = chain(st.synchronize)
+        got = [chain(lambda: None) for _ in range(3)]
+        st.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            captured = chain(lambda: None)
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    for g in got + [captured]:
+        for a, b in zip(g, want):
+            assert torch.equal(a, b)
