@@ -140,7 +140,7 @@ cudaError_t launch_chained(deers_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3
 }
 
 // A long kernel of one block per SM gains nothing from an early start and loses: its blocks then land on the SMs in the order
-// in which the predecessor's leave, not neighbours next to one another (B8 H32 T4096 D128 forward and backward: 10470 us
+// in which the predecessor's leave, not neighbours next to one another (B64 H32 T2048 D128 forward and backward: 10470 us
 // unchained, 10870 chained).  steps: 128 x 128 score tiles (or the like, about half a microsecond) per block.
 struct ChainScope {
     deers_ctx* ctx;

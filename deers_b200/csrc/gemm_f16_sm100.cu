@@ -294,6 +294,12 @@ struct GemmPlan { int gn, parts, kb_chunk; };
 // Clusters of n CTAs (one per SM) the device holds at a time.
 int cluster_room(deers_ctx* ctx) {
     if (ctx->cluster_room_f16[1] > 0) return DEERS_OK;
+    static std::atomic<int> known[64][G_MAX_PARTS + 1];                    // asked once per device: a tenth of a millisecond each
+    std::atomic<int>* dev = known[ctx->device & 63];
+    if (dev[1].load(std::memory_order_acquire) > 0) {
+        for (int parts = 1; parts <= G_MAX_PARTS; ++parts) ctx->cluster_room_f16[parts] = dev[parts].load(std::memory_order_relaxed);
+        return DEERS_OK;
+    }
     const auto kernel = gemm_f16_kernel<0, 1, 256, true>;
     DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<0, 1, 256, true>), g_smem(256));
     for (int parts = 2; parts <= G_MAX_PARTS; ++parts) {
@@ -308,8 +314,10 @@ int cluster_room(deers_ctx* ctx) {
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, kernel, &lc) != cudaSuccess) { cudaGetLastError(); n = 0; }
         ctx->cluster_room_f16[parts] = n;
+        dev[parts].store(n, std::memory_order_relaxed);
     }
     ctx->cluster_room_f16[1] = ctx->sm_count;
+    dev[1].store(ctx->sm_count, std::memory_order_release);
     return DEERS_OK;
 }
 

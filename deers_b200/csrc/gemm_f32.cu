@@ -320,6 +320,12 @@ constexpr Variant kVariants[6] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {
 // GPC, so e.g. 48 clusters of three do not fit 148 SMs although their 144 blocks would.
 int cluster_capacity(deers_ctx* ctx) {
     if (ctx->cluster_capacity[1] > 0) return DEERS_OK;
+    static std::atomic<int> known[64][MAX_PARTS + 1];                    // asked once per device: a tenth of a millisecond each
+    std::atomic<int>* dev = known[ctx->device & 63];
+    if (dev[1].load(std::memory_order_acquire) > 0) {
+        for (int parts = 1; parts <= MAX_PARTS; ++parts) ctx->cluster_capacity[parts] = dev[parts].load(std::memory_order_relaxed);
+        return DEERS_OK;
+    }
     using S = GemmShape<8, 4, 4, false, true>;
     const auto kernel = gemm_f32_kernel<8, 4, 4, false, true>;
     DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<8, 4, 4, false, true>), S::SMEM);
@@ -335,8 +341,10 @@ int cluster_capacity(deers_ctx* ctx) {
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, kernel, &lc) != cudaSuccess) { cudaGetLastError(); n = 0; }
         ctx->cluster_capacity[parts] = n;
+        dev[parts].store(n, std::memory_order_relaxed);
     }
     ctx->cluster_capacity[1] = ctx->sm_count;
+    dev[1].store(ctx->sm_count, std::memory_order_release);
     return DEERS_OK;
 }
 

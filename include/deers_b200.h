@@ -359,9 +359,8 @@ int deers_b200_gemm_f16(deers_ctx* ctx, int32_t M, int32_t N, int32_t K, const v
  *     DEERS_EPI_RELU_SQ   r = max(A*B, 0); C = r*r; aux = r  `relu` and `y * y` of the MLP (`gpt.rs:194-196`)
  *     DEERS_EPI_MUL_AUX2  t = (A*B) * aux; C = t + t         their backward (`src/ops.rs:210-214, 560-568`) given aux = r
  * aux has the shape and leading dimension of C.  Shapes with few output tiles and a long K are split along K;
- * the parts are added in a fixed order, so results are bitwise reproducible.  `workspace` must hold
- * deers_b200_gemm_f32_workspace_bytes(ctx, M, N, K) bytes (0 for most shapes; 256-byte aligned).  Enqueued on
- * the context's stream; no allocation, no synchronisation.
+ * the parts meet in shared memory and are added in a fixed order, so results are bitwise reproducible.  `workspace` is
+ * not used (deers_b200_gemm_f32_workspace_bytes is 0) and may be NULL.  Enqueued on the context's stream; no allocation, no synchronisation.
  */
 enum { DEERS_EPI_NONE = 0, DEERS_EPI_ADD = 1, DEERS_EPI_RELU_SQ = 2, DEERS_EPI_MUL_AUX2 = 3 };
 typedef struct deers_gemm_epilogue {
