@@ -1038,10 +1038,13 @@ attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const
 
 // delta[row] = sum_d dO[row][d] * O[row][d] and lse2[row] = lse[row] * log2(e) on the padded
 // [B*H][Tpad] grid (0 beyond T).  D/8 lanes share a row (16-byte loads); a warp takes 4 * 256 / D
-// consecutive rows per step with all eight loads of a lane in flight before the first is used;
-// grid-stride over such row groups.  The row count fits 32 bits (checked by the launcher).
+// consecutive rows per step, all of one slice (Tpad is a multiple of 128), with all eight loads of a lane in flight
+// before the first is used; grid-stride over such row groups.  The row count fits 32 bits (checked by the launcher).
+// Bound by reading O and dO once.  One slice per group means two divisions instead of sixteen, and the grid is the
+// PREP_BLOCKS blocks an SM holds (eight, in 1.6 waves, before): about 1 % of a forward and backward.
+constexpr int PREP_BLOCKS = 4;
 template <int D>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, PREP_BLOCKS)
 attn_bwd_prep_f16_kernel(const __half* __restrict__ o, const __half* __restrict__ d_o, const float* __restrict__ lse,
                          float* __restrict__ delta, float* __restrict__ lse2, int B, int H, int T, int d, int Tpad,
                          long long so_b, long long so_h, long long so_t, long long sdo_b, long long sdo_h,
@@ -1055,23 +1058,27 @@ attn_bwd_prep_f16_kernel(const __half* __restrict__ o, const __half* __restrict_
     const unsigned rows = (unsigned)B * (unsigned)H * (unsigned)Tpad;
     const unsigned warp_global = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const unsigned warp_count = gridDim.x * (blockDim.x / 32);
-    const unsigned ngroups = (rows + RPW * U - 1) / (RPW * U);
+    static_assert(BT % (RPW * U) == 0, "a group of rows stays inside one slice");
+    const unsigned ngroups = rows / (RPW * U);
     for (unsigned grp = warp_global; grp < ngroups; grp += warp_count) {
         uint4 a[U], g[U];
-        unsigned row[U];
-        bool valid[U];
+        float l[U];
+        const unsigned row0 = grp * (RPW * U), bh = row0 / (unsigned)Tpad, b = bh / (unsigned)H, h = bh - b * (unsigned)H;
+        const unsigned t0 = row0 - bh * (unsigned)Tpad + rw;
+        const __half* ob = o + b * so_b + h * so_h + (long long)t0 * so_t + sub * 8;
+        const __half* gb = d_o + b * sdo_b + h * sdo_h + (long long)t0 * sdo_t + sub * 8;
+        const float* lb = lse + (long long)bh * T + t0;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            row[u] = grp * (RPW * U) + u * RPW + rw;
-            const unsigned t = row[u] % (unsigned)Tpad, bh = row[u] / (unsigned)Tpad;
-            valid[u] = row[u] < rows && t < (unsigned)T;
+            const bool valid = t0 + u * RPW < (unsigned)T;
             a[u] = make_uint4(0u, 0u, 0u, 0u);
             g[u] = a[u];
-            if (valid[u] && sub * 8 < d) {
-                const unsigned b = bh / (unsigned)H, h = bh % (unsigned)H;
-                a[u] = *reinterpret_cast<const uint4*>(o + b * so_b + h * so_h + (long long)t * so_t + sub * 8);
-                g[u] = *reinterpret_cast<const uint4*>(d_o + b * sdo_b + h * sdo_h + (long long)t * sdo_t + sub * 8);
+            l[u] = 0.f;
+            if (valid && sub * 8 < d) {
+                a[u] = *reinterpret_cast<const uint4*>(ob + u * RPW * so_t);
+                g[u] = *reinterpret_cast<const uint4*>(gb + u * RPW * sdo_t);
             }
+            if (valid && sub == 0) l[u] = lb[u * RPW];
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -1086,10 +1093,9 @@ attn_bwd_prep_f16_kernel(const __half* __restrict__ o, const __half* __restrict_
             }
 #pragma unroll
             for (int off = LPR / 2; off >= 1; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-            if (row[u] < rows && sub == 0) {
-                const unsigned t = row[u] % (unsigned)Tpad, bh = row[u] / (unsigned)Tpad;
-                delta[row[u]] = valid[u] ? s : 0.f;
-                lse2[row[u]] = valid[u] ? lse[(long long)bh * T + t] * LOG2E : 0.f;
+            if (sub == 0) {                                          // (beyond T: loads were replaced by zeros)
+                delta[row0 + u * RPW + rw] = s;
+                lse2[row0 + u * RPW + rw] = l[u] * LOG2E;
             }
         }
     }
@@ -1122,7 +1128,7 @@ int bwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
         if (prep_rows > 0x7fffffffLL) return DEERS_ERR_SHAPE;      // 32-bit row indices in the kernel
         const long long per_block = 8LL * 4 * (256 / D);           // 8 warps x 4 loads x rows per load
         const long long want = (prep_rows + per_block - 1) / per_block;
-        const unsigned prep_grid = (unsigned)(want < 8LL * ctx->sm_count ? want : 8LL * ctx->sm_count);
+        const unsigned prep_grid = (unsigned)(want < (long long)PREP_BLOCKS * ctx->sm_count ? want : (long long)PREP_BLOCKS * ctx->sm_count);
         launch_chained(ctx, attn_bwd_prep_f16_kernel<D>, prep_grid, 256, 0, 1,
             (const __half*)o, (const __half*)d_o, lse, delta, lse2, d->B, d->H, d->T, d->D, Tpad, d->o_strides[0],
             d->o_strides[1], d->o_strides[2], d->do_strides[0], d->do_strides[1], d->do_strides[2]);
