@@ -396,12 +396,12 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         // warp seeing a stale 32-byte piece of the delta row in the first iteration of an item.)
         const int ct = (warp - 2) * 32 + lane;
         const bool stager = ct < 2 * BT;
-        const float* stat_src = (ct < BT) ? p.lse2 + ct : p.delta + (ct - BT);
+        const float* stat_src = chained((ct < BT) ? p.lse2 + ct : p.delta + (ct - BT));
         float* stat_dst = (ct < BT) ? lse2_s + ct : delta_s + (ct - BT);
         float stat_next = 0.f;
         {
             const int4 first = next_item(p, 0, n_items, nq);
-            if (stager && first.x >= 0) stat_next = __ldg(stat_src + (long long)first.y * p.Tpad + (p.causal ? first.x : 0) * BT);
+            if (stager && first.x >= 0) stat_next = stat_src[(long long)first.y * p.Tpad + (p.causal ? first.x : 0) * BT];
         }
         // this thread's row of the dS^T tile; its warpgroup's four 16-byte chunks start at chunk ch0 of the row
         uint8_t* ds_row = smem + L::DS + (CW * g / 64) * BLOCK_BYTES + r * 128;   // (of the first stage)
@@ -462,8 +462,8 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                 mbar_arrive_warp(&bars[A_ST_FULL + ss]);
                 // next iteration's value: the next query tile of this item, or the first one of the next item
                 if (stager) {
-                    if (it + 1 < niter) stat_next = __ldg(stat_src + (long long)bh * p.Tpad + (i + 1) * BT);
-                    else if (nxt.x >= 0) stat_next = __ldg(stat_src + (long long)nxt.y * p.Tpad + (p.causal ? nxt.x : 0) * BT);
+                    if (it + 1 < niter) stat_next = stat_src[(long long)bh * p.Tpad + (i + 1) * BT];
+                    else if (nxt.x >= 0) stat_next = stat_src[(long long)nxt.y * p.Tpad + (p.causal ? nxt.x : 0) * BT];
                 }
                 if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_ST_FULL + ss], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 13))) { alive = false; break; }
                 if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[A_S + ss], (gi >> 1) & 1u, DEERS_KERR_BWD_F16 | 14))) { alive = false; break; }
@@ -1045,11 +1045,12 @@ attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const
 constexpr int PREP_BLOCKS = 4;
 template <int D>
 __global__ void __launch_bounds__(256, PREP_BLOCKS)
-attn_bwd_prep_f16_kernel(const __half* __restrict__ o, const __half* __restrict__ d_o, const float* __restrict__ lse,
+attn_bwd_prep_f16_kernel(const __half* o, const __half* d_o, const float* lse,
                          float* __restrict__ delta, float* __restrict__ lse2, int B, int H, int T, int d, int Tpad,
                          long long so_b, long long so_h, long long so_t, long long sdo_b, long long sdo_h,
                          long long sdo_t) {
     chain_begin();
+    o = chained(o); d_o = chained(d_o); lse = chained(lse);
     constexpr int LPR = D / 8;                               // lanes per row
     constexpr int RPW = 32 / LPR;                            // rows per warp load
     constexpr int U = 4;                                     // loads in flight per lane and tensor

@@ -8,6 +8,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <type_traits>
 #include <utility>
 
 #include "../../include/deers_b200.h"
@@ -114,6 +115,22 @@ struct KernelTimerScope {
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void chain_begin() { chain_next(); chain_wait(); }
+// What a predecessor writes may change while a chained kernel is already resident, so its reads must be ordinary (coherent)
+// loads behind the wait.  Pointers to such data are neither `const __restrict__` nor read by __ldg: both allow the read-only
+// path, which promises the values of the kernel's start, and let the compiler move the load in front of the wait.
+// chained(p), taken after the wait, hands out the pointer as a value the compiler knows nothing about but that it is global.
+template <typename T>
+__device__ __forceinline__ T* chained(T* p) {
+    size_t g = __cvta_generic_to_global(p);
+    asm volatile("" : "+l"(g) : : "memory");
+    return static_cast<T*>(const_cast<typename std::remove_const<T>::type*>(static_cast<const typename std::remove_const<T>::type*>(__cvta_global_to_generic(g))));
+}
+// One streaming (read once) float behind the wait.
+__device__ __forceinline__ float ld_stream(const float* p) {
+    float v;
+    asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
 
 // False while capturing, unless a kernel of this stream is the one predecessor (ctx.cu).
 bool deers_can_chain(const deers_ctx* ctx);

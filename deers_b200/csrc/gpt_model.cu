@@ -383,14 +383,15 @@ int run_fwd_bwd(deers_gpt* m, int B, int T, bool with_norm) {
 }
 
 // ids [B, T] -> ids_dev [B, Tp], zeros behind each row's end
-__global__ void __launch_bounds__(256) pad_ids_kernel(const long long* __restrict__ src, long long* __restrict__ dst, int T, int Tp, int n) {
+__global__ void __launch_bounds__(256) pad_ids_kernel(const long long* src, long long* __restrict__ dst, int T, int Tp, int n) {
     chain_begin();
+    src = chained(src);
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i < n) dst[i] = i % Tp < T ? src[(long long)(i / Tp) * T + i % Tp] : 0;
 }
 
 // logits [B, Tp, ld] -> out [B, T, V]; blockIdx.y is a row of out.  Rows of an odd V start on any 4-byte boundary.
-__global__ void __launch_bounds__(256) copy_logits_kernel(const float* __restrict__ src, long long ld, float* __restrict__ dst, int T, int Tp, int V) {
+__global__ void __launch_bounds__(256) copy_logits_kernel(const float* src, long long ld, float* __restrict__ dst, int T, int Tp, int V) {
     chain_begin();
     const int row = blockIdx.y;
     const float* s = src + ((long long)(row / T) * Tp + row % T) * ld;
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(256) copy_logits_kernel(const float* __restric
     for (int c = blockIdx.x * 1024 + threadIdx.x; c < V; c += gridDim.x * 1024) {
         float v[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = c + 256 * e < V ? __ldcs(s + c + 256 * e) : 0.f;
+        for (int e = 0; e < 4; ++e) v[e] = c + 256 * e < V ? ld_stream(s + c + 256 * e) : 0.f;
 #pragma unroll
         for (int e = 0; e < 4; ++e)
             if (c + 256 * e < V) __stcs(d + c + 256 * e, v[e]);

@@ -21,10 +21,11 @@
 
 namespace {
 
-__global__ void __launch_bounds__(256) embedding_fwd_kernel(const float* __restrict__ w, const long long* __restrict__ ids,
+__global__ void __launch_bounds__(256) embedding_fwd_kernel(const float* w, const long long* ids,
                                                             long long n_ids, int C, long long V, float* __restrict__ out,
                                                             int vec, unsigned int* err) {
     chain_begin();
+    w = chained(w); ids = chained(ids);
     const int lane = threadIdx.x & 31;
     const long long n = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (n >= n_ids) return;
@@ -44,10 +45,10 @@ __global__ void __launch_bounds__(256) embedding_fwd_kernel(const float* __restr
 }
 
 // One block per token n.  The block whose token is the first occurrence of its id writes the row.
-__global__ void __launch_bounds__(256) embedding_bwd_kernel(const float* __restrict__ dout,
-                                                            const long long* __restrict__ ids, long long n_ids, int C,
+__global__ void __launch_bounds__(256) embedding_bwd_kernel(const float* dout, const long long* ids, long long n_ids, int C,
                                                             long long V, float* __restrict__ dw) {
     chain_wait();
+    dout = chained(dout); ids = chained(ids);
     __shared__ unsigned char s_flag[256];
     const long long n = blockIdx.x;
     const long long id = ids[n];
@@ -99,11 +100,11 @@ __device__ __forceinline__ void lse_merge(float& m, float& s, float m2, float s2
 // One pass over the row: every thread keeps a running maximum and the sum of exponentials relative to it (the
 // sum is rescaled when the maximum grows), four values at a time when the row is 16-byte aligned; the 256 pairs
 // are merged at the end.  A two-pass version (maximum, then sum) read the 206 MB of logits twice from DRAM.
-__global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const float* __restrict__ logits, long long ld,
-                                                                const long long* __restrict__ targets, long long V,
+__global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const float* logits, long long ld, const long long* targets, long long V,
                                                                 float* __restrict__ lse, float* __restrict__ picked,
                                                                 unsigned int* err) {
     chain_wait();
+    logits = chained(logits); targets = chained(targets);
     __shared__ float red_m[8], red_s[8];
     const long long row = blockIdx.x;
     const float* x = logits + row * ld;
@@ -141,9 +142,10 @@ __global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const float* __r
     }
 }
 
-__global__ void __launch_bounds__(1024) cross_entropy_loss_kernel(const float* __restrict__ picked, long long rows,
+__global__ void __launch_bounds__(1024) cross_entropy_loss_kernel(const float* picked, long long rows,
                                                                   float neg_inv_rows, float* __restrict__ loss) {
     chain_wait();
+    picked = chained(picked);
     __shared__ float red[32];
     float s = 0.f;
     for (long long j = threadIdx.x; j < rows; j += 1024) s += picked[j];
@@ -159,12 +161,11 @@ __global__ void __launch_bounds__(1024) cross_entropy_loss_kernel(const float* _
     }
 }
 
-__global__ void __launch_bounds__(256) cross_entropy_bwd_kernel(const float* __restrict__ logits, long long ld,
-                                                                const long long* __restrict__ targets,
-                                                                const float* __restrict__ lse, long long V, float g,
-                                                                float upstream, float* __restrict__ dlogits,
+__global__ void __launch_bounds__(256) cross_entropy_bwd_kernel(const float* logits, long long ld, const long long* targets, const float* lse,
+                                                                long long V, float g, float upstream, float* dlogits,
                                                                 long long ldd, int vec) {
     chain_wait();
+    logits = chained(logits); targets = chained(targets); lse = chained(lse);
     const long long row = blockIdx.y;
     const float* x = logits + row * ld;
     float* d = dlogits + row * ldd;
@@ -204,12 +205,12 @@ __global__ void __launch_bounds__(256) cross_entropy_bwd_kernel(const float* __r
 // The same gradient written as the f16 pair the tensor-core head products read (gemm_f16x3_sm100.cu):
 // v = dlogit * scale, hi = f16(v), lo = f16((v - hi) * 2^11).  |dlogit| <= 1/rows, so scale = rows * 4096 keeps
 // hi within +-4096 and the smallest probabilities that matter well inside the f16 range.
-__global__ void __launch_bounds__(256) cross_entropy_bwd_split_kernel(const float* __restrict__ logits, long long ld,
-                                                                      const long long* __restrict__ targets,
-                                                                      const float* __restrict__ lse, long long V, float g,
+__global__ void __launch_bounds__(256) cross_entropy_bwd_split_kernel(const float* logits, long long ld, const long long* targets,
+                                                                      const float* lse, long long V, float g,
                                                                       float upstream, float scale, __half* __restrict__ hi,
                                                                       __half* __restrict__ lo, long long ldd) {
     chain_wait();
+    logits = chained(logits); targets = chained(targets); lse = chained(lse);
     const long long row = blockIdx.y;
     const float* x = logits + row * ld;
     __half* dh = hi + row * ldd;

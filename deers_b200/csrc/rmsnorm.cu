@@ -27,12 +27,14 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // BWD = false: y = x * inv, inv_out[row] = inv.   BWD = true: dx from x, dy and the saved inv.
 template <bool BWD, bool VEC, bool VEC2 = false>
-__global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ dy,
-                                                      const float* __restrict__ add, float* __restrict__ out,
-                                                      float* __restrict__ inv_io, long long rows, int C, float eps,
+__global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const float* dy, const float* add, float* __restrict__ out,
+                                                      float* inv_io, long long rows, int C, float eps,
                                                       float inv_n) {
     if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room)
     chain_wait();
+    x = chained(x); inv_io = chained(inv_io);
+    if (BWD) dy = chained(dy);
+    if (BWD && add) add = chained(add);
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * 8;
@@ -145,12 +147,14 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
 
 // Rows of 1025 .. 8192 elements: a whole block owns a row, which still stays in registers (one pass over HBM).
 template <bool BWD>
-__global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* __restrict__ x, const float* __restrict__ dy,
-                                                            const float* __restrict__ add, float* __restrict__ out,
-                                                            float* __restrict__ inv_io, long long rows, int C, float eps,
+__global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* x, const float* dy, const float* add, float* __restrict__ out,
+                                                            float* inv_io, long long rows, int C, float eps,
                                                             float inv_n) {
     if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room)
     chain_wait();
+    x = chained(x); inv_io = chained(inv_io);
+    if (BWD) dy = chained(dy);
+    if (BWD && add) add = chained(add);
     __shared__ float part[8];
     const int nv = C / 4;                                       // <= 256 * RN_MAXV
     for (long long row = blockIdx.x; row < rows; row += gridDim.x) {

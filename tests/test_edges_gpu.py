@@ -235,3 +235,41 @@ def test_chained_kernels_see_their_predecessors(B, H, T, D, dtype):
     for g in got + [captured]:
         for a, b in zip(g, want):
             assert torch.equal(a, b)
+
+
+def gpt_run(tc_head):
+    """Forwards of several lengths, a backward and three optimizer steps of a small model, launched kernel by kernel."""
+    from deers_b200 import gpt
+    from oracle import ref
+    V, L, H, C, Hm, T, B = (1100 if tc_head else 300), 2, 2, 64, 128, 70, 2
+    m = gpt.GPT(gpt.GPTConfig(V, T, L, H, C, Hm), torch.device("cuda", torch.cuda.current_device()), B)
+    m.load_parameters(ref.gpt_init_params((V, L, H, C, Hm), seed=11))
+    m.set_graph(False)
+    rng = np.random.default_rng(12)
+    ids, tgt = (torch.from_numpy(rng.integers(0, V, (B, T))).cuda() for _ in range(2))
+    out = [m.forward(ids[:, :t].contiguous()) for t in (1, 33, 64, 70)]
+    out.append(m.forward_backward(ids, tgt))
+    for _ in range(3):
+        out += list(m.train_step(ids, tgt, lr=1e-2, weight_decay=0.1, max_grad_norm=1.0))
+        out.append(m.forward(ids))
+    m.ctx.sync()
+    return [t.cpu().numpy() for t in out] + [m.parameter(i) for i in range(m.num_parameters())] + [m.grad(i) for i in range(m.num_parameters())]
+
+
+@pytest.mark.parametrize("tc_head", [True, False])
+def test_chained_gpt_kernels_see_their_predecessors(tc_head, tmp_path):
+    """The kernels of a model's forward, backward and optimizer step, each started while the one before it ends, give bit for
+    bit what they give in a process where every launch is waited for."""
+    import os
+    import subprocess
+    import sys
+    path = str(tmp_path / "want.npz")
+    code = f"import numpy as np; from tests.test_edges_gpu import gpt_run; np.savez({path!r}, *gpt_run({tc_head}))"
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=root, timeout=300, env=dict(os.environ, CUDA_LAUNCH_BLOCKING="1"))
+    want = np.load(path)
+    for _ in range(3):
+        got = gpt_run(tc_head)
+        assert len(got) == len(want.files)
+        for i, g in enumerate(got):
+            assert np.array_equal(g, want[f"arr_{i}"], equal_nan=True), i
