@@ -89,7 +89,8 @@ struct deers_gpt {
     // CUDA graphs of the forward alone, one per (B, padded T); the least recently used goes first
     FwdGraph fwd_graph[FWD_GRAPHS];
     unsigned long long fwd_clock;
-    bool head_pair_current;      // w_hi / w_lo hold the present head weight
+    bool head_pair_current;      // w_hi / w_lo hold the present head weight (of calls that ran, not of calls that were captured)
+    bool captured_updates;       // the caller holds a captured training step: its replays change the weights unseen
 };
 
 namespace {
@@ -332,6 +333,14 @@ int stage_ids(deers_gpt* m, const int64_t* ids, const int64_t* targets, long lon
     return DEERS_OK;
 }
 
+// True while the caller records this stream: what is enqueued now runs later, any number of times or never, so nothing
+// about the present may be concluded from it.
+bool recording(const deers_gpt* m) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(m->ctx->stream, &st) != cudaSuccess) { cudaGetLastError(); return false; }
+    return st != cudaStreamCaptureStatusNone;
+}
+
 void drop_graph(deers_gpt* m) {
     if (m->graph_exec) cudaGraphExecDestroy(m->graph_exec);
     m->graph_exec = nullptr;
@@ -417,9 +426,10 @@ void drop_fwd_graphs(deers_gpt* m) {
 // afterwards.
 int run_forward(deers_gpt* m, int B, int T) {
     deers_ctx* ctx = m->ctx;
-    if (m->tc_head && !m->head_pair_current) {
+    const bool rec = recording(m);
+    if (m->tc_head && (rec || m->captured_updates || !m->head_pair_current)) {
         GPT_TRY(launch_split_f16x3(ctx, m->cfg.n_embd, m->cfg.vocab_size, m->arena[0] + m->off_lm, m->Vld, 1.0f, m->w_hi, m->w_lo, m->Vld));
-        m->head_pair_current = true;
+        if (!rec) m->head_pair_current = true;
     }
     if (!m->graph_enabled || ctx->timing) return forward(m, m->ids_dev, B, T, false);
     FwdGraph* slot = &m->fwd_graph[0];
@@ -433,9 +443,7 @@ int run_forward(deers_gpt* m, int B, int T) {
         slot->B = B; slot->T = T;
     }
     slot->last_use = ++m->fwd_clock;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool free_stream = ctx->stream != cudaStreamLegacy && cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess &&
-                             cap == cudaStreamCaptureStatusNone;
+    const bool free_stream = ctx->stream != cudaStreamLegacy && !rec;
     if (!slot->exec && slot->ran && free_stream) {
         cudaGraph_t graph = nullptr;
         if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
@@ -502,7 +510,7 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
     m->tc_head = cfg->vocab_size >= 1024 && cfg->n_embd % 8 == 0 && cfg->n_embd >= 64;
     m->graph_enabled = true; m->graph_exec = nullptr; m->graph_B = m->graph_T = -1; m->eager_steps_BT = 0;
     m->on_side = false;
-    m->head_pair_current = false; m->fwd_clock = 0;
+    m->head_pair_current = m->captured_updates = false; m->fwd_clock = 0;
     for (FwdGraph& g : m->fwd_graph) g = FwdGraph{};
     {
         // the weight-gradient stream and its markers; without them the step simply runs on one stream
@@ -726,7 +734,7 @@ extern "C" int deers_b200_gpt_forward_backward(deers_gpt* m, const int64_t* ids,
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     GPT_TRY(stage_ids(m, ids, targets, (long long)B * T, cudaMemcpyDeviceToDevice));
     GPT_TRY(run_fwd_bwd(m, B, T, false));
-    m->head_pair_current = m->tc_head;
+    if (!recording(m)) m->head_pair_current = m->tc_head;
     if (loss_dev)
         DEERS_CUDA_TRY(ctx, cudaMemcpyAsync(loss_dev, m->loss_dev, sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
     return DEERS_OK;
@@ -735,6 +743,7 @@ extern "C" int deers_b200_gpt_forward_backward(deers_gpt* m, const int64_t* ids,
 static int train_step_common(deers_gpt* m, int B, int T, const deers_adamw_hyper* hyper, double max_grad_norm) {
     GPT_TRY(run_fwd_bwd(m, B, T, true));
     m->head_pair_current = false;                                     // the update below changes the head weight
+    m->captured_updates = m->captured_updates || recording(m);
     // clip_grad_norm + step_with_grads; "if grad_norm.is_finite() { step }" of tinystories_train.rs:213-216
     return launch_adamw(m->ctx, (int)m->opt.size(), m->opt.data(), hyper, m->norm_dev, max_grad_norm, true);
 }

@@ -273,3 +273,64 @@ def test_chained_gpt_kernels_see_their_predecessors(tc_head, tmp_path):
         assert len(got) == len(want.files)
         for i, g in enumerate(got):
             assert np.array_equal(g, want[f"arr_{i}"], equal_nan=True), i
+
+
+def test_captured_gpt_forward_follows_the_weights():
+    """The caller captures a forward (and a training step): whatever was current on the host at capture time, a replay must use
+    the weights of the moment it runs, and an eager forward those that replays have left."""
+    from deers_b200 import gpt
+    from oracle import ref
+    V, L, H, C, Hm, T, B = 1100, 1, 2, 64, 128, 24, 1                     # the head on the tensor core
+    cfg = (V, L, H, C, Hm)
+    rng = np.random.default_rng(21)
+    ids, tgt = (torch.from_numpy(rng.integers(0, V, (B, T))).cuda() for _ in range(2))
+
+    def model(seed):
+        m = gpt.GPT(gpt.GPTConfig(V, T, L, H, C, Hm), torch.device("cuda", torch.cuda.current_device()), B)
+        m.load_parameters(ref.gpt_init_params(cfg, seed=seed))
+        return m
+
+    def captured(m, fn):
+        g = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g, stream=m.stream):
+            out = fn()
+        return g, out
+
+    def check(m, got, what):
+        torch.cuda.synchronize()
+        want = ref.gpt_step(cfg, [m.parameter(i) for i in range(m.num_parameters())], ids.cpu().numpy(), want_grads=False)["logits"]
+        assert_close(got.cpu().numpy().reshape(np.asarray(want).shape), want, 1e-4, what)      # f32 sums of up to 128 terms
+
+    # captured when the head's pair is current; replayed after a step, an upload, a step on the same model
+    m = model(31)
+    check(m, m.forward(ids), "eager")
+    g, out = captured(m, lambda: m.forward(ids))
+    g.replay()
+    check(m, out, "replay")
+    m.train_step(ids, tgt, lr=1e-1)
+    g.replay()
+    check(m, out, "replay after a step")
+    check(m, m.forward(ids), "eager after a replay")
+    m.load_parameters(ref.gpt_init_params(cfg, seed=32))
+    g.replay()
+    check(m, out, "replay after an upload")
+    # captured when the pair has never been made; the first eager forward runs before any replay
+    m = model(33)
+    g, out = captured(m, lambda: m.forward(ids))
+    check(m, m.forward(ids), "eager after a capture")
+    g.replay()
+    check(m, out, "first replay")
+    # forward and backward captured, then an eager forward
+    m = model(34)
+    g, out = captured(m, lambda: m.forward_backward(ids, tgt))
+    check(m, m.forward(ids), "eager after a captured backward")
+    # a captured training step moves the weights without a call
+    m = model(35)
+    m.forward(ids)
+    g, out = captured(m, lambda: m.train_step(ids, tgt, lr=1e-1))
+    check(m, m.forward(ids), "eager before the replay")
+    g.replay()
+    check(m, m.forward(ids), "eager after a replayed step")
+    g.replay()
+    check(m, m.forward(ids), "eager after two replayed steps")
