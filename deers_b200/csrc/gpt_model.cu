@@ -31,17 +31,6 @@ struct LayerAct {
     float *n1, *inv1, *qkv, *qk, *o, *lse, *x1, *inv2, *n2, *r, *h, *x2;
 };
 
-// The forward of a (batch, length) as a graph.  Sampling sends a prefix one token longer on every call, so lengths are
-// padded to a multiple of FWD_PAD: with a causal mask the rows behind a sequence's end change nothing in front of it.
-constexpr int FWD_PAD = 32;
-constexpr int FWD_GRAPHS = 8;
-struct FwdGraph {
-    int B, T;                    // B = 0: empty
-    bool ran;                    // has run eagerly once: the next call of this shape captures
-    cudaGraphExec_t exec;
-    unsigned long long last_use;
-};
-
 size_t align64(size_t n) { return (n + 63) / 64 * 64; }     // floats: 256-byte boundaries
 
 }  // namespace
@@ -86,9 +75,6 @@ struct deers_gpt {
     cudaGraphExec_t graph_exec;
     int graph_B, graph_T;
     int eager_steps_BT;          // eager steps run at (graph_B, graph_T) before capturing
-    // CUDA graphs of the forward alone, one per (B, padded T); the least recently used goes first
-    FwdGraph fwd_graph[FWD_GRAPHS];
-    unsigned long long fwd_clock;
     bool head_pair_current;      // w_hi / w_lo hold the present head weight (of calls that ran, not of calls that were captured)
     bool captured_updates;       // the caller holds a captured training step: its replays change the weights unseen
 };
@@ -391,20 +377,11 @@ int run_fwd_bwd(deers_gpt* m, int B, int T, bool with_norm) {
     return DEERS_OK;
 }
 
-// ids [B, T] -> ids_dev [B, Tp], zeros behind each row's end
-__global__ void __launch_bounds__(256) pad_ids_kernel(const long long* src, long long* __restrict__ dst, int T, int Tp, int n) {
+// logits [rows, ld] -> out [rows, V]; blockIdx.y is a row.  Rows of an odd V start on any 4-byte boundary.
+__global__ void __launch_bounds__(256) copy_logits_kernel(const float* src, long long ld, float* __restrict__ dst, int V) {
     chain_begin();
-    src = chained(src);
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i < n) dst[i] = i % Tp < T ? src[(long long)(i / Tp) * T + i % Tp] : 0;
-}
-
-// logits [B, Tp, ld] -> out [B, T, V]; blockIdx.y is a row of out.  Rows of an odd V start on any 4-byte boundary.
-__global__ void __launch_bounds__(256) copy_logits_kernel(const float* src, long long ld, float* __restrict__ dst, int T, int Tp, int V) {
-    chain_begin();
-    const int row = blockIdx.y;
-    const float* s = src + ((long long)(row / T) * Tp + row % T) * ld;
-    float* d = dst + (long long)row * V;
+    const float* s = src + blockIdx.y * ld;
+    float* d = dst + (long long)blockIdx.y * V;
     for (int c = blockIdx.x * 1024 + threadIdx.x; c < V; c += gridDim.x * 1024) {
         float v[4];
 #pragma unroll
@@ -413,56 +390,6 @@ __global__ void __launch_bounds__(256) copy_logits_kernel(const float* src, long
         for (int e = 0; e < 4; ++e)
             if (c + 256 * e < V) __stcs(d + c + 256 * e, v[e]);
     }
-}
-
-void drop_fwd_graphs(deers_gpt* m) {
-    for (FwdGraph& g : m->fwd_graph) {
-        if (g.exec) cudaGraphExecDestroy(g.exec);
-        g = FwdGraph{};
-    }
-}
-
-// The forward on the ids staged as [B, T]: eagerly the first time a shape is seen, captured the second time, replayed
-// afterwards.
-int run_forward(deers_gpt* m, int B, int T) {
-    deers_ctx* ctx = m->ctx;
-    const bool rec = recording(m);
-    if (m->tc_head && (rec || m->captured_updates || !m->head_pair_current)) {
-        GPT_TRY(launch_split_f16x3(ctx, m->cfg.n_embd, m->cfg.vocab_size, m->arena[0] + m->off_lm, m->Vld, 1.0f, m->w_hi, m->w_lo, m->Vld));
-        if (!rec) m->head_pair_current = true;
-    }
-    if (!m->graph_enabled || ctx->timing) return forward(m, m->ids_dev, B, T, false);
-    FwdGraph* slot = &m->fwd_graph[0];
-    for (FwdGraph& g : m->fwd_graph) {
-        if (g.B == B && g.T == T) { slot = &g; break; }
-        if (g.last_use < slot->last_use) slot = &g;
-    }
-    if (slot->B != B || slot->T != T) {
-        if (slot->exec) cudaGraphExecDestroy(slot->exec);
-        *slot = FwdGraph{};
-        slot->B = B; slot->T = T;
-    }
-    slot->last_use = ++m->fwd_clock;
-    const bool free_stream = ctx->stream != cudaStreamLegacy && !rec;
-    if (!slot->exec && slot->ran && free_stream) {
-        cudaGraph_t graph = nullptr;
-        if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            const int rc = forward(m, m->ids_dev, B, T, false);
-            const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
-            if (rc || ce != cudaSuccess || !graph || cudaGraphInstantiate(&slot->exec, graph, 0) != cudaSuccess) slot->exec = nullptr;
-            if (graph) cudaGraphDestroy(graph);
-            if (rc) return rc;
-        }
-        if (!slot->exec) cudaGetLastError();                          // stays eager
-    }
-    if (slot->exec) {
-        DEERS_CUDA_TRY(ctx, cudaGraphLaunch(slot->exec, ctx->stream));
-        ctx->launches += 1;
-        return DEERS_OK;
-    }
-    GPT_TRY(forward(m, m->ids_dev, B, T, false));
-    slot->ran = free_stream;
-    return DEERS_OK;
 }
 
 const char* kBlockNames[6] = {"attn.q_proj", "attn.k_proj", "attn.v_proj", "attn.out_proj", "mlp.up_proj", "mlp.down_proj"};
@@ -510,8 +437,7 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
     m->tc_head = cfg->vocab_size >= 1024 && cfg->n_embd % 8 == 0 && cfg->n_embd >= 64;
     m->graph_enabled = true; m->graph_exec = nullptr; m->graph_B = m->graph_T = -1; m->eager_steps_BT = 0;
     m->on_side = false;
-    m->head_pair_current = m->captured_updates = false; m->fwd_clock = 0;
-    for (FwdGraph& g : m->fwd_graph) g = FwdGraph{};
+    m->head_pair_current = m->captured_updates = false;
     {
         // the weight-gradient stream and its markers; without them the step simply runs on one stream
         bool ok = cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking) == cudaSuccess;
@@ -635,7 +561,6 @@ extern "C" void deers_b200_gpt_destroy(deers_gpt* m) {
     cudaSetDevice(m->ctx->device);
     cudaStreamSynchronize(m->ctx->stream);
     drop_graph(m);
-    drop_fwd_graphs(m);
     if (m->side) { cudaStreamSynchronize(m->side); cudaStreamDestroy(m->side); }
     {
         cudaEvent_t evs[6] = {m->ev_fork, m->ev_join, m->ev_done[0], m->ev_done[1], m->ev_done[2], m->ev_done[3]};
@@ -699,7 +624,7 @@ extern "C" int deers_b200_gpt_param_get(deers_gpt* m, int index, int what, float
 extern "C" int deers_b200_gpt_set_graph(deers_gpt* m, int enable) {
     if (!m) return DEERS_ERR_NULL;
     m->graph_enabled = enable != 0;
-    if (!enable) { drop_fwd_graphs(m); drop_graph(m); m->graph_B = m->graph_T = -1; }
+    if (!enable) { drop_graph(m); m->graph_B = m->graph_T = -1; }
     return DEERS_OK;
 }
 
@@ -710,16 +635,13 @@ extern "C" int deers_b200_gpt_forward(deers_gpt* m, const int64_t* ids, int32_t 
     GPT_TRY(check_bt(m, B, T));
     deers_ctx* ctx = m->ctx;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    int Tp = (T + FWD_PAD - 1) / FWD_PAD * FWD_PAD;
-    if (Tp > m->cfg.sequence_len) Tp = m->cfg.sequence_len;           // the rotary cache and the buffers end there
-    const int n = B * Tp;
-    launch_chained(ctx, pad_ids_kernel, (n + 255) / 256, 256, 0, 1, (const long long*)ids, m->ids_dev, T, Tp, n);
-    ctx->launches += 1;
-    GPT_TRY(run_forward(m, B, Tp));
+    const bool rec = recording(m), kept = m->head_pair_current && !m->captured_updates && !rec;
+    GPT_TRY(forward(m, (const long long*)ids, B, T, !kept));
+    if (!rec) m->head_pair_current = m->tc_head;
     if (logits) {
         const int V = m->cfg.vocab_size;
         const dim3 grid((unsigned)((V + 4095) / 4096), (unsigned)(B * T));
-        launch_chained(ctx, copy_logits_kernel, grid, 256, 0, 1, m->logits, m->Vld, logits, T, Tp, V);
+        launch_chained(ctx, copy_logits_kernel, grid, 256, 0, 1, m->logits, m->Vld, logits, V);
         ctx->launches += 1;
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());

@@ -94,7 +94,7 @@ def test_f32_attention_tiles_and_groups(T, D, causal):
 
 
 def test_gpt_forward_lengths_share_graphs_and_follow_the_weights():
-    """Lengths are padded to shared graphs (eager, captured, replayed): every length must give what the oracle gives,
+    """Every length must give what the oracle gives, in whatever order lengths come,
     before and after an optimizer step and after a weight upload (the head's f16 pair is kept between calls)."""
     from deers_b200 import gpt
     from oracle import ref
@@ -334,3 +334,32 @@ def test_captured_gpt_forward_follows_the_weights():
     check(m, m.forward(ids), "eager after a replayed step")
     g.replay()
     check(m, m.forward(ids), "eager after two replayed steps")
+
+
+def test_gpt_forward_costs_what_its_tokens_cost():
+    """A length seen for the first time goes the way of every other (the same launches in every call), and a batch of short
+    sequences computes its tokens, not whole blocks of them."""
+    from deers_b200 import gpt
+    V, L, H, C, Hm, T, B = 8192, 2, 4, 128, 512, 64, 256
+    m = gpt.GPT(gpt.GPTConfig(V, T, L, H, C, Hm), torch.device("cuda", torch.cuda.current_device()), B)
+    ids = torch.zeros((B, T), dtype=torch.int64, device="cuda")
+    m.forward(ids)                                                          # makes the head's pair
+    for t in (5, 6, 37):
+        part, counts = ids[:3, :t].contiguous(), []
+        for _ in range(4):
+            before = m.ctx.launch_count()
+            m.forward(part)
+            counts.append(m.ctx.launch_count() - before)
+        assert len(set(counts)) == 1, counts
+
+    def ms(t):
+        part, best = ids[:, :t].contiguous(), float("inf")
+        for _ in range(6):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            m.forward(part)
+            ev[1].record()
+            torch.cuda.synchronize()
+            best = min(best, ev[0].elapsed_time(ev[1]))
+        return best
+    assert ms(33) < 0.8 * ms(64)                                            # 0.52 of the tokens
