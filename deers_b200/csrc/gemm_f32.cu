@@ -39,6 +39,7 @@ struct GemmArgs {
     int a_vec, b_vec, c_vec; // 16-byte accesses allowed
     int epi;
     int k_chunk;             // K elements per part (multiple of BK)
+    int tall;                // blockIdx.x counts tile rows, blockIdx.y tile columns (more than 65535 tile rows)
 };
 
 __device__ __forceinline__ float4 ld4(const float* p, int valid, bool vec) {
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(128 * KS) gemm_f32_kernel(const GemmArgs g) {
     const int tid = threadIdx.x % 128, kg = threadIdx.x / 128;      // position in the tile, k group
     const int w = tid / 32, lane = tid % 32;
     const int ty = (w & 1) * 4 + lane / 8, tx = (w >> 1) * 8 + lane % 8;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int m0 = (g.tall ? blockIdx.x : blockIdx.y) * BM, n0 = (g.tall ? blockIdx.y : blockIdx.x) * BN;
     const int kbeg = blockIdx.z * g.k_chunk;
     const int kend = min(g.K, kbeg + g.k_chunk);
     const int nk = kend > kbeg ? (kend - kbeg + BK - 1) / BK : 0;
@@ -378,7 +379,9 @@ int launch_variant(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g) {
     using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
     const auto kernel = gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>;
     DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>), S::SMEM);
-    DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, dim3(p.tiles_n, p.tiles_m, p.parts), S::GT, S::SMEM, dim3(1, 1, p.parts), g));
+    // gridDim.y ends at 65535.  Products with more tile rows than that have few tile columns (or C would not fit any device).
+    const dim3 grid = g.tall ? dim3(p.tiles_m, p.tiles_n, p.parts) : dim3(p.tiles_n, p.tiles_m, p.parts);
+    DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, grid, S::GT, S::SMEM, dim3(1, 1, p.parts), g));
     return DEERS_OK;
 }
 
@@ -405,6 +408,7 @@ int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long lo
     g.c_vec = ((uintptr_t)c & 15u) == 0 && ldc % 4 == 0 && (!r || (((uintptr_t)r & 15u) == 0 && ldr % 4 == 0)) &&
               (!aux || ((uintptr_t)aux & 15u) == 0);
     g.k_chunk = p.k_chunk;
+    g.tall = p.tiles_m > 65535;
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM);
         if (p.cfg == 0) rc = launch_orders<8, 8, 2>(ctx, p, g, a_mn, b_mn);

@@ -363,3 +363,18 @@ def test_gpt_forward_costs_what_its_tokens_cost():
             best = min(best, ev[0].elapsed_time(ev[1]))
         return best
     assert ms(33) < 0.8 * ms(64)                                            # 0.52 of the tokens
+
+
+@pytest.mark.parametrize("M,N,K", [(3_000_000, 32, 256), (4_300_000, 128, 8), (4_200_001, 3, 5)])
+def test_f32_gemm_more_tile_rows_than_a_grid_has(M, N, K):
+    """Row tiles beyond 65535, with the tile variants a narrow and a wider product take."""
+    from deers_b200 import gpt
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    a, b = torch.randn((M, K), device="cuda", generator=gen), torch.randn((K, N), device="cuda", generator=gen)
+    got = gpt.gemm_f32(a, b)
+    worst = 0.0
+    for r in range(0, M, 1 << 19):
+        want = a[r:r + (1 << 19)].double() @ b.double()
+        worst = max(worst, (got[r:r + (1 << 19)].double() - want).abs().max().item())
+    # K products of unit normals: partial sums stay within 6 sqrt(K), each of the K additions rounds by 2^-24 of that
+    assert worst <= 6.0 * K ** 0.5 * K * 2.0 ** -24
