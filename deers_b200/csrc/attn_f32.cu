@@ -561,14 +561,15 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
     merge_store<DP>(p, grp0, L::BWD_GROUP, p.dq + b * p.sdq.b + h * p.sdq.h, p.sdq.t, q0);
 }
 
-// Both roles in one launch: blockIdx.y = 2 n is the n-th heaviest key tile, 2 n + 1 the n-th heaviest query tile.
+// Both roles in one launch: row n of the grid holds every slice's n-th heaviest key tile, then every slice's n-th heaviest query
+// tile (gridDim.y ends at 65535; the longest sequence, 2^20, has 32768 tiles of a kind).
 template <int DP>
 __global__ void __launch_bounds__(NT, DP <= 64 ? 2 : 1) attn_bwd_f32_kernel(const F32Params p) {
     chain_wait();
     extern __shared__ __align__(16) float smem[];
-    const int n = blockIdx.y >> 1, tiles = (p.T + BM - 1) / BM;
-    if ((blockIdx.y & 1) == 0) bwd_dkdv<DP>(p, smem, n, blockIdx.x);
-    else bwd_dq<DP>(p, smem, tiles - 1 - n, blockIdx.x);
+    const int n = blockIdx.y, slices = p.B * p.H, x = blockIdx.x;
+    if (x < slices) bwd_dkdv<DP>(p, smem, n, x);
+    else bwd_dq<DP>(p, smem, (int)gridDim.y - 1 - n, x - slices);
 }
 
 Strides3 s3(const int64_t* s) { return Strides3{(long long)s[0], (long long)s[1], (long long)s[2]}; }
@@ -593,8 +594,7 @@ int fwd_impl(deers_ctx* ctx, const F32Params& p) {
 template <int DP>
 int bwd_impl(deers_ctx* ctx, const F32Params& p) {
     DEERS_SMEM_ONCE(ctx, (attn_bwd_f32_kernel<DP>), Tile<DP>::BWD_SMEM);
-    const dim3 grid(p.B * p.H, 2 * ((p.T + BM - 1) / BM));
-    if (grid.y > 65535) return DEERS_ERR_SHAPE;
+    const dim3 grid(2 * p.B * p.H, (p.T + BM - 1) / BM);
     {
         KernelTimerScope ts(ctx, DEERS_K_BWD_MAIN);
         launch_chained(ctx, attn_bwd_f32_kernel<DP>, grid, NT, Tile<DP>::BWD_SMEM, 1, p);

@@ -378,3 +378,22 @@ def test_f32_gemm_more_tile_rows_than_a_grid_has(M, N, K):
         worst = max(worst, (got[r:r + (1 << 19)].double() - want).abs().max().item())
     # K products of unit normals: partial sums stay within 6 sqrt(K), each of the K additions rounds by 2^-24 of that
     assert worst <= 6.0 * K ** 0.5 * K * 2.0 ** -24
+
+
+def test_f32_attention_backward_of_the_longest_sequence():
+    """T = 2^20 has as many row tiles as the grid can hold.  With K = 0 the weights of row i are 1 / (i + 1), with V = 1 the
+    output is 1 and dS is 0, so every result has a closed form."""
+    from deers_b200 import ops
+    T, D = 1 << 20, 4
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    q, do = (torch.randn((1, 1, T, D), device="cuda", generator=gen) for _ in range(2))
+    k, v = torch.zeros_like(q), torch.ones_like(q)
+    n = torch.arange(1, T + 1, dtype=torch.float64, device="cuda")
+    dq, dk, dv = ops.attention_bwd(q, k, v, torch.ones_like(q), n.log().float()[None, None], do, ops.default_scale(D))
+    assert dq.abs().max() == 0.0
+    want = torch.flip(torch.cumsum(torch.flip(do[0, 0].double() / n[:, None], (0,)), 0), (0,))
+    # weights carry the rounding of lse * log2(e) (14 * 2^-23); a group adds 2^18 terms whose magnitudes sum to 3.5 ln(T) at
+    # most, and the errors of the additions add up like a random walk
+    assert (dv[0, 0].double() - want).abs().max() <= (14 * 2.0 ** -23 + 2.0 ** 9 * 2.0 ** -24) * 3.5 * 14
+    # dS = P (dP - delta): two sums of D products that cancel up to their rounding, times Q
+    assert dk.abs().max() <= 2 * D * 2.0 ** -24 * 6 * 14 * 6
