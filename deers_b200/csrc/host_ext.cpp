@@ -6,6 +6,8 @@
 // allocations (torch's caching allocator, without the dispatcher) and the C-ABI call happen in one native function.
 // The functions answer None for anything they do not take as it is (wrong type, shape, device or a layout
 // that needs compaction); the Python mirror then raises the matching error or compacts and calls again.
+// Allocations and library calls run without the interpreter lock (a launch waits while the device's queue is full); a lock
+// per context keeps the threads that share a stream, and so a context, apart.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -15,6 +17,9 @@
 
 #include <string.h>
 
+#include <atomic>
+#include <memory>
+#include <mutex>
 #include <vector>
 
 #include "../../include/deers_b200.h"
@@ -24,25 +29,36 @@ namespace {
 PyObject* g_make_context = nullptr;      // ops.Context: device index -> handle as an int
 PyObject* g_raise_status = nullptr;      // (status, handle) -> raises CudaError
 
-struct CtxEntry { int device; cudaStream_t stream; deers_ctx* handle; };
-std::vector<CtxEntry> g_contexts;        // guarded by the GIL; the Python side keeps every context alive
+struct Ctx { int device; cudaStream_t stream; deers_ctx* handle; std::mutex mu; };
+std::vector<std::unique_ptr<Ctx>> g_contexts;        // guarded by the GIL; the Python side keeps every context alive
 
 // The library context of the tensor's device and torch's current stream there; nullptr with an exception set.
-deers_ctx* context_for(int device) {
+Ctx* context_for(int device) {
     const cudaStream_t s = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
-    for (const CtxEntry& e : g_contexts)
-        if (e.stream == s && e.device == device) return e.handle;
+    for (const auto& e : g_contexts)
+        if (e->stream == s && e->device == device) return e.get();
     PyObject* r = PyObject_CallFunction(g_make_context, "i", device);
     if (!r) return nullptr;
     void* p = PyLong_AsVoidPtr(r);
     Py_DECREF(r);
     if (!p) return nullptr;
-    g_contexts.push_back({device, s, (deers_ctx*)p});
-    return (deers_ctx*)p;
+    std::unique_ptr<Ctx> e(new Ctx());
+    e->device = device; e->stream = s; e->handle = (deers_ctx*)p;
+    g_contexts.push_back(std::move(e));
+    return g_contexts.back().get();
 }
 
-PyObject* fail(int status, deers_ctx* ctx) {
-    PyObject* r = PyObject_CallFunction(g_raise_status, "iK", status, (unsigned long long)(uintptr_t)ctx);
+// The part of an operator that touches no Python object.
+struct NoGil {
+    PyThreadState* state;
+    NoGil() : state(PyEval_SaveThread()) {}
+    ~NoGil() { PyEval_RestoreThread(state); }
+    NoGil(const NoGil&) = delete;
+    NoGil& operator=(const NoGil&) = delete;
+};
+
+PyObject* fail(int status, const Ctx* ctx) {
+    PyObject* r = PyObject_CallFunction(g_raise_status, "iK", status, (unsigned long long)(uintptr_t)ctx->handle);
     Py_XDECREF(r);
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "deers_b200 call failed");
     return nullptr;
@@ -137,24 +153,30 @@ PyObject* attn_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (!q || !k || !v || !usable(*q) || !usable(*k) || !usable(*v) || !same(*q, *k) || !same(*q, *v)) Py_RETURN_NONE;
     const double scale = PyFloat_AsDouble(args[3]);
     if (scale == -1.0 && PyErr_Occurred()) return nullptr;
-    deers_ctx* ctx = context_for(q->get_device());
+    Ctx* ctx = context_for(q->get_device());
     if (!ctx) return nullptr;
-    at::Tensor o;
+    at::Tensor o, lse;
     if (args[6] != Py_None) {
         const at::Tensor* given = tensor(args[6]);
         if (!given || !usable(*given) || !same(*q, *given)) Py_RETURN_NONE;
         o = *given;
-    } else if (PyObject_IsTrue(args[5])) {
-        o = empty_like_of({q->size(0), q->size(2), q->size(1), q->size(3)}, q->scalar_type(), *q).permute({0, 2, 1, 3});
-    } else {
-        o = empty_like_of(q->sizes(), q->scalar_type(), *q);
     }
-    at::Tensor lse = empty_like_of(q->sizes().slice(0, 3), at::kFloat, *q);
+    const bool token_major = PyObject_IsTrue(args[5]);
     deers_attn_desc d;
     fill_desc(&d, *q, scale, PyObject_IsTrue(args[4]));
-    put_strides(d.q_strides, *q); put_strides(d.k_strides, *k); put_strides(d.v_strides, *v); put_strides(d.o_strides, o);
-    const int rc = deers_b200_attn_fwd(ctx, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o.data_ptr(),
-                                       (float*)lse.data_ptr(), nullptr, 0);
+    int rc;
+    {
+        NoGil unlocked;
+        if (!o.defined() && token_major)
+            o = empty_like_of({q->size(0), q->size(2), q->size(1), q->size(3)}, q->scalar_type(), *q).permute({0, 2, 1, 3});
+        else if (!o.defined())
+            o = empty_like_of(q->sizes(), q->scalar_type(), *q);
+        lse = empty_like_of(q->sizes().slice(0, 3), at::kFloat, *q);
+        put_strides(d.q_strides, *q); put_strides(d.k_strides, *k); put_strides(d.v_strides, *v); put_strides(d.o_strides, o);
+        std::lock_guard<std::mutex> one(ctx->mu);
+        rc = deers_b200_attn_fwd(ctx->handle, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o.data_ptr(), (float*)lse.data_ptr(),
+                                 nullptr, 0);
+    }
     if (rc) return fail(rc, ctx);
     return wrap2(std::move(o), std::move(lse));
     HOST_END
@@ -163,7 +185,7 @@ PyObject* attn_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // Whether the backward may take the larger workspace (the dS tiles kept between its kernels): when it is a small part
 // of what the device has free.  Asking the driver for the free memory costs tens of microseconds and more under
 // load, so an answer stands for every smaller request on that device until an allocation fails.
-size_t g_workspace_ok[64] = {0};
+std::atomic<size_t> g_workspace_ok[64];
 bool large_workspace_ok(deers_ctx* ctx, int device, size_t bytes) {
     if (device < 0 || device >= 64) return false;
     if (bytes <= g_workspace_ok[device]) return true;
@@ -184,40 +206,45 @@ PyObject* attn_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (!usable(*t) || !same(*q, *t)) Py_RETURN_NONE;
     const double scale = PyFloat_AsDouble(args[6]);
     if (scale == -1.0 && PyErr_Occurred()) return nullptr;
-    deers_ctx* ctx = context_for(q->get_device());
+    Ctx* ctx = context_for(q->get_device());
     if (!ctx) return nullptr;
-    at::Tensor dq = empty_like_of(q->sizes(), q->scalar_type(), *q), dk = empty_like_of(q->sizes(), q->scalar_type(), *q), dv;
+    at::Tensor dq, dk, dv, ws;
     if (args[9] != Py_None) {
         const at::Tensor* given = tensor(args[9]);
         if (!given || !usable(*given) || !same(*q, *given)) Py_RETURN_NONE;
         dv = *given;
-    } else {
-        dv = empty_like_of(q->sizes(), q->scalar_type(), *q);
     }
     deers_attn_desc d;
     fill_desc(&d, *q, scale, PyObject_IsTrue(args[7]));
-    put_strides(d.q_strides, *q); put_strides(d.k_strides, *k); put_strides(d.v_strides, *v); put_strides(d.o_strides, *o);
-    put_strides(d.do_strides, *g); put_strides(d.dq_strides, dq); put_strides(d.dk_strides, dk); put_strides(d.dv_strides, dv);
-    size_t need = deers_b200_attn_workspace_bytes(&d, 1);
-    at::Tensor ws;
+    const size_t need = deers_b200_attn_workspace_bytes(&d, 1);
     if (args[8] != Py_None) {
         const at::Tensor* given = tensor(args[8]);
         if (given && (size_t)(given->numel() * given->element_size()) >= need) ws = *given;
     }
-    if (!ws.defined()) {
-        const size_t fast = deers_b200_attn_workspace_bytes(&d, 2);
-        if (fast > need && large_workspace_ok(ctx, q->get_device(), fast)) {
-            try {
-                ws = scratch(fast, *q);
-            } catch (const c10::OutOfMemoryError&) {
-                g_workspace_ok[q->get_device()] = 0;             // recompute instead
+    int rc;
+    {
+        NoGil unlocked;
+        dq = empty_like_of(q->sizes(), q->scalar_type(), *q);
+        dk = empty_like_of(q->sizes(), q->scalar_type(), *q);
+        if (!dv.defined()) dv = empty_like_of(q->sizes(), q->scalar_type(), *q);
+        put_strides(d.q_strides, *q); put_strides(d.k_strides, *k); put_strides(d.v_strides, *v); put_strides(d.o_strides, *o);
+        put_strides(d.do_strides, *g); put_strides(d.dq_strides, dq); put_strides(d.dk_strides, dk); put_strides(d.dv_strides, dv);
+        if (!ws.defined()) {
+            const size_t fast = deers_b200_attn_workspace_bytes(&d, 2);
+            if (fast > need && large_workspace_ok(ctx->handle, q->get_device(), fast)) {
+                try {
+                    ws = scratch(fast, *q);
+                } catch (const c10::OutOfMemoryError&) {
+                    g_workspace_ok[q->get_device()] = 0;             // recompute instead
+                }
             }
+            if (!ws.defined()) ws = scratch(need < 256 ? 256 : need, *q);
         }
-        if (!ws.defined()) ws = scratch(need < 256 ? 256 : need, *q);
+        std::lock_guard<std::mutex> one(ctx->mu);
+        rc = deers_b200_attn_bwd(ctx->handle, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o->data_ptr(), (const float*)lse->data_ptr(),
+                                 g->data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(),
+                                 (size_t)(ws.numel() * ws.element_size()));
     }
-    const int rc = deers_b200_attn_bwd(ctx, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o->data_ptr(), (const float*)lse->data_ptr(),
-                                       g->data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(),
-                                       (size_t)(ws.numel() * ws.element_size()));
     if (rc) return fail(rc, ctx);
     PyObject* r = PyTuple_New(3);
     PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(std::move(dq)));
@@ -241,23 +268,29 @@ PyObject* attn_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_RETURN_NONE;
     const double scale = PyFloat_AsDouble(args[3]);
     if (scale == -1.0 && PyErr_Occurred()) return nullptr;
-    deers_ctx* ctx = context_for(q->get_device());
+    Ctx* ctx = context_for(q->get_device());
     if (!ctx) return nullptr;
     deers_decode_desc d;
     memset(&d, 0, sizeof(d));
     d.B = (int)q->size(0); d.H = (int)q->size(1); d.Tq = (int)q->size(2); d.Tk = (int)k->size(2); d.D = (int)q->size(3);
     d.dtype = dtype_code(*q); d.causal = PyObject_IsTrue(args[4]); d.scale = (float)scale;
     const bool want_lse = PyObject_IsTrue(args[5]);
-    at::Tensor o = empty_like_of(q->sizes(), q->scalar_type(), *q), lse;
-    if (want_lse) lse = empty_like_of(q->sizes().slice(0, 3), at::kFloat, *q);
-    put_strides(d.q_strides, *q); put_strides(d.k_strides, *k); put_strides(d.v_strides, *v); put_strides(d.o_strides, o);
-    // most calls need no workspace (the chunks of a slice meet in shared memory): ask for one only when told so
-    float* lse_p = want_lse ? (float*)lse.data_ptr() : nullptr;
-    int rc = deers_b200_attn_decode(ctx, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o.data_ptr(), lse_p, nullptr, 0);
-    if (rc == DEERS_ERR_WORKSPACE) {
-        const size_t need = deers_b200_attn_decode_workspace_bytes(&d);
-        at::Tensor ws = scratch(need < 256 ? 256 : need, *q);
-        rc = deers_b200_attn_decode(ctx, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o.data_ptr(), lse_p, ws.data_ptr(), need);
+    at::Tensor o, lse;
+    int rc;
+    {
+        NoGil unlocked;
+        o = empty_like_of(q->sizes(), q->scalar_type(), *q);
+        if (want_lse) lse = empty_like_of(q->sizes().slice(0, 3), at::kFloat, *q);
+        put_strides(d.q_strides, *q); put_strides(d.k_strides, *k); put_strides(d.v_strides, *v); put_strides(d.o_strides, o);
+        // most calls need no workspace (the chunks of a slice meet in shared memory): ask for one only when told so
+        float* lse_p = want_lse ? (float*)lse.data_ptr() : nullptr;
+        std::lock_guard<std::mutex> one(ctx->mu);
+        rc = deers_b200_attn_decode(ctx->handle, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o.data_ptr(), lse_p, nullptr, 0);
+        if (rc == DEERS_ERR_WORKSPACE) {
+            const size_t need = deers_b200_attn_decode_workspace_bytes(&d);
+            at::Tensor ws = scratch(need < 256 ? 256 : need, *q);
+            rc = deers_b200_attn_decode(ctx->handle, &d, q->data_ptr(), k->data_ptr(), v->data_ptr(), o.data_ptr(), lse_p, ws.data_ptr(), need);
+        }
     }
     if (rc) return fail(rc, ctx);
     if (!want_lse) return THPVariable_Wrap(std::move(o));
@@ -273,11 +306,18 @@ PyObject* gemm_f16(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     const at::Tensor *a = tensor(args[3]), *b = tensor(args[5]);
     if (!a || !b || a->dim() != 2 || b->dim() != 2 || !a->is_cuda()) Py_RETURN_NONE;
-    deers_ctx* ctx = context_for(a->get_device());
+    Ctx* ctx = context_for(a->get_device());
     if (!ctx) return nullptr;
-    at::Tensor c = empty_like_of({M, N}, a->scalar_type(), *a);
-    const int rc = deers_b200_gemm_f16(ctx, (int)M, (int)N, (int)K, a->data_ptr(), a->stride(0), PyObject_IsTrue(args[4]), b->data_ptr(),
-                                       b->stride(0), PyObject_IsTrue(args[6]), c.data_ptr(), c.stride(0));
+    const int a_mn = PyObject_IsTrue(args[4]), b_mn = PyObject_IsTrue(args[6]);
+    at::Tensor c;
+    int rc;
+    {
+        NoGil unlocked;
+        c = empty_like_of({M, N}, a->scalar_type(), *a);
+        std::lock_guard<std::mutex> one(ctx->mu);
+        rc = deers_b200_gemm_f16(ctx->handle, (int)M, (int)N, (int)K, a->data_ptr(), a->stride(0), a_mn, b->data_ptr(), b->stride(0), b_mn,
+                                 c.data_ptr(), c.stride(0));
+    }
     if (rc) return fail(rc, ctx);
     return THPVariable_Wrap(std::move(c));
     HOST_END
@@ -292,7 +332,7 @@ PyObject* rope_pack(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (!src || !cs || !sn || !dst || src->dim() != 4 || dst->dim() != 4 || !src->is_cuda() || dtype_code(*src) < 0) Py_RETURN_NONE;
     const bool head_src = PyObject_IsTrue(args[4]);
     const at::Tensor& tok = head_src ? *dst : *src;
-    deers_ctx* ctx = context_for(src->get_device());
+    Ctx* ctx = context_for(src->get_device());
     if (!ctx) return nullptr;
     deers_rope_desc d;
     memset(&d, 0, sizeof(d));
@@ -303,7 +343,12 @@ PyObject* rope_pack(PyObject*, PyObject* const* args, Py_ssize_t n) {
         d.src_strides[i] = src->stride(head_src ? head_order[i] : tok_order[i]);
         d.dst_strides[i] = dst->stride(head_src ? tok_order[i] : head_order[i]);
     }
-    const int rc = deers_b200_rope_pack(ctx, &d, src->data_ptr(), cs->data_ptr(), sn->data_ptr(), dst->data_ptr());
+    int rc;
+    {
+        NoGil unlocked;
+        std::lock_guard<std::mutex> one(ctx->mu);
+        rc = deers_b200_rope_pack(ctx->handle, &d, src->data_ptr(), cs->data_ptr(), sn->data_ptr(), dst->data_ptr());
+    }
     if (rc) return fail(rc, ctx);
     Py_RETURN_TRUE;
     HOST_END

@@ -397,3 +397,51 @@ def test_f32_attention_backward_of_the_longest_sequence():
     assert (dv[0, 0].double() - want).abs().max() <= (14 * 2.0 ** -23 + 2.0 ** 9 * 2.0 ** -24) * 3.5 * 14
     # dS = P (dP - delta): two sums of D products that cancel up to their rounding, times Q
     assert dk.abs().max() <= 2 * D * 2.0 ** -24 * 6 * 14 * 6
+
+
+def test_other_threads_run_while_a_launch_waits():
+    """A launch blocks while the device's queue is full.  The operators hold no interpreter lock then: a second thread keeps
+    ticking; and two threads that share a stream get the results of one."""
+    import threading
+    import time
+    from deers_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn((1, 4, t, 64), device="cuda", generator=gen).half() for t in (1, 256, 256))
+    want = ops.attention_decode(q, k, v)
+    x, w = torch.randn((64, 64), device="cuda", generator=gen).half(), torch.randn((64, 64), device="cuda", generator=gen).half()
+    want_y = ops.Linear.new(x, w).forward()
+    torch.cuda.synchronize()
+    stop, gaps = threading.Event(), [0.0]
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(1e-3)
+            now = time.perf_counter()
+            gaps[0], last = max(gaps[0], now - last), now
+    t = threading.Thread(target=tick)
+    t.start()
+    begin = time.perf_counter()
+    torch.cuda._sleep(1_500_000_000)                                        # about 0.8 s of an idle kernel in front
+    outs = [ops.attention_decode(q, k, v) for _ in range(3000)]             # more than the queue holds
+    waited = time.perf_counter() - begin
+    stop.set()
+    t.join()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in outs)
+    assert waited > 0.4, "the queue never filled: nothing was tested"
+    assert gaps[0] < 0.25 * waited, (gaps[0], waited)
+
+    wrong = []
+
+    def work():
+        for _ in range(300):
+            o, y = ops.attention_decode(q, k, v), ops.Linear.new(x, w).forward()
+            if not (torch.equal(o, want) and torch.equal(y, want_y)):
+                wrong.append(1)
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
