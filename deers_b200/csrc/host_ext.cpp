@@ -11,13 +11,14 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <string.h>
 
-#include <atomic>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -182,17 +183,18 @@ PyObject* attn_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HOST_END
 }
 
-// Whether the backward may take the larger workspace (the dS tiles kept between its kernels): when it is a small part
-// of what the device has free.  Asking the driver for the free memory costs tens of microseconds and more under
-// load, so an answer stands for every smaller request on that device until an allocation fails.
-std::atomic<size_t> g_workspace_ok[64];
-bool large_workspace_ok(deers_ctx* ctx, int device, size_t bytes) {
-    if (device < 0 || device >= 64) return false;
-    if (bytes <= g_workspace_ok[device]) return true;
+// Whether the backward may take the larger workspace (the dS tiles kept between its kernels): when it is at most a quarter
+// of what is free, on the device or in torch's allocator.  Asked anew every time, except for sizes up to 1/512 of the device
+// (350 MB of 180 GB): the question costs 74 us of host time, which the forward in front of a larger backward hides (110 us and
+// more), a smaller one does not; and so little, when it does not fit, is noticed by the allocation itself.
+bool large_workspace_ok(deers_ctx* ctx, const at::Tensor& like, size_t bytes) {
+    const c10::DeviceIndex device = like.device().index();
+    if (bytes <= at::cuda::getDeviceProperties(device)->totalGlobalMem / 512) return true;
     size_t free_bytes = 0, total = 0;
-    if (deers_b200_mem_info(ctx, &free_bytes, &total) != DEERS_OK || bytes > free_bytes / 4) return false;
-    g_workspace_ok[device] = bytes;
-    return true;
+    if (deers_b200_mem_info(ctx, &free_bytes, &total) != DEERS_OK) return false;
+    const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats(device);
+    const int64_t kept = stats.reserved_bytes[0].current - stats.allocated_bytes[0].current;
+    return bytes <= (free_bytes + (size_t)(kept > 0 ? kept : 0)) / 4;
 }
 
 // attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace | None, dv_out | None) -> (dq, dk, dv) | None
@@ -231,12 +233,10 @@ PyObject* attn_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
         put_strides(d.do_strides, *g); put_strides(d.dq_strides, dq); put_strides(d.dk_strides, dk); put_strides(d.dv_strides, dv);
         if (!ws.defined()) {
             const size_t fast = deers_b200_attn_workspace_bytes(&d, 2);
-            if (fast > need && large_workspace_ok(ctx->handle, q->get_device(), fast)) {
+            if (fast > need && large_workspace_ok(ctx->handle, *q, fast)) {
                 try {
                     ws = scratch(fast, *q);
-                } catch (const c10::OutOfMemoryError&) {
-                    g_workspace_ok[q->get_device()] = 0;             // recompute instead
-                }
+                } catch (const c10::OutOfMemoryError&) {}        // recompute instead
             }
             if (!ws.defined()) ws = scratch(need < 256 ? 256 : need, *q);
         }

@@ -445,3 +445,42 @@ def test_other_threads_run_while_a_launch_waits():
     for t in threads:
         t.join()
     assert not wrong
+
+
+def backward_peak(call):
+    """Bytes a call takes at its peak beyond what was held before it."""
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    out = call()
+    torch.cuda.synchronize()
+    return torch.cuda.max_memory_allocated() - before, out
+
+
+def test_backward_weighs_its_workspace_against_the_memory_of_the_moment():
+    """The larger workspace is taken when it is at most a quarter of what is free: after a call that took it on an empty device,
+    one on a nearly full device must not; memory that torch's allocator holds unused counts as free."""
+    from deers_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v, do = (torch.randn((2, 16, 8192, 64), device="cuda", generator=gen).half() for _ in range(4))
+    scale = ops.default_scale(64)
+    o, lse = ops.attention_fwd(q, k, v, scale)
+    least, fast = (ops.workspace_bytes(q, scale, True, p) for p in (1, 2))
+    grads = 3 * q.numel() * 2
+    assert fast > torch.cuda.get_device_properties(0).total_memory // 512
+    torch.cuda.empty_cache()
+    peak, want = backward_peak(lambda: ops.attention_bwd(q, k, v, o, lse, do, scale))
+    assert peak >= fast + grads                                             # empty device: kept dS
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    fill = torch.empty(free - 2 * fast, dtype=torch.uint8, device="cuda")
+    peak, got = backward_peak(lambda: ops.attention_bwd(q, k, v, o, lse, do, scale))
+    assert peak < least + grads + (8 << 20), (peak, least, fast)            # half of what is left: recomputed
+    for a, b in zip(got, want):                                             # f16 rounding of the same dS values
+        assert_close(a.float().cpu().numpy(), b.float().cpu().numpy(), TOL_F16, "gradients")
+    del fill                                                                # unused, and still the allocator's
+    peak, got = backward_peak(lambda: ops.attention_bwd(q, k, v, o, lse, do, scale))
+    assert peak >= fast + grads
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    del got, want
+    torch.cuda.empty_cache()
