@@ -197,6 +197,14 @@ bool large_workspace_ok(deers_ctx* ctx, const at::Tensor& like, size_t bytes) {
     return bytes <= (free_bytes + (size_t)(kept > 0 ? kept : 0)) / 4;
 }
 
+// Bytes the backward uses of its workspace: what deers_b200_attn_workspace_bytes answers for the tile width, without the room
+// it keeps for the padded copies of other f16 head dims.
+size_t used_workspace_bytes(const deers_attn_desc& d, int pass) {
+    deers_attn_desc tile = d;
+    if (d.dtype == DEERS_F16 && d.D % 8 == 0 && d.D < 128) tile.D = d.D <= 64 ? 64 : 128;
+    return deers_b200_attn_workspace_bytes(&tile, pass);
+}
+
 // attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace | None, dv_out | None) -> (dq, dk, dv) | None
 PyObject* attn_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HOST_BEGIN
@@ -218,7 +226,7 @@ PyObject* attn_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
     deers_attn_desc d;
     fill_desc(&d, *q, scale, PyObject_IsTrue(args[7]));
-    const size_t need = deers_b200_attn_workspace_bytes(&d, 1);
+    const size_t need = used_workspace_bytes(d, 1);
     if (args[8] != Py_None) {
         const at::Tensor* given = tensor(args[8]);
         if (given && (size_t)(given->numel() * given->element_size()) >= need) ws = *given;
@@ -232,7 +240,7 @@ PyObject* attn_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
         put_strides(d.q_strides, *q); put_strides(d.k_strides, *k); put_strides(d.v_strides, *v); put_strides(d.o_strides, *o);
         put_strides(d.do_strides, *g); put_strides(d.dq_strides, dq); put_strides(d.dk_strides, dk); put_strides(d.dv_strides, dv);
         if (!ws.defined()) {
-            const size_t fast = deers_b200_attn_workspace_bytes(&d, 2);
+            const size_t fast = used_workspace_bytes(d, 2);
             if (fast > need && large_workspace_ok(ctx->handle, *q, fast)) {
                 try {
                     ws = scratch(fast, *q);

@@ -203,11 +203,8 @@ public:
         const auto& s = q_.layout().shape;
         lse_ = std::make_shared<CudaStorage>((size_t)(s[0] * s[1] * s[2]) * sizeof(float), DType::F32);
         deers_attn_desc d = desc(out_layout);
-        // scratch only for f16 head dims other than 64 / 128 (zero-padded copies)
-        const size_t fwd_ws = deers_b200_attn_workspace_bytes(&d, 0);
-        std::shared_ptr<CudaStorage> ws = fwd_ws ? std::make_shared<CudaStorage>(fwd_ws, DType::F32) : nullptr;
         rt.check(deers_b200_attn_fwd(rt.ctx(), &d, q_.storage().ptr(), k_.storage().ptr(), v_.storage().ptr(), o->ptr(),
-                                     (float*)lse_->ptr(), ws ? ws->ptr() : nullptr, fwd_ws));
+                                     (float*)lse_->ptr(), nullptr, 0));
         o_ = Tensor(o, out_layout);                                     // kept for the backward, like LogSumExp.lse
         return Tensor(o, out_layout, shared_from_this());
     }
@@ -225,8 +222,11 @@ public:
         fill_strides(d.dq_strides, gl); fill_strides(d.dk_strides, gl); fill_strides(d.dv_strides, gl);
         // The larger (pass 2) workspace lets the f16 backward keep its dS tiles between its kernels; taken when
         // it is a small part of what the device has free, else the backward recomputes (pass 1).
-        size_t ws_bytes = deers_b200_attn_workspace_bytes(&d, 1);
-        const size_t fast = deers_b200_attn_workspace_bytes(&d, 2);
+        // Both sizes are those of the tile width: other f16 head dims use no more.
+        deers_attn_desc tile = d;
+        if (d.dtype == DEERS_F16 && d.D % 8 == 0 && d.D < 128) tile.D = d.D <= 64 ? 64 : 128;
+        size_t ws_bytes = deers_b200_attn_workspace_bytes(&tile, 1);
+        const size_t fast = deers_b200_attn_workspace_bytes(&tile, 2);
         size_t free_b = 0, total_b = 0;
         if (fast > ws_bytes && deers_b200_mem_info(rt.ctx(), &free_b, &total_b) == DEERS_OK && fast <= free_b / 4) ws_bytes = fast;
         CudaStorage ws(ws_bytes ? ws_bytes : 256, DType::F32);

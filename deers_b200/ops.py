@@ -200,7 +200,9 @@ def attention_bwd(q, k, v, o, lse, d_o, scale: float, causal: bool = True, works
                   dv_out: Optional[torch.Tensor] = None):
     """Storage-level backward: returns (dq, dk, dv), each compact [B,H,T,D].  `workspace` (uint8, 256-byte
     aligned) of `workspace_bytes(q, pass_=2)` bytes selects the f16 backward that keeps dS tiles, of
-    `pass_=1` bytes the recomputing one; without it the function allocates.  `dv_out` (a [B,H,T,D] view
+    `pass_=1` bytes at head dims 64 and 128 the recomputing one (other head dims are answered more than they use:
+    ask with a q of the tile width, 64 or 128); without it the function allocates, for the kept tiles when that is at
+    most a quarter of the free memory or 1/512 of the device's.  `dv_out` (a [B,H,T,D] view
     with inner stride 1, e.g. the v slice of a fused dqkv buffer seen head-major) receives dV in place
     instead: the kernels write through its strides."""
     got = _host.attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace, dv_out)

@@ -123,15 +123,17 @@ int deers_b200_sync(deers_ctx* ctx);
  * multiple of 8 up to 128 runs on the 64- or 128-wide tensor-core tiles in place.  For f16 head dims other than 64 and
  * 128 the sizes returned here keep the room of the padded copies earlier builds made (four tensors of B*H*T*Dp halves
  * forward, eight backward; Dp = 64 or 128), so that memory plans stay valid; it is not used, the forward takes a NULL
- * workspace for every shape and the backward's passes may be given the sizes without it. Backward keeps rowsum(dO * O) per row (and, for f16, the
- * row lse in log2 units), padded to whole tiles.  The reference allocates the equivalent temporaries
+ * workspace for every shape and the backward's passes may be given the sizes without it: those this function answers for
+ * D = Dp.  The backward goes by the size it is given, so at such head dims pass-1 bytes may be enough for the fast backward.
+ * The f16 backward keeps rowsum(dO * O) and the lse in log2 units per row, padded to whole tiles.  The f32 backward keeps
+ * nothing; it still asks for the 4 bytes per row it used to need.  The reference allocates the equivalent temporaries
  * inside each op (`src/storage/cuda.rs:637-644`; its backward also keeps the whole [B,H,T,T]
  * probability tensor alive from the forward, `src/ops.rs:1162-1175`).
  * Pass 2 (f16; for f32 it equals pass 1) adds room for the dS tiles the mask leaves, 32 KB per
  * (slice, 128-row query tile, 128-row key tile): B*H*nq*(nq+1)/2 tiles causal, nq = ceil(T/128).
  * deers_b200_attn_bwd given at least that much keeps dS between its two main kernels, so dQ is one
  * streaming product instead of a second recomputation of S and dP (7 tile products become 5);
- * given less (but at least the pass-1 size) it recomputes.  Both give the same results up to
+ * given less (but at least the two arrays of the pass-1 size) it recomputes.  Both give the same results up to
  * f16 rounding of the same dS values and both are bitwise reproducible.
  */
 size_t deers_b200_attn_workspace_bytes(const deers_attn_desc* desc, int pass);

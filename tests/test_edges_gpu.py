@@ -484,3 +484,37 @@ def test_backward_weighs_its_workspace_against_the_memory_of_the_moment():
     assert all(torch.equal(a, b) for a, b in zip(got, want))
     del got, want
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("D,T", [(8, 129), (56, 300), (72, 127), (80, 385), (120, 257)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_f16_recomputing_backward_at_other_head_dims(D, T, causal):
+    """A workspace of the two statistics arrays and nothing else, which head dims between the tile widths may be given too:
+    the kernel that recomputes S and dP must run, in that workspace, on several and on ragged tiles."""
+    from deers_b200 import ops
+    from oracle import ref
+    B, H = 2, 3
+    rng = np.random.default_rng(D * T)
+    host = [rng.standard_normal((B, H, T, D)).astype(np.float16).astype(np.float32) for _ in range(4)]
+    q, k, v, do = (torch.from_numpy(a).to("cuda", torch.float16) for a in host)
+    scale = ops.default_scale(D)
+    o, lse = ops.attention_fwd(q, k, v, scale, causal)
+    bytes_used = ops.workspace_bytes(q.new_empty((B, H, T, 64 if D < 64 else 128)), scale, causal, 1)
+    assert bytes_used == 2 * B * H * -(-T // 128) * 128 * 4 < ops.workspace_bytes(q, scale, causal, 1)
+    ws = torch.full((bytes_used + 256,), 0xFF, dtype=torch.uint8, device="cuda")
+    taken, got = backward_peak(lambda: ops.attention_bwd(q, k, v, o, lse, do, scale, causal, workspace=ws[:bytes_used]))
+    assert taken <= 3 * (q.numel() * 2 + 512), "a workspace of its own beside the caller's"
+    assert torch.all(ws[bytes_used:] == 0xFF)
+    want = ref.attn_fwd_bwd(*host, causal=causal)
+    for name, g, w in zip(("dq", "dk", "dv"), got, want[2:]):
+        assert_close(g.float().cpu().numpy(), w, TOL_F16, f"D {D} T {T} {name}")
+
+
+def test_backward_allocates_what_its_kernels_use():
+    from deers_b200 import ops
+    q, k, v, do = (torch.randn((4, 8, 1000, 80), device="cuda").half() for _ in range(4))
+    o, lse = ops.attention_fwd(q, k, v, ops.default_scale(80))
+    fast = ops.workspace_bytes(q.new_empty((4, 8, 1000, 128)), pass_=2)
+    taken, _ = backward_peak(lambda: ops.attention_bwd(q, k, v, o, lse, do, ops.default_scale(80)))
+    # three gradients and 36 dS tiles of 32 KB for each of 32 slices; the allocator rounds each up to 2 MB at most
+    assert taken <= 3 * q.numel() * 2 + fast + 4 * (2 << 20), (taken, fast)
