@@ -39,7 +39,6 @@ struct GemmArgs {
     int a_vec, b_vec, c_vec; // 16-byte accesses allowed
     int epi;
     int k_chunk;             // K elements per part (multiple of BK)
-    int tall;                // blockIdx.x counts tile rows, blockIdx.y tile columns (more than 65535 tile rows)
 };
 
 __device__ __forceinline__ float4 ld4(const float* p, int valid, bool vec) {
@@ -163,7 +162,7 @@ __global__ void __launch_bounds__(128 * KS) gemm_f32_kernel(const GemmArgs g) {
     const int tid = threadIdx.x % 128, kg = threadIdx.x / 128;      // position in the tile, k group
     const int w = tid / 32, lane = tid % 32;
     const int ty = (w & 1) * 4 + lane / 8, tx = (w >> 1) * 8 + lane % 8;
-    const int m0 = (g.tall ? blockIdx.x : blockIdx.y) * BM, n0 = (g.tall ? blockIdx.y : blockIdx.x) * BN;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int kbeg = blockIdx.z * g.k_chunk;
     const int kend = min(g.K, kbeg + g.k_chunk);
     const int nk = kend > kbeg ? (kend - kbeg + BK - 1) / BK : 0;
@@ -379,9 +378,7 @@ int launch_variant(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g) {
     using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
     const auto kernel = gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>;
     DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>), S::SMEM);
-    // gridDim.y ends at 65535.  Products with more tile rows than that have few tile columns (or C would not fit any device).
-    const dim3 grid = g.tall ? dim3(p.tiles_m, p.tiles_n, p.parts) : dim3(p.tiles_n, p.tiles_m, p.parts);
-    DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, grid, S::GT, S::SMEM, dim3(1, 1, p.parts), g));
+    DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, dim3(p.tiles_n, p.tiles_m, p.parts), S::GT, S::SMEM, dim3(1, 1, p.parts), g));
     return DEERS_OK;
 }
 
@@ -396,6 +393,16 @@ int launch_orders(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g, int a_mn
 int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long long lda, int a_mn, const float* b,
                     long long ldb, int b_mn, float* c, long long ldc, int epi, const float* r, long long ldr, float* aux) {
     if (M == 0 || N == 0) return DEERS_OK;
+    // Row tiles lie along gridDim.y, which ends at 65535: taller products (tiles are 32 rows or more) go in several launches.
+    constexpr int MOST = 65535 * 32;
+    for (; M > MOST; M -= MOST) {
+        const int rc = launch_gemm_f32(ctx, MOST, N, K, a, lda, a_mn, b, ldb, b_mn, c, ldc, epi, r, ldr, aux);
+        if (rc) return rc;
+        a += a_mn ? MOST : MOST * lda;
+        c += MOST * ldc;
+        if (r) r += MOST * ldr;
+        if (aux) aux += MOST * ldc;
+    }
     int rc = cluster_capacity(ctx);
     if (rc) return rc;
     GemmPlan p = plan_gemm(M, N, K, ctx->cluster_capacity);
@@ -408,7 +415,6 @@ int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long lo
     g.c_vec = ((uintptr_t)c & 15u) == 0 && ldc % 4 == 0 && (!r || (((uintptr_t)r & 15u) == 0 && ldr % 4 == 0)) &&
               (!aux || ((uintptr_t)aux & 15u) == 0);
     g.k_chunk = p.k_chunk;
-    g.tall = p.tiles_m > 65535;
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM);
         if (p.cfg == 0) rc = launch_orders<8, 8, 2>(ctx, p, g, a_mn, b_mn);
