@@ -396,7 +396,7 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         // warp seeing a stale 32-byte piece of the delta row in the first iteration of an item.)
         const int ct = (warp - 2) * 32 + lane;
         const bool stager = ct < 2 * BT;
-        const float* stat_src = chained((ct < BT) ? p.lse2 + ct : p.delta + (ct - BT));
+        const float* stat_src = (ct < BT) ? p.lse2 + ct : p.delta + (ct - BT);
         float* stat_dst = (ct < BT) ? lse2_s + ct : delta_s + (ct - BT);
         float stat_next = 0.f;
         {
@@ -1050,7 +1050,6 @@ attn_bwd_prep_f16_kernel(const __half* o, const __half* d_o, const float* lse,
                          long long so_b, long long so_h, long long so_t, long long sdo_b, long long sdo_h,
                          long long sdo_t) {
     chain_begin();
-    o = chained(o); d_o = chained(d_o); lse = chained(lse);
     constexpr int LPR = D / 8;                               // lanes per row
     constexpr int RPW = 32 / LPR;                            // rows per warp load
     constexpr int U = 4;                                     // loads in flight per lane and tensor

@@ -8,7 +8,6 @@
 #include <string.h>
 
 #include <atomic>
-#include <type_traits>
 #include <utility>
 
 #include "../../include/deers_b200.h"
@@ -117,14 +116,8 @@ __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.laun
 __device__ __forceinline__ void chain_begin() { chain_next(); chain_wait(); }
 // What a predecessor writes may change while a chained kernel is already resident, so its reads must be ordinary (coherent)
 // loads behind the wait.  Pointers to such data are neither `const __restrict__` nor read by __ldg: both allow the read-only
-// path, which promises the values of the kernel's start, and let the compiler move the load in front of the wait.
-// chained(p), taken after the wait, hands out the pointer as a value the compiler knows nothing about but that it is global.
-template <typename T>
-__device__ __forceinline__ T* chained(T* p) {
-    size_t g = __cvta_generic_to_global(p);
-    asm volatile("" : "+l"(g) : : "memory");
-    return static_cast<T*>(const_cast<typename std::remove_const<T>::type*>(static_cast<const typename std::remove_const<T>::type*>(__cvta_global_to_generic(g))));
-}
+// path, which promises the values of the kernel's start, and let the compiler move the load in front of the wait.  (Pointers
+// that are only written may be __restrict__: it lets the loads of a loop run ahead of its stores.)
 // One streaming (read once) float behind the wait.
 __device__ __forceinline__ float ld_stream(const float* p) {
     float v;

@@ -241,7 +241,6 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_consta
 __global__ void __launch_bounds__(256) x3_reduce_kernel(const float* partial, int parts, long long MN,
                                                         int N, float* __restrict__ c, long long ldc) {
     chain_begin();
-    partial = chained(partial);
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < MN; i += (long long)gridDim.x * 256) {
         float acc = partial[i];
         for (int pz = 1; pz < parts; ++pz) acc += partial[(long long)pz * MN + i];
@@ -254,7 +253,6 @@ __global__ void __launch_bounds__(256) x3_split_kernel(const float* src, long lo
                                                        float scale, __half* __restrict__ hi, __half* __restrict__ lo,
                                                        long long ld_dst, int vec) {
     chain_begin();
-    src = chained(src);
     const int per_row = (cols + 7) / 8;
     const long long total = rows * per_row;
     for (long long t = (long long)blockIdx.x * 256 + threadIdx.x; t < total; t += (long long)gridDim.x * 256) {

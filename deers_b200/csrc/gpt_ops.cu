@@ -25,7 +25,6 @@ __global__ void __launch_bounds__(256) embedding_fwd_kernel(const float* w, cons
                                                             long long n_ids, int C, long long V, float* __restrict__ out,
                                                             int vec, unsigned int* err) {
     chain_begin();
-    w = chained(w); ids = chained(ids);
     const int lane = threadIdx.x & 31;
     const long long n = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (n >= n_ids) return;
@@ -48,7 +47,6 @@ __global__ void __launch_bounds__(256) embedding_fwd_kernel(const float* w, cons
 __global__ void __launch_bounds__(256) embedding_bwd_kernel(const float* dout, const long long* ids, long long n_ids, int C,
                                                             long long V, float* __restrict__ dw) {
     chain_wait();
-    dout = chained(dout); ids = chained(ids);
     __shared__ unsigned char s_flag[256];
     const long long n = blockIdx.x;
     const long long id = ids[n];
@@ -104,7 +102,6 @@ __global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const float* log
                                                                 float* __restrict__ lse, float* __restrict__ picked,
                                                                 unsigned int* err) {
     chain_wait();
-    logits = chained(logits); targets = chained(targets);
     __shared__ float red_m[8], red_s[8];
     const long long row = blockIdx.x;
     const float* x = logits + row * ld;
@@ -145,7 +142,6 @@ __global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const float* log
 __global__ void __launch_bounds__(1024) cross_entropy_loss_kernel(const float* picked, long long rows,
                                                                   float neg_inv_rows, float* __restrict__ loss) {
     chain_wait();
-    picked = chained(picked);
     __shared__ float red[32];
     float s = 0.f;
     for (long long j = threadIdx.x; j < rows; j += 1024) s += picked[j];
@@ -162,10 +158,9 @@ __global__ void __launch_bounds__(1024) cross_entropy_loss_kernel(const float* p
 }
 
 __global__ void __launch_bounds__(256) cross_entropy_bwd_kernel(const float* logits, long long ld, const long long* targets, const float* lse,
-                                                                long long V, float g, float upstream, float* dlogits,
+                                                                long long V, float g, float upstream, float* __restrict__ dlogits,
                                                                 long long ldd, int vec) {
     chain_wait();
-    logits = chained(logits); targets = chained(targets); lse = chained(lse);
     const long long row = blockIdx.y;
     const float* x = logits + row * ld;
     float* d = dlogits + row * ldd;
@@ -194,10 +189,17 @@ __global__ void __launch_bounds__(256) cross_entropy_bwd_kernel(const float* log
             }
         }
     } else {
-        for (long long j = (long long)blockIdx.x * 256 + threadIdx.x; j < V; j += stride) {
-            const float p = expf(x[j] - l);
-            const float gj = (j == t) ? g : 0.f;
-            d[j] = __fmul_rn(__fsub_rn(gj, __fmul_rn(p, g)), upstream);
+        for (long long j0 = (long long)blockIdx.x * 256 + threadIdx.x; j0 < V; j0 += 4 * stride) {
+            float v[4];                                               // four loads in flight
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = j0 + e * stride < V ? x[j0 + e * stride] : 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const long long j = j0 + e * stride;
+                const float p = expf(v[e] - l);
+                const float gj = (j == t) ? g : 0.f;
+                if (j < V) d[j] = __fmul_rn(__fsub_rn(gj, __fmul_rn(p, g)), upstream);
+            }
         }
     }
 }
@@ -210,7 +212,6 @@ __global__ void __launch_bounds__(256) cross_entropy_bwd_split_kernel(const floa
                                                                       float upstream, float scale, __half* __restrict__ hi,
                                                                       __half* __restrict__ lo, long long ldd) {
     chain_wait();
-    logits = chained(logits); targets = chained(targets); lse = chained(lse);
     const long long row = blockIdx.y;
     const float* x = logits + row * ld;
     __half* dh = hi + row * ldd;

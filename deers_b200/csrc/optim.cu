@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256) grad_sq_sum_kernel(const __grid_constant_
         const int ti = find_tensor(t, chunk);
         const long long base = (long long)(chunk - t.chunk_start[ti]) * OPT_CHUNK;
         const long long n = t.n[ti];
-        const float* g = chained(t.g[ti]);
+        const float* g = t.g[ti];
         if (t.vec_ok && base + OPT_CHUNK <= n) {
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
@@ -95,7 +95,6 @@ __global__ void __launch_bounds__(256) grad_sq_sum_kernel(const __grid_constant_
 // norm = sqrt(sum of the partials), summed by one block in a fixed order.
 __global__ void __launch_bounds__(1024) grad_norm_kernel(const float* partial, int n, float* __restrict__ norm) {
     chain_wait();
-    partial = chained(partial);
     __shared__ float sh[1024];
     float acc = 0.f;
     for (int i = threadIdx.x; i < n; i += 1024) acc += partial[i];
@@ -141,7 +140,6 @@ template <int MODE>
 __global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ OptTensors t, const __grid_constant__ OptScalars s,
                                                     const float* norm) {
     chain_wait();
-    norm = chained(norm);
     float scale;
     const bool clip = clip_scale(s, norm, scale);
     if (MODE == MODE_CLIP && !clip) return;
@@ -151,10 +149,10 @@ __global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ OptT
         const int ti = find_tensor(t, chunk);
         const long long base = (long long)(chunk - t.chunk_start[ti]) * OPT_CHUNK;
         const long long n = t.n[ti];
-        float* __restrict__ w = chained(t.w[ti]);
-        float* __restrict__ g = chained(t.g[ti]);
-        float* __restrict__ m = chained(t.m[ti]);
-        float* __restrict__ v = chained(t.v[ti]);
+        float* __restrict__ w = t.w[ti];
+        float* __restrict__ g = t.g[ti];
+        float* __restrict__ m = t.m[ti];
+        float* __restrict__ v = t.v[ti];
         if (t.vec_ok && base + OPT_CHUNK <= n) {
 #pragma unroll
             for (int r = 0; r < 4; ++r) {

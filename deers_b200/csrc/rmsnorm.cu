@@ -28,13 +28,10 @@ __device__ __forceinline__ float warp_sum(float v) {
 // BWD = false: y = x * inv, inv_out[row] = inv.   BWD = true: dx from x, dy and the saved inv.
 template <bool BWD, bool VEC, bool VEC2 = false>
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const float* dy, const float* add, float* __restrict__ out,
-                                                      float* inv_io, long long rows, int C, float eps,
+                                                      float* __restrict__ inv_io, long long rows, int C, float eps,
                                                       float inv_n) {
     if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room)
     chain_wait();
-    x = chained(x); inv_io = chained(inv_io);
-    if (BWD) dy = chained(dy);
-    if (BWD && add) add = chained(add);
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * 8;
@@ -90,13 +87,20 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
             const float4* x4 = reinterpret_cast<const float4*>(xr);
             const float4* g4 = BWD ? reinterpret_cast<const float4*>(dy + row * C) : nullptr;
             float acc = 0.f;
-            for (int p = lane; p < nv; p += 32) {
-                const float4 a = x4[p];
-                if (BWD) {
-                    const float4 b = g4[p];
-                    acc += a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
-                } else {
-                    acc += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+            constexpr int U = BWD ? 8 : 16;                     // pieces of a lane in flight
+            for (int p0 = lane; p0 < nv; p0 += 32 * U) {
+                float4 a[U], b[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int p = p0 + 32 * u;
+                    a[u] = b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (p < nv) a[u] = x4[p];
+                    if (BWD && p < nv) b[u] = g4[p];
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const float4 c = BWD ? b[u] : a[u];
+                    acc += a[u].x * c.x + a[u].y * c.y + a[u].z * c.z + a[u].w * c.w;
                 }
             }
             acc = warp_sum(acc);
@@ -108,20 +112,31 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
                 inv = 1.0f / sqrtf(acc * inv_n + eps);
                 if (lane == 0) inv_io[row] = inv;
             }
-            for (int p = lane; p < nv; p += 32) {               // the row (<= a few KB per lane group) is still in L1 / L2
-                const float4 a = x4[p];
-                float4 o;
-                if (BWD) {
-                    const float4 b = g4[p];
-                    o.x = b.x * inv - a.x * k; o.y = b.y * inv - a.y * k; o.z = b.z * inv - a.z * k; o.w = b.w * inv - a.w * k;
-                    if (add) {
-                        const float4 r = reinterpret_cast<const float4*>(add + row * C)[p];
-                        o.x = r.x + o.x; o.y = r.y + o.y; o.z = r.z + o.z; o.w = r.w + o.w;
-                    }
-                } else {
-                    o.x = a.x * inv; o.y = a.y * inv; o.z = a.z * inv; o.w = a.w * inv;
+            for (int p0 = lane; p0 < nv; p0 += 32 * U) {        // the row (<= a few KB per lane group) is still in L1 / L2
+                float4 a[U], b[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int p = p0 + 32 * u;
+                    if (p < nv) a[u] = x4[p];
+                    if (BWD && p < nv) b[u] = g4[p];
                 }
-                reinterpret_cast<float4*>(orow)[p] = o;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int p = p0 + 32 * u;
+                    if (p >= nv) break;
+                    float4 o;
+                    if (BWD) {
+                        o.x = b[u].x * inv - a[u].x * k; o.y = b[u].y * inv - a[u].y * k;
+                        o.z = b[u].z * inv - a[u].z * k; o.w = b[u].w * inv - a[u].w * k;
+                        if (add) {
+                            const float4 r = reinterpret_cast<const float4*>(add + row * C)[p];
+                            o.x = r.x + o.x; o.y = r.y + o.y; o.z = r.z + o.z; o.w = r.w + o.w;
+                        }
+                    } else {
+                        o.x = a[u].x * inv; o.y = a[u].y * inv; o.z = a[u].z * inv; o.w = a[u].w * inv;
+                    }
+                    reinterpret_cast<float4*>(orow)[p] = o;
+                }
             }
         } else {                                                // any C, any alignment: two passes over the row
             const float* gr = BWD ? dy + row * C : nullptr;
@@ -148,13 +163,10 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
 // Rows of 1025 .. 8192 elements: a whole block owns a row, which still stays in registers (one pass over HBM).
 template <bool BWD>
 __global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* x, const float* dy, const float* add, float* __restrict__ out,
-                                                            float* inv_io, long long rows, int C, float eps,
+                                                            float* __restrict__ inv_io, long long rows, int C, float eps,
                                                             float inv_n) {
     if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room)
     chain_wait();
-    x = chained(x); inv_io = chained(inv_io);
-    if (BWD) dy = chained(dy);
-    if (BWD && add) add = chained(add);
     __shared__ float part[8];
     const int nv = C / 4;                                       // <= 256 * RN_MAXV
     for (long long row = blockIdx.x; row < rows; row += gridDim.x) {

@@ -63,10 +63,10 @@ __global__ void __launch_bounds__(256) rope_pack_kernel(const RopeParams p) {
     const int cpr = half / V;                                   // chunks (threads) per row
     const long long rows = (long long)p.B * p.T * p.H;
     const long long total = rows * cpr;
-    const T* src = chained(static_cast<const T*>(p.src));
+    const T* src = static_cast<const T*>(p.src);
     T* __restrict__ dst = static_cast<T*>(p.dst);
-    const T* cosp = chained(static_cast<const T*>(p.cosp));
-    const T* sinp = chained(static_cast<const T*>(p.sinp));
+    const T* cosp = static_cast<const T*>(p.cosp);
+    const T* sinp = static_cast<const T*>(p.sinp);
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
         const long long row = idx / cpr;                        // (b, t, h) in source order
