@@ -1129,9 +1129,9 @@ int bwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
         const long long per_block = 8LL * 4 * (256 / D);           // 8 warps x 4 loads x rows per load
         const long long want = (prep_rows + per_block - 1) / per_block;
         const unsigned prep_grid = (unsigned)(want < (long long)PREP_BLOCKS * ctx->sm_count ? want : (long long)PREP_BLOCKS * ctx->sm_count);
-        launch_chained(ctx, attn_bwd_prep_f16_kernel<D>, prep_grid, 256, 0, 1,
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, attn_bwd_prep_f16_kernel<D>, prep_grid, 256, 0, 1,
             (const __half*)o, (const __half*)d_o, lse, delta, lse2, d->B, d->H, d->T, d->D, Tpad, d->o_strides[0],
-            d->o_strides[1], d->o_strides[2], d->do_strides[0], d->do_strides[1], d->do_strides[2]);
+            d->o_strides[1], d->o_strides[2], d->do_strides[0], d->do_strides[1], d->do_strides[2]));
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
 
@@ -1156,17 +1156,17 @@ int bwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
     const ChainScope chain(ctx, BH * p.ds_pairs / persistent);
     {
         KernelTimerScope ts(ctx, DEERS_K_BWD_MAIN);
-        launch_chained(ctx, attn_bwd_dkdv_f16_kernel<D>, persistent, DKV_THREADS, smem_a, 1, tq, tk, tv, tdo, p);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, attn_bwd_dkdv_f16_kernel<D>, persistent, DKV_THREADS, smem_a, 1, tq, tk, tv, tdo, p));
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     if (keep_ds) {
         const size_t smem_c = DqsSmem<D>::TOTAL;
         DEERS_SMEM_ONCE(ctx, (attn_bwd_dq_from_ds_f16_kernel<D>), smem_c);
         KernelTimerScope ts(ctx, DEERS_K_BWD_DQ);
-        launch_chained(ctx, attn_bwd_dq_from_ds_f16_kernel<D>, persistent, 192, smem_c, 1, tk, p);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, attn_bwd_dq_from_ds_f16_kernel<D>, persistent, 192, smem_c, 1, tk, p));
     } else {
         KernelTimerScope ts(ctx, DEERS_K_BWD_DQ);
-        launch_chained(ctx, attn_bwd_dq_f16_kernel<D>, persistent, 320, smem_b, 1, tq, tk, tv, tdo, p);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, attn_bwd_dq_f16_kernel<D>, persistent, 320, smem_b, 1, tq, tk, tv, tdo, p));
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     ctx->launches += 3;

@@ -437,8 +437,8 @@ extern "C" size_t deers_b200_attn_decode_workspace_bytes(const deers_decode_desc
 template <typename T, int LPK>
 static int decode_launch_vec(deers_ctx* ctx, const DecodeParams& p, const dim3& grid, bool cluster) {
     if (!cluster || p.splits == 1) {
-        if (cluster) launch_chained(ctx, decode_vec_kernel<T, LPK, DEC_ONE_CHUNK>, grid, 128, 0, 1, p);
-        else launch_chained(ctx, decode_vec_kernel<T, LPK, DEC_TO_WORKSPACE>, grid, 128, 0, 1, p);
+        if (cluster) DEERS_CUDA_TRY(ctx, launch_chained(ctx, decode_vec_kernel<T, LPK, DEC_ONE_CHUNK>, grid, 128, 0, 1, p));
+        else DEERS_CUDA_TRY(ctx, launch_chained(ctx, decode_vec_kernel<T, LPK, DEC_TO_WORKSPACE>, grid, 128, 0, 1, p));
         return DEERS_OK;
     }
     DEERS_CUDA_TRY(ctx, launch_chained(ctx, decode_vec_kernel<T, LPK, DEC_CLUSTER>, grid, 128, 0, p.splits, p));
@@ -449,13 +449,13 @@ template <typename T>
 static int decode_launch(deers_ctx* ctx, const DecodeParams& p, const dim3& grid, bool vec, bool cluster) {
     const int pieces = p.D * (int)sizeof(T) / 16;
     int rc = DEERS_OK;
-    if (!vec) launch_chained(ctx, decode_partial_kernel<T>, grid, 128, 0, 1, p);
+    if (!vec) DEERS_CUDA_TRY(ctx, launch_chained(ctx, decode_partial_kernel<T>, grid, 128, 0, 1, p));
     else if (pieces > 16) rc = decode_launch_vec<T, 32>(ctx, p, grid, cluster);
     else if (pieces > 8) rc = decode_launch_vec<T, 16>(ctx, p, grid, cluster);
     else if (pieces > 4) rc = decode_launch_vec<T, 8>(ctx, p, grid, cluster);
     else rc = decode_launch_vec<T, 4>(ctx, p, grid, cluster);
     if (rc || (vec && cluster)) return rc;
-    launch_chained(ctx, decode_combine_kernel<T>, (unsigned)((long long)p.B * p.H * p.Tq), 128, 0, 1, p);
+    DEERS_CUDA_TRY(ctx, launch_chained(ctx, decode_combine_kernel<T>, (unsigned)((long long)p.B * p.H * p.Tq), 128, 0, 1, p));
     ctx->launches += 1;
     return DEERS_OK;
 }

@@ -584,7 +584,7 @@ int fwd_impl(deers_ctx* ctx, const F32Params& p) {
     const dim3 grid(p.B * p.H, (p.T + BM - 1) / BM);
     {
         KernelTimerScope ts(ctx, DEERS_K_FWD);
-        launch_chained(ctx, attn_fwd_f32_kernel<DP>, grid, NT, Tile<DP>::FWD_SMEM, 1, p);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, attn_fwd_f32_kernel<DP>, grid, NT, Tile<DP>::FWD_SMEM, 1, p));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -597,7 +597,7 @@ int bwd_impl(deers_ctx* ctx, const F32Params& p) {
     const dim3 grid(2 * p.B * p.H, (p.T + BM - 1) / BM);
     {
         KernelTimerScope ts(ctx, DEERS_K_BWD_MAIN);
-        launch_chained(ctx, attn_bwd_f32_kernel<DP>, grid, NT, Tile<DP>::BWD_SMEM, 1, p);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, attn_bwd_f32_kernel<DP>, grid, NT, Tile<DP>::BWD_SMEM, 1, p));
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     ctx->launches += 1;

@@ -554,7 +554,7 @@ int fwd_launch(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const vo
     {
         const ChainScope chain(ctx, items * (d->causal ? (nq + 1) / 2 : nq) / grid);
         KernelTimerScope ts(ctx, DEERS_K_FWD);
-        launch_chained(ctx, attn_fwd_f16_kernel<D>, grid, FWD_THREADS, smem, 1, tq, tk, tv, p);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, attn_fwd_f16_kernel<D>, grid, FWD_THREADS, smem, 1, tq, tk, tv, p));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());

@@ -83,12 +83,15 @@ struct KernelTimerScope {
     }
 };
 
+// Returns DEERS_ERR_CUDA from the caller when `expr` fails.  The runtime keeps a failed call's error for the next
+// cudaGetLastError(): it is taken here, or the next operator, which asks after its launches, would report it as its own.
 #define DEERS_CUDA_TRY(ctx, expr)                                                            \
     do {                                                                                      \
         cudaError_t _e = (expr);                                                              \
         if (_e != cudaSuccess) {                                                              \
             snprintf((ctx)->last_error, sizeof((ctx)->last_error), "%s: %s", #expr,           \
                      cudaGetErrorString(_e));                                                 \
+            cudaGetLastError();                                                               \
             return DEERS_ERR_CUDA;                                                            \
         }                                                                                     \
     } while (0)
@@ -128,8 +131,9 @@ __device__ __forceinline__ float ld_stream(const float* p) {
 // False while capturing, unless a kernel of this stream is the one predecessor (ctx.cu).
 bool deers_can_chain(const deers_ctx* ctx);
 
+// Every call looks at the result: the next kernel would work on what a refused one has not written.
 template <typename... P, typename... A>
-cudaError_t launch_chained(deers_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, dim3 cluster, A&&... args) {
+[[nodiscard]] cudaError_t launch_chained(deers_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, dim3 cluster, A&&... args) {
     cudaLaunchConfig_t lc{};
     lc.gridDim = grid;
     lc.blockDim = block;

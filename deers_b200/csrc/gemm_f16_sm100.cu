@@ -351,7 +351,7 @@ int gemm_launch(deers_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, co
             DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<A_MN, B_MN, GN, false>), g_smem(GN));
             const unsigned grid = (unsigned)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
             const ChainScope chain(ctx, tiles * p.kb_chunk / grid);
-            launch_chained(ctx, gemm_f16_kernel<A_MN, B_MN, GN, false>, grid, G_THREADS, g_smem(GN), 1, ta, tb, p);
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, gemm_f16_kernel<A_MN, B_MN, GN, false>, grid, G_THREADS, g_smem(GN), 1, ta, tb, p));
         } else {
             const auto kernel = gemm_f16_kernel<A_MN, B_MN, GN, true>;
             DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<A_MN, B_MN, GN, true>), g_smem(GN));

@@ -331,7 +331,7 @@ int x3_launch(deers_ctx* ctx, const CUtensorMap* t, const X3Params& p, unsigned 
     DEERS_SMEM_ONCE(ctx, (gemm_f16x3_kernel<A_MN, B_MN>), X_SMEM);
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM_X3);
-        launch_chained(ctx, gemm_f16x3_kernel<A_MN, B_MN>, grid, X_THREADS, X_SMEM, 1, t[0], t[1], t[2], t[3], p);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, gemm_f16x3_kernel<A_MN, B_MN>, grid, X_THREADS, X_SMEM, 1, t[0], t[1], t[2], t[3], p));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -354,8 +354,8 @@ int launch_split_f16x3(deers_ctx* ctx, long long rows, int cols, const float* sr
     const long long cap = 16LL * ctx->sm_count;
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM_X3);
-        launch_chained(ctx, x3_split_kernel, (unsigned)(want < cap ? want : cap), 256, 0, 1, src, ld_src, rows, cols, scale, (__half*)hi,
-                                                                                      (__half*)lo, ld_dst, vec);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, x3_split_kernel, (unsigned)(want < cap ? want : cap), 256, 0, 1, src, ld_src, rows, cols, scale, (__half*)hi,
+                                                                                      (__half*)lo, ld_dst, vec));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -396,7 +396,7 @@ int launch_gemm_f16x3(deers_ctx* ctx, int M, int N, int K, const void* a_hi, con
         const long long cap = 8LL * ctx->sm_count;
         {
             KernelTimerScope ts(ctx, DEERS_K_GEMM_X3);
-            launch_chained(ctx, x3_reduce_kernel, (unsigned)(want < cap ? want : cap), 256, 0, 1, (const float*)workspace, pl.parts, MN, N, c, ldc);
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, x3_reduce_kernel, (unsigned)(want < cap ? want : cap), 256, 0, 1, (const float*)workspace, pl.parts, MN, N, c, ldc));
         }
         ctx->launches += 1;
         DEERS_CUDA_TRY(ctx, cudaGetLastError());

@@ -641,7 +641,7 @@ extern "C" int deers_b200_gpt_forward(deers_gpt* m, const int64_t* ids, int32_t 
     if (logits) {
         const int V = m->cfg.vocab_size;
         const dim3 grid((unsigned)((V + 4095) / 4096), (unsigned)(B * T));
-        launch_chained(ctx, copy_logits_kernel, grid, 256, 0, 1, m->logits, m->Vld, logits, V);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, copy_logits_kernel, grid, 256, 0, 1, m->logits, m->Vld, logits, V));
         ctx->launches += 1;
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());

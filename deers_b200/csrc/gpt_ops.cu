@@ -260,8 +260,8 @@ int launch_cross_entropy_bwd_split(deers_ctx* ctx, const float* logits, long lon
     const dim3 grid((unsigned)per_row, (unsigned)rows);
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        launch_chained(ctx, cross_entropy_bwd_split_kernel, grid, 256, 0, 1, logits, ld, targets, lse, V, (float)(-1.0 / (double)rows),
-                                                                      upstream, scale, (__half*)hi, (__half*)lo, ldd);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_bwd_split_kernel, grid, 256, 0, 1, logits, ld, targets, lse, V, (float)(-1.0 / (double)rows),
+                                                                      upstream, scale, (__half*)hi, (__half*)lo, ldd));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -274,8 +274,8 @@ int launch_embedding_fwd(deers_ctx* ctx, const float* weight, const long long* i
     const int vec = C % 4 == 0 && (((uintptr_t)weight | (uintptr_t)out) & 15u) == 0;
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        launch_chained(ctx, embedding_fwd_kernel, (unsigned)((n_ids + 7) / 8), 256, 0, 1, weight, ids, n_ids, C, V, out, vec,
-                                                                                  ctx->dev_err);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, embedding_fwd_kernel, (unsigned)((n_ids + 7) / 8), 256, 0, 1, weight, ids, n_ids, C, V, out, vec,
+                                                                                  ctx->dev_err));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -288,7 +288,7 @@ int launch_embedding_bwd(deers_ctx* ctx, const float* dout, const long long* ids
     if (n_ids == 0) return DEERS_OK;
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        launch_chained(ctx, embedding_bwd_kernel, (unsigned)n_ids, 256, 0, 1, dout, ids, n_ids, C, V, dweight);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, embedding_bwd_kernel, (unsigned)n_ids, 256, 0, 1, dout, ids, n_ids, C, V, dweight));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -299,8 +299,8 @@ int launch_cross_entropy_fwd(deers_ctx* ctx, const float* logits, long long ld, 
                              long long V, float* lse, float* picked, float* loss) {
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        launch_chained(ctx, cross_entropy_fwd_kernel, (unsigned)rows, 256, 0, 1, logits, ld, targets, V, lse, picked, ctx->dev_err);
-        launch_chained(ctx, cross_entropy_loss_kernel, 1, 1024, 0, 1, picked, rows, (float)(-1.0 / (double)rows), loss);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_fwd_kernel, (unsigned)rows, 256, 0, 1, logits, ld, targets, V, lse, picked, ctx->dev_err));
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_loss_kernel, 1, 1024, 0, 1, picked, rows, (float)(-1.0 / (double)rows), loss));
     }
     ctx->launches += 2;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -310,7 +310,7 @@ int launch_cross_entropy_fwd(deers_ctx* ctx, const float* logits, long long ld, 
 int launch_cross_entropy_loss(deers_ctx* ctx, const float* picked, long long rows, float* loss) {
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        launch_chained(ctx, cross_entropy_loss_kernel, 1, 1024, 0, 1, picked, rows, (float)(-1.0 / (double)rows), loss);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_loss_kernel, 1, 1024, 0, 1, picked, rows, (float)(-1.0 / (double)rows), loss));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -326,8 +326,8 @@ int launch_cross_entropy_bwd(deers_ctx* ctx, const float* logits, long long ld, 
     const dim3 grid((unsigned)per_row, (unsigned)rows);
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        launch_chained(ctx, cross_entropy_bwd_kernel, grid, 256, 0, 1, logits, ld, targets, lse, V, (float)(-1.0 / (double)rows),
-                                                                upstream, dlogits, ldd, vec);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_bwd_kernel, grid, 256, 0, 1, logits, ld, targets, lse, V, (float)(-1.0 / (double)rows),
+                                                                upstream, dlogits, ldd, vec));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());

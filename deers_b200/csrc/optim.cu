@@ -269,14 +269,14 @@ extern "C" int deers_b200_grad_norm(deers_ctx* ctx, int n_tensors, const deers_o
         if ((size_t)(n_partial + grid) * sizeof(float) > scratch_bytes) return DEERS_ERR_WORKSPACE;
         {
             KernelTimerScope ts(ctx, DEERS_K_OPTIM);
-            launch_chained(ctx, grad_sq_sum_kernel, grid, 256, 0, 1, t, partial + n_partial);
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, grad_sq_sum_kernel, grid, 256, 0, 1, t, partial + n_partial));
         }
         ctx->launches += 1;
         n_partial += (int)grid;
     }
     {
         KernelTimerScope ts(ctx, DEERS_K_OPTIM);
-        launch_chained(ctx, grad_norm_kernel, 1, 1024, 0, 1, partial, n_partial, norm_dev);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, grad_norm_kernel, 1, 1024, 0, 1, partial, n_partial, norm_dev));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -294,8 +294,8 @@ static int optim_apply(deers_ctx* ctx, int n_tensors, const deers_optim_tensor* 
         const unsigned grid = optim_grid(ctx, t.chunk_start[t.count]);
         {
             KernelTimerScope ts(ctx, DEERS_K_OPTIM);
-            if (mode == MODE_STEP) launch_chained(ctx, adamw_kernel<MODE_STEP>, grid, 256, 0, 1, t, s, norm_dev);
-            else launch_chained(ctx, adamw_kernel<MODE_CLIP>, grid, 256, 0, 1, t, s, norm_dev);
+            if (mode == MODE_STEP) DEERS_CUDA_TRY(ctx, launch_chained(ctx, adamw_kernel<MODE_STEP>, grid, 256, 0, 1, t, s, norm_dev));
+            else DEERS_CUDA_TRY(ctx, launch_chained(ctx, adamw_kernel<MODE_CLIP>, grid, 256, 0, 1, t, s, norm_dev));
         }
         ctx->launches += 1;
     }

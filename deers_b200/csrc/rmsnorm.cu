@@ -237,12 +237,12 @@ int rms_launch(deers_ctx* ctx, long long rows, int C, float eps, const float* x,
     const float inv_n = (float)(1.0 / (double)C);               // mean = sum * (1/n as f64 -> f32), src/tensor.rs:461-465
     {
         KernelTimerScope ts(ctx, DEERS_K_NORM);
-        if (vec) launch_chained(ctx, rmsnorm_kernel<BWD, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n);
+        if (vec) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n));
         else if (aligned && C <= 256 * RN_MAXV * 4) {
             const unsigned bgrid = (unsigned)(rows < cap ? rows : cap);
-            launch_chained(ctx, rmsnorm_block_kernel<BWD>, bgrid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n);
-        } else if (aligned) launch_chained(ctx, rmsnorm_kernel<BWD, false, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n);
-        else launch_chained(ctx, rmsnorm_kernel<BWD, false>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n);
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_block_kernel<BWD>, bgrid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n));
+        } else if (aligned) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n));
+        else DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());

@@ -142,8 +142,8 @@ int rope_launch(deers_ctx* ctx, const deers_rope_desc* d, const RopeParams& p) {
     const unsigned grid = (unsigned)(want < cap ? want : cap);
     {
         KernelTimerScope ts(ctx, DEERS_K_ROPE);
-        if (vec) launch_chained(ctx, rope_pack_kernel<T, VMAX>, grid, 256, 0, 1, p);
-        else launch_chained(ctx, rope_pack_kernel<T, 1>, grid, 256, 0, 1, p);
+        if (vec) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rope_pack_kernel<T, VMAX>, grid, 256, 0, 1, p));
+        else DEERS_CUDA_TRY(ctx, launch_chained(ctx, rope_pack_kernel<T, 1>, grid, 256, 0, 1, p));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());

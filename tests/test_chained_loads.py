@@ -58,3 +58,10 @@ def test_no_read_only_loads(file):
     assert not re.search(r"__ldg\(|__ldcs\(|__ldca\(|ld\.global(\.\w+)*\.nc", FILES[file]), file
     # locals of kernels: a restrict pointer to const data taken from a parameter structure
     assert not re.search(r"const\s+\w+\s*\*\s*__restrict__\s+\w+\s*=", FILES[file]), file
+
+
+@pytest.mark.parametrize("file", sorted(f for f in FILES if f.endswith(".cu")))
+def test_refused_launches_end_the_call(file):
+    """Behind a launch that was refused, the next kernel would work on what has not been written."""
+    for m in re.finditer(r"launch_chained\(", FILES[file]):
+        assert FILES[file][:m.start()].rstrip().endswith("DEERS_CUDA_TRY(ctx,"), FILES[file][m.start():m.start() + 80]

@@ -518,3 +518,34 @@ def test_backward_allocates_what_its_kernels_use():
     taken, _ = backward_peak(lambda: ops.attention_bwd(q, k, v, o, lse, do, ops.default_scale(80)))
     # three gradients and 36 dS tiles of 32 KB for each of 32 slices; the allocator rounds each up to 2 MB at most
     assert taken <= 3 * q.numel() * 2 + fast + 4 * (2 << 20), (taken, fast)
+
+
+def test_a_failed_call_leaves_no_error_for_the_next():
+    """A stream whose recording has been invalidated refuses every launch, on the host.  The call that meets it answers with the
+    error; the next call, on a stream that is well, has none."""
+    import ctypes
+
+    from deers_b200 import _lib, ops
+    rt, L = ctypes.CDLL("libcudart.so.12"), _lib.lib()                      # the runtime torch has loaded
+    a, b, c = (torch.ones((64, 64), device="cuda") for _ in range(3))
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        sick = ops.Context.current(a.device)
+    well = ops.Context.current(a.device)
+    assert sick.handle != well.handle
+
+    def product(ctx):
+        return L.deers_b200_gemm_f32(ctx.handle, 64, 64, 64, a.data_ptr(), 64, 0, b.data_ptr(), 64, 1, c.data_ptr(), 64, None, None, 0)
+
+    assert product(well) == _lib.OK and product(sick) == _lib.OK
+    torch.cuda.synchronize()
+    assert rt.cudaStreamBeginCapture(ctypes.c_void_p(st.cuda_stream), 2) == 0
+    assert rt.cudaStreamSynchronize(ctypes.c_void_p(st.cuda_stream)) != 0   # not allowed while recording: invalidates it
+    assert product(sick) == _lib.ERR_CUDA
+    assert product(well) == _lib.OK
+    graph = ctypes.c_void_p()
+    assert rt.cudaStreamEndCapture(ctypes.c_void_p(st.cuda_stream), ctypes.byref(graph)) != 0 and not graph.value
+    rt.cudaGetLastError()
+    assert product(sick) == _lib.OK and product(well) == _lib.OK
+    torch.cuda.synchronize()
+    assert torch.all(c == 64.0)
