@@ -228,22 +228,22 @@ __global__ void __launch_bounds__(128, END == DEC_CLUSTER ? 6 : 7) decode_vec_ke
                 s[u] = ok[u] ? s[u] * sl2 : -INFINITY;
                 mx = fmaxf(mx, s[u]);
             }
-            if (mx != -INFINITY) {                               // at least one key of this lane group so far
-                const float corr = exp2f(m - mx);
-                l *= corr;
+            // The maximum is -inf before this lane group's first key, but also while all its scores are NaN (fmaxf passes over
+            // them): those must reach the sums, so no step is skipped.
+            const float ms = mx == -INFINITY ? 0.f : mx, corr = exp2f(m - ms);
+            l *= corr;
 #pragma unroll
-                for (int c = 0; c < VEC; ++c) acc[c] *= corr;
+            for (int c = 0; c < VEC; ++c) acc[c] *= corr;
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const float pj = exp2f(s[u] - mx);           // 0 for keys that do not exist
-                    l += pj;
-                    float vf[VEC];
-                    unpack(vr[u], vf);
+            for (int u = 0; u < U; ++u) {
+                const float pj = exp2f(s[u] - ms);               // 0 for keys that do not exist
+                l += pj;
+                float vf[VEC];
+                unpack(vr[u], vf);
 #pragma unroll
-                    for (int c = 0; c < VEC; ++c) acc[c] = fmaf(pj, vf[c], acc[c]);
-                }
-                m = mx;
+                for (int c = 0; c < VEC; ++c) acc[c] = fmaf(pj, vf[c], acc[c]);
             }
+            m = mx;
         }
         // merge the lane groups of the warp (they saw different keys), then the four warps
 #pragma unroll

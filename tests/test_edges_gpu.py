@@ -549,3 +549,31 @@ def test_a_failed_call_leaves_no_error_for_the_next():
     assert product(sick) == _lib.OK and product(well) == _lib.OK
     torch.cuda.synchronize()
     assert torch.all(c == 64.0)
+
+
+@pytest.mark.parametrize("dtype,D,Tk,Tq", [(torch.float16, 80, 2, 1), (torch.float16, 64, 9, 1), (torch.float16, 128, 40, 3),
+                                           (torch.float32, 56, 17, 17), (torch.float16, 96, 700, 1), (torch.float32, 128, 3000, 2)])
+def test_decode_nan_and_inf_scores(dtype, D, Tk, Tq):
+    """A NaN in a key is in the result of every query that sees it, also where the lanes that hold the key hold no other; a
+    score of -inf is a weight of zero."""
+    from deers_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(Tk)
+    q = torch.rand((2, 2, Tq, D), device="cuda", generator=g).to(dtype) + 0.5
+    k, v = (torch.randn((2, 2, Tk, D), device="cuda", generator=g).to(dtype) for _ in range(2))
+    for j in sorted({0, 1, Tk // 2, Tk - 1}):
+        sees = torch.arange(Tq, device="cuda") + Tk - Tq >= j
+        bad = k.clone()
+        bad[1, 0, j, D - 1] = float("nan")
+        o, lse = ops.attention_decode(q, bad, v, want_lse=True)
+        want = torch.zeros((2, 2, Tq), dtype=torch.bool, device="cuda")
+        want[1, 0] = sees
+        assert torch.equal(lse.isnan(), want) and torch.equal(o.isnan(), want[..., None].expand_as(o)), j
+        bad[1, 0, j, D - 1] = float("-inf")
+        o = ops.attention_decode(q, bad, v)
+        alone = Tq == Tk and j == 0                                         # the first query sees nothing else: 0 / 0
+        s = (q.double() @ k.double().transpose(2, 3)) / D ** 0.5
+        s[1, 0, :, j] = float("-inf")
+        s = s.masked_fill(torch.ones(Tq, Tk, dtype=torch.bool, device="cuda").triu(Tk - Tq + 1), float("-inf"))
+        exact = s.softmax(-1) @ v.double()
+        assert torch.equal(o.isnan(), exact.isnan()) and bool(exact.isnan().any()) == alone, j
+        assert_close(o.nan_to_num().float().cpu().numpy(), exact.nan_to_num().cpu().numpy(), TOL_F16 if dtype == torch.float16 else 1e-4, f"{j}")
