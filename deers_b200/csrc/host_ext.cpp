@@ -5,7 +5,8 @@
 // stride and on allocating through the dispatcher.  Here the checks, the output and workspace
 // allocations (torch's caching allocator, without the dispatcher) and the C-ABI call happen in one native function.
 // The functions answer None for anything they do not take as it is (wrong type, shape, device or a layout
-// that needs compaction); the Python mirror then raises the matching error or compacts and calls again.
+// that needs compaction); the Python mirror then raises the matching error or compacts and calls again, saying so: what is
+// still not to the library's liking (a head_dim, a contiguous tensor off a 16-byte boundary) is refused with its status.
 // Allocations and library calls run without the interpreter lock (a launch waits while the device's queue is full); a lock
 // per context keeps the threads that share a stream, and so a context, apart.
 #include <Python.h>
@@ -71,9 +72,11 @@ inline int dtype_code(const at::Tensor& t) {
     return t.scalar_type() == at::kHalf ? DEERS_F16 : t.scalar_type() == at::kFloat ? DEERS_F32 : -1;
 }
 
-// 4-D, on a CUDA device, f16 or f32, and the kernels can read it in place (ops._usable).
+// 4-D, on a CUDA device, f16 or f32: the library can be asked.
+inline bool offerable(const at::Tensor& t) { return t.dim() == 4 && t.is_cuda() && dtype_code(t) >= 0; }
+// The same, and the kernels can read it in place (ops._usable).
 inline bool usable(const at::Tensor& t) {
-    if (t.dim() != 4 || !t.is_cuda() || dtype_code(t) < 0 || t.stride(3) != 1) return false;
+    if (!offerable(t) || t.stride(3) != 1) return false;
     const int64_t align = t.scalar_type() == at::kHalf ? 16 : 4, es = t.element_size();
     if ((uintptr_t)t.data_ptr() % align) return false;
     // a repeated (expanded) axis is compacted where the tile is wider than the row: TMA maps want real strides
@@ -146,12 +149,16 @@ PyObject* compatible(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Py_RETURN_TRUE;
 }
 
-// attn_fwd(q, k, v, scale, causal, token_major, out | None) -> (o, lse) | None
+// attn_fwd(q, k, v, scale, causal, token_major, out | None, compacted) -> (o, lse) | None.  compacted: what compaction could do
+// has been done, the library judges the layout.
 PyObject* attn_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HOST_BEGIN
-    if (n != 7) Py_RETURN_NONE;
+    if (n != 8) Py_RETURN_NONE;
     const at::Tensor *q = tensor(args[0]), *k = tensor(args[1]), *v = tensor(args[2]);
-    if (!q || !k || !v || !usable(*q) || !usable(*k) || !usable(*v) || !same(*q, *k) || !same(*q, *v)) Py_RETURN_NONE;
+    const bool compacted = PyObject_IsTrue(args[7]);
+    if (!q || !k || !v) Py_RETURN_NONE;
+    for (const at::Tensor* t : {q, k, v})
+        if (!(compacted ? offerable(*t) : usable(*t)) || !same(*q, *t)) Py_RETURN_NONE;
     const double scale = PyFloat_AsDouble(args[3]);
     if (scale == -1.0 && PyErr_Occurred()) return nullptr;
     Ctx* ctx = context_for(q->get_device());
@@ -205,15 +212,16 @@ size_t used_workspace_bytes(const deers_attn_desc& d, int pass) {
     return deers_b200_attn_workspace_bytes(&tile, pass);
 }
 
-// attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace | None, dv_out | None) -> (dq, dk, dv) | None
+// attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace | None, dv_out | None, compacted) -> (dq, dk, dv) | None
 PyObject* attn_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HOST_BEGIN
-    if (n != 10) Py_RETURN_NONE;
+    if (n != 11) Py_RETURN_NONE;
     const at::Tensor *q = tensor(args[0]), *k = tensor(args[1]), *v = tensor(args[2]), *o = tensor(args[3]), *lse = tensor(args[4]),
                      *g = tensor(args[5]);
+    const bool compacted = PyObject_IsTrue(args[10]);
     if (!q || !k || !v || !o || !lse || !g) Py_RETURN_NONE;
     for (const at::Tensor* t : {q, k, v, o, g})
-        if (!usable(*t) || !same(*q, *t)) Py_RETURN_NONE;
+        if (!(compacted ? offerable(*t) : usable(*t)) || !same(*q, *t)) Py_RETURN_NONE;
     const double scale = PyFloat_AsDouble(args[6]);
     if (scale == -1.0 && PyErr_Occurred()) return nullptr;
     Ctx* ctx = context_for(q->get_device());

@@ -180,7 +180,7 @@ def attention_fwd(q, k, v, scale: float, causal: bool = True, token_major_out: b
     and the returned tensor is the [B,H,T,D] view of it, so the module's
     ``permute([0,2,1,3]).reshape([B,T,C])`` (src/models/gpt.rs:144) is a free view instead of the
     compaction copy of src/ops.rs:913: the kernels write through the view's strides."""
-    got = _host.attn_fwd(q, k, v, scale, causal, token_major_out, out)
+    got = _host.attn_fwd(q, k, v, scale, causal, token_major_out, out, False)
     if got is not None:
         return got
     _check_inputs("attention_fwd", (q, k, v))
@@ -188,7 +188,7 @@ def attention_fwd(q, k, v, scale: float, causal: bool = True, token_major_out: b
     Context.current(q.device)                # raises for a CPU tensor
     if out is not None and (out.shape != q.shape or out.dtype != q.dtype or out.device != q.device or not _usable(out)):
         raise LayoutMismatch(f"attention_fwd: out must match q ({tuple(q.shape)}, {q.dtype}) with unit inner stride")
-    return _taken("attention_fwd", _host.attn_fwd(q, k, v, scale, causal, token_major_out, out))
+    return _taken("attention_fwd", _host.attn_fwd(q, k, v, scale, causal, token_major_out, out, True))
 
 
 def workspace_bytes(q, scale: float = 1.0, causal: bool = True, pass_: int = 1) -> int:
@@ -205,7 +205,7 @@ def attention_bwd(q, k, v, o, lse, d_o, scale: float, causal: bool = True, works
     most a quarter of the free memory or 1/512 of the device's.  `dv_out` (a [B,H,T,D] view
     with inner stride 1, e.g. the v slice of a fused dqkv buffer seen head-major) receives dV in place
     instead: the kernels write through its strides."""
-    got = _host.attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace, dv_out)
+    got = _host.attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace, dv_out, False)
     if got is not None:
         return got
     _check_inputs("attention_bwd", (q, k, v, o, d_o))
@@ -213,7 +213,7 @@ def attention_bwd(q, k, v, o, lse, d_o, scale: float, causal: bool = True, works
     Context.current(q.device)
     if dv_out is not None and (tuple(dv_out.shape) != tuple(q.shape) or dv_out.dtype != q.dtype or not _usable(dv_out)):
         raise LayoutMismatch("attention_bwd: dv_out must be a [B,H,T,D] view with inner stride 1 and aligned rows")
-    return _taken("attention_bwd", _host.attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace, dv_out))
+    return _taken("attention_bwd", _host.attn_bwd(q, k, v, o, lse, d_o, scale, causal, workspace, dv_out, True))
 
 
 def precompute_rotary_embeddings(seq_len: int, head_dim: int, base: float = 10000.0,

@@ -551,6 +551,32 @@ def test_a_failed_call_leaves_no_error_for_the_next():
     assert torch.all(c == 64.0)
 
 
+def test_f16_tensors_off_a_16_byte_boundary():
+    """A view that starts anywhere is compacted; a contiguous tensor that does, or a head_dim there are no tiles for, is refused
+    with the library's own status."""
+    from deers_b200 import _lib, ops
+    from deers_b200.errors import CudaError
+    B, H, T, D = 1, 2, 20, 64
+    g = torch.Generator(device="cuda").manual_seed(3)
+    good = torch.randn((B, H, T, D), dtype=torch.float16, device="cuda", generator=g)
+    wide = torch.randn((B, H, T, D + 8), dtype=torch.float16, device="cuda", generator=g)
+    view = wide[..., 1:D + 1]
+    off = torch.randn(B * H * T * D + 1, dtype=torch.float16, device="cuda", generator=g)[1:].view(B, H, T, D)
+    scale = ops.default_scale(D)
+    o, lse = ops.attention_fwd(view, good, good, scale)
+    o2, lse2 = ops.attention_fwd(view.contiguous(), good, good, scale)
+    assert torch.equal(o, o2) and torch.equal(lse, lse2)
+    for call in (lambda: ops.attention_fwd(off, good, good, scale), lambda: ops.attention_bwd(good, good, off, o, lse, good, scale)):
+        with pytest.raises(CudaError) as e:
+            call()
+        assert e.value.status == _lib.ERR_LAYOUT
+    x = torch.zeros((1, 2, 4, 100), dtype=torch.float16, device="cuda")
+    for call in (lambda: ops.attention_fwd(x, x, x, scale), lambda: ops.attention_bwd(x, x, x, x, lse, x, scale)):
+        with pytest.raises(CudaError) as e:
+            call()
+        assert e.value.status == _lib.ERR_SHAPE
+
+
 @pytest.mark.parametrize("dtype,D,Tk,Tq", [(torch.float16, 80, 2, 1), (torch.float16, 64, 9, 1), (torch.float16, 128, 40, 3),
                                            (torch.float32, 56, 17, 17), (torch.float16, 96, 700, 1), (torch.float32, 128, 3000, 2)])
 def test_decode_nan_and_inf_scores(dtype, D, Tk, Tq):
