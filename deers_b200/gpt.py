@@ -246,12 +246,9 @@ def gemm_f32(a: torch.Tensor, b: torch.Tensor, a_mn_major: bool = False, b_mn_ma
     ep = _lib.GemmEpilogue(epilogue, residual.data_ptr() if residual is not None else None,
                            residual.stride(0) if residual is not None else 0,
                            aux.data_ptr() if aux is not None else None)
-    L = _lib.lib()
-    nbytes = int(L.deers_b200_gemm_f32_workspace_bytes(ctx.handle, M, N, K))
-    ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=a.device)
-    _lib.check(L.deers_b200_gemm_f32(ctx.handle, M, N, K, a.data_ptr(), a.stride(0), int(a_mn_major), b.data_ptr(),
-                                     b.stride(0), int(b_mn_major), c.data_ptr(), c.stride(0), ctypes.byref(ep),
-                                     ws.data_ptr(), ws.numel()), ctx.handle)
+    _lib.check(_lib.lib().deers_b200_gemm_f32(ctx.handle, M, N, K, a.data_ptr(), a.stride(0), int(a_mn_major), b.data_ptr(),
+                                              b.stride(0), int(b_mn_major), c.data_ptr(), c.stride(0), ctypes.byref(ep),
+                                              None, 0), ctx.handle)
     return c
 
 
