@@ -7,13 +7,13 @@
 //   2. attn_bwd_dkdv_f16_kernel   per (batch*head, KV tile of 128 rows), KV-stationary: walks the
 //                                  query tiles at or below the diagonal with the dK and dV
 //                                  accumulators resident in TMEM for the whole walk
-//   3. attn_bwd_dq_f16_kernel     per (batch*head, query tile of 128 rows), Q-stationary: walks the
-//                                  KV tiles at or left of the diagonal with the dQ accumulator
-//                                  resident in TMEM
-// Both main kernels recompute P from the saved lse.  Recomputing S and dP in the dQ kernel costs
-// two extra products per tile pair (7 instead of 5), but the alternative - adding every
-// 128 x D partial dQ tile into a float32 accumulator in global memory - was measured to be
-// bound by the L2's reduction throughput (about 4 TB/s: 35 GB of reductions at B=64, H=32,
+//   3. dQ, per (batch*head, query tile of 128 rows), Q-stationary: walks the KV tiles at or left of the diagonal with the
+//      dQ accumulator resident in TMEM
+//        attn_bwd_dq_from_ds_f16_kernel   when the workspace has room for the dS tiles (the host layers' default): kernel 2 has
+//                                         kept them, and dQ is one streaming product, 5 products per tile pair in all
+//        attn_bwd_dq_f16_kernel           otherwise: recomputes S and dP, 7 products per tile pair
+// P is recomputed from the saved lse.  Adding every 128 x D partial dQ tile into a float32 accumulator in global memory
+// instead was measured to be bound by the L2's reduction throughput (about 4 TB/s: 35 GB of reductions at B=64, H=32,
 // T=2048, D=128) and needed two more memory passes to clear and convert that accumulator.
 //
 // dK/dV kernel: everything is computed transposed so that no operand needs a data movement
@@ -119,8 +119,9 @@ __device__ __forceinline__ int4 next_item(const BwdParams& p, int n, int n_items
 // at a time and the multiply-adds run two to an instruction; arrivals are one per warp; a finished dS^T tile goes through
 // the stage of the dO tile it no longer needs and ONE bulk copy to global memory (stores from the compute threads cost
 // 1200 cycles a step); and an item's dK / dV leave TMEM after the next item's first P^T has been handed over.
-// B2 H16 T4096 D128, cycles per CTA: 433 k -> 378 k with dS kept, 357 k -> 328 k without.  A share of the exponentials
-// on the FMA pipe (polynomial) changed nothing: the phase is then bound by its instructions.
+// B2 H16 T4096 D128 (114 steps), cycles per CTA: 496 k -> 371 k with dS kept, 448 k -> 315 k without; B16 H12 T1024 D64
+// (47 steps): 157 k.  A share of the exponentials on the FMA pipe (polynomial) changed nothing: the phase is then bound by its
+// instructions.
 // Dynamic shared memory only; the base must be 1024-byte aligned for the 128-byte swizzle (checked).
 template <int D>
 struct DkvSmem {

@@ -20,9 +20,9 @@
 //               end of an item the partial sums are combined, O is normalised and O and the row lse are stored.
 //   What bounds it at D = 128, per 128 x 128 step: 1024 cycles each of tensor pipe and special-function unit, 1280 of
 //   shared memory.  With all sixteen softmax warps in step (one step at a time, 32 columns each) a step took 2170 cycles; two
-//   groups with two S tiles 2250 (a group then waits for P V of its last step and for S), with three 1720.  The loops are
+//   groups with two S tiles 2250 (a group then waits for P V of its last step and for S), with three 1770.  The loops are
 //   rolled to 32 columns: unrolled further, warps in different phases evict one another's code.
-//   B2 H16 T4096 D128: 247 k -> 197 k cycles per CTA; B16 H12 T1024 D64: 118 k -> 99 k.
+//   B2 H16 T4096 D128: 247 k -> 202 k cycles per CTA; B16 H12 T1024 D64: 118 k -> 98 k.
 // Scale, causal mask, softmax and both products happen in this one pass; the T x T scores
 // never reach global memory.
 #include "sm100_ptx.cuh"

@@ -61,8 +61,8 @@ struct deers_ctx {
     cudaEvent_t pipe_ev[3][3];      // [buffer set][h2d done, compute done, d2h done]
     bool pipe_ready;
     bool no_chain;                  // launches follow work of another stream: nothing to overlap with (launch_chained)
-    int cluster_room_f16[9];        // the same for the f16 GEMM's CTAs (gemm_f16_sm100.cu)
     int cluster_capacity[9];        // [n]: clusters of n blocks the device holds at once (gemm_f32.cu; 0: not asked yet)
+    int cluster_room_f16[9];        // the same for the f16 GEMM's CTAs (gemm_f16_sm100.cu)
 };
 
 // Brackets one kernel launch with events when timing is on.  A full ring drops the sample.
@@ -111,7 +111,8 @@ struct KernelTimerScope {
 // Back-to-back kernels.  A kernel launched by launch_chained() may be set up while the one before it still runs: it calls
 // chain_wait() before its first access to global memory (the predecessor has finished and its writes are visible; every
 // kernel of a chain waits, so this covers all before it) and chain_next() where its own successor may be set up.
-// Saves the launch gap of a microsecond or two: 54 kernels of a GPT forward on a short prompt 232 -> 206 us.  Where chain_next()
+// Saves the launch gap of a microsecond or two: 54 kernels of a GPT forward on a short prompt, replayed from a graph,
+// 232 -> 206 us; launched one by one, where the host's time hides as well, 495 -> 214 us.  Where chain_next()
 // stands matters: a successor set up at the start of a kernel of few large blocks takes the idle SMs unevenly (252 us), so
 // those call it once their last loads are under way; kernels of small blocks call it first.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -153,9 +154,11 @@ template <typename... P, typename... A>
     return cudaLaunchKernelEx(&lc, kernel, std::forward<A>(args)...);
 }
 
-// A long kernel of one block per SM gains nothing from an early start and loses: its blocks then land on the SMs in the order
-// in which the predecessor's leave, not neighbours next to one another (B64 H32 T2048 D128 forward and backward: 10470 us
-// unchained, 10870 chained).  steps: 128 x 128 score tiles (or the like, about half a microsecond) per block.
+// A long kernel of one block per SM gains nothing from an early start, and its blocks then land on the SMs in the order in
+// which the predecessor's leave, not neighbours next to one another.  B64 H32 T2048 D128 forward and backward was never faster
+// chained: 10870 us against 10470 unchained in one call, 11300 against 11180 and 11360 against 11220 in two more (runs of one
+// side differ by 1.5 % and more there, so this is a choice between near equals); B2 H16 T8192 D128 2279 against 2264.
+// steps: 128 x 128 score tiles (or the like, about half a microsecond) per block.
 struct ChainScope {
     deers_ctx* ctx;
     bool was;
@@ -192,7 +195,7 @@ int launch_attn_bwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q
                         const float* v, const float* o, const float* lse, const float* d_o, float* dq,
                         float* dk, float* dv);
 
-// f16 tcgen05 path (attn_f16_sm100.cu)
+// f16 tcgen05 path (attn_fwd_f16_sm100.cu, attn_bwd_f16_sm100.cu)
 int launch_attn_fwd_f16(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const void* k,
                         const void* v, void* o, float* lse);
 int launch_attn_bwd_f16(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const void* k,

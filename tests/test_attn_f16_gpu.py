@@ -73,13 +73,13 @@ def test_forward_rescale_path():
 @pytest.mark.parametrize("shape", [
     (2, 3, 300, 32),     # the reference GPT's head_dim (n_embd 192 / 6 heads) in f16
     (1, 2, 130, 16),
-    (1, 2, 257, 96),     # padded to 128
+    (1, 2, 257, 96),     # on 128-wide tiles
     (1, 1, 64, 8),
 ])
 def test_head_dims_other_than_64_and_128(shape):
     """The reference derives head_dim = n_embd / n_head freely (src/models/gpt.rs:86-100).  f16 head dims that
-    are not a tensor-core tile width run on zero-padded copies: forward and backward against the oracle, and
-    the workspace sizes the padded path asks for."""
+    are not a tensor-core tile width run in place on the 64- or 128-wide tiles: forward and backward against the
+    oracle, and the sizes reported for them, which keep the room that callers may have planned for."""
     from deers_b200 import ops
     from tests.gpu_util import check_case
     check_case(*shape, torch.float16, TOL_F16, seed=sum(shape))
