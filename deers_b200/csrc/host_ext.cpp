@@ -44,6 +44,8 @@ Ctx* context_for(int device) {
     void* p = PyLong_AsVoidPtr(r);
     Py_DECREF(r);
     if (!p) return nullptr;
+    for (const auto& e : g_contexts)                 // another thread may have got here while Python ran
+        if (e->stream == s && e->device == device) return e.get();
     std::unique_ptr<Ctx> e(new Ctx());
     e->device = device; e->stream = s; e->handle = (deers_ctx*)p;
     g_contexts.push_back(std::move(e));

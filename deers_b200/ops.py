@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import threading
 from typing import Dict, List, Optional, Tuple
 
 import torch
@@ -49,6 +50,7 @@ class Context:
     (src/storage/cuda.rs:455-521).  Work is enqueued on torch's current stream."""
 
     _cache: Dict[Tuple[int, int], "Context"] = {}
+    _making = threading.Lock()
 
     def __init__(self, device: int, stream_ptr: int):
         self.handle = ctypes.c_void_p()
@@ -68,9 +70,12 @@ class Context:
         key = (idx, stream)
         ctx = cls._cache.get(key)
         if ctx is None:
-            ctx = cls(idx, stream)
-            ctx._stream_obj = stream_obj     # keeps the stream alive: its handle value cannot be reused by another
-            cls._cache[key] = ctx
+            with cls._making:                # one context per stream, also when two threads meet it first
+                ctx = cls._cache.get(key)
+                if ctx is None:
+                    ctx = cls(idx, stream)
+                    ctx._stream_obj = stream_obj     # keeps the stream alive: its handle value cannot be reused by another
+                    cls._cache[key] = ctx
         return ctx
 
     @classmethod

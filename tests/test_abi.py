@@ -120,3 +120,29 @@ def test_rotary_pack_validation_without_a_gpu():
         ops.RotaryPack.new(torch.zeros(2, 5, 3, 8, dtype=torch.int64), cos, sin)
     with pytest.raises(LayoutMismatch):
         ops.precompute_rotary_embeddings(5, 7)
+
+
+def test_two_threads_that_meet_a_stream_first_share_its_context(monkeypatch):
+    """A kernel's error word belongs to a context: with two on one stream, a synchronise would ask the wrong one."""
+    import threading
+    import time
+    from types import SimpleNamespace
+
+    import torch
+    from deers_b200 import ops
+    made = []
+
+    def slow_init(self, device, stream_ptr):
+        made.append(stream_ptr)
+        time.sleep(0.2)
+
+    monkeypatch.setattr(ops.Context, "__init__", slow_init)
+    monkeypatch.setattr(ops.Context, "_cache", {})
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda idx: SimpleNamespace(cuda_stream=77))
+    got = []
+    threads = [threading.Thread(target=lambda: got.append(ops.Context.current(torch.device("cuda", 0)))) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert made == [77] and len(got) == 4 and all(c is got[0] for c in got)
