@@ -371,7 +371,7 @@ def run_decode(args, dtype, B, T, H, D):
                                    f"cache T={T} head_dim={D}",
                        "l2": "256 MB flush write between steps" if small else "cache larger than L2"},
             "gpu_launches": int(launches), "clocks": clocks, "e2e": None,
-            "roofline": {"bound": "hbm", "kernel": "decode_partial_kernel + decode_combine_kernel", "achieved": achieved,
+            "roofline": {"bound": "hbm", "kernel": "decode_vec_kernel (decode_partial_kernel for other rows, decode_combine_kernel behind many chunks)", "achieved": achieved,
                          "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"], "traffic": None,
                          "bytes_per_step": bytes_step, "kernel_ms_per_step": k_ms / args.steps,
                          "peak_source": peaks["source"] + " copy bandwidth"},

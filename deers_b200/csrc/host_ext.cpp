@@ -1,8 +1,8 @@
 // Native host layer of the Python mirror (deers_b200/ops.py): one CPython call per operator.
 //
-// What bounds the small calls of the operator interface is the host, not the GPU: a decode step is two kernels of
-// 7 us together, and the same call spent 28 us of Python on argument checks, on filling a ctypes descriptor stride by
-// stride and on allocating through the dispatcher.  Here the checks, the output and workspace
+// What bounds the small calls of the operator interface is the host, not the GPU: around a decode step's 5 - 7 us of kernels
+// the same call spent 28 us of Python on argument checks, on filling a ctypes descriptor stride by
+// stride and on allocating through the dispatcher (9 us now).  Here the checks, the output and workspace
 // allocations (torch's caching allocator, without the dispatcher) and the C-ABI call happen in one native function.
 // The functions answer None for anything they do not take as it is (wrong type, shape, device or a layout
 // that needs compaction); the Python mirror then raises the matching error or compacts and calls again, saying so: what is

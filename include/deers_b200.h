@@ -309,7 +309,7 @@ int deers_b200_rmsnorm_bwd(deers_ctx* ctx, int64_t rows, int32_t C, const float*
  * the mask `functional::causal_mask(batch, tgt_len = Tq, seqlen_offset = Tk - Tq)` builds
  * (`src/nn/functional.rs:12-55`).  The reference has no cache: its sampling loop re-runs the whole prefix
  * through `GPT::forward` for every token; with this entry point a step reads K and V once (split over the
- * keys across CTAs, merged by a second launch).  q, o: [B,H,Tq,D]; k_cache, v_cache: [B,H,Tk,D]; strides in
+ * keys across CTAs, merged inside a cluster or by a second launch).  q, o: [B,H,Tq,D]; k_cache, v_cache: [B,H,Tk,D]; strides in
  * elements, inner stride 1 (a cache allocated for more than Tk rows is passed with its own row / slice
  * strides).  f16 or f32 storage, f32 arithmetic; D <= 256, Tq <= 128, B*H <= 65535.  lse (optional, [B,H,Tq]
  * f32, natural log) like deers_b200_attn_fwd.  Workspace: deers_b200_attn_decode_workspace_bytes(desc)
