@@ -12,10 +12,20 @@
 //
 // What bounds it: the model's products are small (1024 x 576 x 192 and the like): 150 tiles of 64 x 64, one per SM, so
 // a product takes as long as ONE block takes for its walk over K.  The block is built around that walk:
-//   * 128 threads own the tile (patches of PM x PN) and KS such groups split every stage's k, so that each scheduler
-//     has four warps to hide shared-memory and FFMA latency with, at 3 LDS.128 per 32 FFMA;
+//   * 128 threads own the tile (patches of PM x PN) and KS such groups take a share of every stage's k each: loads,
+//     waits and arithmetic of a group are its own, so the groups drift apart and one's shared-memory bursts meet another's
+//     multiply-adds;
+//   * the loop is bound by issue slots, register banks and shared memory together.  Two products share a slot
+//     (fma.rn.f32x2, each an IEEE f32 fma): neighbouring columns where B is in MN order, even and odd k in small K-order
+//     patches (large ones would need twice the accumulators and stay with single products; packing columns there costs
+//     two moves per pair and was slower: 11.4 -> 15.4 us at 1024 x 768 x 192).  Lanes lie in the tile so that a 16-byte
+//     shared-memory read costs 2.1 cycles instead of 4: it does when each quarter warp asks for at most four addresses and
+//     neighbouring lanes share them (lane % 8 along a row does not, (lane / 2) % 4 does; measured);
 //   * operands travel by cp.async straight into shared memory in their storage order (no transposition, no
-//     registers), up to STAGES * 32 k ahead: for K = 192 the whole operand is in flight at once;
+//     registers), up to STAGES * 64 k ahead: for K = 192 the whole operand is in flight at once.
+// Back to back in a graph, single products and 512-thread stages before, pairs and groups now (us):
+//   1024 x 768 x 192 11.2 -> 10.7, 1024 x 192 x 768 13.0 -> 12.5, 100 x 576 x 192 3.8 -> 3.5, weight gradients (both
+//   operands in MN order) 768 x 192 x 1024 13.5 -> 10.9, 192 x 500 x 231 4.8 -> 4.0.
 //   * k groups, and the blocks of a cluster that split a long K among them (weight gradients), meet in shared
 //     memory: group 0..KS-1 of block 0..P-1 are added in that order by the threads that write the tile (distributed
 //     shared memory, one cluster barrier), so nothing goes through global memory, no counter, no workspace, and the
@@ -27,7 +37,8 @@
 namespace {
 namespace cg = cooperative_groups;
 
-constexpr int BK = 64;                                  // depth of one stage
+constexpr int GT = 128;                                 // threads of a k group
+constexpr int BK = 64;                                  // depth of one stage, shared evenly by the k groups
 constexpr int MAX_PARTS = 8;                            // blocks of a cluster along K (portable cluster size)
 
 struct GemmArgs {
@@ -62,27 +73,43 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// One operand's stage in shared memory, in its storage order: R rows (m or n) of BK k when k is contiguous, BK rows of
-// R when m / n is.  Row strides are 4 mod 32 words (16-byte pieces of 8 consecutive rows fall into different banks).
-template <int R, bool MN, int GT>
+// The threads of a k group meet (barrier 0 is __syncthreads).
+__device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
+
+// Two f32 products in one issue slot (each a plain IEEE fma).
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// One operand's stage of one k group in shared memory, in its storage order: R rows (m or n) of KG k when k is contiguous,
+// KG rows of R when m / n is.  Row strides are 4 mod 16 words (16-byte pieces of neighbouring rows fall into different banks).
+template <int R, bool MN, int KG>
 struct Operand {
-    static constexpr int LD = MN ? R + 4 : BK + 4;
-    static constexpr int FLOATS = MN ? BK * LD : R * LD;
-    static constexpr int LEN = MN ? R : BK, ROWS = MN ? BK : R;     // contiguous floats per row, rows
+    static constexpr int LD = MN ? R + 4 : KG + 4;
+    static constexpr int FLOATS = MN ? KG * LD : R * LD;
+    static constexpr int LEN = MN ? R : KG, ROWS = MN ? KG : R;     // contiguous floats per row, rows
     static constexpr int NP = ROWS * LEN / 4 / GT;                  // 16-byte pieces per thread and stage
     static_assert(NP * GT * 4 == ROWS * LEN, "whole pieces per thread");
     const float* base;
     const float* src[NP];    // this thread's pieces of the next stage
     int dst[NP];             // their places in the stage (floats)
     int along_r[NP];         // floats of a piece inside the matrix along m / n (K order: 4 or 0)
-    int along_k[NP];         // k of a piece inside the stage
+    int along_k[NP];         // k of a piece inside the group's share of the stage
     long long step;          // from one stage to the next
-    __device__ __forceinline__ void init(const float* b, long long ld, int r0, int rmax, int k0) {
+    __device__ __forceinline__ void init(const float* b, long long ld, int r0, int rmax, int k0, int t) {
         base = b;
         step = MN ? BK * ld : BK;
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
-            const int idx = threadIdx.x + i * GT;
+            const int idx = t + i * GT;
             const int row = idx / (LEN / 4), col = (idx % (LEN / 4)) * 4;
             const int r = r0 + (MN ? col : row), k = MN ? row : col;
             along_k[i] = k;
@@ -91,12 +118,12 @@ struct Operand {
             src[i] = b + (MN ? (long long)(k0 + k) * ld + r : (long long)r * ld + k0 + k);
         }
     }
-    // Enqueues the next stage's pieces; kv is the number of its k that exist.
+    // Enqueues the next stage's pieces; kv is the number of the group's k that exist.
     __device__ __forceinline__ void fetch(float* s, int kv, bool vec) {
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
             int valid = along_r[i];
-            if (kv < BK) valid = MN ? (along_k[i] < kv ? valid : 0) : min(valid, max(0, kv - along_k[i]));
+            if (kv < KG) valid = MN ? (along_k[i] < kv ? valid : 0) : min(valid, max(0, kv - along_k[i]));
             const float* p = valid > 0 ? src[i] : base;
             if (vec) {
                 cp16(s + dst[i], p, 4 * valid);
@@ -116,52 +143,63 @@ struct Operand {
         const int q = i / 4 * 4, w = P - q >= 4 ? 4 : P - q;       // first element and width of i's group
         return q * G + t * w + (i - q);
     }
-    // The P elements of this thread: K order reads four k at a time (v[i][kk]), MN order one k at a time (v[i][0]).
-    static constexpr int KV = MN ? 1 : 4;
-    template <int P>
-    static __device__ __forceinline__ void read(const float* s, int t, int k, float (&v)[P][KV]) {
+    // The P elements of this thread for U (2 or 4) consecutive k.
+    template <int P, int U>
+    static __device__ __forceinline__ void read(const float* s, int t, int k, float (&v)[U][P]) {
         if constexpr (!MN) {
 #pragma unroll
             for (int i = 0; i < P; ++i) {
-                const float4 x = *reinterpret_cast<const float4*>(s + index<P>(t, i) * LD + k);
-                v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+                const float* q = s + index<P>(t, i) * LD + k;
+                if constexpr (U == 4) {
+                    const float4 x = *reinterpret_cast<const float4*>(q);
+                    v[0][i] = x.x; v[1][i] = x.y; v[2][i] = x.z; v[3][i] = x.w;
+                } else {
+                    const float2 x = *reinterpret_cast<const float2*>(q);
+                    v[0][i] = x.x; v[1][i] = x.y;
+                }
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < P; i += 4) {
-                if (P - i >= 4) {
-                    const float4 x = *reinterpret_cast<const float4*>(s + k * LD + index<P>(t, i));
-                    v[i][0] = x.x; v[i + 1][0] = x.y; v[i + 2][0] = x.z; v[i + 3][0] = x.w;
-                } else {
-                    const float2 x = *reinterpret_cast<const float2*>(s + k * LD + index<P>(t, i));
-                    v[i][0] = x.x; v[i + 1][0] = x.y;
+            for (int kk = 0; kk < U; ++kk)
+#pragma unroll
+                for (int i = 0; i < P; i += 4) {
+                    if (P - i >= 4) {
+                        const float4 x = *reinterpret_cast<const float4*>(s + (k + kk) * LD + index<P>(t, i));
+                        v[kk][i] = x.x; v[kk][i + 1] = x.y; v[kk][i + 2] = x.z; v[kk][i + 3] = x.w;
+                    } else {
+                        const float2 x = *reinterpret_cast<const float2*>(s + (k + kk) * LD + index<P>(t, i));
+                        v[kk][i] = x.x; v[kk][i + 1] = x.y;
+                    }
                 }
-            }
         }
     }
 };
 
 template <int PM, int PN, int KS, bool A_MN, bool B_MN>
 struct GemmShape {
-    static constexpr int BM = 8 * PM, BN = 16 * PN, GT = 128 * KS;
-    using OA = Operand<BM, A_MN, GT>;
-    using OB = Operand<BN, B_MN, GT>;
-    static constexpr int STAGE = OA::FLOATS + OB::FLOATS;
+    static constexpr int BM = 8 * PM, BN = 16 * PN, THREADS = GT * KS, KG = BK / KS;
+    using OA = Operand<BM, A_MN, KG>;
+    using OB = Operand<BN, B_MN, KG>;
+    static constexpr int STAGE = KS * (OA::FLOATS + OB::FLOATS);
     static constexpr int RLD = BN + 4;                              // row stride of the patch staging tile
     static constexpr int RED = KS * BM * RLD;
     static constexpr int STAGES = BM * BN > 64 * 64 ? 3 : 4;
-    static constexpr size_t SMEM = (size_t)(STAGES * STAGE > RED ? STAGES * STAGE : RED) * sizeof(float);
+    static constexpr size_t NEED = (size_t)(STAGES * STAGE > RED ? STAGES * STAGE : RED) * sizeof(float);
+    // A large block has an SM to itself: two of them share its issue slots while others idle (chained launches place the
+    // next product's blocks before this one's have left).
+    static constexpr size_t ALONE = 116 * 1024;
+    static constexpr size_t SMEM = PM * PN >= 16 && NEED < ALONE ? ALONE : NEED;
 };
 
 template <int PM, int PN, int KS, bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(128 * KS) gemm_f32_kernel(const GemmArgs g) {
+__global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
     chain_wait();
     using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
-    constexpr int BM = S::BM, BN = S::BN, GT = S::GT, STAGES = S::STAGES, KG = BK / KS;
+    constexpr int BM = S::BM, BN = S::BN, STAGES = S::STAGES, KG = S::KG;
     extern __shared__ __align__(16) float smem[];
-    const int tid = threadIdx.x % 128, kg = threadIdx.x / 128;      // position in the tile, k group
+    const int tid = threadIdx.x % GT, kg = threadIdx.x / GT;        // position in the tile, k group
     const int w = tid / 32, lane = tid % 32;
-    const int ty = (w & 1) * 4 + lane / 8, tx = (w >> 1) * 8 + lane % 8;
+    const int ty = (w & 1) * 4 + (lane & 1) + 2 * ((lane >> 3) & 1), tx = (w >> 1) * 8 + ((lane >> 1) & 3) + 4 * (lane >> 4);
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int kbeg = blockIdx.z * g.k_chunk;
     const int kend = min(g.K, kbeg + g.k_chunk);
@@ -169,53 +207,103 @@ __global__ void __launch_bounds__(128 * KS) gemm_f32_kernel(const GemmArgs g) {
 
     typename S::OA la;
     typename S::OB lb;
-    la.init(g.a, g.lda, m0, g.M, kbeg);
-    lb.init(g.b, g.ldb, n0, g.N, kbeg);
-    int kv = kend - kbeg;                                           // k left to fetch
-    float* st_in = smem;                                            // stage to fill next
+    la.init(g.a, g.lda, m0, g.M, kbeg + kg * KG, tid);
+    lb.init(g.b, g.ldb, n0, g.N, kbeg + kg * KG, tid);
+    int kv = kend - kbeg - kg * KG;                                 // k left to fetch (of the group's share and what follows)
+    float* const ring = smem + kg * (S::OA::FLOATS + S::OB::FLOATS);
+    int st_in = 0, left = nk;                                       // stage to fill next
     auto fetch = [&]() {
-        if (kv > 0) {
-            la.fetch(st_in, kv, g.a_vec);
-            lb.fetch(st_in + S::OA::FLOATS, kv, g.b_vec);
+        if (left > 0) {
+            la.fetch(ring + st_in, kv, g.a_vec);
+            lb.fetch(ring + st_in + S::OA::FLOATS, kv, g.b_vec);
             kv -= BK;
-            st_in = st_in + S::STAGE == smem + STAGES * S::STAGE ? smem : st_in + S::STAGE;
+            --left;
+            st_in = st_in == (STAGES - 1) * S::STAGE ? 0 : st_in + S::STAGE;
         }
         cp_commit();
     };
 #pragma unroll
     for (int t = 0; t < STAGES - 1; ++t) fetch();
 
+    // Pairs of products: neighbouring columns with B in MN order (a's element twice), even and odd k with B in K order.
+    constexpr bool PAIR_N = B_MN, PAIR_K = !B_MN && PM * PN <= 16;
+    constexpr bool AHEAD = B_MN || PM * PN <= 16;                   // registers for the next fragments as well
+    constexpr int U = !AHEAD || (!A_MN && PM * PN <= 16) ? 4 : 2;
+    constexpr int PC = PAIR_N ? PN / 2 : PAIR_K ? PN : 1;
+    uint64_t acc2[PM][PC];
+#pragma unroll
+    for (int i = 0; i < PM; ++i)
+#pragma unroll
+        for (int j = 0; j < PC; ++j) acc2[i][j] = 0;
     float acc[PM][PN];
 #pragma unroll
     for (int i = 0; i < PM; ++i)
 #pragma unroll
         for (int j = 0; j < PN; ++j) acc[i][j] = 0.f;
 
-    const float* sa = smem;
+    int st_out = 0;
     for (int t = 0; t < nk; ++t) {
         cp_wait<STAGES - 2>();
-        __syncthreads();                                            // stage t has landed, stage t-1 is free
+        group_sync(kg);                                             // stage t has landed, stage t-1 is free
         fetch();
+        const float* sa = ring + st_out;
         const float* sb = sa + S::OA::FLOATS;
+        float a[AHEAD ? 2 : 1][U][PM], b[AHEAD ? 2 : 1][U][PN];     // fragments of U k (and of the next U)
+        if constexpr (AHEAD) {
+            S::OA::template read<PM, U>(sa, ty, 0, a[0]);
+            S::OB::template read<PN, U>(sb, tx, 0, b[0]);
+        }
 #pragma unroll
-        for (int k = 0; k < KG; k += 4) {
-            float a[PM][S::OA::KV], b[PN][S::OB::KV];
-            if constexpr (!A_MN) S::OA::template read<PM>(sa, ty, kg * KG + k, a);
-            if constexpr (!B_MN) S::OB::template read<PN>(sb, tx, kg * KG + k, b);
+        for (int k = 0; k < KG; k += U) {
+            const int cur = AHEAD ? (k / U) & 1 : 0;
+            if constexpr (!AHEAD) {
+                S::OA::template read<PM, U>(sa, ty, k, a[0]);
+                S::OB::template read<PN, U>(sb, tx, k, b[0]);
+            } else if (k + U < KG) {
+                S::OA::template read<PM, U>(sa, ty, k + U, a[cur ^ 1]);
+                S::OB::template read<PN, U>(sb, tx, k + U, b[cur ^ 1]);
+            }
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                if constexpr (A_MN) S::OA::template read<PM>(sa, ty, kg * KG + k + kk, a);
-                if constexpr (B_MN) S::OB::template read<PN>(sb, tx, kg * KG + k + kk, b);
+            for (int kk = 0; kk < U; ++kk) {
+                if constexpr (PAIR_K) {
+                    if (kk % 2 == 0) {
 #pragma unroll
-                for (int i = 0; i < PM; ++i)
+                        for (int j = 0; j < PN; ++j)
 #pragma unroll
-                    for (int j = 0; j < PN; ++j) acc[i][j] = fmaf(a[i][A_MN ? 0 : kk], b[j][B_MN ? 0 : kk], acc[i][j]);
+                            for (int i = 0; i < PM; ++i)
+                                acc2[i][j] = fma2(pack2(a[cur][kk][i], a[cur][kk + 1][i]), pack2(b[cur][kk][j], b[cur][kk + 1][j]), acc2[i][j]);
+                    }
+                } else if constexpr (PAIR_N) {
+                    uint64_t ad[PM];
+#pragma unroll
+                    for (int i = 0; i < PM; ++i) ad[i] = pack2(a[cur][kk][i], a[cur][kk][i]);
+#pragma unroll
+                    for (int j = 0; j < PN / 2; ++j)
+#pragma unroll
+                        for (int i = 0; i < PM; ++i) acc2[i][j] = fma2(ad[i], pack2(b[cur][kk][2 * j], b[cur][kk][2 * j + 1]), acc2[i][j]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < PM; ++i)
+#pragma unroll
+                        for (int j = 0; j < PN; ++j) acc[i][j] = fmaf(a[cur][kk][i], b[cur][kk][j], acc[i][j]);
+                }
             }
         }
-        sa = sa + S::STAGE == smem + STAGES * S::STAGE ? smem : sa + S::STAGE;
+        st_out = st_out == (STAGES - 1) * S::STAGE ? 0 : st_out + S::STAGE;
     }
     cp_wait<0>();
     __syncthreads();                                                // operand stages are free: patches meet here
+#pragma unroll
+    for (int i = 0; i < PM; ++i)
+#pragma unroll
+        for (int j = 0; j < PC; ++j) {
+            if constexpr (PAIR_N) unpack2(acc2[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
+            if constexpr (PAIR_K) {
+                float even, odd;
+                unpack2(acc2[i][j], even, odd);
+                acc[i][j] = even + odd;
+            }
+        }
 
     float* red = smem;
 #pragma unroll
@@ -239,7 +327,7 @@ __global__ void __launch_bounds__(128 * KS) gemm_f32_kernel(const GemmArgs g) {
     const int parts = gridDim.z, rank = blockIdx.z;
     int r_begin = 0, r_end = BM;
     if (parts > 1) {
-        for (int idx = threadIdx.x; idx < BM * BN / 4; idx += GT) {
+        for (int idx = threadIdx.x; idx < BM * BN / 4; idx += S::THREADS) {
             float* q = red + (idx / (BN / 4)) * S::RLD + (idx % (BN / 4)) * 4;
             float4 v = *reinterpret_cast<float4*>(q);
 #pragma unroll
@@ -255,7 +343,7 @@ __global__ void __launch_bounds__(128 * KS) gemm_f32_kernel(const GemmArgs g) {
         r_end = min(BM, r_begin + share);
     }
     chain_next();                                                   // (at the loop or earlier, successors crowd out the side stream)
-    for (int idx = r_begin * (BN / 4) + threadIdx.x; idx < r_end * (BN / 4); idx += GT) {
+    for (int idx = r_begin * (BN / 4) + threadIdx.x; idx < r_end * (BN / 4); idx += S::THREADS) {
         const int row = idx / (BN / 4), col = (idx % (BN / 4)) * 4;
         const int m = m0 + row, n = n0 + col;
         const float* q = red + row * S::RLD + col;
@@ -332,7 +420,7 @@ int cluster_capacity(deers_ctx* ctx) {
     for (int parts = 2; parts <= MAX_PARTS; ++parts) {
         cudaLaunchConfig_t lc{};
         lc.gridDim = dim3(1, 1, parts);
-        lc.blockDim = dim3(S::GT);
+        lc.blockDim = dim3(S::THREADS);
         lc.dynamicSmemBytes = S::SMEM;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -378,7 +466,7 @@ int launch_variant(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g) {
     using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
     const auto kernel = gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>;
     DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>), S::SMEM);
-    DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, dim3(p.tiles_n, p.tiles_m, p.parts), S::GT, S::SMEM, dim3(1, 1, p.parts), g));
+    DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, dim3(p.tiles_n, p.tiles_m, p.parts), S::THREADS, S::SMEM, dim3(1, 1, p.parts), g));
     return DEERS_OK;
 }
 
