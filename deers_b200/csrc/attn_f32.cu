@@ -11,9 +11,13 @@
 // warps meet at a named barrier, and the P / dS tile a product reads was written by the same warp.
 // Within a group thread (ty, tx) of 8 x 8 owns rows 4 ty .. 4 ty + 3 and columns tx, tx + 8, ... of a 32 x BN score tile
 // (4 x 8 or 4 x 4 patches: 12 LDS.128 per 128 FFMA) and rows 4 ty .. with float4 columns 4 tx + 32 j of the
-// accumulators.  Tiles arrive by cp.async: the next K (or Q) is fetched while the current one's scores are turned
+// accumulators.  Products run two to an issue slot where the registers allow (forward, and from 64 wide tiles on backward), and
+// lanes lie so that shared-memory reads cost half: B8 H12 T2048 D64 forward 1909 -> 1659 us, backward 5821 -> 5642; B3 H4 T77 D48
+// forward 10.3 -> 8.8; B4 H6 T256 D32 unchanged (10.6 and 19.8).  Tiles arrive by cp.async: the next K (or Q) is fetched while the current one's scores are turned
 // into the second product, the next V (or dO) while the next scores are computed.
 #include "common.cuh"
+
+#include <type_traits>
 
 namespace {
 
@@ -46,6 +50,31 @@ __device__ __forceinline__ void cp4(float* dst, const float* src, int n) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// Two f32 products in one issue slot (each a plain IEEE fma).
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// Place of a thread in its group's 8 x 8 arrangement.  A quarter warp holds two rows and four columns, neighbouring lanes a
+// column each: a 16-byte shared-memory read along either side then costs 2.1 cycles (4 with lane % 8 along the columns).
+__device__ __forceinline__ int place_y(int t) { return (t / 32) * 4 + (t & 1) + 2 * ((t >> 3) & 1); }
+__device__ __forceinline__ int place_x(int t) { return ((t >> 1) & 3) + 4 * ((t >> 4) & 1); }
 // The two warps of a group meet (barrier 0 is __syncthreads).
 __device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory"); }
 
@@ -77,36 +106,80 @@ __device__ __forceinline__ void fetch_tile(float* __restrict__ dst, const float*
     }
 }
 
-// s[r][c] = sum_d A[4 ty + r][d] * B[tx + 8 c][d]
-template <int DP, int NC>
+// s[r][c] = sum_d A[4 ty + r][d] * B[tx + 8 c][d].  PAIRS: even and odd d side by side, where the registers for twice the
+// sums are there without spilling or losing the second block of an SM (forward from 64 wide tiles, backward from 96).
+template <int DP, int NC, bool PAIRS>
 __device__ __forceinline__ void tile_nt(const float* __restrict__ A, const float* __restrict__ Bm, int ty, int tx, float (&s)[4][NC]) {
     constexpr int LD = DP + 4;
+    if constexpr (PAIRS) {
+        uint64_t s2[4][NC];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) s[r][c] = 0.f;
+            for (int c = 0; c < NC; ++c) s2[r][c] = 0;
 #pragma unroll 2
-    for (int d = 0; d < DP; d += 4) {
-        float4 a[4];
+        for (int d = 0; d < DP; d += 4) {
+            ulonglong2 a[4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(A + (ty * 4 + r) * LD + d);
+            for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const ulonglong2*>(A + (ty * 4 + r) * LD + d);
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            const float4 b = *reinterpret_cast<const float4*>(Bm + (tx + 8 * c) * LD + d);
+            for (int c = 0; c < NC; ++c) {
+                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(Bm + (tx + 8 * c) * LD + d);
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                s[r][c] = fmaf(a[r].x, b.x, s[r][c]);
-                s[r][c] = fmaf(a[r].y, b.y, s[r][c]);
-                s[r][c] = fmaf(a[r].z, b.z, s[r][c]);
-                s[r][c] = fmaf(a[r].w, b.w, s[r][c]);
+                for (int r = 0; r < 4; ++r) s2[r][c] = fma2(a[r].x, b.x, s2[r][c]);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) s2[r][c] = fma2(a[r].y, b.y, s2[r][c]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const float2 v = unpack2(s2[r][c]);
+                s[r][c] = v.x + v.y;
+            }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) s[r][c] = 0.f;
+#pragma unroll 2
+        for (int d = 0; d < DP; d += 4) {
+            float4 a[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(A + (ty * 4 + r) * LD + d);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const float4 b = *reinterpret_cast<const float4*>(Bm + (tx + 8 * c) * LD + d);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    s[r][c] = fmaf(a[r].x, b.x, s[r][c]);
+                    s[r][c] = fmaf(a[r].y, b.y, s[r][c]);
+                    s[r][c] = fmaf(a[r].z, b.z, s[r][c]);
+                    s[r][c] = fmaf(a[r].w, b.w, s[r][c]);
+                }
             }
         }
     }
 }
 
-// acc[r][4 j + e] += sum_k P[4 ty + r][k] * X[k][4 tx + 32 j + e], k < KN (P row stride PLD)
-template <int DP, int KN, int PLD>
-__device__ __forceinline__ void tile_pv(const float* __restrict__ Ps, const float* __restrict__ X, int ty, int tx, float (&acc)[4][DP / 8]) {
+// A row of an accumulator: DP / 8 floats, as pairs or one by one.
+template <int DP, bool PAIRS>
+struct Acc {
+    using T = typename std::conditional<PAIRS, uint64_t, float>::type;
+    T v[PAIRS ? DP / 16 : DP / 8];
+    __device__ __forceinline__ T& operator[](int i) { return v[i]; }
+    __device__ __forceinline__ const T& operator[](int i) const { return v[i]; }
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (auto& x : v) x = 0;
+    }
+};
+
+// acc[r][2 j], acc[r][2 j + 1] (pairs of columns 4 tx + 32 j ..) += sum_k P[4 ty + r][k] * X[k][..], k < KN (P row stride PLD)
+// PAIRS as above: the 32-wide backward has no registers for the doubled P.
+template <int DP, int KN, int PLD, bool PAIRS>
+__device__ __forceinline__ void tile_pv(const float* __restrict__ Ps, const float* __restrict__ X, int ty, int tx, Acc<DP, PAIRS> (&acc)[4]) {
     constexpr int LD = DP + 4;
 #pragma unroll 2
     for (int k = 0; k < KN; k += 4) {
@@ -115,16 +188,27 @@ __device__ __forceinline__ void tile_pv(const float* __restrict__ Ps, const floa
         for (int r = 0; r < 4; ++r) p[r] = *reinterpret_cast<const float4*>(Ps + (ty * 4 + r) * PLD + k);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
+            float pr[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) pr[r] = kk == 0 ? p[r].x : kk == 1 ? p[r].y : kk == 2 ? p[r].z : p[r].w;
 #pragma unroll
             for (int j = 0; j < DP / 32; ++j) {
-                const float4 x = *reinterpret_cast<const float4*>(X + (k + kk) * LD + tx * 4 + 32 * j);
+                const float* q = X + (k + kk) * LD + tx * 4 + 32 * j;
+                if constexpr (PAIRS) {
+                    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(q);
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float pr = kk == 0 ? p[r].x : kk == 1 ? p[r].y : kk == 2 ? p[r].z : p[r].w;
-                    acc[r][4 * j + 0] = fmaf(pr, x.x, acc[r][4 * j + 0]);
-                    acc[r][4 * j + 1] = fmaf(pr, x.y, acc[r][4 * j + 1]);
-                    acc[r][4 * j + 2] = fmaf(pr, x.z, acc[r][4 * j + 2]);
-                    acc[r][4 * j + 3] = fmaf(pr, x.w, acc[r][4 * j + 3]);
+                    for (int r = 0; r < 4; ++r) acc[r][2 * j] = fma2(pack2(pr[r], pr[r]), x.x, acc[r][2 * j]);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) acc[r][2 * j + 1] = fma2(pack2(pr[r], pr[r]), x.y, acc[r][2 * j + 1]);
+                } else {
+                    const float4 x = *reinterpret_cast<const float4*>(q);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        acc[r][4 * j + 0] = fmaf(pr[r], x.x, acc[r][4 * j + 0]);
+                        acc[r][4 * j + 1] = fmaf(pr[r], x.y, acc[r][4 * j + 1]);
+                        acc[r][4 * j + 2] = fmaf(pr[r], x.z, acc[r][4 * j + 2]);
+                        acc[r][4 * j + 3] = fmaf(pr[r], x.w, acc[r][4 * j + 3]);
+                    }
                 }
             }
         }
@@ -134,23 +218,26 @@ __device__ __forceinline__ void tile_pv(const float* __restrict__ Ps, const floa
 // Row reductions over the eight threads that share a row.
 __device__ __forceinline__ float row_max(float x) {
 #pragma unroll
-    for (int o = 4; o >= 1; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+    for (int o = 0; o < 3; ++o) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o == 0 ? 16 : o == 1 ? 4 : 2));    // the bits of place_x
     return x;
 }
 __device__ __forceinline__ float row_sum(float x) {
 #pragma unroll
-    for (int o = 4; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    for (int o = 0; o < 3; ++o) x += __shfl_xor_sync(0xffffffffu, x, o == 0 ? 16 : o == 1 ? 4 : 2);
     return x;
 }
 
-template <int DP>
-__device__ __forceinline__ void put_acc(float* dst, int ty, int tx, const float (&acc)[4][DP / 8]) {
+template <int DP, bool PAIRS>
+__device__ __forceinline__ void put_acc(float* dst, int ty, int tx, const Acc<DP, PAIRS> (&acc)[4]) {
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int j = 0; j < DP / 32; ++j)
-            *reinterpret_cast<float4*>(dst + (ty * 4 + r) * (DP + 4) + tx * 4 + 32 * j) =
-                make_float4(acc[r][4 * j], acc[r][4 * j + 1], acc[r][4 * j + 2], acc[r][4 * j + 3]);
+            if constexpr (PAIRS)
+                *reinterpret_cast<ulonglong2*>(dst + (ty * 4 + r) * (DP + 4) + tx * 4 + 32 * j) = make_ulonglong2(acc[r][2 * j], acc[r][2 * j + 1]);
+            else
+                *reinterpret_cast<float4*>(dst + (ty * 4 + r) * (DP + 4) + tx * 4 + 32 * j) =
+                    make_float4(acc[r][4 * j], acc[r][4 * j + 1], acc[r][4 * j + 2], acc[r][4 * j + 3]);
 }
 
 // One 16-byte piece of an output row, element by element where alignment or D ask for it.
@@ -176,6 +263,7 @@ struct Tile {
     // backward: two stationary tiles | per group: two streamed tiles, half a P / dS tile (32 columns), row statistics
     static constexpr int BWD_PLD = 36;
     static constexpr int BWD_BN = 32;
+    static constexpr bool BWD_PAIRS = DP >= 64;                 // pairs of products in the backward's second products
     static constexpr int BWD_STREAM = BWD_BN * LD;
     static constexpr int BWD_GROUP = 2 * BWD_STREAM + BM * BWD_PLD + 2 * BWD_BN;
     static constexpr size_t BWD_SMEM = (size_t)(2 * ROWS + 2 * BM + NG * BWD_GROUP) * sizeof(float);
@@ -185,13 +273,13 @@ struct Tile {
 // Forward: one block per (batch*head, 32-row query tile); the heaviest (latest) query tiles of all slices first.
 // ---------------------------------------------------------------------------
 template <int DP>
-__global__ void __launch_bounds__(NT) attn_fwd_f32_kernel(const F32Params p) {
+__global__ void __launch_bounds__(NT, DP <= 32 ? 2 : 1) attn_fwd_f32_kernel(const F32Params p) {
     chain_wait();
     using L = Tile<DP>;
     constexpr int BN = L::BN, NC = L::NC, LD = L::LD, PLD = L::FWD_PLD;
     extern __shared__ __align__(16) float smem[];
     const int g = threadIdx.x / 64, t = threadIdx.x % 64;
-    const int ty = (t / 32) * 4 + (t % 32) / 8, tx = t % 8;
+    const int ty = place_y(t), tx = place_x(t);
     float* Qs = smem;
     float* Ks = Qs + L::ROWS + g * L::FWD_GROUP;
     float* Vs = Ks + L::STREAM;
@@ -214,12 +302,12 @@ __global__ void __launch_bounds__(NT) attn_fwd_f32_kernel(const F32Params p) {
     cp_wait<1>();
     __syncthreads();                                            // Q is shared by the groups
 
-    float m[4], l[4], acc[4][DP / 8];
+    float m[4], l[4];
+    Acc<DP, true> acc[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         m[r] = -INFINITY; l[r] = 0.f;
-#pragma unroll
-        for (int c = 0; c < DP / 8; ++c) acc[r][c] = 0.f;
+        acc[r].clear();
     }
     const float sl2 = p.scale * LOG2E;
 
@@ -227,7 +315,7 @@ __global__ void __launch_bounds__(NT) attn_fwd_f32_kernel(const F32Params p) {
         const int k0 = j * BN;
         if (j != g) { cp_wait<1>(); group_sync(g); }            // this K tile has landed for both warps
         float s[4][NC];
-        tile_nt<DP, NC>(Qs, Ks, ty, tx, s);
+        tile_nt<DP, NC, (DP >= 64)>(Qs, Ks, ty, tx, s);
         group_sync(g);                                          // K is consumed: the next one may land
         if (j + NG < ntiles) fetch_tile<DP, BN, 64>(Ks, kb, k0 + NG * BN, p.T, p.D, p.sk.t, p.vec, t);
         cp_commit();
@@ -260,11 +348,11 @@ __global__ void __launch_bounds__(NT) attn_fwd_f32_kernel(const F32Params p) {
             l[r] = l[r] * alpha + row_sum(rs);
             m[r] = m_new;
 #pragma unroll
-            for (int c = 0; c < DP / 8; ++c) acc[r][c] *= alpha;
+            for (int c = 0; c < DP / 16; ++c) acc[r][c] = mul2(acc[r][c], pack2(alpha, alpha));
         }
         cp_wait<1>();
         group_sync(g);                                          // V has landed (and this warp's P rows are visible)
-        tile_pv<DP, BN, PLD>(Ps, Vs, ty, tx, acc);
+        tile_pv<DP, BN, PLD, true>(Ps, Vs, ty, tx, acc);
         group_sync(g);                                          // V is consumed
         if (j + NG < ntiles) fetch_tile<DP, BN, 64>(Vs, vb, k0 + NG * BN, p.T, p.D, p.sv.t, p.vec, t);
         cp_commit();
@@ -273,7 +361,7 @@ __global__ void __launch_bounds__(NT) attn_fwd_f32_kernel(const F32Params p) {
     chain_next();
 
     // The groups meet: O = sum_g 2^(m_g - M) O_g / sum_g 2^(m_g - M) l_g, in group order.
-    put_acc<DP>(Ks, ty, tx, acc);
+    put_acc(Ks, ty, tx, acc);
     if (tx == 0) {
 #pragma unroll
         for (int r = 0; r < 4; ++r) { Ps[ty * 4 + r] = m[r]; Ps[BM + ty * 4 + r] = l[r]; }
@@ -385,7 +473,7 @@ __device__ __forceinline__ void probabilities(const F32Params& p, float (&s)[4][
 
 // acc += tile * X with the 32 x BN tile handed through shared memory 32 columns at a time (rows stay inside a warp).
 template <int DP, int NC>
-__device__ __forceinline__ void staged_product(float* stage, const float (&v)[4][NC], const float* X, int ty, int tx, float (&acc)[4][DP / 8]) {
+__device__ __forceinline__ void staged_product(float* stage, const float (&v)[4][NC], const float* X, int ty, int tx, Acc<DP, Tile<DP>::BWD_PAIRS> (&acc)[4]) {
     constexpr int PLD = Tile<DP>::BWD_PLD;
 #pragma unroll
     for (int half = 0; half < NC / 4; ++half) {
@@ -395,7 +483,7 @@ __device__ __forceinline__ void staged_product(float* stage, const float (&v)[4]
 #pragma unroll
             for (int c = 0; c < 4; ++c) stage[(ty * 4 + r) * PLD + tx + 8 * c] = v[r][half * 4 + c];
         __syncwarp();
-        tile_pv<DP, 32, PLD>(stage, X + half * 32 * (DP + 4), ty, tx, acc);
+        tile_pv<DP, 32, PLD, Tile<DP>::BWD_PAIRS>(stage, X + half * 32 * (DP + 4), ty, tx, acc);
     }
 }
 
@@ -405,7 +493,7 @@ __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt
     using L = Tile<DP>;
     constexpr int BN = L::BWD_BN, NC = BN / 8, LD = L::LD;
     const int g = threadIdx.x / 64, t = threadIdx.x % 64;
-    const int ty = (t / 32) * 4 + (t % 32) / 8, tx = t % 8;
+    const int ty = DP <= 32 ? t / 8 : place_y(t), tx = DP <= 32 ? t % 8 : place_x(t);     // (DP 32: plain, it spills less)
     float* Ks = smem;
     float* Vs = Ks + L::ROWS;
     float* grp0 = smem + 2 * L::ROWS + 2 * BM;
@@ -432,11 +520,9 @@ __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt
     cp_wait<0>();
     __syncthreads();                                            // K and V are shared by the groups
 
-    float dk[4][DP / 8], dv[4][DP / 8];
+    Acc<DP, L::BWD_PAIRS> dk[4], dv[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < DP / 8; ++c) { dk[r][c] = 0.f; dv[r][c] = 0.f; }
+    for (int r = 0; r < 4; ++r) { dk[r].clear(); dv[r].clear(); }
 
     RowDelta<DP, 2> rd;                                         // two threads per row of the 32-row tile
     float lse_next = 0.f;
@@ -451,13 +537,13 @@ __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt
         const int q0 = i * BN;
         if (i != i0) { cp_wait<1>(); group_sync(g); }           // this Q tile has landed for both warps
         float pp[4][NC], ds[4][NC];
-        tile_nt<DP, NC>(Ks, Qs, ty, tx, pp);                    // S^T
+        tile_nt<DP, NC, (DP >= 96)>(Ks, Qs, ty, tx, pp);                    // S^T
         if (i != i0) { cp_wait<0>(); group_sync(g); }           // and so has dO
         {
             const float d = rd.dot(p, ob, Gs + (t / 2) * LD, q0 + t / 2, t % 2);
             if (t % 2 == 0) { l2[t / 2] = lse_next; dl[t / 2] = d; }
         }
-        tile_nt<DP, NC>(Vs, Gs, ty, tx, ds);                    // dP^T
+        tile_nt<DP, NC, (DP >= 96)>(Vs, Gs, ty, tx, ds);                    // dP^T
         group_sync(g);                                          // statistics are visible
         probabilities<NC, false>(p, pp, l2, k0, q0, ty, tx);
 #pragma unroll
@@ -476,8 +562,8 @@ __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt
     }
     cp_wait<0>();
     chain_next();
-    put_acc<DP>(Qs, ty, tx, dk);
-    put_acc<DP>(Gs, ty, tx, dv);
+    put_acc(Qs, ty, tx, dk);
+    put_acc(Gs, ty, tx, dv);
     __syncthreads();
     merge_store<DP>(p, grp0, L::BWD_GROUP, p.dk + b * p.sdk.b + h * p.sdk.h, p.sdk.t, k0);
     merge_store<DP>(p, grp0 + L::BWD_STREAM, L::BWD_GROUP, p.dv + b * p.sdv.b + h * p.sdv.h, p.sdv.t, k0);
@@ -489,7 +575,7 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
     using L = Tile<DP>;
     constexpr int BN = L::BWD_BN, NC = BN / 8, LD = L::LD;
     const int g = threadIdx.x / 64, t = threadIdx.x % 64;
-    const int ty = (t / 32) * 4 + (t % 32) / 8, tx = t % 8;
+    const int ty = DP <= 32 ? t / 8 : place_y(t), tx = DP <= 32 ? t % 8 : place_x(t);     // (DP 32: plain, it spills less)
     float* Qs = smem;
     float* Gs = Qs + L::ROWS;
     float* l2 = smem + 2 * L::ROWS;
@@ -522,13 +608,11 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
         if (threadIdx.x % 8 == 0) { l2[r] = row < p.T ? p.lse[(long long)bh * p.T + row] * LOG2E : 0.f; dl[r] = d; }
     }
 
-    float dq[4][DP / 8];
+    Acc<DP, L::BWD_PAIRS> dq[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < DP / 8; ++c) dq[r][c] = 0.f;
+    for (int r = 0; r < 4; ++r) dq[r].clear();
     float pp[4][NC], ds[4][NC];
-    if (g < ntiles) tile_nt<DP, NC>(Qs, Ks, ty, tx, pp);        // the first S while the statistics are made
+    if (g < ntiles) tile_nt<DP, NC, (DP >= 96)>(Qs, Ks, ty, tx, pp);        // the first S while the statistics are made
     __syncthreads();
 
     for (int j = g; j < ntiles; j += NG) {
@@ -536,9 +620,9 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
         if (j != g) {
             cp_wait<0>();
             group_sync(g);
-            tile_nt<DP, NC>(Qs, Ks, ty, tx, pp);
+            tile_nt<DP, NC, (DP >= 96)>(Qs, Ks, ty, tx, pp);
         }
-        tile_nt<DP, NC>(Gs, Vs, ty, tx, ds);                    // dP
+        tile_nt<DP, NC, (DP >= 96)>(Gs, Vs, ty, tx, ds);                    // dP
         group_sync(g);                                          // V is consumed
         if (j + NG < ntiles) fetch_tile<DP, BN, 64>(Vs, vb, k0 + NG * BN, p.T, p.D, p.sv.t, p.vec, t);
         cp_commit();
@@ -556,7 +640,7 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
     }
     cp_wait<0>();
     chain_next();
-    put_acc<DP>(Ks, ty, tx, dq);
+    put_acc(Ks, ty, tx, dq);
     __syncthreads();
     merge_store<DP>(p, grp0, L::BWD_GROUP, p.dq + b * p.sdq.b + h * p.sdq.h, p.sdq.t, q0);
 }
