@@ -39,6 +39,7 @@ struct F32Params {
     int vec;            // 1: every row start of the inputs is 16-byte aligned and D % 4 == 0
     int vec_out;        // the same for the outputs
     float scale;
+    const float* cosv; const float* sinv;   // backward: dQ and dK leave rotated back by their position ([T][D / 2]; nullptr: not)
 };
 
 __device__ __forceinline__ void cp16(float* dst, const float* src, int n) {
@@ -438,8 +439,35 @@ struct RowDelta {
 
 // Adds the groups' partial gradients (each parked in its first streamed tile) and stores the block's rows.
 template <int DP>
-__device__ __forceinline__ void merge_store(const F32Params& p, const float* parts, int stride, float* dst, long long st, int row0) {
+__device__ __forceinline__ void merge_store(const F32Params& p, const float* parts, int stride, float* dst, long long st, int row0, bool rotate) {
     constexpr int C4 = DP / 4;
+    if (rotate) {                                               // D % 8 == 0: a thread takes four columns of both halves
+        const int half = p.D / 2, h4 = half / 4;
+        for (int idx = threadIdx.x; idx < BM * h4; idx += NT) {
+            const int r = idx / h4, c = (idx % h4) * 4, row = row0 + r;
+            if (row >= p.T) continue;
+            float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int z = 0; z < NG; ++z) {
+                const float* q = parts + z * stride + r * (DP + 4) + c;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { a[e] += q[e]; b[e] += q[half + e]; }
+            }
+            const long long at = (long long)row * half + c;
+            const float4 c4 = *reinterpret_cast<const float4*>(p.cosv + at), s4 = *reinterpret_cast<const float4*>(p.sinv + at);
+            const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {-s4.x, -s4.y, -s4.z, -s4.w};
+            float o1[4], o2[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {                       // rounded as the rotary pack does
+                o1[e] = __fadd_rn(__fmul_rn(a[e], cs[e]), __fmul_rn(b[e], sn[e]));
+                o2[e] = __fadd_rn(__fmul_rn(a[e], -sn[e]), __fmul_rn(b[e], cs[e]));
+            }
+            float* o = dst + (long long)row * st + c;
+            store4(o, make_float4(o1[0], o1[1], o1[2], o1[3]), 4, p.vec_out);
+            store4(o + half, make_float4(o2[0], o2[1], o2[2], o2[3]), 4, p.vec_out);
+        }
+        return;
+    }
     for (int idx = threadIdx.x; idx < BM * C4; idx += NT) {
         const int r = idx / C4, c = (idx % C4) * 4, row = row0 + r;
         if (row >= p.T || c >= p.D) continue;
@@ -565,8 +593,8 @@ __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt
     put_acc(Qs, ty, tx, dk);
     put_acc(Gs, ty, tx, dv);
     __syncthreads();
-    merge_store<DP>(p, grp0, L::BWD_GROUP, p.dk + b * p.sdk.b + h * p.sdk.h, p.sdk.t, k0);
-    merge_store<DP>(p, grp0 + L::BWD_STREAM, L::BWD_GROUP, p.dv + b * p.sdv.b + h * p.sdv.h, p.sdv.t, k0);
+    merge_store<DP>(p, grp0, L::BWD_GROUP, p.dk + b * p.sdk.b + h * p.sdk.h, p.sdk.t, k0, p.cosv != nullptr);
+    merge_store<DP>(p, grp0 + L::BWD_STREAM, L::BWD_GROUP, p.dv + b * p.sdv.b + h * p.sdv.h, p.sdv.t, k0, false);
 }
 
 // dQ of 32 query rows: the groups walk the key tiles at or left of the diagonal.
@@ -642,7 +670,7 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
     chain_next();
     put_acc(Ks, ty, tx, dq);
     __syncthreads();
-    merge_store<DP>(p, grp0, L::BWD_GROUP, p.dq + b * p.sdq.b + h * p.sdq.h, p.sdq.t, q0);
+    merge_store<DP>(p, grp0, L::BWD_GROUP, p.dq + b * p.sdq.b + h * p.sdq.h, p.sdq.t, q0, p.cosv != nullptr);
 }
 
 // Both roles in one launch: row n of the grid holds every slice's n-th heaviest key tile, then every slice's n-th heaviest query
@@ -716,8 +744,9 @@ int launch_attn_fwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q
 
 int launch_attn_bwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q, const float* k,
                         const float* v, const float* o, const float* lse, const float* d_o, float* dq,
-                        float* dk, float* dv) {
+                        float* dk, float* dv, const float* cosv, const float* sinv) {
     F32Params p = base_params(d);
+    p.cosv = cosv; p.sinv = sinv;
     p.q = q; p.k = k; p.v = v; p.o = o; p.lse = lse; p.d_o = d_o;
     p.dq = dq; p.dk = dk; p.dv = dv;
     p.vec = (d->D % 4 == 0) && rows_vec_ok(q, d->q_strides) && rows_vec_ok(k, d->k_strides) &&

@@ -193,7 +193,7 @@ int launch_attn_fwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q
                         const float* v, float* o, float* lse);
 int launch_attn_bwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q, const float* k,
                         const float* v, const float* o, const float* lse, const float* d_o, float* dq,
-                        float* dk, float* dv);
+                        float* dk, float* dv, const float* cosv = nullptr, const float* sinv = nullptr);
 
 // f16 tcgen05 path (attn_fwd_f16_sm100.cu, attn_bwd_f16_sm100.cu)
 int launch_attn_fwd_f16(deers_ctx* ctx, const deers_attn_desc* d, const void* q, const void* k,
@@ -208,10 +208,27 @@ int run_selftest_wait(deers_ctx* ctx, unsigned int limit_ms, int* result_host);
 // f32 GEMM (gemm_f32.cu)
 int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long long lda, int a_mn, const float* b,
                     long long ldb, int b_mn, float* c, long long ldc, int epi, const float* r, long long ldr, float* aux);
+// The same with the rows of A normalised on the way, C [M,N] = rmsnorm(A [M,K]) * B [K,N], all dense: what a block's pre-norms
+// feed (launch_gemm_f32_norm).  inv (may be nullptr) receives the inverse norms.  Columns [0, rope_cols), heads of rope_d columns,
+// are rotated by position m % rope_t with the tables cosv, sinv [rope_t][rope_d / 2] (0 columns: none); the head width has to
+// pass gemm_f32_can_rotate().
+struct GemmNorm {
+    float eps;
+    float* inv;
+    const float* cosv; const float* sinv;
+    int rope_cols, rope_d, rope_t;
+};
+int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, const float* b, float* c, int epi, float* aux, const GemmNorm& f);
+bool gemm_f32_can_rotate(int head_dim);
+// Products C_i [M_i,N_i] = A_i^T B_i with A_i [K,M_i], B_i [K,N_i], dense, in one launch.
+constexpr int GEMM_GROUP_MAX = 4;
+struct GemmTN { int M, N; const float* a; const float* b; float* c; };
+int launch_gemm_f32_group(deers_ctx* ctx, int n, const GemmTN* t, int K);
 // RMSNorm (rmsnorm.cu)
 int launch_rmsnorm_fwd(deers_ctx* ctx, long long rows, int C, double eps, const float* x, float* y, float* inv_norm);
 int launch_rmsnorm_bwd(deers_ctx* ctx, long long rows, int C, const float* x, const float* inv_norm, const float* dy,
-                       const float* add, float* dx);
+                       const float* add, float* dx, float* n_out = nullptr);
+int launch_rmsnorm_split(deers_ctx* ctx, long long rows, int C, double eps, const float* x, float* inv_norm, void* hi, void* lo);
 // embedding and cross-entropy (gpt_ops.cu)
 int launch_embedding_fwd(deers_ctx* ctx, const float* weight, const long long* ids, long long n_ids, int C, long long V,
                          float* out);

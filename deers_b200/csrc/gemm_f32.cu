@@ -50,6 +50,12 @@ struct GemmArgs {
     int a_vec, b_vec, c_vec; // 16-byte accesses allowed
     int epi;
     int k_chunk;             // K elements per part (multiple of BK)
+    // FUSED kernels only: A is a residual stream, its rows are normalised on the way (C = rmsnorm(A) * B), and the columns
+    // [0, rope_cols) of C, heads of rope_d columns, are rotated by the row's position (m % rope_t)
+    float eps, inv_n;        // inverse norm of a row: 1 / sqrt(sum(a * a) * inv_n + eps)
+    float* inv;              // written [M] (nullptr: not wanted)
+    const float* cosv; const float* sinv;
+    int rope_cols, rope_d, rope_t;
 };
 
 __device__ __forceinline__ float4 ld4(const float* p, int valid, bool vec) {
@@ -184,31 +190,66 @@ struct GemmShape {
     static constexpr int RLD = BN + 4;                              // row stride of the patch staging tile
     static constexpr int RED = KS * BM * RLD;
     static constexpr int STAGES = BM * BN > 64 * 64 ? 3 : 4;
-    static constexpr size_t NEED = (size_t)(STAGES * STAGE > RED ? STAGES * STAGE : RED) * sizeof(float);
+    static constexpr int SQ_AT = STAGES * STAGE > RED ? STAGES * STAGE : RED;    // row sums of squares of the FUSED kernels
+    static constexpr size_t NEED = (size_t)(SQ_AT + KS * BM) * sizeof(float);
     // A large block has an SM to itself: two of them share its issue slots while others idle (chained launches place the
     // next product's blocks before this one's have left).
     static constexpr size_t ALONE = 116 * 1024;
     static constexpr size_t SMEM = PM * PN >= 16 && NEED < ALONE ? ALONE : NEED;
 };
 
-template <int PM, int PN, int KS, bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
-    chain_wait();
+// Sum of a tile element's partial sums: the k groups of this block, or the blocks of the cluster.
+template <int KS, int PATCH>
+__device__ __forceinline__ float4 patch_sum(const float* q, int parts) {
+    if (parts > 1) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int z = 0; z < parts; ++z) {
+            const float4 u = *reinterpret_cast<const float4*>(cg::this_cluster().map_shared_rank(q, z));
+            v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+        }
+        return v;
+    }
+    float4 v = *reinterpret_cast<const float4*>(q);
+#pragma unroll
+    for (int z = 1; z < KS; ++z) {
+        const float4 u = *reinterpret_cast<const float4*>(q + z * PATCH);
+        v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+    }
+    return v;
+}
+
+// One tile (tile_m, tile_n) of a product and one part of its K.  setup() only computes addresses and may run before the
+// predecessor has finished; run() does the work.
+template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED>
+struct TileProduct {
     using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
-    constexpr int BM = S::BM, BN = S::BN, STAGES = S::STAGES, KG = S::KG;
+    static constexpr int BM = S::BM, BN = S::BN, STAGES = S::STAGES, KG = S::KG;
+    typename S::OA la;
+    typename S::OB lb;
+    int m0, n0, kbeg, kend;
+    __device__ __forceinline__ void setup(const GemmArgs& g, int tile_m, int tile_n, int part) {
+        const int tid = threadIdx.x % GT, kg = threadIdx.x / GT;
+        m0 = tile_m * BM; n0 = tile_n * BN;
+        kbeg = part * g.k_chunk;
+        kend = min(g.K, kbeg + g.k_chunk);
+        la.init(g.a, g.lda, m0, g.M, kbeg + kg * KG, tid);
+        lb.init(g.b, g.ldb, n0, g.N, kbeg + kg * KG, tid);
+    }
+    __device__ __forceinline__ void run(const GemmArgs& g, int parts, int rank);
+};
+
+template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED>
+__device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED>::run(const GemmArgs& g, const int parts, const int rank) {
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x % GT, kg = threadIdx.x / GT;        // position in the tile, k group
     const int w = tid / 32, lane = tid % 32;
     const int ty = (w & 1) * 4 + (lane & 1) + 2 * ((lane >> 3) & 1), tx = (w >> 1) * 8 + ((lane >> 1) & 3) + 4 * (lane >> 4);
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int kbeg = blockIdx.z * g.k_chunk;
-    const int kend = min(g.K, kbeg + g.k_chunk);
     const int nk = kend > kbeg ? (kend - kbeg + BK - 1) / BK : 0;
+    // FUSED: SQ_LANES threads of a group share a row's squares of the group's k, SQ_K each
+    constexpr int SQ_LANES = GT / BM, SQ_K = KG / SQ_LANES;
+    float sq = 0.f;
+    float* const sq_s = smem + S::SQ_AT;                            // [KS][BM]
 
-    typename S::OA la;
-    typename S::OB lb;
-    la.init(g.a, g.lda, m0, g.M, kbeg + kg * KG, tid);
-    lb.init(g.b, g.ldb, n0, g.N, kbeg + kg * KG, tid);
     int kv = kend - kbeg - kg * KG;                                 // k left to fetch (of the group's share and what follows)
     float* const ring = smem + kg * (S::OA::FLOATS + S::OB::FLOATS);
     int st_in = 0, left = nk;                                       // stage to fill next
@@ -248,6 +289,14 @@ __global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
         fetch();
         const float* sa = ring + st_out;
         const float* sb = sa + S::OA::FLOATS;
+        if constexpr (FUSED) {
+            const float* q = sa + (tid / SQ_LANES) * S::OA::LD + (tid % SQ_LANES) * SQ_K;
+#pragma unroll
+            for (int e = 0; e < SQ_K; e += 4) {
+                const float4 x = *reinterpret_cast<const float4*>(q + e);
+                sq = fmaf(x.x, x.x, sq); sq = fmaf(x.y, x.y, sq); sq = fmaf(x.z, x.z, sq); sq = fmaf(x.w, x.w, sq);
+            }
+        }
         float a[AHEAD ? 2 : 1][U][PM], b[AHEAD ? 2 : 1][U][PN];     // fragments of U k (and of the next U)
         if constexpr (AHEAD) {
             S::OA::template read<PM, U>(sa, ty, 0, a[0]);
@@ -305,6 +354,11 @@ __global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
             }
         }
 
+    if constexpr (FUSED) {
+#pragma unroll
+        for (int o = 1; o < SQ_LANES; o *= 2) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if (tid % SQ_LANES == 0) sq_s[kg * BM + tid / SQ_LANES] = sq;
+    }
     float* red = smem;
 #pragma unroll
     for (int i = 0; i < PM; ++i) {
@@ -324,7 +378,6 @@ __global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
     __syncthreads();
 
     // Rows of the tile this block finishes: all of them, or its share of the cluster's.
-    const int parts = gridDim.z, rank = blockIdx.z;
     int r_begin = 0, r_end = BM;
     if (parts > 1) {
         for (int idx = threadIdx.x; idx < BM * BN / 4; idx += S::THREADS) {
@@ -337,6 +390,14 @@ __global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
             }
             *reinterpret_cast<float4*>(q) = v;
         }
+        if constexpr (FUSED) {
+            if (threadIdx.x < BM) {
+                float v = sq_s[threadIdx.x];
+#pragma unroll
+                for (int z = 1; z < KS; ++z) v += sq_s[z * BM + threadIdx.x];
+                sq_s[threadIdx.x] = v;
+            }
+        }
         cg::this_cluster().sync();
         const int share = (BM + parts - 1) / parts;
         r_begin = rank * share;
@@ -347,25 +408,36 @@ __global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
         const int row = idx / (BN / 4), col = (idx % (BN / 4)) * 4;
         const int m = m0 + row, n = n0 + col;
         const float* q = red + row * S::RLD + col;
-        float4 v;
-        if (parts > 1) {
-            v = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int z = 0; z < parts; ++z) {
-                const float4 u = *reinterpret_cast<const float4*>(cg::this_cluster().map_shared_rank(q, z));
-                v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
-            }
-        } else {
-            v = *reinterpret_cast<const float4*>(q);
-#pragma unroll
-            for (int z = 1; z < KS; ++z) {
-                const float4 u = *reinterpret_cast<const float4*>(q + z * BM * S::RLD);
-                v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
-            }
-        }
+        const float4 v = patch_sum<KS, BM * S::RLD>(q, parts);
         if (m >= g.M || n >= g.N) continue;
         const int valid = g.N - n;
         float o[4] = {v.x, v.y, v.z, v.w}, x[4] = {0.f, 0.f, 0.f, 0.f};
         float* cp = g.c + (long long)m * g.ldc + n;
+        if constexpr (FUSED) {
+            float t = 0.f;
+            if (parts > 1) {
+                for (int z = 0; z < parts; ++z) t += *cg::this_cluster().map_shared_rank(sq_s + row, z);
+            } else {
+#pragma unroll
+                for (int z = 0; z < KS; ++z) t += sq_s[z * BM + row];
+            }
+            const float inv = 1.0f / sqrtf(t * g.inv_n + g.eps);
+            if (g.inv && n == 0) g.inv[m] = inv;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] *= inv;
+            if (n < g.rope_cols) {
+                // the other half of the head lies in this tile (tiles hold whole heads); rounded as the rotary pack does
+                const int half = g.rope_d / 2, hc = n % g.rope_d;
+                const bool second = hc >= half;
+                const float4 u = patch_sum<KS, BM * S::RLD>(second ? q - half : q + half, parts);
+                const long long at = (long long)(m % g.rope_t) * half + (second ? hc - half : hc);
+                const float4 c4 = *reinterpret_cast<const float4*>(g.cosv + at), s4 = *reinterpret_cast<const float4*>(g.sinv + at);
+                const float p[4] = {u.x * inv, u.y * inv, u.z * inv, u.w * inv}, cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    o[e] = second ? __fadd_rn(__fmul_rn(p[e], -sn[e]), __fmul_rn(o[e], cs[e])) : __fadd_rn(__fmul_rn(o[e], cs[e]), __fmul_rn(p[e], sn[e]));
+            }
+        }
         if (g.epi == DEERS_EPI_ADD) {
             const float4 t = ld4(g.r + (long long)m * g.ldr + n, valid, g.c_vec);
             o[0] = t.x + o[0]; o[1] = t.y + o[1]; o[2] = t.z + o[2]; o[3] = t.w + o[3];
@@ -380,21 +452,55 @@ __global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
         }
         if (g.c_vec && valid >= 4) {
             *reinterpret_cast<float4*>(cp) = make_float4(o[0], o[1], o[2], o[3]);
-            if (g.epi == DEERS_EPI_RELU_SQ)
+            if (g.epi == DEERS_EPI_RELU_SQ && g.aux)
                 *reinterpret_cast<float4*>(g.aux + (long long)m * g.ldc + n) = make_float4(x[0], x[1], x[2], x[3]);
         } else {
             for (int e = 0; e < 4 && e < valid; ++e) {
                 cp[e] = o[e];
-                if (g.epi == DEERS_EPI_RELU_SQ) g.aux[(long long)m * g.ldc + n + e] = x[e];
+                if (g.epi == DEERS_EPI_RELU_SQ && g.aux) g.aux[(long long)m * g.ldc + n + e] = x[e];
             }
         }
     }
     if (parts > 1) cg::this_cluster().sync();                       // nobody leaves while a peer still reads its patch
 }
 
+template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED>
+__global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
+    TileProduct<PM, PN, KS, A_MN, B_MN, FUSED> tile;
+    tile.setup(g, blockIdx.y, blockIdx.x, blockIdx.z);
+    chain_wait();
+    tile.run(g, gridDim.z, blockIdx.z);
+}
+
+// Several products of one shape of operands (both in MN order) and one K in a launch: the weight gradients of a block, whose
+// tiles do not fill the chip one product at a time.  blockIdx.x counts the tiles of all of them.
+struct GemmGroup {
+    GemmArgs g[GEMM_GROUP_MAX];
+    int first[GEMM_GROUP_MAX];       // first tile of a product
+    int tiles_n[GEMM_GROUP_MAX];
+    int n;
+    __device__ __forceinline__ int pick(int tile) const {
+        int i = 0;
+        while (i + 1 < n && tile >= first[i + 1]) ++i;
+        return i;
+    }
+    __device__ __forceinline__ int tile_m(int i, int tile) const { return (tile - first[i]) / tiles_n[i]; }
+    __device__ __forceinline__ int tile_n(int i, int tile) const { return (tile - first[i]) % tiles_n[i]; }
+    __device__ __forceinline__ const GemmArgs& args(int i) const { return g[i]; }
+};
+
+template <int PM, int PN, int KS>
+__global__ void __launch_bounds__(GT * KS) gemm_f32_group_kernel(const __grid_constant__ GemmGroup gg) {
+    const int i = gg.pick(blockIdx.x);
+    TileProduct<PM, PN, KS, true, true, false> tile;
+    tile.setup(gg.args(i), gg.tile_m(i, blockIdx.x), gg.tile_n(i, blockIdx.x), blockIdx.z);
+    chain_wait();
+    tile.run(gg.args(i), gridDim.z, blockIdx.z);
+}
+
 struct GemmPlan {
     int cfg;        // index into kVariants
-    int tiles_m, tiles_n, parts, k_chunk;
+    int parts, k_chunk;
 };
 
 // Tile variants with what was measured of them (cycles at 1.965 GHz, from products of several K in a graph): a
@@ -415,8 +521,8 @@ int cluster_capacity(deers_ctx* ctx) {
         return DEERS_OK;
     }
     using S = GemmShape<8, 4, 4, false, true>;
-    const auto kernel = gemm_f32_kernel<8, 4, 4, false, true>;
-    DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<8, 4, 4, false, true>), S::SMEM);
+    const auto kernel = gemm_f32_kernel<8, 4, 4, false, true, false>;
+    DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<8, 4, 4, false, true, false>), S::SMEM);
     for (int parts = 2; parts <= MAX_PARTS; ++parts) {
         cudaLaunchConfig_t lc{};
         lc.gridDim = dim3(1, 1, parts);
@@ -438,22 +544,26 @@ int cluster_capacity(deers_ctx* ctx) {
 
 // Picks the variant and the K split with the least estimated time: the blocks an SM has to run one after another times
 // a block's walk over its K, plus what a block spends before and after it (and at the cluster's meeting).
-GemmPlan plan_gemm(int M, int N, int K, const int* capacity) {
+// n products of one K; whole_heads: tiles must hold whole heads of that many columns (0: any).  cfg < 0: no variant does.
+GemmPlan plan_gemm(int n, const int* M, const int* N, int K, const int* capacity, int whole_heads) {
     GemmPlan best{};
+    best.cfg = -1;
     double best_cost = -1.0;
     const int steps = (K + BK - 1) / BK;
     for (int c = 0; c < 6; ++c) {
         const Variant& v = kVariants[c];
-        const long long tm = (M + v.bm - 1) / v.bm, tn = (N + v.bn - 1) / v.bn;
+        if (whole_heads && v.bn % whole_heads) continue;
+        long long tiles = 0;
+        for (int i = 0; i < n; ++i) tiles += (long long)((M[i] + v.bm - 1) / v.bm) * ((N[i] + v.bn - 1) / v.bn);
         for (int parts = 1; parts <= MAX_PARTS; ++parts) {
             const int chunk = (steps + parts - 1) / parts;
             if (parts > 1 && (chunk < 2 || (long long)chunk * (parts - 1) >= steps)) continue;      // no empty part
             if (capacity[parts] < 1) continue;
-            const double waves = (double)((tm * tn + capacity[parts] - 1) / capacity[parts]);
+            const double waves = (double)((tiles + capacity[parts] - 1) / capacity[parts]);
             const double cost = waves * chunk * v.walk + v.around + 1200.0 * (waves - 1.0) + (parts > 1 ? 3300.0 : 0.0);
             if (best_cost < 0.0 || cost < best_cost) {
                 best_cost = cost;
-                best.cfg = c; best.tiles_m = (int)tm; best.tiles_n = (int)tn; best.parts = parts; best.k_chunk = chunk * BK;
+                best.cfg = c; best.parts = parts; best.k_chunk = chunk * BK;
             }
         }
     }
@@ -461,19 +571,66 @@ GemmPlan plan_gemm(int M, int N, int K, const int* capacity) {
     return best;
 }
 
-template <int PM, int PN, int KS, bool A_MN, bool B_MN>
+template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED = false>
 int launch_variant(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g) {
     using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
-    const auto kernel = gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>;
-    DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<PM, PN, KS, A_MN, B_MN>), S::SMEM);
-    DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, dim3(p.tiles_n, p.tiles_m, p.parts), S::THREADS, S::SMEM, dim3(1, 1, p.parts), g));
+    const auto kernel = gemm_f32_kernel<PM, PN, KS, A_MN, B_MN, FUSED>;
+    DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<PM, PN, KS, A_MN, B_MN, FUSED>), S::SMEM);
+    const dim3 grid((g.N + S::BN - 1) / S::BN, (g.M + S::BM - 1) / S::BM, p.parts);
+    DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, grid, S::THREADS, S::SMEM, dim3(1, 1, p.parts), g));
     return DEERS_OK;
 }
 
 template <int PM, int PN, int KS>
-int launch_orders(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g, int a_mn, int b_mn) {
+int launch_orders(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g, int a_mn, int b_mn, bool fused) {
+    if (fused) return launch_variant<PM, PN, KS, false, true, true>(ctx, p, g);
     if (a_mn) return b_mn ? launch_variant<PM, PN, KS, true, true>(ctx, p, g) : launch_variant<PM, PN, KS, true, false>(ctx, p, g);
     return b_mn ? launch_variant<PM, PN, KS, false, true>(ctx, p, g) : launch_variant<PM, PN, KS, false, false>(ctx, p, g);
+}
+
+template <int PM, int PN, int KS>
+int launch_group(deers_ctx* ctx, const GemmPlan& p, GemmGroup& gg) {
+    using S = GemmShape<PM, PN, KS, true, true>;
+    const auto kernel = gemm_f32_group_kernel<PM, PN, KS>;
+    DEERS_SMEM_ONCE(ctx, (gemm_f32_group_kernel<PM, PN, KS>), S::SMEM);
+    int tiles = 0;
+    for (int i = 0; i < gg.n; ++i) {
+        gg.first[i] = tiles;
+        gg.tiles_n[i] = (gg.g[i].N + S::BN - 1) / S::BN;
+        tiles += gg.tiles_n[i] * ((gg.g[i].M + S::BM - 1) / S::BM);
+        gg.g[i].k_chunk = p.k_chunk;
+    }
+    DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, dim3(tiles, 1, p.parts), S::THREADS, S::SMEM, dim3(1, 1, p.parts), gg));
+    return DEERS_OK;
+}
+
+GemmArgs gemm_args(int M, int N, int K, const float* a, long long lda, const float* b, long long ldb, float* c, long long ldc, int epi,
+                   const float* r, long long ldr, float* aux) {
+    GemmArgs g{};
+    g.a = a; g.b = b; g.c = c; g.r = r; g.aux = aux;
+    g.lda = lda; g.ldb = ldb; g.ldc = ldc; g.ldr = ldr;
+    g.M = M; g.N = N; g.K = K; g.epi = epi;
+    g.a_vec = ((uintptr_t)a & 15u) == 0 && lda % 4 == 0;
+    g.b_vec = ((uintptr_t)b & 15u) == 0 && ldb % 4 == 0;
+    g.c_vec = ((uintptr_t)c & 15u) == 0 && ldc % 4 == 0 && (!r || (((uintptr_t)r & 15u) == 0 && ldr % 4 == 0)) &&
+              (!aux || ((uintptr_t)aux & 15u) == 0);
+    return g;
+}
+
+int launch_planned(deers_ctx* ctx, const GemmPlan& p, GemmArgs& g, int a_mn, int b_mn, bool fused) {
+    g.k_chunk = p.k_chunk;
+    int rc;
+    {
+        KernelTimerScope ts(ctx, DEERS_K_GEMM);
+        if (p.cfg == 0) rc = launch_orders<8, 8, 2>(ctx, p, g, a_mn, b_mn, fused);
+        else if (p.cfg == 1) rc = launch_orders<8, 4, 4>(ctx, p, g, a_mn, b_mn, fused);
+        else if (p.cfg == 2) rc = launch_orders<4, 4, 4>(ctx, p, g, a_mn, b_mn, fused);
+        else if (p.cfg == 3) rc = launch_orders<4, 2, 4>(ctx, p, g, a_mn, b_mn, fused);
+        else if (p.cfg == 4) rc = launch_orders<8, 6, 4>(ctx, p, g, a_mn, b_mn, fused);
+        else rc = launch_orders<4, 6, 4>(ctx, p, g, a_mn, b_mn, fused);
+    }
+    ctx->launches += 1;
+    return rc;
 }
 
 }  // namespace
@@ -491,29 +648,59 @@ int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long lo
         if (r) r += MOST * ldr;
         if (aux) aux += MOST * ldc;
     }
-    int rc = cluster_capacity(ctx);
+    const int rc = cluster_capacity(ctx);
     if (rc) return rc;
-    GemmPlan p = plan_gemm(M, N, K, ctx->cluster_capacity);
-    GemmArgs g{};
-    g.a = a; g.b = b; g.c = c; g.r = r; g.aux = aux;
-    g.lda = lda; g.ldb = ldb; g.ldc = ldc; g.ldr = ldr;
-    g.M = M; g.N = N; g.K = K; g.epi = epi;
-    g.a_vec = ((uintptr_t)a & 15u) == 0 && lda % 4 == 0;
-    g.b_vec = ((uintptr_t)b & 15u) == 0 && ldb % 4 == 0;
-    g.c_vec = ((uintptr_t)c & 15u) == 0 && ldc % 4 == 0 && (!r || (((uintptr_t)r & 15u) == 0 && ldr % 4 == 0)) &&
-              (!aux || ((uintptr_t)aux & 15u) == 0);
-    g.k_chunk = p.k_chunk;
+    const GemmPlan p = plan_gemm(1, &M, &N, K, ctx->cluster_capacity, 0);
+    GemmArgs g = gemm_args(M, N, K, a, lda, b, ldb, c, ldc, epi, r, ldr, aux);
+    return launch_planned(ctx, p, g, a_mn, b_mn, false);
+}
+
+// C = rmsnorm(A) * B with an optional rotation of the leading columns (see GemmNorm in common.cuh); M <= 65535 rows.
+int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, const float* b, float* c, int epi, float* aux, const GemmNorm& f) {
+    if (M == 0 || N == 0) return DEERS_OK;
+    const int rc = cluster_capacity(ctx);
+    if (rc) return rc;
+    const GemmPlan p = plan_gemm(1, &M, &N, K, ctx->cluster_capacity, f.rope_cols ? f.rope_d : 0);
+    if (p.cfg < 0) return DEERS_ERR_UNSUPPORTED;
+    GemmArgs g = gemm_args(M, N, K, a, K, b, N, c, N, epi, nullptr, 0, aux);
+    g.eps = f.eps; g.inv_n = (float)(1.0 / (double)K); g.inv = f.inv;
+    g.cosv = f.cosv; g.sinv = f.sinv; g.rope_cols = f.rope_cols; g.rope_d = f.rope_d; g.rope_t = f.rope_t;
+    return launch_planned(ctx, p, g, 0, 1, true);
+}
+
+// Heads that a tile holds whole, with halves of whole 16-byte pieces.
+bool gemm_f32_can_rotate(int head_dim) {
+    if (head_dim % 8) return false;
+    for (const Variant& v : kVariants)
+        if (v.bn % head_dim == 0) return true;
+    return false;
+}
+
+// C_i = A_i^T B_i, A_i [K, M_i] and B_i [K, N_i] row-major, one K, in one launch.
+int launch_gemm_f32_group(deers_ctx* ctx, int n, const GemmTN* t, int K) {
+    if (n < 1 || n > GEMM_GROUP_MAX) return DEERS_ERR_SHAPE;
+    const int rc = cluster_capacity(ctx);
+    if (rc) return rc;
+    GemmGroup gg{};
+    int M[GEMM_GROUP_MAX], N[GEMM_GROUP_MAX];
+    gg.n = n;
+    for (int i = 0; i < n; ++i) {
+        M[i] = t[i].M; N[i] = t[i].N;
+        gg.g[i] = gemm_args(t[i].M, t[i].N, K, t[i].a, t[i].M, t[i].b, t[i].N, t[i].c, t[i].N, DEERS_EPI_NONE, nullptr, 0, nullptr);
+    }
+    const GemmPlan p = plan_gemm(n, M, N, K, ctx->cluster_capacity, 0);
+    int res;
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM);
-        if (p.cfg == 0) rc = launch_orders<8, 8, 2>(ctx, p, g, a_mn, b_mn);
-        else if (p.cfg == 1) rc = launch_orders<8, 4, 4>(ctx, p, g, a_mn, b_mn);
-        else if (p.cfg == 2) rc = launch_orders<4, 4, 4>(ctx, p, g, a_mn, b_mn);
-        else if (p.cfg == 3) rc = launch_orders<4, 2, 4>(ctx, p, g, a_mn, b_mn);
-        else if (p.cfg == 4) rc = launch_orders<8, 6, 4>(ctx, p, g, a_mn, b_mn);
-        else rc = launch_orders<4, 6, 4>(ctx, p, g, a_mn, b_mn);
+        if (p.cfg == 0) res = launch_group<8, 8, 2>(ctx, p, gg);
+        else if (p.cfg == 1) res = launch_group<8, 4, 4>(ctx, p, gg);
+        else if (p.cfg == 2) res = launch_group<4, 4, 4>(ctx, p, gg);
+        else if (p.cfg == 3) res = launch_group<4, 2, 4>(ctx, p, gg);
+        else if (p.cfg == 4) res = launch_group<8, 6, 4>(ctx, p, gg);
+        else res = launch_group<4, 6, 4>(ctx, p, gg);
     }
     ctx->launches += 1;
-    return rc;
+    return res;
 }
 
 extern "C" size_t deers_b200_gemm_f32_workspace_bytes(deers_ctx* ctx, int32_t M, int32_t N, int32_t K) {

@@ -1,19 +1,19 @@
 // The f32 GPT of src/models/gpt.rs as a device-resident object and its training step.
 //
-// Forward (GPT::forward, gpt.rs:329-355), per block (Block::forward, gpt.rs:236-240):
-//   n1 = rmsnorm(x); qkv = n1 * [Wq|Wk|Wv] (one GEMM); q, k rotated and packed head-major in one launch
-//   (rope over 2H "heads" of the fused buffer), v read in place as a strided view; fused attention writing
-//   O token-major; x1 = x + O * Wout (residual in the GEMM epilogue); n2 = rmsnorm(x1);
-//   r = relu(n2 * Wup), h = r*r (GEMM epilogue); x2 = x1 + h * Wdown (epilogue).
-// Head: xf = rmsnorm(x); logits = xf * Wlm; cross-entropy reads the logits once; the backward overwrites
+// Forward (GPT::forward, gpt.rs:329-355), per block (Block::forward, gpt.rs:236-240), five launches:
+//   qkv = rmsnorm(x) * [Wq|Wk|Wv] (one GEMM; the norm's scale and the rotation of q and k in its epilogue); fused attention
+//   reading q, k, v in place as strided views and writing O token-major; x1 = x + O * Wout (residual in the GEMM epilogue);
+//   r = relu(rmsnorm(x1) * Wup), h = r*r (norm and relu in the GEMM); x2 = x1 + h * Wdown (epilogue).
+//   Separate norm and rotary kernels, nine launches per block before, cost 1.4 to 2 us each at these sizes.
+// Head: xf = rmsnorm(x) as an f16 pair; logits = xf * Wlm; cross-entropy reads the logits once; the backward overwrites
 // them with their gradient in one pass and feeds the two head GEMMs.
 // Backward: the exact transposes of the above, with the relu^2 backward in a GEMM epilogue, the residual
-// gradient added inside the RMSNorm backward, dQ / dK rotated back straight into the fused [N, 3C]
-// gradient buffer next to dV, and one GEMM each for d[Wq|Wk|Wv] and for the sum of the three input
-// gradients.  Every launch is one of this library's kernels; there is no host round trip in a step.
-// The weight gradients are off the critical path (nothing in the backward reads them): they run on a second
-// stream, forked from the main one where their operands are complete and joined before the gradient norm;
-// captured, the two streams become two branches of the step's graph.
+// gradient added inside the RMSNorm backward (which also writes the normalised rows again, for the weight gradients), dQ / dK
+// rotated back by the attention backward straight into the fused [N, 3C] gradient buffer next to dV, and one GEMM for the sum of
+// the three input gradients.  Every launch is one of this library's kernels; there is no host round trip in a step.
+// The weight gradients are off the critical path (nothing in the backward reads them): the four of a block are one
+// launch on a second stream, forked from the main one where their operands are complete and joined before the gradient norm;
+// captured, the two streams become two branches of the step's graph.  What they read is double-buffered by block.
 #include "common.cuh"
 
 #include <math.h>
@@ -28,7 +28,12 @@ struct LayerW {              // offsets (in floats) into the parameter-shaped ar
 };
 
 struct LayerAct {
-    float *n1, *inv1, *qkv, *qk, *o, *lse, *x1, *inv2, *n2, *r, *h, *x2;
+    float *inv1, *qkv, *o, *lse, *x1, *inv2, *r, *h, *x2;
+};
+
+// Gradients inside a block (and its normalised rows): read by the weight gradients while the next block's are made.
+struct LayerGrad {
+    float *dx, *dh, *dx1, *dqkv, *n1, *n2;      // of the block's output, MLP hidden, x1, q|k|v; rmsnorm(x), rmsnorm(x1)
 };
 
 size_t align64(size_t n) { return (n + 63) / 64 * 64; }     // floats: 256-byte boundaries
@@ -51,12 +56,13 @@ struct deers_gpt {
     float* act_base;
     float *x0, *invf, *xf, *logits, *ce_lse, *picked, *cosv, *sinv;
     std::vector<LayerAct> la;
-    float *dx_a, *dx_b, *dtmp, *dh, *dqkv, *dqk, *attn_ws;
-    size_t attn_ws_bytes;
+    LayerGrad lg[2];
+    float* dtmp;
+    bool rotate_fused;           // heads fit the GEMM's tiles whole: no rotary launches of their own
     // second stream for the weight gradients; events are markers only (no timing)
     cudaStream_t side;
-    cudaEvent_t ev_fork, ev_join, ev_done[4];
-    bool done_valid[4];          // ev_done[i] was recorded in the current backward pass
+    cudaEvent_t ev_fork, ev_join, ev_done[2];
+    bool done_valid[2];          // ev_done[i] was recorded in the current backward pass
     bool on_side;                // launches currently go to the side stream
     void* optim_scratch;
     float *loss_dev, *norm_dev;
@@ -143,35 +149,40 @@ void attn_desc(const deers_gpt* m, int B, int T, deers_attn_desc* d) {
     d->B = B; d->H = H; d->T = T; d->D = D;
     d->dtype = DEERS_F32; d->causal = 1;
     d->scale = (float)(1.0 / sqrt((double)D));                       // gpt.rs:139, storage.rs:115-117
-    const int64_t qk[4] = {(int64_t)2 * H * T * D, (int64_t)T * D, D, 1};        // inside the [B, 2H, T, D] pack
-    const int64_t v[4] = {(int64_t)T * 3 * C, D, (int64_t)3 * C, 1};             // column slice of [N, 3C]
+    const int64_t qkv[4] = {(int64_t)T * 3 * C, D, (int64_t)3 * C, 1};           // column slices of [N, 3C]
     const int64_t o[4] = {(int64_t)T * C, D, C, 1};                              // token-major [B, T, H, D]
     for (int i = 0; i < 4; ++i) {
-        d->q_strides[i] = qk[i]; d->k_strides[i] = qk[i]; d->dq_strides[i] = qk[i]; d->dk_strides[i] = qk[i];
-        d->v_strides[i] = v[i]; d->dv_strides[i] = v[i];
+        d->q_strides[i] = d->k_strides[i] = d->v_strides[i] = qkv[i];
+        d->dq_strides[i] = d->dk_strides[i] = d->dv_strides[i] = qkv[i];
         d->o_strides[i] = o[i]; d->do_strides[i] = o[i];
     }
 }
 
-void rope_desc(const deers_gpt* m, int B, int T, int inverse, deers_rope_desc* d) {
+// Rotation of q | k inside [N, 3C], in place: heads that the GEMM's tiles do not hold whole.
+int rotate_in_place(deers_gpt* m, int B, int T, int inverse, float* qkv) {
+    deers_rope_desc desc, *d = &desc;
     const int H = m->cfg.n_head, D = m->D, C = m->cfg.n_embd;
     memset(d, 0, sizeof(*d));
     d->B = B; d->T = T; d->H = 2 * H; d->D = D;                      // q and k heads side by side
     d->dtype = DEERS_F32; d->inverse = inverse;
     const int64_t tok[4] = {(int64_t)T * 3 * C, (int64_t)3 * C, D, 1};           // (b, t, h, d) in [N, 3C]
-    const int64_t head[4] = {(int64_t)2 * H * T * D, D, (int64_t)T * D, 1};      // (b, t, h, d) in [B, 2H, T, D]
-    for (int i = 0; i < 4; ++i) {
-        d->src_strides[i] = inverse ? head[i] : tok[i];
-        d->dst_strides[i] = inverse ? tok[i] : head[i];
-    }
+    for (int i = 0; i < 4; ++i) d->src_strides[i] = d->dst_strides[i] = tok[i];
+    return deers_b200_rope_pack(m->ctx, d, qkv, m->cosv, m->sinv, qkv);
+}
+
+GemmNorm norm_in(const deers_gpt* m, float* inv) {
+    GemmNorm f{};
+    f.eps = (float)m->cfg.rms_norm_eps;
+    f.inv = inv;
+    return f;
 }
 
 // with_head_pair: the head weight's f16 pair is made here (a training step changes the weight every time); otherwise the
-// caller has it current.
-int forward(deers_gpt* m, const long long* ids, int B, int T, bool with_head_pair) {
+// caller has it current.  keep: a backward follows (inverse norms and relu are wanted).  The logits go to `logits`, rows of ldl.
+int forward(deers_gpt* m, const long long* ids, int B, int T, bool with_head_pair, bool keep, float* logits, long long ldl) {
     deers_ctx* ctx = m->ctx;
     const deers_gpt_config& c = m->cfg;
-    const int C = c.n_embd, Hm = c.mlp_hidden_dim, V = c.vocab_size, H = c.n_head, D = m->D;
+    const int C = c.n_embd, Hm = c.mlp_hidden_dim, V = c.vocab_size;
     const long long N = (long long)B * T;
     float* W = m->arena[0];
     for (bool& v : m->done_valid) v = false;
@@ -185,31 +196,35 @@ int forward(deers_gpt* m, const long long* ids, int B, int T, bool with_head_pai
     GPT_TRY(launch_embedding_fwd(ctx, W + m->off_wte, ids, N, C, V, m->x0));                 // gpt.rs:343
     deers_attn_desc ad;
     attn_desc(m, B, T, &ad);
-    deers_rope_desc rd;
-    rope_desc(m, B, T, 0, &rd);
     const float* x = m->x0;
     for (int l = 0; l < c.n_layer; ++l) {
         const LayerW& w = m->lw[l];
         LayerAct& a = m->la[l];
-        GPT_TRY(launch_rmsnorm_fwd(ctx, N, C, c.rms_norm_eps, x, a.n1, a.inv1));             // norm1
-        GPT_TRY(gemm(m, (int)N, 3 * C, C, a.n1, C, 0, W + w.qkv, 3 * C, 1, a.qkv, 3 * C));   // q | k | v projections
-        GPT_TRY(deers_b200_rope_pack(ctx, &rd, a.qkv, m->cosv, m->sinv, a.qk));              // gpt.rs:135-136
-        GPT_TRY(deers_b200_attn_fwd(ctx, &ad, a.qk, a.qk + (size_t)H * T * D, a.qkv + 2 * C, a.o, a.lse, nullptr, 0));
+        GemmNorm f = norm_in(m, keep ? a.inv1 : nullptr);
+        if (m->rotate_fused) { f.cosv = m->cosv; f.sinv = m->sinv; f.rope_cols = 2 * C; f.rope_d = m->D; f.rope_t = T; }   // gpt.rs:135-136
+        GPT_TRY(launch_gemm_f32_norm(ctx, (int)N, 3 * C, C, x, W + w.qkv, a.qkv, DEERS_EPI_NONE, nullptr, f));   // norm1, q | k | v projections
+        if (!m->rotate_fused) GPT_TRY(rotate_in_place(m, B, T, 0, a.qkv));
+        GPT_TRY(deers_b200_attn_fwd(ctx, &ad, a.qkv, a.qkv + C, a.qkv + 2 * C, a.o, a.lse, nullptr, 0));
         GPT_TRY(gemm(m, (int)N, C, C, a.o, C, 0, W + w.out, C, 1, a.x1, C, DEERS_EPI_ADD, x, C));       // x + out_proj
-        GPT_TRY(launch_rmsnorm_fwd(ctx, N, C, c.rms_norm_eps, a.x1, a.n2, a.inv2));          // norm2
-        GPT_TRY(gemm(m, (int)N, Hm, C, a.n2, C, 0, W + w.up, Hm, 1, a.h, Hm, DEERS_EPI_RELU_SQ, nullptr, 0, a.r));
+        GPT_TRY(launch_gemm_f32_norm(ctx, (int)N, Hm, C, a.x1, W + w.up, a.h, DEERS_EPI_RELU_SQ, keep ? a.r : nullptr,
+                                     norm_in(m, keep ? a.inv2 : nullptr)));                  // norm2, up_proj, relu^2
         GPT_TRY(gemm(m, (int)N, C, Hm, a.h, Hm, 0, W + w.down, C, 1, a.x2, C, DEERS_EPI_ADD, a.x1, C)); // x1 + down_proj
         x = a.x2;
     }
-    GPT_TRY(launch_rmsnorm_fwd(ctx, N, C, c.rms_norm_eps, x, m->xf, m->invf));               // gpt.rs:347
     if (m->tc_head) {
-        // lm_head on the tensor core at f32 accuracy: both operands as f16 pairs (the weight changes every step)
-        GPT_TRY(launch_split_f16x3(ctx, N, C, m->xf, C, 1.0f, m->xf_hi, m->xf_lo, C));
+        // lm_head on the tensor core at f32 accuracy: both operands as f16 pairs (the weight changes every step); gpt.rs:347
+        int rc = launch_rmsnorm_split(ctx, N, C, c.rms_norm_eps, x, m->invf, m->xf_hi, m->xf_lo);
+        if (rc == DEERS_ERR_UNSUPPORTED) {
+            GPT_TRY(launch_rmsnorm_fwd(ctx, N, C, c.rms_norm_eps, x, m->xf, m->invf));
+            rc = launch_split_f16x3(ctx, N, C, m->xf, C, 1.0f, m->xf_hi, m->xf_lo, C);
+        }
+        GPT_TRY(rc);
         GPT_TRY(wait_done(m, 0));
-        GPT_TRY(launch_gemm_f16x3(ctx, (int)N, V, C, m->xf_hi, m->xf_lo, C, 0, m->w_hi, m->w_lo, m->Vld, 1, m->logits, m->Vld,
+        GPT_TRY(launch_gemm_f16x3(ctx, (int)N, V, C, m->xf_hi, m->xf_lo, C, 0, m->w_hi, m->w_lo, m->Vld, 1, logits, ldl,
                                   1.0f, m->x3_ws, m->x3_ws_bytes));
     } else {
-        GPT_TRY(gemm(m, (int)N, V, C, m->xf, C, 0, W + m->off_lm, m->Vld, 1, m->logits, m->Vld)); // lm_head
+        GPT_TRY(launch_rmsnorm_fwd(ctx, N, C, c.rms_norm_eps, x, m->xf, m->invf));
+        GPT_TRY(gemm(m, (int)N, V, C, m->xf, C, 0, W + m->off_lm, m->Vld, 1, logits, ldl));  // lm_head
     }
     return DEERS_OK;
 }
@@ -217,7 +232,7 @@ int forward(deers_gpt* m, const long long* ids, int B, int T, bool with_head_pai
 int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targets, int B, int T) {
     deers_ctx* ctx = m->ctx;
     const deers_gpt_config& c = m->cfg;
-    const int C = c.n_embd, Hm = c.mlp_hidden_dim, V = c.vocab_size, H = c.n_head, D = m->D;
+    const int C = c.n_embd, Hm = c.mlp_hidden_dim, V = c.vocab_size;
     const long long N = (long long)B * T;
     const int Vld = m->Vld;
     float* W = m->arena[0];
@@ -246,56 +261,39 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
             GPT_TRY(gemm(m, C, V, (int)N, m->xf, C, 1, m->logits, Vld, 1, G + m->off_lm, Vld));  // d lm_head = xf^T dlogits
         }
     }
-    GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, x_last, m->invf, m->dtmp, nullptr, m->dx_a));
+    const int last = c.n_layer ? (c.n_layer - 1) & 1 : 0;
+    GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, x_last, m->invf, m->dtmp, nullptr, m->lg[last].dx));
+    const float* dx0 = m->lg[last].dx;
     deers_attn_desc ad;
     attn_desc(m, B, T, &ad);
-    deers_rope_desc rd;
-    rope_desc(m, B, T, 1, &rd);
     for (int l = c.n_layer - 1; l >= 0; --l) {
         const LayerW& w = m->lw[l];
         LayerAct& a = m->la[l];
+        LayerGrad &d = m->lg[l & 1], &below = m->lg[(l & 1) ^ 1];
         const float* x_in = l ? m->la[l - 1].x2 : m->x0;
-        // MLP branch: x2 = x1 + relu(n2 Wup)^2 Wdown
+        // MLP branch: x2 = x1 + relu(rmsnorm(x1) Wup)^2 Wdown
+        GPT_TRY(gemm(m, (int)N, Hm, C, d.dx, C, 0, W + w.down, C, 0, d.dh, Hm, DEERS_EPI_MUL_AUX2, nullptr, 0, a.r));
+        GPT_TRY(gemm(m, (int)N, C, Hm, d.dh, Hm, 0, W + w.up, Hm, 0, m->dtmp, C));           // d n2 = du Wup^T
+        GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, a.x1, a.inv2, m->dtmp, d.dx, d.dx1, d.n2));    // d x1
+        // attention branch: x1 = x + attn(rmsnorm(x)) Wout
+        GPT_TRY(gemm(m, (int)N, C, C, d.dx1, C, 0, W + w.out, C, 0, m->dtmp, C));            // d o (token-major)
+        GPT_TRY(launch_attn_bwd_f32(ctx, &ad, a.qkv, a.qkv + C, a.qkv + 2 * C, a.o, a.lse, m->dtmp, d.dqkv, d.dqkv + C, d.dqkv + 2 * C,
+                                    m->rotate_fused ? m->cosv : nullptr, m->rotate_fused ? m->sinv : nullptr));
+        if (!m->rotate_fused) GPT_TRY(rotate_in_place(m, B, T, 1, d.dqkv));
+        GPT_TRY(gemm(m, (int)N, C, 3 * C, d.dqkv, 3 * C, 0, W + w.qkv, 3 * C, 0, m->dtmp, C)); // d n1 (three terms in one)
+        GPT_TRY(wait_done(m, (l & 1) ^ 1));                                                  // the block above has read what this block's input gradient replaces
+        GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, x_in, a.inv1, m->dtmp, d.dx1, below.dx, d.n1)); // d x
+        dx0 = below.dx;
         {
             SideScope side(m);
             GPT_TRY(side.rc);
-            GPT_TRY(gemm(m, Hm, C, (int)N, a.h, Hm, 1, m->dx_a, C, 1, G + w.down, C));       // d Wdown = h^T dx
-            GPT_TRY(side.done(0));
+            const GemmTN grads[4] = {{Hm, C, a.h, d.dx, G + w.down}, {C, Hm, d.n2, d.dh, G + w.up},              // d Wdown = h^T dx, d Wup = n2^T du
+                                     {C, C, a.o, d.dx1, G + w.out}, {C, 3 * C, d.n1, d.dqkv, G + w.qkv}};        // d Wout = o^T dx1, d [Wq|Wk|Wv]
+            GPT_TRY(launch_gemm_f32_group(ctx, 4, grads, (int)N));
+            GPT_TRY(side.done(l & 1));
         }
-        GPT_TRY(wait_done(m, 1));                                                            // the previous d Wup has read dh
-        GPT_TRY(gemm(m, (int)N, Hm, C, m->dx_a, C, 0, W + w.down, C, 0, m->dh, Hm, DEERS_EPI_MUL_AUX2, nullptr, 0, a.r));
-        {
-            SideScope side(m);
-            GPT_TRY(side.rc);
-            GPT_TRY(gemm(m, C, Hm, (int)N, a.n2, C, 1, m->dh, Hm, 1, G + w.up, Hm));         // d Wup = n2^T du
-            GPT_TRY(side.done(1));
-        }
-        GPT_TRY(gemm(m, (int)N, C, Hm, m->dh, Hm, 0, W + w.up, Hm, 0, m->dtmp, C));          // d n2 = du Wup^T
-        GPT_TRY(wait_done(m, 2));                                                            // the previous d Wout has read dx_b
-        GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, a.x1, a.inv2, m->dtmp, m->dx_a, m->dx_b));     // d x1
-        // attention branch: x1 = x + attn(n1) Wout
-        {
-            SideScope side(m);
-            GPT_TRY(side.rc);
-            GPT_TRY(gemm(m, C, C, (int)N, a.o, C, 1, m->dx_b, C, 1, G + w.out, C));          // d Wout = o^T dx1
-            GPT_TRY(side.done(2));
-        }
-        GPT_TRY(gemm(m, (int)N, C, C, m->dx_b, C, 0, W + w.out, C, 0, m->dtmp, C));          // d o (token-major)
-        GPT_TRY(wait_done(m, 3));                                                            // the previous d Wqkv has read dqkv
-        GPT_TRY(deers_b200_attn_bwd(ctx, &ad, a.qk, a.qk + (size_t)H * T * D, a.qkv + 2 * C, a.o, a.lse, m->dtmp, m->dqk,
-                                    m->dqk + (size_t)H * T * D, m->dqkv + 2 * C, m->attn_ws, m->attn_ws_bytes));
-        GPT_TRY(deers_b200_rope_pack(ctx, &rd, m->dqk, m->cosv, m->sinv, m->dqkv));          // d q | d k back to [N, 3C]
-        {
-            SideScope side(m);
-            GPT_TRY(side.rc);
-            GPT_TRY(gemm(m, C, 3 * C, (int)N, a.n1, C, 1, m->dqkv, 3 * C, 1, G + w.qkv, 3 * C)); // d [Wq|Wk|Wv]
-            GPT_TRY(side.done(3));
-        }
-        GPT_TRY(gemm(m, (int)N, C, 3 * C, m->dqkv, 3 * C, 0, W + w.qkv, 3 * C, 0, m->dtmp, C)); // d n1 (three terms in one)
-        GPT_TRY(wait_done(m, 0));                                                            // this layer's d Wdown has read dx_a
-        GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, x_in, a.inv1, m->dtmp, m->dx_b, m->dx_a));     // d x
     }
-    GPT_TRY(launch_embedding_bwd(ctx, m->dx_a, ids, N, C, V, G + m->off_wte));
+    GPT_TRY(launch_embedding_bwd(ctx, dx0, ids, N, C, V, G + m->off_wte));
     return join_side(m);
 }
 
@@ -349,7 +347,7 @@ int run_fwd_bwd(deers_gpt* m, int B, int T, bool with_norm) {
         // the shape has run eagerly once (every kernel's attributes are set): capture it
         cudaGraph_t graph = nullptr;
         if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            int rc = forward(m, m->ids_dev, B, T, true);
+            int rc = forward(m, m->ids_dev, B, T, true, true, m->logits, m->Vld);
             if (!rc) rc = loss_and_backward(m, m->ids_dev, m->tgt_dev, B, T);
             if (!rc) rc = grad_norm(m);
             const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
@@ -370,7 +368,7 @@ int run_fwd_bwd(deers_gpt* m, int B, int T, bool with_norm) {
             m->graph_enabled = false;
         }
     }
-    GPT_TRY(forward(m, m->ids_dev, B, T, true));
+    GPT_TRY(forward(m, m->ids_dev, B, T, true, true, m->logits, m->Vld));
     GPT_TRY(loss_and_backward(m, m->ids_dev, m->tgt_dev, B, T));
     if (with_norm) GPT_TRY(grad_norm(m));
     if (can_graph) m->eager_steps_BT += 1;
@@ -437,12 +435,13 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
     m->tc_head = cfg->vocab_size >= 1024 && cfg->n_embd % 8 == 0 && cfg->n_embd >= 64;
     m->graph_enabled = true; m->graph_exec = nullptr; m->graph_B = m->graph_T = -1; m->eager_steps_BT = 0;
     m->on_side = false;
+    m->rotate_fused = gemm_f32_can_rotate(D);
     m->head_pair_current = m->captured_updates = false;
     {
         // the weight-gradient stream and its markers; without them the step simply runs on one stream
         bool ok = cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking) == cudaSuccess;
         if (!ok) m->side = nullptr;
-        cudaEvent_t* evs[6] = {&m->ev_fork, &m->ev_join, &m->ev_done[0], &m->ev_done[1], &m->ev_done[2], &m->ev_done[3]};
+        cudaEvent_t* evs[4] = {&m->ev_fork, &m->ev_join, &m->ev_done[0], &m->ev_done[1]};
         for (cudaEvent_t* e : evs)
             if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) { *e = nullptr; ok = false; }
         if (!ok && m->side) { cudaStreamDestroy(m->side); m->side = nullptr; }
@@ -477,7 +476,6 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
 
     // ---- activations, scratch
     off = 0;
-    const size_t HTD = N * C;                                          // B * H * T * D
     struct Slot { float** p; size_t n; };
     std::vector<Slot> slots;
     auto want = [&slots](float** p, size_t n) { slots.push_back({p, n}); };
@@ -486,16 +484,14 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
     want(&m->cosv, (size_t)cfg->sequence_len * (D / 2)); want(&m->sinv, (size_t)cfg->sequence_len * (D / 2));
     m->la.resize(cfg->n_layer);
     for (auto& a : m->la) {
-        want(&a.n1, N * C); want(&a.inv1, N); want(&a.qkv, N * 3 * C); want(&a.qk, 2 * HTD); want(&a.o, N * C);
-        want(&a.lse, N * cfg->n_head); want(&a.x1, N * C); want(&a.inv2, N); want(&a.n2, N * C);
+        want(&a.inv1, N); want(&a.qkv, N * 3 * C); want(&a.o, N * C);
+        want(&a.lse, N * cfg->n_head); want(&a.x1, N * C); want(&a.inv2, N);
         want(&a.r, N * Hm); want(&a.h, N * Hm); want(&a.x2, N * C);
     }
-    want(&m->dx_a, N * C); want(&m->dx_b, N * C); want(&m->dtmp, N * C); want(&m->dh, N * Hm);
-    want(&m->dqkv, N * 3 * C); want(&m->dqk, 2 * HTD);
-    deers_attn_desc ad;
-    attn_desc(m, max_batch, cfg->sequence_len, &ad);
-    m->attn_ws_bytes = deers_b200_attn_workspace_bytes(&ad, 1);
-    want(&m->attn_ws, m->attn_ws_bytes / sizeof(float) + 64);
+    for (auto& d : m->lg) {
+        want(&d.dx, N * C); want(&d.dh, N * Hm); want(&d.dx1, N * C); want(&d.dqkv, N * 3 * C); want(&d.n1, N * C); want(&d.n2, N * C);
+    }
+    want(&m->dtmp, N * C);
     want(&m->loss_dev, 64);
     m->norm_dev = nullptr;
     size_t total = 0;
@@ -563,7 +559,7 @@ extern "C" void deers_b200_gpt_destroy(deers_gpt* m) {
     drop_graph(m);
     if (m->side) { cudaStreamSynchronize(m->side); cudaStreamDestroy(m->side); }
     {
-        cudaEvent_t evs[6] = {m->ev_fork, m->ev_join, m->ev_done[0], m->ev_done[1], m->ev_done[2], m->ev_done[3]};
+        cudaEvent_t evs[4] = {m->ev_fork, m->ev_join, m->ev_done[0], m->ev_done[1]};
         for (cudaEvent_t e : evs)
             if (e) cudaEventDestroy(e);
     }
@@ -636,7 +632,7 @@ extern "C" int deers_b200_gpt_forward(deers_gpt* m, const int64_t* ids, int32_t 
     deers_ctx* ctx = m->ctx;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     const bool rec = recording(m), kept = m->head_pair_current && !m->captured_updates && !rec;
-    GPT_TRY(forward(m, (const long long*)ids, B, T, !kept));
+    GPT_TRY(forward(m, (const long long*)ids, B, T, !kept, false, m->logits, m->Vld));
     if (!rec) m->head_pair_current = m->tc_head;
     if (logits) {
         const int V = m->cfg.vocab_size;

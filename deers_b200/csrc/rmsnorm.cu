@@ -13,6 +13,8 @@
 // pass over HBM); longer rows take two passes of 16-byte loads.
 // HBM-bound: 8 bytes per element forward, 12 backward.  Sums are f32 shuffle trees (the reference
 // sums left to right), so parity is to rounding, not to the bit.
+#include <cuda_fp16.h>
+
 #include "common.cuh"
 
 namespace {
@@ -25,11 +27,26 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// BWD = false: y = x * inv, inv_out[row] = inv.   BWD = true: dx from x, dy and the saved inv.
-template <bool BWD, bool VEC, bool VEC2 = false>
+// Four elements of y as the f16 pair the split-f16 products read (hi = f16(v), lo = f16((v - hi) * 2^11); gemm_f16x3_sm100.cu).
+__device__ __forceinline__ void put_pair(__half* hi, __half* lo, long long at, const float4& v) {
+    const float x[4] = {v.x, v.y, v.z, v.w};
+    __half h[4], l[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        h[e] = __float2half_rn(x[e]);
+        l[e] = __float2half_rn((x[e] - __half2float(h[e])) * 2048.0f);
+    }
+    *reinterpret_cast<uint2*>(hi + at) = *reinterpret_cast<const uint2*>(h);
+    *reinterpret_cast<uint2*>(lo + at) = *reinterpret_cast<const uint2*>(l);
+}
+
+// BWD = false: y = x * inv, inv_out[row] = inv (PAIR: y leaves as the f16 pair hi, lo, rows dense, instead of out).
+// BWD = true: dx from x, dy and the saved inv; n_out (may be nullptr) receives y again for the weight gradient.
+template <bool BWD, bool VEC, bool VEC2 = false, bool PAIR = false>
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const float* dy, const float* add, float* __restrict__ out,
                                                       float* __restrict__ inv_io, long long rows, int C, float eps,
-                                                      float inv_n) {
+                                                      float inv_n, float* __restrict__ n_out, __half* __restrict__ hi,
+                                                      __half* __restrict__ lo) {
     if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room)
     chain_wait();
     const int lane = threadIdx.x & 31;
@@ -76,10 +93,12 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
                             const float4 r = reinterpret_cast<const float4*>(add + row * C)[p];
                             o.x = r.x + o.x; o.y = r.y + o.y; o.z = r.z + o.z; o.w = r.w + o.w;
                         }
+                        if (n_out) reinterpret_cast<float4*>(n_out + row * C)[p] = make_float4(xv[i].x * inv, xv[i].y * inv, xv[i].z * inv, xv[i].w * inv);
                     } else {
                         o.x = xv[i].x * inv; o.y = xv[i].y * inv; o.z = xv[i].z * inv; o.w = xv[i].w * inv;
                     }
-                    reinterpret_cast<float4*>(orow)[p] = o;
+                    if constexpr (PAIR) put_pair(hi, lo, row * C + 4 * p, o);
+                    else reinterpret_cast<float4*>(orow)[p] = o;
                 }
             }
         } else if (VEC2) {                                      // long aligned rows: two passes of 16-byte loads
@@ -132,6 +151,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
                             const float4 r = reinterpret_cast<const float4*>(add + row * C)[p];
                             o.x = r.x + o.x; o.y = r.y + o.y; o.z = r.z + o.z; o.w = r.w + o.w;
                         }
+                        if (n_out) reinterpret_cast<float4*>(n_out + row * C)[p] = make_float4(a[u].x * inv, a[u].y * inv, a[u].z * inv, a[u].w * inv);
                     } else {
                         o.x = a[u].x * inv; o.y = a[u].y * inv; o.z = a[u].z * inv; o.w = a[u].w * inv;
                     }
@@ -154,6 +174,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
             for (int c = lane; c < C; c += 32) {
                 float o = BWD ? gr[c] * inv - xr[c] * k : xr[c] * inv;
                 if (BWD && add) o = add[row * C + c] + o;
+                if (BWD && n_out) n_out[row * C + c] = xr[c] * inv;
                 orow[c] = o;
             }
         }
@@ -161,10 +182,11 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
 }
 
 // Rows of 1025 .. 8192 elements: a whole block owns a row, which still stays in registers (one pass over HBM).
-template <bool BWD>
+template <bool BWD, bool PAIR = false>
 __global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* x, const float* dy, const float* add, float* __restrict__ out,
                                                             float* __restrict__ inv_io, long long rows, int C, float eps,
-                                                            float inv_n) {
+                                                            float inv_n, float* __restrict__ n_out, __half* __restrict__ hi,
+                                                            __half* __restrict__ lo) {
     if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room)
     chain_wait();
     __shared__ float part[8];
@@ -215,10 +237,12 @@ __global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* x, cons
                         const float4 r = reinterpret_cast<const float4*>(add + row * C)[p];
                         o.x = r.x + o.x; o.y = r.y + o.y; o.z = r.z + o.z; o.w = r.w + o.w;
                     }
+                    if (n_out) reinterpret_cast<float4*>(n_out + row * C)[p] = make_float4(xv[i].x * inv, xv[i].y * inv, xv[i].z * inv, xv[i].w * inv);
                 } else {
                     o.x = xv[i].x * inv; o.y = xv[i].y * inv; o.z = xv[i].z * inv; o.w = xv[i].w * inv;
                 }
-                o4[p] = o;
+                if constexpr (PAIR) put_pair(hi, lo, row * C + 4 * p, o);
+                else o4[p] = o;
             }
         }
     }
@@ -226,9 +250,9 @@ __global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* x, cons
 
 template <bool BWD>
 int rms_launch(deers_ctx* ctx, long long rows, int C, float eps, const float* x, const float* dy, float* out, float* inv,
-               const float* add = nullptr) {
+               const float* add = nullptr, float* n_out = nullptr) {
     if (rows == 0) return DEERS_OK;
-    uintptr_t bits = (uintptr_t)x | (uintptr_t)out | (BWD ? (uintptr_t)dy : 0) | (uintptr_t)add;
+    uintptr_t bits = (uintptr_t)x | (uintptr_t)out | (BWD ? (uintptr_t)dy : 0) | (uintptr_t)add | (uintptr_t)n_out;
     const bool aligned = (C % 4) == 0 && (bits & 15u) == 0;
     const bool vec = aligned && C <= 32 * RN_MAXV * 4;
     const long long want = (rows + 7) / 8;
@@ -237,12 +261,12 @@ int rms_launch(deers_ctx* ctx, long long rows, int C, float eps, const float* x,
     const float inv_n = (float)(1.0 / (double)C);               // mean = sum * (1/n as f64 -> f32), src/tensor.rs:461-465
     {
         KernelTimerScope ts(ctx, DEERS_K_NORM);
-        if (vec) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n));
+        if (vec) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
         else if (aligned && C <= 256 * RN_MAXV * 4) {
             const unsigned bgrid = (unsigned)(rows < cap ? rows : cap);
-            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_block_kernel<BWD>, bgrid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n));
-        } else if (aligned) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n));
-        else DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n));
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_block_kernel<BWD>, bgrid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
+        } else if (aligned) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
+        else DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -271,8 +295,28 @@ int launch_rmsnorm_fwd(deers_ctx* ctx, long long rows, int C, double eps, const 
     return rms_launch<false>(ctx, rows, C, (float)eps, x, nullptr, y, inv_norm);
 }
 int launch_rmsnorm_bwd(deers_ctx* ctx, long long rows, int C, const float* x, const float* inv_norm, const float* dy,
-                       const float* add, float* dx) {
-    return rms_launch<true>(ctx, rows, C, 0.f, x, dy, dx, const_cast<float*>(inv_norm), add);
+                       const float* add, float* dx, float* n_out) {
+    return rms_launch<true>(ctx, rows, C, 0.f, x, dy, dx, const_cast<float*>(inv_norm), add, n_out);
+}
+// y as an f16 pair, one pass where the row stays in registers.  DEERS_ERR_UNSUPPORTED otherwise: the caller normalises and
+// splits in two.
+int launch_rmsnorm_split(deers_ctx* ctx, long long rows, int C, double eps, const float* x, float* inv_norm, void* hi, void* lo) {
+    if (C % 4 || C > 256 * RN_MAXV * 4 || (((uintptr_t)x | (uintptr_t)hi | (uintptr_t)lo) & 15u)) return DEERS_ERR_UNSUPPORTED;
+    const long long cap = 16LL * ctx->sm_count, want = C <= 32 * RN_MAXV * 4 ? (rows + 7) / 8 : rows;
+    const unsigned grid = (unsigned)(want < cap ? want : cap);
+    const float inv_n = (float)(1.0 / (double)C);
+    {
+        KernelTimerScope ts(ctx, DEERS_K_NORM);
+        if (C <= 32 * RN_MAXV * 4)
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<false, true, false, true>, grid, 256, 0, 1, x, nullptr, nullptr, nullptr, inv_norm,
+                                               rows, C, (float)eps, inv_n, nullptr, (__half*)hi, (__half*)lo));
+        else
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_block_kernel<false, true>, grid, 256, 0, 1, x, nullptr, nullptr, nullptr, inv_norm, rows, C,
+                                               (float)eps, inv_n, nullptr, (__half*)hi, (__half*)lo));
+    }
+    ctx->launches += 1;
+    DEERS_CUDA_TRY(ctx, cudaGetLastError());
+    return DEERS_OK;
 }
 
 extern "C" int deers_b200_rmsnorm_bwd_add(deers_ctx* ctx, int64_t rows, int32_t C, const float* x, const float* inv_norm,
