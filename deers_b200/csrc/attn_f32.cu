@@ -250,9 +250,10 @@ __device__ __forceinline__ void store4(float* p, float4 v, int valid, int vec) {
     if (valid > 3) p[3] = v.w;
 }
 
-template <int DP>
+// FBN: rows of a tile streamed in the forward
+template <int DP, int FBN = 32>
 struct Tile {
-    static constexpr int BN = DP <= 64 ? 64 : 32;               // rows of a streamed tile
+    static constexpr int BN = FBN;
     static constexpr int NC = BN / 8;                           // score columns per thread
     static constexpr int LD = DP + 4;
     static constexpr int ROWS = BM * LD;                        // a stationary tile
@@ -273,10 +274,10 @@ struct Tile {
 // ---------------------------------------------------------------------------
 // Forward: one block per (batch*head, 32-row query tile); the heaviest (latest) query tiles of all slices first.
 // ---------------------------------------------------------------------------
-template <int DP>
+template <int DP, int FBN>
 __global__ void __launch_bounds__(NT, DP <= 32 ? 2 : 1) attn_fwd_f32_kernel(const F32Params p) {
     chain_wait();
-    using L = Tile<DP>;
+    using L = Tile<DP, FBN>;
     constexpr int BN = L::BN, NC = L::NC, LD = L::LD, PLD = L::FWD_PLD;
     extern __shared__ __align__(16) float smem[];
     const int g = threadIdx.x / 64, t = threadIdx.x % 64;
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(NT, DP <= 32 ? 2 : 1) attn_fwd_f32_kernel(cons
         const int k0 = j * BN;
         if (j != g) { cp_wait<1>(); group_sync(g); }            // this K tile has landed for both warps
         float s[4][NC];
-        tile_nt<DP, NC, (DP >= 64)>(Qs, Ks, ty, tx, s);
+        tile_nt<DP, NC, (DP >= 64 || FBN == 32)>(Qs, Ks, ty, tx, s);
         group_sync(g);                                          // K is consumed: the next one may land
         if (j + NG < ntiles) fetch_tile<DP, BN, 64>(Ks, kb, k0 + NG * BN, p.T, p.D, p.sk.t, p.vec, t);
         cp_commit();
@@ -690,17 +691,28 @@ bool rows_vec_ok(const void* ptr, const int64_t* s) {
     return (((uintptr_t)ptr) & 15u) == 0 && (s[0] & 3) == 0 && (s[1] & 3) == 0 && (s[2] & 3) == 0;
 }
 
-template <int DP>
-int fwd_impl(deers_ctx* ctx, const F32Params& p) {
-    DEERS_SMEM_ONCE(ctx, (attn_fwd_f32_kernel<DP>), Tile<DP>::FWD_SMEM);
+template <int DP, int FBN>
+int fwd_launch_f32(deers_ctx* ctx, const F32Params& p) {
+    DEERS_SMEM_ONCE(ctx, (attn_fwd_f32_kernel<DP, FBN>), (Tile<DP, FBN>::FWD_SMEM));
     const dim3 grid(p.B * p.H, (p.T + BM - 1) / BM);
+    const auto kernel = attn_fwd_f32_kernel<DP, FBN>;
     {
         KernelTimerScope ts(ctx, DEERS_K_FWD);
-        DEERS_CUDA_TRY(ctx, launch_chained(ctx, attn_fwd_f32_kernel<DP>, grid, NT, Tile<DP>::FWD_SMEM, 1, p));
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, grid, NT, (Tile<DP, FBN>::FWD_SMEM), 1, p));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     return DEERS_OK;
+}
+
+// Narrow heads stream 64 keys at a time (half the reads of Q per score), unless the sequence has so few tiles that groups
+// would go without: up to NG * 32 keys, tiles of 32.
+template <int DP>
+int fwd_impl(deers_ctx* ctx, const F32Params& p) {
+    if constexpr (DP <= 64) {
+        if (p.T > NG * 32) return fwd_launch_f32<DP, 64>(ctx, p);
+    }
+    return fwd_launch_f32<DP, 32>(ctx, p);
 }
 
 template <int DP>

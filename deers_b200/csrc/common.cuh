@@ -210,16 +210,16 @@ int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long lo
                     long long ldb, int b_mn, float* c, long long ldc, int epi, const float* r, long long ldr, float* aux);
 // The same with the rows of A normalised on the way, C [M,N] = rmsnorm(A [M,K]) * B [K,N], all dense: what a block's pre-norms
 // feed (launch_gemm_f32_norm).  inv (may be nullptr) receives the inverse norms.  Columns [0, rope_cols), heads of rope_d columns,
-// are rotated by position m % rope_t with the tables cosv, sinv [rope_t][rope_d / 2] (0 columns: none); the head width has to
-// pass gemm_f32_can_rotate().
+// may be rotated by position m % rope_t with the tables cosv, sinv [rope_t][rope_d / 2] (0 columns: none); *rotated tells whether
+// they were.
 struct GemmNorm {
     float eps;
     float* inv;
     const float* cosv; const float* sinv;
     int rope_cols, rope_d, rope_t;
 };
-int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, const float* b, float* c, int epi, float* aux, const GemmNorm& f);
-bool gemm_f32_can_rotate(int head_dim);
+int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, const float* b, float* c, int epi, float* aux, const GemmNorm& f,
+                         bool* rotated);
 // Products C_i [M_i,N_i] = A_i^T B_i with A_i [K,M_i], B_i [K,N_i], dense, in one launch.
 constexpr int GEMM_GROUP_MAX = 4;
 struct GemmTN { int M, N; const float* a; const float* b; float* c; };
@@ -233,14 +233,16 @@ int launch_rmsnorm_split(deers_ctx* ctx, long long rows, int C, double eps, cons
 int launch_embedding_fwd(deers_ctx* ctx, const float* weight, const long long* ids, long long n_ids, int C, long long V,
                          float* out);
 int launch_embedding_bwd(deers_ctx* ctx, const float* dout, const long long* ids, long long n_ids, int C, long long V,
-                         float* dweight);
+                         float* dweight, bool cleared = false);
 int launch_cross_entropy_fwd(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, long long rows,
                              long long V, float* lse, float* picked, float* loss);
 int launch_cross_entropy_bwd(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, const float* lse,
                              long long rows, long long V, float upstream, float* dlogits, long long ldd);
-// AdamW with the trainer's rule "no update when the gradient norm is not finite" (optim.cu)
+// AdamW with the trainer's rule "no update when the gradient norm is not finite" (optim.cu).  said: what the caller wants to
+// know of the step, written by the same launch.
+struct StepSaid { const float* loss; float* loss_out; float* norm_out; };
 int launch_adamw(deers_ctx* ctx, int n_tensors, const deers_optim_tensor* tensors, const deers_adamw_hyper* h,
-                 const float* norm_dev, double max_norm, bool skip_nonfinite);
+                 const float* norm_dev, double max_norm, bool skip_nonfinite, const StepSaid& said = StepSaid{});
 // f32-accurate tensor-core GEMM on split f16 operands (gemm_f16x3_sm100.cu) and the split writers
 size_t gemm_f16x3_workspace_bytes(const deers_ctx* ctx, int M, int N, int K);
 int launch_split_f16x3(deers_ctx* ctx, long long rows, int cols, const float* src, long long ld_src, float scale,

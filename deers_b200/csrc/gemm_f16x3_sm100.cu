@@ -26,7 +26,7 @@ constexpr int XM = 128, XN = 128, XK = 64;
 constexpr uint32_t X_TILE = 128 * XK * 2;          // 16 KB: one operand tile of a stage
 constexpr uint32_t X_STAGE = 4 * X_TILE;           // A_hi | A_lo | B_hi | B_lo
 constexpr int X_STAGES = 3;
-constexpr uint32_t X_SMEM = X_STAGES * X_STAGE + 256;
+
 constexpr uint32_t X_MN_BLOCK = XK * 128;          // 8 KB: 64 K-rows x 64 columns of an MN-major operand
 constexpr float X_LO = 1.0f / 2048.0f;
 
@@ -34,6 +34,10 @@ constexpr float X_LO = 1.0f / 2048.0f;
 // head's forward product waits on its epilogue (206 MB of logits through 4 warps per SM), not on the tensor pipe
 constexpr int X_EPI_WG = 2;
 constexpr int X_THREADS = 64 + 128 * X_EPI_WG;
+
+constexpr uint32_t X_TURN = X_STAGES * X_STAGE + 256;              // per epilogue warp: 32 x 32 elements, padded
+constexpr int X_TURN_FLOATS = 32 * 33;
+constexpr uint32_t X_SMEM = X_TURN + 4 * X_EPI_WG * X_TURN_FLOATS * 4;
 
 enum XBar { X_FULL = 0, X_EMPTY = 3, X_ACC_FULL = 6, X_ACC_EMPTY = 8, X_COUNT = 10 };
 
@@ -204,29 +208,44 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_consta
                     tc_fence_before_sync();
                     mbar_arrive(&bars[X_ACC_EMPTY + buf]);
                 }
-                uint4 pc[8];
+                float o[32];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    float o[4];
+                for (int e = 0; e < 32; ++e) o[e] = fmaf(__uint_as_float(rc[e]), X_LO, __uint_as_float(rm[e])) * p.out_scale;
+                if (p.vec) {
+                    uint4 pc[8];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        o[e] = fmaf(__uint_as_float(rc[q * 4 + e]), X_LO, __uint_as_float(rm[q * 4 + e])) * p.out_scale;
-                    pc[q] = make_uint4(__float_as_uint(o[0]), __float_as_uint(o[1]), __float_as_uint(o[2]), __float_as_uint(o[3]));
-                }
-                // 16-byte pieces transposed within 8-lane groups: a store instruction writes 128 contiguous bytes per row
-                transpose_pieces<8>(pc, (uint32_t)lane);
-                const int col = tn * XN + chunk * 32 + (lane & 7) * 4;
+                    for (int q = 0; q < 8; ++q)
+                        pc[q] = make_uint4(__float_as_uint(o[q * 4]), __float_as_uint(o[q * 4 + 1]), __float_as_uint(o[q * 4 + 2]), __float_as_uint(o[q * 4 + 3]));
+                    // 16-byte pieces transposed within 8-lane groups: a store instruction writes 128 contiguous bytes per row
+                    transpose_pieces<8>(pc, (uint32_t)lane);
+                    const int col = tn * XN + chunk * 32 + (lane & 7) * 4;
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const int row = row0 + c;
-                    if (row >= p.M || col >= p.N) continue;
-                    float* dst = cbase + (long long)row * p.ldc + col;
-                    if (p.vec && col + 4 <= p.N) {
-                        *reinterpret_cast<uint4*>(dst) = pc[c];
-                    } else {
-                        const uint32_t v[4] = {pc[c].x, pc[c].y, pc[c].z, pc[c].w};
-                        for (int e = 0; e < 4 && col + e < p.N; ++e) dst[e] = __uint_as_float(v[e]);
+                    for (int c = 0; c < 8; ++c) {
+                        const int row = row0 + c;
+                        if (row >= p.M || col >= p.N) continue;
+                        float* dst = cbase + (long long)row * p.ldc + col;
+                        if (col + 4 <= p.N) {
+                            *reinterpret_cast<uint4*>(dst) = pc[c];
+                        } else {
+                            const uint32_t v[4] = {pc[c].x, pc[c].y, pc[c].z, pc[c].w};
+                            for (int e = 0; e < 4 && col + e < p.N; ++e) dst[e] = __uint_as_float(v[e]);
+                        }
                     }
+                } else {
+                    // Rows on any 4-byte boundary (logits of an odd vocabulary, straight into the caller's tensor): 32 x 32 elements
+                    // turned round in the warp's own shared memory, a row per store instruction.  100 x 50257 x 192: 16 us, as
+                    // with padded rows, and the copy behind those took 11.
+                    float* turn = reinterpret_cast<float*>(smem + X_TURN) + (warp - 2) * X_TURN_FLOATS;
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) turn[lane * 33 + e] = o[e];
+                    __syncwarp();
+                    const int col = tn * XN + chunk * 32 + lane, first = tm * XM + lane_base;
+                    if (col < p.N) {
+#pragma unroll 8
+                        for (int r = 0; r < 32; ++r)
+                            if (first + r < p.M) cbase[(long long)(first + r) * p.ldc + col] = turn[r * 33 + lane];
+                    }
+                    __syncwarp();
                 }
             }
         }

@@ -267,13 +267,15 @@ __device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED>::run(
     for (int t = 0; t < STAGES - 1; ++t) fetch();
 
     // Pairs of products: neighbouring columns with B in MN order (a's element twice), even and odd k with B in K order.
-    constexpr bool PAIR_N = B_MN, PAIR_K = !B_MN && PM * PN <= 16;
+    // Tall patches with both operands in MN order pair rows instead: fewer doubled elements (0.89 of the FMA rate in a bare loop
+    // of 8 x 6, 0.81 with columns).
+    constexpr bool PAIR_M = A_MN && B_MN && PM >= 8, PAIR_N = B_MN && !PAIR_M, PAIR_K = !B_MN && PM * PN <= 16;
     constexpr bool AHEAD = B_MN || PM * PN <= 16;                   // registers for the next fragments as well
     constexpr int U = !AHEAD || (!A_MN && PM * PN <= 16) ? 4 : 2;
-    constexpr int PC = PAIR_N ? PN / 2 : PAIR_K ? PN : 1;
-    uint64_t acc2[PM][PC];
+    constexpr int PR = PAIR_M ? PM / 2 : PM, PC = PAIR_N ? PN / 2 : PAIR_K || PAIR_M ? PN : 1;
+    uint64_t acc2[PR][PC];
 #pragma unroll
-    for (int i = 0; i < PM; ++i)
+    for (int i = 0; i < PR; ++i)
 #pragma unroll
         for (int j = 0; j < PC; ++j) acc2[i][j] = 0;
     float acc[PM][PN];
@@ -322,6 +324,14 @@ __device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED>::run(
                             for (int i = 0; i < PM; ++i)
                                 acc2[i][j] = fma2(pack2(a[cur][kk][i], a[cur][kk + 1][i]), pack2(b[cur][kk][j], b[cur][kk + 1][j]), acc2[i][j]);
                     }
+                } else if constexpr (PAIR_M) {
+                    uint64_t bd[PN];
+#pragma unroll
+                    for (int j = 0; j < PN; ++j) bd[j] = pack2(b[cur][kk][j], b[cur][kk][j]);
+#pragma unroll
+                    for (int i = 0; i < PM / 2; ++i)
+#pragma unroll
+                        for (int j = 0; j < PN; ++j) acc2[i][j] = fma2(pack2(a[cur][kk][2 * i], a[cur][kk][2 * i + 1]), bd[j], acc2[i][j]);
                 } else if constexpr (PAIR_N) {
                     uint64_t ad[PM];
 #pragma unroll
@@ -343,9 +353,10 @@ __device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED>::run(
     cp_wait<0>();
     __syncthreads();                                                // operand stages are free: patches meet here
 #pragma unroll
-    for (int i = 0; i < PM; ++i)
+    for (int i = 0; i < PR; ++i)
 #pragma unroll
         for (int j = 0; j < PC; ++j) {
+            if constexpr (PAIR_M) unpack2(acc2[i][j], acc[2 * i][j], acc[2 * i + 1][j]);
             if constexpr (PAIR_N) unpack2(acc2[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
             if constexpr (PAIR_K) {
                 float even, odd;
@@ -501,6 +512,7 @@ __global__ void __launch_bounds__(GT * KS) gemm_f32_group_kernel(const __grid_co
 struct GemmPlan {
     int cfg;        // index into kVariants
     int parts, k_chunk;
+    double cost;    // cycles
 };
 
 // Tile variants with what was measured of them (cycles at 1.965 GHz, from products of several K in a graph): a
@@ -548,6 +560,7 @@ int cluster_capacity(deers_ctx* ctx) {
 GemmPlan plan_gemm(int n, const int* M, const int* N, int K, const int* capacity, int whole_heads) {
     GemmPlan best{};
     best.cfg = -1;
+    best.cost = 1e30;
     double best_cost = -1.0;
     const int steps = (K + BK - 1) / BK;
     for (int c = 0; c < 6; ++c) {
@@ -563,7 +576,7 @@ GemmPlan plan_gemm(int n, const int* M, const int* N, int K, const int* capacity
             const double cost = waves * chunk * v.walk + v.around + 1200.0 * (waves - 1.0) + (parts > 1 ? 3300.0 : 0.0);
             if (best_cost < 0.0 || cost < best_cost) {
                 best_cost = cost;
-                best.cfg = c; best.parts = parts; best.k_chunk = chunk * BK;
+                best.cost = cost; best.cfg = c; best.parts = parts; best.k_chunk = chunk * BK;
             }
         }
     }
@@ -656,24 +669,26 @@ int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long lo
 }
 
 // C = rmsnorm(A) * B with an optional rotation of the leading columns (see GemmNorm in common.cuh); M <= 65535 rows.
-int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, const float* b, float* c, int epi, float* aux, const GemmNorm& f) {
+int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, const float* b, float* c, int epi, float* aux, const GemmNorm& f,
+                         bool* rotated) {
+    *rotated = false;
     if (M == 0 || N == 0) return DEERS_OK;
     const int rc = cluster_capacity(ctx);
     if (rc) return rc;
-    const GemmPlan p = plan_gemm(1, &M, &N, K, ctx->cluster_capacity, f.rope_cols ? f.rope_d : 0);
-    if (p.cfg < 0) return DEERS_ERR_UNSUPPORTED;
+    GemmPlan p = plan_gemm(1, &M, &N, K, ctx->cluster_capacity, 0);
     GemmArgs g = gemm_args(M, N, K, a, K, b, N, c, N, epi, nullptr, 0, aux);
+    if (f.rope_cols && f.rope_d % 8 == 0) {
+        // A rotary launch of its own takes about 3000 cycles (1.5 us): rotate here unless tiles that hold whole heads cost more
+        // than that (heads of 48 columns leave 32 x 96 and 64 x 96 tiles: 231 x 576 x 192 takes 7.5 us in them, 3.6 in 32 x 32).
+        const GemmPlan w = plan_gemm(1, &M, &N, K, ctx->cluster_capacity, f.rope_d);
+        if (w.cfg >= 0 && w.cost < p.cost + 3000.0) {
+            p = w;
+            *rotated = true;
+            g.cosv = f.cosv; g.sinv = f.sinv; g.rope_cols = f.rope_cols; g.rope_d = f.rope_d; g.rope_t = f.rope_t;
+        }
+    }
     g.eps = f.eps; g.inv_n = (float)(1.0 / (double)K); g.inv = f.inv;
-    g.cosv = f.cosv; g.sinv = f.sinv; g.rope_cols = f.rope_cols; g.rope_d = f.rope_d; g.rope_t = f.rope_t;
     return launch_planned(ctx, p, g, 0, 1, true);
-}
-
-// Heads that a tile holds whole, with halves of whole 16-byte pieces.
-bool gemm_f32_can_rotate(int head_dim) {
-    if (head_dim % 8) return false;
-    for (const Variant& v : kVariants)
-        if (v.bn % head_dim == 0) return true;
-    return false;
 }
 
 // C_i = A_i^T B_i, A_i [K, M_i] and B_i [K, N_i] row-major, one K, in one launch.

@@ -58,7 +58,6 @@ struct deers_gpt {
     std::vector<LayerAct> la;
     LayerGrad lg[2];
     float* dtmp;
-    bool rotate_fused;           // heads fit the GEMM's tiles whole: no rotary launches of their own
     // second stream for the weight gradients; events are markers only (no timing)
     cudaStream_t side;
     cudaEvent_t ev_fork, ev_join, ev_done[2];
@@ -186,31 +185,40 @@ int forward(deers_gpt* m, const long long* ids, int B, int T, bool with_head_pai
     const long long N = (long long)B * T;
     float* W = m->arena[0];
     for (bool& v : m->done_valid) v = false;
-    if (m->tc_head && with_head_pair) {
-        // the head weight's f16 pair (it changes every step) is made beside the blocks, not in front of the head
+    GPT_TRY(launch_embedding_fwd(ctx, W + m->off_wte, ids, N, C, V, m->x0));                 // gpt.rs:343
+    // Beside the blocks, which leave most of the memory bandwidth idle: the head weight's f16 pair (it changes every step) and the
+    // cleared gradient of the embedding (its backward adds rows).  Behind the first product: SMs set up for kernels without
+    // shared memory have to empty before a product can start on them (10 us at the head of a step).
+    auto beside = [&]() -> int {
+        const bool make_pair = m->tc_head && with_head_pair;
+        if (!make_pair && !keep) return DEERS_OK;
         SideScope side(m);
         GPT_TRY(side.rc);
-        GPT_TRY(launch_split_f16x3(ctx, C, V, W + m->off_lm, m->Vld, 1.0f, m->w_hi, m->w_lo, m->Vld));
-        GPT_TRY(side.done(0));
-    }
-    GPT_TRY(launch_embedding_fwd(ctx, W + m->off_wte, ids, N, C, V, m->x0));                 // gpt.rs:343
+        if (make_pair) GPT_TRY(launch_split_f16x3(ctx, C, V, W + m->off_lm, m->Vld, 1.0f, m->w_hi, m->w_lo, m->Vld));
+        if (keep) DEERS_CUDA_TRY(ctx, cudaMemsetAsync(m->arena[1] + m->off_wte, 0, (size_t)V * C * sizeof(float), ctx->stream));
+        return side.done(0);
+    };
     deers_attn_desc ad;
     attn_desc(m, B, T, &ad);
+    if (c.n_layer == 0) GPT_TRY(beside());
     const float* x = m->x0;
     for (int l = 0; l < c.n_layer; ++l) {
         const LayerW& w = m->lw[l];
         LayerAct& a = m->la[l];
         GemmNorm f = norm_in(m, keep ? a.inv1 : nullptr);
-        if (m->rotate_fused) { f.cosv = m->cosv; f.sinv = m->sinv; f.rope_cols = 2 * C; f.rope_d = m->D; f.rope_t = T; }   // gpt.rs:135-136
-        GPT_TRY(launch_gemm_f32_norm(ctx, (int)N, 3 * C, C, x, W + w.qkv, a.qkv, DEERS_EPI_NONE, nullptr, f));   // norm1, q | k | v projections
-        if (!m->rotate_fused) GPT_TRY(rotate_in_place(m, B, T, 0, a.qkv));
+        f.cosv = m->cosv; f.sinv = m->sinv; f.rope_cols = 2 * C; f.rope_d = m->D; f.rope_t = T;             // gpt.rs:135-136
+        bool rotated;
+        GPT_TRY(launch_gemm_f32_norm(ctx, (int)N, 3 * C, C, x, W + w.qkv, a.qkv, DEERS_EPI_NONE, nullptr, f, &rotated));   // norm1, q | k | v projections
+        if (l == 0) GPT_TRY(beside());
+        if (!rotated) GPT_TRY(rotate_in_place(m, B, T, 0, a.qkv));
         GPT_TRY(deers_b200_attn_fwd(ctx, &ad, a.qkv, a.qkv + C, a.qkv + 2 * C, a.o, a.lse, nullptr, 0));
         GPT_TRY(gemm(m, (int)N, C, C, a.o, C, 0, W + w.out, C, 1, a.x1, C, DEERS_EPI_ADD, x, C));       // x + out_proj
         GPT_TRY(launch_gemm_f32_norm(ctx, (int)N, Hm, C, a.x1, W + w.up, a.h, DEERS_EPI_RELU_SQ, keep ? a.r : nullptr,
-                                     norm_in(m, keep ? a.inv2 : nullptr)));                  // norm2, up_proj, relu^2
+                                     norm_in(m, keep ? a.inv2 : nullptr), &rotated));        // norm2, up_proj, relu^2
         GPT_TRY(gemm(m, (int)N, C, Hm, a.h, Hm, 0, W + w.down, C, 1, a.x2, C, DEERS_EPI_ADD, a.x1, C)); // x1 + down_proj
         x = a.x2;
     }
+    GPT_TRY(wait_done(m, 0));
     if (m->tc_head) {
         // lm_head on the tensor core at f32 accuracy: both operands as f16 pairs (the weight changes every step); gpt.rs:347
         int rc = launch_rmsnorm_split(ctx, N, C, c.rms_norm_eps, x, m->invf, m->xf_hi, m->xf_lo);
@@ -219,7 +227,6 @@ int forward(deers_gpt* m, const long long* ids, int B, int T, bool with_head_pai
             rc = launch_split_f16x3(ctx, N, C, m->xf, C, 1.0f, m->xf_hi, m->xf_lo, C);
         }
         GPT_TRY(rc);
-        GPT_TRY(wait_done(m, 0));
         GPT_TRY(launch_gemm_f16x3(ctx, (int)N, V, C, m->xf_hi, m->xf_lo, C, 0, m->w_hi, m->w_lo, m->Vld, 1, logits, ldl,
                                   1.0f, m->x3_ws, m->x3_ws_bytes));
     } else {
@@ -278,8 +285,8 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
         // attention branch: x1 = x + attn(rmsnorm(x)) Wout
         GPT_TRY(gemm(m, (int)N, C, C, d.dx1, C, 0, W + w.out, C, 0, m->dtmp, C));            // d o (token-major)
         GPT_TRY(launch_attn_bwd_f32(ctx, &ad, a.qkv, a.qkv + C, a.qkv + 2 * C, a.o, a.lse, m->dtmp, d.dqkv, d.dqkv + C, d.dqkv + 2 * C,
-                                    m->rotate_fused ? m->cosv : nullptr, m->rotate_fused ? m->sinv : nullptr));
-        if (!m->rotate_fused) GPT_TRY(rotate_in_place(m, B, T, 1, d.dqkv));
+                                    m->D % 8 ? nullptr : m->cosv, m->D % 8 ? nullptr : m->sinv));
+        if (m->D % 8) GPT_TRY(rotate_in_place(m, B, T, 1, d.dqkv));
         GPT_TRY(gemm(m, (int)N, C, 3 * C, d.dqkv, 3 * C, 0, W + w.qkv, 3 * C, 0, m->dtmp, C)); // d n1 (three terms in one)
         GPT_TRY(wait_done(m, (l & 1) ^ 1));                                                  // the block above has read what this block's input gradient replaces
         GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, x_in, a.inv1, m->dtmp, d.dx1, below.dx, d.n1)); // d x
@@ -293,7 +300,7 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
             GPT_TRY(side.done(l & 1));
         }
     }
-    GPT_TRY(launch_embedding_bwd(ctx, dx0, ids, N, C, V, G + m->off_wte));
+    GPT_TRY(launch_embedding_bwd(ctx, dx0, ids, N, C, V, G + m->off_wte, true));           // (cleared in the forward)
     return join_side(m);
 }
 
@@ -307,9 +314,25 @@ int check_bt(const deers_gpt* m, int B, int T) {
     return DEERS_OK;
 }
 
+// n ids and n targets in one launch.
+__global__ void __launch_bounds__(256) stage_ids_kernel(const long long* ids, const long long* targets, long long n, long long* __restrict__ ids_out,
+                                                        long long* __restrict__ targets_out) {
+    chain_begin();
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const long long a = ids[i], b = targets[i];
+        ids_out[i] = a; targets_out[i] = b;
+    }
+}
+
 // Brings the caller's ids / targets into the model's own buffers, so that a captured graph reads fixed addresses.
 int stage_ids(deers_gpt* m, const int64_t* ids, const int64_t* targets, long long N, cudaMemcpyKind kind) {
     deers_ctx* ctx = m->ctx;
+    if (kind == cudaMemcpyDeviceToDevice && targets && (const long long*)ids != m->ids_dev && (const long long*)targets != m->tgt_dev) {
+        const unsigned grid = (unsigned)((N + 255) / 256);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, stage_ids_kernel, grid, 256, 0, 1, (const long long*)ids, (const long long*)targets, N, m->ids_dev, m->tgt_dev));
+        ctx->launches += 1;
+        return DEERS_OK;
+    }
     if ((const long long*)ids != m->ids_dev)
         DEERS_CUDA_TRY(ctx, cudaMemcpyAsync(m->ids_dev, ids, (size_t)N * sizeof(long long), kind, ctx->stream));
     if (targets && (const long long*)targets != m->tgt_dev)
@@ -435,7 +458,6 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
     m->tc_head = cfg->vocab_size >= 1024 && cfg->n_embd % 8 == 0 && cfg->n_embd >= 64;
     m->graph_enabled = true; m->graph_exec = nullptr; m->graph_B = m->graph_T = -1; m->eager_steps_BT = 0;
     m->on_side = false;
-    m->rotate_fused = gemm_f32_can_rotate(D);
     m->head_pair_current = m->captured_updates = false;
     {
         // the weight-gradient stream and its markers; without them the step simply runs on one stream
@@ -632,10 +654,12 @@ extern "C" int deers_b200_gpt_forward(deers_gpt* m, const int64_t* ids, int32_t 
     deers_ctx* ctx = m->ctx;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     const bool rec = recording(m), kept = m->head_pair_current && !m->captured_updates && !rec;
-    GPT_TRY(forward(m, (const long long*)ids, B, T, !kept, false, m->logits, m->Vld));
+    const int V = m->cfg.vocab_size;
+    // The tensor-core head writes the caller's dense rows itself; the small head's 16-byte stores want padded ones.
+    const bool direct = logits && m->tc_head;
+    GPT_TRY(forward(m, (const long long*)ids, B, T, !kept, false, direct ? logits : m->logits, direct ? V : m->Vld));
     if (!rec) m->head_pair_current = m->tc_head;
-    if (logits) {
-        const int V = m->cfg.vocab_size;
+    if (logits && !direct) {
         const dim3 grid((unsigned)((V + 4095) / 4096), (unsigned)(B * T));
         DEERS_CUDA_TRY(ctx, launch_chained(ctx, copy_logits_kernel, grid, 256, 0, 1, m->logits, m->Vld, logits, V));
         ctx->launches += 1;
@@ -658,12 +682,13 @@ extern "C" int deers_b200_gpt_forward_backward(deers_gpt* m, const int64_t* ids,
     return DEERS_OK;
 }
 
-static int train_step_common(deers_gpt* m, int B, int T, const deers_adamw_hyper* hyper, double max_grad_norm) {
+static int train_step_common(deers_gpt* m, int B, int T, const deers_adamw_hyper* hyper, double max_grad_norm,
+                             float* loss_out, float* norm_out) {
     GPT_TRY(run_fwd_bwd(m, B, T, true));
     m->head_pair_current = false;                                     // the update below changes the head weight
     m->captured_updates = m->captured_updates || recording(m);
     // clip_grad_norm + step_with_grads; "if grad_norm.is_finite() { step }" of tinystories_train.rs:213-216
-    return launch_adamw(m->ctx, (int)m->opt.size(), m->opt.data(), hyper, m->norm_dev, max_grad_norm, true);
+    return launch_adamw(m->ctx, (int)m->opt.size(), m->opt.data(), hyper, m->norm_dev, max_grad_norm, true, StepSaid{m->loss_dev, loss_out, norm_out});
 }
 
 extern "C" int deers_b200_gpt_train_step(deers_gpt* m, const int64_t* ids, const int64_t* targets, int32_t B, int32_t T,
@@ -675,12 +700,7 @@ extern "C" int deers_b200_gpt_train_step(deers_gpt* m, const int64_t* ids, const
     deers_ctx* ctx = m->ctx;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     GPT_TRY(stage_ids(m, ids, targets, (long long)B * T, cudaMemcpyDeviceToDevice));
-    GPT_TRY(train_step_common(m, B, T, hyper, max_grad_norm));
-    if (loss_dev)
-        DEERS_CUDA_TRY(ctx, cudaMemcpyAsync(loss_dev, m->loss_dev, sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
-    if (grad_norm_dev)
-        DEERS_CUDA_TRY(ctx, cudaMemcpyAsync(grad_norm_dev, m->norm_dev, sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
-    return DEERS_OK;
+    return train_step_common(m, B, T, hyper, max_grad_norm, loss_dev, grad_norm_dev);
 }
 
 extern "C" int deers_b200_gpt_train_step_host(deers_gpt* m, const int64_t* ids_host, const int64_t* targets_host, int32_t B,
@@ -695,7 +715,7 @@ extern "C" int deers_b200_gpt_train_step_host(deers_gpt* m, const int64_t* ids_h
     memcpy(m->ids_pin, ids_host, (size_t)N * sizeof(long long));
     memcpy(m->ids_pin + m->max_tokens, targets_host, (size_t)N * sizeof(long long));
     GPT_TRY(stage_ids(m, (const int64_t*)m->ids_pin, (const int64_t*)(m->ids_pin + m->max_tokens), N, cudaMemcpyHostToDevice));
-    GPT_TRY(train_step_common(m, B, T, hyper, max_grad_norm));
+    GPT_TRY(train_step_common(m, B, T, hyper, max_grad_norm, nullptr, nullptr));
     DEERS_CUDA_TRY(ctx, cudaMemcpyAsync(m->out_pin, m->loss_dev, 2 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     const int rc = deers_b200_sync(ctx);
     if (loss_host) *loss_host = m->out_pin[0];

@@ -283,8 +283,8 @@ int launch_embedding_fwd(deers_ctx* ctx, const float* weight, const long long* i
 }
 
 int launch_embedding_bwd(deers_ctx* ctx, const float* dout, const long long* ids, long long n_ids, int C, long long V,
-                         float* dweight) {
-    DEERS_CUDA_TRY(ctx, cudaMemsetAsync(dweight, 0, (size_t)V * C * sizeof(float), ctx->stream));
+                         float* dweight, bool cleared) {
+    if (!cleared) DEERS_CUDA_TRY(ctx, cudaMemsetAsync(dweight, 0, (size_t)V * C * sizeof(float), ctx->stream));
     if (n_ids == 0) return DEERS_OK;
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);

@@ -44,6 +44,7 @@ struct OptScalars {                     // f64 hyper-parameters rounded to f32 w
     int use_clip;
     int skip_nonfinite;                 // leave w, m, v untouched when the norm is not finite
     double max_norm;
+    StepSaid said;                      // MODE_STEP: loss and norm for the caller (the first launch of a call; null pointers: nobody asks)
 };
 
 __device__ __forceinline__ int find_tensor(const OptTensors& t, int chunk) {
@@ -140,6 +141,10 @@ template <int MODE>
 __global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ OptTensors t, const __grid_constant__ OptScalars s,
                                                     const float* norm) {
     chain_wait();
+    if (MODE == MODE_STEP && blockIdx.x == 0 && threadIdx.x == 0) {
+        if (s.said.loss_out) *s.said.loss_out = *s.said.loss;
+        if (s.said.norm_out) *s.said.norm_out = *norm;
+    }
     float scale;
     const bool clip = clip_scale(s, norm, scale);
     if (MODE == MODE_CLIP && !clip) return;
@@ -283,7 +288,7 @@ extern "C" int deers_b200_grad_norm(deers_ctx* ctx, int n_tensors, const deers_o
     return DEERS_OK;
 }
 
-static int optim_apply(deers_ctx* ctx, int n_tensors, const deers_optim_tensor* tensors, const OptScalars& s,
+static int optim_apply(deers_ctx* ctx, int n_tensors, const deers_optim_tensor* tensors, OptScalars s,
                        const float* norm_dev, int mode) {
     for (int first = 0; first < n_tensors;) {
         OptTensors t;
@@ -298,6 +303,7 @@ static int optim_apply(deers_ctx* ctx, int n_tensors, const deers_optim_tensor* 
             else DEERS_CUDA_TRY(ctx, launch_chained(ctx, adamw_kernel<MODE_CLIP>, grid, 256, 0, 1, t, s, norm_dev));
         }
         ctx->launches += 1;
+        s.said = StepSaid{};
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     return DEERS_OK;
@@ -322,7 +328,7 @@ extern "C" int deers_b200_adamw_step(deers_ctx* ctx, int n_tensors, const deers_
 }
 
 int launch_adamw(deers_ctx* ctx, int n_tensors, const deers_optim_tensor* tensors, const deers_adamw_hyper* h,
-                 const float* norm_dev, double max_norm, bool skip_nonfinite) {
+                 const float* norm_dev, double max_norm, bool skip_nonfinite, const StepSaid& said) {
     if (!ctx || !h) return DEERS_ERR_NULL;
     if (h->step < 1) return DEERS_ERR_SHAPE;
     if (norm_dev && !(max_norm > 0.0) && !skip_nonfinite) return DEERS_ERR_SHAPE;
@@ -343,5 +349,6 @@ int launch_adamw(deers_ctx* ctx, int n_tensors, const deers_optim_tensor* tensor
     s.use_clip = (norm_dev && max_norm > 0.0) ? 1 : 0;
     s.skip_nonfinite = (skip_nonfinite && norm_dev) ? 1 : 0;
     s.max_norm = max_norm;
+    s.said = said;
     return optim_apply(ctx, n_tensors, tensors, s, norm_dev, MODE_STEP);
 }
