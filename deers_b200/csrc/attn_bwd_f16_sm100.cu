@@ -155,11 +155,43 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tme
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_x16(taddr, r); }
 
 
+// The part of the start that needs nothing of global memory (see started()).
+template <int D>
+__device__ __forceinline__ void attn_bwd_dkdv_f16_prologue(const void* tmap_q, const void* tmap_k, const void* tmap_v, const void* tmap_do) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    constexpr int NCW = 4 * DKV_NWG;                        // compute warps (arrivals are one per warp)
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + DkvSmem<D>::BARS);
+    uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + A_COUNT);
+    if (threadIdx.x == 0) {
+        tmem_base_s[1] = 0;                                     // the abort flag
+        mbar_init(&bars[A_KV_FULL], 1);
+        mbar_init(&bars[A_KV_EMPTY], 1);
+        for (int s = 0; s < 3; ++s) { mbar_init(&bars[A_Q_FULL + s], 1); mbar_init(&bars[A_Q_EMPTY + s], 1); }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&bars[A_DO_FULL + s], 1); mbar_init(&bars[A_DO_EMPTY + s], 1);
+            mbar_init(&bars[A_ST_FULL + s], NCW);
+            mbar_init(&bars[A_S + s], 1); mbar_init(&bars[A_P + s], NCW); mbar_init(&bars[A_P2 + s], NCW);
+            mbar_init(&bars[A_DST + s], NCW);
+        }
+        mbar_init(&bars[A_DP], 1);
+        mbar_init(&bars[A_DS], NCW);
+        mbar_init(&bars[A_DONE], 1);
+        mbar_init(&bars[A_ACC_FREE], NCW);
+        fence_barrier_init();
+        tma_prefetch_desc(tmap_q); tma_prefetch_desc(tmap_k); tma_prefetch_desc(tmap_v); tma_prefetch_desc(tmap_do);
+    }
+    if (uniform((int)threadIdx.x / 32) == 1) {
+        tmem_alloc(tmem_base_s, 512);
+        tmem_relinquish();
+    }
+}
+
 template <int D>
 __global__ void __launch_bounds__(DKV_THREADS, 1)
 attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                          const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                          const BwdParams p) {
+    attn_bwd_dkdv_f16_prologue<D>(&tmap_q, &tmap_k, &tmap_v, &tmap_do);
     chain_wait();
     using L = DkvSmem<D>;
     constexpr uint32_t TILE_BYTES = L::TILE;
@@ -190,39 +222,10 @@ attn_bwd_dkdv_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     const int nq = (p.T + BT - 1) / BT;
     const int n_items = p.B * p.H * nq;
 
-    if (threadIdx.x == 0) {
-        *abort_s = 0;
-        uint32_t skip = (*(volatile unsigned int*)p.err != 0) ? 1u : 0u;   // an earlier CTA gave up
-        if ((smem_u32(smem) & 1023u) != 0) {
-            atomicCAS(p.err, 0u, DEERS_KERR_BWD_F16 | 0x20);
-            skip = 1;
-        }
-        *skip_s = skip;
-        mbar_init(&bars[A_KV_FULL], 1);
-        mbar_init(&bars[A_KV_EMPTY], 1);
-        for (int s = 0; s < 3; ++s) { mbar_init(&bars[A_Q_FULL + s], 1); mbar_init(&bars[A_Q_EMPTY + s], 1); }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(&bars[A_DO_FULL + s], 1); mbar_init(&bars[A_DO_EMPTY + s], 1);
-            mbar_init(&bars[A_ST_FULL + s], NCW);
-            mbar_init(&bars[A_S + s], 1); mbar_init(&bars[A_P + s], NCW); mbar_init(&bars[A_P2 + s], NCW);
-            mbar_init(&bars[A_DST + s], NCW);
-        }
-        mbar_init(&bars[A_DP], 1);
-        mbar_init(&bars[A_DS], NCW);
-        mbar_init(&bars[A_DONE], 1);
-        mbar_init(&bars[A_ACC_FREE], NCW);
-        fence_barrier_init();
-        tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v); tma_prefetch_desc(&tmap_do);
+    if (!started(smem, skip_s, p.err, DEERS_KERR_BWD_F16 | 0x20)) {
+        if (warp == 1) tmem_dealloc(*tmem_base_s, 512);
+        return;
     }
-    __syncthreads();
-    if (*skip_s) return;
-    if (warp == 1) {
-        tmem_alloc(tmem_base_s, TMEM_COLS);
-        tmem_relinquish();
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
     const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 
@@ -894,9 +897,30 @@ struct DqsSmem {
 
 enum DqsBar { R_FULL = 0, R_EMPTY = 3, R_ACC_FULL = 6, R_ACC_EMPTY = 8, R_COUNT = 10 };
 
+// The part of the start that needs nothing of global memory (see started()).
+template <int D>
+__device__ __forceinline__ void attn_bwd_dq_from_ds_f16_prologue(const void* tmap_k) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    using L = DqsSmem<D>;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BARS);
+    uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + R_COUNT);
+    if (threadIdx.x == 0) {
+        tmem_base_s[1] = 0;                                     // the abort flag
+        for (int s = 0; s < L::STAGES; ++s) { mbar_init(&bars[R_FULL + s], 1); mbar_init(&bars[R_EMPTY + s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&bars[R_ACC_FULL + s], 1); mbar_init(&bars[R_ACC_EMPTY + s], 128); }
+        fence_barrier_init();
+        tma_prefetch_desc(tmap_k);
+    }
+    if (uniform((int)threadIdx.x / 32) == 1) {
+        tmem_alloc(tmem_base_s, 2 * D);
+        tmem_relinquish();
+    }
+}
+
 template <int D>
 __global__ void __launch_bounds__(192, 1)
 attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const BwdParams p) {
+    attn_bwd_dq_from_ds_f16_prologue<D>(&tmap_k);
     chain_wait();
     using L = DqsSmem<D>;
     constexpr int DBLK = D / 64;
@@ -912,28 +936,10 @@ attn_bwd_dq_from_ds_f16_kernel(const __grid_constant__ CUtensorMap tmap_k, const
     const int nq = (p.T + BT - 1) / BT;
     const int n_items = p.B * p.H * nq;
 
-    if (threadIdx.x == 0) {
-        *abort_s = 0;
-        uint32_t skip = (*(volatile unsigned int*)p.err != 0) ? 1u : 0u;
-        if ((smem_u32(smem) & 1023u) != 0) {
-            atomicCAS(p.err, 0u, DEERS_KERR_BWD_F16 | 0x20);
-            skip = 1;
-        }
-        *skip_s = skip;
-        for (int s = 0; s < L::STAGES; ++s) { mbar_init(&bars[R_FULL + s], 1); mbar_init(&bars[R_EMPTY + s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&bars[R_ACC_FULL + s], 1); mbar_init(&bars[R_ACC_EMPTY + s], 128); }
-        fence_barrier_init();
-        tma_prefetch_desc(&tmap_k);
+    if (!started(smem, skip_s, p.err, DEERS_KERR_BWD_F16 | 0x20)) {
+        if (warp == 1) tmem_dealloc(*tmem_base_s, 2 * D);
+        return;
     }
-    __syncthreads();
-    if (*skip_s) return;
-    if (warp == 1) {
-        tmem_alloc(tmem_base_s, TMEM_COLS);
-        tmem_relinquish();
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
     const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 

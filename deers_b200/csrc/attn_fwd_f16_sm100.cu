@@ -138,10 +138,40 @@ struct WorkCursor {
     }
 };
 
+// The part of the start that needs nothing of global memory (see started()).
+template <int D>
+__device__ __forceinline__ void attn_fwd_f16_prologue(const void* tmap_q, const void* tmap_k, const void* tmap_v) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FwdSmem<D>::BARS);
+    uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + F_COUNT);
+    if (threadIdx.x == 0) {
+        tmem_base_s[1] = 0;                                     // the abort flag
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&bars[F_Q_FULL + s], 1); mbar_init(&bars[F_Q_EMPTY + s], 1);
+            mbar_init(&bars[F_K_FULL + s], 1);
+            mbar_init(&bars[F_V_FULL + s], 1);
+            mbar_init(&bars[F_O_DONE + s], 1); mbar_init(&bars[F_O_FREE + s], 4 * NWG);
+            mbar_init(&bars[F_XCH + s], 8); mbar_init(&bars[F_MREF + s], 4);
+        }
+        for (int s = 0; s < 3; ++s) {
+            mbar_init(&bars[F_S_FULL + s], 1); mbar_init(&bars[F_PV_DONE + s], 1);
+            mbar_init(&bars[F_P_FULL + s], 8); mbar_init(&bars[F_P2_FULL + s], 8); // one arrival per warp of the step's group
+        }
+        mbar_init(&bars[F_LX], 4 * NWG);
+        fence_barrier_init();
+        tma_prefetch_desc(tmap_q); tma_prefetch_desc(tmap_k); tma_prefetch_desc(tmap_v);
+    }
+    if (uniform((int)threadIdx.x / 32) == 1) {
+        tmem_alloc(tmem_base_s, 512);
+        tmem_relinquish();
+    }
+}
+
 template <int D>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const FwdParams p) {
+    attn_fwd_f16_prologue<D>(&tmap_q, &tmap_k, &tmap_v);
     chain_wait();
     using L = FwdSmem<D>;
     constexpr uint32_t TILE_BYTES = L::TILE;
@@ -169,38 +199,10 @@ attn_fwd_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const int nq = (p.T + BM - 1) / BM;
     const int n_items = p.B * p.H * nq;
 
-    if (threadIdx.x == 0) {
-        *abort_s = 0;
-        uint32_t skip = (*(volatile unsigned int*)p.err != 0) ? 1u : 0u;   // an earlier CTA gave up: exit at once
-        if ((smem_u32(smem) & 1023u) != 0) {
-            atomicCAS(p.err, 0u, DEERS_KERR_FWD_F16 | 0x20);
-            skip = 1;
-        }
-        *skip_s = skip;
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(&bars[F_Q_FULL + s], 1); mbar_init(&bars[F_Q_EMPTY + s], 1);
-            mbar_init(&bars[F_K_FULL + s], 1);
-            mbar_init(&bars[F_V_FULL + s], 1);
-            mbar_init(&bars[F_O_DONE + s], 1); mbar_init(&bars[F_O_FREE + s], 4 * NWG);
-            mbar_init(&bars[F_XCH + s], 8); mbar_init(&bars[F_MREF + s], 4);
-        }
-        for (int s = 0; s < 3; ++s) {
-            mbar_init(&bars[F_S_FULL + s], 1); mbar_init(&bars[F_PV_DONE + s], 1);
-            mbar_init(&bars[F_P_FULL + s], 8); mbar_init(&bars[F_P2_FULL + s], 8); // one arrival per warp of the step's group
-        }
-        mbar_init(&bars[F_LX], 4 * NWG);
-        fence_barrier_init();
-        tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v);
+    if (!started(smem, skip_s, p.err, DEERS_KERR_FWD_F16 | 0x20)) {
+        if (warp == 1) tmem_dealloc(*tmem_base_s, 512);
+        return;
     }
-    __syncthreads();
-    if (*skip_s) return;
-    if (warp == 1) {
-        tmem_alloc(tmem_base_s, TMEM_COLS);
-        tmem_relinquish();
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
     const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 

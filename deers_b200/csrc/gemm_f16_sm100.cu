@@ -52,11 +52,32 @@ struct GemmParams {
     unsigned int* err;
 };
 
+// The part of the start that needs nothing of global memory (see started()).
+template <int GN>
+__device__ __forceinline__ void gemm_f16_prologue(const void* tmap_a, const void* tmap_b) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + G_STAGES * (G_A_BYTES + GN * GK * 2));
+    uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + G_COUNT);
+    if (threadIdx.x == 0) {
+        tmem_base_s[1] = 0;                                     // the abort flag
+        tmem_base_s[3] = 0;                                     // epilogue threads whose rows are parked
+        for (int s = 0; s < G_STAGES; ++s) { mbar_init(&bars[G_FULL + s], 1); mbar_init(&bars[G_EMPTY + s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&bars[G_ACC_FULL + s], 1); mbar_init(&bars[G_ACC_EMPTY + s], 128); }
+        fence_barrier_init();
+        tma_prefetch_desc(tmap_a); tma_prefetch_desc(tmap_b);
+    }
+    if (uniform((int)threadIdx.x / 32) == 1) {
+        tmem_alloc(tmem_base_s, 512);
+        tmem_relinquish();
+    }
+}
+
 // SPLIT: one tile per cluster, whose CTAs take a share of K each; the partial tiles meet in distributed shared memory and are
 // added in the order of their K ranges (reproducible, no workspace).
 template <int A_MN, int B_MN, int GN, bool SPLIT>
 __global__ void __launch_bounds__(G_THREADS, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+    gemm_f16_prologue<GN>(&tmap_a, &tmap_b);
     chain_wait();
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr uint32_t G_B_BYTES = GN * GK * 2;
@@ -76,31 +97,12 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     const int kb0 = part * p.kb_chunk, kb1 = SPLIT ? min(kb_all, kb0 + p.kb_chunk) : kb_all;   // this CTA's K blocks: never none
     const int t0 = SPLIT ? (int)blockIdx.x / parts : (int)blockIdx.x, t_step = SPLIT ? n_tiles : (int)gridDim.x;
 
-    if (threadIdx.x == 0) {
-        *abort_s = 0;
-        uint32_t skip = (*(volatile unsigned int*)p.err != 0) ? 1u : 0u;
-        if ((smem_u32(smem) & 1023u) != 0) {
-            atomicCAS(p.err, 0u, DEERS_KERR_GEMM | 0x20);
-            skip = 1;
-        }
-        *skip_s = skip;
-        skip_s[1] = 0;
-        for (int s = 0; s < G_STAGES; ++s) { mbar_init(&bars[G_FULL + s], 1); mbar_init(&bars[G_EMPTY + s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&bars[G_ACC_FULL + s], 1); mbar_init(&bars[G_ACC_EMPTY + s], 128); }
-        fence_barrier_init();
-        tma_prefetch_desc(&tmap_a); tma_prefetch_desc(&tmap_b);
-    }
-    __syncthreads();
     // (a split-K CTA stays: its peers read its shared memory)
-    const bool skip = *skip_s != 0;
-    if (!SPLIT && skip) return;
-    if (warp == 1) {
-        tmem_alloc(tmem_base_s, 512);
-        tmem_relinquish();
+    const bool skip = !started(smem, skip_s, p.err, DEERS_KERR_GEMM | 0x20);
+    if (!SPLIT && skip) {
+        if (warp == 1) tmem_dealloc(*tmem_base_s, 512);
+        return;
     }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
     const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 

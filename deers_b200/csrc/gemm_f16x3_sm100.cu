@@ -51,10 +51,30 @@ struct X3Params {
     unsigned int* err;
 };
 
+// The part of the start that needs nothing of global memory (see started()).
+template <int A_MN, int B_MN>
+__device__ __forceinline__ void gemm_f16x3_prologue(const void* tm_ah, const void* tm_al, const void* tm_bh, const void* tm_bl) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + X_STAGES * X_STAGE);
+    uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + X_COUNT);
+    if (threadIdx.x == 0) {
+        tmem_base_s[1] = 0;                                     // the abort flag
+        for (int s = 0; s < X_STAGES; ++s) { mbar_init(&bars[X_FULL + s], 1); mbar_init(&bars[X_EMPTY + s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&bars[X_ACC_FULL + s], 1); mbar_init(&bars[X_ACC_EMPTY + s], 128 * X_EPI_WG); }
+        fence_barrier_init();
+        tma_prefetch_desc(tm_ah); tma_prefetch_desc(tm_al); tma_prefetch_desc(tm_bh); tma_prefetch_desc(tm_bl);
+    }
+    if (uniform((int)threadIdx.x / 32) == 1) {
+        tmem_alloc(tmem_base_s, 512);
+        tmem_relinquish();
+    }
+}
+
 template <int A_MN, int B_MN>
 __global__ void __launch_bounds__(X_THREADS, 1)
 gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_constant__ CUtensorMap tm_al,
                   const __grid_constant__ CUtensorMap tm_bh, const __grid_constant__ CUtensorMap tm_bl, const X3Params p) {
+    gemm_f16x3_prologue<A_MN, B_MN>(&tm_ah, &tm_al, &tm_bh, &tm_bl);
     chain_wait();
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + X_STAGES * X_STAGE);
@@ -66,28 +86,10 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_consta
     const int tiles_m = (p.M + XM - 1) / XM, tiles_n = (p.N + XN - 1) / XN;
     const int n_units = tiles_m * tiles_n * p.parts;
 
-    if (threadIdx.x == 0) {
-        *abort_s = 0;
-        uint32_t skip = (*(volatile unsigned int*)p.err != 0) ? 1u : 0u;
-        if ((smem_u32(smem) & 1023u) != 0) {
-            atomicCAS(p.err, 0u, DEERS_KERR_GEMM | 0x21);
-            skip = 1;
-        }
-        *skip_s = skip;
-        for (int s = 0; s < X_STAGES; ++s) { mbar_init(&bars[X_FULL + s], 1); mbar_init(&bars[X_EMPTY + s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&bars[X_ACC_FULL + s], 1); mbar_init(&bars[X_ACC_EMPTY + s], 128 * X_EPI_WG); }
-        fence_barrier_init();
-        tma_prefetch_desc(&tm_ah); tma_prefetch_desc(&tm_al); tma_prefetch_desc(&tm_bh); tma_prefetch_desc(&tm_bl);
+    if (!started(smem, skip_s, p.err, DEERS_KERR_GEMM | 0x21)) {
+        if (warp == 1) tmem_dealloc(*tmem_base_s, 512);
+        return;
     }
-    __syncthreads();
-    if (*skip_s) return;
-    if (warp == 1) {
-        tmem_alloc(tmem_base_s, 512);
-        tmem_relinquish();
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
     const uint32_t tmem = (uint32_t)uniform((int)*tmem_base_s);
     WaitState ws{abort_s, p.err};
 

@@ -160,6 +160,24 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 
+// A persistent tcgen05 kernel starts in two parts.  Before it waits for its predecessor it sets up its barriers (thread 0) and
+// takes its tensor memory (warp 1), which touch nothing of global memory; behind the wait this joins the two and looks at the
+// error word: false (for the whole CTA) when an earlier kernel gave up, or the shared memory is not 1024-byte aligned.
+__device__ __forceinline__ bool started(const void* smem, uint32_t* skip_s, unsigned int* err, uint32_t code) {
+    if (threadIdx.x == 0) {
+        uint32_t skip = (*(volatile unsigned int*)err != 0) ? 1u : 0u;
+        if ((smem_u32(smem) & 1023u) != 0) {
+            atomicCAS(err, 0u, code);
+            skip = 1;
+        }
+        *skip_s = skip;
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    return *skip_s == 0;
+}
+
 // ---------------------------------------------------------------------------
 // tcgen05.mma operand descriptors
 // ---------------------------------------------------------------------------
