@@ -22,8 +22,6 @@
 namespace {
 
 constexpr int BM = 32;        // stationary rows per block
-constexpr int NG = 4;         // groups of 64 threads per block
-constexpr int NT = 64 * NG;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LN2 = 0.6931471805599453f;
 
@@ -250,9 +248,10 @@ __device__ __forceinline__ void store4(float* p, float4 v, int valid, int vec) {
     if (valid > 3) p[3] = v.w;
 }
 
-// FBN: rows of a tile streamed in the forward
-template <int DP, int FBN = 32>
+// NG: groups of 64 threads per block; FBN: rows of a tile streamed in the forward
+template <int DP, int NG = 4, int FBN = 32>
 struct Tile {
+    static constexpr int NT = 64 * NG;
     static constexpr int BN = FBN;
     static constexpr int NC = BN / 8;                           // score columns per thread
     static constexpr int LD = DP + 4;
@@ -274,11 +273,11 @@ struct Tile {
 // ---------------------------------------------------------------------------
 // Forward: one block per (batch*head, 32-row query tile); the heaviest (latest) query tiles of all slices first.
 // ---------------------------------------------------------------------------
-template <int DP, int FBN>
-__global__ void __launch_bounds__(NT, DP <= 32 ? 2 : 1) attn_fwd_f32_kernel(const F32Params p) {
+template <int DP, int NG, int FBN>
+__global__ void __launch_bounds__(64 * NG, DP <= 32 && NG == 4 ? 2 : 1) attn_fwd_f32_kernel(const F32Params p) {
     chain_wait();
-    using L = Tile<DP, FBN>;
-    constexpr int BN = L::BN, NC = L::NC, LD = L::LD, PLD = L::FWD_PLD;
+    using L = Tile<DP, NG, FBN>;
+    constexpr int NT = L::NT, BN = L::BN, NC = L::NC, LD = L::LD, PLD = L::FWD_PLD;
     extern __shared__ __align__(16) float smem[];
     const int g = threadIdx.x / 64, t = threadIdx.x % 64;
     const int ty = place_y(t), tx = place_x(t);
@@ -360,7 +359,9 @@ __global__ void __launch_bounds__(NT, DP <= 32 ? 2 : 1) attn_fwd_f32_kernel(cons
         cp_commit();
     }
     cp_wait<0>();
-    chain_next();
+    // Where a block fills its SM, successors set up in front of its last stores take the idle SMs unevenly (forward and backward
+    // in turn, B4 H6 T256 D32: 31.0 us, with the call at the end 29.3).
+    if (NG == 4) chain_next();
 
     // The groups meet: O = sum_g 2^(m_g - M) O_g / sum_g 2^(m_g - M) l_g, in group order.
     put_acc(Ks, ty, tx, acc);
@@ -390,6 +391,7 @@ __global__ void __launch_bounds__(NT, DP <= 32 ? 2 : 1) attn_fwd_f32_kernel(cons
         store4(ob + (long long)row * p.so.t + c, make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv), p.D - c, p.vec_out);
         if (c == 0) p.lse_out[(long long)bh * p.T + row] = (M + log2f(sum)) * LN2;
     }
+    if (NG != 4) chain_next();
 }
 
 // ---------------------------------------------------------------------------
@@ -439,9 +441,9 @@ struct RowDelta {
 };
 
 // Adds the groups' partial gradients (each parked in its first streamed tile) and stores the block's rows.
-template <int DP>
+template <int DP, int NG>
 __device__ __forceinline__ void merge_store(const F32Params& p, const float* parts, int stride, float* dst, long long st, int row0, bool rotate) {
-    constexpr int C4 = DP / 4;
+    constexpr int C4 = DP / 4, NT = 64 * NG;
     if (rotate) {                                               // D % 8 == 0: a thread takes four columns of both halves
         const int half = p.D / 2, h4 = half / 4;
         for (int idx = threadIdx.x; idx < BM * h4; idx += NT) {
@@ -517,10 +519,10 @@ __device__ __forceinline__ void staged_product(float* stage, const float (&v)[4]
 }
 
 // dK / dV of 32 key rows: the groups walk the query tiles at or below the diagonal.
-template <int DP>
+template <int DP, int NG>
 __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt, int bh) {
-    using L = Tile<DP>;
-    constexpr int BN = L::BWD_BN, NC = BN / 8, LD = L::LD;
+    using L = Tile<DP, NG>;
+    constexpr int NT = L::NT, BN = L::BWD_BN, NC = BN / 8, LD = L::LD;
     const int g = threadIdx.x / 64, t = threadIdx.x % 64;
     const int ty = DP <= 32 ? t / 8 : place_y(t), tx = DP <= 32 ? t % 8 : place_x(t);     // (DP 32: plain, it spills less)
     float* Ks = smem;
@@ -594,15 +596,15 @@ __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt
     put_acc(Qs, ty, tx, dk);
     put_acc(Gs, ty, tx, dv);
     __syncthreads();
-    merge_store<DP>(p, grp0, L::BWD_GROUP, p.dk + b * p.sdk.b + h * p.sdk.h, p.sdk.t, k0, p.cosv != nullptr);
-    merge_store<DP>(p, grp0 + L::BWD_STREAM, L::BWD_GROUP, p.dv + b * p.sdv.b + h * p.sdv.h, p.sdv.t, k0, false);
+    merge_store<DP, NG>(p, grp0, L::BWD_GROUP, p.dk + b * p.sdk.b + h * p.sdk.h, p.sdk.t, k0, p.cosv != nullptr);
+    merge_store<DP, NG>(p, grp0 + L::BWD_STREAM, L::BWD_GROUP, p.dv + b * p.sdv.b + h * p.sdv.h, p.sdv.t, k0, false);
 }
 
 // dQ of 32 query rows: the groups walk the key tiles at or left of the diagonal.
-template <int DP>
+template <int DP, int NG>
 __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, int bh) {
-    using L = Tile<DP>;
-    constexpr int BN = L::BWD_BN, NC = BN / 8, LD = L::LD;
+    using L = Tile<DP, NG>;
+    constexpr int NT = L::NT, BN = L::BWD_BN, NC = BN / 8, LD = L::LD;
     const int g = threadIdx.x / 64, t = threadIdx.x % 64;
     const int ty = DP <= 32 ? t / 8 : place_y(t), tx = DP <= 32 ? t % 8 : place_x(t);     // (DP 32: plain, it spills less)
     float* Qs = smem;
@@ -629,7 +631,7 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
     cp_wait<0>();
     __syncthreads();                                            // Q and dO are shared by the groups
     RowDelta<DP, 8> rd;
-    {
+    if (threadIdx.x < 8 * BM) {
         const int r = threadIdx.x / 8, row = q0 + r;            // eight threads per row
         const float* ob = p.o + b * p.so.b + h * p.so.h;
         rd.load(p, ob, row, threadIdx.x % 8);
@@ -671,18 +673,18 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
     chain_next();
     put_acc(Ks, ty, tx, dq);
     __syncthreads();
-    merge_store<DP>(p, grp0, L::BWD_GROUP, p.dq + b * p.sdq.b + h * p.sdq.h, p.sdq.t, q0, p.cosv != nullptr);
+    merge_store<DP, NG>(p, grp0, L::BWD_GROUP, p.dq + b * p.sdq.b + h * p.sdq.h, p.sdq.t, q0, p.cosv != nullptr);
 }
 
 // Both roles in one launch: row n of the grid holds every slice's n-th heaviest key tile, then every slice's n-th heaviest query
 // tile (gridDim.y ends at 65535; the longest sequence, 2^20, has 32768 tiles of a kind).
-template <int DP>
-__global__ void __launch_bounds__(NT, DP <= 64 ? 2 : 1) attn_bwd_f32_kernel(const F32Params p) {
+template <int DP, int NG>
+__global__ void __launch_bounds__(64 * NG, DP <= 64 && NG == 4 ? 2 : 1) attn_bwd_f32_kernel(const F32Params p) {
     chain_wait();
     extern __shared__ __align__(16) float smem[];
     const int n = blockIdx.y, slices = p.B * p.H, x = blockIdx.x;
-    if (x < slices) bwd_dkdv<DP>(p, smem, n, x);
-    else bwd_dq<DP>(p, smem, (int)gridDim.y - 1 - n, x - slices);
+    if (x < slices) bwd_dkdv<DP, NG>(p, smem, n, x);
+    else bwd_dq<DP, NG>(p, smem, (int)gridDim.y - 1 - n, x - slices);
 }
 
 Strides3 s3(const int64_t* s) { return Strides3{(long long)s[0], (long long)s[1], (long long)s[2]}; }
@@ -691,41 +693,65 @@ bool rows_vec_ok(const void* ptr, const int64_t* s) {
     return (((uintptr_t)ptr) & 15u) == 0 && (s[0] & 3) == 0 && (s[1] & 3) == 0 && (s[2] & 3) == 0;
 }
 
-template <int DP, int FBN>
+template <int DP, int NG, int FBN>
 int fwd_launch_f32(deers_ctx* ctx, const F32Params& p) {
-    DEERS_SMEM_ONCE(ctx, (attn_fwd_f32_kernel<DP, FBN>), (Tile<DP, FBN>::FWD_SMEM));
+    using L = Tile<DP, NG, FBN>;
+    DEERS_SMEM_ONCE(ctx, (attn_fwd_f32_kernel<DP, NG, FBN>), L::FWD_SMEM);
     const dim3 grid(p.B * p.H, (p.T + BM - 1) / BM);
-    const auto kernel = attn_fwd_f32_kernel<DP, FBN>;
+    const auto kernel = attn_fwd_f32_kernel<DP, NG, FBN>;
     {
         KernelTimerScope ts(ctx, DEERS_K_FWD);
-        DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, grid, NT, (Tile<DP, FBN>::FWD_SMEM), 1, p));
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, grid, L::NT, L::FWD_SMEM, 1, p));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     return DEERS_OK;
+}
+
+// Blocks of a call that has at most two per SM: then a block's walk is what the call takes.
+bool few_blocks(const deers_ctx* ctx, const F32Params& p, int kinds, int per_sm) {
+    return (long long)kinds * p.B * p.H * ((p.T + BM - 1) / BM) <= (long long)per_sm * ctx->sm_count;
 }
 
 // Narrow heads stream 64 keys at a time (half the reads of Q per score), unless the sequence has so few tiles that groups
-// would go without: up to NG * 32 keys, tiles of 32.
+// would go without: up to 128 keys, tiles of 32 (B1 H6 T100 D32 5.8 -> 4.7 us, B3 H4 T77 D48 8.8 -> 6.7).  Heads up to 32 wide
+// take eight groups of 32 keys each where the blocks are few: up to 256 keys that is one tile per group (B4 H6 T256 D32 10.7 ->
+// 8.7), beyond, with an SM per block, half the walk (B1 H2 T1024 23.2 -> 21.5).  Heads of 64 do not gain (T 256 11.1 against 11.9,
+// T 512 19.9 against 20.6).
 template <int DP>
 int fwd_impl(deers_ctx* ctx, const F32Params& p) {
-    if constexpr (DP <= 64) {
-        if (p.T > NG * 32) return fwd_launch_f32<DP, 64>(ctx, p);
+    if constexpr (DP <= 32) {
+        if (p.T > 128 && few_blocks(ctx, p, 1, p.T <= 256 ? 2 : 1)) return fwd_launch_f32<DP, 8, 32>(ctx, p);
     }
-    return fwd_launch_f32<DP, 32>(ctx, p);
+    if constexpr (DP <= 64) {
+        if (p.T > 128) return fwd_launch_f32<DP, 4, 64>(ctx, p);
+    }
+    return fwd_launch_f32<DP, 4, 32>(ctx, p);
 }
 
-template <int DP>
-int bwd_impl(deers_ctx* ctx, const F32Params& p) {
-    DEERS_SMEM_ONCE(ctx, (attn_bwd_f32_kernel<DP>), Tile<DP>::BWD_SMEM);
+template <int DP, int NG>
+int bwd_launch_f32(deers_ctx* ctx, const F32Params& p) {
+    using L = Tile<DP, NG>;
+    DEERS_SMEM_ONCE(ctx, (attn_bwd_f32_kernel<DP, NG>), L::BWD_SMEM);
     const dim3 grid(2 * p.B * p.H, (p.T + BM - 1) / BM);
+    const auto kernel = attn_bwd_f32_kernel<DP, NG>;
     {
         KernelTimerScope ts(ctx, DEERS_K_BWD_MAIN);
-        DEERS_CUDA_TRY(ctx, launch_chained(ctx, attn_bwd_f32_kernel<DP>, grid, NT, Tile<DP>::BWD_SMEM, 1, p));
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, grid, L::NT, L::BWD_SMEM, 1, p));
     }
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     ctx->launches += 1;
     return DEERS_OK;
+}
+
+// Eight groups where every block has an SM to itself and more tiles than four groups take at once (B1 H6 T256 D32 14.5 -> 13.0 us,
+// B1 H4 T256 D64 27.7 -> 23.3); with more blocks than SMs two of four groups each share one (B4 H6 T256 D32: 20.2 against 23.3).
+template <int DP>
+int bwd_impl(deers_ctx* ctx, const F32Params& p) {
+    if constexpr (DP <= 64) {
+        if (p.T > 128 && few_blocks(ctx, p, 2, 1)) return bwd_launch_f32<DP, 8>(ctx, p);
+    }
+    return bwd_launch_f32<DP, 4>(ctx, p);
 }
 
 F32Params base_params(const deers_attn_desc* d) {

@@ -603,3 +603,56 @@ def test_decode_nan_and_inf_scores(dtype, D, Tk, Tq):
         exact = s.softmax(-1) @ v.double()
         assert torch.equal(o.isnan(), exact.isnan()) and bool(exact.isnan().any()) == alone, j
         assert_close(o.nan_to_num().float().cpu().numpy(), exact.nan_to_num().cpu().numpy(), TOL_F16 if dtype == torch.float16 else 1e-4, f"{j}")
+
+
+@pytest.mark.parametrize("B,H,T,D", [(1, 1, 128, 32), (1, 1, 129, 32), (4, 6, 256, 32), (10, 4, 255, 16), (3, 13, 241, 30), (1, 2, 300, 32),
+                                     (1, 1, 513, 20), (1, 3, 257, 64), (2, 3, 200, 52)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_f32_attention_group_counts(B, H, T, D, causal):
+    """Four or eight groups per block, tiles of 32 or 64 keys: by sequence length, head width and number of blocks."""
+    from deers_b200 import ops
+    from oracle import ref
+    from tests.helpers import TOL_F32
+    rng = np.random.default_rng(T * 17 + D)
+    host = [rng.standard_normal((B, H, T, D)).astype(np.float32) for _ in range(4)]
+    q, k, v, do = (torch.from_numpy(a).cuda() for a in host)
+    op = ops.CausalAttention.new(q, k, v, None, causal)
+    o = op.forward()
+    grads = ops.GradientStore()
+    op.backward(grads, do)
+    ops.Context.current(q.device).sync()
+    want = ref.attn_fwd_bwd(*host, causal=causal)
+    for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), [o, op.lse] + [grads.get(t) for t in (q, k, v)], want):
+        assert_close(g.cpu().numpy(), w, TOL_F32, f"B {B} H {H} T {T} D {D} {name}")
+
+
+@pytest.mark.parametrize("V,L,H,D,Hm,B,T", [
+    (1031, 2, 2, 48, 100, 2, 33),      # heads that fit the 96 wide tiles only; odd vocabulary, dense logits off 16-byte boundaries
+    (1024, 1, 3, 32, 64, 1, 129),      # heads that fit every tile
+    (50, 2, 2, 12, 20, 2, 17),         # halves of six: no rotation inside the kernels, on either side
+    (61, 1, 4, 24, 36, 3, 20), (1100, 2, 2, 80, 64, 2, 40),              # ... no tile holds heads of 80 whole; backward rotates
+    (1033, 3, 5, 16, 60, 1, 70), (1040, 1, 2, 128, 513, 1, 65), (37, 0, 2, 8, 5, 1, 9)])
+def test_gpt_norms_rotations_and_grouped_gradients(V, L, H, D, Hm, B, T):
+    """Head widths, depths and sizes at which norm, rotation, logits and weight gradients take another route."""
+    from deers_b200 import gpt
+    from oracle import ref
+    C = H * D
+    cfg = (V, L, H, C, Hm)
+    params = ref.gpt_init_params(cfg, seed=3)
+    rng = np.random.default_rng(V + T)
+    ids, tgt = rng.integers(0, V, (B, T)), rng.integers(0, V, B * T)
+    m = gpt.GPT(gpt.GPTConfig(V, T, L, H, C, Hm), torch.device("cuda", torch.cuda.current_device()), B)
+    m.load_parameters(params)
+    tid, ttg = torch.from_numpy(ids).cuda(), torch.from_numpy(tgt).cuda()
+    logits = m.forward(tid)
+    loss = m.forward_backward(tid, ttg)
+    again = m.forward(tid)
+    m.ctx.sync()
+    want = ref.gpt_step(cfg, params, ids, tgt)
+    got = logits.cpu().numpy().reshape(B * T, V)
+    assert np.isfinite(got).all() and torch.equal(logits, again)
+    assert np.abs(got - want["logits"]).max() <= 1e-4 * np.abs(want["logits"]).max()
+    assert abs(loss.item() - want["loss"]) < 1e-5 * max(1.0, abs(want["loss"]))
+    for i in range(2 + 6 * L):
+        g, w = m.grad(i), want["grads"][i]
+        assert np.abs(g - w).max() <= 1e-4 * np.abs(w).max() + 1e-7, m.parameter_info(i)
