@@ -111,7 +111,7 @@ struct KernelTimerScope {
 // Back-to-back kernels.  A kernel launched by launch_chained() may be set up while the one before it still runs: it calls
 // chain_wait() before its first access to global memory (the predecessor has finished and its writes are visible; every
 // kernel of a chain waits, so this covers all before it) and chain_next() where its own successor may be set up.
-// Saves the launch gap of a microsecond or two: 54 kernels of a GPT forward on a short prompt, replayed from a graph,
+// Saves the launch gap of a microsecond or two: 54 kernels (of then) of a GPT forward on a short prompt, replayed from a graph,
 // 232 -> 206 us; launched one by one, where the host's time hides as well, 495 -> 214 us.  Where chain_next()
 // stands matters: a successor set up at the start of a kernel of few large blocks takes the idle SMs unevenly (252 us), so
 // those call it once their last loads are under way; kernels of small blocks call it first.
