@@ -11,9 +11,9 @@
 // warps meet at a named barrier, and the P / dS tile a product reads was written by the same warp.
 // Within a group thread (ty, tx) of 8 x 8 owns rows 4 ty .. 4 ty + 3 and columns tx, tx + 8, ... of a 32 x BN score tile
 // (4 x 8 or 4 x 4 patches: 12 LDS.128 per 128 FFMA) and rows 4 ty .. with float4 columns 4 tx + 32 j of the
-// accumulators.  Products run two to an issue slot where the registers allow (forward, and from 64 wide tiles on backward), and
-// lanes lie so that shared-memory reads cost half: B8 H12 T2048 D64 forward 1909 -> 1659 us, backward 5821 -> 5642; B3 H4 T77 D48
-// forward 10.3 -> 8.8; B4 H6 T256 D32 unchanged (10.6 and 19.8).  Tiles arrive by cp.async: the next K (or Q) is fetched while the current one's scores are turned
+// accumulators.  Second products run two to an issue slot (forward, and from 64 wide tiles on backward; score products from
+// 96), and lanes lie so that shared-memory reads cost half: B8 H12 T2048 D64 forward 1909 -> 1688 us, backward 5821 -> 5642;
+// B3 H4 T77 D48 forward 10.3 -> 6.8.  Tiles arrive by cp.async: the next K (or Q) is fetched while the current one's scores are turned
 // into the second product, the next V (or dO) while the next scores are computed.
 #include "common.cuh"
 
@@ -105,8 +105,10 @@ __device__ __forceinline__ void fetch_tile(float* __restrict__ dst, const float*
     }
 }
 
-// s[r][c] = sum_d A[4 ty + r][d] * B[tx + 8 c][d].  PAIRS: even and odd d side by side, where the registers for twice the
-// sums are there without spilling or losing the second block of an SM (forward from 64 wide tiles, backward from 96).
+// s[r][c] = sum_d A[4 ty + r][d] * B[tx + 8 c][d].  PAIRS: even and odd d side by side, from 96 wide tiles on, where both
+// directions have the registers for twice the sums.  Both, because the backward makes the probabilities again from the forward's
+// row sums: with pairs in the forward alone the two round the scores differently, and at B4 H6 T256 D32 the gradients were 7 to
+// 11 % further from 64 bits (dQ 3.1e-7 -> 3.5e-7) than with the same sums on both sides.
 template <int DP, int NC, bool PAIRS>
 __device__ __forceinline__ void tile_nt(const float* __restrict__ A, const float* __restrict__ Bm, int ty, int tx, float (&s)[4][NC]) {
     constexpr int LD = DP + 4;
@@ -316,7 +318,7 @@ __global__ void __launch_bounds__(64 * NG, DP <= 32 && NG == 4 ? 2 : 1) attn_fwd
         const int k0 = j * BN;
         if (j != g) { cp_wait<1>(); group_sync(g); }            // this K tile has landed for both warps
         float s[4][NC];
-        tile_nt<DP, NC, (DP >= 64 || FBN == 32)>(Qs, Ks, ty, tx, s);
+        tile_nt<DP, NC, (DP >= 96)>(Qs, Ks, ty, tx, s);
         group_sync(g);                                          // K is consumed: the next one may land
         if (j + NG < ntiles) fetch_tile<DP, BN, 64>(Ks, kb, k0 + NG * BN, p.T, p.D, p.sk.t, p.vec, t);
         cp_commit();
@@ -714,8 +716,8 @@ bool few_blocks(const deers_ctx* ctx, const F32Params& p, int kinds, int per_sm)
 }
 
 // Narrow heads stream 64 keys at a time (half the reads of Q per score), unless the sequence has so few tiles that groups
-// would go without: up to 128 keys, tiles of 32 (B1 H6 T100 D32 5.8 -> 4.7 us, B3 H4 T77 D48 8.8 -> 6.7).  Heads up to 32 wide
-// take eight groups of 32 keys each where the blocks are few: up to 256 keys that is one tile per group (B4 H6 T256 D32 10.7 ->
+// would go without: up to 128 keys, tiles of 32 (B1 H6 T100 D32 5.8 -> 4.8 us, B3 H4 T77 D48 8.8 -> 6.8).  Heads up to 32 wide
+// take eight groups of 32 keys each where the blocks are few: up to 256 keys that is one tile per group (B4 H6 T256 D32 10.8 ->
 // 8.7), beyond, with an SM per block, half the walk (B1 H2 T1024 23.2 -> 21.5).  Heads of 64 do not gain (T 256 11.1 against 11.9,
 // T 512 19.9 against 20.6).
 template <int DP>
