@@ -97,7 +97,11 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 
 // One operand's stage of one k group in shared memory, in its storage order: R rows (m or n) of KG k when k is contiguous,
 // KG rows of R when m / n is.  Row strides are 4 mod 16 words (16-byte pieces of neighbouring rows fall into different banks).
-template <int R, bool MN, int KG>
+// LOOSE: takes rows that lie on no 16-byte boundary as well, float by float with neighbouring lanes side by side: a copy
+// instruction of a warp then touches one or two rows of 16 k, where four floats per lane touch eight, four times over.
+// 66 x 249 x 689 7.6 -> 5.4 us, 2133 x 769 x 1405 185 -> 147.  Kernels of their own, because the branch costs aligned products
+// 2 to 4 % (192 x 768 x 1024 12.85 -> 13.4).  Rows of 96 floats do not fit the lanes and keep the four floats per lane.
+template <int R, bool MN, int KG, bool LOOSE>
 struct Operand {
     static constexpr int LD = MN ? R + 4 : KG + 4;
     static constexpr int FLOATS = MN ? KG * LD : R * LD;
@@ -124,8 +128,24 @@ struct Operand {
             src[i] = b + (MN ? (long long)(k0 + k) * ld + r : (long long)r * ld + k0 + k);
         }
     }
-    // Enqueues the next stage's pieces; kv is the number of the group's k that exist.
-    __device__ __forceinline__ void fetch(float* s, int kv, bool vec) {
+    // Enqueues the next stage's pieces; kv is the number of the group's k that exist, rv that of the tile's m / n.
+    __device__ __forceinline__ void fetch(float* s, int kv, bool vec, long long ld, int rv, int t) {
+        if constexpr (LOOSE && GT % LEN == 0) {
+            if (!vec) {
+                int row = t / LEN;
+                const int col = t % LEN;
+                const float* p = src[0] - (t / (LEN / 4) * ld + t % (LEN / 4) * 4) + (row * ld + col);
+                float* d = s + row * LD + col;
+#pragma unroll 4
+                for (int i = 0; i < 4 * NP; ++i) {
+                    const bool in = MN ? row < kv && col < rv : row < rv && col < kv;
+                    cp4(d, in ? p : base, in ? 4 : 0);
+                    row += GT / LEN; p += GT / LEN * ld; d += GT / LEN * LD;
+                }
+                src[0] += step;
+                return;
+            }
+        }
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
             int valid = along_r[i];
@@ -181,11 +201,11 @@ struct Operand {
     }
 };
 
-template <int PM, int PN, int KS, bool A_MN, bool B_MN>
+template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool LOOSE>
 struct GemmShape {
     static constexpr int BM = 8 * PM, BN = 16 * PN, THREADS = GT * KS, KG = BK / KS;
-    using OA = Operand<BM, A_MN, KG>;
-    using OB = Operand<BN, B_MN, KG>;
+    using OA = Operand<BM, A_MN, KG, LOOSE>;
+    using OB = Operand<BN, B_MN, KG, LOOSE>;
     static constexpr int STAGE = KS * (OA::FLOATS + OB::FLOATS);
     static constexpr int RLD = BN + 4;                              // row stride of the patch staging tile
     static constexpr int RED = KS * BM * RLD;
@@ -220,9 +240,9 @@ __device__ __forceinline__ float4 patch_sum(const float* q, int parts) {
 
 // One tile (tile_m, tile_n) of a product and one part of its K.  setup() only computes addresses and may run before the
 // predecessor has finished; run() does the work.
-template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED>
+template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED, bool LOOSE>
 struct TileProduct {
-    using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
+    using S = GemmShape<PM, PN, KS, A_MN, B_MN, LOOSE>;
     static constexpr int BM = S::BM, BN = S::BN, STAGES = S::STAGES, KG = S::KG;
     typename S::OA la;
     typename S::OB lb;
@@ -238,8 +258,8 @@ struct TileProduct {
     __device__ __forceinline__ void run(const GemmArgs& g, int parts, int rank);
 };
 
-template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED>
-__device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED>::run(const GemmArgs& g, const int parts, const int rank) {
+template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED, bool LOOSE>
+__device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED, LOOSE>::run(const GemmArgs& g, const int parts, const int rank) {
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x % GT, kg = threadIdx.x / GT;        // position in the tile, k group
     const int w = tid / 32, lane = tid % 32;
@@ -255,8 +275,8 @@ __device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED>::run(
     int st_in = 0, left = nk;                                       // stage to fill next
     auto fetch = [&]() {
         if (left > 0) {
-            la.fetch(ring + st_in, kv, g.a_vec);
-            lb.fetch(ring + st_in + S::OA::FLOATS, kv, g.b_vec);
+            la.fetch(ring + st_in, kv, g.a_vec, g.lda, g.M - m0, tid);
+            lb.fetch(ring + st_in + S::OA::FLOATS, kv, g.b_vec, g.ldb, g.N - n0, tid);
             kv -= BK;
             --left;
             st_in = st_in == (STAGES - 1) * S::STAGE ? 0 : st_in + S::STAGE;
@@ -476,9 +496,9 @@ __device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED>::run(
     if (parts > 1) cg::this_cluster().sync();                       // nobody leaves while a peer still reads its patch
 }
 
-template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED>
+template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED, bool LOOSE>
 __global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
-    TileProduct<PM, PN, KS, A_MN, B_MN, FUSED> tile;
+    TileProduct<PM, PN, KS, A_MN, B_MN, FUSED, LOOSE> tile;
     tile.setup(g, blockIdx.y, blockIdx.x, blockIdx.z);
     chain_wait();
     tile.run(g, gridDim.z, blockIdx.z);
@@ -504,7 +524,7 @@ struct GemmGroup {
 template <int PM, int PN, int KS>
 __global__ void __launch_bounds__(GT * KS) gemm_f32_group_kernel(const __grid_constant__ GemmGroup gg) {
     const int i = gg.pick(blockIdx.x);
-    TileProduct<PM, PN, KS, true, true, false> tile;
+    TileProduct<PM, PN, KS, true, true, false, true> tile;
     tile.setup(gg.args(i), gg.tile_m(i, blockIdx.x), gg.tile_n(i, blockIdx.x), blockIdx.z);
     chain_wait();
     tile.run(gg.args(i), gridDim.z, blockIdx.z);
@@ -533,9 +553,9 @@ int cluster_capacity(deers_ctx* ctx) {
         for (int parts = 1; parts <= MAX_PARTS; ++parts) ctx->cluster_capacity[parts] = dev[parts].load(std::memory_order_relaxed);
         return DEERS_OK;
     }
-    using S = GemmShape<8, 4, 4, false, true>;
-    const auto kernel = gemm_f32_kernel<8, 4, 4, false, true, false>;
-    DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<8, 4, 4, false, true, false>), S::SMEM);
+    using S = GemmShape<8, 4, 4, false, true, false>;
+    const auto kernel = gemm_f32_kernel<8, 4, 4, false, true, false, false>;
+    DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<8, 4, 4, false, true, false, false>), S::SMEM);
     for (int parts = 2; parts <= MAX_PARTS; ++parts) {
         cudaLaunchConfig_t lc{};
         lc.gridDim = dim3(1, 1, parts);
@@ -585,11 +605,14 @@ GemmPlan plan_gemm(int n, const int* M, const int* N, int K, const int* capacity
     return best;
 }
 
-template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED = false>
+template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED = false, bool LOOSE = false>
 int launch_variant(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g) {
-    using S = GemmShape<PM, PN, KS, A_MN, B_MN>;
-    const auto kernel = gemm_f32_kernel<PM, PN, KS, A_MN, B_MN, FUSED>;
-    DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<PM, PN, KS, A_MN, B_MN, FUSED>), S::SMEM);
+    if constexpr (!LOOSE) {
+        if (!g.a_vec || !g.b_vec) return launch_variant<PM, PN, KS, A_MN, B_MN, FUSED, true>(ctx, p, g);
+    }
+    using S = GemmShape<PM, PN, KS, A_MN, B_MN, LOOSE>;
+    const auto kernel = gemm_f32_kernel<PM, PN, KS, A_MN, B_MN, FUSED, LOOSE>;
+    DEERS_SMEM_ONCE(ctx, (gemm_f32_kernel<PM, PN, KS, A_MN, B_MN, FUSED, LOOSE>), S::SMEM);
     const dim3 grid((g.N + S::BN - 1) / S::BN, (g.M + S::BM - 1) / S::BM, p.parts);
     DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, grid, S::THREADS, S::SMEM, dim3(1, 1, p.parts), g));
     return DEERS_OK;
@@ -604,7 +627,7 @@ int launch_orders(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g, int a_mn
 
 template <int PM, int PN, int KS>
 int launch_group(deers_ctx* ctx, const GemmPlan& p, GemmGroup& gg) {
-    using S = GemmShape<PM, PN, KS, true, true>;
+    using S = GemmShape<PM, PN, KS, true, true, true>;
     const auto kernel = gemm_f32_group_kernel<PM, PN, KS>;
     DEERS_SMEM_ONCE(ctx, (gemm_f32_group_kernel<PM, PN, KS>), S::SMEM);
     int tiles = 0;
