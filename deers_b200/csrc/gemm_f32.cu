@@ -101,7 +101,8 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 // instruction of a warp then touches one or two rows of 16 k, where four floats per lane touch eight, four times over.
 // 66 x 249 x 689 7.6 -> 5.4 us, 2133 x 769 x 1405 185 -> 147.  Kernels of their own, because the branch costs aligned products
 // 2 to 4 % (192 x 768 x 1024 12.85 -> 13.4).  Rows of 96 floats do not fit the lanes and keep the four floats per lane.
-template <int R, bool MN, int KG, bool LOOSE>
+// PERM: see row_of(); for small patches (32 x 96 tiles lose more by the registers, 1024 x 192 x 576 11.9 -> 12.9).
+template <int R, bool MN, int KG, bool LOOSE, bool PERM>
 struct Operand {
     static constexpr int LD = MN ? R + 4 : KG + 4;
     static constexpr int FLOATS = MN ? KG * LD : R * LD;
@@ -114,13 +115,16 @@ struct Operand {
     int along_r[NP];         // floats of a piece inside the matrix along m / n (K order: 4 or 0)
     int along_k[NP];         // k of a piece inside the group's share of the stage
     long long step;          // from one stage to the next
+    // A quarter warp stores two rows of 16 floats: rows i and i + 4 lie 16 banks apart, i and i + 1 would meet in four banks
+    // (231 x 192 x 500 5.67 -> 5.50 us, 192 x 768 x 1024 12.4 -> 11.4; B in MN order).
+    static __device__ __forceinline__ int row_of(int i) { return PERM && LEN == 16 ? (i & ~7) | (i & 1) * 4 | ((i >> 1) & 3) : i; }
     __device__ __forceinline__ void init(const float* b, long long ld, int r0, int rmax, int k0, int t) {
         base = b;
         step = MN ? BK * ld : BK;
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
             const int idx = t + i * GT;
-            const int row = idx / (LEN / 4), col = (idx % (LEN / 4)) * 4;
+            const int row = row_of(idx / (LEN / 4)), col = (idx % (LEN / 4)) * 4;
             const int r = r0 + (MN ? col : row), k = MN ? row : col;
             along_k[i] = k;
             along_r[i] = MN ? min(4, max(0, rmax - r)) : (r < rmax ? 4 : 0);
@@ -134,7 +138,7 @@ struct Operand {
             if (!vec) {
                 int row = t / LEN;
                 const int col = t % LEN;
-                const float* p = src[0] - (t / (LEN / 4) * ld + t % (LEN / 4) * 4) + (row * ld + col);
+                const float* p = src[0] - (row_of(t / (LEN / 4)) * ld + t % (LEN / 4) * 4) + (row * ld + col);
                 float* d = s + row * LD + col;
 #pragma unroll 4
                 for (int i = 0; i < 4 * NP; ++i) {
@@ -204,8 +208,8 @@ struct Operand {
 template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool LOOSE>
 struct GemmShape {
     static constexpr int BM = 8 * PM, BN = 16 * PN, THREADS = GT * KS, KG = BK / KS;
-    using OA = Operand<BM, A_MN, KG, LOOSE>;
-    using OB = Operand<BN, B_MN, KG, LOOSE>;
+    using OA = Operand<BM, A_MN, KG, LOOSE, (PM * PN <= 16)>;
+    using OB = Operand<BN, B_MN, KG, LOOSE, (PM * PN <= 16)>;
     static constexpr int STAGE = KS * (OA::FLOATS + OB::FLOATS);
     static constexpr int RLD = BN + 4;                              // row stride of the patch staging tile
     static constexpr int RED = KS * BM * RLD;
