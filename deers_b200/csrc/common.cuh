@@ -224,6 +224,7 @@ int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, co
 constexpr int GEMM_GROUP_MAX = 4;
 struct GemmTN { int M, N; const float* a; const float* b; float* c; };
 int launch_gemm_f32_group(deers_ctx* ctx, int n, const GemmTN* t, int K);
+bool gemm_f32_group_fits(deers_ctx* ctx, int n, const GemmTN* t, int K);
 // RMSNorm (rmsnorm.cu)
 int launch_rmsnorm_fwd(deers_ctx* ctx, long long rows, int C, double eps, const float* x, float* y, float* inv_norm);
 int launch_rmsnorm_bwd(deers_ctx* ctx, long long rows, int C, const float* x, const float* inv_norm, const float* dy,

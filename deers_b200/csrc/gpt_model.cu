@@ -12,8 +12,9 @@
 // rotated back by the attention backward straight into the fused [N, 3C] gradient buffer next to dV, and one GEMM for the sum of
 // the three input gradients.  Every launch is one of this library's kernels; there is no host round trip in a step.
 // The weight gradients are off the critical path (nothing in the backward reads them): the four of a block are one
-// launch on a second stream, forked from the main one where their operands are complete and joined before the gradient norm;
-// captured, the two streams become two branches of the step's graph.  What they read is double-buffered by block.
+// launch on a second stream, or four where one would be several waves of blocks, forked from the main one where their operands
+// are complete and joined before the gradient norm; captured, the two streams become two branches of the step's graph.  What
+// they read is double-buffered by block.
 #include "common.cuh"
 
 #include <math.h>
@@ -273,15 +274,31 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
     const float* dx0 = m->lg[last].dx;
     deers_attn_desc ad;
     attn_desc(m, B, T, &ad);
+    bool together = false;
     for (int l = c.n_layer - 1; l >= 0; --l) {
         const LayerW& w = m->lw[l];
         LayerAct& a = m->la[l];
         LayerGrad &d = m->lg[l & 1], &below = m->lg[(l & 1) ^ 1];
         const float* x_in = l ? m->la[l - 1].x2 : m->x0;
+        // On the second stream: all four at the block's end in one launch, or each as soon as its operands are there.
+        const GemmTN grads[4] = {{Hm, C, a.h, d.dx, G + w.down}, {C, Hm, d.n2, d.dh, G + w.up},              // d Wdown = h^T dx, d Wup = n2^T du
+                                 {C, C, a.o, d.dx1, G + w.out}, {C, 3 * C, d.n1, d.dqkv, G + w.qkv}};        // d Wout = o^T dx1, d [Wq|Wk|Wv]
+        if (l == c.n_layer - 1) together = gemm_f32_group_fits(ctx, 4, grads, (int)N);
+        auto weight_grads = [&](int first, int n) -> int {
+            SideScope side(m);
+            GPT_TRY(side.rc);
+            if (n == 4) GPT_TRY(launch_gemm_f32_group(ctx, 4, grads, (int)N));
+            else
+                for (const GemmTN* t = grads + first; t < grads + first + n; ++t)
+                    GPT_TRY(gemm(m, t->M, t->N, (int)N, t->a, t->M, 1, t->b, t->N, 1, t->c, t->N));
+            return first + n == 4 ? side.done(l & 1) : DEERS_OK;
+        };
+        if (!together) GPT_TRY(weight_grads(0, 1));
         // MLP branch: x2 = x1 + relu(rmsnorm(x1) Wup)^2 Wdown
         GPT_TRY(gemm(m, (int)N, Hm, C, d.dx, C, 0, W + w.down, C, 0, d.dh, Hm, DEERS_EPI_MUL_AUX2, nullptr, 0, a.r));
         GPT_TRY(gemm(m, (int)N, C, Hm, d.dh, Hm, 0, W + w.up, Hm, 0, m->dtmp, C));           // d n2 = du Wup^T
         GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, a.x1, a.inv2, m->dtmp, d.dx, d.dx1, d.n2));    // d x1
+        if (!together) GPT_TRY(weight_grads(1, 2));
         // attention branch: x1 = x + attn(rmsnorm(x)) Wout
         GPT_TRY(gemm(m, (int)N, C, C, d.dx1, C, 0, W + w.out, C, 0, m->dtmp, C));            // d o (token-major)
         GPT_TRY(launch_attn_bwd_f32(ctx, &ad, a.qkv, a.qkv + C, a.qkv + 2 * C, a.o, a.lse, m->dtmp, d.dqkv, d.dqkv + C, d.dqkv + 2 * C,
@@ -291,14 +308,7 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
         GPT_TRY(wait_done(m, (l & 1) ^ 1));                                                  // the block above has read what this block's input gradient replaces
         GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, x_in, a.inv1, m->dtmp, d.dx1, below.dx, d.n1)); // d x
         dx0 = below.dx;
-        {
-            SideScope side(m);
-            GPT_TRY(side.rc);
-            const GemmTN grads[4] = {{Hm, C, a.h, d.dx, G + w.down}, {C, Hm, d.n2, d.dh, G + w.up},              // d Wdown = h^T dx, d Wup = n2^T du
-                                     {C, C, a.o, d.dx1, G + w.out}, {C, 3 * C, d.n1, d.dqkv, G + w.qkv}};        // d Wout = o^T dx1, d [Wq|Wk|Wv]
-            GPT_TRY(launch_gemm_f32_group(ctx, 4, grads, (int)N));
-            GPT_TRY(side.done(l & 1));
-        }
+        GPT_TRY(together ? weight_grads(0, 4) : weight_grads(3, 1));
     }
     GPT_TRY(launch_embedding_bwd(ctx, dx0, ids, N, C, V, G + m->off_wte, true));           // (cleared in the forward)
     return join_side(m);

@@ -656,3 +656,53 @@ def test_gpt_norms_rotations_and_grouped_gradients(V, L, H, D, Hm, B, T):
     for i in range(2 + 6 * L):
         g, w = m.grad(i), want["grads"][i]
         assert np.abs(g - w).max() <= 1e-4 * np.abs(w).max() + 1e-7, m.parameter_info(i)
+
+
+def _gpt_and_oracle(V, L, H, D, Hm, B, T):
+    """A model with its gradients made and the oracle's step on the same batch: (model, ids, targets, logits, loss, launches of the
+    forward and of forward_backward, the oracle's results)."""
+    from deers_b200 import gpt
+    from oracle import ref
+    cfg = (V, L, H, H * D, Hm)
+    params = ref.gpt_init_params(cfg, seed=5)
+    rng = np.random.default_rng(V + T)
+    ids, tgt = rng.integers(0, V, (B, T)), rng.integers(0, V, B * T)
+    m = gpt.GPT(gpt.GPTConfig(V, T, L, H, H * D, Hm), torch.device("cuda", torch.cuda.current_device()), B)
+    m.load_parameters(params)
+    tid, ttg = torch.from_numpy(ids).cuda(), torch.from_numpy(tgt).cuda()
+    m.forward(tid)
+    at = [m.ctx.launch_count()]
+    logits = m.forward(tid)
+    at.append(m.ctx.launch_count())
+    loss = m.forward_backward(tid, ttg)
+    at.append(m.ctx.launch_count())
+    m.ctx.sync()
+    return m, tid, ttg, logits, loss, (at[1] - at[0], at[2] - at[1]), ref.gpt_step(cfg, params, ids, tgt)
+
+
+def _check_gpt(m, logits, loss, want):
+    """f32 sums on either side: 1e-4 of the largest value, as for the other models."""
+    got = logits.cpu().numpy().reshape(want["logits"].shape)
+    assert np.abs(got - want["logits"]).max() <= 1e-4 * np.abs(want["logits"]).max()
+    assert abs(loss.item() - want["loss"]) < 1e-5 * max(1.0, abs(want["loss"]))
+    for i, w in enumerate(want["grads"]):
+        assert np.abs(m.grad(i) - w).max() <= 1e-4 * np.abs(w).max() + 1e-7, m.parameter_info(i)
+
+
+@pytest.mark.parametrize("H,D,Hm,B,T,launches", [(4, 32, 512, 2, 40, 1), (6, 32, 768, 1, 70, 1), (5, 64, 1280, 2, 35, 4), (4, 128, 300, 1, 33, 4)])
+def test_gpt_weight_gradients_in_one_launch_or_apart(H, D, Hm, B, T, launches):
+    """One launch per block where that is one wave of blocks, four where it would be several; the second stream changes no bit."""
+    fwd, step = [], []
+    for L in (1, 3):
+        m, ids, tgt, logits, loss, n, want = _gpt_and_oracle(64, L, H, D, Hm, B, T)
+        fwd.append(n[0]), step.append(n[1])
+        _check_gpt(m, logits, loss, want)
+    # of a block's backward: three input gradients, two norms, the attention, the input gradient of the projection
+    assert (step[1] - step[0]) - (fwd[1] - fwd[0]) == 2 * (7 + launches)
+    grads = [m.grad(i) for i in range(m.num_parameters())]
+    m.ctx.kernel_timing(True)                                     # everything on one stream
+    m.forward_backward(ids, tgt)
+    m.ctx.sync()
+    m.ctx.kernel_timing(False)
+    for i, g in enumerate(grads):
+        assert np.array_equal(g, m.grad(i)), m.parameter_info(i)
