@@ -709,8 +709,10 @@ int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, co
     if (f.rope_cols && f.rope_d % 8 == 0) {
         // A rotary launch of its own takes about 3000 cycles (1.5 us): rotate here unless tiles that hold whole heads cost more
         // than that (heads of 48 columns leave 32 x 96 and 64 x 96 tiles: 231 x 576 x 192 takes 7.5 us in them, 3.6 in 32 x 32).
+        // Several waves of clusters do not count: the estimate takes them to follow one another without a gap (forwards of 4 layers,
+        // rotating in them and beside: C 512, 256 tokens 363 and 335 us, C 384, 640 tokens 533 and 501).
         const GemmPlan w = plan_gemm(1, &M, &N, K, ctx->cluster_capacity, f.rope_d);
-        if (w.cfg >= 0 && w.cost < p.cost + 3000.0) {
+        if (w.cfg >= 0 && w.cost < p.cost + 3000.0 && (w.cost == p.cost || w.parts == 1 || w.waves == 1)) {
             p = w;
             *rotated = true;
             g.cosv = f.cosv; g.sinv = f.sinv; g.rope_cols = f.rope_cols; g.rope_d = f.rope_d; g.rope_t = f.rope_t;

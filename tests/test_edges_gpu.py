@@ -627,7 +627,7 @@ def test_f32_attention_group_counts(B, H, T, D, causal):
 
 
 @pytest.mark.parametrize("V,L,H,D,Hm,B,T", [
-    (1031, 2, 2, 48, 100, 2, 33),      # heads that fit the 96 wide tiles only; odd vocabulary, dense logits off 16-byte boundaries
+    (1031, 2, 2, 48, 100, 2, 33),      # 96 wide tiles, the ones for such heads, cost too much here; odd vocabulary, dense logits off 16-byte boundaries
     (1024, 1, 3, 32, 64, 1, 129),      # heads that fit every tile
     (50, 2, 2, 12, 20, 2, 17),         # halves of six: no rotation inside the kernels, on either side
     (61, 1, 4, 24, 36, 3, 20), (1100, 2, 2, 80, 64, 2, 40),              # ... no tile holds heads of 80 whole; backward rotates
@@ -706,3 +706,22 @@ def test_gpt_weight_gradients_in_one_launch_or_apart(H, D, Hm, B, T, launches):
     m.ctx.kernel_timing(False)
     for i, g in enumerate(grads):
         assert np.array_equal(g, m.grad(i)), m.parameter_info(i)
+
+
+@pytest.mark.parametrize("H,D,B,T,inside", [
+    # the projection's tile and the blocks of a cluster along K
+    (6, 32, 1, 100, True), (20, 16, 1, 64, True),                 # 32 x 32; in clusters
+    (16, 16, 3, 100, True), (4, 64, 1, 4, True), (6, 64, 1, 3, True),     # 32 x 64; in clusters of 2, of 3
+    (2, 64, 4, 250, True), (5, 64, 2, 66, True),                  # 64 x 64; in clusters
+    (5, 32, 2, 320, True), (5, 48, 1, 196, True),                 # 32 x 96; in clusters
+    (12, 32, 1, 700, True), (13, 48, 1, 33, True),                # 64 x 96; in clusters
+    (5, 64, 1, 932, True), (6, 64, 1, 281, True),                 # 64 x 128; in clusters
+    # no tile holds the heads, or such tiles cost more than a launch, or they would be several waves of clusters
+    (3, 80, 1, 40, False), (3, 10, 2, 25, False), (4, 48, 1, 231, False), (2, 96, 1, 100, False), (8, 64, 1, 256, False)])
+def test_gpt_rotation_inside_the_projection(H, D, B, T, inside):
+    """Norm and rotation in each tile of the projection, whole K and K split over a cluster (the other half of a head and the rows'
+    squares then lie in several blocks)."""
+    m, ids, tgt, logits, loss, n, want = _gpt_and_oracle(64, 1, H, D, 64, B, T)
+    _check_gpt(m, logits, loss, want)
+    # embedding; projection, attention, output, up, down (and the rotation); norm, head, copy of its padded rows
+    assert n[0] == 1 + 5 + (not inside) + 3
