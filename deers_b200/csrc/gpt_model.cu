@@ -334,10 +334,19 @@ __global__ void __launch_bounds__(256) stage_ids_kernel(const long long* ids, co
     }
 }
 
+// Whether a kernel may touch the caller's memory at p: of this device and on a boundary of `size` bytes.  What is not (pinned or
+// managed memory, another device's, a host pointer) is left to the copies, which take or refuse it.
+bool plain_device(const deers_ctx* ctx, const void* p, size_t size) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return false; }
+    return at.type == cudaMemoryTypeDevice && at.device == ctx->device && (uintptr_t)p % size == 0;
+}
+
 // Brings the caller's ids / targets into the model's own buffers, so that a captured graph reads fixed addresses.
 int stage_ids(deers_gpt* m, const int64_t* ids, const int64_t* targets, long long N, cudaMemcpyKind kind) {
     deers_ctx* ctx = m->ctx;
-    if (kind == cudaMemcpyDeviceToDevice && targets && (const long long*)ids != m->ids_dev && (const long long*)targets != m->tgt_dev) {
+    if (kind == cudaMemcpyDeviceToDevice && targets && (const long long*)ids != m->ids_dev && (const long long*)targets != m->tgt_dev &&
+        plain_device(ctx, ids, sizeof(long long)) && plain_device(ctx, targets, sizeof(long long))) {
         const unsigned grid = (unsigned)((N + 255) / 256);
         DEERS_CUDA_TRY(ctx, launch_chained(ctx, stage_ids_kernel, grid, 256, 0, 1, (const long long*)ids, (const long long*)targets, N, m->ids_dev, m->tgt_dev));
         ctx->launches += 1;
@@ -710,7 +719,14 @@ extern "C" int deers_b200_gpt_train_step(deers_gpt* m, const int64_t* ids, const
     deers_ctx* ctx = m->ctx;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     GPT_TRY(stage_ids(m, ids, targets, (long long)B * T, cudaMemcpyDeviceToDevice));
-    return train_step_common(m, B, T, hyper, max_grad_norm, loss_dev, grad_norm_dev);
+    float* const loss_out = loss_dev && plain_device(ctx, loss_dev, sizeof(float)) ? loss_dev : nullptr;
+    float* const norm_out = grad_norm_dev && plain_device(ctx, grad_norm_dev, sizeof(float)) ? grad_norm_dev : nullptr;
+    GPT_TRY(train_step_common(m, B, T, hyper, max_grad_norm, loss_out, norm_out));
+    if (loss_dev && !loss_out)
+        DEERS_CUDA_TRY(ctx, cudaMemcpyAsync(loss_dev, m->loss_dev, sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
+    if (grad_norm_dev && !norm_out)
+        DEERS_CUDA_TRY(ctx, cudaMemcpyAsync(grad_norm_dev, m->norm_dev, sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
+    return DEERS_OK;
 }
 
 extern "C" int deers_b200_gpt_train_step_host(deers_gpt* m, const int64_t* ids_host, const int64_t* targets_host, int32_t B,

@@ -725,3 +725,31 @@ def test_gpt_rotation_inside_the_projection(H, D, B, T, inside):
     _check_gpt(m, logits, loss, want)
     # embedding; projection, attention, output, up, down (and the rotation); norm, head, copy of its padded rows
     assert n[0] == 1 + 5 + (not inside) + 3
+
+
+def test_gpt_train_step_takes_pointers_on_any_boundary():
+    """What a copy takes and a kernel cannot: ids four bytes off their boundary, loss and norm one byte off."""
+    import ctypes
+    from deers_b200 import _lib, gpt
+    from oracle import ref
+    V, T, B = 40, 9, 2
+    cfg = (V, 1, 2, 16, 24)
+    params = ref.gpt_init_params(cfg, seed=1)
+    rng = np.random.default_rng(2)
+    ids, tgt = (torch.from_numpy(rng.integers(0, V, B * T)).cuda() for _ in range(2))
+    said = []
+    for off, out_off in ((0, 0), (4, 1)):
+        m = gpt.GPT(gpt.GPTConfig(V, T, 1, 2, 16, 24), ids.device, B)
+        m.load_parameters(params)
+        buf = torch.zeros(2 * (8 * B * T + 8) + 24, dtype=torch.uint8, device="cuda")
+        ia, ta, oa = off, 8 * B * T + 8 + off, 2 * (8 * B * T + 8) + out_off
+        buf[ia:ia + 8 * B * T] = ids.view(torch.uint8)
+        buf[ta:ta + 8 * B * T] = tgt.view(torch.uint8)
+        torch.cuda.synchronize()
+        h = _lib.AdamWHyper(1e-3, 0.9, 0.999, 1e-8, 0.1, 1)
+        p = buf.data_ptr()
+        assert _lib.lib().deers_b200_gpt_train_step(m.handle, p + ia, p + ta, B, T, ctypes.byref(h), 1.0, p + oa, p + oa + 4) == _lib.OK
+        m.ctx.sync()
+        said.append((buf[oa:oa + 8].cpu().numpy().tobytes(), [m.parameter(i) for i in range(m.num_parameters())]))
+    assert said[0][0] == said[1][0] and np.isfinite(np.frombuffer(said[0][0], np.float32)).all()
+    assert all(np.array_equal(a, b) for a, b in zip(said[0][1], said[1][1]))
