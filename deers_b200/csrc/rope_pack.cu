@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256) rope_pack_kernel(const RopeParams p) {
     const I rows = (I)p.B * (I)p.T * (I)p.H;
     const I total = rows * (I)cpr;
     const T* src = static_cast<const T*>(p.src);
-    T* __restrict__ dst = static_cast<T*>(p.dst);
+    T* dst = static_cast<T*>(p.dst);                            // may be src: a thread has read both pieces when it writes them
     const T* cosp = static_cast<const T*>(p.cosp);
     const T* sinp = static_cast<const T*>(p.sinp);
     for (I idx = (I)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (I)gridDim.x * blockDim.x) {

@@ -225,7 +225,8 @@ int deers_b200_attn_bwd_f16_static(deers_ctx* ctx, const deers_attn_desc* desc, 
  * tensors, inner stride 1: the forward call passes the [B,T,H,D] strides of the projection output as
  * src and the strides of a [B,H,T,D] buffer (b: H*T*D, t: D, h: T*D) as dst; the backward call swaps
  * them.  Rows, halves and cache rows on 16-byte boundaries take the 16-byte path, anything else a
- * scalar path.  Enqueued on the context's stream; no allocation, no synchronisation.
+ * scalar path.  dst may be src where the strides of both are the same (rotation in place); they may not overlap in any other
+ * way.  Enqueued on the context's stream; no allocation, no synchronisation.
  */
 typedef struct deers_rope_desc {
     int32_t B, T, H, D;        /* D even */

@@ -65,3 +65,9 @@ def test_refused_launches_end_the_call(file):
     """Behind a launch that was refused, the next kernel would work on what has not been written."""
     for m in re.finditer(r"launch_chained\(", FILES[file]):
         assert FILES[file][:m.start()].rstrip().endswith("DEERS_CUDA_TRY(ctx,"), FILES[file][m.start():m.start() + 80]
+
+
+def test_rotation_promises_nothing_about_its_buffers():
+    """The model rotates in place: source and destination are one buffer, which a restrict pointer to either would deny."""
+    (body,) = [body for f, name, _, body in CHAINED if name == "rope_pack_kernel"]
+    assert "p.dst" in body and "__restrict__" not in body

@@ -156,3 +156,29 @@ def test_full_size_rotation_properties():
         assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
     del back, grads, y, x
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("D", [6, 16, 24, 128])                  # halves of whole 16-byte pieces, and not
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("inverse", [0, 1])
+def test_in_place(D, dtype, inverse):
+    """src and dst one buffer: the leading columns of wider rows are rotated where they lie, the others stay."""
+    import ctypes
+
+    from deers_b200 import _lib, ops
+    B, T, H = 3, 37, 4
+    wide = H * D + 8
+    g = torch.Generator(device="cuda").manual_seed(D)
+    x = torch.randn((B, T, wide), device="cuda", generator=g).to(dtype)
+    cos, sin = (t.reshape(T, D // 2).contiguous() for t in ops.precompute_rotary_embeddings(T, D, dtype=dtype, device="cuda"))
+    ctx = ops.Context.current(x.device)
+    d = _lib.RopeDesc()
+    d.B, d.T, d.H, d.D, d.dtype, d.inverse = B, T, H, D, (_lib.F32 if dtype == torch.float32 else _lib.F16), inverse
+    for i, v in enumerate((T * wide, wide, D, 1)):
+        d.src_strides[i] = d.dst_strides[i] = v
+    out = x.clone()
+    for src, dst in ((x, out), (x, x)):                          # apart, then in place
+        _lib.check(_lib.lib().deers_b200_rope_pack(ctx.handle, ctypes.byref(d), src.data_ptr(), cos.data_ptr(), sin.data_ptr(),
+                                                   dst.data_ptr()), ctx.handle)
+    ctx.sync()
+    assert torch.equal(x.view(torch.int16), out.view(torch.int16))
