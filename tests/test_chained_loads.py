@@ -53,6 +53,106 @@ def test_chained_kernels_wait_and_read_coherently(file, name, params, body):
     assert wait and not re.search(r"\*|\[", body[:wait.start()].split("{", 1)[1]), f"{name}: something precedes the wait"
 
 
+def definitions(text):
+    """{name: [(parameters, body)]} of the functions defined in a source."""
+    out = {}
+    for m in re.finditer(r"\b(\w+)\s*\(((?:[^()]|\([^()]*\))*)\)\s*(?:const\s*)?\{", text):
+        if m.group(1) in ("if", "for", "while", "switch", "catch"):
+            continue
+        depth, i = 1, m.end()
+        while depth and i < len(text):
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+        out.setdefault(m.group(1), []).append((m.group(2), text[m.end():i - 1]))
+    return out
+
+
+def reached(files, file, head):
+    """Bodies of the functions a kernel calls before its wait, and of those they call: defined in its file, else in a header."""
+    here = definitions(files[file])
+    headers = {}
+    for f, text in files.items():
+        if f.endswith(".cuh"):
+            for name, found in definitions(text).items():
+                headers.setdefault(name, []).extend(found)
+    seen, todo, out = set(), [head], []
+    while todo:
+        for name in re.findall(r"\b(\w+)\s*(?:<[^<>;(){}]*>)?\s*\(", todo.pop()):
+            if name not in seen:
+                seen.add(name)
+                for params, body in here.get(name) or headers.get(name, []):
+                    out.append((name, params, body))
+                    todo.append(body)
+    return out
+
+
+def touches_global(files, file, head):
+    """What a kernel's calls before the wait do that could reach global memory: an access through anything but shared memory and
+    the arrays of a structure, or an instruction that loads, stores or copies outside shared memory."""
+    arrays, found = set(), []
+    for m in re.finditer(r"\bstruct\s+\w+\s*\{", files[file]):                 # arrays that are members
+        depth, members = 1, ""
+        for c in files[file][m.end():]:
+            depth += {"{": 1, "}": -1}.get(c, 0)
+            if not depth:
+                break
+            members += c if depth == 1 else ""
+        arrays |= set(re.findall(r"\b(\w+)\[[^\]]+\];", members))
+    for name, params, body in reached(files, file, head):
+        asm = " ".join(re.findall(r"asm\s*(?:volatile)?\s*\((.*?)\);", body, re.S))
+        code = re.sub(r"asm\s*(?:volatile)?\s*\(.*?\);", "", body, flags=re.S)
+        for ins in re.findall(r"(?:^|[\"\s;{])((?:ld|st|atom|red|cp|multimem|tcgen05\.(?:ld|st|cp|mma))\.[\w.:]+)", asm):
+            if "global" in ins or ".shared" not in ins:
+                found.append((name, ins))
+        shared = set(re.findall(r"__shared__[^;]*?\b(\w+)\s*\[", code)) | set(re.findall(r"\b(?!return\b)\w+ (\w+)\[[^\]]+\];", code))
+        for _ in range(3):                                       # pointers into it, and pointers from those
+            for var, init in re.findall(r"\*\s*(?:const\s+)?(\w+)\s*=\s*([^;]*);", code):
+                if set(re.findall(r"\w+", init)) & shared:
+                    shared.add(var)
+        for var in re.findall(r"(\w+)\s*\[", re.sub(r"__shared__[^;]*;", "", code)):
+            if var not in shared | arrays and not re.search(r"\w+&?\s*\(&" + var + r"\)\[", params):
+                found.append((name, var + "[]"))
+        if re.search(r"\)\s*\[", code) or re.search(r"(?:^|[=(,;{}&|+\-!?:<>]|return)\s*\*\s*[\w(]", code) or "->" in code:
+            found.append((name, "*"))
+        found += [(name, f) for f in re.findall(r"\b(atomic\w+|__ld\w+|__st\w+)\s*\(", code)]
+    return found
+
+
+def head_of(body):
+    """A kernel's text up to its wait."""
+    return body[:re.search(r"chain_(wait|begin)\(\);", body).start()].split("{", 1)[1]
+
+
+@pytest.mark.parametrize("file,name,params,body", CHAINED, ids=[f"{f}:{n}" for f, n, _, _ in CHAINED])
+def test_what_runs_before_the_wait_stays_off_global_memory(file, name, params, body):
+    assert touches_global(FILES, file, head_of(body)) == []
+
+
+def test_calls_before_the_wait_are_followed():
+    names = {n for f, _, _, body in CHAINED for n, _, _ in reached(FILES, f, head_of(body))}
+    assert {"setup", "init", "row_of", "pick", "tile_m", "tile_n", "args", "attn_fwd_f16_prologue", "attn_bwd_dkdv_f16_prologue",
+            "attn_bwd_dq_from_ds_f16_prologue", "gemm_f16_prologue", "gemm_f16x3_prologue", "mbar_init", "tmem_alloc",
+            "tma_prefetch_desc"} <= names
+
+
+@pytest.mark.parametrize("file,kernel,before,planted", [
+    ("gemm_f32.cu", "gemm_f32_kernel", "        base = b;\n", "        step = (long long)b[r0];\n"),
+    ("gemm_f32.cu", "gemm_f32_kernel", "        base = b;\n", "        step = *(b + r0);\n"),
+    ("gemm_f32.cu", "gemm_f32_kernel", "        base = b;\n", "        cp4(nullptr, b, 4);\n"),
+    ("gemm_f32.cu", "gemm_f32_kernel", "        base = b;\n", "        return b[r0];\n"),
+    ("gemm_f32.cu", "gemm_f32_kernel", "        kbeg = part * g.k_chunk;\n", "        if (g.a[0] > 0.f) return;\n"),
+    ("gemm_f32.cu", "gemm_f32_group_kernel", "        int i = 0;\n", "        if (*g->c > 0.f) ++i;\n"),
+    ("gemm_f16_sm100.cu", "gemm_f16_kernel", "        fence_barrier_init();\n", "        atomicCAS(err, 0u, 1u);\n"),
+    ("gemm_f16_sm100.cu", "gemm_f16_kernel", "        fence_barrier_init();\n", "        tmem_base_s[2] = *(volatile unsigned int*)tmap_a;\n"),
+    ("attn_fwd_f16_sm100.cu", "attn_fwd_f16_kernel", "        fence_barrier_init();\n", "        tmem_base_s[2] = ((const uint32_t*)tmap_q)[0];\n")])
+def test_an_early_access_is_seen(file, kernel, before, planted):
+    """The same sources with an access put into what runs before the wait (as text: nothing of it is built)."""
+    assert before in FILES[file]
+    files = dict(FILES, **{file: FILES[file].replace(before, before + planted)})
+    heads = [head_of(body) for name, _, body in kernels(files[file]) if name == kernel]
+    assert heads and all(touches_global(files, file, h) for h in heads)
+
+
 @pytest.mark.parametrize("file", sorted(FILES))
 def test_no_read_only_loads(file):
     assert not re.search(r"__ldg\(|__ldcs\(|__ldca\(|ld\.global(\.\w+)*\.nc", FILES[file]), file
