@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(1024) cross_entropy_loss_kernel(const float* p
 }
 
 __global__ void __launch_bounds__(256) cross_entropy_bwd_kernel(const float* logits, long long ld, const long long* targets, const float* lse,
-                                                                long long V, float g, float upstream, float* __restrict__ dlogits,
-                                                                long long ldd, int vec) {
+                                                                long long V, float g, float upstream, float* dlogits,
+                                                                long long ldd, int vec) {         // dlogits may be logits
     chain_wait();
     const long long row = blockIdx.y;
     const float* x = logits + row * ld;

@@ -167,7 +167,8 @@ def test_refused_launches_end_the_call(file):
         assert FILES[file][:m.start()].rstrip().endswith("DEERS_CUDA_TRY(ctx,"), FILES[file][m.start():m.start() + 80]
 
 
-def test_rotation_promises_nothing_about_its_buffers():
-    """The model rotates in place: source and destination are one buffer, which a restrict pointer to either would deny."""
-    (body,) = [body for f, name, _, body in CHAINED if name == "rope_pack_kernel"]
-    assert "p.dst" in body and "__restrict__" not in body
+@pytest.mark.parametrize("kernel", ["rope_pack_kernel", "cross_entropy_bwd_kernel"])
+def test_kernels_that_work_in_place_promise_nothing_of_their_buffers(kernel):
+    """Source and destination may be one buffer, which a restrict pointer to either would deny."""
+    (found,) = [params + body[:body.index("__global__") if "__global__" in body else None] for f, name, params, body in CHAINED if name == kernel]
+    assert re.search("p.dst|dlogits", found) and "__restrict__" not in found
