@@ -753,3 +753,13 @@ def test_gpt_train_step_takes_pointers_on_any_boundary():
         said.append((buf[oa:oa + 8].cpu().numpy().tobytes(), [m.parameter(i) for i in range(m.num_parameters())]))
     assert said[0][0] == said[1][0] and np.isfinite(np.frombuffer(said[0][0], np.float32)).all()
     assert all(np.array_equal(a, b) for a, b in zip(said[0][1], said[1][1]))
+
+
+@pytest.mark.parametrize("V,L,H,D,Hm,B,T", [
+    (1024, 1, 12, 86, 64, 1, 5),       # rows of 1032: a block each, in the backward with the normalised row and in the head's f16 pair
+    (1031, 0, 82, 100, 8, 2, 3),       # rows of 8200: no pair in one pass, the head normalises and splits
+    (40, 1, 82, 100, 16, 1, 3),        # ... and two passes of 16-byte loads in the backward
+    (1024, 2, 3, 10, 21, 2, 9)])       # rows of 30: element by element everywhere
+def test_gpt_norms_of_wide_and_ragged_rows(V, L, H, D, Hm, B, T):
+    m, ids, tgt, logits, loss, n, want = _gpt_and_oracle(V, L, H, D, Hm, B, T)
+    _check_gpt(m, logits, loss, want)
