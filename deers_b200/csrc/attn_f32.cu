@@ -12,10 +12,11 @@
 // Within a group thread (ty, tx) of 8 x 8 owns rows 4 ty .. 4 ty + 3 and columns tx, tx + 8, ... of a 32 x BN score tile
 // (4 x 8 or 4 x 4 patches: 12 LDS.128 per 128 FFMA) and rows 4 ty .. with float4 columns 4 tx + 32 j of the
 // accumulators.  Second products run two to an issue slot (forward, and from 64 wide tiles on backward; score products from
-// 96), and lanes lie so that shared-memory reads cost half: B8 H12 T2048 D64 forward 1909 -> 1688 us, backward 5821 -> 5642;
-// B3 H4 T77 D48 forward 10.3 -> 6.8.  Tiles arrive by cp.async: the next K (or Q) is fetched while the current one's scores are turned
-// into the second product, the next V (or dO) while the next scores are computed.
+// 96), and lanes lie so that shared-memory reads cost half.  Tiles arrive by cp.async: the next K (or Q) is fetched while the
+// current one's scores are turned into the second product, the next V (or dO) while the next scores are computed.
+// B8 H12 T2048 D64 forward 1909 -> 1688 us, backward 5821 -> 5642; B3 H4 T77 D48 forward 10.3 -> 6.8.
 #include "common.cuh"
+#include "f32_util.cuh"
 
 #include <type_traits>
 
@@ -40,36 +41,6 @@ struct F32Params {
     const float* cosv; const float* sinv;   // backward: dQ and dK leave rotated back by their position ([T][D / 2]; nullptr: not)
 };
 
-__device__ __forceinline__ void cp16(float* dst, const float* src, int n) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp4(float* dst, const float* src, int n) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-// Two f32 products in one issue slot (each a plain IEEE fma).
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 // Place of a thread in its group's 8 x 8 arrangement.  A quarter warp holds two rows and four columns, neighbouring lanes a
 // column each: a 16-byte shared-memory read along either side then costs 2.1 cycles (4 with lane % 8 along the columns).
 __device__ __forceinline__ int place_y(int t) { return (t / 32) * 4 + (t & 1) + 2 * ((t >> 3) & 1); }
@@ -136,8 +107,9 @@ __device__ __forceinline__ void tile_nt(const float* __restrict__ A, const float
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                const float2 v = unpack2(s2[r][c]);
-                s[r][c] = v.x + v.y;
+                float even, odd;
+                unpack_f32x2(s2[r][c], even, odd);
+                s[r][c] = even + odd;
             }
     } else {
 #pragma unroll
@@ -178,7 +150,8 @@ struct Acc {
 };
 
 // acc[r][2 j], acc[r][2 j + 1] (pairs of columns 4 tx + 32 j ..) += sum_k P[4 ty + r][k] * X[k][..], k < KN (P row stride PLD)
-// PAIRS as above: the 32-wide backward has no registers for the doubled P.
+// PAIRS as above: the 32-wide backward has no registers for the doubled P.  (The 64-wide one spills with them, 136 / 208 bytes of stores /
+// loads where single products spill 64 / 116, and is 1 to 3 % faster all the same.)
 template <int DP, int KN, int PLD, bool PAIRS>
 __device__ __forceinline__ void tile_pv(const float* __restrict__ Ps, const float* __restrict__ X, int ty, int tx, Acc<DP, PAIRS> (&acc)[4]) {
     constexpr int LD = DP + 4;
@@ -198,9 +171,9 @@ __device__ __forceinline__ void tile_pv(const float* __restrict__ Ps, const floa
                 if constexpr (PAIRS) {
                     const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(q);
 #pragma unroll
-                    for (int r = 0; r < 4; ++r) acc[r][2 * j] = fma2(pack2(pr[r], pr[r]), x.x, acc[r][2 * j]);
+                    for (int r = 0; r < 4; ++r) acc[r][2 * j] = fma2(pack_f32x2(pr[r], pr[r]), x.x, acc[r][2 * j]);
 #pragma unroll
-                    for (int r = 0; r < 4; ++r) acc[r][2 * j + 1] = fma2(pack2(pr[r], pr[r]), x.y, acc[r][2 * j + 1]);
+                    for (int r = 0; r < 4; ++r) acc[r][2 * j + 1] = fma2(pack_f32x2(pr[r], pr[r]), x.y, acc[r][2 * j + 1]);
                 } else {
                     const float4 x = *reinterpret_cast<const float4*>(q);
 #pragma unroll
@@ -351,7 +324,7 @@ __global__ void __launch_bounds__(64 * NG, DP <= 32 && NG == 4 ? 2 : 1) attn_fwd
             l[r] = l[r] * alpha + row_sum(rs);
             m[r] = m_new;
 #pragma unroll
-            for (int c = 0; c < DP / 16; ++c) acc[r][c] = mul2(acc[r][c], pack2(alpha, alpha));
+            for (int c = 0; c < DP / 16; ++c) acc[r][c] = mul2(acc[r][c], pack_f32x2(alpha, alpha));
         }
         cp_wait<1>();
         group_sync(g);                                          // V has landed (and this warp's P rows are visible)

@@ -52,7 +52,6 @@ struct X3Params {
 };
 
 // The part of the start that needs nothing of global memory (see started()).
-template <int A_MN, int B_MN>
 __device__ __forceinline__ void gemm_f16x3_prologue(const void* tm_ah, const void* tm_al, const void* tm_bh, const void* tm_bl) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + X_STAGES * X_STAGE);
@@ -74,7 +73,7 @@ template <int A_MN, int B_MN>
 __global__ void __launch_bounds__(X_THREADS, 1)
 gemm_f16x3_kernel(const __grid_constant__ CUtensorMap tm_ah, const __grid_constant__ CUtensorMap tm_al,
                   const __grid_constant__ CUtensorMap tm_bh, const __grid_constant__ CUtensorMap tm_bl, const X3Params p) {
-    gemm_f16x3_prologue<A_MN, B_MN>(&tm_ah, &tm_al, &tm_bh, &tm_bl);
+    gemm_f16x3_prologue(&tm_ah, &tm_al, &tm_bh, &tm_bl);
     chain_wait();
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + X_STAGES * X_STAGE);

@@ -16,21 +16,22 @@
 //     waits and arithmetic of a group are its own, so the groups drift apart and one's shared-memory bursts meet another's
 //     multiply-adds;
 //   * the loop is bound by issue slots, register banks and shared memory together.  Two products share a slot
-//     (fma.rn.f32x2, each an IEEE f32 fma): neighbouring columns where B is in MN order, even and odd k in small K-order
-//     patches (large ones would need twice the accumulators and stay with single products; packing columns there costs
-//     two moves per pair and was slower: 11.4 -> 15.4 us at 1024 x 768 x 192).  Lanes lie in the tile so that a 16-byte
+//     (fma.rn.f32x2, each an IEEE f32 fma): neighbouring columns where B is in MN order, even and odd k in small patches with both
+//     operands in K order (large ones would need twice the accumulators and stay with single products; packing columns there
+//     costs two moves per pair and was slower: 11.4 -> 15.4 us at 1024 x 768 x 192).  Lanes lie in the tile so that a 16-byte
 //     shared-memory read costs 2.1 cycles instead of 4: it does when each quarter warp asks for at most four addresses and
 //     neighbouring lanes share them (lane % 8 along a row does not, (lane / 2) % 4 does; measured);
 //   * operands travel by cp.async straight into shared memory in their storage order (no transposition, no
-//     registers), up to STAGES * 64 k ahead: for K = 192 the whole operand is in flight at once.
-// Back to back in a graph, single products and 512-thread stages before, pairs and groups now (us):
-//   1024 x 768 x 192 11.2 -> 10.7, 1024 x 192 x 768 13.0 -> 12.5, 100 x 576 x 192 3.8 -> 3.5, weight gradients (both
-//   operands in MN order) 768 x 192 x 1024 13.5 -> 10.9, 192 x 500 x 231 4.8 -> 4.0.
+//     registers), up to (STAGES - 1) * 64 k ahead: 192 in tiles of up to 4096 elements, 128 in the wider ones;
 //   * k groups, and the blocks of a cluster that split a long K among them (weight gradients), meet in shared
 //     memory: group 0..KS-1 of block 0..P-1 are added in that order by the threads that write the tile (distributed
 //     shared memory, one cluster barrier), so nothing goes through global memory, no counter, no workspace, and the
 //     result does not depend on timing.
+// Back to back in a graph, with single products and stages shared by 512 threads and now (us): 1024 x 768 x 192 11.4 -> 10.7,
+// 1024 x 192 x 768 13.1 -> 12.5, 231 x 500 x 192 4.0 -> 3.7; both operands in MN order (weight gradients) 192 x 768 x 1024
+// 13.6 -> 11.0, 231 x 500 x 192 4.6 -> 4.1; both in K order with large patches as it was (1024 x 576 x 192 8.5 -> 8.6).
 #include "common.cuh"
+#include "f32_util.cuh"
 
 #include <cooperative_groups.h>
 
@@ -68,32 +69,8 @@ __device__ __forceinline__ float4 ld4(const float* p, int valid, bool vec) {
     return v;
 }
 
-// Asynchronous copies of 16 / 4 bytes; bytes beyond `n` are written as zeros without being read.
-__device__ __forceinline__ void cp16(float* dst, const float* src, int n) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp4(float* dst, const float* src, int n) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 // The threads of a k group meet (barrier 0 is __syncthreads).
 __device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
-
-// Two f32 products in one issue slot (each a plain IEEE fma).
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 
 // One operand's stage of one k group in shared memory, in its storage order: R rows (m or n) of KG k when k is contiguous,
 // KG rows of R when m / n is.  Row strides are 4 mod 16 words (16-byte pieces of neighbouring rows fall into different banks).
@@ -217,7 +194,8 @@ struct GemmShape {
     static constexpr int SQ_AT = STAGES * STAGE > RED ? STAGES * STAGE : RED;    // row sums of squares of the FUSED kernels
     static constexpr size_t NEED = (size_t)(SQ_AT + KS * BM) * sizeof(float);
     // A large block has an SM to itself: two of them share its issue slots while others idle (chained launches place the
-    // next product's blocks before this one's have left).
+    // next product's blocks before this one's have left).  Only the 32 x 64 tiles fit twice: 512 x 512 x 64 4.0 -> 3.2 us, GPT forward of
+    // 4 layers, C 320, 200 tokens 234 -> 204; nothing measured got slower.
     static constexpr size_t ALONE = 116 * 1024;
     static constexpr size_t SMEM = PM * PN >= 16 && NEED < ALONE ? ALONE : NEED;
 };
@@ -347,24 +325,24 @@ __device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED, LOOSE
                         for (int j = 0; j < PN; ++j)
 #pragma unroll
                             for (int i = 0; i < PM; ++i)
-                                acc2[i][j] = fma2(pack2(a[cur][kk][i], a[cur][kk + 1][i]), pack2(b[cur][kk][j], b[cur][kk + 1][j]), acc2[i][j]);
+                                acc2[i][j] = fma2(pack_f32x2(a[cur][kk][i], a[cur][kk + 1][i]), pack_f32x2(b[cur][kk][j], b[cur][kk + 1][j]), acc2[i][j]);
                     }
                 } else if constexpr (PAIR_M) {
                     uint64_t bd[PN];
 #pragma unroll
-                    for (int j = 0; j < PN; ++j) bd[j] = pack2(b[cur][kk][j], b[cur][kk][j]);
+                    for (int j = 0; j < PN; ++j) bd[j] = pack_f32x2(b[cur][kk][j], b[cur][kk][j]);
 #pragma unroll
                     for (int i = 0; i < PM / 2; ++i)
 #pragma unroll
-                        for (int j = 0; j < PN; ++j) acc2[i][j] = fma2(pack2(a[cur][kk][2 * i], a[cur][kk][2 * i + 1]), bd[j], acc2[i][j]);
+                        for (int j = 0; j < PN; ++j) acc2[i][j] = fma2(pack_f32x2(a[cur][kk][2 * i], a[cur][kk][2 * i + 1]), bd[j], acc2[i][j]);
                 } else if constexpr (PAIR_N) {
                     uint64_t ad[PM];
 #pragma unroll
-                    for (int i = 0; i < PM; ++i) ad[i] = pack2(a[cur][kk][i], a[cur][kk][i]);
+                    for (int i = 0; i < PM; ++i) ad[i] = pack_f32x2(a[cur][kk][i], a[cur][kk][i]);
 #pragma unroll
                     for (int j = 0; j < PN / 2; ++j)
 #pragma unroll
-                        for (int i = 0; i < PM; ++i) acc2[i][j] = fma2(ad[i], pack2(b[cur][kk][2 * j], b[cur][kk][2 * j + 1]), acc2[i][j]);
+                        for (int i = 0; i < PM; ++i) acc2[i][j] = fma2(ad[i], pack_f32x2(b[cur][kk][2 * j], b[cur][kk][2 * j + 1]), acc2[i][j]);
                 } else {
 #pragma unroll
                     for (int i = 0; i < PM; ++i)
@@ -381,11 +359,11 @@ __device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED, LOOSE
     for (int i = 0; i < PR; ++i)
 #pragma unroll
         for (int j = 0; j < PC; ++j) {
-            if constexpr (PAIR_M) unpack2(acc2[i][j], acc[2 * i][j], acc[2 * i + 1][j]);
-            if constexpr (PAIR_N) unpack2(acc2[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
+            if constexpr (PAIR_M) unpack_f32x2(acc2[i][j], acc[2 * i][j], acc[2 * i + 1][j]);
+            if constexpr (PAIR_N) unpack_f32x2(acc2[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
             if constexpr (PAIR_K) {
                 float even, odd;
-                unpack2(acc2[i][j], even, odd);
+                unpack_f32x2(acc2[i][j], even, odd);
                 acc[i][j] = even + odd;
             }
         }
@@ -541,10 +519,12 @@ struct GemmPlan {
     double cost;    // cycles
 };
 
-// Tile variants with what was measured of them (cycles at 1.965 GHz, from products of several K in a graph): a
-// block's walk over 64 k, and what a launch costs around it.  The 96-wide tiles are there for products whose 64-wide tiles
-// just miss one wave (1024 x 768: 192 tiles on 148 SMs, 128 of 64 x 96; 13.3 -> 11.7 us at K = 192, and 16.3 -> 13.7 for
-// 1024 x 192 x 768 in clusters of four).
+// Tile variants: the cycles at 1.965 GHz that the choice reckons with, a block's walk over 64 k and what a launch costs around it.
+// They were measured on loops of single products, one figure for every order.  The present ones walk (both in MN order / A in K and B in
+// MN / both in K): 64 x 128 5810 / 6210 / 8180, 64 x 64 2920 / 3680 / 3990, 32 x 64 1850 / 1810 / 2200, 32 x 32 1690 / 1910 / 1740,
+// 64 x 96 4620 / 4710 / 5250, 32 x 96 2430 / 2900 / 3280, and 3800 to 9200 around it (148 tiles, K 320 and 1600).  The 96-wide tiles are
+// there for products whose 64-wide ones just miss one wave (1024 x 768: 192 tiles on 148 SMs, 128 of 64 x 96; 13.3 -> 11.7 us at K =
+// 192, and 16.3 -> 13.7 for 1024 x 192 x 768 in clusters of four).
 struct Variant { int bm, bn; double walk, around; };
 constexpr Variant kVariants[6] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {32, 64, 2360, 4000}, {32, 32, 1680, 3200}, {64, 96, 5400, 5300}, {32, 96, 3200, 4300}};
 

@@ -4,7 +4,7 @@
 //   qkv = rmsnorm(x) * [Wq|Wk|Wv] (one GEMM; the norm's scale and the rotation of q and k in its epilogue); fused attention
 //   reading q, k, v in place as strided views and writing O token-major; x1 = x + O * Wout (residual in the GEMM epilogue);
 //   r = relu(rmsnorm(x1) * Wup), h = r*r (norm and relu in the GEMM); x2 = x1 + h * Wdown (epilogue).
-//   Separate norm and rotary kernels, nine launches per block before, cost 1.4 to 2 us each at these sizes.
+//   Separate norm and rotary kernels, eight launches per block before, cost 1.4 to 2 us each at these sizes.
 // Head: xf = rmsnorm(x) as an f16 pair; logits = xf * Wlm; cross-entropy reads the logits once; the backward overwrites
 // them with their gradient in one pass and feeds the two head GEMMs.
 // Backward: the exact transposes of the above, with the relu^2 backward in a GEMM epilogue, the residual

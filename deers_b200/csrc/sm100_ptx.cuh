@@ -6,6 +6,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include "f32_util.cuh"
+
 namespace sm100 {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -317,30 +319,6 @@ __device__ __forceinline__ uint32_t sw128_chunk_offset(int row, int chunk) {
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&h);
-}
-
-// Two f32 per instruction (fma / add / mul .f32x2, each IEEE f32): they halve the issue slots of the softmax loops.
-__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ uint64_t pack_f32x2(uint32_t lo, uint32_t hi) { return pack_f32x2(__uint_as_float(lo), __uint_as_float(hi)); }
-__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
 }
 
 // Packs 8 f32 values (scaled by s) into eight f16 values: one 16-byte piece of an output row.
