@@ -205,7 +205,7 @@ size_t attn_bwd_f16_workspace_bytes(const deers_attn_desc* d, bool keep_ds);
 int run_selftest_umma(deers_ctx* ctx, float* max_abs_err);
 int run_selftest_wait(deers_ctx* ctx, unsigned int limit_ms, int* result_host);
 
-// f32 GEMM (gemm_f32.cu)
+// f32 GEMM (gemm_f32.cu, gemm_f32_kernel.cuh)
 int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long long lda, int a_mn, const float* b,
                     long long ldb, int b_mn, float* c, long long ldc, int epi, const float* r, long long ldr, float* aux);
 // The same with the rows of A normalised on the way, C [M,N] = rmsnorm(A [M,K]) * B [K,N], all dense: what a block's pre-norms

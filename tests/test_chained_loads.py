@@ -90,9 +90,10 @@ def touches_global(files, file, head):
     """What a kernel's calls before the wait do that could reach global memory: an access through anything but shared memory and
     the arrays of a structure, or an instruction that loads, stores or copies outside shared memory."""
     arrays, found = set(), []
-    for m in re.finditer(r"\bstruct\s+\w+\s*\{", files[file]):                 # arrays that are members
+    text = files[file] + "".join(t for f, t in files.items() if f.endswith(".cuh") and f != file)
+    for m in re.finditer(r"\bstruct\s+\w+\s*\{", text):                        # arrays that are members
         depth, members = 1, ""
-        for c in files[file][m.end():]:
+        for c in text[m.end():]:
             depth += {"{": 1, "}": -1}.get(c, 0)
             if not depth:
                 break
@@ -136,11 +137,11 @@ def test_calls_before_the_wait_are_followed():
 
 
 @pytest.mark.parametrize("file,kernel,before,planted", [
-    ("gemm_f32.cu", "gemm_f32_kernel", "        base = b;\n", "        step = (long long)b[r0];\n"),
-    ("gemm_f32.cu", "gemm_f32_kernel", "        base = b;\n", "        step = *(b + r0);\n"),
-    ("gemm_f32.cu", "gemm_f32_kernel", "        base = b;\n", "        cp4(nullptr, b, 4);\n"),
-    ("gemm_f32.cu", "gemm_f32_kernel", "        base = b;\n", "        return b[r0];\n"),
-    ("gemm_f32.cu", "gemm_f32_kernel", "        kbeg = part * g.k_chunk;\n", "        if (g.a[0] > 0.f) return;\n"),
+    ("gemm_f32_kernel.cuh", "gemm_f32_kernel", "        base = b;\n", "        step = (long long)b[r0];\n"),
+    ("gemm_f32_kernel.cuh", "gemm_f32_kernel", "        base = b;\n", "        step = *(b + r0);\n"),
+    ("gemm_f32_kernel.cuh", "gemm_f32_kernel", "        base = b;\n", "        cp4(nullptr, b, 4);\n"),
+    ("gemm_f32_kernel.cuh", "gemm_f32_kernel", "        base = b;\n", "        return b[r0];\n"),
+    ("gemm_f32_kernel.cuh", "gemm_f32_kernel", "        kbeg = part * g.k_chunk;\n", "        if (g.a[0] > 0.f) return;\n"),
     ("gemm_f32.cu", "gemm_f32_group_kernel", "        int i = 0;\n", "        if (*g->c > 0.f) ++i;\n"),
     ("gemm_f16_sm100.cu", "gemm_f16_kernel", "        fence_barrier_init();\n", "        atomicCAS(err, 0u, 1u);\n"),
     ("gemm_f16_sm100.cu", "gemm_f16_kernel", "        fence_barrier_init();\n", "        tmem_base_s[2] = *(volatile unsigned int*)tmap_a;\n"),
@@ -160,7 +161,7 @@ def test_no_read_only_loads(file):
     assert not re.search(r"const\s+\w+\s*\*\s*__restrict__\s+\w+\s*=", FILES[file]), file
 
 
-@pytest.mark.parametrize("file", sorted(f for f in FILES if f.endswith(".cu")))
+@pytest.mark.parametrize("file", sorted(f for f in FILES if f != "common.cuh"))
 def test_refused_launches_end_the_call(file):
     """Behind a launch that was refused, the next kernel would work on what has not been written."""
     for m in re.finditer(r"launch_chained\(", FILES[file]):
