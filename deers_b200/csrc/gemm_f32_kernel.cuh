@@ -61,7 +61,7 @@ struct GemmPlan {
 };
 
 // Products with an operand whose rows lie on no 16-byte boundary (gemm_f32_loose.cu).  A module of their own: the first product of a
-// process loads all kernels of its module, and most programs never need these (first training step of a process 9 ms, 17 with them).
+// process loads all kernels of its module, and most programs never need these (first training step of a process 8.4 ms, 17 with them).
 int launch_gemm_f32_loose(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g, int a_mn, int b_mn, bool fused);
 
 namespace {
