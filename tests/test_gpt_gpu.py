@@ -154,14 +154,14 @@ def gemm_f32_us(M, N, K, a_mn, b_mn):
 @pytest.mark.parametrize("M,N,K", [(192, 768, 1024), (16, 4096, 1024)])
 def test_gemm_f32_storage_orders_cost_alike(M, N, K):
     """A in MN with B in K order takes 0.96 times as long as both in K order (measured); 1.32 when its products went in pairs over k."""
-    assert gemm_f32_us(M, N, K, 1, 0) < 1.18 * gemm_f32_us(M, N, K, 0, 0)
+    assert gemm_f32_us(M, N, K, 1, 0) < 1.25 * gemm_f32_us(M, N, K, 0, 0)
 
 
 @pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(66, 249, 689, 0, 0), (1306, 19, 1574, 0, 0), (2133, 769, 1405, 0, 0)])
 def test_gemm_f32_rows_on_no_boundary_cost_little_more(M, N, K, a_mn, b_mn):
     """0.92 to 1.05 times the product of the next multiples of four (measured); 1.32 to 1.52 when a lane copied four floats in turn."""
     up = [(n + 3) // 4 * 4 for n in (M, N, K)]
-    assert gemm_f32_us(M, N, K, a_mn, b_mn) < 1.18 * gemm_f32_us(*up, a_mn, b_mn)
+    assert gemm_f32_us(M, N, K, a_mn, b_mn) < 1.25 * gemm_f32_us(*up, a_mn, b_mn)
 
 
 def test_gemm_f32_rejects_bad_arguments():
