@@ -763,3 +763,15 @@ def test_gpt_train_step_takes_pointers_on_any_boundary():
 def test_gpt_norms_of_wide_and_ragged_rows(V, L, H, D, Hm, B, T):
     m, ids, tgt, logits, loss, n, want = _gpt_and_oracle(V, L, H, D, Hm, B, T)
     _check_gpt(m, logits, loss, want)
+
+
+@pytest.mark.parametrize("n,V,C", [(1, 1, 5), (257, 2, 24), (1023, 40, 33), (1025, 3, 8), (2600, 7, 2049), (3000, 100000, 16)])
+def test_embedding_backward_of_repeated_ids(n, V, C):
+    """Ids that repeat within and across the 1024 looked at together, up to every token the same: the sum in token order, bit for bit."""
+    from deers_b200 import gpt
+    from oracle import ref
+    rng = np.random.default_rng(n)
+    ids, d = rng.integers(0, V, n), rng.standard_normal((n, C)).astype(np.float32)
+    got = gpt.embedding_backward(torch.from_numpy(d).cuda(), torch.from_numpy(ids).cuda(), V)
+    torch.cuda.synchronize()
+    assert np.array_equal(got.cpu().numpy(), ref.embedding_bwd(d, ids, V))
