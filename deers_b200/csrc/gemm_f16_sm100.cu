@@ -10,15 +10,15 @@
 //     dgrad    dx = dy  * W^T    : A = dy [M,N]  K-major,  B = W  [K,N] read as [N'=K, K'=N]: K-major
 //     wgrad    dW = x^T * dy     : A = x  [m,K]  read as [K'=m, M'=K]: MN-major,  B = dy [m,N] MN-major
 // Persistent: one CTA per SM walks 128 x 256 (or 192) output tiles (consecutive CTAs share a B column block, which
-// L2 then serves).  Warp 0 streams 64-deep K blocks of A (16 KB) and B (32 KB) through a 4-stage ring (TMA,
+// L2 then serves), or a pair of CTAs on two SMs walks tiles of 256 x 256.  Warp 0 streams 64-deep K blocks of A (16 KB) and B (32 KB) through a 4-stage ring (TMA,
 // 128-byte swizzle, out-of-range rows / columns read as zero), warp 1 issues four 128x256x16 tcgen05.mma
-// per K block into one of two TMEM accumulators, warps 2-5 move a finished accumulator to
+// per K block into one of two TMEM accumulators, warps 2-9 move a finished accumulator to
 // registers 64 columns at a time, convert to f16 and store rows transposed within 8-lane groups
 // (contiguous 128-byte segments), then release the accumulator.
 // Few tiles and a long K (weight gradients) leave most SMs idle: there a cluster of CTAs shares a tile and its K
 // (768 x 768 x 8192: 18 tiles, 51 us on 18 SMs; 22 us as 24 narrower tiles of five parts.  768 x 2304 x 8192: 52 -> 31 us).
 // 192 columns where 256-wide tiles just miss a wave (8192 x 768 x 2304: 192 tiles on 148 SMs, 29 us; 256 tiles 24 us).
-// Bound: tensor pipe for large products (4096^3: 1.3 PFLOP/s), L2 reads of both operands for the split ones.
+// Bound: tensor pipe for large products (4096^3: 1.38 PFLOP/s by pairs, 1.25 without), L2 reads of both operands for the split ones.
 #include "sm100_ptx.cuh"
 #include "tma_host.cuh"
 
@@ -30,19 +30,26 @@ using namespace sm100;
 
 constexpr int GM = 128, GK = 64;                // output tile rows and K block
 constexpr uint32_t G_A_BYTES = GM * GK * 2;     // 16 KB per stage
-constexpr int G_STAGES = 4;
-constexpr int G_THREADS = 192;
+constexpr int G_EPI_WG = 2;                     // epilogue warpgroups, each with half of a tile's columns
+constexpr int G_THREADS = 64 + 128 * G_EPI_WG;
 constexpr int G_MAX_PARTS = 6;                  // CTAs of a cluster along K (of eight only 15 clusters fit the device)
-// Shared memory for tiles of gn columns: the ring; a split-K CTA then parks its f32 partial tile (rows of gn + 4) over it.
-constexpr uint32_t g_ring(int gn) { return G_STAGES * (G_A_BYTES + (uint32_t)gn * GK * 2u); }
-constexpr uint32_t g_smem(int gn) { return g_ring(gn) + 256; }
-static_assert((uint32_t)GM * (256 + 4) * 4 <= g_ring(256) && (uint32_t)GM * (192 + 4) * 4 <= g_ring(192), "partial tile fits over the ring");
+// Tiles of GN columns by one CTA, or of 256 rows by a pair of CTAs, each with half of the rows and half of B's columns.
+template <int GN, bool PAIR>
+struct GemmShape {
+    static constexpr int BN = PAIR ? GN / 2 : GN;                            // columns of B in a CTA's stage
+    static constexpr uint32_t B_BYTES = BN * GK * 2u;
+    static constexpr int STAGES = PAIR ? 6 : 4;
+    static constexpr uint32_t RING = STAGES * (G_A_BYTES + B_BYTES);         // a split-K CTA parks its f32 partial tile (rows of GN + 4) over it
+    static constexpr uint32_t SMEM = RING + 256;
+    static_assert((uint32_t)GM * (GN + 4) * 4 <= RING && SMEM <= 232448, "partial tile fits over the ring, and the ring in shared memory");
+    // barriers
+    static constexpr int FULL = 0, EMPTY = STAGES, ACC_FULL = 2 * STAGES, ACC_EMPTY = ACC_FULL + 2, COUNT = ACC_EMPTY + 2;
+    static_assert(COUNT * 8 + 16 <= 256, "barriers");
+};
 // Shared-memory layouts of a stage (what the TMA boxes below write, 128-byte swizzle):
 //   K-major operand of R rows (R = 128 for A, 256 for B): one block of R rows x 64 K-columns (R * 128 bytes)
 //   MN-major operand of C columns (C = 128 / 256): C / 64 blocks of 64 K-rows x 64 columns (8 KB each)
 constexpr uint32_t G_MN_BLOCK = GK * 128;       // 8 KB
-
-enum GBar { G_FULL = 0, G_EMPTY = 4, G_ACC_FULL = 8, G_ACC_EMPTY = 10, G_COUNT = 12 };
 
 struct GemmParams {
     __half* c;
@@ -53,53 +60,66 @@ struct GemmParams {
 };
 
 // The part of the start that needs nothing of global memory (see started()).
-template <int GN>
+template <int GN, bool PAIR>
 __device__ __forceinline__ void gemm_f16_prologue(const void* tmap_a, const void* tmap_b) {
+    using S = GemmShape<GN, PAIR>;
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + G_STAGES * (G_A_BYTES + GN * GK * 2));
-    uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + G_COUNT);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::RING);
+    uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + S::COUNT);
     if (threadIdx.x == 0) {
         tmem_base_s[1] = 0;                                     // the abort flag
         tmem_base_s[3] = 0;                                     // epilogue threads whose rows are parked
-        for (int s = 0; s < G_STAGES; ++s) { mbar_init(&bars[G_FULL + s], 1); mbar_init(&bars[G_EMPTY + s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&bars[G_ACC_FULL + s], 1); mbar_init(&bars[G_ACC_EMPTY + s], 128); }
+        for (int s = 0; s < S::STAGES; ++s) { mbar_init(&bars[S::FULL + s], 1); mbar_init(&bars[S::EMPTY + s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&bars[S::ACC_FULL + s], 1); mbar_init(&bars[S::ACC_EMPTY + s], (PAIR ? 8 : 4) * G_EPI_WG); }
         fence_barrier_init();
         tma_prefetch_desc(tmap_a); tma_prefetch_desc(tmap_b);
     }
     if (uniform((int)threadIdx.x / 32) == 1) {
-        tmem_alloc(tmem_base_s, 512);
-        tmem_relinquish();
+        if (PAIR) { tmem_alloc_pair(tmem_base_s, 512); tmem_relinquish_pair(); }
+        else { tmem_alloc(tmem_base_s, 512); tmem_relinquish(); }
     }
 }
 
 // SPLIT: one tile per cluster, whose CTAs take a share of K each; the partial tiles meet in distributed shared memory and are
 // added in the order of their K ranges (reproducible, no workspace).
-template <int A_MN, int B_MN, int GN, bool SPLIT>
+// PAIR: a cluster of two, the first of which issues the products of both; either brings its rows of A and half of B's columns and
+// finishes its own 128 rows.  A CTA alone is held up by its shared memory: a stage's operands arrive there and are read from it at
+// 187 bytes a cycle against the 128 it has; of a pair's, B is read from both memories, 128.
+template <int A_MN, int B_MN, int GN, bool SPLIT, bool PAIR>
 __global__ void __launch_bounds__(G_THREADS, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
-    gemm_f16_prologue<GN>(&tmap_a, &tmap_b);
+    gemm_f16_prologue<GN, PAIR>(&tmap_a, &tmap_b);
     chain_wait();
+    namespace cg = cooperative_groups;
+    using S = GemmShape<GN, PAIR>;
     extern __shared__ __align__(1024) uint8_t smem[];
-    constexpr uint32_t G_B_BYTES = GN * GK * 2;
+    constexpr int G_STAGES = S::STAGES, TM = PAIR ? 2 * GM : GM;
+    constexpr uint32_t G_B_BYTES = S::B_BYTES;
     uint8_t* sA = smem;
     uint8_t* sB = smem + G_STAGES * G_A_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + G_STAGES * (G_A_BYTES + G_B_BYTES));
-    uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + G_COUNT);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::RING);
+    uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + S::COUNT);
     volatile uint32_t* abort_s = tmem_base_s + 1;
     uint32_t* skip_s = tmem_base_s + 2;
 
     const int warp = uniform((int)threadIdx.x / 32), lane = threadIdx.x % 32;
-    const int tiles_m = (p.M + GM - 1) / GM, tiles_n = (p.N + GN - 1) / GN;
+    const int tiles_m = (p.M + TM - 1) / TM, tiles_n = (p.N + GN - 1) / GN;
     const int n_tiles = tiles_m * tiles_n;
+    static_assert(!(SPLIT && PAIR), "pairs do not share K");
     const int kb_all = (p.K + GK - 1) / GK;
-    const int parts = SPLIT ? (int)cooperative_groups::this_cluster().num_blocks() : 1;
-    const int part = SPLIT ? (int)cooperative_groups::this_cluster().block_rank() : 0;
+    const int rank = SPLIT || PAIR ? (int)cg::this_cluster().block_rank() : 0, half = PAIR ? rank & 1 : 0;
+    const int group = SPLIT ? (int)cg::this_cluster().num_blocks() : PAIR ? 2 : 1;             // CTAs per tile
+    const int parts = SPLIT ? group : 1, part = SPLIT ? rank : 0;
     const int kb0 = part * p.kb_chunk, kb1 = SPLIT ? min(kb_all, kb0 + p.kb_chunk) : kb_all;   // this CTA's K blocks: never none
-    const int t0 = SPLIT ? (int)blockIdx.x / parts : (int)blockIdx.x, t_step = SPLIT ? n_tiles : (int)gridDim.x;
+    const int t0 = (int)blockIdx.x / group, t_step = SPLIT ? n_tiles : (int)gridDim.x / group;
 
-    // (a split-K CTA stays: its peers read its shared memory)
-    const bool skip = !started(smem, skip_s, p.err, DEERS_KERR_GEMM | 0x20);
-    if (!SPLIT && skip) {
+    // (a CTA of a cluster stays: its peers read its shared memory)
+    bool skip = !started(smem, skip_s, p.err, DEERS_KERR_GEMM | 0x20);
+    if constexpr (PAIR) {
+        cg::this_cluster().sync();                          // both have their barriers, and both go on or neither
+        skip = skip || *cg::this_cluster().map_shared_rank(skip_s, rank ^ 1) != 0;
+    }
+    if (!SPLIT && !PAIR && skip) {
         if (warp == 1) tmem_dealloc(*tmem_base_s, 512);
         return;
     }
@@ -117,24 +137,29 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
                 const int tm = t % tiles_m, tn = t / tiles_m;
                 for (int kb = kb0; kb < kb1; ++kb, ++g) {
                     const uint32_t s = g % G_STAGES;
-                    if (!mbar_wait(ws, &bars[G_EMPTY + s], ((g / G_STAGES) & 1u) ^ 1u, DEERS_KERR_GEMM | 1)) { ok = false; break; }
-                    mbar_arrive_expect_tx(&bars[G_FULL + s], G_A_BYTES + G_B_BYTES);
+                    if (!mbar_wait(ws, &bars[S::EMPTY + s], ((g / G_STAGES) & 1u) ^ 1u, DEERS_KERR_GEMM | 1)) { ok = false; break; }
+                    // (a pair's stage is announced at its first CTA, for the bytes of both)
+                    constexpr uint32_t BYTES = G_A_BYTES + G_B_BYTES;
+                    if (half == 0) mbar_arrive_expect_tx(&bars[S::FULL + s], PAIR ? 2 * BYTES : BYTES);
                     uint8_t* a_dst = sA + s * G_A_BYTES;
                     uint8_t* b_dst = sB + s * G_B_BYTES;
+                    const int m0 = tm * TM + half * GM, n0 = tn * GN + half * S::BN;
+                    const auto load = [&](uint8_t* dst, const CUtensorMap* map, int x, int y) {
+                        if constexpr (PAIR) tma_load_4d_pair(dst, map, cluster_addr(&bars[S::FULL + s], 0), x, y, 0, 0);
+                        else tma_load_4d(dst, map, &bars[S::FULL + s], x, y, 0, 0);
+                    };
                     // K-major: box {64 of K, rows}; MN-major: boxes {64 of M / N, 64 rows of K}
                     if (A_MN) {
 #pragma unroll
-                        for (int blk = 0; blk < GM / 64; ++blk)
-                            tma_load_4d(a_dst + blk * G_MN_BLOCK, &tmap_a, &bars[G_FULL + s], tm * GM + blk * 64, kb * GK, 0, 0);
+                        for (int blk = 0; blk < GM / 64; ++blk) load(a_dst + blk * G_MN_BLOCK, &tmap_a, m0 + blk * 64, kb * GK);
                     } else {
-                        tma_load_4d(a_dst, &tmap_a, &bars[G_FULL + s], kb * GK, tm * GM, 0, 0);
+                        load(a_dst, &tmap_a, kb * GK, m0);
                     }
                     if (B_MN) {
 #pragma unroll
-                        for (int blk = 0; blk < GN / 64; ++blk)
-                            tma_load_4d(b_dst + blk * G_MN_BLOCK, &tmap_b, &bars[G_FULL + s], tn * GN + blk * 64, kb * GK, 0, 0);
+                        for (int blk = 0; blk < S::BN / 64; ++blk) load(b_dst + blk * G_MN_BLOCK, &tmap_b, n0 + blk * 64, kb * GK);
                     } else {
-                        tma_load_4d(b_dst, &tmap_b, &bars[G_FULL + s], kb * GK, tn * GN, 0, 0);
+                        load(b_dst, &tmap_b, kb * GK, n0);
                     }
                 }
             }
@@ -144,8 +169,12 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp runs this; one elected lane issues (see elect_one).
-        {
-            constexpr uint32_t IDESC = idesc_f16(GM, GN, A_MN, B_MN);
+        if (half == 0) {
+            constexpr uint32_t IDESC = idesc_f16(TM, GN, A_MN, B_MN);
+                        const auto commit = [&](uint64_t* bar) {
+                if constexpr (PAIR) umma_commit_pair(bar, 3u);
+                else umma_commit(bar);
+            };
             constexpr uint64_t A_STEP = G_A_BYTES >> 4, B_STEP = G_B_BYTES >> 4;
             const uint32_t sa0 = (uint32_t)uniform((int)smem_u32(sA)), sb0 = (uint32_t)uniform((int)smem_u32(sB));
             const uint64_t a0 = A_MN ? desc_mnmajor(sa0, 0, G_MN_BLOCK) : desc_kmajor(sa0, 0, 0);
@@ -155,19 +184,22 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             bool ok = true;
             for (int t = t0; ok && t < n_tiles; t += t_step, ++n) {
                 const uint32_t buf = (uint32_t)n & 1u;
-                if (!mbar_wait_warp(ws, &bars[G_ACC_EMPTY + buf], (((uint32_t)n >> 1) & 1u) ^ 1u, DEERS_KERR_GEMM | 2)) break;
+                if (!mbar_wait_warp(ws, &bars[S::ACC_EMPTY + buf], (((uint32_t)n >> 1) & 1u) ^ 1u, DEERS_KERR_GEMM | 2)) break;
+                if (PAIR) fence_acq_rel_cluster();
                 for (int kb = kb0; kb < kb1; ++kb, ++g) {
                     const uint32_t s = g % G_STAGES;
-                    if (!mbar_wait_warp(ws, &bars[G_FULL + s], (g / G_STAGES) & 1u, DEERS_KERR_GEMM | 3)) { ok = false; break; }
+                    if (!mbar_wait_warp(ws, &bars[S::FULL + s], (g / G_STAGES) & 1u, DEERS_KERR_GEMM | 3)) { ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t a = a0 + (uint64_t)s * A_STEP, b = b0 + (uint64_t)s * B_STEP;
                     if (elect_one()) {
 #pragma unroll
-                        for (int ks = 0; ks < GK / 16; ++ks)               // ks < 4: a K-major step stays inside its block
-                            umma_ss(tmem + buf * 256u, a + (A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0)),
-                                    b + (B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0)), IDESC, (kb > kb0 || ks > 0));
-                        umma_commit(&bars[G_EMPTY + s]);
-                        if (kb == kb1 - 1) umma_commit(&bars[G_ACC_FULL + buf]);
+                        for (int ks = 0; ks < GK / 16; ++ks) {             // ks < 4: a K-major step stays inside its block
+                            const uint64_t ad = a + (A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0)), bd = b + (B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0));
+                            if constexpr (PAIR) umma_ss_pair(tmem + buf * 256u, ad, bd, IDESC, (kb > kb0 || ks > 0));
+                            else umma_ss(tmem + buf * 256u, ad, bd, IDESC, (kb > kb0 || ks > 0));
+                        }
+                        commit(&bars[S::EMPTY + s]);
+                        if (kb == kb1 - 1) commit(&bars[S::ACC_FULL + buf]);
                     }
                     __syncwarp();
                 }
@@ -177,17 +209,19 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         // ------------------------------ epilogue ------------------------------
         const int lane_base = (warp & 3) * 32;
         const uint32_t t_lane = (uint32_t)lane_base << 16;
+        constexpr int SHARE = GN / G_EPI_WG, CH = SHARE % 64 ? 32 : 64;      // a warpgroup's columns, and those it takes at a time
+        const int share0 = ((warp - 2) >> 2) * SHARE;
         int n = 0;
         for (int t = t0; t < n_tiles; t += t_step, ++n) {
             const int tm = t % tiles_m, tn = t / tiles_m;
             const uint32_t buf = (uint32_t)n & 1u;
-            if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[G_ACC_FULL + buf], ((uint32_t)n >> 1) & 1u, DEERS_KERR_GEMM | 4))) { done = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(ws, &bars[S::ACC_FULL + buf], ((uint32_t)n >> 1) & 1u, DEERS_KERR_GEMM | 4))) { done = false; break; }
             tc_fence_after_sync();
             if constexpr (SPLIT) {
                 // every product of this CTA has finished: the ring is free for its partial tile
                 float* row = reinterpret_cast<float*>(smem) + (lane_base + lane) * (GN + 4);
 #pragma unroll 1
-                for (int c0 = 0; c0 < GN; c0 += 32) {
+                for (int c0 = share0; c0 < share0 + SHARE; c0 += 32) {
                     uint32_t r[32];
                     tmem_ld_x32(tmem + t_lane + c0, r);
                     tmem_wait_ld();
@@ -196,24 +230,26 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
                 }
                 break;
             }
-            const int row0 = tm * GM + lane_base + (lane & ~7);
+            constexpr int NP = CH / 8;                          // 16-byte pieces of a row
+            const int row0 = tm * TM + half * GM + lane_base + (lane & ~(NP - 1));
 #pragma unroll 1
-            for (int part = 0; part < GN / 64; ++part) {        // 64 columns at a time
-                uint32_t r[64];
-                uint4 pc[8];
-                tmem_ld_x32(tmem + buf * 256u + t_lane + part * 64, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-                tmem_ld_x32(tmem + buf * 256u + t_lane + part * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+            for (int c0 = share0; c0 < share0 + SHARE; c0 += CH) {
+                uint32_t r[CH];
+                uint4 pc[NP];
+#pragma unroll
+                for (int c = 0; c < CH; c += 32) tmem_ld_x32(tmem + buf * 256u + t_lane + c0 + c, *reinterpret_cast<uint32_t(*)[32]>(&r[c]));
                 tmem_wait_ld();
-                if (part == GN / 64 - 1) {                      // accumulator is in registers: the next tile may use it
+                if (c0 == share0 + SHARE - CH) {                // this warp's share of the accumulator is in registers
                     tc_fence_before_sync();
-                    mbar_arrive(&bars[G_ACC_EMPTY + buf]);
+                    if constexpr (PAIR) mbar_arrive_cluster_warp(cluster_addr(&bars[S::ACC_EMPTY + buf], 0));
+                    else mbar_arrive_warp(&bars[S::ACC_EMPTY + buf]);
                 }
 #pragma unroll
-                for (int q8 = 0; q8 < 8; ++q8) pc[q8] = pack8_f16(r + q8 * 8, 1.0f);
-                transpose_pieces<8>(pc, (uint32_t)lane);
-                const int col = tn * GN + part * 64 + (lane & 7) * 8;
+                for (int q8 = 0; q8 < NP; ++q8) pc[q8] = pack8_f16(r + q8 * 8, 1.0f);
+                transpose_pieces<NP>(pc, (uint32_t)lane);
+                const int col = tn * GN + c0 + (lane & (NP - 1)) * 8;
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
+                for (int c = 0; c < NP; ++c) {
                     const int row = row0 + c;
                     if (row < p.M && col < p.N) *reinterpret_cast<uint4*>(p.c + (long long)row * p.ldc + col) = pc[c];
                 }
@@ -221,14 +257,13 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         }
     }
     if constexpr (SPLIT) {
-        namespace cg = cooperative_groups;
         cg::cluster_group cluster = cg::this_cluster();
         uint32_t* have_s = skip_s + 1;                          // (zeroed at the start) epilogue threads whose rows are parked
         if (warp >= 2 && done) atomicAdd(have_s, 1u);
         __syncwarp();
         cluster.sync();
         bool all = true;
-        for (int z = 0; z < parts; ++z) all = all && *cluster.map_shared_rank(have_s, z) == 128u;
+        for (int z = 0; z < parts; ++z) all = all && *cluster.map_shared_rank(have_s, z) == 128u * G_EPI_WG;
         const int tm = t0 % tiles_m, tn = t0 / tiles_m;
         const int share = (GM + parts - 1) / parts, r_end = min(GM, (part + 1) * share);
         if (all) {
@@ -276,12 +311,15 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
                 default: add(std::integral_constant<int, 6>()); break;
             }
         }
-        cluster.sync();                                         // nobody leaves while a peer still reads its partial tile
     }
     __syncwarp();
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, 512);
+    if constexpr (SPLIT || PAIR) cg::this_cluster().sync();     // nobody leaves while a peer still reads its memory or arrives at its barriers
+    if (warp == 1) {
+        if constexpr (PAIR) tmem_dealloc_pair(tmem, 512);
+        else tmem_dealloc(tmem, 512);
+    }
 }
 
 // 2-D tensor map over a row-major f16 matrix [rows][inner] with leading dimension ld (elements).
@@ -291,45 +329,50 @@ int make_tmap_matrix(deers_ctx* ctx, CUtensorMap* out, const void* base, long lo
     return make_tmap_bhtd_f16(ctx, out, base, 1, 1, (int)rows, (int)inner, strides, box_rows);
 }
 
-struct GemmPlan { int gn, parts, kb_chunk; };
+struct GemmPlan { int gn, parts, kb_chunk; bool pair; };
 
 // Clusters of n CTAs (one per SM) the device holds at a time.
 int cluster_room(deers_ctx* ctx) {
     if (ctx->cluster_room_f16[1] > 0) return DEERS_OK;
-    static std::atomic<int> known[64][G_MAX_PARTS + 1];                    // asked once per device: a tenth of a millisecond each
+    constexpr int MOST = G_MAX_PARTS;
+    static std::atomic<int> known[64][MOST + 1];                           // asked once per device: a tenth of a millisecond each
     std::atomic<int>* dev = known[ctx->device & 63];
     if (dev[1].load(std::memory_order_acquire) > 0) {
-        for (int parts = 1; parts <= G_MAX_PARTS; ++parts) ctx->cluster_room_f16[parts] = dev[parts].load(std::memory_order_relaxed);
+        for (int n = 1; n <= MOST; ++n) ctx->cluster_room_f16[n] = dev[n].load(std::memory_order_relaxed);
         return DEERS_OK;
     }
-    const auto kernel = gemm_f16_kernel<0, 1, 256, true>;
-    DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<0, 1, 256, true>), g_smem(256));
-    for (int parts = 2; parts <= G_MAX_PARTS; ++parts) {
+    using S = GemmShape<256, false>;
+    const auto kernel = gemm_f16_kernel<0, 1, 256, true, false>;
+    DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<0, 1, 256, true, false>), S::SMEM);
+    for (int n = 2; n <= MOST; ++n) {
         cudaLaunchConfig_t lc{};
-        lc.gridDim = dim3(parts);
+        lc.gridDim = dim3(n);
         lc.blockDim = dim3(G_THREADS);
-        lc.dynamicSmemBytes = g_smem(256);
+        lc.dynamicSmemBytes = S::SMEM;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)parts; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        at[0].val.clusterDim.x = (unsigned)n; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         lc.attrs = at; lc.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kernel, &lc) != cudaSuccess) { cudaGetLastError(); n = 0; }
-        ctx->cluster_room_f16[parts] = n;
-        dev[parts].store(n, std::memory_order_relaxed);
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &lc) != cudaSuccess) { cudaGetLastError(); clusters = 0; }
+        ctx->cluster_room_f16[n] = clusters;
+        dev[n].store(clusters, std::memory_order_relaxed);
     }
     ctx->cluster_room_f16[1] = ctx->sm_count;
     dev[1].store(ctx->sm_count, std::memory_order_release);
     return DEERS_OK;
 }
 
-// Tile width and K split with the least estimated time, in microseconds as measured: a K block takes 0.40 with 256 columns and
-// 0.335 with 192 (A passes through shared memory as often), the tiles an SM has to take follow one another, and a meeting of
-// the parts costs 4.0 + 0.9 for each (launch of the cluster, partial tiles through shared memory, two cluster barriers).
+// Tile width, K split, and pair or single CTA, with the least estimated time, in microseconds as measured: a K block takes 0.40 with
+// 256 columns and 0.335 with 192 (A passes through shared memory as often), 0.35 with a pair's 256 x 256, whose launch costs 1.5 more; the
+// tiles an SM has to take follow one another, and a meeting of the parts costs 4.0 + 0.9 for each (launch of the cluster, partial tiles
+// through shared memory, two cluster barriers).  Pairs and the best of the others: 8192 x 2304 x 768 24.4 and 26.2 us, 4096^3 100 and 110,
+// 16384 x 6144 x 2048 298 and 340, 2048 x 6144 x 16384 335 and 462; 8192 x 768 x 2304 28.7 and 24.0, 1024 x 1536 x 512 8.1 and 6.2.  Pairs on
+// 192 columns and pairs that share K were never the quickest (768 x 2304 x 8192 31.0 and 29.1, 8192 x 768 x 768 13.5 and 12.4).
 GemmPlan plan_gemm_f16(deers_ctx* ctx, int M, int N, int K) {
-    GemmPlan best{256, 1, (K + GK - 1) / GK};
-    double best_cost = -1.0;
     const int kb = (K + GK - 1) / GK;
+    GemmPlan best{256, 1, kb, false};
+    double best_cost = -1.0;
     for (int gn = 256; gn >= 192; gn -= 64) {
         const long long tiles = (long long)((M + GM - 1) / GM) * ((N + gn - 1) / gn);
         for (int parts = 1; parts <= G_MAX_PARTS; ++parts) {
@@ -338,26 +381,35 @@ GemmPlan plan_gemm_f16(deers_ctx* ctx, int M, int N, int K) {
             if (room < 1 || (parts > 1 && (chunk < 4 || chunk * (parts - 1) >= kb))) continue;      // no empty part
             const double waves = (double)((tiles + room - 1) / room);
             const double cost = waves * (chunk * (gn == 256 ? 0.40 : 0.335) + (parts > 1 ? 4.0 + 0.9 * parts : 0.4));
-            if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = GemmPlan{gn, parts, chunk}; }
+            if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = GemmPlan{gn, parts, chunk, false}; }
         }
+    }
+    const int pairs = ctx->cluster_room_f16[2];
+    if (pairs > 0) {
+        const long long tiles = (long long)((M + 2 * GM - 1) / (2 * GM)) * ((N + 255) / 256);
+        const double cost = (double)((tiles + pairs - 1) / pairs) * (kb * 0.35 + 0.4) + 1.5;
+        if (cost < best_cost) best = GemmPlan{256, 1, kb, true};
     }
     return best;
 }
 
-template <int A_MN, int B_MN, int GN>
+template <int A_MN, int B_MN, int GN, bool PAIR>
 int gemm_launch(deers_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int parts) {
-    const long long tiles = (long long)((p.M + GM - 1) / GM) * ((p.N + GN - 1) / GN);
+    using S = GemmShape<GN, PAIR>;
+    constexpr int TM = PAIR ? 2 * GM : GM, CTAS = PAIR ? 2 : 1;
+    const long long tiles = (long long)((p.M + TM - 1) / TM) * ((p.N + GN - 1) / GN);
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM);
-        if (parts == 1) {
-            DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<A_MN, B_MN, GN, false>), g_smem(GN));
-            const unsigned grid = (unsigned)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
+        if (PAIR || parts == 1) {
+            DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<A_MN, B_MN, GN, false, PAIR>), S::SMEM);
+            const int room = ctx->cluster_room_f16[CTAS];
+            const unsigned grid = (unsigned)(tiles < room ? tiles : room);
             const ChainScope chain(ctx, tiles * p.kb_chunk / grid);
-            DEERS_CUDA_TRY(ctx, launch_chained(ctx, gemm_f16_kernel<A_MN, B_MN, GN, false>, grid, G_THREADS, g_smem(GN), 1, ta, tb, p));
-        } else {
-            const auto kernel = gemm_f16_kernel<A_MN, B_MN, GN, true>;
-            DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<A_MN, B_MN, GN, true>), g_smem(GN));
-            DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, (unsigned)(tiles * parts), G_THREADS, g_smem(GN), parts, ta, tb, p));
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, gemm_f16_kernel<A_MN, B_MN, GN, false, PAIR>, grid * CTAS, G_THREADS, S::SMEM, CTAS, ta, tb, p));
+        } else if constexpr (!PAIR) {
+            const auto kernel = gemm_f16_kernel<A_MN, B_MN, GN, true, false>;
+            DEERS_SMEM_ONCE(ctx, (gemm_f16_kernel<A_MN, B_MN, GN, true, false>), S::SMEM);
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, (unsigned)(tiles * parts), G_THREADS, S::SMEM, parts, ta, tb, p));
         }
     }
     ctx->launches += 1;
@@ -365,10 +417,10 @@ int gemm_launch(deers_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, co
     return DEERS_OK;
 }
 
-template <int GN>
+template <int GN, bool PAIR>
 int gemm_orders(deers_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int parts, int a_mn, int b_mn) {
-    if (a_mn) return b_mn ? gemm_launch<1, 1, GN>(ctx, ta, tb, p, parts) : gemm_launch<1, 0, GN>(ctx, ta, tb, p, parts);
-    return b_mn ? gemm_launch<0, 1, GN>(ctx, ta, tb, p, parts) : gemm_launch<0, 0, GN>(ctx, ta, tb, p, parts);
+    if (a_mn) return b_mn ? gemm_launch<1, 1, GN, PAIR>(ctx, ta, tb, p, parts) : gemm_launch<1, 0, GN, PAIR>(ctx, ta, tb, p, parts);
+    return b_mn ? gemm_launch<0, 1, GN, PAIR>(ctx, ta, tb, p, parts) : gemm_launch<0, 0, GN, PAIR>(ctx, ta, tb, p, parts);
 }
 
 }  // namespace
@@ -389,9 +441,9 @@ extern "C" int deers_b200_gemm_f16(deers_ctx* ctx, int32_t M, int32_t N, int32_t
     // K-major A: [M rows][K inner], box {64, 128}; MN-major A: [K rows][M inner], box {64, 64}.  Same for B with
     // N (K-major box {64, tile columns}).
     if ((rc = a_mn_major ? make_tmap_matrix(ctx, &ta, a, K, M, lda, GK) : make_tmap_matrix(ctx, &ta, a, M, K, lda, GM))) return rc;
-    if ((rc = b_mn_major ? make_tmap_matrix(ctx, &tb, b, K, N, ldb, GK) : make_tmap_matrix(ctx, &tb, b, N, K, ldb, plan.gn))) return rc;
+    if ((rc = b_mn_major ? make_tmap_matrix(ctx, &tb, b, K, N, ldb, GK) : make_tmap_matrix(ctx, &tb, b, N, K, ldb, plan.pair ? plan.gn / 2 : plan.gn))) return rc;
     GemmParams p;
     p.c = (__half*)c; p.ldc = ldc; p.M = M; p.N = N; p.K = K; p.kb_chunk = plan.kb_chunk; p.err = ctx->dev_err;
-    return plan.gn == 256 ? gemm_orders<256>(ctx, ta, tb, p, plan.parts, a_mn_major, b_mn_major)
-                          : gemm_orders<192>(ctx, ta, tb, p, plan.parts, a_mn_major, b_mn_major);
+    const auto orders = plan.pair ? gemm_orders<256, true> : plan.gn == 256 ? gemm_orders<256, false> : gemm_orders<192, false>;
+    return orders(ctx, ta, tb, p, plan.parts, a_mn_major, b_mn_major);
 }

@@ -105,6 +105,23 @@ __device__ __forceinline__ bool mbar_wait_warp(const WaitState& ws, uint64_t* ba
 }
 
 // ---------------------------------------------------------------------------
+// Barriers of another CTA of the cluster
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster_warp(uint32_t bar) {
+    __syncwarp();
+    if (elect_one()) mbar_arrive_cluster(bar);
+}
+__device__ __forceinline__ void fence_acq_rel_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------
 // Proxy fences
 // ---------------------------------------------------------------------------
 // Makes generic-proxy writes to shared memory visible to the async proxy (TMA, tcgen05.mma).
@@ -127,6 +144,14 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const void* tmap, uint64_
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
         "[%0], [%1, {%3, %4, %5, %6}], [%2];"
         ::"r"(smem_u32(dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        : "memory");
+}
+// The same by one CTA of a pair, completion on the barrier at the shared::cluster address `bar` (of either CTA).
+__device__ __forceinline__ void tma_load_4d_pair(void* dst, const void* tmap, uint32_t bar, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+        "[%0], [%1, {%3, %4, %5, %6}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
@@ -160,6 +185,19 @@ __device__ __forceinline__ void tmem_relinquish() {
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+
+// The same for a pair of CTAs (cluster ranks 2i and 2i + 1) whose products run on both SMs; a warp of each CTA calls them.  Every
+// tcgen05 instruction of a kernel names the same group.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(smem_u32(smem_result)), "r"(cols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 
 // A persistent tcgen05 kernel starts in two parts.  Before it waits for its predecessor it sets up its barriers (thread 0) and
@@ -249,6 +287,21 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+// The same over a pair of CTAs: M = 256, the rows of A and of D split between the CTAs, and half of B's columns in either's shared
+// memory (same offsets).  Issued by ONE thread of the pair's first CTA.
+__device__ __forceinline__ void umma_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// One arrival on this barrier of every CTA in `ctas` (a bit per cluster rank).
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint32_t ctas) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)ctas) : "memory");
 }
 // The mbarrier receives one arrival when every MMA this thread issued so far has finished.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {

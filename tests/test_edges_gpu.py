@@ -775,3 +775,23 @@ def test_embedding_backward_of_repeated_ids(n, V, C):
     got = gpt.embedding_backward(torch.from_numpy(d).cuda(), torch.from_numpy(ids).cuda(), V)
     torch.cuda.synchronize()
     assert np.array_equal(got.cpu().numpy(), ref.embedding_bwd(d, ids, V))
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (264, 264, 328), (520, 192, 1032), (512, 520, 8192), (640, 1544, 4104), (1280, 768, 8192), (2056, 2304, 776),
+                                   (4104, 1288, 200), (8192, 96, 72), (9472, 768, 64), (304, 3000, 16392), (4104, 2056, 72),
+                                   (2184, 4488, 1032), (9480, 4864, 264)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+def test_f16_gemm_pairs_of_ctas(M, N, K, a_mn, b_mn):
+    """Tiles of 256 rows by two CTAs where the choice falls on them: a second half of few or no rows, columns that end in either half, one
+    or several tiles a pair.  Small integers, as above; sums of up to 16392 terms of which few are not zero."""
+    from deers_b200 import ops
+    rng = np.random.default_rng(M + N + K)
+    a = rng.integers(-1, 2, (K, M) if a_mn else (M, K)).astype(np.float16)
+    b = rng.integers(-1, 2, (K, N) if b_mn else (N, K)).astype(np.float16)
+    a *= rng.random(a.shape) < 0.3
+    ta, tb = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    got = ops._gemm(M, N, K, ta, int(a_mn), tb, int(b_mn))
+    ops.Context.current(got.device).sync()
+    want = (ta.float().T if a_mn else ta.float()).double() @ (tb if b_mn else tb.T).double()
+    assert want.abs().max().item() <= 2048
+    assert torch.equal(got.double(), want)
