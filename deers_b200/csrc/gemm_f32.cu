@@ -1,5 +1,5 @@
 // f32 GEMM: the choice of tile and split, the launches and the C ABI (the kernels: gemm_f32_kernel.cuh).
-#include "gemm_f32_kernel.cuh"
+#include "gemm_f32_tc.cuh"
 
 namespace {
 
@@ -21,12 +21,19 @@ struct GemmGroup {
 };
 
 template <int PM, int PN, int KS>
-__global__ void __launch_bounds__(GT * KS) gemm_f32_group_kernel(const __grid_constant__ GemmGroup gg) {
+__global__ void __launch_bounds__(GT * KS, PM * PN < 16 ? 2 : 1) gemm_f32_group_kernel(const __grid_constant__ GemmGroup gg) {
     const int i = gg.pick(blockIdx.x);
     TileProduct<PM, PN, KS, true, true, false, false> tile;
     tile.setup(gg.args(i), gg.tile_m(i, blockIdx.x), gg.tile_n(i, blockIdx.x), blockIdx.z);
     chain_wait();
     tile.run(gg.args(i), gridDim.z, blockIdx.z);
+}
+
+__global__ void __launch_bounds__(TC_T, 1) gemm_f32_tc_group_kernel(const __grid_constant__ GemmGroup gg, unsigned int* err) {
+    gemm_f32_tc_prologue();
+    chain_wait();
+    const int i = gg.pick(blockIdx.x);
+    gemm_f32_tc_tile<true, true, false, false>(gg.args(i), gg.tile_m(i, blockIdx.x), gg.tile_n(i, blockIdx.x), blockIdx.z, gridDim.z, err);
 }
 
 // Tile variants: the cycles at 1.965 GHz that the choice reckons with, a block's walk over 64 k and what a launch costs around it.
@@ -35,8 +42,15 @@ __global__ void __launch_bounds__(GT * KS) gemm_f32_group_kernel(const __grid_co
 // 64 x 96 4620 / 4710 / 5250, 32 x 96 2430 / 2900 / 3280, and 3800 to 9200 around it (148 tiles, K 320 and 1600).  The 96-wide tiles are
 // there for products whose 64-wide ones just miss one wave (1024 x 768: 192 tiles on 148 SMs, 128 of 64 x 96; 13.3 -> 11.7 us at K =
 // 192, and 16.3 -> 13.7 for 1024 x 192 x 768 in clusters of four).
+// The last is the tensor core's: a block starts only where one has left, and so do clusters, so all of it counts per wave.  Measured in a graph:
+// K = 64 4.6 us, 192 7.8, 384 12.0, 768 19.8, 1024 25.1; 1024 x 192 x 768 in clusters of four 9.5; three waves of K = 192 22.2.  Rows on no
+// 16-byte boundary take a tenth to a fifth more (TC_LOOSE).  Short products stay with the FFMA tiles (1024 x 192 x 192 5.1 us, here 6.3; 231 x 576 x 192
+// 3.8 and 6.1).
 struct Variant { int bm, bn; double walk, around; };
-constexpr Variant kVariants[6] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {32, 64, 2360, 4000}, {32, 32, 1680, 3200}, {64, 96, 5400, 5300}, {32, 96, 3200, 4300}};
+constexpr int TC_CFG = 6;
+constexpr double TC_LOOSE = 1.1;
+constexpr Variant kVariants[7] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {32, 64, 2360, 4000}, {32, 32, 1680, 3200}, {64, 96, 5400, 5300}, {32, 96, 3200, 4300},
+                                  {TC_M, TC_N, 2640, 7300}};
 
 // How many clusters of 1..MAX_PARTS blocks (one block per SM) the device holds at a time: a cluster lives inside one
 // GPC, so e.g. 48 clusters of three do not fit 148 SMs although their 144 blocks would.
@@ -72,24 +86,27 @@ int cluster_capacity(deers_ctx* ctx) {
 
 // Picks the variant and the K split with the least estimated time: the blocks an SM has to run one after another times
 // a block's walk over its K, plus what a block spends before and after it (and at the cluster's meeting).
-// n products of one K; whole_heads: tiles must hold whole heads of that many columns (0: any).  cfg < 0: no variant does.
-GemmPlan plan_gemm(int n, const int* M, const int* N, int K, const int* capacity, int whole_heads) {
+// n products of one K; tc: what a tensor core's tile costs of its figure (0: not for these products); whole_heads: tiles must hold whole heads of that many columns (0: any).
+// cfg < 0: no variant does.
+GemmPlan plan_gemm(int n, const int* M, const int* N, int K, double tc, const int* capacity, int whole_heads) {
     GemmPlan best{};
     best.cfg = -1;
     best.cost = 1e30;
     double best_cost = -1.0;
     const int steps = (K + BK - 1) / BK;
-    for (int c = 0; c < 6; ++c) {
+    for (int c = 0; c < 7; ++c) {
         const Variant& v = kVariants[c];
         if (whole_heads && v.bn % whole_heads) continue;
+        if (c == TC_CFG && (tc == 0.0 || K == 0)) continue;
         long long tiles = 0;
         for (int i = 0; i < n; ++i) tiles += (long long)((M[i] + v.bm - 1) / v.bm) * ((N[i] + v.bn - 1) / v.bn);
         for (int parts = 1; parts <= MAX_PARTS; ++parts) {
             const int chunk = (steps + parts - 1) / parts;
-            if (parts > 1 && (chunk < 2 || (long long)chunk * (parts - 1) >= steps)) continue;      // no empty part
+            if (parts > 1 && ((chunk < 2 && c != TC_CFG) || (long long)chunk * (parts - 1) >= steps)) continue;      // no empty part
             if (capacity[parts] < 1) continue;
             const double waves = (double)((tiles + capacity[parts] - 1) / capacity[parts]);
-            const double cost = waves * chunk * v.walk + v.around + 1200.0 * (waves - 1.0) + (parts > 1 ? 3300.0 : 0.0);
+            const double meet = parts > 1 ? 3300.0 : 0.0;
+            const double cost = c == TC_CFG ? waves * (tc * (chunk * v.walk + v.around) + meet) : waves * chunk * v.walk + v.around + 1200.0 * (waves - 1.0) + meet;
             if (best_cost < 0.0 || cost < best_cost) {
                 best_cost = cost;
                 best.cost = cost; best.cfg = c; best.parts = parts; best.k_chunk = chunk * BK; best.waves = (int)waves;
@@ -100,19 +117,31 @@ GemmPlan plan_gemm(int n, const int* M, const int* N, int K, const int* capacity
     return best;
 }
 
-template <int PM, int PN, int KS>
-int launch_group(deers_ctx* ctx, const GemmPlan& p, GemmGroup& gg) {
-    using S = GemmShape<PM, PN, KS, true, true, false>;
-    const auto kernel = gemm_f32_group_kernel<PM, PN, KS>;
-    DEERS_SMEM_ONCE(ctx, (gemm_f32_group_kernel<PM, PN, KS>), S::SMEM);
+// Lays the group's tiles out one product after another; their number.
+int lay_out_group(GemmGroup& gg, const GemmPlan& p) {
+    const Variant& v = kVariants[p.cfg];
     int tiles = 0;
     for (int i = 0; i < gg.n; ++i) {
         gg.first[i] = tiles;
-        gg.tiles_n[i] = (gg.g[i].N + S::BN - 1) / S::BN;
-        tiles += gg.tiles_n[i] * ((gg.g[i].M + S::BM - 1) / S::BM);
+        gg.tiles_n[i] = (gg.g[i].N + v.bn - 1) / v.bn;
+        tiles += gg.tiles_n[i] * ((gg.g[i].M + v.bm - 1) / v.bm);
         gg.g[i].k_chunk = p.k_chunk;
     }
+    return tiles;
+}
+
+template <int PM, int PN, int KS>
+int launch_group(deers_ctx* ctx, const GemmPlan& p, const GemmGroup& gg, int tiles) {
+    using S = GemmShape<PM, PN, KS, true, true, false>;
+    const auto kernel = gemm_f32_group_kernel<PM, PN, KS>;
+    DEERS_SMEM_ONCE(ctx, (gemm_f32_group_kernel<PM, PN, KS>), S::SMEM);
     DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, dim3(tiles, 1, p.parts), S::THREADS, S::SMEM, dim3(1, 1, p.parts), gg));
+    return DEERS_OK;
+}
+
+int launch_group_tc(deers_ctx* ctx, const GemmPlan& p, const GemmGroup& gg, int tiles) {
+    DEERS_SMEM_ONCE(ctx, gemm_f32_tc_group_kernel, TC_SMEM);
+    DEERS_CUDA_TRY(ctx, launch_chained(ctx, gemm_f32_tc_group_kernel, dim3(tiles, 1, p.parts), TC_T, TC_SMEM, dim3(1, 1, p.parts), gg, ctx->dev_err));
     return DEERS_OK;
 }
 
@@ -134,7 +163,9 @@ int launch_planned(deers_ctx* ctx, const GemmPlan& p, GemmArgs& g, int a_mn, int
     int rc;
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM);
-        rc = g.a_vec && g.b_vec ? launch_tiles<false>(ctx, p, g, a_mn, b_mn, fused) : launch_gemm_f32_loose(ctx, p, g, a_mn, b_mn, fused);
+        const bool aligned = g.a_vec && g.b_vec;
+        rc = p.cfg == TC_CFG ? (aligned ? launch_gemm_f32_tc(ctx, p.parts, g, a_mn, b_mn, fused) : launch_gemm_f32_tc_loose(ctx, p.parts, g, a_mn, b_mn))
+             : aligned ? launch_tiles<false>(ctx, p, g, a_mn, b_mn, fused) : launch_gemm_f32_loose(ctx, p, g, a_mn, b_mn, fused);
     }
     ctx->launches += 1;
     return rc;
@@ -157,8 +188,8 @@ int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long lo
     }
     const int rc = cluster_capacity(ctx);
     if (rc) return rc;
-    const GemmPlan p = plan_gemm(1, &M, &N, K, ctx->cluster_capacity, 0);
     GemmArgs g = gemm_args(M, N, K, a, lda, b, ldb, c, ldc, epi, r, ldr, aux);
+    const GemmPlan p = plan_gemm(1, &M, &N, K, g.a_vec && g.b_vec ? 1.0 : TC_LOOSE, ctx->cluster_capacity, 0);
     return launch_planned(ctx, p, g, a_mn, b_mn, false);
 }
 
@@ -169,14 +200,16 @@ int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, co
     if (M == 0 || N == 0) return DEERS_OK;
     const int rc = cluster_capacity(ctx);
     if (rc) return rc;
-    GemmPlan p = plan_gemm(1, &M, &N, K, ctx->cluster_capacity, 0);
     GemmArgs g = gemm_args(M, N, K, a, K, b, N, c, N, epi, nullptr, 0, aux);
+    // (the choice below between rotating in a tile and beside it was measured for the tensor core's tiles up to 384 columns only)
+    const double tc = g.a_vec && g.b_vec && K <= 384 ? 1.0 : 0.0;
+    GemmPlan p = plan_gemm(1, &M, &N, K, tc, ctx->cluster_capacity, 0);
     if (f.rope_cols && f.rope_d % 8 == 0) {
         // A rotary launch of its own takes about 3000 cycles (1.5 us): rotate here unless tiles that hold whole heads cost more
         // than that (heads of 48 columns leave 32 x 96 and 64 x 96 tiles: 231 x 576 x 192 takes 7.5 us in them, 3.6 in 32 x 32).
         // Several waves of clusters do not count: the estimate takes them to follow one another without a gap (forwards of 4 layers,
         // rotating in them and beside: C 512, 256 tokens 363 and 335 us, C 384, 640 tokens 533 and 501).
-        const GemmPlan w = plan_gemm(1, &M, &N, K, ctx->cluster_capacity, f.rope_d);
+        const GemmPlan w = plan_gemm(1, &M, &N, K, tc, ctx->cluster_capacity, f.rope_d);
         if (w.cfg >= 0 && w.cost < p.cost + 3000.0 && (w.cost == p.cost || w.parts == 1 || w.waves == 1)) {
             p = w;
             *rotated = true;
@@ -187,14 +220,25 @@ int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, co
     return launch_planned(ctx, p, g, 0, 1, true);
 }
 
+namespace {
+// The plan of a group of products with dense operands (rows of M_i and N_i).
+GemmPlan plan_group(deers_ctx* ctx, int n, const GemmTN* t, int K) {
+    int M[GEMM_GROUP_MAX], N[GEMM_GROUP_MAX];
+    bool aligned = true;
+    for (int i = 0; i < n; ++i) {
+        M[i] = t[i].M; N[i] = t[i].N;
+        aligned = aligned && M[i] % 4 == 0 && N[i] % 4 == 0 && (((uintptr_t)t[i].a | (uintptr_t)t[i].b) & 15u) == 0;
+    }
+    return plan_gemm(n, M, N, K, aligned ? 1.0 : 0.0, ctx->cluster_capacity, 0);
+}
+}  // namespace
+
 // Whether the group of these products is one wave of blocks.  One of several waves keeps the SMs from what runs beside it until
 // its last, where products on their own take turns with it (GPT training step of 6 layers, 1024 tokens: C 192, one wave, 980 us
 // grouped and 998 apart; C 320 2235 and 2219; C 512 4472 and 4028).
 bool gemm_f32_group_fits(deers_ctx* ctx, int n, const GemmTN* t, int K) {
     if (n < 1 || n > GEMM_GROUP_MAX || cluster_capacity(ctx)) return false;
-    int M[GEMM_GROUP_MAX], N[GEMM_GROUP_MAX];
-    for (int i = 0; i < n; ++i) { M[i] = t[i].M; N[i] = t[i].N; }
-    return plan_gemm(n, M, N, K, ctx->cluster_capacity, 0).waves == 1;
+    return plan_group(ctx, n, t, K).waves == 1;
 }
 
 // C_i = A_i^T B_i, A_i [K, M_i] and B_i [K, N_i] row-major, one K, in one launch.
@@ -203,22 +247,21 @@ int launch_gemm_f32_group(deers_ctx* ctx, int n, const GemmTN* t, int K) {
     const int rc = cluster_capacity(ctx);
     if (rc) return rc;
     GemmGroup gg{};
-    int M[GEMM_GROUP_MAX], N[GEMM_GROUP_MAX];
     gg.n = n;
-    for (int i = 0; i < n; ++i) {
-        M[i] = t[i].M; N[i] = t[i].N;
+    for (int i = 0; i < n; ++i)
         gg.g[i] = gemm_args(t[i].M, t[i].N, K, t[i].a, t[i].M, t[i].b, t[i].N, t[i].c, t[i].N, DEERS_EPI_NONE, nullptr, 0, nullptr);
-    }
-    const GemmPlan p = plan_gemm(n, M, N, K, ctx->cluster_capacity, 0);
+    const GemmPlan p = plan_group(ctx, n, t, K);
+    const int tiles = lay_out_group(gg, p);
     int res;
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM);
-        if (p.cfg == 0) res = launch_group<8, 8, 2>(ctx, p, gg);
-        else if (p.cfg == 1) res = launch_group<8, 4, 4>(ctx, p, gg);
-        else if (p.cfg == 2) res = launch_group<4, 4, 4>(ctx, p, gg);
-        else if (p.cfg == 3) res = launch_group<4, 2, 4>(ctx, p, gg);
-        else if (p.cfg == 4) res = launch_group<8, 6, 4>(ctx, p, gg);
-        else res = launch_group<4, 6, 4>(ctx, p, gg);
+        if (p.cfg == 0) res = launch_group<8, 8, 2>(ctx, p, gg, tiles);
+        else if (p.cfg == 1) res = launch_group<8, 4, 4>(ctx, p, gg, tiles);
+        else if (p.cfg == 2) res = launch_group<4, 4, 4>(ctx, p, gg, tiles);
+        else if (p.cfg == 3) res = launch_group<4, 2, 4>(ctx, p, gg, tiles);
+        else if (p.cfg == 4) res = launch_group<8, 6, 4>(ctx, p, gg, tiles);
+        else if (p.cfg == 5) res = launch_group<4, 6, 4>(ctx, p, gg, tiles);
+        else res = launch_group_tc(ctx, p, gg, tiles);
     }
     ctx->launches += 1;
     return res;

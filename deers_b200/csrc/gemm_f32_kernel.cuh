@@ -64,6 +64,10 @@ struct GemmPlan {
 // process loads all kernels of its module, and most programs never need these (first training step of a process 8.4 ms, 17 with them).
 int launch_gemm_f32_loose(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g, int a_mn, int b_mn, bool fused);
 
+// Products on the tensor core (gemm_f32_tc.cu, the tile: gemm_f32_tc.cuh).
+int launch_gemm_f32_tc(deers_ctx* ctx, int parts, const GemmArgs& g, int a_mn, int b_mn, bool fused);
+int launch_gemm_f32_tc_loose(deers_ctx* ctx, int parts, const GemmArgs& g, int a_mn, int b_mn);
+
 namespace {
 namespace cg = cooperative_groups;
 
@@ -212,15 +216,19 @@ struct GemmShape {
     static constexpr size_t SMEM = PM * PN >= 16 && NEED < ALONE ? ALONE : NEED;
 };
 
-// Sum of a tile element's partial sums: the k groups of this block, or the blocks of the cluster.
+// Sum of a tile element's partial sums: the k groups of this block, or the blocks of the cluster (every load on its way before the
+// first addition).
 template <int KS, int PATCH>
 __device__ __forceinline__ float4 patch_sum(const float* q, int parts) {
     if (parts > 1) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int z = 0; z < parts; ++z) {
-            const float4 u = *reinterpret_cast<const float4*>(cg::this_cluster().map_shared_rank(q, z));
-            v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
-        }
+        float4 u[MAX_PARTS];
+#pragma unroll
+        for (int z = 0; z < MAX_PARTS; ++z)
+            if (z < parts) u[z] = *reinterpret_cast<const float4*>(cg::this_cluster().map_shared_rank(q, z));
+        float4 v = u[0];
+#pragma unroll
+        for (int z = 1; z < MAX_PARTS; ++z)
+            if (z < parts) { v.x += u[z].x; v.y += u[z].y; v.z += u[z].z; v.w += u[z].w; }
         return v;
     }
     float4 v = *reinterpret_cast<const float4*>(q);
@@ -230,6 +238,124 @@ __device__ __forceinline__ float4 patch_sum(const float* q, int parts) {
         v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
     }
     return v;
+}
+
+// What follows a tile's products: KS patches of BM x BN partial sums lie in `red` (rows of BN + 4), with FUSED the rows' sums of squares
+// in sq_s [KS][BM].  Meets, adds the k groups and the blocks of the cluster, applies norm, rotation and epilogue, and stores.
+// What the epilogue reads from global memory is requested before the block's meeting (behind it, it cost 400 to 700 cycles of a product's 5000), and
+// behind a cluster's, whose arrival would wait for it, beside the reads of the other blocks' patches.
+template <int BM, int BN, int KS, int THREADS, bool FUSED>
+__device__ __forceinline__ void finish_tile(const GemmArgs& g, float* const red, float* const sq_s, const int m0, const int n0, const int parts, const int rank) {
+    constexpr int RLD = BN + 4, ITEMS = (BM * BN / 4 + THREADS - 1) / THREADS;     // four columns each
+    // Rows of the tile this block finishes: all of them, or its share of the cluster's.
+    int r_begin = 0, r_end = BM;
+    if (parts > 1) {
+        const int share = (BM + parts - 1) / parts;
+        r_begin = rank * share;
+        r_end = min(BM, r_begin + share);
+    }
+    const int first = r_begin * (BN / 4) + threadIdx.x, last = r_end * (BN / 4);
+    const bool from_r = g.epi == DEERS_EPI_ADD, from_aux = g.epi == DEERS_EPI_MUL_AUX2;
+    float4 ext[ITEMS], c4[FUSED ? ITEMS : 1], s4[FUSED ? ITEMS : 1];
+    auto request = [&]() {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const int idx = first + i * THREADS, m = m0 + idx / (BN / 4), n = n0 + (idx % (BN / 4)) * 4;
+            const bool in = idx < last && m < g.M && n < g.N;
+            if (in && (from_r || from_aux))
+                ext[i] = ld4(from_r ? g.r + (long long)m * g.ldr + n : g.aux + (long long)m * g.ldc + n, g.N - n, g.c_vec);
+            if constexpr (FUSED) {
+                if (in && n < g.rope_cols) {
+                    const int half = g.rope_d / 2, hc = n % g.rope_d;
+                    const long long at = (long long)(m % g.rope_t) * half + (hc >= half ? hc - half : hc);
+                    c4[i] = *reinterpret_cast<const float4*>(g.cosv + at);
+                    s4[i] = *reinterpret_cast<const float4*>(g.sinv + at);
+                }
+            }
+        }
+    };
+    if (parts == 1) request();
+    __syncthreads();
+    if (parts > 1) {
+        for (int idx = threadIdx.x; idx < BM * BN / 4; idx += THREADS) {
+            float* q = red + (idx / (BN / 4)) * RLD + (idx % (BN / 4)) * 4;
+            float4 v = *reinterpret_cast<float4*>(q);
+#pragma unroll
+            for (int z = 1; z < KS; ++z) {
+                const float4 u = *reinterpret_cast<const float4*>(q + z * BM * RLD);
+                v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+            }
+            *reinterpret_cast<float4*>(q) = v;
+        }
+        if constexpr (FUSED) {
+            if (threadIdx.x < BM) {
+                float v = sq_s[threadIdx.x];
+#pragma unroll
+                for (int z = 1; z < KS; ++z) v += sq_s[z * BM + threadIdx.x];
+                sq_s[threadIdx.x] = v;
+            }
+        }
+        cg::this_cluster().sync();
+        request();
+    }
+    chain_next();                                                   // (at the loop or earlier, successors crowd out the side stream)
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const int idx = first + i * THREADS;
+        if (idx >= last) break;
+        const int row = idx / (BN / 4), col = (idx % (BN / 4)) * 4;
+        const int m = m0 + row, n = n0 + col;
+        if (m >= g.M || n >= g.N) continue;
+        const float* q = red + row * RLD + col;
+        const float4 v = patch_sum<KS, BM * RLD>(q, parts);
+        const int valid = g.N - n;
+        float o[4] = {v.x, v.y, v.z, v.w}, x[4] = {0.f, 0.f, 0.f, 0.f};
+        float* cp = g.c + (long long)m * g.ldc + n;
+        if constexpr (FUSED) {
+            float t = 0.f;
+            if (parts > 1) {
+                for (int z = 0; z < parts; ++z) t += *cg::this_cluster().map_shared_rank(sq_s + row, z);
+            } else {
+#pragma unroll
+                for (int z = 0; z < KS; ++z) t += sq_s[z * BM + row];
+            }
+            const float inv = 1.0f / sqrtf(t * g.inv_n + g.eps);
+            if (g.inv && n == 0) g.inv[m] = inv;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] *= inv;
+            if (n < g.rope_cols) {
+                // the other half of the head lies in this tile (tiles hold whole heads); rounded as the rotary pack does
+                const int half = g.rope_d / 2;
+                const bool second = n % g.rope_d >= half;
+                const float4 u = patch_sum<KS, BM * RLD>(second ? q - half : q + half, parts);
+                const float p[4] = {u.x * inv, u.y * inv, u.z * inv, u.w * inv}, cs[4] = {c4[i].x, c4[i].y, c4[i].z, c4[i].w}, sn[4] = {s4[i].x, s4[i].y, s4[i].z, s4[i].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    o[e] = second ? __fadd_rn(__fmul_rn(p[e], -sn[e]), __fmul_rn(o[e], cs[e])) : __fadd_rn(__fmul_rn(o[e], cs[e]), __fmul_rn(p[e], sn[e]));
+            }
+        }
+        if (from_r) {
+            o[0] = ext[i].x + o[0]; o[1] = ext[i].y + o[1]; o[2] = ext[i].z + o[2]; o[3] = ext[i].w + o[3];
+        } else if (g.epi == DEERS_EPI_RELU_SQ) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { x[e] = fmaxf(o[e], 0.f); o[e] = x[e] * x[e]; }
+        } else if (from_aux) {
+            o[0] *= ext[i].x; o[1] *= ext[i].y; o[2] *= ext[i].z; o[3] *= ext[i].w;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = o[e] + o[e];
+        }
+        if (g.c_vec && valid >= 4) {
+            *reinterpret_cast<float4*>(cp) = make_float4(o[0], o[1], o[2], o[3]);
+            if (g.epi == DEERS_EPI_RELU_SQ && g.aux)
+                *reinterpret_cast<float4*>(g.aux + (long long)m * g.ldc + n) = make_float4(x[0], x[1], x[2], x[3]);
+        } else {
+            for (int e = 0; e < 4 && e < valid; ++e) {
+                cp[e] = o[e];
+                if (g.epi == DEERS_EPI_RELU_SQ && g.aux) g.aux[(long long)m * g.ldc + n + e] = x[e];
+            }
+        }
+    }
+    if (parts > 1) cg::this_cluster().sync();                       // nobody leaves while a peer still reads its patch
 }
 
 // One tile (tile_m, tile_n) of a product and one part of its K.  setup() only computes addresses and may run before the
@@ -401,97 +527,11 @@ __device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED, LOOSE
             for (int j = 0; j < PN; ++j) row[S::OB::template index<PN>(tx, j)] = acc[i][j];
         }
     }
-    __syncthreads();
-
-    // Rows of the tile this block finishes: all of them, or its share of the cluster's.
-    int r_begin = 0, r_end = BM;
-    if (parts > 1) {
-        for (int idx = threadIdx.x; idx < BM * BN / 4; idx += S::THREADS) {
-            float* q = red + (idx / (BN / 4)) * S::RLD + (idx % (BN / 4)) * 4;
-            float4 v = *reinterpret_cast<float4*>(q);
-#pragma unroll
-            for (int z = 1; z < KS; ++z) {
-                const float4 u = *reinterpret_cast<const float4*>(q + z * BM * S::RLD);
-                v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
-            }
-            *reinterpret_cast<float4*>(q) = v;
-        }
-        if constexpr (FUSED) {
-            if (threadIdx.x < BM) {
-                float v = sq_s[threadIdx.x];
-#pragma unroll
-                for (int z = 1; z < KS; ++z) v += sq_s[z * BM + threadIdx.x];
-                sq_s[threadIdx.x] = v;
-            }
-        }
-        cg::this_cluster().sync();
-        const int share = (BM + parts - 1) / parts;
-        r_begin = rank * share;
-        r_end = min(BM, r_begin + share);
-    }
-    chain_next();                                                   // (at the loop or earlier, successors crowd out the side stream)
-    for (int idx = r_begin * (BN / 4) + threadIdx.x; idx < r_end * (BN / 4); idx += S::THREADS) {
-        const int row = idx / (BN / 4), col = (idx % (BN / 4)) * 4;
-        const int m = m0 + row, n = n0 + col;
-        const float* q = red + row * S::RLD + col;
-        const float4 v = patch_sum<KS, BM * S::RLD>(q, parts);
-        if (m >= g.M || n >= g.N) continue;
-        const int valid = g.N - n;
-        float o[4] = {v.x, v.y, v.z, v.w}, x[4] = {0.f, 0.f, 0.f, 0.f};
-        float* cp = g.c + (long long)m * g.ldc + n;
-        if constexpr (FUSED) {
-            float t = 0.f;
-            if (parts > 1) {
-                for (int z = 0; z < parts; ++z) t += *cg::this_cluster().map_shared_rank(sq_s + row, z);
-            } else {
-#pragma unroll
-                for (int z = 0; z < KS; ++z) t += sq_s[z * BM + row];
-            }
-            const float inv = 1.0f / sqrtf(t * g.inv_n + g.eps);
-            if (g.inv && n == 0) g.inv[m] = inv;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[e] *= inv;
-            if (n < g.rope_cols) {
-                // the other half of the head lies in this tile (tiles hold whole heads); rounded as the rotary pack does
-                const int half = g.rope_d / 2, hc = n % g.rope_d;
-                const bool second = hc >= half;
-                const float4 u = patch_sum<KS, BM * S::RLD>(second ? q - half : q + half, parts);
-                const long long at = (long long)(m % g.rope_t) * half + (second ? hc - half : hc);
-                const float4 c4 = *reinterpret_cast<const float4*>(g.cosv + at), s4 = *reinterpret_cast<const float4*>(g.sinv + at);
-                const float p[4] = {u.x * inv, u.y * inv, u.z * inv, u.w * inv}, cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    o[e] = second ? __fadd_rn(__fmul_rn(p[e], -sn[e]), __fmul_rn(o[e], cs[e])) : __fadd_rn(__fmul_rn(o[e], cs[e]), __fmul_rn(p[e], sn[e]));
-            }
-        }
-        if (g.epi == DEERS_EPI_ADD) {
-            const float4 t = ld4(g.r + (long long)m * g.ldr + n, valid, g.c_vec);
-            o[0] = t.x + o[0]; o[1] = t.y + o[1]; o[2] = t.z + o[2]; o[3] = t.w + o[3];
-        } else if (g.epi == DEERS_EPI_RELU_SQ) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) { x[e] = fmaxf(o[e], 0.f); o[e] = x[e] * x[e]; }
-        } else if (g.epi == DEERS_EPI_MUL_AUX2) {
-            const float4 t = ld4(g.aux + (long long)m * g.ldc + n, valid, g.c_vec);
-            o[0] *= t.x; o[1] *= t.y; o[2] *= t.z; o[3] *= t.w;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[e] = o[e] + o[e];
-        }
-        if (g.c_vec && valid >= 4) {
-            *reinterpret_cast<float4*>(cp) = make_float4(o[0], o[1], o[2], o[3]);
-            if (g.epi == DEERS_EPI_RELU_SQ && g.aux)
-                *reinterpret_cast<float4*>(g.aux + (long long)m * g.ldc + n) = make_float4(x[0], x[1], x[2], x[3]);
-        } else {
-            for (int e = 0; e < 4 && e < valid; ++e) {
-                cp[e] = o[e];
-                if (g.epi == DEERS_EPI_RELU_SQ && g.aux) g.aux[(long long)m * g.ldc + n + e] = x[e];
-            }
-        }
-    }
-    if (parts > 1) cg::this_cluster().sync();                       // nobody leaves while a peer still reads its patch
+    finish_tile<BM, BN, KS, S::THREADS, FUSED>(g, red, sq_s, m0, n0, parts, rank);
 }
 
 template <int PM, int PN, int KS, bool A_MN, bool B_MN, bool FUSED, bool LOOSE>
-__global__ void __launch_bounds__(GT * KS) gemm_f32_kernel(const GemmArgs g) {
+__global__ void __launch_bounds__(GT * KS, PM * PN < 16 && !LOOSE ? 2 : 1) gemm_f32_kernel(const GemmArgs g) {
     TileProduct<PM, PN, KS, A_MN, B_MN, FUSED, LOOSE> tile;
     tile.setup(g, blockIdx.y, blockIdx.x, blockIdx.z);
     chain_wait();

@@ -268,6 +268,11 @@ __host__ __device__ constexpr uint32_t idesc_f16(int M, int N, int a_mn_major, i
            | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// The same with bf16 inputs.
+__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, int a_mn_major, int b_mn_major) {
+    return idesc_f16(M, N, a_mn_major, b_mn_major) | (1u << 7) | (1u << 10);
+}
+
 // D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
 __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                         uint32_t accumulate) {

@@ -795,3 +795,52 @@ def test_f16_gemm_pairs_of_ctas(M, N, K, a_mn, b_mn):
     want = (ta.float().T if a_mn else ta.float()).double() @ (tb if b_mn else tb.T).double()
     assert want.abs().max().item() <= 2048
     assert torch.equal(got.double(), want)
+
+
+@pytest.mark.parametrize("aligned", [True, False])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, True), (False, False), (True, True), (True, False)])
+@pytest.mark.parametrize("M,N,K", [(2052, 1540, 4), (1156, 1028, 20), (2048, 640, 64), (1028, 1092, 68), (1100, 644, 132), (1024, 768, 192), (1284, 196, 1000), (260, 1540, 772),
+                                   (196, 772, 2052)])
+def test_f32_gemm_on_the_tensor_core(M, N, K, a_mn, b_mn, aligned):
+    """Tiles that end in rows, columns and k, one to many stages, whole K and K shared by a cluster, each storage order, rows on 16-byte
+    boundaries and on none.  Values of three bf16 each, sums that start anew every 16 k: 1e-7 of the result in the 2-norm (measured 5e-8 to
+    8.1e-8; two f16 per value or one accumulator give 2.8e-7), and small integers exactly."""
+    from deers_b200 import gpt
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    pad = 0 if aligned else 1
+
+    def operand(rows, cols, whole):
+        t = torch.empty((rows, cols + pad), device="cuda")
+        t.copy_(torch.randint(-8, 9, t.shape, device="cuda", generator=g) if whole else torch.randn(t.shape, device="cuda", generator=g))
+        return t[:, pad:]
+
+    for whole in (False, True):
+        a = operand(*((K, M) if a_mn else (M, K)), whole)
+        b = operand(*((K, N) if b_mn else (N, K)), whole)
+        got = gpt.gemm_f32(a, b, a_mn, b_mn)
+        again = gpt.gemm_f32(a, b, a_mn, b_mn)
+        want = (a.double().T if a_mn else a.double()) @ (b.double() if b_mn else b.double().T)
+        assert torch.equal(got, again)
+        if whole:
+            assert torch.equal(got.double(), want)
+        else:
+            assert ((got.double() - want).norm() / want.norm()).item() < 1e-7
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, True), (True, True), (False, False)])
+def test_f32_gemm_on_the_tensor_core_of_what_is_not_finite(value, a_mn, b_mn):
+    """Infinities, NaN and values that round to an infinity of bf16, in either operand and against zeros: what the products of f32 give."""
+    from deers_b200 import gpt
+    M, N, K = 1024, 768, 192
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a, b = (torch.randn(s, device="cuda", generator=g) * 0.25 for s in ((M, K), (K, N)))
+    a[700, 100], b[30, 5], b[100, 77] = value, value, 0.0
+    got = gpt.gemm_f32(a.T.contiguous() if a_mn else a, b if b_mn else b.T.contiguous(), a_mn, b_mn).double()
+    want = a.double() @ b.double()
+    assert torch.equal(got.isnan(), want.isnan())
+    fin = want.abs() < 3e38
+    assert torch.equal(got[~fin & ~want.isnan()].sign(), want[~fin & ~want.isnan()].sign())
+    big = want[fin].abs() > 1e30
+    assert (got[fin][~big] - want[fin][~big]).abs().max().item() < 1e-5
+    assert ((got[fin][big] - want[fin][big]) / want[fin][big]).abs().nan_to_num(0).max().item() < 1e-5 if big.any() else True
