@@ -237,6 +237,11 @@ int launch_embedding_bwd(deers_ctx* ctx, const float* dout, const long long* ids
                          float* dweight, bool cleared = false);
 int launch_cross_entropy_fwd(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, long long rows,
                              long long V, float* lse, float* picked, float* loss);
+int launch_cross_entropy_merge(deers_ctx* ctx, const float2* stats, int parts, const float* logits, long long ld, const long long* targets, long long rows,
+                               long long V, float* lse, float* picked);
+int launch_cross_entropy_rows(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, long long rows, long long V, float* lse,
+                              float* picked);
+int launch_cross_entropy_loss(deers_ctx* ctx, const float* picked, long long rows, float* loss);
 int launch_cross_entropy_bwd(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, const float* lse,
                              long long rows, long long V, float upstream, float* dlogits, long long ldd);
 // AdamW with the trainer's rule "no update when the gradient norm is not finite" (optim.cu).  said: what the caller wants to
@@ -250,7 +255,10 @@ int launch_split_f16x3(deers_ctx* ctx, long long rows, int cols, const float* sr
                        void* hi, void* lo, long long ld_dst);
 int launch_gemm_f16x3(deers_ctx* ctx, int M, int N, int K, const void* a_hi, const void* a_lo, long long lda, int a_mn,
                       const void* b_hi, const void* b_lo, long long ldb, int b_mn, float* c, long long ldc, float out_scale,
-                      void* workspace, size_t ws_bytes);
+                      void* workspace, size_t ws_bytes, float2* stats = nullptr, int* stat_parts = nullptr);
+// (stats, stat_parts: with A in K and B in MN order the product may leave, per row and 32 columns, (maximum, sum of exponentials relative to
+// it), [stat_parts][M]; 0 parts: it did not.  Room for 4 * ceil(N / 128) parts.)
+int gemm_f16_pairs(deers_ctx* ctx, int* pairs);
 int launch_cross_entropy_bwd_split(deers_ctx* ctx, const float* logits, long long ld, const long long* targets,
                                    const float* lse, long long rows, long long V, float upstream, float scale, void* hi,
                                    void* lo, long long ldd);

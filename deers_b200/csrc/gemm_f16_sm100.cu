@@ -185,7 +185,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             for (int t = t0; ok && t < n_tiles; t += t_step, ++n) {
                 const uint32_t buf = (uint32_t)n & 1u;
                 if (!mbar_wait_warp(ws, &bars[S::ACC_EMPTY + buf], (((uint32_t)n >> 1) & 1u) ^ 1u, DEERS_KERR_GEMM | 2)) break;
-                if (PAIR) fence_acq_rel_cluster();
+                tc_fence_after_sync();
                 for (int kb = kb0; kb < kb1; ++kb, ++g) {
                     const uint32_t s = g % G_STAGES;
                     if (!mbar_wait_warp(ws, &bars[S::FULL + s], (g / G_STAGES) & 1u, DEERS_KERR_GEMM | 3)) { ok = false; break; }
@@ -424,6 +424,13 @@ int gemm_orders(deers_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, co
 }
 
 }  // namespace
+
+// How many pairs of CTAs (one CTA per SM) the device holds at a time.
+int gemm_f16_pairs(deers_ctx* ctx, int* pairs) {
+    const int rc = cluster_room(ctx);
+    *pairs = rc ? 0 : ctx->cluster_room_f16[2];
+    return rc;
+}
 
 extern "C" int deers_b200_gemm_f16(deers_ctx* ctx, int32_t M, int32_t N, int32_t K, const void* a, int64_t lda, int32_t a_mn_major,
                                    const void* b, int64_t ldb, int32_t b_mn_major, void* c, int64_t ldc) {

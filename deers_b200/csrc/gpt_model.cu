@@ -72,6 +72,8 @@ struct deers_gpt {
     void *xf_hi, *xf_lo, *w_hi, *w_lo, *dl_hi, *dl_lo;
     void* x3_ws;
     void* x3_ws_side;
+    float2* ce_stats;            // what a training step's head product leaves of its rows, ce_parts (0: nothing) per row
+    int ce_parts;
     size_t x3_ws_bytes;
     // pinned staging for train_step_host
     long long* ids_pin;
@@ -229,7 +231,7 @@ int forward(deers_gpt* m, const long long* ids, int B, int T, bool with_head_pai
         }
         GPT_TRY(rc);
         GPT_TRY(launch_gemm_f16x3(ctx, (int)N, V, C, m->xf_hi, m->xf_lo, C, 0, m->w_hi, m->w_lo, m->Vld, 1, logits, ldl,
-                                  1.0f, m->x3_ws, m->x3_ws_bytes));
+                                  1.0f, m->x3_ws, m->x3_ws_bytes, keep ? m->ce_stats : nullptr, &m->ce_parts));
     } else {
         GPT_TRY(launch_rmsnorm_fwd(ctx, N, C, c.rms_norm_eps, x, m->xf, m->invf));
         GPT_TRY(gemm(m, (int)N, V, C, m->xf, C, 0, W + m->off_lm, m->Vld, 1, logits, ldl));  // lm_head
@@ -246,7 +248,9 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
     float* W = m->arena[0];
     float* G = m->arena[1];
     for (bool& v : m->done_valid) v = false;
-    GPT_TRY(launch_cross_entropy_fwd(ctx, m->logits, Vld, targets, N, V, m->ce_lse, m->picked, m->loss_dev));
+    // (the loss itself is added up beside the backward)
+    if (m->tc_head && m->ce_parts) GPT_TRY(launch_cross_entropy_merge(ctx, m->ce_stats, m->ce_parts, m->logits, Vld, targets, N, V, m->ce_lse, m->picked));
+    else GPT_TRY(launch_cross_entropy_rows(ctx, m->logits, Vld, targets, N, V, m->ce_lse, m->picked));
     const float* x_last = c.n_layer ? m->la[c.n_layer - 1].x2 : m->x0;
     if (m->tc_head) {
         // dlogits leave the cross-entropy backward as f16 pairs scaled by rows * 4096 (|dlogit| <= 1 / rows)
@@ -259,6 +263,7 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
             GPT_TRY(side.rc);
             GPT_TRY(launch_gemm_f16x3(ctx, C, V, (int)N, m->xf_hi, m->xf_lo, C, 1, m->dl_hi, m->dl_lo, Vld, 1, G + m->off_lm, Vld,
                                       1.0f / dscale, m->x3_ws_side, m->x3_ws_bytes));         // d lm_head = xf^T dlogits
+            GPT_TRY(launch_cross_entropy_loss(ctx, m->picked, N, m->loss_dev));               // (in front of it, it would start 2 us later)
         }
     } else {
         GPT_TRY(launch_cross_entropy_bwd(ctx, m->logits, Vld, targets, m->ce_lse, N, V, 1.0f, m->logits, Vld));
@@ -267,6 +272,7 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
             SideScope side(m);
             GPT_TRY(side.rc);
             GPT_TRY(gemm(m, C, V, (int)N, m->xf, C, 1, m->logits, Vld, 1, G + m->off_lm, Vld));  // d lm_head = xf^T dlogits
+            GPT_TRY(launch_cross_entropy_loss(ctx, m->picked, N, m->loss_dev));
         }
     }
     const int last = c.n_layer ? (c.n_layer - 1) & 1 : 0;
@@ -280,14 +286,16 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
         LayerAct& a = m->la[l];
         LayerGrad &d = m->lg[l & 1], &below = m->lg[(l & 1) ^ 1];
         const float* x_in = l ? m->la[l - 1].x2 : m->x0;
-        // On the second stream: all four at the block's end in one launch, or each as soon as its operands are there.
+        // On the second stream: all four at the block's end in one launch, or each as soon as its operands are there.  Of the last block
+        // the first three go ahead in one launch: nothing follows that all four could run beside (22 M parameters, 1024 tokens: 25 us of the four
+        // behind the last norm, then 16 of the one).
         const GemmTN grads[4] = {{Hm, C, a.h, d.dx, G + w.down}, {C, Hm, d.n2, d.dh, G + w.up},              // d Wdown = h^T dx, d Wup = n2^T du
                                  {C, C, a.o, d.dx1, G + w.out}, {C, 3 * C, d.n1, d.dqkv, G + w.qkv}};        // d Wout = o^T dx1, d [Wq|Wk|Wv]
         if (l == c.n_layer - 1) together = gemm_f32_group_fits(ctx, 4, grads, (int)N);
         auto weight_grads = [&](int first, int n) -> int {
             SideScope side(m);
             GPT_TRY(side.rc);
-            if (n == 4) GPT_TRY(launch_gemm_f32_group(ctx, 4, grads, (int)N));
+            if (together && n > 1) GPT_TRY(launch_gemm_f32_group(ctx, n, grads + first, (int)N));
             else
                 for (const GemmTN* t = grads + first; t < grads + first + n; ++t)
                     GPT_TRY(gemm(m, t->M, t->N, (int)N, t->a, t->M, 1, t->b, t->N, 1, t->c, t->N));
@@ -298,7 +306,9 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
         GPT_TRY(gemm(m, (int)N, Hm, C, d.dx, C, 0, W + w.down, C, 0, d.dh, Hm, DEERS_EPI_MUL_AUX2, nullptr, 0, a.r));
         GPT_TRY(gemm(m, (int)N, C, Hm, d.dh, Hm, 0, W + w.up, Hm, 0, m->dtmp, C));           // d n2 = du Wup^T
         GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, a.x1, a.inv2, m->dtmp, d.dx, d.dx1, d.n2));    // d x1
+        const bool ahead = together && l == 0;
         if (!together) GPT_TRY(weight_grads(1, 2));
+        if (ahead) GPT_TRY(weight_grads(0, 3));
         // attention branch: x1 = x + attn(rmsnorm(x)) Wout
         GPT_TRY(gemm(m, (int)N, C, C, d.dx1, C, 0, W + w.out, C, 0, m->dtmp, C));            // d o (token-major)
         GPT_TRY(launch_attn_bwd_f32(ctx, &ad, a.qkv, a.qkv + C, a.qkv + 2 * C, a.o, a.lse, m->dtmp, d.dqkv, d.dqkv + C, d.dqkv + 2 * C,
@@ -308,7 +318,7 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
         GPT_TRY(wait_done(m, (l & 1) ^ 1));                                                  // the block above has read what this block's input gradient replaces
         GPT_TRY(launch_rmsnorm_bwd(ctx, N, C, x_in, a.inv1, m->dtmp, d.dx1, below.dx, d.n1)); // d x
         dx0 = below.dx;
-        GPT_TRY(together ? weight_grads(0, 4) : weight_grads(3, 1));
+        GPT_TRY(together && !ahead ? weight_grads(0, 4) : weight_grads(3, 1));
     }
     GPT_TRY(launch_embedding_bwd(ctx, dx0, ids, N, C, V, G + m->off_wte, true));           // (cleared in the forward)
     return join_side(m);
@@ -541,10 +551,11 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
     const size_t id_bytes = ((size_t)N * sizeof(long long) + 255) / 256 * 256;
     auto up256 = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t xf_h = up256(N * C * 2), w_h = up256(C * (size_t)m->Vld * 2), dl_h = up256(N * (size_t)m->Vld * 2);
-    // K-split partial tiles of the head's input gradient: parts * tokens <= 148 * 128 * 128 / C + tokens
+    // K-split partial tiles of the head's input gradient: parts * tokens <= 148 * 128 * 128 / C + tokens, by pairs 74 * 256 * 192 / C
     const size_t x3 = m->tc_head ? up256(((size_t)148 * 16384 + N * C) * sizeof(float) * 2) : 0;
     m->x3_ws_bytes = x3;
-    const size_t tc_bytes = m->tc_head ? 2 * (xf_h + w_h + dl_h) + 2 * x3 : 0;
+    const size_t stats = up256(4 * ((V + 127) / 128) * N * sizeof(float2));
+    const size_t tc_bytes = m->tc_head ? 2 * (xf_h + w_h + dl_h) + 2 * x3 + stats : 0;
     const size_t bytes = total * sizeof(float) + opt_bytes + 256 + 2 * id_bytes + tc_bytes;
     char* base = nullptr;
     if (!rc && cudaMalloc((void**)&base, bytes) != cudaSuccess) rc = DEERS_ERR_CUDA;
@@ -564,6 +575,7 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
             m->dl_hi = q; q += dl_h; m->dl_lo = q; q += dl_h;
             m->x3_ws = q; q += x3;
             m->x3_ws_side = q; q += x3;
+            m->ce_stats = (float2*)q; q += stats;
         }
         // rotary cache, f32 arithmetic of gpt.rs:12-46
         const int half = D / 2;

@@ -192,6 +192,54 @@ __global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const float* log
     }
 }
 
+// The same rows from what the head product has left of them: `parts` pairs (maximum, sum of exponentials relative to it) per row, [parts][rows].
+// A block takes eight rows, 128 threads each, every thread eight loads at a time.  1024 rows of 1572 parts 7 us behind the product where the pass over
+// the 206 MB of logits takes 42 (with 32 threads a row 18).
+__global__ void __launch_bounds__(1024) cross_entropy_merge_kernel(const float2* stats, int parts, const float* logits, long long ld, const long long* targets,
+                                                                   long long rows, long long V, float* __restrict__ lse, float* __restrict__ picked,
+                                                                   unsigned int* err) {
+    chain_wait();
+    __shared__ float red_m[32][8], red_s[32][8];
+    const int r = threadIdx.x & 7, seg = threadIdx.x >> 3, warp = threadIdx.x >> 5;
+    const long long row = (long long)blockIdx.x * 8 + r;
+    float m = -INFINITY, s = 0.f;
+    if (row < rows) {
+        for (int p0 = seg; p0 < parts; p0 += 8 * 128) {
+            float2 v[8];
+            float M = m;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = p0 + q * 128 < parts ? stats[(long long)(p0 + q * 128) * rows + row] : make_float2(-INFINITY, 0.f);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) M = fmaxf(M, v[q].x);
+            const float ref = M == -INFINITY ? 0.f : M;               // (all empty so far: sums of zeros)
+            s *= expf(m - ref);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) s += v[q].y * expf(v[q].x - ref);
+            m = M;
+        }
+    }
+    // lanes r, r + 8, r + 16, r + 24 of a warp, then the warps
+#pragma unroll
+    for (int off = 8; off <= 16; off *= 2) lse_merge(m, s, __shfl_xor_sync(0xffffffffu, m, off), __shfl_xor_sync(0xffffffffu, s, off));
+    if ((threadIdx.x & 31) < 8) { red_m[warp][r] = m; red_s[warp][r] = s; }
+    __syncthreads();
+    if (warp) return;
+    m = red_m[seg][r]; s = red_s[seg][r];
+    for (int w = 4; w < 32; w += 4) lse_merge(m, s, red_m[w + seg][r], red_s[w + seg][r]);
+#pragma unroll
+    for (int off = 8; off <= 16; off *= 2) lse_merge(m, s, __shfl_xor_sync(0xffffffffu, m, off), __shfl_xor_sync(0xffffffffu, s, off));
+    if (row >= rows || seg) return;
+    const float l = logf(s) + m;
+    lse[row] = l;
+    const long long t = targets[row];
+    if (t < 0 || t >= V) {
+        atomicCAS(err, 0u, (unsigned)DEERS_KERR_GPT | 2u);
+        picked[row] = 0.f;
+    } else {
+        picked[row] = logits[row * ld + t] - l;
+    }
+}
+
 __global__ void __launch_bounds__(1024) cross_entropy_loss_kernel(const float* picked, long long rows,
                                                                   float neg_inv_rows, float* __restrict__ loss) {
     chain_wait();
@@ -348,15 +396,24 @@ int launch_embedding_bwd(deers_ctx* ctx, const float* dout, const long long* ids
     return DEERS_OK;
 }
 
-int launch_cross_entropy_fwd(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, long long rows,
-                             long long V, float* lse, float* picked, float* loss) {
+int launch_cross_entropy_merge(deers_ctx* ctx, const float2* stats, int parts, const float* logits, long long ld, const long long* targets, long long rows,
+                               long long V, float* lse, float* picked) {
+    {
+        KernelTimerScope ts(ctx, DEERS_K_GPT);
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_merge_kernel, (unsigned)((rows + 7) / 8), 1024, 0, 1, stats, parts, logits, ld, targets, rows, V, lse,
+                                           picked, ctx->dev_err));
+    }
+    ctx->launches += 1;
+    return DEERS_OK;
+}
+
+int launch_cross_entropy_rows(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, long long rows, long long V, float* lse,
+                              float* picked) {
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
         DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_fwd_kernel, (unsigned)rows, 256, 0, 1, logits, ld, targets, V, lse, picked, ctx->dev_err));
-        DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_loss_kernel, 1, 1024, 0, 1, picked, rows, (float)(-1.0 / (double)rows), loss));
     }
-    ctx->launches += 2;
-    DEERS_CUDA_TRY(ctx, cudaGetLastError());
+    ctx->launches += 1;
     return DEERS_OK;
 }
 
@@ -366,8 +423,13 @@ int launch_cross_entropy_loss(deers_ctx* ctx, const float* picked, long long row
         DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_loss_kernel, 1, 1024, 0, 1, picked, rows, (float)(-1.0 / (double)rows), loss));
     }
     ctx->launches += 1;
-    DEERS_CUDA_TRY(ctx, cudaGetLastError());
     return DEERS_OK;
+}
+
+int launch_cross_entropy_fwd(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, long long rows,
+                             long long V, float* lse, float* picked, float* loss) {
+    const int rc = launch_cross_entropy_rows(ctx, logits, ld, targets, rows, V, lse, picked);
+    return rc ? rc : launch_cross_entropy_loss(ctx, picked, rows, loss);
 }
 
 int launch_cross_entropy_bwd(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, const float* lse,

@@ -112,14 +112,14 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
     return a;
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
+// One arrival for the warp that has read an accumulator (tcgen05.wait::ld and tc_fence_before_sync precede it).  Relaxed: it passes on nothing in
+// memory, and a release at cluster scope would first wait for the warp's stores to global memory.  For the same reason there is no
+// fence behind the wait on the other side: fence.acq_rel.cluster took 4800 cycles beside a storing epilogue, 105000 of the 150000 cycles of
+// a head product by pairs.
 __device__ __forceinline__ void mbar_arrive_cluster_warp(uint32_t bar) {
     __syncwarp();
-    if (elect_one()) mbar_arrive_cluster(bar);
+    if (elect_one()) asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void fence_acq_rel_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // Proxy fences

@@ -844,3 +844,58 @@ def test_f32_gemm_on_the_tensor_core_of_what_is_not_finite(value, a_mn, b_mn):
     big = want[fin].abs() > 1e30
     assert (got[fin][~big] - want[fin][~big]).abs().max().item() < 1e-5
     assert ((got[fin][big] - want[fin][big]) / want[fin][big]).abs().nan_to_num(0).max().item() < 1e-5 if big.any() else True
+
+
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn", [
+    # logits: A resident (one, three, four K blocks) and not; runs of pairs that change rows; rows and columns that end in a tile or its half
+    (1024, 5008, 192, 0, 1), (300, 12296, 64, 0, 1), (2056, 2568, 256, 0, 1), (520, 9608, 328, 0, 1), (136, 20008, 24, 0, 1),
+    # input gradient: K shared out, 128 and 192 columns, one and two of them
+    (1024, 192, 50264, 0, 0), (264, 128, 30008, 0, 0), (2000, 320, 16392, 0, 0), (200, 64, 70000, 0, 0),
+    # weight gradient: transposed, 128 and 192 columns
+    (192, 50264, 1024, 1, 1), (64, 40008, 264, 1, 1), (320, 12296, 520, 1, 1), (384, 30008, 72, 1, 1)])
+def test_f16x3_gemm_pairs_of_ctas(M, N, K, a_mn, b_mn):
+    """The head's products by pairs of CTAs.  Operands of 22 bits (two f16), f32 sums in the tensor core: 2e-6 of the largest value times
+    max(1, sqrt(K) / 16), as for single CTAs; small integers exactly, so any tile, half or K range dropped or taken twice shows."""
+    from deers_b200 import gpt
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    for whole in (True, False):
+        def operand(*shape):
+            if whole:
+                return torch.randint(-1, 2, shape, device="cuda", generator=g).float()
+            return torch.randn(shape, device="cuda", generator=g)
+        a, b = operand(*((K, M) if a_mn else (M, K))), operand(*((K, N) if b_mn else (N, K)))
+        got = gpt.gemm_f16x3(a, b, bool(a_mn), bool(b_mn))
+        again = gpt.gemm_f16x3(a, b, bool(a_mn), bool(b_mn))
+        torch.cuda.synchronize()
+        want = (a.double().T if a_mn else a.double()) @ (b.double() if b_mn else b.double().T)
+        assert torch.equal(got, again)
+        if whole:
+            assert torch.equal(got.double(), want)
+        else:
+            assert (got.double() - want).abs().max().item() <= 2e-6 * max(1.0, K ** 0.5 / 16) * want.abs().max().item()
+
+
+@pytest.mark.parametrize("V,H,D,B,T", [(12289, 2, 32, 2, 100), (50257, 6, 32, 1, 257), (9601, 5, 64, 3, 99), (10111, 4, 64, 2, 131), (1024, 2, 32, 1, 9),
+                                       (131073, 1, 64, 1, 130)])
+def test_gpt_cross_entropy_from_the_head_product(V, H, D, B, T):
+    """Row statistics left by the head product (resident A or not, ragged rows and columns) or taken by a pass of their own: loss and
+    gradients of a model that is only embedding, norm and head, against float64.  The bound is the head products' (2e-6 of the largest value)
+    with room for sums of V terms."""
+    from deers_b200 import gpt
+    C = H * D
+    m = gpt.GPT(gpt.GPTConfig(V, T, 0, H, C, 8), torch.device("cuda", torch.cuda.current_device()), B)
+    g = torch.Generator().manual_seed(V)
+    wte, head = torch.randn((V, C), generator=g), torch.randn((C, V), generator=g) * 0.5
+    m.load_parameters([wte.numpy(), head.numpy()])
+    ids, tgt = torch.randint(0, V, (B, T), generator=g), torch.randint(0, V, (B, T), generator=g)
+    tgt[0, 0], tgt[-1, -1] = 0, V - 1
+    loss = m.forward_backward(ids.cuda(), tgt.cuda())
+    m.ctx.sync()
+    w, h = wte.double().requires_grad_(), head.double().requires_grad_()
+    x = w[ids.reshape(-1)]
+    x = x / torch.sqrt((x * x).mean(1, keepdim=True) + 1e-5)
+    want = torch.nn.functional.cross_entropy(x @ h, tgt.reshape(-1))
+    want.backward()
+    assert abs(loss.item() - want.item()) < 1e-6 * max(1.0, want.item())
+    for i, t in enumerate((w, h)):
+        assert np.abs(m.grad(i) - t.grad.numpy()).max() <= 1e-5 * t.grad.abs().max().item()
