@@ -899,3 +899,27 @@ def test_gpt_cross_entropy_from_the_head_product(V, H, D, B, T):
     assert abs(loss.item() - want.item()) < 1e-6 * max(1.0, want.item())
     for i, t in enumerate((w, h)):
         assert np.abs(m.grad(i) - t.grad.numpy()).max() <= 1e-5 * t.grad.abs().max().item()
+
+
+@pytest.mark.parametrize("B,H,T,D", [
+    (1, 1, 2, 32), (1, 2, 7, 30), (1, 1, 8, 64), (2, 2, 9, 16), (1, 3, 33, 48), (1, 1, 257, 32), (1, 2, 200, 64), (1, 1, 90, 96), (1, 1, 70, 128),     # 8 rows a block
+    (2, 5, 97, 32), (3, 4, 77, 48), (1, 6, 256, 32), (1, 12, 333, 20), (1, 2, 1000, 32), (1, 7, 130, 64), (1, 3, 300, 96), (2, 4, 100, 126)])         # 16 rows
+@pytest.mark.parametrize("causal", [True, False])
+def test_f32_attention_in_blocks_of_few_rows(B, H, T, D, causal):
+    """Calls of few blocks, in blocks of 8 and 16 stationary rows: sequences that end inside a block and a streamed tile, both group counts, either
+    direction (whose blocks may differ in size), widths off 16-byte boundaries.  (Not one key alone: its score gradient is the difference of
+    two equal sums of D products, zero with a rounding of 2^-24 sqrt(D) times the largest product, and no value to hold that against.)"""
+    from deers_b200 import ops
+    from oracle import ref
+    from tests.helpers import TOL_F32
+    rng = np.random.default_rng(T * 19 + D)
+    host = [rng.standard_normal((B, H, T, D)).astype(np.float32) for _ in range(4)]
+    q, k, v, do = (torch.from_numpy(a).cuda() for a in host)
+    op = ops.CausalAttention.new(q, k, v, None, causal)
+    o = op.forward()
+    grads = ops.GradientStore()
+    op.backward(grads, do)
+    ops.Context.current(q.device).sync()
+    want = ref.attn_fwd_bwd(*host, causal=causal)
+    for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), [o, op.lse] + [grads.get(t) for t in (q, k, v)], want):
+        assert_close(g.cpu().numpy(), w, TOL_F32, f"B {B} H {H} T {T} D {D} {name}")
