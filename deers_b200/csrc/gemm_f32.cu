@@ -42,15 +42,18 @@ __global__ void __launch_bounds__(TC_T, 1) gemm_f32_tc_group_kernel(const __grid
 // 64 x 96 4620 / 4710 / 5250, 32 x 96 2430 / 2900 / 3280, and 3800 to 9200 around it (148 tiles, K 320 and 1600).  The 96-wide tiles are
 // there for products whose 64-wide ones just miss one wave (1024 x 768: 192 tiles on 148 SMs, 128 of 64 x 96; 13.3 -> 11.7 us at K =
 // 192, and 16.3 -> 13.7 for 1024 x 192 x 768 in clusters of four).
+// 16 x 32 is for products that leave half of the SMs idle in 32 x 32: 100 x 576 x 192 3.7 -> 3.1 us, 231 x 192 x 192 3.7 -> 3.1, 64 x 64 x 400 in clusters
+// of four 3.9 -> 3.5, 100 x 192 x 768 in clusters of three, where 32 x 32 takes six, 5.5 -> 4.7 (five and more blocks meet for longer); two
+// blocks on an SM gain nothing (231 x 576 x 192 3.8 and 4.7).
 // The last is the tensor core's: a block starts only where one has left, and so do clusters, so all of it counts per wave.  Measured in a graph:
 // K = 64 4.6 us, 192 7.8, 384 12.0, 768 19.8, 1024 25.1; 1024 x 192 x 768 in clusters of four 9.5; three waves of K = 192 22.2.  Rows on no
 // 16-byte boundary take a tenth to a fifth more (TC_LOOSE).  Short products stay with the FFMA tiles (1024 x 192 x 192 5.1 us, here 6.3; 231 x 576 x 192
 // 3.8 and 6.1).
 struct Variant { int bm, bn; double walk, around; };
-constexpr int TC_CFG = 6;
+constexpr int TC_CFG = 7;
 constexpr double TC_LOOSE = 1.1;
-constexpr Variant kVariants[7] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {32, 64, 2360, 4000}, {32, 32, 1680, 3200}, {64, 96, 5400, 5300}, {32, 96, 3200, 4300},
-                                  {TC_M, TC_N, 2640, 7300}};
+constexpr Variant kVariants[8] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {32, 64, 2360, 4000}, {32, 32, 1680, 3200}, {64, 96, 5400, 5300}, {32, 96, 3200, 4300},
+                                  {16, 32, 970, 3800},                                   {TC_M, TC_N, 2640, 7300}};
 
 // How many clusters of 1..MAX_PARTS blocks (one block per SM) the device holds at a time: a cluster lives inside one
 // GPC, so e.g. 48 clusters of three do not fit 148 SMs although their 144 blocks would.
@@ -94,7 +97,7 @@ GemmPlan plan_gemm(int n, const int* M, const int* N, int K, double tc, const in
     best.cost = 1e30;
     double best_cost = -1.0;
     const int steps = (K + BK - 1) / BK;
-    for (int c = 0; c < 7; ++c) {
+    for (int c = 0; c < 8; ++c) {
         const Variant& v = kVariants[c];
         if (whole_heads && v.bn % whole_heads) continue;
         if (c == TC_CFG && (tc == 0.0 || K == 0)) continue;
@@ -105,7 +108,7 @@ GemmPlan plan_gemm(int n, const int* M, const int* N, int K, double tc, const in
             if (parts > 1 && ((chunk < 2 && c != TC_CFG) || (long long)chunk * (parts - 1) >= steps)) continue;      // no empty part
             if (capacity[parts] < 1) continue;
             const double waves = (double)((tiles + capacity[parts] - 1) / capacity[parts]);
-            const double meet = parts > 1 ? 3300.0 : 0.0;
+            const double meet = parts > 1 ? 3300.0 + (c != TC_CFG && parts > 4 ? 600.0 * (parts - 4) : 0.0) : 0.0;
             const double cost = c == TC_CFG ? waves * (tc * (chunk * v.walk + v.around) + meet) : waves * chunk * v.walk + v.around + 1200.0 * (waves - 1.0) + meet;
             if (best_cost < 0.0 || cost < best_cost) {
                 best_cost = cost;
@@ -205,12 +208,12 @@ int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, co
     const double tc = g.a_vec && g.b_vec && K <= 384 ? 1.0 : 0.0;
     GemmPlan p = plan_gemm(1, &M, &N, K, tc, ctx->cluster_capacity, 0);
     if (f.rope_cols && f.rope_d % 8 == 0) {
-        // A rotary launch of its own takes about 3000 cycles (1.5 us): rotate here unless tiles that hold whole heads cost more
+        // A rotary launch of its own takes up to 4400 of these cycles (1.4 to 2 us): rotate here unless tiles that hold whole heads cost more
         // than that (heads of 48 columns leave 32 x 96 and 64 x 96 tiles: 231 x 576 x 192 takes 7.5 us in them, 3.6 in 32 x 32).
         // Several waves of clusters do not count: the estimate takes them to follow one another without a gap (forwards of 4 layers,
         // rotating in them and beside: C 512, 256 tokens 363 and 335 us, C 384, 640 tokens 533 and 501).
         const GemmPlan w = plan_gemm(1, &M, &N, K, tc, ctx->cluster_capacity, f.rope_d);
-        if (w.cfg >= 0 && w.cost < p.cost + 3000.0 && (w.cost == p.cost || w.parts == 1 || w.waves == 1)) {
+        if (w.cfg >= 0 && w.cost < p.cost + 4400.0 && (w.cost == p.cost || w.parts == 1 || w.waves == 1)) {
             p = w;
             *rotated = true;
             g.cosv = f.cosv; g.sinv = f.sinv; g.rope_cols = f.rope_cols; g.rope_d = f.rope_d; g.rope_t = f.rope_t;
@@ -261,6 +264,7 @@ int launch_gemm_f32_group(deers_ctx* ctx, int n, const GemmTN* t, int K) {
         else if (p.cfg == 3) res = launch_group<4, 2, 4>(ctx, p, gg, tiles);
         else if (p.cfg == 4) res = launch_group<8, 6, 4>(ctx, p, gg, tiles);
         else if (p.cfg == 5) res = launch_group<4, 6, 4>(ctx, p, gg, tiles);
+        else if (p.cfg == 6) res = launch_group<2, 2, 4>(ctx, p, gg, tiles);
         else res = launch_group_tc(ctx, p, gg, tiles);
     }
     ctx->launches += 1;

@@ -100,8 +100,10 @@ struct Operand {
     static constexpr int LD = MN ? R + 4 : KG + 4;
     static constexpr int FLOATS = MN ? KG * LD : R * LD;
     static constexpr int LEN = MN ? R : KG, ROWS = MN ? KG : R;     // contiguous floats per row, rows
-    static constexpr int NP = ROWS * LEN / 4 / GT;                  // 16-byte pieces per thread and stage
-    static_assert(NP * GT * 4 == ROWS * LEN, "whole pieces per thread");
+    static constexpr int PIECES = ROWS * LEN / 4;
+    static constexpr int NP = (PIECES + GT - 1) / GT;               // 16-byte pieces per thread and stage
+    static constexpr bool HALF = PIECES < GT;                       // 16 rows of 16 k: half of the threads have one
+    static_assert(HALF || NP * GT == PIECES, "whole pieces per thread");
     const float* base;
     const float* src[NP];    // this thread's pieces of the next stage
     int dst[NP];             // their places in the stage (floats)
@@ -116,7 +118,7 @@ struct Operand {
         step = MN ? BK * ld : BK;
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
-            const int idx = t + i * GT;
+            const int idx = HALF ? t % PIECES : t + i * GT;
             const int row = row_of(idx / (LEN / 4)), col = (idx % (LEN / 4)) * 4;
             const int r = r0 + (MN ? col : row), k = MN ? row : col;
             along_k[i] = k;
@@ -131,10 +133,11 @@ struct Operand {
             if (!vec) {
                 int row = t / LEN;
                 const int col = t % LEN;
-                const float* p = src[0] - (row_of(t / (LEN / 4)) * ld + t % (LEN / 4) * 4) + (row * ld + col);
+                const int piece = HALF ? t % PIECES : t;
+                const float* p = src[0] - (row_of(piece / (LEN / 4)) * ld + piece % (LEN / 4) * 4) + (row * ld + col);
                 float* d = s + row * LD + col;
 #pragma unroll 4
-                for (int i = 0; i < 4 * NP; ++i) {
+                for (int i = 0; i < ROWS * LEN / GT; ++i) {
                     const bool in = MN ? row < kv && col < rv : row < rv && col < kv;
                     cp4(d, in ? p : base, in ? 4 : 0);
                     row += GT / LEN; p += GT / LEN * ld; d += GT / LEN * LD;
@@ -143,6 +146,7 @@ struct Operand {
                 return;
             }
         }
+        if (HALF && t >= PIECES) return;
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
             int valid = along_r[i];
@@ -434,10 +438,15 @@ __device__ __forceinline__ void TileProduct<PM, PN, KS, A_MN, B_MN, FUSED, LOOSE
         const float* sb = sa + S::OA::FLOATS;
         if constexpr (FUSED) {
             const float* q = sa + (tid / SQ_LANES) * S::OA::LD + (tid % SQ_LANES) * SQ_K;
+            if constexpr (SQ_K == 2) {
+                const float2 x = *reinterpret_cast<const float2*>(q);
+                sq = fmaf(x.x, x.x, sq); sq = fmaf(x.y, x.y, sq);
+            } else {
 #pragma unroll
-            for (int e = 0; e < SQ_K; e += 4) {
-                const float4 x = *reinterpret_cast<const float4*>(q + e);
-                sq = fmaf(x.x, x.x, sq); sq = fmaf(x.y, x.y, sq); sq = fmaf(x.z, x.z, sq); sq = fmaf(x.w, x.w, sq);
+                for (int e = 0; e < SQ_K; e += 4) {
+                    const float4 x = *reinterpret_cast<const float4*>(q + e);
+                    sq = fmaf(x.x, x.x, sq); sq = fmaf(x.y, x.y, sq); sq = fmaf(x.z, x.z, sq); sq = fmaf(x.w, x.w, sq);
+                }
             }
         }
         float a[AHEAD ? 2 : 1][U][PM], b[AHEAD ? 2 : 1][U][PN];     // fragments of U k (and of the next U)
@@ -563,7 +572,8 @@ int launch_tiles(deers_ctx* ctx, const GemmPlan& p, const GemmArgs& g, int a_mn,
         case 2: return launch_orders<4, 4, 4, LOOSE>(ctx, p, g, a_mn, b_mn, fused);
         case 3: return launch_orders<4, 2, 4, LOOSE>(ctx, p, g, a_mn, b_mn, fused);
         case 4: return launch_orders<8, 6, 4, LOOSE>(ctx, p, g, a_mn, b_mn, fused);
-        default: return launch_orders<4, 6, 4, LOOSE>(ctx, p, g, a_mn, b_mn, fused);
+        case 5: return launch_orders<4, 6, 4, LOOSE>(ctx, p, g, a_mn, b_mn, fused);
+        default: return launch_orders<2, 2, 4, LOOSE>(ctx, p, g, a_mn, b_mn, fused);
     }
 }
 

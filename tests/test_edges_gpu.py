@@ -923,3 +923,29 @@ def test_f32_attention_in_blocks_of_few_rows(B, H, T, D, causal):
     want = ref.attn_fwd_bwd(*host, causal=causal)
     for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), [o, op.lse] + [grads.get(t) for t in (q, k, v)], want):
         assert_close(g.cpu().numpy(), w, TOL_F32, f"B {B} H {H} T {T} D {D} {name}")
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 32, 64), (15, 31, 60), (16, 33, 68), (17, 96, 192), (100, 576, 192), (100, 192, 768), (64, 64, 400), (20, 384, 384), (231, 192, 190), (9, 1020, 256)])
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 1), (0, 0), (1, 1), (1, 0)])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_f32_gemm_tiles_of_16_rows(M, N, K, a_mn, b_mn, aligned):
+    """Products of few tiles: rows, columns and k that end inside a tile of 16 x 32 or a group's share, clusters, each order, rows on 16-byte boundaries
+    and on none; 2e-6 max(1, sqrt(K) / 4) of the largest value, as for the other tiles."""
+    from deers_b200 import gpt
+    rng = np.random.default_rng(M * 5 + N * 3 + K)
+    pad = 0 if aligned else 1
+
+    def operand(rows, cols):
+        whole = torch.from_numpy(rng.standard_normal((rows, (cols + 3) // 4 * 4 + pad)).astype(np.float32)).cuda()
+        return whole[:, pad:cols + pad]
+
+    a, b = operand(*((K, M) if a_mn else (M, K))), operand(*((K, N) if b_mn else (N, K)))
+    out = torch.full((M, (N + 3) // 4 * 4 + 4), float("nan"), device="cuda")
+    r = torch.from_numpy(rng.standard_normal((M, (N + 3) // 4 * 4)).astype(np.float32)).cuda()
+    gpt.gemm_f32(a, b, bool(a_mn), bool(b_mn), out=out[:, :N])
+    want = (a.double().T if a_mn else a.double()) @ (b.double() if b_mn else b.double().T)
+    bound = 2e-6 * max(1.0, K ** 0.5 / 4) * want.abs().max().item()
+    assert (out[:, :N].double() - want).abs().max().item() <= bound and out[:, N:].isnan().all()
+    from deers_b200 import _lib
+    got = gpt.gemm_f32(a, b, bool(a_mn), bool(b_mn), epilogue=_lib.EPI_ADD, residual=r[:, :N])
+    assert (got.double() - want - r[:, :N].double()).abs().max().item() <= bound + 1e-6
