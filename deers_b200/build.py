@@ -14,7 +14,7 @@ LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libdeers_b200.so")
 HOST_SRC = os.path.join(CSRC, "host_ext.cpp")
 HOST_EXT = os.path.join(LIB_DIR, "_deers_host.so")      # native host layer of the Python mirror (ops.py)
-SOURCES = ["ctx.cu", "attn_f32.cu", "attn_f32_few.cu", "umma_selftest.cu", "attn_fwd_f16_sm100.cu", "attn_bwd_f16_sm100.cu",
+SOURCES = ["ctx.cu", "attn_f32.cu", "attn_f32_few32.cu", "attn_f32_few64.cu", "attn_f32_few96.cu", "attn_f32_few128.cu", "umma_selftest.cu", "attn_fwd_f16_sm100.cu", "attn_bwd_f16_sm100.cu",
            "rope_pack.cu", "optim.cu", "rmsnorm.cu", "attn_decode.cu", "gemm_f16_sm100.cu", "gemm_f16x3_sm100.cu", "gemm_f32.cu",
            "gemm_f32_loose.cu", "gemm_f32_tc.cu", "gemm_f32_tc_loose.cu", "gpt_ops.cu", "gpt_model.cu", "comm.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -27,12 +27,16 @@ int bwd_rows(const deers_ctx* ctx, const F32Params& p, int resident) {
 template <int DP, int NG, int FBN>
 int fwd_any_rows(deers_ctx* ctx, const F32Params& p) {
     const int rm = fwd_rows(ctx, p);
-    return rm == 4 ? fwd_launch_f32<DP, NG, FBN, 4>(ctx, p) : launch_attn_fwd_f32_few(ctx, p, DP, NG, FBN, rm);
+    if (rm == 4) return fwd_launch_f32<DP, NG, FBN, 4>(ctx, p);
+    return DP == 32 ? launch_attn_fwd_f32_few32(ctx, p, NG, FBN, rm) : DP == 64 ? launch_attn_fwd_f32_few64(ctx, p, NG, FBN, rm)
+         : DP == 96 ? launch_attn_fwd_f32_few96(ctx, p, NG, FBN, rm) : launch_attn_fwd_f32_few128(ctx, p, NG, FBN, rm);
 }
 template <int DP, int NG>
 int bwd_any_rows(deers_ctx* ctx, const F32Params& p) {
     const int rm = bwd_rows(ctx, p, DP <= 64 && NG == 4 ? 2 : 1);
-    return rm == 4 ? bwd_launch_f32<DP, NG, 4>(ctx, p) : launch_attn_bwd_f32_few(ctx, p, DP, NG, rm);
+    if (rm == 4) return bwd_launch_f32<DP, NG, 4>(ctx, p);
+    return DP == 32 ? launch_attn_bwd_f32_few32(ctx, p, NG, rm) : DP == 64 ? launch_attn_bwd_f32_few64(ctx, p, NG, rm)
+         : DP == 96 ? launch_attn_bwd_f32_few96(ctx, p, NG, rm) : launch_attn_bwd_f32_few128(ctx, p, NG, rm);
 }
 
 // Narrow heads stream 64 keys at a time (half the reads of Q per score), unless the sequence has so few tiles that groups

@@ -38,9 +38,15 @@ struct F32Params {
     const float* cosv; const float* sinv;   // backward: dQ and dK leave rotated back by their position ([T][D / 2]; nullptr: not)
 };
 
-// Blocks of 16 or 8 stationary rows (attn_f32_few.cu; a module of its own: the first call of a process loads all kernels of its module).
-int launch_attn_fwd_f32_few(deers_ctx* ctx, const F32Params& p, int dp, int groups, int stream, int rm);
-int launch_attn_bwd_f32_few(deers_ctx* ctx, const F32Params& p, int dp, int groups, int rm);
+// Blocks of 16 or 8 stationary rows (attn_f32_few.cuh), by tile width.
+int launch_attn_fwd_f32_few32(deers_ctx* ctx, const F32Params& p, int groups, int stream, int rm);
+int launch_attn_bwd_f32_few32(deers_ctx* ctx, const F32Params& p, int groups, int rm);
+int launch_attn_fwd_f32_few64(deers_ctx* ctx, const F32Params& p, int groups, int stream, int rm);
+int launch_attn_bwd_f32_few64(deers_ctx* ctx, const F32Params& p, int groups, int rm);
+int launch_attn_fwd_f32_few96(deers_ctx* ctx, const F32Params& p, int groups, int stream, int rm);
+int launch_attn_bwd_f32_few96(deers_ctx* ctx, const F32Params& p, int groups, int rm);
+int launch_attn_fwd_f32_few128(deers_ctx* ctx, const F32Params& p, int groups, int stream, int rm);
+int launch_attn_bwd_f32_few128(deers_ctx* ctx, const F32Params& p, int groups, int rm);
 
 namespace {
 
