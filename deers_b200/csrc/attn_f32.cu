@@ -44,10 +44,13 @@ int bwd_any_rows(deers_ctx* ctx, const F32Params& p) {
 // take eight groups of 32 keys each where the blocks are few: up to 256 keys that is one tile per group (B4 H6 T256 D32 10.8 ->
 // 8.7), beyond, with an SM per block, half the walk (B1 H2 T1024 23.2 -> 21.5).  Heads of 64 do not gain (T 256 11.1 against 11.9,
 // T 512 19.9 against 20.6).
+// With more blocks heads up to 32 wide keep tiles of 32 keys to 512 of them, in blocks of 16 rows up to two of 32 per SM (tiles of 64 / these: B8 H6 T256
+// D32 14.4 / 12.4, B32 H12 T160 48.9 / 39.9, B4 H8 T400 19.4 / 18.2, B8 H8 T512 46.2 / 45.4; B2 H8 T300 13.2 / 8.8; error of O 1.9e-7 / 1.8e-7).
 template <int DP>
 int fwd_impl(deers_ctx* ctx, const F32Params& p) {
     if constexpr (DP <= 32) {
         if (p.T > 128 && few_blocks(ctx, p, 1, p.T <= 256 ? 2 : 1)) return fwd_any_rows<DP, 8, 32>(ctx, p);
+        if (p.T > 128 && p.T <= 512) return few_blocks(ctx, p, 1, 2) ? launch_attn_fwd_f32_few32(ctx, p, 4, 32, 2) : fwd_launch_f32<DP, 4, 32, 4>(ctx, p);
     }
     if constexpr (DP <= 64) {
         if (p.T > 128) return fwd_any_rows<DP, 4, 64>(ctx, p);

@@ -903,7 +903,7 @@ def test_gpt_cross_entropy_from_the_head_product(V, H, D, B, T):
 
 @pytest.mark.parametrize("B,H,T,D", [
     (1, 1, 2, 32), (1, 2, 7, 30), (1, 1, 8, 64), (2, 2, 9, 16), (1, 3, 33, 48), (1, 1, 257, 32), (1, 2, 200, 64), (1, 1, 90, 96), (1, 1, 70, 128),     # 8 rows a block
-    (2, 5, 97, 32), (3, 4, 77, 48), (1, 6, 256, 32), (1, 12, 333, 20), (1, 2, 1000, 32), (1, 7, 130, 64), (1, 3, 300, 96), (2, 4, 100, 126)])         # 16 rows
+    (2, 5, 97, 32), (3, 4, 77, 48), (1, 6, 256, 32), (2, 8, 300, 30), (10, 4, 260, 16), (16, 4, 161, 32), (1, 12, 333, 20), (1, 2, 1000, 32), (1, 7, 130, 64), (1, 3, 300, 96), (2, 4, 100, 126)])         # 16 rows
 @pytest.mark.parametrize("causal", [True, False])
 def test_f32_attention_in_blocks_of_few_rows(B, H, T, D, causal):
     """Calls of few blocks, in blocks of 8 and 16 stationary rows: sequences that end inside a block and a streamed tile, both group counts, either
