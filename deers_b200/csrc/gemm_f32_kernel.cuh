@@ -212,7 +212,7 @@ struct GemmShape {
     static constexpr int RED = KS * BM * RLD;
     static constexpr int STAGES = BM * BN > 64 * 64 ? 3 : 4;
     static constexpr int SQ_AT = STAGES * STAGE > RED ? STAGES * STAGE : RED;    // row sums of squares of the FUSED kernels
-    static constexpr size_t NEED = (size_t)(SQ_AT + KS * BM) * sizeof(float);
+    static constexpr size_t NEED = (size_t)(SQ_AT + (KS + 1) * BM) * sizeof(float);
     // A large block has an SM to itself: two of them share its issue slots while others idle (chained launches place the
     // next product's blocks before this one's have left).  Only the 32 x 64 tiles fit twice: 512 x 512 x 64 4.0 -> 3.2 us, GPT forward of
     // 4 layers, C 320, 200 tokens 234 -> 204; nothing measured got slower.
@@ -245,7 +245,7 @@ __device__ __forceinline__ float4 patch_sum(const float* q, int parts) {
 }
 
 // What follows a tile's products: KS patches of BM x BN partial sums lie in `red` (rows of BN + 4), with FUSED the rows' sums of squares
-// in sq_s [KS][BM].  Meets, adds the k groups and the blocks of the cluster, applies norm, rotation and epilogue, and stores.
+// in sq_s [KS][BM] (and room for BM more).  Meets, adds the k groups and the blocks of the cluster, applies norm, rotation and epilogue, and stores.
 // What the epilogue reads from global memory is requested before the block's meeting (behind it, it cost 400 to 700 cycles of a product's 5000), and
 // behind a cluster's, whose arrival would wait for it, beside the reads of the other blocks' patches.
 template <int BM, int BN, int KS, int THREADS, bool FUSED>
@@ -261,17 +261,41 @@ __device__ __forceinline__ void finish_tile(const GemmArgs& g, float* const red,
     const int first = r_begin * (BN / 4) + threadIdx.x, last = r_end * (BN / 4);
     const bool from_r = g.epi == DEERS_EPI_ADD, from_aux = g.epi == DEERS_EPI_MUL_AUX2;
     float4 ext[ITEMS], c4[FUSED ? ITEMS : 1], s4[FUSED ? ITEMS : 1];
+    // Where a thread's items lie in one column (all tiles but the 96 wide) it divides once, not per item: with that and the square root
+    // and division of the norm in every item a tile of 128 x 64 took 9000 to 11000 cycles here, one of 16 x 32 2500 (1024 x 576 and 768 x 192 in the
+    // model 13.7 -> 12.0 us; 22 M parameters, 4 training steps and a forward 5130 -> 5040).
+    constexpr bool ONE_COLUMN = THREADS % (BN / 4) == 0;
+    constexpr int ROW_STEP = THREADS / (BN / 4);
+    bool second[ITEMS];                                             // the column lies in the second half of its head
     auto request = [&]() {
+        unsigned pos = 0, hc = 0;
+        if constexpr (FUSED) {
+            if (g.rope_cols) {
+                pos = (unsigned)(m0 + first / (BN / 4)) % (unsigned)g.rope_t;
+                hc = (unsigned)(n0 + first % (BN / 4) * 4) % (unsigned)g.rope_d;
+            }
+        }
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
             const int idx = first + i * THREADS, m = m0 + idx / (BN / 4), n = n0 + (idx % (BN / 4)) * 4;
             const bool in = idx < last && m < g.M && n < g.N;
             if (in && (from_r || from_aux))
                 ext[i] = ld4(from_r ? g.r + (long long)m * g.ldr + n : g.aux + (long long)m * g.ldc + n, g.N - n, g.c_vec);
+            second[i] = false;
             if constexpr (FUSED) {
+                if (g.rope_cols && i > 0) {
+                    if constexpr (ONE_COLUMN) {
+                        pos += ROW_STEP;
+                        if (pos >= (unsigned)g.rope_t) pos = g.rope_t >= ROW_STEP ? pos - g.rope_t : pos % (unsigned)g.rope_t;
+                    } else {
+                        pos = (unsigned)m % (unsigned)g.rope_t;
+                        hc = (unsigned)n % (unsigned)g.rope_d;
+                    }
+                }
                 if (in && n < g.rope_cols) {
-                    const int half = g.rope_d / 2, hc = n % g.rope_d;
-                    const long long at = (long long)(m % g.rope_t) * half + (hc >= half ? hc - half : hc);
+                    const unsigned half = (unsigned)g.rope_d / 2;
+                    second[i] = hc >= half;
+                    const size_t at = (size_t)(pos * half + (second[i] ? hc - half : hc));
                     c4[i] = *reinterpret_cast<const float4*>(g.cosv + at);
                     s4[i] = *reinterpret_cast<const float4*>(g.sinv + at);
                 }
@@ -302,6 +326,22 @@ __device__ __forceinline__ void finish_tile(const GemmArgs& g, float* const red,
         cg::this_cluster().sync();
         request();
     }
+    if constexpr (FUSED) {                                          // inverse norms, once per row, behind the sums [KS][BM]
+        if (threadIdx.x < BM) {
+            const int row = threadIdx.x;
+            float t = 0.f;
+            if (parts > 1) {
+                for (int z = 0; z < parts; ++z) t += *cg::this_cluster().map_shared_rank(sq_s + row, z);
+            } else {
+#pragma unroll
+                for (int z = 0; z < KS; ++z) t += sq_s[z * BM + row];
+            }
+            const float inv = 1.0f / sqrtf(t * g.inv_n + g.eps);
+            sq_s[KS * BM + row] = inv;
+            if (g.inv && n0 == 0 && row >= r_begin && row < r_end && m0 + row < g.M) g.inv[m0 + row] = inv;
+        }
+        __syncthreads();
+    }
     chain_next();                                                   // (at the loop or earlier, successors crowd out the side stream)
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
@@ -316,26 +356,17 @@ __device__ __forceinline__ void finish_tile(const GemmArgs& g, float* const red,
         float o[4] = {v.x, v.y, v.z, v.w}, x[4] = {0.f, 0.f, 0.f, 0.f};
         float* cp = g.c + (long long)m * g.ldc + n;
         if constexpr (FUSED) {
-            float t = 0.f;
-            if (parts > 1) {
-                for (int z = 0; z < parts; ++z) t += *cg::this_cluster().map_shared_rank(sq_s + row, z);
-            } else {
-#pragma unroll
-                for (int z = 0; z < KS; ++z) t += sq_s[z * BM + row];
-            }
-            const float inv = 1.0f / sqrtf(t * g.inv_n + g.eps);
-            if (g.inv && n == 0) g.inv[m] = inv;
+            const float inv = sq_s[KS * BM + row];
 #pragma unroll
             for (int e = 0; e < 4; ++e) o[e] *= inv;
             if (n < g.rope_cols) {
                 // the other half of the head lies in this tile (tiles hold whole heads); rounded as the rotary pack does
                 const int half = g.rope_d / 2;
-                const bool second = n % g.rope_d >= half;
-                const float4 u = patch_sum<KS, BM * RLD>(second ? q - half : q + half, parts);
+                const float4 u = patch_sum<KS, BM * RLD>(second[i] ? q - half : q + half, parts);
                 const float p[4] = {u.x * inv, u.y * inv, u.z * inv, u.w * inv}, cs[4] = {c4[i].x, c4[i].y, c4[i].z, c4[i].w}, sn[4] = {s4[i].x, s4[i].y, s4[i].z, s4[i].w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    o[e] = second ? __fadd_rn(__fmul_rn(p[e], -sn[e]), __fmul_rn(o[e], cs[e])) : __fadd_rn(__fmul_rn(o[e], cs[e]), __fmul_rn(p[e], sn[e]));
+                    o[e] = second[i] ? __fadd_rn(__fmul_rn(p[e], -sn[e]), __fmul_rn(o[e], cs[e])) : __fadd_rn(__fmul_rn(o[e], cs[e]), __fmul_rn(p[e], sn[e]));
             }
         }
         if (from_r) {

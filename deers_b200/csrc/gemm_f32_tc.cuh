@@ -32,7 +32,7 @@ constexpr uint32_t TC_A = 128 * 128, TC_B = 64 * 128;            // one of the t
 constexpr uint32_t TC_STAGE = 3 * (TC_A + TC_B);
 constexpr uint32_t TC_BLOCK = 64 * 128;                          // MN order: 64 k by 64 columns
 constexpr uint32_t TC_SQ = TC_RING * TC_STAGE;                 // rows' sums of squares
-constexpr uint32_t TC_BARS = TC_SQ + TC_M * 4;
+constexpr uint32_t TC_BARS = TC_SQ + 2 * TC_M * 4;               // (and the inverse norms)
 constexpr uint32_t TC_SMEM = TC_BARS + 64;                      // a barrier per stage, TMEM base, abort flag
 static_assert(TC_M * (TC_N + 4) * 4 <= TC_SQ && TC_SMEM <= 232448, "shared memory");
 // TMEM columns: main of six steps of 16 k, used in turn | corr1 | corr2
