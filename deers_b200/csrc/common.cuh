@@ -188,7 +188,7 @@ int deers_check_tensor(const deers_attn_desc* d, const void* p, const int64_t* s
 int deers_check_bwd_args(const deers_attn_desc* d, const void* q, const void* k, const void* v, const void* o,
                          const float* lse, const void* d_o, void* dq, void* dk, void* dv);
 
-// f32 FFMA path (attn_f32.cu)
+// f32 attention, FFMA (attn_f32.cu)
 int launch_attn_fwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q, const float* k,
                         const float* v, float* o, float* lse);
 int launch_attn_bwd_f32(deers_ctx* ctx, const deers_attn_desc* d, const float* q, const float* k,

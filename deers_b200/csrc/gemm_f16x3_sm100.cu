@@ -10,7 +10,8 @@
 // It serves `lm_head` of src/models/gpt.rs:351 and the two products of its backward (src/ops.rs:1089-1101):
 // 80 % of the FLOPs of a training step of the reference's GPT.
 //
-// Persistent kernel, 128 x 128 output tiles, 64-deep K blocks, 3-stage TMA ring of four operand tiles (A_hi,
+// Two kernels.  gemm_f16x3_pair_kernel (described there): pairs of CTAs, the head of a training step.  gemm_f16x3_kernel, for products of few
+// tiles: persistent, 128 x 128 output tiles, 64-deep K blocks, 3-stage TMA ring of four operand tiles (A_hi,
 // A_lo, B_hi, B_lo: 64 KB per stage, 128-byte swizzle, out-of-range rows / columns read as zero), twelve MMAs
 // per K block, two pairs of TMEM accumulators so the epilogue of a tile overlaps the next tile's products.
 // Either storage order of A and of B (the operand orders of forward, dgrad and wgrad), as in gemm_f16_sm100.cu.

@@ -1,15 +1,16 @@
 // A tile of an f32 GEMM on the tensor core without the loss of f32: every operand value is three bf16,
-//     x = h + m + l,    h = bf16(x), m = bf16(x - h), l = bf16(x - h - m)      (all 24 bits: the remainders are exact)
-// and a product is the six of their nine products that reach 2^-24:
-//     main += Ah Bh          corr1 += Ah Bm + Am Bh          corr2 += Ah Bl + Am Bm + Al Bh
+//     x = h + m 2^-8 + l 2^-16,    h = bf16(x), m = bf16((x - h) 2^8), l = bf16(((x - h) 2^8 - m) 2^8)
+// (all 24 bits: the remainders are exact; the tensor core takes parts below 2^-126 for zeros, which the scaling keeps away from
+// every value of 2^-111 and more, unscaled ones lost bits from 2^-103 on; smaller values lose less than 2^-134) and a product is the six of their nine products that reach 2^-24:
+//     main += Ah Bh          corr1 += Ah Bm + Am Bh          corr2 += Ah Bl + Am Bm + Al Bh          C = main + corr1 2^-8 + corr2 2^-16
 // The tensor core rounds its sums towards zero, which a long walk in one accumulator shows (two f16 per value and one accumulator:
 // 2-norm error 2.8e-7 at K = 192, all positive 8e-7, where FFMA sums have 1.3e-7 and 7e-8).  So `main` starts anew with every 16 k, in
 // columns of its own, and these sums are added in f32, rounded to nearest, by the threads that take them out; the
 // corrections are 2^-8 of it and smaller and may run on.  2-norm errors against 64 bits, FFMA kernels and these: normal operands K = 192 1.3e-7
 // and 5.8e-8, K = 768 1.4e-7 and 7.0e-8, K = 1024 2.1e-7 and 7.3e-8; all positive K = 192 6.3e-8 and 4.5e-8, K = 768 4.6e-8 and 4.3e-8
 // (every 32 k instead: 6.2e-8 and 5.6e-8).
-// bf16 has the exponents of f32, so no scaling; a block that meets an infinity, a NaN or a value whose h overflows works its tile out
-// again with FFMA sums (0 * inf must not appear where x * y has none).
+// bf16 has the exponents of f32; a block that meets an infinity, a NaN or a value whose h overflows, or whose sums overflow, works its tile
+// out again with FFMA sums (0 * inf must not appear where x * y has none).
 //
 // A block owns a tile of 128 x 64: 512 threads load, split and store a stage of 64 k (128-byte swizzle, in the operand's own storage
 // order) while the products of the stage before run and the one after is on its way.  Blocks of a cluster share a long K and
@@ -57,6 +58,11 @@ __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
     return v;
 }
 
+// What two values' parts leave, times 2^8.
+__device__ __forceinline__ void remainders(float& a, float& b, float fa, float fb) {
+    unpack_f32x2(mul2(fma2(pack_f32x2(fa, fb), pack_f32x2(-1.f, -1.f), pack_f32x2(a, b)), pack_f32x2(256.f, 256.f)), a, b);
+}
+
 // Splits eight values and stores the three parts, `part` bytes apart.  `bad` turns NaN when an h is not finite.
 __device__ __forceinline__ void split8(uint8_t* dst, uint32_t part, const float (&x)[8], float& bad) {
     uint32_t w[3][4];
@@ -69,7 +75,7 @@ __device__ __forceinline__ void split8(uint8_t* dst, uint32_t part, const float 
             if (q == 2) break;
             const float fa = __uint_as_float(w[q][e] << 16), fb = __uint_as_float(w[q][e] & 0xffff0000u);
             if (q == 0) bad = fmaf(fa, 0.f, fmaf(fb, 0.f, bad));
-            a -= fa; b -= fb;
+            remainders(a, b, fa, fb);
         }
     }
 #pragma unroll
@@ -84,7 +90,7 @@ __device__ __forceinline__ void split2(uint8_t* dst, uint32_t part, float a, flo
         *reinterpret_cast<uint32_t*>(dst + q * part) = w;
         const float fa = __uint_as_float(w << 16), fb = __uint_as_float(w & 0xffff0000u);
         if (q == 0) bad = fmaf(fa, 0.f, fmaf(fb, 0.f, bad));
-        a -= fa; b -= fb;
+        remainders(a, b, fa, fb);
     }
 }
 
@@ -216,7 +222,7 @@ __device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int ti
             tmem_ld_x16(t_out + TC_C2, u[1]);
             tmem_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 16; ++e) v[e] += __uint_as_float(u[0][e]) + __uint_as_float(u[1][e]);
+            for (int e = 0; e < 16; ++e) v[e] = fmaf(fmaf(__uint_as_float(u[1][e]), 0x1p-8f, __uint_as_float(u[0][e])), 0x1p-8f, v[e]);
         }
 #pragma unroll
         for (int e = 0; e < 16; ++e) sum[e] += v[e];
@@ -281,13 +287,14 @@ __device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int ti
             if (lane % 8 == 0) sq_s[oa.row + i * OA::ROW_STEP] = sq[i];
         }
     }
-    const bool slow = __syncthreads_or(!(bad == 0.f)) != 0;
     drain(min(4, (left + 15) / 16), true);
     float* red = reinterpret_cast<float*>(tc_smem);                // every product has read its operands
 #pragma unroll
+    for (int e = 0; e < 16; ++e) bad = fmaf(sum[e], 0.f, bad);
+#pragma unroll
     for (int e = 0; e < 16; e += 4)
         *reinterpret_cast<float4*>(red + out_row * (TC_N + 4) + out_col + e) = make_float4(sum[e], sum[e + 1], sum[e + 2], sum[e + 3]);
-    __syncthreads();
+    const bool slow = __syncthreads_or(!(bad == 0.f)) != 0;
     if (warp == 1) tmem_dealloc(tmem, 512);
     if (slow) {
         for (int i = t; i < TC_M * TC_N; i += TC_T) {

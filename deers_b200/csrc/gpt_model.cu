@@ -5,14 +5,14 @@
 //   reading q, k, v in place as strided views and writing O token-major; x1 = x + O * Wout (residual in the GEMM epilogue);
 //   r = relu(rmsnorm(x1) * Wup), h = r*r (norm and relu in the GEMM); x2 = x1 + h * Wdown (epilogue).
 //   Separate norm and rotary kernels, eight launches per block before, cost 1.4 to 2 us each at these sizes.
-// Head: xf = rmsnorm(x) as an f16 pair; logits = xf * Wlm; cross-entropy reads the logits once; the backward overwrites
-// them with their gradient in one pass and feeds the two head GEMMs.
+// Head: xf = rmsnorm(x) as an f16 pair; logits = xf * Wlm with each row's maximum and sum of exponentials per tile, from which a small kernel
+// makes lse and the picked log-probabilities; the backward reads the logits once, in one pass, and feeds the two head GEMMs.
 // Backward: the exact transposes of the above, with the relu^2 backward in a GEMM epilogue, the residual
 // gradient added inside the RMSNorm backward (which also writes the normalised rows again, for the weight gradients), dQ / dK
 // rotated back by the attention backward straight into the fused [N, 3C] gradient buffer next to dV, and one GEMM for the sum of
 // the three input gradients.  Every launch is one of this library's kernels; there is no host round trip in a step.
 // The weight gradients are off the critical path (nothing in the backward reads them): the four of a block are one
-// launch on a second stream, or four where one would be several waves of blocks, forked from the main one where their operands
+// launch on a second stream (four where one would be several waves of blocks, three and one for the block the backward ends with), forked from the main one where their operands
 // are complete and joined before the gradient norm; captured, the two streams become two branches of the step's graph.  What
 // they read is double-buffered by block.
 #include "common.cuh"
@@ -286,7 +286,7 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
         LayerAct& a = m->la[l];
         LayerGrad &d = m->lg[l & 1], &below = m->lg[(l & 1) ^ 1];
         const float* x_in = l ? m->la[l - 1].x2 : m->x0;
-        // On the second stream: all four at the block's end in one launch, or each as soon as its operands are there.  Of the last block
+        // On the second stream: all four at the block's end in one launch, or each as soon as its operands are there.  Of block 0
         // the first three go ahead in one launch: nothing follows that all four could run beside (22 M parameters, 1024 tokens: 25 us of the four
         // behind the last norm, then 16 of the one).
         const GemmTN grads[4] = {{Hm, C, a.h, d.dx, G + w.down}, {C, Hm, d.n2, d.dh, G + w.up},              // d Wdown = h^T dx, d Wup = n2^T du
@@ -483,7 +483,7 @@ extern "C" int deers_b200_gpt_create(deers_ctx* ctx, const deers_gpt_config* cfg
     if (!m) return DEERS_ERR_CUDA;
     m->ctx = ctx; m->cfg = *cfg; m->max_batch = max_batch; m->max_tokens = max_tokens; m->D = D;
     m->Vld = (cfg->vocab_size + 7) / 8 * 8;                           // rows of the head, of the logits and of their f16 pairs start 16-byte aligned
-    // Heads that fill the tensor core take the split-f16 products; small ones stay on the FFMA kernel.
+    // Heads that fill the tensor core take the split-f16 products; small ones are products like those of the blocks.
     m->tc_head = cfg->vocab_size >= 1024 && cfg->n_embd % 8 == 0 && cfg->n_embd >= 64;
     m->graph_enabled = true; m->graph_exec = nullptr; m->graph_B = m->graph_T = -1; m->eager_steps_BT = 0;
     m->on_side = false;

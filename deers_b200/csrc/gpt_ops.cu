@@ -8,8 +8,8 @@
 //                   owns the row and adds the later occurrences in order, so the result is reproducible
 //                   and equals the CPU backend's left-to-right sum.
 //   cross_entropy   one block per row reads the logits once (running maximum / sum of exponentials),
-//                   writes lse[row] and the picked log-probability; a one-block kernel adds the rows in a
-//                   fixed order: loss = sum * (float)(-1/rows).
+//                   writes lse[row] and the picked log-probability (in the model these come from the head product's statistics
+//                   per row and tile, merged in order); a one-block kernel adds the rows in a fixed order: loss = sum * (float)(-1/rows).
 //   cross_entropy_bwd  dlogits = (onehot * g - softmax * g) * upstream, g = (float)(-1/rows): the chain
 //                   gather backward -> log_softmax backward of src/ops.rs:210-214, 777-799, 1162-1175 in one
 //                   element-wise pass (in place over the logits if asked).
