@@ -779,8 +779,8 @@ def run_gpt_step(args):
     if rank == 0:
         peaks = load_peaks()
         # Two GEMM families: the head (lm_head forward, its weight and input gradients: 3 products of
-        # 2 * 1024 * 50257 * 192 FLOPs) on the tensor core as split-f16 products, and the 72 products of the blocks on
-        # the FFMA pipe.  The roofline entry is the family that takes longer.
+        # 2 * 1024 * 50257 * 192 FLOPs) on the tensor core as split-f16 products, and the 72 products of the blocks, the
+        # larger on the tensor core as split-bf16 products, the smaller on the FFMA pipe, whose peak is what they are held against.  The roofline entry is the family that takes longer.
         n_tok, C_, Hm_, V_ = c["B"] * c["T"], c["n_embd"], c["mlp"], c["vocab"]
         head_flops = 6.0 * n_tok * C_ * V_
         block_flops = 6.0 * n_tok * c["n_layer"] * (4 * C_ * C_ + 2 * C_ * Hm_)
@@ -791,22 +791,22 @@ def run_gpt_step(args):
         at_max_clock = bool(clocks and clocks.get("sm_mhz") and clocks["sm_mhz"] >= 0.95 * sm_max and
                             "sw_power_cap" not in clocks.get("reasons", []))
         tc_peak = peaks["tflops_burst" if at_max_clock else "tflops_sustained"]
-        head = {"bound": "tensor", "kernel": "gemm_f16x3_kernel + split / reduce (lm_head forward, wgrad, dgrad)",
+        head = {"bound": "tensor", "kernel": "gemm_f16x3_pair_kernel + split / reduce (lm_head forward, wgrad, dgrad)",
                 "achieved": head_flops / (head_ms * 1e-3) / 1e12 if head_ms else None, "peak": tc_peak, "unit": "TFLOP/s",
                 "frac": (head_flops / (head_ms * 1e-3) / 1e12 / tc_peak) if head_ms else None,
                 # DRAM bytes per step of the three products, the two splits and the reduction, from the ncu capture of
                 # this very workload (profiles/gpt_step_cfg3_kernels.md); None at other model sizes
-                "traffic": 725.0e6 if (n_tok, C_, V_) == (1024, 192, 50257) else None,
+                "traffic": 730.0e6 if (n_tok, C_, V_) == (1024, 192, 50257) else None,
                 "flops_per_step": head_flops, "kernel_ms_per_step": head_ms,
                 "note": "algorithmic f32 FLOPs; the kernel executes three f16 products per f32 product",
                 "peak_source": f"{peaks['source']} {'burst' if at_max_clock else 'sustained'} bf16"}
-        block = {"bound": "fp32 FFMA pipe (the reference computes these products in full f32, CUBLAS_COMPUTE_32F)",
-                 "kernel": "gemm_f32_kernel (the 72 Linear forward / dgrad / wgrad products of the blocks)",
+        block = {"bound": "full f32 accuracy (CUBLAS_COMPUTE_32F in the reference), against the FFMA pipe's peak; the kernels on the tensor core: shared memory",
+                 "kernel": "gemm_f32_tc_kernel, gemm_f32_kernel (the 72 Linear forward / dgrad / wgrad products of the blocks)",
                  "achieved": block_flops / (block_ms * 1e-3) / 1e12 if block_ms else None, "peak": ffma_peak, "unit": "TFLOP/s",
                  "frac": (block_flops / (block_ms * 1e-3) / 1e12 / ffma_peak) if block_ms else None,
-                 # DRAM bytes per step: 72 launches x 2.24 MB, the mean of the four forward shapes captured by ncu at this
+                 # DRAM bytes per step: all 55 launches of these products as captured by ncu at this
                  # workload (operands and results live in L2; profiles/gpt_step_cfg3_kernels.md); None at other sizes
-                 "traffic": 161.0e6 if (n_tok, C_, Hm_, c["n_layer"]) == (1024, 192, 768, 6) else None,
+                 "traffic": 204.0e6 if (n_tok, C_, Hm_, c["n_layer"]) == (1024, 192, 768, 6) else None,
                  "flops_per_step": block_flops, "kernel_ms_per_step": block_ms,
                  "peak_source": f"148 SMs x 128 FFMA lanes x 2 x {sm_max:.0f} MHz (nominal; MEASURED_PEAKS.json holds no f32 figure)"}
         roofline = dict(head if head_ms >= block_ms else block)

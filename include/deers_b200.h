@@ -345,7 +345,8 @@ int deers_b200_gemm_f16(deers_ctx* ctx, int32_t M, int32_t N, int32_t K, const v
                         const void* b, int64_t ldb, int32_t b_mn_major, void* c, int64_t ldc);
 
 /*
- * f32 GEMM in full f32 arithmetic (FFMA; no TF32) for the projections of the f32 model: C[M,N] = A * B,
+ * f32 GEMM at full f32 accuracy (FFMA, or for large products the tensor core on exact three-way bf16 splits whose sums are
+ * added in f32: errors no larger than FFMA's; no TF32) for the projections of the f32 model: C[M,N] = A * B,
  * C row-major with leading dimension ldc.  Replaces the `cublasGemmStridedBatchedEx` call with
  * CUBLAS_COMPUTE_32F behind `Tensor::matmul` for f32 operands (`src/storage/cuda.rs:1098-1128`) as
  * `Linear::forward` uses it (`src/nn.rs:184-190`, weight stored [in_features, out_features]) and as the
