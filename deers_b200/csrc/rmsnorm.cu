@@ -42,7 +42,10 @@ __device__ __forceinline__ void put_pair(__half* hi, __half* lo, long long at, c
 
 // BWD = false: y = x * inv, inv_out[row] = inv (PAIR: y leaves as the f16 pair hi, lo, rows dense, instead of out).
 // BWD = true: dx from x, dy and the saved inv; n_out (may be nullptr) receives y again for the weight gradient.
-template <bool BWD, bool VEC, bool VEC2 = false, bool PAIR = false>
+// NV: 16-byte pieces of a lane.  Of rows of up to 256 the backward requests everything at once, the residual and the norm too: behind the sum
+// they were two more trips to L2 (22 M parameters, 1024 rows of 192, 13 a step: 4 steps and a forward 5057 -> 4996 us; 3 layers,
+// 231 rows 1230 -> 1203).  Longer rows do not have the registers.
+template <bool BWD, bool VEC, bool VEC2 = false, bool PAIR = false, int NV = RN_MAXV>
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const float* dy, const float* add, float* __restrict__ out,
                                                       float* __restrict__ inv_io, long long rows, int C, float eps,
                                                       float inv_n, float* __restrict__ n_out, __half* __restrict__ hi,
@@ -56,11 +59,18 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
         const float* xr = x + row * C;
         float* orow = out + row * C;
         if (VEC) {
-            const int nv = C / 4;                               // float4 pieces in the row (<= 32 * RN_MAXV)
-            float4 xv[RN_MAXV], gv[RN_MAXV];
-            float acc = 0.f;
+            const int nv = C / 4;                               // float4 pieces in the row (<= 32 * NV)
+            float4 xv[NV], gv[NV], av[NV];
+            constexpr bool EARLY = BWD && NV <= 2;
+            float acc = 0.f, early_inv = 0.f;
+            if (EARLY) early_inv = inv_io[row];
 #pragma unroll
-            for (int i = 0; i < RN_MAXV; ++i) {
+            for (int i = 0; i < NV; ++i) {
+                const int p = lane + 32 * i;
+                if (EARLY && add && p < nv) av[i] = reinterpret_cast<const float4*>(add + row * C)[p];
+            }
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
                 const int p = lane + 32 * i;
                 if (p < nv) {
                     xv[i] = reinterpret_cast<const float4*>(xr)[p];
@@ -75,14 +85,14 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
             acc = warp_sum(acc);
             float inv, k = 0.f;
             if (BWD) {
-                inv = inv_io[row];
+                inv = EARLY ? early_inv : inv_io[row];
                 k = acc * inv * inv * inv * inv_n;
             } else {
                 inv = 1.0f / sqrtf(acc * inv_n + eps);
                 if (lane == 0) inv_io[row] = inv;
             }
 #pragma unroll
-            for (int i = 0; i < RN_MAXV; ++i) {
+            for (int i = 0; i < NV; ++i) {
                 const int p = lane + 32 * i;
                 if (p < nv) {
                     float4 o;
@@ -90,7 +100,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
                         o.x = gv[i].x * inv - xv[i].x * k; o.y = gv[i].y * inv - xv[i].y * k;
                         o.z = gv[i].z * inv - xv[i].z * k; o.w = gv[i].w * inv - xv[i].w * k;
                         if (add) {
-                            const float4 r = reinterpret_cast<const float4*>(add + row * C)[p];
+                            const float4 r = EARLY ? av[i] : reinterpret_cast<const float4*>(add + row * C)[p];
                             o.x = r.x + o.x; o.y = r.y + o.y; o.z = r.z + o.z; o.w = r.w + o.w;
                         }
                         if (n_out) reinterpret_cast<float4*>(n_out + row * C)[p] = make_float4(xv[i].x * inv, xv[i].y * inv, xv[i].z * inv, xv[i].w * inv);
@@ -261,7 +271,9 @@ int rms_launch(deers_ctx* ctx, long long rows, int C, float eps, const float* x,
     const float inv_n = (float)(1.0 / (double)C);               // mean = sum * (1/n as f64 -> f32), src/tensor.rs:461-465
     {
         KernelTimerScope ts(ctx, DEERS_K_NORM);
-        if (vec) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
+        if (BWD && vec && C <= 256)
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true, false, false, 2>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
+        else if (vec) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
         else if (aligned && C <= 256 * RN_MAXV * 4) {
             const unsigned bgrid = (unsigned)(rows < cap ? rows : cap);
             DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_block_kernel<BWD>, bgrid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));

@@ -972,3 +972,25 @@ def test_f32_gemm_tiles_of_16_rows(M, N, K, a_mn, b_mn, aligned):
     from deers_b200 import _lib
     got = gpt.gemm_f32(a, b, bool(a_mn), bool(b_mn), epilogue=_lib.EPI_ADD, residual=r[:, :N])
     assert (got.double() - want - r[:, :N].double()).abs().max().item() <= bound + 1e-6
+
+
+@pytest.mark.parametrize("C", [4, 124, 128, 132, 192, 252, 256, 260])
+@pytest.mark.parametrize("rows", [1, 9, 20000])
+def test_rmsnorm_backward_of_short_rows(rows, C):
+    """Rows of up to 256, whose loads all go out at once, and the next longer ones; fewer rows than a block's warps and more than a grid's.  A lane
+    adds C / 32 products, five sums of lanes and a few roundings follow: (C / 32 + 12) 2^-24 for the dot product, half as much for the norm, whose third power
+    stands in the second term: 3 (C / 32 + 12) 2^-24 of the terms' magnitudes."""
+    from deers_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows + C)
+    x, dy = (torch.randn((rows, C), device="cuda", generator=g) for _ in range(2))
+    op = ops.RMSNorm.new(x, 1e-5)
+    op.forward()
+    grads = ops.GradientStore()
+    op.backward(grads, dy)
+    dx = grads.get(op.dependencies()[0])
+    xd, gd = x.double(), dy.double()
+    r = (xd.square().mean(1, keepdim=True) + 1e-5).rsqrt()
+    dot = (xd * gd).sum(1, keepdim=True)
+    want = gd * r - xd * dot * r ** 3 / C
+    terms = (gd * r).abs() + xd.abs() * (xd * gd).abs().sum(1, keepdim=True) * r ** 3 / C
+    assert ((dx.double() - want).abs() <= 3 * (C / 32 + 12) * 2.0 ** -24 * terms).all()
