@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(1024) cross_entropy_merge_kernel(const float2*
             m = M;
         }
     }
+    chain_next();
     // lanes r, r + 8, r + 16, r + 24 of a warp, then the warps
 #pragma unroll
     for (int off = 8; off <= 16; off *= 2) lse_merge(m, s, __shfl_xor_sync(0xffffffffu, m, off), __shfl_xor_sync(0xffffffffu, s, off));

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
                                                       float* __restrict__ inv_io, long long rows, int C, float eps,
                                                       float inv_n, float* __restrict__ n_out, __half* __restrict__ hi,
                                                       __half* __restrict__ lo) {
-    if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room)
+    if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room; short rows below)
     chain_wait();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
                     }
                 }
             }
+            if (EARLY && row + nwarps >= rows) chain_next();       // (a step of 3 layers, 231 rows, four of them and a forward: 1203 -> 1191 us)
             acc = warp_sum(acc);
             float inv, k = 0.f;
             if (BWD) {
