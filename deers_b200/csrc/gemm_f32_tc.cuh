@@ -1,7 +1,7 @@
 // A tile of an f32 GEMM on the tensor core without the loss of f32: every operand value is three bf16,
 //     x = h + m 2^-8 + l 2^-16,    h = bf16(x), m = bf16((x - h) 2^8), l = bf16(((x - h) 2^8 - m) 2^8)
-// (all 24 bits: the remainders are exact; the tensor core takes parts below 2^-126 for zeros, which the scaling keeps away from
-// every value of 2^-111 and more, unscaled ones lost bits from 2^-103 on; smaller values lose less than 2^-134) and a product is the six of their nine products that reach 2^-24:
+// (all 24 bits: the remainders are exact, and the tensor core keeps subnormal bf16, so the parts reach down to f32's 2^-149; unscaled
+// ones would end at 2^-133) and a product is the six of their nine products that reach 2^-24:
 //     main += Ah Bh          corr1 += Ah Bm + Am Bh          corr2 += Ah Bl + Am Bm + Al Bh          C = main + corr1 2^-8 + corr2 2^-16
 // The tensor core rounds its sums towards zero, which a long walk in one accumulator shows (two f16 per value and one accumulator:
 // 2-norm error 2.8e-7 at K = 192, all positive 8e-7, where FFMA sums have 1.3e-7 and 7e-8).  So `main` starts anew with every 16 k, in
@@ -9,8 +9,13 @@
 // corrections are 2^-8 of it and smaller and may run on.  2-norm errors against 64 bits, FFMA kernels and these: normal operands K = 192 1.3e-7
 // and 5.8e-8, K = 768 1.4e-7 and 7.0e-8, K = 1024 2.1e-7 and 7.3e-8; all positive K = 192 6.3e-8 and 4.5e-8, K = 768 4.6e-8 and 4.3e-8
 // (every 32 k instead: 6.2e-8 and 5.6e-8).
-// bf16 has the exponents of f32; a block that meets an infinity, a NaN or a value whose h overflows, or whose sums overflow, works its tile
-// out again with FFMA sums (0 * inf must not appear where x * y has none).
+// A block works its tile out again with FFMA sums (plain_tile) where these cannot stand for them:
+//   - a sum that is not finite: bf16 has the exponents of f32, but values from 2^128 - 2^119 on round to an infinity, a correction may overflow
+//     ahead of its whole, and 0 * inf must not appear where x * y has none.  An h that is not finite makes every sum of its row or column such;
+//   - subnormal operands that a result rests on: their h, and below 2^-134 their m, holds few bits or none, and the three products left
+//     out, 1.5 2^-151 of the other operand at most, are then not 2^-24 of the result but 4e-6 at 2^-134 and 2e-3 at 2^-146.  Sums of 2^-120
+//     times the largest value of either operand or more have them below 2^-24 whatever K, so only smaller ones (not zeros) make the block
+//     look for subnormal operands.
 //
 // A block owns a tile of 128 x 64: 512 threads load, split and store a stage of 64 k (128-byte swizzle, in the operand's own storage
 // order) while the products of the stage before run and the one after is on its way.  Blocks of a cluster share a long K and
@@ -63,8 +68,12 @@ __device__ __forceinline__ void remainders(float& a, float& b, float fa, float f
     unpack_f32x2(mul2(fma2(pack_f32x2(fa, fb), pack_f32x2(-1.f, -1.f), pack_f32x2(a, b)), pack_f32x2(256.f, 256.f)), a, b);
 }
 
-// Splits eight values and stores the three parts, `part` bytes apart.  `bad` turns NaN when an h is not finite.
-__device__ __forceinline__ void split8(uint8_t* dst, uint32_t part, const float (&x)[8], float& bad) {
+// What `large` adds up of the h: not finite any more when one of them is 2^25 or more (or several come near).
+constexpr float TC_LARGE = 0x1p104f;
+constexpr uint32_t TC_SMALL_SUM = (127u - 95u) << 23, TC_SMALL_SUM_OF_LARGE = (127u + 8u) << 23;     // bits of 2^-95 and 2^8: 2^-120 of values below 2^25, and of any
+
+// Splits eight values and stores the three parts, `part` bytes apart.
+__device__ __forceinline__ void split8(uint8_t* dst, uint32_t part, const float (&x)[8], float& large) {
     uint32_t w[3][4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -74,7 +83,7 @@ __device__ __forceinline__ void split8(uint8_t* dst, uint32_t part, const float 
             w[q][e] = bf16x2(a, b);
             if (q == 2) break;
             const float fa = __uint_as_float(w[q][e] << 16), fb = __uint_as_float(w[q][e] & 0xffff0000u);
-            if (q == 0) bad = fmaf(fa, 0.f, fmaf(fb, 0.f, bad));
+            if (q == 0) large = fmaf(fa, TC_LARGE, fmaf(fb, TC_LARGE, large));
             remainders(a, b, fa, fb);
         }
     }
@@ -83,13 +92,13 @@ __device__ __forceinline__ void split8(uint8_t* dst, uint32_t part, const float 
 }
 
 // The same for two values.
-__device__ __forceinline__ void split2(uint8_t* dst, uint32_t part, float a, float b, float& bad) {
+__device__ __forceinline__ void split2(uint8_t* dst, uint32_t part, float a, float b, float& large) {
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         const uint32_t w = bf16x2(a, b);
         *reinterpret_cast<uint32_t*>(dst + q * part) = w;
         const float fa = __uint_as_float(w << 16), fb = __uint_as_float(w & 0xffff0000u);
-        if (q == 0) bad = fmaf(fa, 0.f, fmaf(fb, 0.f, bad));
+        if (q == 0) large = fmaf(fa, TC_LARGE, fmaf(fb, TC_LARGE, large));
         remainders(a, b, fa, fb);
     }
 }
@@ -125,17 +134,47 @@ struct TcOperand {
             }
         }
     }
-    __device__ __forceinline__ void store(uint8_t* s, uint32_t part, const float (&x)[FLOATS], float& bad) const {
+    __device__ __forceinline__ void store(uint8_t* s, uint32_t part, const float (&x)[FLOATS], float& large) const {
 #pragma unroll
         for (int i = 0; i < PIECES; ++i) {
             if constexpr (LOOSE) {
-                split2(s + at + i * ROW_STEP * 128u, part, x[2 * i], x[2 * i + 1], bad);
+                split2(s + at + i * ROW_STEP * 128u, part, x[2 * i], x[2 * i + 1], large);
             } else {
-                split8(s + at + i * ROW_STEP * 128u, part, reinterpret_cast<const float(&)[8]>(x[8 * i]), bad);
+                split8(s + at + i * ROW_STEP * 128u, part, reinterpret_cast<const float(&)[8]>(x[8 * i]), large);
             }
         }
     }
 };
+
+// Whether this thread's share of a piece of an operand, `rows` rows of `len` floats, holds a subnormal value.
+__device__ __forceinline__ bool subnormals(const float* p, long long ld, int rows, int len) {
+    bool any = false;
+    for (int r = threadIdx.x / 32; r < rows; r += TC_T / 32)
+        for (int i = threadIdx.x % 32; i < len; i += 32) {
+            const float x = p[r * ld + i];
+            any |= x != 0.f && fabsf(x) < 0x1p-126f;
+        }
+    return any;
+}
+
+// The tile's sums by FFMA, four to an element as the FFMA kernels' groups have them.  a, b: the first values; rows, cols: those there are.
+template <bool A_MN, bool B_MN>
+__device__ __forceinline__ void plain_tile(float* red, const float* a, long long lda, const float* b, long long ldb, int rows, int cols, int klen) {
+    for (int i = threadIdx.x; i < TC_M * TC_N; i += TC_T) {
+        const int row = i / TC_N, col = i % TC_N;
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        if (row < rows && col < cols) {
+            const float* pa = a + (A_MN ? row : row * lda);
+            const float* pb = b + (B_MN ? col : col * ldb);
+            for (int k = 0; k < klen; k += 4) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (k + e < klen) acc[e] = fmaf(pa[(k + e) * (A_MN ? lda : 1)], pb[(k + e) * (B_MN ? ldb : 1)], acc[e]);
+            }
+        }
+        red[row * (TC_N + 4) + col] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    }
+}
 
 // The part of the start that needs nothing of global memory.
 __device__ __forceinline__ void gemm_f32_tc_prologue() {
@@ -229,13 +268,13 @@ __device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int ti
         tc_fence_before_sync();
     };
 
-    float bad = 0.f, sq[2] = {0.f, 0.f};
+    float large = 0.f, sq[2] = {0.f, 0.f};
     // The place a stage takes is free: the products of the one three before have been waited for (drain).
     auto stage = [&](int s, Stage& x) {
         const int now = s == 0 ? 0 : slot == TC_RING - 1 ? 0 : slot + 1;
         uint8_t* st = tc_smem + now * TC_STAGE;
-        oa.store(st, TC_A, x.of_a, bad);
-        ob.store(st + 3 * TC_A, TC_B, x.of_b, bad);
+        oa.store(st, TC_A, x.of_a, large);
+        ob.store(st + 3 * TC_A, TC_B, x.of_b, large);
         if constexpr (FUSED) {
 #pragma unroll
             for (int e = 0; e < OA::FLOATS; ++e) sq[e / 8] = fmaf(x.of_a[e], x.of_a[e], sq[e / 8]);
@@ -290,22 +329,30 @@ __device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int ti
     drain(min(4, (left + 15) / 16), true);
     float* red = reinterpret_cast<float*>(tc_smem);                // every product has read its operands
 #pragma unroll
-    for (int e = 0; e < 16; ++e) bad = fmaf(sum[e], 0.f, bad);
-#pragma unroll
     for (int e = 0; e < 16; e += 4)
         *reinterpret_cast<float4*>(red + out_row * (TC_N + 4) + out_col + e) = make_float4(sum[e], sum[e + 1], sum[e + 2], sum[e + 3]);
-    const bool slow = __syncthreads_or(!(bad == 0.f)) != 0;
+    float finite = 0.f;
+    uint32_t least = 0xffffffffu;                                  // of the sums' magnitudes but zeros: twice the bits less one
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        finite = fmaf(sum[e], 0.f, finite);
+        least = min(least, 2u * __float_as_uint(sum[e]) - 1u);
+    }
+    bool again = !(finite == 0.f);
+    const bool of_large = !(fabsf(large) < INFINITY);
+    const bool look = __syncthreads_or(again || of_large || least < 2u * TC_SMALL_SUM - 1u) != 0;
     if (warp == 1) tmem_dealloc(tmem, 512);
-    if (slow) {
-        for (int i = t; i < TC_M * TC_N; i += TC_T) {
-            const int row = i / TC_N, col = i % TC_N, m = m0 + row, n = n0 + col;
-            float acc = 0.f;
-            if (m < g.M && n < g.N)
-                for (int k = kbeg; k < kbeg + klen; ++k)
-                    acc = fmaf(g.a[A_MN ? (long long)k * g.lda + m : (long long)m * g.lda + k], g.b[B_MN ? (long long)k * g.ldb + n : (long long)n * g.ldb + k], acc);
-            red[row * (TC_N + 4) + col] = acc;
+    if (look) {
+        const float* a = g.a + (A_MN ? (long long)kbeg * g.lda + m0 : (long long)m0 * g.lda + kbeg);
+        const float* b = g.b + (B_MN ? (long long)kbeg * g.ldb + n0 : (long long)n0 * g.ldb + kbeg);
+        const int rows = min(TC_M, g.M - m0), cols = min(TC_N, g.N - n0);
+        const uint32_t limit = __syncthreads_or(of_large) ? TC_SMALL_SUM_OF_LARGE : TC_SMALL_SUM;
+        if (__syncthreads_or(least < 2u * limit - 1u))
+            again |= subnormals(a, g.lda, A_MN ? klen : rows, A_MN ? rows : klen) || subnormals(b, g.ldb, B_MN ? klen : cols, B_MN ? cols : klen);
+        if (__syncthreads_or(again)) {
+            plain_tile<A_MN, B_MN>(red, a, g.lda, b, g.ldb, rows, cols, klen);
+            __syncthreads();
         }
-        __syncthreads();
     }
     finish_tile<TC_M, TC_N, 1, TC_T, FUSED>(g, red, sq_s, m0, n0, parts, part);
 }

@@ -346,7 +346,7 @@ int deers_b200_gemm_f16(deers_ctx* ctx, int32_t M, int32_t N, int32_t K, const v
 
 /*
  * f32 GEMM at full f32 accuracy (FFMA, or for large products the tensor core on exact three-way bf16 splits whose sums are
- * added in f32: errors no larger than FFMA's; no TF32) for the projections of the f32 model: C[M,N] = A * B,
+ * added in f32: errors no larger than FFMA's, over all of f32's range; no TF32) for the projections of the f32 model: C[M,N] = A * B,
  * C row-major with leading dimension ldc.  Replaces the `cublasGemmStridedBatchedEx` call with
  * CUBLAS_COMPUTE_32F behind `Tensor::matmul` for f32 operands (`src/storage/cuda.rs:1098-1128`) as
  * `Linear::forward` uses it (`src/nn.rs:184-190`, weight stored [in_features, out_features]) and as the

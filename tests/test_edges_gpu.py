@@ -831,10 +831,9 @@ def test_f32_gemm_on_the_tensor_core(M, N, K, a_mn, b_mn, aligned):
 @pytest.mark.parametrize("small", ["a", "b"])
 @pytest.mark.parametrize("power", [-99, -112])
 def test_f32_gemm_on_the_tensor_core_of_small_values(power, small, aligned):
-    """One operand times 2^-99 or 2^-112, the other times 2^64, no value of the unscaled ones below 2^-12.  The tensor core takes parts below 2^-126
-    for zeros.  A value's last bit is 2^-23 of it and stands 2^8 higher in its second part, so values from 2^-111 on lose nothing: bit for bit the
-    unscaled result times a power of two.  From there on a value loses less than 2^-134, here 2^-22 of what the operand typically holds and only where a
-    remainder is that small: 1e-7 in the 2-norm as for other operands (measured 5.8e-8 scaled and not)."""
+    """One operand times 2^-99 or 2^-112, the other times 2^64, no value of the unscaled ones below 2^-12.  The three parts hold every bit of a value;
+    from 2^-111 on its two leading parts are full, and all are the unscaled ones times a power of two: bit for bit the unscaled result so scaled.  Smaller
+    values have fewer bits in the leading parts and more in the last: 1e-7 in the 2-norm as for other operands (measured 5.8e-8 scaled and not)."""
     from deers_b200 import gpt
     M, N, K = 1024, 768, 192
     g = torch.Generator(device="cuda").manual_seed(9)
@@ -848,6 +847,32 @@ def test_f32_gemm_on_the_tensor_core_of_small_values(power, small, aligned):
     assert ((got - want).norm() / want.norm()).item() < 1e-7
     if power == -99:
         assert torch.equal(got, base)
+
+
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn,aligned", [(1024, 768, 192, 0, 1, 1), (1000, 768, 190, 1, 0, 0), (1024, 192, 768, 0, 0, 1)])
+@pytest.mark.parametrize("small", ["a", "b"])
+@pytest.mark.parametrize("power,other", [(-127, 100), (-130, 20), (-134, 100), (-138, 118), (-142, 24), (-146, 60)])
+def test_f32_gemm_on_the_tensor_core_of_subnormal_operands(power, other, small, M, N, K, a_mn, b_mn, aligned):
+    """An operand of subnormal values, the other one small or large, whole (as the second half of the rows or columns beside normal ones in the same
+    tiles), K shared by a cluster, rows on any boundary.  Products of the two halves stand each for itself: a sum in f32 of at most K / 4 + 4 rounded
+    terms of one size has a 2-norm error of about 2^-24 sqrt(K / 4) / 2, 2.1e-7 at K = 192 and 4.2e-7 at K = 768 (FFMA kernels measured 1.3e-7 at
+    K = 192); the tensor core's six products alone gave 4.0e-6 at 2^-134 and 1.7e-3 at 2^-146."""
+    from deers_b200 import gpt
+    g = torch.Generator(device="cuda").manual_seed(power * power)
+    a, b = (torch.randn(s, device="cuda", generator=g) for s in ((M, K), (K, N)))
+    x, y = (a, b.T) if small == "a" else (b.T, a)
+    x[x.shape[0] // 2:] *= 2.0 ** power
+    y *= 2.0 ** other
+    pad = 0 if aligned else 1
+    store = [t.T if mn else t for t, mn in ((a, a_mn), (b.T, b_mn))]
+    held = [torch.empty((t.shape[0], t.shape[1] + pad), device="cuda")[:, pad:].copy_(t) for t in store]
+    got = gpt.gemm_f32(*held, bool(a_mn), bool(b_mn)).double()
+    want = a.double() @ b.double()
+    if small == "b":
+        got, want = got.T, want.T
+    half = x.shape[0] // 2
+    assert ((got[:half] - want[:half]).norm() / want[:half].norm()).item() < 1e-7 * max(1.0, (K / 192) ** 0.5)
+    assert ((got[half:] - want[half:]).norm() / want[half:].norm()).item() < 2.0 ** -25 * (K / 4) ** 0.5
 
 
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38])
