@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ OptT
         const long long base = (long long)(chunk - t.chunk_start[ti]) * OPT_CHUNK;
         const long long n = t.n[ti];
         float* __restrict__ w = t.w[ti];
-        float* __restrict__ g = t.g[ti];
+        float* g = t.g[ti];
         float* __restrict__ m = t.m[ti];
         float* __restrict__ v = t.v[ti];
         if (t.vec_ok && base + OPT_CHUNK <= n) {

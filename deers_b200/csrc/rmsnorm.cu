@@ -41,13 +41,13 @@ __device__ __forceinline__ void put_pair(__half* hi, __half* lo, long long at, c
 }
 
 // BWD = false: y = x * inv, inv_out[row] = inv (PAIR: y leaves as the f16 pair hi, lo, rows dense, instead of out).
-// BWD = true: dx from x, dy and the saved inv; n_out (may be nullptr) receives y again for the weight gradient.
+// BWD = true: dx from x, dy and the saved inv_in; n_out (may be nullptr) receives y again for the weight gradient.
 // NV: 16-byte pieces of a lane.  Of rows of up to 256 the backward requests everything at once, the residual and the norm too: behind the sum
 // they were two more trips to L2 (22 M parameters, 1024 rows of 192, 13 a step: 4 steps and a forward 5057 -> 4996 us; 3 layers,
 // 231 rows 1230 -> 1203).  Longer rows do not have the registers.
 template <bool BWD, bool VEC, bool VEC2 = false, bool PAIR = false, int NV = RN_MAXV>
-__global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const float* dy, const float* add, float* __restrict__ out,
-                                                      float* __restrict__ inv_io, long long rows, int C, float eps,
+__global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const float* dy, const float* add, const float* inv_in, float* __restrict__ out,
+                                                      float* __restrict__ inv_out, long long rows, int C, float eps,
                                                       float inv_n, float* __restrict__ n_out, __half* __restrict__ hi,
                                                       __half* __restrict__ lo) {
     if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room; short rows below)
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
             float4 xv[NV], gv[NV], av[NV];
             constexpr bool EARLY = BWD && NV <= 2;
             float acc = 0.f, early_inv = 0.f;
-            if (EARLY) early_inv = inv_io[row];
+            if (EARLY) early_inv = inv_in[row];
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
                 const int p = lane + 32 * i;
@@ -86,11 +86,11 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
             acc = warp_sum(acc);
             float inv, k = 0.f;
             if (BWD) {
-                inv = EARLY ? early_inv : inv_io[row];
+                inv = EARLY ? early_inv : inv_in[row];
                 k = acc * inv * inv * inv * inv_n;
             } else {
                 inv = 1.0f / sqrtf(acc * inv_n + eps);
-                if (lane == 0) inv_io[row] = inv;
+                if (lane == 0) inv_out[row] = inv;
             }
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
@@ -136,11 +136,11 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
             acc = warp_sum(acc);
             float inv, k = 0.f;
             if (BWD) {
-                inv = inv_io[row];
+                inv = inv_in[row];
                 k = acc * inv * inv * inv * inv_n;
             } else {
                 inv = 1.0f / sqrtf(acc * inv_n + eps);
-                if (lane == 0) inv_io[row] = inv;
+                if (lane == 0) inv_out[row] = inv;
             }
             for (int p0 = lane; p0 < nv; p0 += 32 * U) {        // the row (<= a few KB per lane group) is still in L1 / L2
                 float4 a[U], b[U];
@@ -176,11 +176,11 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
             acc = warp_sum(acc);
             float inv, k = 0.f;
             if (BWD) {
-                inv = inv_io[row];
+                inv = inv_in[row];
                 k = acc * inv * inv * inv * inv_n;
             } else {
                 inv = 1.0f / sqrtf(acc * inv_n + eps);
-                if (lane == 0) inv_io[row] = inv;
+                if (lane == 0) inv_out[row] = inv;
             }
             for (int c = lane; c < C; c += 32) {
                 float o = BWD ? gr[c] * inv - xr[c] * k : xr[c] * inv;
@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const floa
 
 // Rows of 1025 .. 8192 elements: a whole block owns a row, which still stays in registers (one pass over HBM).
 template <bool BWD, bool PAIR = false>
-__global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* x, const float* dy, const float* add, float* __restrict__ out,
-                                                            float* __restrict__ inv_io, long long rows, int C, float eps,
+__global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* x, const float* dy, const float* add, const float* inv_in, float* __restrict__ out,
+                                                            float* __restrict__ inv_out, long long rows, int C, float eps,
                                                             float inv_n, float* __restrict__ n_out, __half* __restrict__ hi,
                                                             __half* __restrict__ lo) {
     if (!BWD) chain_next();                                     // (backward: weight gradients run beside it, leave them the room)
@@ -229,11 +229,11 @@ __global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* x, cons
         for (int w = 0; w < 8; ++w) tot += part[w];
         float inv, k = 0.f;
         if (BWD) {
-            inv = inv_io[row];
+            inv = inv_in[row];
             k = tot * inv * inv * inv * inv_n;
         } else {
             inv = 1.0f / sqrtf(tot * inv_n + eps);
-            if (threadIdx.x == 0) inv_io[row] = inv;
+            if (threadIdx.x == 0) inv_out[row] = inv;
         }
         float4* o4 = reinterpret_cast<float4*>(out + row * C);
 #pragma unroll
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(256) rmsnorm_block_kernel(const float* x, cons
 }
 
 template <bool BWD>
-int rms_launch(deers_ctx* ctx, long long rows, int C, float eps, const float* x, const float* dy, float* out, float* inv,
+int rms_launch(deers_ctx* ctx, long long rows, int C, float eps, const float* x, const float* dy, const float* inv_in, float* out, float* inv_out,
                const float* add = nullptr, float* n_out = nullptr) {
     if (rows == 0) return DEERS_OK;
     uintptr_t bits = (uintptr_t)x | (uintptr_t)out | (BWD ? (uintptr_t)dy : 0) | (uintptr_t)add | (uintptr_t)n_out;
@@ -273,13 +273,13 @@ int rms_launch(deers_ctx* ctx, long long rows, int C, float eps, const float* x,
     {
         KernelTimerScope ts(ctx, DEERS_K_NORM);
         if (BWD && vec && C <= 256)
-            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true, false, false, 2>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
-        else if (vec) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true, false, false, 2>, grid, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
+        else if (vec) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true>, grid, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
         else if (aligned && C <= 256 * RN_MAXV * 4) {
             const unsigned bgrid = (unsigned)(rows < cap ? rows : cap);
-            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_block_kernel<BWD>, bgrid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
-        } else if (aligned) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false, true>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
-        else DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false>, grid, 256, 0, 1, x, dy, add, out, inv, rows, C, eps, inv_n, n_out, nullptr, nullptr));
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_block_kernel<BWD>, bgrid, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
+        } else if (aligned) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false, true>, grid, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
+        else DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false>, grid, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
     }
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
@@ -300,16 +300,16 @@ extern "C" int deers_b200_rmsnorm_fwd(deers_ctx* ctx, int64_t rows, int32_t C, d
     int rc = rms_check(ctx, rows, C, x, y, inv_norm, x);
     if (rc) return rc;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    return rms_launch<false>(ctx, rows, C, (float)eps, x, nullptr, y, inv_norm);
+    return rms_launch<false>(ctx, rows, C, (float)eps, x, nullptr, nullptr, y, inv_norm);
 }
 
 // Internal launchers for the model step (gpt_model.cu).
 int launch_rmsnorm_fwd(deers_ctx* ctx, long long rows, int C, double eps, const float* x, float* y, float* inv_norm) {
-    return rms_launch<false>(ctx, rows, C, (float)eps, x, nullptr, y, inv_norm);
+    return rms_launch<false>(ctx, rows, C, (float)eps, x, nullptr, nullptr, y, inv_norm);
 }
 int launch_rmsnorm_bwd(deers_ctx* ctx, long long rows, int C, const float* x, const float* inv_norm, const float* dy,
                        const float* add, float* dx, float* n_out) {
-    return rms_launch<true>(ctx, rows, C, 0.f, x, dy, dx, const_cast<float*>(inv_norm), add, n_out);
+    return rms_launch<true>(ctx, rows, C, 0.f, x, dy, inv_norm, dx, nullptr, add, n_out);
 }
 // y as an f16 pair, one pass where the row stays in registers.  DEERS_ERR_UNSUPPORTED otherwise: the caller normalises and
 // splits in two.
@@ -321,10 +321,10 @@ int launch_rmsnorm_split(deers_ctx* ctx, long long rows, int C, double eps, cons
     {
         KernelTimerScope ts(ctx, DEERS_K_NORM);
         if (C <= 32 * RN_MAXV * 4)
-            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<false, true, false, true>, grid, 256, 0, 1, x, nullptr, nullptr, nullptr, inv_norm,
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<false, true, false, true>, grid, 256, 0, 1, x, nullptr, nullptr, nullptr, nullptr, inv_norm,
                                                rows, C, (float)eps, inv_n, nullptr, (__half*)hi, (__half*)lo));
         else
-            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_block_kernel<false, true>, grid, 256, 0, 1, x, nullptr, nullptr, nullptr, inv_norm, rows, C,
+            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_block_kernel<false, true>, grid, 256, 0, 1, x, nullptr, nullptr, nullptr, nullptr, inv_norm, rows, C,
                                                (float)eps, inv_n, nullptr, (__half*)hi, (__half*)lo));
     }
     ctx->launches += 1;
@@ -339,7 +339,7 @@ extern "C" int deers_b200_rmsnorm_bwd_add(deers_ctx* ctx, int64_t rows, int32_t 
     if (!residual_grad) return DEERS_ERR_NULL;
     if ((uintptr_t)residual_grad & 3u) return DEERS_ERR_LAYOUT;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    return rms_launch<true>(ctx, rows, C, 0.f, x, dy, dx, const_cast<float*>(inv_norm), residual_grad);
+    return rms_launch<true>(ctx, rows, C, 0.f, x, dy, inv_norm, dx, nullptr, residual_grad);
 }
 
 extern "C" int deers_b200_rmsnorm_bwd(deers_ctx* ctx, int64_t rows, int32_t C, const float* x, const float* inv_norm,
@@ -347,5 +347,5 @@ extern "C" int deers_b200_rmsnorm_bwd(deers_ctx* ctx, int64_t rows, int32_t C, c
     int rc = rms_check(ctx, rows, C, x, inv_norm, dy, dx);
     if (rc) return rc;
     DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    return rms_launch<true>(ctx, rows, C, 0.f, x, dy, dx, const_cast<float*>(inv_norm));
+    return rms_launch<true>(ctx, rows, C, 0.f, x, dy, inv_norm, dx, nullptr);
 }

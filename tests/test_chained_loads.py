@@ -173,3 +173,82 @@ def test_kernels_that_work_in_place_promise_nothing_of_their_buffers(kernel):
     """Source and destination may be one buffer, which a restrict pointer to either would deny."""
     (found,) = [params + body[:body.index("__global__") if "__global__" in body else None] for f, name, params, body in CHAINED if name == kernel]
     assert re.search("p.dst|dlogits", found) and "__restrict__" not in found
+
+
+def body_of(text, name):
+    """The whole body of a kernel."""
+    m = re.search(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?" + name + r"\s*\(", text)
+    i = text.index("{", m.end())
+    start, depth = i + 1, 1
+    while depth:
+        i += 1
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+    return text[start:i]
+
+
+def closing(text, i):
+    """Place of the bracket that closes the one at i."""
+    depth, pair = 0, {"(": ")", "[": "]"}[text[i]]
+    while True:
+        depth += {text[i]: 0, "(": 1, "[": 1, ")": -1, "]": -1}.get(text[i], 0)
+        if text[i] == pair and depth == 0:
+            return i
+        i += 1
+
+
+def read_through(files, file, body, names):
+    """Those of the pointers `names`, and of the pointers made from them, that a body dereferences other than as the target of an assignment, or
+    hands to a function of the file that does."""
+    out, todo, seen = [], list(names), set()
+    while todo:
+        p = todo.pop()
+        if p in seen:
+            continue
+        seen.add(p)
+        todo += re.findall(r"\*\s*(?:__restrict__\s+)?(\w+)\s*=[^;=]*\b" + p + r"\b", body)
+        for m in re.finditer(r"\b" + p + r"\b", body):
+            end, star = m.end(), re.search(r"(?:[;{}=(,]|\breturn)\s*\*\s*$", body[:m.start()])
+            outer = [c for c in re.finditer(r"(\w+)(<[\w ]+\*>)?\(", body[:m.start()]) if closing(body, c.end() - 1) > m.start()]
+            if not star and outer and outer[-1].group(1) == "reinterpret_cast":
+                end = closing(body, outer[-1].end() - 1) + 1
+                star = re.search(r"(?:[;{}=(,]|\breturn)\s*\*\s*$", body[:outer[-1].start()])
+            elif outer:
+                place = body[outer[-1].end():m.start()].count(",")
+                for params, inner in definitions(files[file]).get(outer[-1].group(1), []):
+                    if read_through(files, file, inner, [re.findall(r"(\w+)\s*(?:,|$)", params)[place]]):
+                        out.append(p)
+            after = body[end:].lstrip()
+            if after.startswith("["):
+                after = after[closing(after, 0) + 1:].lstrip()
+            elif not star:
+                continue
+            if not re.match(r"=[^=]", after):
+                out.append(p)
+    return out
+
+
+@pytest.mark.parametrize("file,name,params", [c[:3] for c in CHAINED if "__restrict__" in c[2]], ids=[f"{f}:{n}" for f, n, p, _ in CHAINED if "__restrict__" in p])
+def test_restrict_pointers_of_chained_kernels_are_only_written(file, name, params):
+    """The promise that nothing else reaches what a pointer points to lets a load through it run ahead of the wait, const or not."""
+    names = re.findall(r"\*\s*__restrict__\s+(\w+)", params)
+    assert read_through(FILES, file, body_of(FILES[file], name), names) == []
+
+
+@pytest.mark.parametrize("file,kernel,before,planted", [
+    ("rmsnorm.cu", "rmsnorm_kernel", "            acc = warp_sum(acc);\n", "            inv = inv_out[row];\n"),
+    ("rmsnorm.cu", "rmsnorm_block_kernel", "        acc = warp_sum(acc);\n", "        acc += reinterpret_cast<const float4*>(out + row * C)[0].x;\n"),
+    ("rmsnorm.cu", "rmsnorm_kernel", "    const float x[4] = {v.x, v.y, v.z, v.w};\n", "    const float y = __half2float(hi[at]);\n"),
+    ("gpt_ops.cu", "cross_entropy_merge_kernel", "    lse[row] = l;\n", "    picked[row] = lse[row];\n"),
+    ("gemm_f16x3_sm100.cu", "x3_split_kernel", "        __half* dh = hi + r * ld_dst + c0;\n", "        if (dh[0] == h[0]) continue;\n")])
+def test_a_read_through_a_restrict_pointer_is_seen(file, kernel, before, planted):
+    assert before in FILES[file]
+    files = dict(FILES, **{file: FILES[file].replace(before, before + planted)})
+    (params,) = [params for f, name, params, _ in CHAINED if name == kernel]
+    assert read_through(files, file, body_of(files[file], kernel), re.findall(r"\*\s*__restrict__\s+(\w+)", params))
+
+
+def test_no_restrict_locals_that_are_only_read():
+    for file, text in FILES.items():
+        for m in re.finditer(r"\*\s*__restrict__\s+(\w+)\s*=", text):
+            rest = text[m.end():m.end() + 4000]
+            assert re.search(r"(?:\*reinterpret_cast<\w+\*>\(" + m.group(1) + r"\b[^;]*\)|\b" + m.group(1) + r"\[[^\]]*\])\s*=[^=]", rest), (file, m.group(1))
