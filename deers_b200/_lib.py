@@ -33,11 +33,12 @@ SYMBOLS = [
     "deers_b200_gpt_forward_backward", "deers_b200_gpt_train_step", "deers_b200_gpt_train_step_host",
     "deers_b200_shard_range", "deers_b200_comm_init_all", "deers_b200_comm_export", "deers_b200_comm_init_ipc",
     "deers_b200_comm_destroy", "deers_b200_comm_set_lanes", "deers_b200_allgather_o", "deers_b200_allgather_join", "deers_b200_allgather_flush",
-    "deers_b200_selftest_wait", "deers_b200_split_f16x3", "deers_b200_gemm_f16x3_workspace_bytes", "deers_b200_gemm_f16x3",
+    "deers_b200_selftest_wait", "deers_b200_product_route", "deers_b200_split_f16x3", "deers_b200_gemm_f16x3_workspace_bytes", "deers_b200_gemm_f16x3",
 ]
 IPC_HANDLE_BYTES = 72
 K_FWD, K_BWD_PREP, K_BWD_MAIN, K_BWD_DQ, K_ROPE, K_OPTIM, K_NORM, K_DECODE, K_GEMM, K_GPT, K_GEMM_X3 = range(11)
 EPI_NONE, EPI_ADD, EPI_RELU_SQ, EPI_MUL_AUX2 = range(4)
+PRODUCT_F16, PRODUCT_F32, PRODUCT_F32_NORM, PRODUCT_F16X3 = range(4)
 
 
 class AttnDesc(ctypes.Structure):
@@ -75,6 +76,10 @@ class DecodeDesc(ctypes.Structure):
 class GemmEpilogue(ctypes.Structure):
     _fields_ = [("kind", ctypes.c_int32), ("residual", ctypes.c_void_p), ("ld_residual", ctypes.c_int64),
                 ("aux", ctypes.c_void_p)]
+
+
+class ProductRoute(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int32) for n in ("tile_m", "tile_n", "parts", "tensor_core", "pair", "resident", "rotated")]
 
 
 class GptConfig(ctypes.Structure):
@@ -184,6 +189,8 @@ def lib() -> ctypes.CDLL:
     L.deers_b200_launch_count.restype = ctypes.c_uint64
     L.deers_b200_selftest_umma.argtypes = [vp, ctypes.POINTER(ctypes.c_float)]
     L.deers_b200_selftest_wait.argtypes = [vp, ctypes.c_uint32, ctypes.POINTER(ctypes.c_int32)]
+    p32 = ctypes.POINTER(ctypes.c_int32)
+    L.deers_b200_product_route.argtypes = [vp, i32, i32, p32, p32, i32, i32, i32, i32, i32, ctypes.POINTER(ProductRoute)]
     L.deers_b200_kernel_timing.argtypes = [vp, i32]
     L.deers_b200_kernel_time.argtypes = [vp, i32, i32, ctypes.POINTER(ctypes.c_double),
                                          ctypes.POINTER(ctypes.c_uint64)]

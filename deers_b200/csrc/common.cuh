@@ -259,6 +259,8 @@ int launch_gemm_f16x3(deers_ctx* ctx, int M, int N, int K, const void* a_hi, con
 // (stats, stat_parts: with A in K and B in MN order the product may leave, per row and 32 columns, (maximum, sum of exponentials relative to
 // it), [stat_parts][M]; 0 parts: it did not.  Room for 4 * ceil(N / 128) parts.)
 int gemm_f16_pairs(deers_ctx* ctx, int* pairs);
+int route_gemm_f16(deers_ctx* ctx, int M, int N, int K, deers_product_route* r);
+int route_gemm_f16x3(deers_ctx* ctx, int M, int N, int K, int a_mn, int b_mn, int rows16, deers_product_route* r);
 int launch_cross_entropy_bwd_split(deers_ctx* ctx, const float* logits, long long ld, const long long* targets,
                                    const float* lse, long long rows, long long V, float upstream, float scale, void* hi,
                                    void* lo, long long ldd);

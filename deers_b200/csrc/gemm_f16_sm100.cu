@@ -171,7 +171,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         // The whole warp runs this; one elected lane issues (see elect_one).
         if (half == 0) {
             constexpr uint32_t IDESC = idesc_f16(TM, GN, A_MN, B_MN);
-                        const auto commit = [&](uint64_t* bar) {
+            const auto commit = [&](uint64_t* bar) {
                 if constexpr (PAIR) umma_commit_pair(bar, 3u);
                 else umma_commit(bar);
             };
@@ -430,6 +430,14 @@ int gemm_f16_pairs(deers_ctx* ctx, int* pairs) {
     const int rc = cluster_room(ctx);
     *pairs = rc ? 0 : ctx->cluster_room_f16[2];
     return rc;
+}
+
+int route_gemm_f16(deers_ctx* ctx, int M, int N, int K, deers_product_route* r) {
+    const int rc = cluster_room(ctx);
+    if (rc) return rc;
+    const GemmPlan p = plan_gemm_f16(ctx, M, N, K);
+    r->tile_m = p.pair ? 2 * GM : GM; r->tile_n = p.gn; r->parts = p.parts; r->tensor_core = 1; r->pair = p.pair;
+    return DEERS_OK;
 }
 
 extern "C" int deers_b200_gemm_f16(deers_ctx* ctx, int32_t M, int32_t N, int32_t K, const void* a, int64_t lda, int32_t a_mn_major,

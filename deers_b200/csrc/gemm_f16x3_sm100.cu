@@ -726,6 +726,17 @@ X3Plan x3_plan(int M, int N, int K, int a_mn, int b_mn, int sm_count, int pairs)
     return pl;
 }
 
+size_t x3_partials(const X3Plan& pl, int M, int N) { return pl.parts > 1 ? (size_t)pl.parts * M * N * sizeof(float) : 0; }
+
+// The plan of a call.  Input gradients by pairs store 16 bytes at a time; and the workspace may be one for single CTAs.
+int x3_choose(deers_ctx* ctx, int M, int N, int K, int a_mn, int b_mn, bool rows16, size_t ws_bytes, int* pairs, X3Plan* pl) {
+    const int rc = gemm_f16_pairs(ctx, pairs);
+    if (rc) return rc;
+    *pl = x3_plan(M, N, K, a_mn, b_mn, ctx->sm_count, *pairs);
+    if (pl->pair && ((!a_mn && !b_mn && !rows16 && pl->parts == 1) || ws_bytes < x3_partials(*pl, M, N))) *pl = x3_plan(M, N, K, a_mn, b_mn, ctx->sm_count, 0);
+    return DEERS_OK;
+}
+
 template <int A_MN, int B_MN>
 int x3_launch(deers_ctx* ctx, const CUtensorMap* t, const X3Params& p, unsigned grid) {
     DEERS_SMEM_ONCE(ctx, (gemm_f16x3_kernel<A_MN, B_MN>), X_SMEM);
@@ -774,10 +785,19 @@ size_t gemm_f16x3_workspace_bytes(const deers_ctx* ctx, int M, int N, int K) {
     for (int pairs : {0, sms / 2})                                      // whichever of the two the product takes
         for (int b_mn = 0; b_mn <= 1; ++b_mn) {
             const X3Plan pl = x3_plan(M, N, K, 0, b_mn, sms, pairs);
-            const size_t need = pl.parts > 1 ? (size_t)pl.parts * M * N * sizeof(float) : 0;
-            if (need > most) most = need;
+            if (x3_partials(pl, M, N) > most) most = x3_partials(pl, M, N);
         }
     return most;
+}
+
+int route_gemm_f16x3(deers_ctx* ctx, int M, int N, int K, int a_mn, int b_mn, int rows16, deers_product_route* r) {
+    X3Plan pl;
+    int pairs = 0;
+    const int rc = x3_choose(ctx, M, N, K, a_mn, b_mn, rows16 != 0, gemm_f16x3_workspace_bytes(ctx, M, N, K), &pairs, &pl);
+    if (rc) return rc;
+    r->tile_m = !pl.pair ? XM : pl.trans ? pl.tn : P_M; r->tile_n = !pl.pair ? XN : pl.trans ? P_M : pl.tn;
+    r->parts = pl.parts; r->tensor_core = 1; r->pair = pl.pair; r->resident = pl.resident;
+    return DEERS_OK;
 }
 
 int launch_split_f16x3(deers_ctx* ctx, long long rows, int cols, const float* src, long long ld_src, float scale,
@@ -803,15 +823,12 @@ int launch_gemm_f16x3(deers_ctx* ctx, int M, int N, int K, const void* a_hi, con
     if (stat_parts) *stat_parts = 0;
     if (M == 0 || N == 0) return DEERS_OK;
     CUtensorMap t[4];
-    int rc, pairs = 0;
-    if ((rc = gemm_f16_pairs(ctx, &pairs))) return rc;
-    X3Plan pl = x3_plan(M, N, K, a_mn, b_mn, ctx->sm_count, pairs);
-    auto need = [&]() { return pl.parts > 1 ? (size_t)pl.parts * M * N * sizeof(float) : 0; };
-    // (input gradients by pairs store 16 bytes at a time; and the workspace may be one for single CTAs)
+    X3Plan pl;
     const bool rows16 = ldc % 4 == 0 && ((uintptr_t)c & 15u) == 0;
-    if (pl.pair && ((!a_mn && !b_mn && !rows16 && pl.parts == 1) || ws_bytes < need() || (need() && !workspace))) pl = x3_plan(M, N, K, a_mn, b_mn, ctx->sm_count, 0);
+    int pairs = 0, rc = x3_choose(ctx, M, N, K, a_mn, b_mn, rows16, workspace ? ws_bytes : 0, &pairs, &pl);
+    if (rc) return rc;
     const bool split = pl.parts > 1;
-    if (split && (!workspace || ws_bytes < need() || ((uintptr_t)workspace & 15u))) return DEERS_ERR_WORKSPACE;
+    if (split && (!workspace || ws_bytes < x3_partials(pl, M, N) || ((uintptr_t)workspace & 15u))) return DEERS_ERR_WORKSPACE;
     float* out = split ? (float*)workspace : c;
     const long long ldo = split ? N : ldc;
     const int vec = ldo % 4 == 0 && ((uintptr_t)out & 15u) == 0;

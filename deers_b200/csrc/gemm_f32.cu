@@ -174,6 +174,23 @@ int launch_planned(deers_ctx* ctx, const GemmPlan& p, GemmArgs& g, int a_mn, int
     return rc;
 }
 
+GemmPlan plan_single(deers_ctx* ctx, int M, int N, int K, bool aligned) { return plan_gemm(1, &M, &N, K, aligned ? 1.0 : TC_LOOSE, ctx->cluster_capacity, 0); }
+
+// The plan of a product of normalised rows, and whether its tiles rotate heads of `heads` columns (0: there are none).
+GemmPlan plan_norm(deers_ctx* ctx, int M, int N, int K, bool aligned, int heads, bool* rotated) {
+    // (the choice below between rotating in a tile and beside it was measured for the tensor core's tiles up to 384 columns only)
+    const double tc = aligned && K <= 384 ? 1.0 : 0.0;
+    const GemmPlan p = plan_gemm(1, &M, &N, K, tc, ctx->cluster_capacity, 0);
+    *rotated = false;
+    if (heads == 0 || heads % 8) return p;
+    // A rotary launch of its own takes up to 4400 of these cycles (1.4 to 2 us): rotate here unless tiles that hold whole heads cost more
+    // than that (heads of 48 columns leave 32 x 96 and 64 x 96 tiles: 231 x 576 x 192 takes 7.5 us in them, 3.6 in 32 x 32).
+    // Several waves of clusters do not count: the estimate takes them to follow one another without a gap (forwards of 4 layers,
+    // rotating in them and beside: C 512, 256 tokens 363 and 335 us, C 384, 640 tokens 533 and 501).
+    const GemmPlan w = plan_gemm(1, &M, &N, K, tc, ctx->cluster_capacity, heads);
+    *rotated = w.cfg >= 0 && w.cost < p.cost + 4400.0 && (w.cost == p.cost || w.parts == 1 || w.waves == 1);
+    return *rotated ? w : p;
+}
 }  // namespace
 
 int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long long lda, int a_mn, const float* b,
@@ -192,7 +209,7 @@ int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long lo
     const int rc = cluster_capacity(ctx);
     if (rc) return rc;
     GemmArgs g = gemm_args(M, N, K, a, lda, b, ldb, c, ldc, epi, r, ldr, aux);
-    const GemmPlan p = plan_gemm(1, &M, &N, K, g.a_vec && g.b_vec ? 1.0 : TC_LOOSE, ctx->cluster_capacity, 0);
+    const GemmPlan p = plan_single(ctx, M, N, K, g.a_vec && g.b_vec);
     return launch_planned(ctx, p, g, a_mn, b_mn, false);
 }
 
@@ -204,27 +221,17 @@ int launch_gemm_f32_norm(deers_ctx* ctx, int M, int N, int K, const float* a, co
     const int rc = cluster_capacity(ctx);
     if (rc) return rc;
     GemmArgs g = gemm_args(M, N, K, a, K, b, N, c, N, epi, nullptr, 0, aux);
-    // (the choice below between rotating in a tile and beside it was measured for the tensor core's tiles up to 384 columns only)
-    const double tc = g.a_vec && g.b_vec && K <= 384 ? 1.0 : 0.0;
-    GemmPlan p = plan_gemm(1, &M, &N, K, tc, ctx->cluster_capacity, 0);
-    if (f.rope_cols && f.rope_d % 8 == 0) {
-        // A rotary launch of its own takes up to 4400 of these cycles (1.4 to 2 us): rotate here unless tiles that hold whole heads cost more
-        // than that (heads of 48 columns leave 32 x 96 and 64 x 96 tiles: 231 x 576 x 192 takes 7.5 us in them, 3.6 in 32 x 32).
-        // Several waves of clusters do not count: the estimate takes them to follow one another without a gap (forwards of 4 layers,
-        // rotating in them and beside: C 512, 256 tokens 363 and 335 us, C 384, 640 tokens 533 and 501).
-        const GemmPlan w = plan_gemm(1, &M, &N, K, tc, ctx->cluster_capacity, f.rope_d);
-        if (w.cfg >= 0 && w.cost < p.cost + 4400.0 && (w.cost == p.cost || w.parts == 1 || w.waves == 1)) {
-            p = w;
-            *rotated = true;
-            g.cosv = f.cosv; g.sinv = f.sinv; g.rope_cols = f.rope_cols; g.rope_d = f.rope_d; g.rope_t = f.rope_t;
-        }
-    }
+    const GemmPlan p = plan_norm(ctx, M, N, K, g.a_vec && g.b_vec, f.rope_cols ? f.rope_d : 0, rotated);
+    if (*rotated) { g.cosv = f.cosv; g.sinv = f.sinv; g.rope_cols = f.rope_cols; g.rope_d = f.rope_d; g.rope_t = f.rope_t; }
     g.eps = f.eps; g.inv_n = (float)(1.0 / (double)K); g.inv = f.inv;
     return launch_planned(ctx, p, g, 0, 1, true);
 }
 
 namespace {
-// The plan of a group of products with dense operands (rows of M_i and N_i).
+GemmPlan plan_group(deers_ctx* ctx, int n, const int* M, const int* N, int K, bool aligned) {
+    return plan_gemm(n, M, N, K, aligned ? 1.0 : 0.0, ctx->cluster_capacity, 0);
+}
+// The same of products with dense operands (rows of M_i and N_i).
 GemmPlan plan_group(deers_ctx* ctx, int n, const GemmTN* t, int K) {
     int M[GEMM_GROUP_MAX], N[GEMM_GROUP_MAX];
     bool aligned = true;
@@ -232,7 +239,7 @@ GemmPlan plan_group(deers_ctx* ctx, int n, const GemmTN* t, int K) {
         M[i] = t[i].M; N[i] = t[i].N;
         aligned = aligned && M[i] % 4 == 0 && N[i] % 4 == 0 && (((uintptr_t)t[i].a | (uintptr_t)t[i].b) & 15u) == 0;
     }
-    return plan_gemm(n, M, N, K, aligned ? 1.0 : 0.0, ctx->cluster_capacity, 0);
+    return plan_group(ctx, n, M, N, K, aligned);
 }
 }  // namespace
 
@@ -269,6 +276,28 @@ int launch_gemm_f32_group(deers_ctx* ctx, int n, const GemmTN* t, int K) {
     }
     ctx->launches += 1;
     return res;
+}
+
+extern "C" int deers_b200_product_route(deers_ctx* ctx, int32_t which, int32_t n, const int32_t* M, const int32_t* N, int32_t K, int32_t a_mn_major,
+                                        int32_t b_mn_major, int32_t aligned, int32_t heads, deers_product_route* route) {
+    if (!ctx || !M || !N || !route) return DEERS_ERR_NULL;
+    if (n < 1 || n > (which == DEERS_PRODUCT_F32 && a_mn_major && b_mn_major ? GEMM_GROUP_MAX : 1) || K < 1 || heads < 0) return DEERS_ERR_SHAPE;
+    for (int i = 0; i < n; ++i)
+        if (M[i] < 1 || N[i] < 1) return DEERS_ERR_SHAPE;
+    DEERS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
+    deers_product_route r{};
+    int rc = DEERS_OK;
+    if (which == DEERS_PRODUCT_F16) rc = route_gemm_f16(ctx, M[0], N[0], K, &r);
+    else if (which == DEERS_PRODUCT_F16X3) rc = route_gemm_f16x3(ctx, M[0], N[0], K, a_mn_major != 0, b_mn_major != 0, aligned, &r);
+    else if (which != DEERS_PRODUCT_F32 && which != DEERS_PRODUCT_F32_NORM) return DEERS_ERR_UNSUPPORTED;
+    else if (!(rc = cluster_capacity(ctx))) {
+        bool rotated = false;
+        const GemmPlan p = which == DEERS_PRODUCT_F32_NORM ? plan_norm(ctx, M[0], N[0], K, aligned != 0, heads, &rotated)
+                         : n > 1 ? plan_group(ctx, n, M, N, K, aligned != 0) : plan_single(ctx, M[0], N[0], K, aligned != 0);
+        r.tile_m = kVariants[p.cfg].bm; r.tile_n = kVariants[p.cfg].bn; r.parts = p.parts; r.tensor_core = p.cfg == TC_CFG; r.rotated = rotated;
+    }
+    if (!rc) *route = r;
+    return rc;
 }
 
 extern "C" size_t deers_b200_gemm_f32_workspace_bytes(deers_ctx* ctx, int32_t M, int32_t N, int32_t K) {

@@ -107,6 +107,13 @@ class Context:
         _lib.check(_lib.lib().deers_b200_selftest_wait(self.handle, limit_ms, res), self.handle)
         return [int(v) for v in res]
 
+    def product_route(self, which: int, sizes, K: int, a_mn: bool = False, b_mn: bool = True, aligned: bool = True, heads: int = 0) -> "_lib.ProductRoute":
+        """How products of the given sizes [(M, N), ...] would run (deers_b200_product_route); which: _lib.PRODUCT_*."""
+        route, ints = _lib.ProductRoute(), ctypes.c_int32 * len(sizes)
+        _lib.check(_lib.lib().deers_b200_product_route(self.handle, which, len(sizes), ints(*(m for m, _ in sizes)), ints(*(n for _, n in sizes)), K,
+                                                       int(a_mn), int(b_mn), int(aligned), heads, ctypes.byref(route)), self.handle)
+        return route
+
     def selftest_umma(self) -> List[float]:
         errs = (ctypes.c_float * 6)()
         _lib.check(_lib.lib().deers_b200_selftest_umma(self.handle, errs), self.handle)

@@ -574,6 +574,28 @@ enum { DEERS_SELFTEST_CASES = 6 };
 int deers_b200_selftest_umma(deers_ctx* ctx, float* max_abs_err);
 
 /*
+ * How a matrix product of these sizes would run on this context's device (nothing is launched): what a test of one route asks before it
+ * takes a result for that route's.  n products of one K (one, but for F32 products that the model launches together: up to four, a_mn =
+ * b_mn = 1).
+ *     DEERS_PRODUCT_F16        deers_b200_gemm_f16
+ *     DEERS_PRODUCT_F32        deers_b200_gemm_f32;  aligned: rows of A and B start on 16-byte boundaries
+ *     DEERS_PRODUCT_F32_NORM   the model's products of normalised rows;  heads: columns of the heads that are rotated, 0 if none are
+ *     DEERS_PRODUCT_F16X3      deers_b200_gemm_f16x3 with the workspace it asks for;  aligned: rows of C do
+ * No counterpart in the reference.
+ */
+enum { DEERS_PRODUCT_F16 = 0, DEERS_PRODUCT_F32 = 1, DEERS_PRODUCT_F32_NORM = 2, DEERS_PRODUCT_F16X3 = 3 };
+typedef struct deers_product_route {
+    int32_t tile_m, tile_n;   /* output tile of a block, or of a pair of blocks */
+    int32_t parts;            /* blocks (or passes) that share a tile's K */
+    int32_t tensor_core;      /* 0: FFMA */
+    int32_t pair;             /* two blocks work on one tile */
+    int32_t resident;         /* F16X3: K blocks of A that stay in shared memory */
+    int32_t rotated;          /* F32_NORM: the heads are rotated in the product's own tiles */
+} deers_product_route;
+int deers_b200_product_route(deers_ctx* ctx, int32_t which, int32_t n, const int32_t* M, const int32_t* N, int32_t K, int32_t a_mn_major,
+                             int32_t b_mn_major, int32_t aligned, int32_t heads, deers_product_route* route);
+
+/*
  * Bounded-wait self-test: runs the give-up path of the device-side waits without a fault or a hang.  One small
  * kernel waits, through the same helper every kernel of the library uses, on a barrier that nothing completes,
  * with a limit of `limit_ms` (1..1000) milliseconds instead of the usual two seconds.  result (4 ints, host):

@@ -72,6 +72,7 @@ def test_null_arguments_are_rejected_not_crashed():
     assert L.deers_b200_sync(None) == _lib.ERR_NULL
     assert L.deers_b200_attn_fwd(None, None, None, None, None, None, None, None, 0) == _lib.ERR_NULL
     assert L.deers_b200_launch_count(None) == 0
+    assert L.deers_b200_product_route(None, 0, 1, None, None, 1, 0, 0, 1, 0, None) == _lib.ERR_NULL
     L.deers_b200_destroy(None)
 
 

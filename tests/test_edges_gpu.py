@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+from deers_b200 import _lib
 from tests.helpers import TOL_F16, assert_close
 
 pytestmark = pytest.mark.gpu
@@ -708,19 +709,25 @@ def test_gpt_weight_gradients_in_one_launch_or_apart(H, D, Hm, B, T, launches):
         assert np.array_equal(g, m.grad(i)), m.parameter_info(i)
 
 
-@pytest.mark.parametrize("H,D,B,T,inside", [
-    # the projection's tile and the blocks of a cluster along K
-    (6, 32, 1, 100, True), (20, 16, 1, 64, True),                 # 32 x 32; in clusters
-    (16, 16, 3, 100, True), (4, 64, 1, 4, True), (6, 64, 1, 3, True),     # 32 x 64; in clusters of 2, of 3
-    (2, 64, 4, 250, True), (5, 64, 2, 66, True),                  # 64 x 64; in clusters
-    (5, 32, 2, 320, True), (5, 48, 1, 196, True),                 # 32 x 96; in clusters
-    (12, 32, 1, 700, True), (13, 48, 1, 33, True),                # 64 x 96; in clusters
-    (5, 64, 1, 932, True), (6, 64, 1, 281, True),                 # 64 x 128; in clusters
+@pytest.mark.parametrize("H,D,B,T,tile", [
+    # the projection's tile and whether blocks of a cluster share its K
+    (6, 32, 1, 100, (16, 32, 0)), (20, 16, 1, 64, (16, 32, 0)), (21, 16, 1, 2, (16, 32, 1)),
+    (1, 16, 5, 239, (32, 32, 0)), (15, 32, 1, 19, (32, 32, 1)),
+    (2, 64, 1, 4, (32, 64, 0)), (16, 16, 3, 100, (32, 64, 0)), (4, 64, 1, 4, (32, 64, 1)), (6, 64, 1, 3, (32, 64, 1)),
+    (2, 64, 4, 250, (64, 64, 0)), (5, 64, 2, 66, (64, 64, 1)),
+    (1, 48, 1, 4, (32, 96, 0)), (5, 48, 1, 196, (32, 96, 1)),
+    (5, 24, 5, 239, (64, 96, 0)), (13, 48, 1, 33, (64, 96, 1)),
+    (4, 128, 1, 584, (64, 128, 0)), (17, 32, 1, 175, (64, 128, 1)),
+    (12, 32, 1, 700, (128, 64, 0)), (5, 64, 1, 932, (128, 64, 0)),            # the tensor core's
+    (20, 16, 3, 100, (128, 64, 1)), (5, 32, 2, 320, (128, 64, 1)), (6, 64, 1, 281, (128, 64, 1)),
     # no tile holds the heads, or such tiles cost more than a launch, or they would be several waves of clusters
-    (3, 80, 1, 40, False), (3, 10, 2, 25, False), (4, 48, 1, 231, False), (2, 96, 1, 100, False), (8, 64, 1, 256, False)])
-def test_gpt_rotation_inside_the_projection(H, D, B, T, inside):
+    (3, 80, 1, 40, None), (3, 10, 2, 25, None), (4, 48, 1, 231, None), (2, 96, 1, 100, None), (8, 64, 1, 256, None)])
+def test_gpt_rotation_inside_the_projection(H, D, B, T, tile):
     """Norm and rotation in each tile of the projection, whole K and K split over a cluster (the other half of a head and the rows'
     squares then lie in several blocks)."""
+    inside = tile is not None
+    r = _route(_lib.PRODUCT_F32_NORM, B * T, 3 * H * D, H * D, aligned=H * D % 4 == 0, heads=D)
+    assert r.rotated == inside and (not inside or (r.tile_m, r.tile_n, r.parts > 1) == tile)
     m, ids, tgt, logits, loss, n, want = _gpt_and_oracle(64, 1, H, D, 64, B, T)
     _check_gpt(m, logits, loss, want)
     # embedding; projection, attention, output, up, down (and the rotation); norm, head, copy of its padded rows
@@ -777,13 +784,21 @@ def test_embedding_backward_of_repeated_ids(n, V, C):
     assert np.array_equal(got.cpu().numpy(), ref.embedding_bwd(d, ids, V))
 
 
-@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (264, 264, 328), (520, 192, 1032), (512, 520, 8192), (640, 1544, 4104), (1280, 768, 8192), (2056, 2304, 776),
-                                   (4104, 1288, 200), (8192, 96, 72), (9472, 768, 64), (304, 3000, 16392), (4104, 2056, 72),
-                                   (2184, 4488, 1032), (9480, 4864, 264)])
+def _route(which, M, N, K, a_mn=False, b_mn=True, aligned=True, heads=0):
+    """How a product would run: a test of one route asks, or a change of the choice would leave it testing another."""
+    from deers_b200 import ops
+    return ops.Context.current(torch.device("cuda", torch.cuda.current_device())).product_route(which, [(M, N)], K, a_mn, b_mn, aligned, heads)
+
+
+@pytest.mark.parametrize("M,N,K,pair", [(*size, False) for size in (
+    (256, 256, 64), (264, 264, 328), (520, 192, 1032), (512, 520, 8192), (640, 1544, 4104), (1280, 768, 8192), (2056, 2304, 776), (4104, 1288, 200), (8192, 96, 72),
+    (9472, 768, 64), (304, 3000, 16392), (4104, 2056, 72), (2184, 4488, 1032))] + [(*size, True) for size in (
+    (9480, 4864, 264), (8072, 2264, 776), (7992, 2104, 1032), (3848, 4472, 776), (4744, 3832, 840))])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
-def test_f16_gemm_pairs_of_ctas(M, N, K, a_mn, b_mn):
-    """Tiles of 256 rows by two CTAs where the choice falls on them: a second half of few or no rows, columns that end in either half, one
-    or several tiles a pair.  Small integers, as above; sums of up to 16392 terms of which few are not zero."""
+def test_f16_gemm_pairs_of_ctas(M, N, K, pair, a_mn, b_mn):
+    """Tiles of 256 rows by two CTAs: a second half of few or no rows, columns that end in either half, fewer K blocks than stages and more, several tiles a
+    pair; and sizes near them that stay with single CTAs.  Small integers, as above; sums of up to 16392 terms of which few are not zero."""
+    assert _route(_lib.PRODUCT_F16, M, N, K, a_mn, b_mn).pair == pair
     from deers_b200 import ops
     rng = np.random.default_rng(M + N + K)
     a = rng.integers(-1, 2, (K, M) if a_mn else (M, K)).astype(np.float16)
@@ -799,10 +814,12 @@ def test_f16_gemm_pairs_of_ctas(M, N, K, a_mn, b_mn):
 
 @pytest.mark.parametrize("aligned", [True, False])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, True), (False, False), (True, True), (True, False)])
-@pytest.mark.parametrize("M,N,K", [(2052, 1540, 4), (1156, 1028, 20), (2048, 640, 64), (1028, 1092, 68), (1100, 644, 132), (1024, 768, 192), (1284, 196, 1000), (260, 1540, 772),
-                                   (196, 772, 2052)])
-def test_f32_gemm_on_the_tensor_core(M, N, K, a_mn, b_mn, aligned):
-    """Tiles that end in rows, columns and k, one to many stages, whole K and K shared by a cluster, each storage order, rows on 16-byte
+@pytest.mark.parametrize("M,N,K,tensor_core", [
+    (2052, 1540, 4, "aligned"), (1156, 1028, 20, "no"), (2048, 640, 64, "no"), (1028, 1092, 68, "aligned"), (1100, 644, 132, "yes"), (1024, 768, 192, "yes"),
+    (1284, 196, 1000, "yes"), (260, 1540, 772, "yes"), (196, 772, 2052, "yes"),
+    (1660, 508, 4, "yes"), (1404, 636, 20, "yes"), (1276, 700, 64, "yes"), (636, 956, 68, "yes")])
+def test_f32_gemm_on_the_tensor_core(M, N, K, tensor_core, a_mn, b_mn, aligned):
+    """Tiles that end in rows, columns and k, one short stage to many, whole K and K shared by a cluster, each storage order, rows on 16-byte
     boundaries and on none.  Values of three bf16 each, sums that start anew every 16 k: 1e-7 of the result in the 2-norm (measured 5e-8 to
     8.1e-8; two f16 per value or one accumulator give 2.8e-7), and small integers exactly."""
     from deers_b200 import gpt
@@ -814,6 +831,7 @@ def test_f32_gemm_on_the_tensor_core(M, N, K, a_mn, b_mn, aligned):
         t.copy_(torch.randint(-8, 9, t.shape, device="cuda", generator=g) if whole else torch.randn(t.shape, device="cuda", generator=g))
         return t[:, pad:]
 
+    assert _route(_lib.PRODUCT_F32, M, N, K, a_mn, b_mn, aligned).tensor_core == (tensor_core == "yes" or tensor_core == "aligned" and aligned)
     for whole in (False, True):
         a = operand(*((K, M) if a_mn else (M, K)), whole)
         b = operand(*((K, N) if b_mn else (N, K)), whole)
@@ -871,20 +889,26 @@ def test_f32_gemm_on_the_tensor_core_of_subnormal_operands(power, other, small, 
     if small == "b":
         got, want = got.T, want.T
     half = x.shape[0] // 2
+    assert _route(_lib.PRODUCT_F32, M, N, K, a_mn, b_mn, aligned).tensor_core
     assert ((got[:half] - want[:half]).norm() / want[:half].norm()).item() < 1e-7 * max(1.0, (K / 192) ** 0.5)
     assert ((got[half:] - want[half:]).norm() / want[half:].norm()).item() < 2.0 ** -25 * (K / 4) ** 0.5
 
 
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38])
-@pytest.mark.parametrize("a_mn,b_mn", [(False, True), (True, True), (False, False)])
-def test_f32_gemm_on_the_tensor_core_of_what_is_not_finite(value, a_mn, b_mn):
-    """Infinities, NaN and values that round to an infinity of bf16, in either operand and against zeros: what the products of f32 give."""
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn,aligned,parts", [(1024, 768, 192, False, True, True, 1), (1024, 768, 192, True, True, True, 1), (1024, 768, 192, False, False, True, 1),
+                                                           (1024, 192, 768, False, True, True, 4), (1000, 770, 190, True, False, False, 1), (1001, 190, 770, False, True, False, 5)])
+def test_f32_gemm_on_the_tensor_core_of_what_is_not_finite(value, M, N, K, a_mn, b_mn, aligned, parts):
+    """Infinities, NaN and values that round to an infinity of bf16, in either operand and against zeros: what the products of f32 give.  One block a
+    tile, and a cluster in which one block alone has them; rows on any boundary."""
     from deers_b200 import gpt
-    M, N, K = 1024, 768, 192
     g = torch.Generator(device="cuda").manual_seed(5)
     a, b = (torch.randn(s, device="cuda", generator=g) * 0.25 for s in ((M, K), (K, N)))
     a[700, 100], b[30, 5], b[100, 77] = value, value, 0.0
-    got = gpt.gemm_f32(a.T.contiguous() if a_mn else a, b if b_mn else b.T.contiguous(), a_mn, b_mn).double()
+    r = _route(_lib.PRODUCT_F32, M, N, K, a_mn, b_mn, aligned)
+    assert (r.tensor_core, r.parts) == (1, parts)
+    pad = 0 if aligned else 1
+    held = [torch.empty((t.shape[0], t.shape[1] + pad), device="cuda")[:, pad:].copy_(t) for t in (a.T if a_mn else a, b if b_mn else b.T)]
+    got = gpt.gemm_f32(*held, a_mn, b_mn).double()
     want = a.double() @ b.double()
     assert torch.equal(got.isnan(), want.isnan())
     fin = want.abs() < 3e38
@@ -894,16 +918,24 @@ def test_f32_gemm_on_the_tensor_core_of_what_is_not_finite(value, a_mn, b_mn):
     assert ((got[fin][big] - want[fin][big]) / want[fin][big]).abs().nan_to_num(0).max().item() < 1e-5 if big.any() else True
 
 
-@pytest.mark.parametrize("M,N,K,a_mn,b_mn", [
-    # logits: A resident (one, three, four K blocks) and not; runs of pairs that change rows; rows and columns that end in a tile or its half
-    (1024, 5008, 192, 0, 1), (300, 12296, 64, 0, 1), (2056, 2568, 256, 0, 1), (520, 9608, 328, 0, 1), (136, 20008, 24, 0, 1),
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn,tile,resident", [
+    # logits: few waves, single CTAs
+    (1024, 5008, 192, 0, 1, None, 0), (300, 12296, 64, 0, 1, None, 0), (2056, 2568, 256, 0, 1, None, 0), (520, 9608, 328, 0, 1, None, 0), (136, 20008, 24, 0, 1, None, 0),
+    # many waves, pairs: A resident (one to four K blocks), and not (rows of tiles that would leave pairs idle, deeper K); rows that end in either half
+    (1024, 12296, 64, 0, 1, (256, 128), 1), (1000, 12296, 128, 0, 1, (256, 128), 2), (136, 95000, 24, 0, 1, (256, 128), 1), (760, 18056, 192, 0, 1, (256, 128), 3),
+    (2056, 6024, 256, 0, 1, (256, 128), 4), (1160, 9992, 64, 0, 1, (256, 128), 0), (1000, 12040, 328, 0, 1, (256, 128), 0),
     # input gradient: K shared out, 128 and 192 columns, one and two of them
-    (1024, 192, 50264, 0, 0), (264, 128, 30008, 0, 0), (2000, 320, 16392, 0, 0), (200, 64, 70000, 0, 0),
-    # weight gradient: transposed, 128 and 192 columns
-    (192, 50264, 1024, 1, 1), (64, 40008, 264, 1, 1), (320, 12296, 520, 1, 1), (384, 30008, 72, 1, 1)])
-def test_f16x3_gemm_pairs_of_ctas(M, N, K, a_mn, b_mn):
-    """The head's products by pairs of CTAs.  Operands of 22 bits (two f16), f32 sums in the tensor core: 2e-6 of the largest value times
-    max(1, sqrt(K) / 16), as for single CTAs; small integers exactly, so any tile, half or K range dropped or taken twice shows."""
+    (1024, 192, 50264, 0, 0, (256, 192), 0), (264, 128, 30008, 0, 0, None, 0), (2000, 320, 16392, 0, 0, (256, 192), 0), (200, 64, 70000, 0, 0, (256, 128), 0),
+    (520, 128, 40000, 0, 0, (256, 128), 0),
+    # weight gradient, transposed: columns of the tile that are there in part, one to three of them; and few tokens or tiles, single CTAs
+    (192, 50264, 1024, 1, 1, (192, 256), 0), (320, 50264, 520, 1, 1, (192, 256), 0), (576, 30008, 584, 1, 1, (192, 256), 0),
+    (64, 40008, 264, 1, 1, None, 0), (320, 12296, 520, 1, 1, None, 0), (384, 30008, 72, 1, 1, None, 0)])
+def test_f16x3_gemm_pairs_of_ctas(M, N, K, a_mn, b_mn, tile, resident):
+    """The head's products by pairs of CTAs, and those near them that stay with single CTAs (tile None).  Operands of 22 bits (two f16), f32 sums in the
+    tensor core: 2e-6 of the largest value times max(1, sqrt(K) / 16), as for single CTAs; small integers exactly, so any tile, half or K range
+    dropped or taken twice shows."""
+    r = _route(_lib.PRODUCT_F16X3, M, N, K, a_mn, b_mn)
+    assert (r.pair, r.resident) == (tile is not None, resident) and (r.tile_m, r.tile_n) == (tile or (128, 128))
     from deers_b200 import gpt
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     for whole in (True, False):
@@ -923,12 +955,18 @@ def test_f16x3_gemm_pairs_of_ctas(M, N, K, a_mn, b_mn):
             assert (got.double() - want).abs().max().item() <= 2e-6 * max(1.0, K ** 0.5 / 16) * want.abs().max().item()
 
 
-@pytest.mark.parametrize("V,H,D,B,T", [(12289, 2, 32, 2, 100), (50257, 6, 32, 1, 257), (9601, 5, 64, 3, 99), (10111, 4, 64, 2, 131), (1024, 2, 32, 1, 9),
-                                       (131073, 1, 64, 1, 130)])
-def test_gpt_cross_entropy_from_the_head_product(V, H, D, B, T):
-    """Row statistics left by the head product (resident A or not, ragged rows and columns) or taken by a pass of their own: loss and
-    gradients of a model that is only embedding, norm and head, against float64.  The bound is the head products' (2e-6 of the largest value)
-    with room for sums of V terms."""
+@pytest.mark.parametrize("V,H,D,B,T,pair,resident", [
+    # a pass over the logits
+    (12289, 2, 32, 2, 100, 0, 0), (50257, 6, 32, 1, 257, 0, 0), (9601, 5, 64, 3, 99, 0, 0), (10111, 4, 64, 2, 131, 0, 0), (1024, 2, 32, 1, 9, 0, 0),
+    # statistics of the head product: one to four resident K blocks of A, deeper K, rows of tiles that would leave pairs idle; V that ends in a tile
+    (131073, 1, 64, 1, 130, 1, 1), (50257, 2, 32, 2, 128, 1, 1), (24101, 4, 32, 2, 250, 1, 2), (12289, 6, 32, 4, 250, 1, 3), (12301, 4, 64, 4, 253, 1, 4),
+    (24077, 5, 64, 2, 254, 1, 0), (9601, 6, 32, 5, 250, 1, 0)])
+def test_gpt_cross_entropy_from_the_head_product(V, H, D, B, T, pair, resident):
+    """Row statistics left by the head product or taken by a pass of their own: loss, logits (of an odd vocabulary: rows on any boundary, turned round in
+    shared memory) and gradients of a model that is only embedding, norm and head, against float64.  The bound is the head products' (2e-6 of the
+    largest value) with room for sums of V terms."""
+    r = _route(_lib.PRODUCT_F16X3, B * T, V, H * D)
+    assert (r.pair, r.resident) == (pair, resident)
     from deers_b200 import gpt
     C = H * D
     m = gpt.GPT(gpt.GPTConfig(V, T, 0, H, C, 8), torch.device("cuda", torch.cuda.current_device()), B)
@@ -939,14 +977,112 @@ def test_gpt_cross_entropy_from_the_head_product(V, H, D, B, T):
     tgt[0, 0], tgt[-1, -1] = 0, V - 1
     loss = m.forward_backward(ids.cuda(), tgt.cuda())
     m.ctx.sync()
-    w, h = wte.double().requires_grad_(), head.double().requires_grad_()
-    x = w[ids.reshape(-1)]
+    logits = m.forward(ids.cuda())
+    w, h = wte.double().cuda().requires_grad_(), head.double().cuda().requires_grad_()
+    x = w[ids.reshape(-1).cuda()]
     x = x / torch.sqrt((x * x).mean(1, keepdim=True) + 1e-5)
-    want = torch.nn.functional.cross_entropy(x @ h, tgt.reshape(-1))
+    exact = x @ h
+    want = torch.nn.functional.cross_entropy(exact, tgt.reshape(-1).cuda())
     want.backward()
     assert abs(loss.item() - want.item()) < 1e-6 * max(1.0, want.item())
+    assert (logits.reshape(-1, V).double() - exact).abs().max().item() <= 2e-6 * exact.abs().max().item()
     for i, t in enumerate((w, h)):
-        assert np.abs(m.grad(i) - t.grad.numpy()).max() <= 1e-5 * t.grad.abs().max().item()
+        assert np.abs(m.grad(i) - t.grad.cpu().numpy()).max() <= 1e-5 * t.grad.abs().max().item()
+
+
+@pytest.mark.parametrize("scale,peak", [(1e-3, 0.0), (0.5, 0.0), (3.0, 0.0), (40.0, 0.0), (0.1, 20.0), (1.0, -30.0)])
+def test_row_statistics_of_the_head_product(scale, peak):
+    """Every token the same and every target the same, so that the mean loss is one row's: lse from the exponentials the head product's epilogue sums, for flat
+    rows, rows of one large or one small logit and rows whose logits spread over hundreds (most exponentials zero), against float64 on the
+    model's own logits.  log(s) + m, the picked logit less it and the mean round once each: 3 2^-24 of the largest of them.  s: an exponential is
+    within 4 2^-24 of its value (two roundings of its argument's parts and the power of two), 32 of a thread are added in pairs and 3 more
+    sums follow to 393 parts of 128 columns: 24 roundings of 2^-24."""
+    from deers_b200 import gpt
+    V, C, B, T = 50264, 64, 2, 128
+    assert _route(_lib.PRODUCT_F16X3, B * T, V, C).pair
+    m = gpt.GPT(gpt.GPTConfig(V, T, 0, 2, C, 8), torch.device("cuda", torch.cuda.current_device()), B)
+    g = torch.Generator().manual_seed(7)
+    wte, head = torch.randn((V, C), generator=g), torch.randn((C, V), generator=g) * scale
+    for token in (0, 1, 77, V - 1):
+        x = wte[token] / wte[token].square().mean().sqrt()
+        head[:, 31 * token % V] = x * (peak / C) if peak else head[:, 31 * token % V]
+    m.load_parameters([wte.numpy(), head.numpy()])
+    for token in (0, 1, 77, V - 1):
+        ids = torch.full((B, T), token, device="cuda")
+        row = m.forward(ids)[0, 0].double()
+        for t in (0, 31 * token % V, V - 1):
+            loss = m.forward_backward(ids, torch.full((B, T), t, device="cuda")).item()
+            want = (row.logsumexp(0) - row[t]).item()
+            most = max(row.abs().max().item(), abs(want))
+            assert abs(loss - want) <= 2.0 ** -24 * (3 * most + 28), (token, t)
+
+
+def test_row_statistics_keep_a_nan_to_its_row():
+    """One token's row of the embedding holds a NaN: its logits, its gradient and the mean loss are NaN, every other token's gradient is as it was."""
+    from deers_b200 import gpt
+    V, C, B, T = 50257, 64, 2, 128
+    assert _route(_lib.PRODUCT_F16X3, B * T, V, C).pair
+    m = gpt.GPT(gpt.GPTConfig(V, T, 0, 2, C, 8), torch.device("cuda", torch.cuda.current_device()), B)
+    g = torch.Generator().manual_seed(3)
+    wte, head = torch.randn((V, C), generator=g), torch.randn((C, V), generator=g) * 0.5
+    ids = torch.randperm(V, generator=g)[:B * T].reshape(B, T)
+    tgt = torch.randint(0, V, (B, T), generator=g).cuda()
+    m.load_parameters([wte.numpy(), head.numpy()])
+    m.forward_backward(ids.cuda(), tgt)
+    m.ctx.sync()
+    before = m.grad(0)[ids.reshape(-1).numpy()]
+    wte[ids[1, 5], 9] = float("nan")
+    m.load_parameters([wte.numpy(), head.numpy()])
+    assert np.isnan(m.forward_backward(ids.cuda(), tgt).item())
+    m.ctx.sync()
+    after = m.grad(0)[ids.reshape(-1).numpy()]
+    hit = T + 5
+    assert np.isnan(after[hit]).all() and np.array_equal(np.delete(after, hit, 0), np.delete(before, hit, 0))
+
+
+def test_gpt_products_of_values_that_are_infinite_in_bf16():
+    """A channel of one head's values reaches 3.396e38 at the first token, which f32 holds and bf16 does not: the projection (with its norm), and the weight
+    gradients in one launch, work out again what the tensor core's parts cannot hold.  Everything is finite; the gradients of the rows
+    and columns concerned are compared each by its own size, as the other parameters are."""
+    from deers_b200 import gpt, ops
+    from oracle import ref
+    V, L, H, D, Hm, B, T = 64, 1, 6, 32, 768, 4, 256
+    C = H * D
+    cfg = (V, L, H, C, Hm)
+    params = [p.copy() for p in ref.gpt_init_params(cfg, seed=5)]
+    m = gpt.GPT(gpt.GPTConfig(V, T, L, H, C, Hm), torch.device("cuda", torch.cuda.current_device()), B)
+    at = {n: i for i, (n, _) in enumerate(m.named_parameters())}
+    wte, wv, wo = (params[next(i for n, i in at.items() if k in n)] for k in ("wte", "v_proj", "out_proj"))
+    channel, held = 5, 7
+    wte[0, channel], wte[1:, channel] = 2.0, 0.0                 # (f32 attention sums before it divides: one such value, no overflow)
+    n1 = wte[0] / np.sqrt((wte[0].astype(np.float64) ** 2).mean() + 1e-5)
+    wv[:, held] = 0.0
+    wv[channel, held] = np.float32(3.396e38 / n1[channel])
+    wo[held] = np.random.default_rng(1).standard_normal(C).astype(np.float32) * np.float32(1e-37)
+    rng = np.random.default_rng(2)
+    ids, tgt = rng.integers(1, V, (B, T)), rng.integers(0, V, B * T)
+    ids[:, 0] = 0
+    m.load_parameters(params)
+    route = m.ctx.product_route
+    assert route(_lib.PRODUCT_F32_NORM, [(B * T, 3 * C)], C, heads=D).tensor_core
+    assert route(_lib.PRODUCT_F32, [(Hm, C), (C, Hm), (C, C), (C, 3 * C)], B * T, True, True).tensor_core
+    tid, ttg = torch.from_numpy(ids).cuda(), torch.from_numpy(tgt).cuda()
+    logits, loss = m.forward(tid), m.forward_backward(tid, ttg)
+    m.ctx.sync()
+    want = ref.gpt_step(cfg, params, ids, tgt)
+    got = logits.cpu().numpy().reshape(B * T, V)
+    assert np.isfinite(want["logits"]).all() and np.abs(got - want["logits"]).max() <= 1e-4 * np.abs(want["logits"]).max()
+    assert abs(loss.item() - want["loss"]) < 1e-5 * max(1.0, abs(want["loss"]))
+    for name, i in at.items():
+        g, w = m.grad(i), want["grads"][i]
+        assert np.isfinite(w).all(), name
+        if "out_proj" in name:
+            assert np.abs(w[held]).max() > 1e30 and np.abs(g[held] - w[held]).max() <= 1e-4 * np.abs(w[held]).max()
+            g, w = np.delete(g, held, 0), np.delete(w, held, 0)
+        if "v_proj" in name:
+            assert 0 < np.abs(w[:, held]).max() < 1e-35 and np.abs(g[:, held] - w[:, held]).max() <= 1e-4 * np.abs(w[:, held]).max()
+            g, w = np.delete(g, held, 1), np.delete(w, held, 1)
+        assert np.abs(g - w).max() <= 1e-4 * np.abs(w).max() + 1e-7, name
 
 
 @pytest.mark.parametrize("B,H,T,D", [
