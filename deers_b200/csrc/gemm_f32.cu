@@ -178,11 +178,15 @@ GemmPlan plan_single(deers_ctx* ctx, int M, int N, int K, bool aligned) { return
 
 // The plan of a product of normalised rows, and whether its tiles rotate heads of `heads` columns (0: there are none).
 GemmPlan plan_norm(deers_ctx* ctx, int M, int N, int K, bool aligned, int heads, bool* rotated) {
-    // (the choice below between rotating in a tile and beside it was measured for the tensor core's tiles up to 384 columns only)
-    const double tc = aligned && K <= 384 ? 1.0 : 0.0;
+    const bool rotates = heads && heads % 8 == 0;
+    // Products that may rotate heads take the tensor core up to 384 columns: so far was the choice between rotating in a tile and beside it
+    // measured on its tiles (further on it would gain too, C 512 626 -> 552 us, with that choice drawn anew).  What rotates nothing has no
+    // such line: forwards with the up projection on FFMA and on the tensor core, C 512, 4 layers, 1024 tokens 825 and 626 us, 256 tokens
+    // 292 and 271, 128 tokens 201 and 204; C 1024, 2 layers, 1024 tokens 1196 and 1010.
+    const double tc = aligned && (!rotates || K <= 384) ? 1.0 : 0.0;
     const GemmPlan p = plan_gemm(1, &M, &N, K, tc, ctx->cluster_capacity, 0);
     *rotated = false;
-    if (heads == 0 || heads % 8) return p;
+    if (!rotates) return p;
     // A rotary launch of its own takes up to 4400 of these cycles (1.4 to 2 us): rotate here unless tiles that hold whole heads cost more
     // than that (heads of 48 columns leave 32 x 96 and 64 x 96 tiles: 231 x 576 x 192 takes 7.5 us in them, 3.6 in 32 x 32).
     // Several waves of clusters do not count: the estimate takes them to follow one another without a gap (forwards of 4 layers,

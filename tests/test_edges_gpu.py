@@ -734,6 +734,19 @@ def test_gpt_rotation_inside_the_projection(H, D, B, T, tile):
     assert n[0] == 1 + 5 + (not inside) + 3
 
 
+@pytest.mark.parametrize("H,D,Hm,B,T,parts", [(7, 64, 2048, 1, 130, 2), (8, 64, 2048, 1, 260, 1), (10, 64, 1024, 2, 258, 1), (40, 10, 1500, 1, 260, 2)])
+def test_gpt_up_projection_of_wide_models_on_the_tensor_core(H, D, Hm, B, T, parts):
+    """Norm and product of an up projection, which rotates nothing, whatever its width; whole K and K shared by a cluster.  (Heads of ten columns: the
+    other norm's product rotates nothing either.)"""
+    C = H * D
+    r = _route(_lib.PRODUCT_F32_NORM, B * T, Hm, C)
+    assert (r.tensor_core, r.parts, r.rotated) == (1, parts, 0)
+    if D % 8:
+        assert _route(_lib.PRODUCT_F32_NORM, B * T, 3 * C, C, heads=D).tensor_core
+    m, ids, tgt, logits, loss, n, want = _gpt_and_oracle(64, 1, H, D, Hm, B, T)
+    _check_gpt(m, logits, loss, want)
+
+
 def test_gpt_train_step_takes_pointers_on_any_boundary():
     """What a copy takes and a kernel cannot: ids four bytes off their boundary, loss and norm one byte off."""
     import ctypes
