@@ -24,19 +24,22 @@ int bwd_rows(const deers_ctx* ctx, const F32Params& p, int resident) {
     return p.T > 128 ? (2 * blocks <= 2 * slots ? 2 : 4) : (2 * blocks * 5 <= 6 * slots ? 2 : 4);
 }
 
+// Blocks of 8 or 16 rows (rm 1 or 2), from the module of the tile width.
+template <int DP>
+int fwd_few_blocks(deers_ctx* ctx, const F32Params& p, int groups, int stream, int rm) {
+    return DP == 32 ? launch_attn_fwd_f32_few32(ctx, p, groups, stream, rm) : DP == 64 ? launch_attn_fwd_f32_few64(ctx, p, groups, stream, rm)
+         : DP == 96 ? launch_attn_fwd_f32_few96(ctx, p, groups, stream, rm) : launch_attn_fwd_f32_few128(ctx, p, groups, stream, rm);
+}
+template <int DP>
+int bwd_few_blocks(deers_ctx* ctx, const F32Params& p, int groups, int rm) {
+    return DP == 32 ? launch_attn_bwd_f32_few32(ctx, p, groups, rm) : DP == 64 ? launch_attn_bwd_f32_few64(ctx, p, groups, rm)
+         : DP == 96 ? launch_attn_bwd_f32_few96(ctx, p, groups, rm) : launch_attn_bwd_f32_few128(ctx, p, groups, rm);
+}
+
 template <int DP, int NG, int FBN>
 int fwd_any_rows(deers_ctx* ctx, const F32Params& p) {
     const int rm = fwd_rows(ctx, p);
-    if (rm == 4) return fwd_launch_f32<DP, NG, FBN, 4>(ctx, p);
-    return DP == 32 ? launch_attn_fwd_f32_few32(ctx, p, NG, FBN, rm) : DP == 64 ? launch_attn_fwd_f32_few64(ctx, p, NG, FBN, rm)
-         : DP == 96 ? launch_attn_fwd_f32_few96(ctx, p, NG, FBN, rm) : launch_attn_fwd_f32_few128(ctx, p, NG, FBN, rm);
-}
-template <int DP, int NG>
-int bwd_any_rows(deers_ctx* ctx, const F32Params& p) {
-    const int rm = bwd_rows(ctx, p, DP <= 64 && NG == 4 ? 2 : 1);
-    if (rm == 4) return bwd_launch_f32<DP, NG, 4>(ctx, p);
-    return DP == 32 ? launch_attn_bwd_f32_few32(ctx, p, NG, rm) : DP == 64 ? launch_attn_bwd_f32_few64(ctx, p, NG, rm)
-         : DP == 96 ? launch_attn_bwd_f32_few96(ctx, p, NG, rm) : launch_attn_bwd_f32_few128(ctx, p, NG, rm);
+    return rm == 4 ? fwd_launch_f32<DP, NG, FBN, 4>(ctx, p) : fwd_few_blocks<DP>(ctx, p, NG, FBN, rm);
 }
 
 // Narrow heads stream 64 keys at a time (half the reads of Q per score), unless the sequence has so few tiles that groups
@@ -50,9 +53,10 @@ template <int DP>
 int fwd_impl(deers_ctx* ctx, const F32Params& p) {
     if constexpr (DP <= 32) {
         if (p.T > 128 && few_blocks(ctx, p, 1, p.T <= 256 ? 2 : 1)) return fwd_any_rows<DP, 8, 32>(ctx, p);
-        if (p.T > 128 && p.T <= 512) return few_blocks(ctx, p, 1, 2) ? launch_attn_fwd_f32_few32(ctx, p, 4, 32, 2) : fwd_launch_f32<DP, 4, 32, 4>(ctx, p);
+        if (p.T > 128 && p.T <= 512) return few_blocks(ctx, p, 1, 2) ? fwd_few_blocks<DP>(ctx, p, 4, 32, 2) : fwd_launch_f32<DP, 4, 32, 4>(ctx, p);
+        if (p.T > 128) return fwd_launch_f32<DP, 4, 64, 4>(ctx, p);         // (more blocks than SMs: of 32 rows)
     }
-    if constexpr (DP <= 64) {
+    if constexpr (DP == 64) {
         if (p.T > 128) return fwd_any_rows<DP, 4, 64>(ctx, p);
     }
     return fwd_any_rows<DP, 4, 32>(ctx, p);
@@ -63,9 +67,10 @@ int fwd_impl(deers_ctx* ctx, const F32Params& p) {
 template <int DP>
 int bwd_impl(deers_ctx* ctx, const F32Params& p) {
     if constexpr (DP <= 64) {
-        if (p.T > 128 && few_blocks(ctx, p, 2, 1)) return bwd_any_rows<DP, 8>(ctx, p);
+        if (p.T > 128 && few_blocks(ctx, p, 2, 1)) return bwd_few_blocks<DP>(ctx, p, 8, bwd_rows(ctx, p, 1));       // (one block per SM at most: never 32 rows)
     }
-    return bwd_any_rows<DP, 4>(ctx, p);
+    const int rm = bwd_rows(ctx, p, DP <= 64 ? 2 : 1);
+    return rm == 4 ? bwd_launch_f32<DP, 4, 4>(ctx, p) : bwd_few_blocks<DP>(ctx, p, 4, rm);
 }
 
 F32Params base_params(const deers_attn_desc* d) {

@@ -10,7 +10,7 @@ int fwd_few(deers_ctx* ctx, const F32Params& p, int groups, int stream) {
     if constexpr (DP <= 32) {
         if (groups == 8) return fwd_launch_f32<DP, 8, 32, RM>(ctx, p);
     }
-    if constexpr (DP <= 64) {
+    if constexpr (DP == 64) {
         if (stream == 64) return fwd_launch_f32<DP, 4, 64, RM>(ctx, p);
     }
     return fwd_launch_f32<DP, 4, 32, RM>(ctx, p);
