@@ -701,7 +701,8 @@ void x3_split(X3Plan& pl, long long tiles, int K, int room, int least) {
 
 // Single CTAs on 128 x 128, or pairs: for logits of many waves (1024 x 50257 x 192 77 -> 61 us, in the model with the row statistics 77 and no
 // pass of 42 for them; 300 x 12000 x 320, two waves, 11.2 and 15.3), input gradients with long parts of K (1024 x 192 x 50257 87 -> 57) and weight
-// gradients of many tokens (192 x 50257 x 1024 76 -> 56; of 300 tokens 11.2 and 14.7: one pair of accumulators, nothing beside its epilogue).
+// gradients of many tokens (192 x 50257 x 1024 76 -> 56; of 300 tokens 11.2 and 14.7: one pair of accumulators, nothing beside its epilogue;
+// 128 columns never leave fewer waves than single CTAs have).
 X3Plan x3_plan(int M, int N, int K, int a_mn, int b_mn, int sm_count, int pairs) {
     X3Plan pl{};
     const int kblocks = (K + XK - 1) / XK;
@@ -714,7 +715,7 @@ X3Plan x3_plan(int M, int N, int K, int a_mn, int b_mn, int sm_count, int pairs)
     const long long pair_tiles = (long long)rows * ((n + tn - 1) / tn);
     const long long waves = (tiles + sm_count - 1) / sm_count, pair_waves = (pair_tiles + pairs - 1) / pairs;
     if (m <= XM) return pl;                                           // one CTA of a pair would have nothing to do
-    if (a_mn ? !(K >= 512 && pair_waves < waves) : b_mn ? !(waves >= 6 && pair_waves <= waves) : !(pl.k_chunk >= 16 * XK && N % 4 == 0)) return pl;
+    if (a_mn ? !(K >= 512 && tn == 192 && pair_waves < waves) : b_mn ? !(waves >= 6 && pair_waves <= waves) : !(pl.k_chunk >= 16 * XK && N % 4 == 0)) return pl;
     pl = X3Plan{};
     pl.pair = true;
     pl.trans = a_mn != 0;
@@ -850,7 +851,7 @@ int launch_gemm_f16x3(deers_ctx* ctx, int M, int N, int K, const void* a_hi, con
         p.c = out; p.ldc = ldo; p.M = m; p.N = n; p.K = K; p.parts = pl.parts; p.k_chunk = pl.k_chunk; p.out_scale = out_scale;
         p.resident = pl.resident; p.stats = stats; p.err = ctx->dev_err;
         const bool wide = pl.tn == 192;
-        if (pl.trans) rc = wide ? x3_launch_pair<1, 1, 192, true, false, false>(ctx, t, p, pairs) : x3_launch_pair<1, 1, 128, true, false, false>(ctx, t, p, pairs);
+        if (pl.trans) rc = x3_launch_pair<1, 1, 192, true, false, false>(ctx, t, p, pairs);
         else if (!b_mn) rc = wide ? x3_launch_pair<0, 0, 192, false, false, false>(ctx, t, p, pairs) : x3_launch_pair<0, 0, 128, false, false, false>(ctx, t, p, pairs);
         else if (!vec) rc = x3_launch_pair<0, 1, 128, false, false, true>(ctx, t, p, pairs);
         else if (stats && !split) {
