@@ -41,9 +41,8 @@ constexpr uint32_t TC_SQ = TC_RING * TC_STAGE;                 // rows' sums of 
 constexpr uint32_t TC_BARS = TC_SQ + 2 * TC_M * 4;               // (and the inverse norms)
 constexpr uint32_t TC_SMEM = TC_BARS + 64;                      // a barrier per stage, TMEM base, abort flag
 static_assert(TC_M * (TC_N + 4) * 4 <= TC_SQ && TC_SMEM <= 232448, "shared memory");
-// TMEM columns: main of six steps of 16 k, used in turn | corr1 | corr2
-constexpr int TC_SLOTS = 6;
-constexpr uint32_t TC_C1 = TC_SLOTS * TC_N, TC_C2 = TC_C1 + TC_N;
+// TMEM columns: main of a stage's four steps of 16 k | corr1 | corr2
+constexpr uint32_t TC_C1 = 4 * TC_N, TC_C2 = TC_C1 + TC_N;
 static_assert(TC_C2 + TC_N <= 512, "TMEM");
 
 // Eight consecutive floats of which `valid` exist (p on a 16-byte boundary).
@@ -233,8 +232,8 @@ __device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int ti
     float sum[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) sum[e] = 0.f;
-    // The sums of the last stage issued.  slot, base: its place in the ring and its first step's columns; phase: of that place's barrier.
-    int slot = 0, base = 0, left = klen;                           // left: k from the present stage on
+    // The sums of the last stage issued.  slot: its place in the ring; phase: of that place's barrier.
+    int slot = 0, left = klen;                           // left: k from the present stage on
     uint32_t phase = 0;
     auto drain = [&](int steps, bool last) {
         mbar_wait(ws, &done[slot], phase, DEERS_KERR_GEMM | 0x31);
@@ -244,8 +243,7 @@ __device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int ti
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
             if (ks < steps) {
-                const int at = base + ks >= TC_SLOTS ? base + ks - TC_SLOTS : base + ks;
-                tmem_ld_x16(t_out + (uint32_t)at * TC_N, u[ks]);
+                tmem_ld_x16(t_out + (uint32_t)ks * TC_N, u[ks]);
             } else {
 #pragma unroll
                 for (int e = 0; e < 16; ++e) u[ks][e] = 0;
@@ -282,9 +280,8 @@ __device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int ti
         if (s + 2 < stages) load(x);
         fence_proxy_async_smem();
         if (s > 0) {
-            drain(4, false);                                       // frees columns that this stage uses again
+            drain(4, false);                                       // frees the columns, which this stage uses again
             if (now == 0) phase ^= 1u;
-            base = base >= 2 ? base - 2 : base + 4;                // four steps on, modulo six
             left -= 64;
         }
         slot = now;
@@ -295,15 +292,14 @@ __device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int ti
             const uint32_t s0 = (uint32_t)uniform((int)smem_u32(st));
             const uint64_t a = A_MN ? desc_mnmajor(s0, 0, TC_BLOCK) : desc_kmajor(s0, 0, 0);
             const uint64_t b = B_MN ? desc_mnmajor(s0 + 3 * TC_A, 0, TC_BLOCK) : desc_kmajor(s0 + 3 * TC_A, 0, 0);
-            const int steps = min(4, (left + 15) / 16), first = uniform(base);
+            const int steps = min(4, (left + 15) / 16);
             if (elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
                     if (ks < steps) {
                         const uint64_t ah = a + (A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0)), bh = b + (B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0));
                         const uint64_t am = ah + (TC_A >> 4), al = am + (TC_A >> 4), bm = bh + (TC_B >> 4);
-                        const int at = first + ks >= TC_SLOTS ? first + ks - TC_SLOTS : first + ks;
-                        umma_ss(tmem + (uint32_t)at * TC_N, ah, bh, ID64, 0u);
+                        umma_ss(tmem + (uint32_t)ks * TC_N, ah, bh, ID64, 0u);
                         umma_ss(tmem + TC_C1, ah, bm, ID128, s + ks > 0);              // h m | h l  (the parts of B follow one another)
                         umma_ss(tmem + TC_C1, am, bh, ID128, 1u);                      // m h | m m
                         umma_ss(tmem + TC_C2, al, bh, ID64, 1u);                       // l h
