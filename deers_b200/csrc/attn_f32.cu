@@ -10,14 +10,15 @@ long long blocks_of(const F32Params& p, int kinds) { return (long long)kinds * p
 bool few_blocks(const deers_ctx* ctx, const F32Params& p, int kinds, int per_sm) { return blocks_of(p, kinds) <= (long long)per_sm * ctx->sm_count; }
 
 // Stationary rows per thread (an eighth of a block's).  Forward: 8 rows a block while those are one per SM, 16 up to two (us, 32 / 16 / 8 rows:
-// B1 H6 T128 D64 7.4 / 5.0 / 4.2, B1 H6 T256 D32 7.2 / 4.8 / 5.4, B1 H12 T333 D32 10.0 / 8.9 / 12.7, B8 H4 T100 D32 4.8 / 4.3 / 5.4, B4 H6 T256 D32 8.7 /
-// 10.4 / 16.5).
+// B1 H6 T128 D64 7.4 / 5.0 / 4.2, B1 H6 T256 D32 7.2 / 4.8 / 5.4, B1 H12 T333 D32 10.0 / 8.9 / 12.7, B8 H4 T100 D32 4.8 / 4.3 / 5.4, B4 H6 T256
+// D32 8.7 / 10.4 / 16.5).
 int fwd_rows(const deers_ctx* ctx, const F32Params& p) {
     const long long blocks = blocks_of(p, 1);
     return 4 * blocks <= ctx->sm_count ? 1 : 2 * blocks <= 2 * ctx->sm_count ? 2 : 4;
 }
 // Backward, `resident` blocks of a kind's size per SM: a wave and a fifth of short walks, two of longer ones, whose causal halves differ (B3 H4 T77
-// D48 13.6 / 8.2 / 9.3, B8 H4 T100 D32 10.1 / 12.0 / 16.4; B1 H8 T512 D32 33.0 / 29.3 / 45.6, B2 H6 T256 D96 36 / 48 / 69, B1 H3 T200 D48 20.5 / 12.4 / 10.1).
+// D48 13.6 / 8.2 / 9.3, B8 H4 T100 D32 10.1 / 12.0 / 16.4; B1 H8 T512 D32 33.0 / 29.3 / 45.6, B2 H6 T256 D96 36 / 48 / 69, B1 H3 T200 D48 20.5 /
+// 12.4 / 10.1).
 int bwd_rows(const deers_ctx* ctx, const F32Params& p, int resident) {
     const long long blocks = blocks_of(p, 2), slots = (long long)resident * ctx->sm_count;
     if (4 * blocks * 5 <= 6 * ctx->sm_count) return 1;
@@ -47,8 +48,9 @@ int fwd_any_rows(deers_ctx* ctx, const F32Params& p) {
 // take eight groups of 32 keys each where the blocks are few: up to 256 keys that is one tile per group (B4 H6 T256 D32 10.8 ->
 // 8.7), beyond, with an SM per block, half the walk (B1 H2 T1024 23.2 -> 21.5).  Heads of 64 do not gain (T 256 11.1 against 11.9,
 // T 512 19.9 against 20.6).
-// With more blocks heads up to 32 wide keep tiles of 32 keys to 512 of them, in blocks of 16 rows up to two of 32 per SM (tiles of 64 / these: B8 H6 T256
-// D32 14.4 / 12.4, B32 H12 T160 48.9 / 39.9, B4 H8 T400 19.4 / 18.2, B8 H8 T512 46.2 / 45.4; B2 H8 T300 13.2 / 8.8; error of O 1.9e-7 / 1.8e-7).
+// With more blocks heads up to 32 wide keep tiles of 32 keys to 512 of them, in blocks of 16 rows up to two of 32 per SM (tiles of 64 / these:
+// B8 H6 T256 D32 14.4 / 12.4, B32 H12 T160 48.9 / 39.9, B4 H8 T400 19.4 / 18.2, B8 H8 T512 46.2 / 45.4; B2 H8 T300 13.2 / 8.8; error of O 1.9e-7
+// / 1.8e-7).
 template <int DP>
 int fwd_impl(deers_ctx* ctx, const F32Params& p) {
     if constexpr (DP <= 32) {
@@ -67,7 +69,8 @@ int fwd_impl(deers_ctx* ctx, const F32Params& p) {
 template <int DP>
 int bwd_impl(deers_ctx* ctx, const F32Params& p) {
     if constexpr (DP <= 64) {
-        if (p.T > 128 && few_blocks(ctx, p, 2, 1)) return bwd_few_blocks<DP>(ctx, p, 8, bwd_rows(ctx, p, 1));       // (one block per SM at most: never 32 rows)
+        // (one block per SM at most: never 32 rows)
+        if (p.T > 128 && few_blocks(ctx, p, 2, 1)) return bwd_few_blocks<DP>(ctx, p, 8, bwd_rows(ctx, p, 1));
     }
     const int rm = bwd_rows(ctx, p, DP <= 64 ? 2 : 1);
     return rm == 4 ? bwd_launch_f32<DP, 4, 4>(ctx, p) : bwd_few_blocks<DP>(ctx, p, 4, rm);

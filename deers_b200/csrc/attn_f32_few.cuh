@@ -29,6 +29,8 @@ int fwd_few_rows(deers_ctx* ctx, const F32Params& p, int groups, int stream, int
     return rm == 2 ? fwd_few<DP, 2>(ctx, p, groups, stream) : fwd_few<DP, 1>(ctx, p, groups, stream);
 }
 template <int DP>
-int bwd_few_rows(deers_ctx* ctx, const F32Params& p, int groups, int rm) { return rm == 2 ? bwd_few<DP, 2>(ctx, p, groups) : bwd_few<DP, 1>(ctx, p, groups); }
+int bwd_few_rows(deers_ctx* ctx, const F32Params& p, int groups, int rm) {
+    return rm == 2 ? bwd_few<DP, 2>(ctx, p, groups) : bwd_few<DP, 1>(ctx, p, groups);
+}
 
 }  // namespace

@@ -13,10 +13,10 @@
 // (4 x 8 or 4 x 4 patches with RM = 4: 12 LDS.128 per 128 FFMA) and the same rows with float4 columns 4 tx + 32 j of the
 // accumulators.  RM = 2 and 1, blocks of 16 and 8 rows, are for calls of few blocks: each walks in half or a quarter of the time on SMs
 // that would idle, and every row is summed in the same order (B3 H4 T77 D48 forward 6.7 -> 4.6 -> 3.9 us, backward 13.6 -> 8.2; B1 H6 T100 D32
-// forward 4.9 -> 3.5 -> 2.9; the rules: attn_f32.cu).  Second products run two to an issue slot (forward, and from 64 wide tiles on backward; score products from
-// 96), and lanes lie so that shared-memory reads cost half.  Tiles arrive by cp.async: the next K (or Q) is fetched while the
-// current one's scores are turned into the second product, the next V (or dO) while the next scores are computed.
-// B8 H12 T2048 D64 forward 1909 -> 1688 us, backward 5821 -> 5642; B3 H4 T77 D48 forward 10.3 -> 6.8.
+// forward 4.9 -> 3.5 -> 2.9; the rules: attn_f32.cu).  Second products run two to an issue slot (forward, and from 64 wide tiles on backward;
+// score products from 96), and lanes lie so that shared-memory reads cost half.  Tiles arrive by cp.async: the next K (or Q) is fetched while
+// the current one's scores are turned into the second product, the next V (or dO) while the next scores are computed.  B8 H12 T2048 D64 forward
+// 1909 -> 1688 us, backward 5821 -> 5642; B3 H4 T77 D48 forward 10.3 -> 6.8.
 #pragma once
 #include "common.cuh"
 #include "f32_util.cuh"
@@ -259,7 +259,7 @@ struct Tile {
 };
 
 // ---------------------------------------------------------------------------
-// Forward: one block per (batch*head, 32-row query tile); the heaviest (latest) query tiles of all slices first.
+// Forward: one block per (batch*head, query tile of BM rows); the heaviest (latest) query tiles of all slices first.
 // ---------------------------------------------------------------------------
 template <int DP, int NG, int FBN, int RM>
 __global__ void __launch_bounds__(64 * NG, DP <= 32 && NG == 4 ? 2 : 1) attn_fwd_f32_kernel(const F32Params p) {
@@ -472,7 +472,7 @@ __device__ __forceinline__ void merge_store(const F32Params& p, const float* par
     }
 }
 
-// Scores to P in place: rows are query rows (ROWS_ARE_Q) or key rows of the 32 x BN tile; l2 / dl hold lse * log2e and delta
+// Scores to P in place: rows are query rows (ROWS_ARE_Q) or key rows of the BM x BN tile; l2 / dl hold lse * log2e and delta
 // of the tile's query rows.
 template <bool ROWS_ARE_Q, int RM, int NC>
 __device__ __forceinline__ void probabilities(const F32Params& p, float (&s)[RM][NC], const float* l2, int row0, int col0, int ty, int tx) {
@@ -490,9 +490,10 @@ __device__ __forceinline__ void probabilities(const F32Params& p, float (&s)[RM]
     }
 }
 
-// acc += tile * X with the 32 x BN tile handed through shared memory 32 columns at a time (rows stay inside a warp).
+// acc += tile * X with the BM x BN tile handed through shared memory 32 columns at a time (rows stay inside a warp).
 template <int DP, int RM, int NC>
-__device__ __forceinline__ void staged_product(float* stage, const float (&v)[RM][NC], const float* X, int ty, int tx, Acc<DP, Tile<DP>::BWD_PAIRS> (&acc)[RM]) {
+__device__ __forceinline__ void staged_product(float* stage, const float (&v)[RM][NC], const float* X, int ty, int tx,
+                                               Acc<DP, Tile<DP>::BWD_PAIRS> (&acc)[RM]) {
     constexpr int PLD = Tile<DP>::BWD_PLD;
 #pragma unroll
     for (int half = 0; half < NC / 4; ++half) {
@@ -506,7 +507,7 @@ __device__ __forceinline__ void staged_product(float* stage, const float (&v)[RM
     }
 }
 
-// dK / dV of 32 key rows: the groups walk the query tiles at or below the diagonal.
+// dK / dV of BM key rows: the groups walk the query tiles at or below the diagonal.
 template <int DP, int NG, int RM>
 __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt, int bh) {
     using L = Tile<DP, NG, 32, RM>;
@@ -543,7 +544,7 @@ __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt
 #pragma unroll
     for (int r = 0; r < RM; ++r) { dk[r].clear(); dv[r].clear(); }
 
-    RowDelta<DP, 2> rd;                                         // two threads per row of the 32-row tile
+    RowDelta<DP, 2> rd;                                         // two threads per row of the streamed tile
     float lse_next = 0.f;
     auto stats_ahead = [&](int q0) {
         const int row = q0 + t / 2;
@@ -588,7 +589,7 @@ __device__ __forceinline__ void bwd_dkdv(const F32Params& p, float* smem, int kt
     merge_store<DP, NG, BM>(p, grp0 + L::BWD_STREAM, L::BWD_GROUP, p.dv + b * p.sdv.b + h * p.sdv.h, p.sdv.t, k0, false);
 }
 
-// dQ of 32 query rows: the groups walk the key tiles at or left of the diagonal.
+// dQ of BM query rows: the groups walk the key tiles at or left of the diagonal.
 template <int DP, int NG, int RM>
 __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, int bh) {
     using L = Tile<DP, NG, 32, RM>;
@@ -665,7 +666,7 @@ __device__ __forceinline__ void bwd_dq(const F32Params& p, float* smem, int qt, 
 }
 
 // Both roles in one launch: row n of the grid holds every slice's n-th heaviest key tile, then every slice's n-th heaviest query
-// tile (gridDim.y ends at 65535; the longest sequence, 2^20, has 32768 tiles of a kind).
+// tile (gridDim.y ends at 65535; the longest sequence, 2^20, has 32768 tiles of a kind, and comes with too many blocks for smaller ones).
 template <int DP, int NG, int RM>
 __global__ void __launch_bounds__(64 * NG, DP <= 64 && NG == 4 ? 2 : 1) attn_bwd_f32_kernel(const F32Params p) {
     chain_wait();

@@ -237,8 +237,8 @@ int launch_embedding_bwd(deers_ctx* ctx, const float* dout, const long long* ids
                          float* dweight, bool cleared = false);
 int launch_cross_entropy_fwd(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, long long rows,
                              long long V, float* lse, float* picked, float* loss);
-int launch_cross_entropy_merge(deers_ctx* ctx, const float2* stats, int parts, const float* logits, long long ld, const long long* targets, long long rows,
-                               long long V, float* lse, float* picked);
+int launch_cross_entropy_merge(deers_ctx* ctx, const float2* stats, int parts, const float* logits, long long ld, const long long* targets,
+                               long long rows, long long V, float* lse, float* picked);
 int launch_cross_entropy_rows(deers_ctx* ctx, const float* logits, long long ld, const long long* targets, long long rows, long long V, float* lse,
                               float* picked);
 int launch_cross_entropy_loss(deers_ctx* ctx, const float* picked, long long rows, float* loss);

@@ -10,15 +10,13 @@
 //     dgrad    dx = dy  * W^T    : A = dy [M,N]  K-major,  B = W  [K,N] read as [N'=K, K'=N]: K-major
 //     wgrad    dW = x^T * dy     : A = x  [m,K]  read as [K'=m, M'=K]: MN-major,  B = dy [m,N] MN-major
 // Persistent: one CTA per SM walks 128 x 256 (or 192) output tiles (consecutive CTAs share a B column block, which
-// L2 then serves), or a pair of CTAs on two SMs walks tiles of 256 x 256.  Warp 0 streams 64-deep K blocks of A (16 KB) and B (32 KB) through a 4-stage ring (TMA,
-// 128-byte swizzle, out-of-range rows / columns read as zero), warp 1 issues four 128x256x16 tcgen05.mma
-// per K block into one of two TMEM accumulators, warps 2-9 move a finished accumulator to
-// registers 64 columns at a time, convert to f16 and store rows transposed within 8-lane groups
-// (contiguous 128-byte segments), then release the accumulator.
-// Few tiles and a long K (weight gradients) leave most SMs idle: there a cluster of CTAs shares a tile and its K
-// (768 x 768 x 8192: 18 tiles, 51 us on 18 SMs; 22 us as 24 narrower tiles of five parts.  768 x 2304 x 8192: 52 -> 31 us).
-// 192 columns where 256-wide tiles just miss a wave (8192 x 768 x 2304: 192 tiles on 148 SMs, 29 us; 256 tiles 24 us).
-// Bound: tensor pipe for large products (4096^3: 1.38 PFLOP/s by pairs, 1.25 without), L2 reads of both operands for the split ones.
+// L2 then serves), or a pair of CTAs on two SMs walks tiles of 256 x 256.  Warp 0 streams 64-deep K blocks of A (16 KB) and B (32 KB) through a
+// 4-stage ring (TMA, 128-byte swizzle, out-of-range rows / columns read as zero), warp 1 issues four 128x256x16 tcgen05.mma per K block into one
+// of two TMEM accumulators, warps 2-9 move a finished accumulator to registers 64 columns at a time, convert to f16 and store rows transposed
+// within 8-lane groups (contiguous 128-byte segments), then release the accumulator.  Few tiles and a long K (weight gradients) leave most SMs
+// idle: there a cluster of CTAs shares a tile and its K (768 x 768 x 8192: 18 tiles, 51 us on 18 SMs; 22 us as 24 narrower tiles of five parts.
+// 768 x 2304 x 8192: 52 -> 31 us).  192 columns where 256-wide tiles just miss a wave (8192 x 768 x 2304: 192 tiles on 148 SMs, 29 us; 256 tiles
+// 24 us).  Bound: tensor pipe for large products (4096^3: 1.38 PFLOP/s by pairs, 1.25 without), L2 reads of both operands for the split ones.
 #include "sm100_ptx.cuh"
 #include "tma_host.cuh"
 
@@ -194,7 +192,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
                     if (elect_one()) {
 #pragma unroll
                         for (int ks = 0; ks < GK / 16; ++ks) {             // ks < 4: a K-major step stays inside its block
-                            const uint64_t ad = a + (A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0)), bd = b + (B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0));
+                            const uint64_t ad = a + (A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0));
+                            const uint64_t bd = b + (B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0));
                             if constexpr (PAIR) umma_ss_pair(tmem + buf * 256u, ad, bd, IDESC, (kb > kb0 || ks > 0));
                             else umma_ss(tmem + buf * 256u, ad, bd, IDESC, (kb > kb0 || ks > 0));
                         }
@@ -456,7 +455,8 @@ extern "C" int deers_b200_gemm_f16(deers_ctx* ctx, int32_t M, int32_t N, int32_t
     // K-major A: [M rows][K inner], box {64, 128}; MN-major A: [K rows][M inner], box {64, 64}.  Same for B with
     // N (K-major box {64, tile columns}).
     if ((rc = a_mn_major ? make_tmap_matrix(ctx, &ta, a, K, M, lda, GK) : make_tmap_matrix(ctx, &ta, a, M, K, lda, GM))) return rc;
-    if ((rc = b_mn_major ? make_tmap_matrix(ctx, &tb, b, K, N, ldb, GK) : make_tmap_matrix(ctx, &tb, b, N, K, ldb, plan.pair ? plan.gn / 2 : plan.gn))) return rc;
+    const int b_rows = plan.pair ? plan.gn / 2 : plan.gn;
+    if ((rc = b_mn_major ? make_tmap_matrix(ctx, &tb, b, K, N, ldb, GK) : make_tmap_matrix(ctx, &tb, b, N, K, ldb, b_rows))) return rc;
     GemmParams p;
     p.c = (__half*)c; p.ldc = ldc; p.M = M; p.N = N; p.K = K; p.kb_chunk = plan.kb_chunk; p.err = ctx->dev_err;
     const auto orders = plan.pair ? gemm_orders<256, true> : plan.gn == 256 ? gemm_orders<256, false> : gemm_orders<192, false>;

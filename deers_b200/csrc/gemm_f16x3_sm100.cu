@@ -325,7 +325,7 @@ template <int TN, int B_MN, bool TURN>
 struct X3PairShape {
     static constexpr uint32_t RING = p_ring(TURN);
     static constexpr int BN = TN / 2;                                                    // columns of B a CTA brings
-    static constexpr int B_BLOCKS = (BN + 63) / 64;                                      // MN order: of 64 columns (half of the second is not used for 192)
+    static constexpr int B_BLOCKS = (BN + 63) / 64;    // MN order: of 64 columns (half of the second is not used for 192)
     static constexpr uint32_t B_TILE = B_MN ? B_BLOCKS * X_MN_BLOCK : BN * XK * 2u;      // hi or lo of a stage
     static constexpr uint32_t A_STAGE = 2 * X_TILE, B_STAGE = 2 * B_TILE;
     static constexpr int STAGES = RING / (A_STAGE + B_STAGE);
@@ -607,7 +607,10 @@ __global__ void __launch_bounds__(256) x3_reduce_kernel(const float* partial, in
             for (int q = 0; q < 8; ++q)
                 if (p0 + q < parts)
 #pragma unroll
-                    for (int e = 0; e < W; ++e) acc[e] = p0 + q ? acc[e] + reinterpret_cast<const float*>(&v[q])[e] : reinterpret_cast<const float*>(&v[q])[e];
+                    for (int e = 0; e < W; ++e) {
+                        const float x = reinterpret_cast<const float*>(&v[q])[e];
+                        acc[e] = p0 + q ? acc[e] + x : x;
+                    }
         }
         V o;
 #pragma unroll
@@ -715,7 +718,10 @@ X3Plan x3_plan(int M, int N, int K, int a_mn, int b_mn, int sm_count, int pairs)
     const long long pair_tiles = (long long)rows * ((n + tn - 1) / tn);
     const long long waves = (tiles + sm_count - 1) / sm_count, pair_waves = (pair_tiles + pairs - 1) / pairs;
     if (m <= XM) return pl;                                           // one CTA of a pair would have nothing to do
-    if (a_mn ? !(K >= 512 && tn == 192 && pair_waves < waves) : b_mn ? !(waves >= 6 && pair_waves <= waves) : !(pl.k_chunk >= 16 * XK && N % 4 == 0)) return pl;
+    const bool by_pairs = a_mn   ? K >= 512 && tn == 192 && pair_waves < waves
+                          : b_mn ? waves >= 6 && pair_waves <= waves
+                                 : pl.k_chunk >= 16 * XK && N % 4 == 0;
+    if (!by_pairs) return pl;
     pl = X3Plan{};
     pl.pair = true;
     pl.trans = a_mn != 0;
@@ -734,7 +740,8 @@ int x3_choose(deers_ctx* ctx, int M, int N, int K, int a_mn, int b_mn, bool rows
     const int rc = gemm_f16_pairs(ctx, pairs);
     if (rc) return rc;
     *pl = x3_plan(M, N, K, a_mn, b_mn, ctx->sm_count, *pairs);
-    if (pl->pair && ((!a_mn && !b_mn && !rows16 && pl->parts == 1) || ws_bytes < x3_partials(*pl, M, N))) *pl = x3_plan(M, N, K, a_mn, b_mn, ctx->sm_count, 0);
+    if (pl->pair && ((!a_mn && !b_mn && !rows16 && pl->parts == 1) || ws_bytes < x3_partials(*pl, M, N)))
+        *pl = x3_plan(M, N, K, a_mn, b_mn, ctx->sm_count, 0);
     return DEERS_OK;
 }
 
@@ -844,15 +851,16 @@ int launch_gemm_f16x3(deers_ctx* ctx, int M, int N, int K, const void* a_hi, con
     // K-major operand: [rows = M or N][inner = K], boxes of 64 K by the rows a CTA brings; MN-major: [rows = K][inner = M or N], box {64, 64}
     for (int h = 0; h < 2; ++h) {
         if ((rc = a_mn ? make_tmap_x3(ctx, &t[h], ap[h], K, m, lda, XK) : make_tmap_x3(ctx, &t[h], ap[h], m, K, lda, XM))) return rc;
-        if ((rc = b_mn ? make_tmap_x3(ctx, &t[2 + h], bp[h], K, n, ldb, XK) : make_tmap_x3(ctx, &t[2 + h], bp[h], n, K, ldb, pl.pair ? pl.tn / 2 : XN))) return rc;
+        const int b_rows = pl.pair ? pl.tn / 2 : XN;
+        if ((rc = b_mn ? make_tmap_x3(ctx, &t[2 + h], bp[h], K, n, ldb, XK) : make_tmap_x3(ctx, &t[2 + h], bp[h], n, K, ldb, b_rows))) return rc;
     }
     if (pl.pair) {
         X3PairParams p;
         p.c = out; p.ldc = ldo; p.M = m; p.N = n; p.K = K; p.parts = pl.parts; p.k_chunk = pl.k_chunk; p.out_scale = out_scale;
         p.resident = pl.resident; p.stats = stats; p.err = ctx->dev_err;
-        const bool wide = pl.tn == 192;
         if (pl.trans) rc = x3_launch_pair<1, 1, 192, true, false, false>(ctx, t, p, pairs);
-        else if (!b_mn) rc = wide ? x3_launch_pair<0, 0, 192, false, false, false>(ctx, t, p, pairs) : x3_launch_pair<0, 0, 128, false, false, false>(ctx, t, p, pairs);
+        else if (!b_mn) rc = pl.tn == 192 ? x3_launch_pair<0, 0, 192, false, false, false>(ctx, t, p, pairs)
+                                          : x3_launch_pair<0, 0, 128, false, false, false>(ctx, t, p, pairs);
         else if (!vec) rc = x3_launch_pair<0, 1, 128, false, false, true>(ctx, t, p, pairs);
         else if (stats && !split) {
             rc = x3_launch_pair<0, 1, 128, false, true, false>(ctx, t, p, pairs);

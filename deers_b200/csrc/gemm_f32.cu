@@ -42,18 +42,17 @@ __global__ void __launch_bounds__(TC_T, 1) gemm_f32_tc_group_kernel(const __grid
 // 64 x 96 4620 / 4710 / 5250, 32 x 96 2430 / 2900 / 3280, and 3800 to 9200 around it (148 tiles, K 320 and 1600).  The 96-wide tiles are
 // there for products whose 64-wide ones just miss one wave (1024 x 768: 192 tiles on 148 SMs, 128 of 64 x 96; 13.3 -> 11.7 us at K =
 // 192, and 16.3 -> 13.7 for 1024 x 192 x 768 in clusters of four).
-// 16 x 32 is for products that leave half of the SMs idle in 32 x 32: 100 x 576 x 192 3.7 -> 3.1 us, 231 x 192 x 192 3.7 -> 3.1, 64 x 64 x 400 in clusters
-// of four 3.9 -> 3.5, 100 x 192 x 768 in clusters of three, where 32 x 32 takes six, 5.5 -> 4.7 (five and more blocks meet for longer); two
-// blocks on an SM gain nothing (231 x 576 x 192 3.8 and 4.7).
-// The last is the tensor core's: a block starts only where one has left, and so do clusters, so all of it counts per wave.  Measured in a graph:
-// K = 64 4.6 us, 192 7.8, 384 12.0, 768 19.8, 1024 25.1; 1024 x 192 x 768 in clusters of four 9.5; three waves of K = 192 22.2.  Rows on no
-// 16-byte boundary take a tenth to a fifth more (TC_LOOSE).  Short products stay with the FFMA tiles (1024 x 192 x 192 5.1 us, here 6.3; 231 x 576 x 192
-// 3.8 and 6.1).
+// 16 x 32 is for products that leave half of the SMs idle in 32 x 32: 100 x 576 x 192 3.7 -> 3.1 us, 231 x 192 x 192 3.7 -> 3.1, 64 x 64 x 400
+// in clusters of four 3.9 -> 3.5, 100 x 192 x 768 in clusters of three, where 32 x 32 takes six, 5.5 -> 4.7 (five and more blocks meet for
+// longer); two blocks on an SM gain nothing (231 x 576 x 192 3.8 and 4.7).  The last is the tensor core's: a block starts only where one has
+// left, and so do clusters, so all of it counts per wave.  Measured in a graph: K = 64 4.6 us, 192 7.7, 384 12.0, 768 19.8, 1024 24.5; 1024 x
+// 192 x 768 in clusters of four 9.5; three waves of K = 192 22.2.  Rows on no 16-byte boundary take a tenth to a fifth more (TC_LOOSE).  Short
+// products stay with the FFMA tiles (1024 x 192 x 192 5.1 us, here 6.3; 231 x 576 x 192 3.8 and 6.1).
 struct Variant { int bm, bn; double walk, around; };
 constexpr int TC_CFG = 7;
 constexpr double TC_LOOSE = 1.1;
-constexpr Variant kVariants[8] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {32, 64, 2360, 4000}, {32, 32, 1680, 3200}, {64, 96, 5400, 5300}, {32, 96, 3200, 4300},
-                                  {16, 32, 970, 3800},                                   {TC_M, TC_N, 2640, 7300}};
+constexpr Variant kVariants[8] = {{64, 128, 7420, 6000}, {64, 64, 3700, 4900}, {32, 64, 2360, 4000}, {32, 32, 1680, 3200},
+                                  {64, 96, 5400, 5300},  {32, 96, 3200, 4300}, {16, 32, 970, 3800},  {TC_M, TC_N, 2640, 7300}};
 
 // How many clusters of 1..MAX_PARTS blocks (one block per SM) the device holds at a time: a cluster lives inside one
 // GPC, so e.g. 48 clusters of three do not fit 148 SMs although their 144 blocks would.
@@ -89,8 +88,8 @@ int cluster_capacity(deers_ctx* ctx) {
 
 // Picks the variant and the K split with the least estimated time: the blocks an SM has to run one after another times
 // a block's walk over its K, plus what a block spends before and after it (and at the cluster's meeting).
-// n products of one K; tc: what a tensor core's tile costs of its figure (0: not for these products); whole_heads: tiles must hold whole heads of that many columns (0: any).
-// cfg < 0: no variant does.
+// n products of one K; tc: what a tensor core's tile costs of its figure (0: not for these products); whole_heads: tiles must hold whole heads
+// of that many columns (0: any).  cfg < 0: no variant does.
 GemmPlan plan_gemm(int n, const int* M, const int* N, int K, double tc, const int* capacity, int whole_heads) {
     GemmPlan best{};
     best.cfg = -1;
@@ -109,7 +108,8 @@ GemmPlan plan_gemm(int n, const int* M, const int* N, int K, double tc, const in
             if (capacity[parts] < 1) continue;
             const double waves = (double)((tiles + capacity[parts] - 1) / capacity[parts]);
             const double meet = parts > 1 ? 3300.0 + (c != TC_CFG && parts > 4 ? 600.0 * (parts - 4) : 0.0) : 0.0;
-            const double cost = c == TC_CFG ? waves * (tc * (chunk * v.walk + v.around) + meet) : waves * chunk * v.walk + v.around + 1200.0 * (waves - 1.0) + meet;
+            const double cost = c == TC_CFG ? waves * (tc * (chunk * v.walk + v.around) + meet)
+                                            : waves * chunk * v.walk + v.around + 1200.0 * (waves - 1.0) + meet;
             if (best_cost < 0.0 || cost < best_cost) {
                 best_cost = cost;
                 best.cost = cost; best.cfg = c; best.parts = parts; best.k_chunk = chunk * BK; best.waves = (int)waves;
@@ -167,14 +167,16 @@ int launch_planned(deers_ctx* ctx, const GemmPlan& p, GemmArgs& g, int a_mn, int
     {
         KernelTimerScope ts(ctx, DEERS_K_GEMM);
         const bool aligned = g.a_vec && g.b_vec;
-        rc = p.cfg == TC_CFG ? (aligned ? launch_gemm_f32_tc(ctx, p.parts, g, a_mn, b_mn, fused) : launch_gemm_f32_tc_loose(ctx, p.parts, g, a_mn, b_mn))
-             : aligned ? launch_tiles<false>(ctx, p, g, a_mn, b_mn, fused) : launch_gemm_f32_loose(ctx, p, g, a_mn, b_mn, fused);
+        if (p.cfg == TC_CFG) rc = aligned ? launch_gemm_f32_tc(ctx, p.parts, g, a_mn, b_mn, fused) : launch_gemm_f32_tc_loose(ctx, p.parts, g, a_mn, b_mn);
+        else rc = aligned ? launch_tiles<false>(ctx, p, g, a_mn, b_mn, fused) : launch_gemm_f32_loose(ctx, p, g, a_mn, b_mn, fused);
     }
     ctx->launches += 1;
     return rc;
 }
 
-GemmPlan plan_single(deers_ctx* ctx, int M, int N, int K, bool aligned) { return plan_gemm(1, &M, &N, K, aligned ? 1.0 : TC_LOOSE, ctx->cluster_capacity, 0); }
+GemmPlan plan_single(deers_ctx* ctx, int M, int N, int K, bool aligned) {
+    return plan_gemm(1, &M, &N, K, aligned ? 1.0 : TC_LOOSE, ctx->cluster_capacity, 0);
+}
 
 // The plan of a product of normalised rows, and whether its tiles rotate heads of `heads` columns (0: there are none).
 GemmPlan plan_norm(deers_ctx* ctx, int M, int N, int K, bool aligned, int heads, bool* rotated) {
@@ -200,7 +202,8 @@ GemmPlan plan_norm(deers_ctx* ctx, int M, int N, int K, bool aligned, int heads,
 int launch_gemm_f32(deers_ctx* ctx, int M, int N, int K, const float* a, long long lda, int a_mn, const float* b,
                     long long ldb, int b_mn, float* c, long long ldc, int epi, const float* r, long long ldr, float* aux) {
     if (M == 0 || N == 0) return DEERS_OK;
-    // Row tiles lie along gridDim.y, which ends at 65535: taller products (tiles are 32 rows or more) go in several launches.
+    // Row tiles lie along gridDim.y, which ends at 65535: taller products go in several launches.  (Tiles of
+    // 16 rows are for products of few tiles: one so tall never takes them.)
     constexpr int MOST = 65535 * 32;
     for (; M > MOST; M -= MOST) {
         const int rc = launch_gemm_f32(ctx, MOST, N, K, a, lda, a_mn, b, ldb, b_mn, c, ldc, epi, r, ldr, aux);

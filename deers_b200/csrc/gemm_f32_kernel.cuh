@@ -249,7 +249,8 @@ __device__ __forceinline__ float4 patch_sum(const float* q, int parts) {
 // What the epilogue reads from global memory is requested before the block's meeting (behind it, it cost 400 to 700 cycles of a product's 5000), and
 // behind a cluster's, whose arrival would wait for it, beside the reads of the other blocks' patches.
 template <int BM, int BN, int KS, int THREADS, bool FUSED>
-__device__ __forceinline__ void finish_tile(const GemmArgs& g, float* const red, float* const sq_s, const int m0, const int n0, const int parts, const int rank) {
+__device__ __forceinline__ void finish_tile(const GemmArgs& g, float* const red, float* const sq_s, const int m0, const int n0, const int parts,
+                                            const int rank) {
     constexpr int RLD = BN + 4, ITEMS = (BM * BN / 4 + THREADS - 1) / THREADS;     // four columns each
     // Rows of the tile this block finishes: all of them, or its share of the cluster's.
     int r_begin = 0, r_end = BM;
@@ -363,10 +364,12 @@ __device__ __forceinline__ void finish_tile(const GemmArgs& g, float* const red,
                 // the other half of the head lies in this tile (tiles hold whole heads); rounded as the rotary pack does
                 const int half = g.rope_d / 2;
                 const float4 u = patch_sum<KS, BM * RLD>(second[i] ? q - half : q + half, parts);
-                const float p[4] = {u.x * inv, u.y * inv, u.z * inv, u.w * inv}, cs[4] = {c4[i].x, c4[i].y, c4[i].z, c4[i].w}, sn[4] = {s4[i].x, s4[i].y, s4[i].z, s4[i].w};
+                const float p[4] = {u.x * inv, u.y * inv, u.z * inv, u.w * inv};
+                const float cs[4] = {c4[i].x, c4[i].y, c4[i].z, c4[i].w}, sn[4] = {s4[i].x, s4[i].y, s4[i].z, s4[i].w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    o[e] = second[i] ? __fadd_rn(__fmul_rn(p[e], -sn[e]), __fmul_rn(o[e], cs[e])) : __fadd_rn(__fmul_rn(o[e], cs[e]), __fmul_rn(p[e], sn[e]));
+                    o[e] = second[i] ? __fadd_rn(__fmul_rn(p[e], -sn[e]), __fmul_rn(o[e], cs[e]))
+                                     : __fadd_rn(__fmul_rn(o[e], cs[e]), __fmul_rn(p[e], sn[e]));
             }
         }
         if (from_r) {

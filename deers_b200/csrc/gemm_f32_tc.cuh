@@ -22,8 +22,8 @@
 // meet as those of gemm_f32_kernel do; norm, rotation and epilogues are the same code.
 // What bounds it: shared memory, 185 KB a stage stored and read by the products (1470 cycles of its 128 bytes; the products take 900, the
 // conversions 700 issue slots), around it launch, first load and the way out;
-// 2600 cycles a stage as it is, because the sums of a stage are taken out between its products and the next one's.
-// In a graph, FFMA kernels and these (us): 1024 x 768 x 192 10.9 -> 7.8, 1024 x 192 x 768 12.8 -> 9.5, 1024 x 192 x 576 12.2 -> 8.3,
+// 2500 cycles a stage as it is, because the sums of a stage are taken out between its products and the next one's.
+// In a graph, FFMA kernels and these (us): 1024 x 768 x 192 10.9 -> 7.7, 1024 x 192 x 768 12.8 -> 9.1, 1024 x 192 x 576 12.2 -> 8.3,
 // 4096 x 768 x 192 40 -> 22, 1024 x 1152 x 384 27 -> 12.
 #pragma once
 #include "gemm_f32_kernel.cuh"
@@ -69,7 +69,8 @@ __device__ __forceinline__ void remainders(float& a, float& b, float fa, float f
 
 // What `large` adds up of the h: not finite any more when one of them is 2^25 or more (or several come near).
 constexpr float TC_LARGE = 0x1p104f;
-constexpr uint32_t TC_SMALL_SUM = (127u - 95u) << 23, TC_SMALL_SUM_OF_LARGE = (127u + 8u) << 23;     // bits of 2^-95 and 2^8: 2^-120 of values below 2^25, and of any
+// The bits of 2^-95 and 2^8: 2^-120 of values below 2^25, and of any.
+constexpr uint32_t TC_SMALL_SUM = (127u - 95u) << 23, TC_SMALL_SUM_OF_LARGE = (127u + 8u) << 23;
 
 // Splits eight values and stores the three parts, `part` bytes apart.
 __device__ __forceinline__ void split8(uint8_t* dst, uint32_t part, const float (&x)[8], float& large) {
@@ -105,7 +106,7 @@ __device__ __forceinline__ void split2(uint8_t* dst, uint32_t part, float a, flo
 // How the 512 threads take a stage of one operand, R rows of L floats (rows: m, n in K order, k in MN order) of which rv rows and lv floats
 // exist, from global memory and, split, into shared memory.
 // Rows on 16-byte boundaries go by eights.  Rows on any boundary go by twos, neighbouring lanes side by side: a warp's load touches 8 sectors
-// where single floats of eights would touch 32 (2133 x 769 x 1405 71 us, the next multiples of four by eights 59; FFMA kernels 146).
+// where single floats of eights would touch 32 (2133 x 769 x 1405 68 us; FFMA kernels 146).
 template <int R, int L, bool LOOSE>
 struct TcOperand {
     static constexpr int W = LOOSE ? 2 : 8;                        // floats of a piece
@@ -192,7 +193,8 @@ __device__ __forceinline__ void gemm_f32_tc_prologue() {
 }
 
 template <bool A_MN, bool B_MN, bool FUSED, bool LOOSE>
-__device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int tile_m, const int tile_n, const int part, const int parts, unsigned int* err) {
+__device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int tile_m, const int tile_n, const int part, const int parts,
+                                                 unsigned int* err) {
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint64_t* done = reinterpret_cast<uint64_t*>(tc_smem + TC_BARS);
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(done + TC_RING);
@@ -297,7 +299,8 @@ __device__ __forceinline__ void gemm_f32_tc_tile(const GemmArgs& g, const int ti
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
                     if (ks < steps) {
-                        const uint64_t ah = a + (A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0)), bh = b + (B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0));
+                        const uint64_t ah = a + (A_MN ? mnmajor_step(ks) : kmajor_step(ks, 0));
+                        const uint64_t bh = b + (B_MN ? mnmajor_step(ks) : kmajor_step(ks, 0));
                         const uint64_t am = ah + (TC_A >> 4), al = am + (TC_A >> 4), bm = bh + (TC_B >> 4);
                         umma_ss(tmem + (uint32_t)ks * TC_N, ah, bh, ID64, 0u);
                         umma_ss(tmem + TC_C1, ah, bm, ID128, s + ks > 0);              // h m | h l  (the parts of B follow one another)

@@ -12,9 +12,9 @@
 // rotated back by the attention backward straight into the fused [N, 3C] gradient buffer next to dV, and one GEMM for the sum of
 // the three input gradients.  Every launch is one of this library's kernels; there is no host round trip in a step.
 // The weight gradients are off the critical path (nothing in the backward reads them): the four of a block are one
-// launch on a second stream (four where one would be several waves of blocks, three and one for the block the backward ends with), forked from the main one where their operands
-// are complete and joined before the gradient norm; captured, the two streams become two branches of the step's graph.  What
-// they read is double-buffered by block.
+// launch on a second stream (four where one would be several waves of blocks, three and one for the block the backward ends with), forked from
+// the main one where their operands are complete and joined before the gradient norm; captured, the two streams become two branches of the
+// step's graph.  What they read is double-buffered by block.
 #include "common.cuh"
 
 #include <math.h>
@@ -249,7 +249,8 @@ int loss_and_backward(deers_gpt* m, const long long* ids, const long long* targe
     float* G = m->arena[1];
     for (bool& v : m->done_valid) v = false;
     // (the loss itself is added up beside the backward)
-    if (m->tc_head && m->ce_parts) GPT_TRY(launch_cross_entropy_merge(ctx, m->ce_stats, m->ce_parts, m->logits, Vld, targets, N, V, m->ce_lse, m->picked));
+    if (m->tc_head && m->ce_parts)
+        GPT_TRY(launch_cross_entropy_merge(ctx, m->ce_stats, m->ce_parts, m->logits, Vld, targets, N, V, m->ce_lse, m->picked));
     else GPT_TRY(launch_cross_entropy_rows(ctx, m->logits, Vld, targets, N, V, m->ce_lse, m->picked));
     const float* x_last = c.n_layer ? m->la[c.n_layer - 1].x2 : m->x0;
     if (m->tc_head) {

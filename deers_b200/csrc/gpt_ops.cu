@@ -193,9 +193,10 @@ __global__ void __launch_bounds__(256) cross_entropy_fwd_kernel(const float* log
 }
 
 // The same rows from what the head product has left of them: `parts` pairs (maximum, sum of exponentials relative to it) per row, [parts][rows].
-// A block takes eight rows, 128 threads each, every thread eight loads at a time.  1024 rows of 1572 parts 7 us behind the product where the pass over
-// the 206 MB of logits takes 42 (with 32 threads a row 18).
-__global__ void __launch_bounds__(1024) cross_entropy_merge_kernel(const float2* stats, int parts, const float* logits, long long ld, const long long* targets,
+// A block takes eight rows, 128 threads each, every thread eight loads at a time.  1024 rows of 1572 parts 7 us behind the product where the
+// pass over the 206 MB of logits takes 42 (with 32 threads a row 18).
+__global__ void __launch_bounds__(1024) cross_entropy_merge_kernel(const float2* stats, int parts, const float* logits, long long ld,
+                                                                   const long long* targets,
                                                                    long long rows, long long V, float* __restrict__ lse, float* __restrict__ picked,
                                                                    unsigned int* err) {
     chain_wait();
@@ -397,12 +398,12 @@ int launch_embedding_bwd(deers_ctx* ctx, const float* dout, const long long* ids
     return DEERS_OK;
 }
 
-int launch_cross_entropy_merge(deers_ctx* ctx, const float2* stats, int parts, const float* logits, long long ld, const long long* targets, long long rows,
-                               long long V, float* lse, float* picked) {
+int launch_cross_entropy_merge(deers_ctx* ctx, const float2* stats, int parts, const float* logits, long long ld, const long long* targets,
+                               long long rows, long long V, float* lse, float* picked) {
     {
         KernelTimerScope ts(ctx, DEERS_K_GPT);
-        DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_merge_kernel, (unsigned)((rows + 7) / 8), 1024, 0, 1, stats, parts, logits, ld, targets, rows, V, lse,
-                                           picked, ctx->dev_err));
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, cross_entropy_merge_kernel, (unsigned)((rows + 7) / 8), 1024, 0, 1, stats, parts, logits, ld, targets,
+                                           rows, V, lse, picked, ctx->dev_err));
     }
     ctx->launches += 1;
     return DEERS_OK;

@@ -270,17 +270,17 @@ int rms_launch(deers_ctx* ctx, long long rows, int C, float eps, const float* x,
     const long long cap = 16LL * ctx->sm_count;
     const unsigned grid = (unsigned)(want < cap ? want : cap);
     const float inv_n = (float)(1.0 / (double)C);               // mean = sum * (1/n as f64 -> f32), src/tensor.rs:461-465
-    {
+    const auto launch = [&](auto kernel, unsigned blocks) -> int {
         KernelTimerScope ts(ctx, DEERS_K_NORM);
-        if (BWD && vec && C <= 256)
-            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true, false, false, 2>, grid, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
-        else if (vec) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, true>, grid, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
-        else if (aligned && C <= 256 * RN_MAXV * 4) {
-            const unsigned bgrid = (unsigned)(rows < cap ? rows : cap);
-            DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_block_kernel<BWD>, bgrid, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
-        } else if (aligned) DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false, true>, grid, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
-        else DEERS_CUDA_TRY(ctx, launch_chained(ctx, rmsnorm_kernel<BWD, false>, grid, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
-    }
+        DEERS_CUDA_TRY(ctx, launch_chained(ctx, kernel, blocks, 256, 0, 1, x, dy, add, inv_in, out, inv_out, rows, C, eps, inv_n, n_out, nullptr, nullptr));
+        return DEERS_OK;
+    };
+    const int rc = BWD && vec && C <= 256              ? launch(rmsnorm_kernel<BWD, true, false, false, BWD ? 2 : RN_MAXV>, grid)
+                 : vec                                 ? launch(rmsnorm_kernel<BWD, true>, grid)
+                 : aligned && C <= 256 * RN_MAXV * 4   ? launch(rmsnorm_block_kernel<BWD>, (unsigned)(rows < cap ? rows : cap))
+                 : aligned                             ? launch(rmsnorm_kernel<BWD, false, true>, grid)
+                                                       : launch(rmsnorm_kernel<BWD, false>, grid);
+    if (rc) return rc;
     ctx->launches += 1;
     DEERS_CUDA_TRY(ctx, cudaGetLastError());
     return DEERS_OK;
