@@ -780,7 +780,8 @@ def run_gpt_step(args):
         peaks = load_peaks()
         # Two GEMM families: the head (lm_head forward, its weight and input gradients: 3 products of
         # 2 * 1024 * 50257 * 192 FLOPs) on the tensor core as split-f16 products, and the 72 products of the blocks, the
-        # larger on the tensor core as split-bf16 products, the smaller on the FFMA pipe, whose peak is what they are held against.  The roofline entry is the family that takes longer.
+        # larger on the tensor core as split-bf16 products, the smaller on the FFMA pipe, whose peak is what they are held
+        # against.  The roofline entry is the family that takes longer.
         n_tok, C_, Hm_, V_ = c["B"] * c["T"], c["n_embd"], c["mlp"], c["vocab"]
         head_flops = 6.0 * n_tok * C_ * V_
         block_flops = 6.0 * n_tok * c["n_layer"] * (4 * C_ * C_ + 2 * C_ * Hm_)
